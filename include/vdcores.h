@@ -69,6 +69,37 @@ int vdc_launch_async_full(int num_sms, int insts_per_sm, const void* compute_ins
                           const void* tma_descs, int* bars, const int* bars_init, uint64_t* profile, uint64_t stream,
                           uint64_t timeout_ns);
 
+/* One stage of a batched decode step or of a prefill chunk (2..128 rows), run as a kernel of its own.
+ *   kind VDC_STAGE_GEMM: projection of the k-chunk-major rows `x` [Bpad, K] with the M x K weights `w` (blocks of
+ *     VDC_STAGE_BLOCK rows; wfmt 0 bf16, 1 e4m3, 2 NVFP4, fp32 per-row `scales` for the last two); every block's K is
+ *     shared by `splits` CTAs of one cluster.  stats_in: sums of squares of the rows, which are
+ *     then RMS-normalised with the weights norm_w on their way to the tensor cores (0: taken as they are).  `mode` says where the result goes:
+ *       VDC_STAGE_QKV    heads: q/k norm (qk_norm, 0: none), rotation (`rope`), query rows to `out` [B, heads, 128], key
+ *                        and value rows to the pages state.NEWROW names in kpool / vpool
+ *       VDC_STAGE_RESID  hid += result; stats_out += squares of hid
+ *       VDC_STAGE_SILU   gate/up row pairs to out = silu(gate) * up
+ *       VDC_STAGE_ARGMAX the rows' largest logit into keys
+ *   kind VDC_STAGE_ATTN: attention of every row over its own pages (one row per sequence), queries `q`, result `out`
+ *   kind VDC_STAGE_ATTN_PREFILL: the same for rows that are consecutive positions of ONE sequence
+ *   kind VDC_STAGE_EMBED: embedding rows (table `w`, width K) to hid, stats_out[0] = squares, the other n_stats - 1 rows
+ *     of stats_out zeroed
+ *   kind VDC_STAGE_ADVANCE: keys -> next tokens, token log, state blocks moved on by one position
+ *   kind VDC_STAGE_COPY: M bytes from x to out
+ * Pointers are device addresses; 0 where a stage has no use for one. */
+typedef struct {
+  int32_t kind, mode, wfmt, B, Bpad, M, K, splits;
+  int32_t group, n_kv, n_pages, state_stride, log_stride, n_stats;
+  float eps, qk_eps;
+  uint64_t w, scales, x, stats_in, out, hid, norm_w, stats_out, keys;
+  uint64_t state, log, rope, qk_norm, kpool, vpool, q;
+} vdc_stage;
+
+/* Enqueues `n` stages (host array) on `stream`, in order, without synchronising: every stage is launched with
+ * programmatic stream serialisation, so that its CTAs start (and fetch weights) while the one in front finishes.
+ * Waits inside the kernels are bounded by timeout_ns (0 selects 2 s); what they report is fetched with
+ * vdc_read_status.  The stages are checked before anything is enqueued.  No counterpart in the reference. */
+int vdc_launch_stages(const vdc_stage* stages, int n, uint64_t stream, uint64_t timeout_ns);
+
 /* Synchronises `stream` and copies the device status block to *status; returns
  * its code.  Clears the block when `clear` is non-zero. */
 int vdc_read_status(uint64_t stream, vdc_status* status, int clear);

@@ -1,0 +1,187 @@
+"""The stage kernels of a batched step one by one (runtime.launch_stages), at the sizes where a tile, a K-split or a page
+walk can go wrong, against plain fp32 matmuls and softmaxes of the same bf16 inputs.
+
+Bounds: a result rounded once to bf16 is within 2^-8 of the exact one per element, 2^-9 rms and less in the 2-norm; the
+fp32 accumulation adds about 1e-6.  Rounding twice (bf16 product, then bf16 sum or norm weight) doubles that.  Attention
+rounds the probabilities to bf16 as well (another 2^-9).  4e-3 covers each of them."""
+import math
+
+import pytest
+import torch
+
+from tests.test_gpu_ops import seeded
+
+pytestmark = pytest.mark.gpu
+BF16 = torch.bfloat16
+REL = 4e-3
+
+
+def rel(a, b):
+    return float((a.float() - b.float()).norm() / b.float().norm().clamp_min(1e-20))
+
+
+def bpad(B):
+    return next(p for p in (16, 32, 64, 128) if B <= p)
+
+
+def packed_rows(x, dev):
+    from vdcores_b200.batch import pack_kc
+    full = torch.zeros(bpad(x.shape[0]), x.shape[1], dtype=BF16)
+    full[:x.shape[0]] = x
+    return pack_kc(full.to(dev))
+
+
+def run(dev, *stages):
+    from vdcores_b200 import runtime
+    arr = (runtime.Stage * len(stages))(*stages)
+    runtime.launch_stages(arr, torch.cuda.current_stream(dev).cuda_stream, 500_000_000)
+    runtime.read_status(torch.cuda.current_stream(dev).cuda_stream)
+
+
+def weights(M, K, fmt, dev, seed=2):
+    """(device tensor in the stages' layout, scales or None, the fp32 matrix it stands for)"""
+    from vdcores_b200 import isa
+    from vdcores_b200.batch import pack_blocks, pack_blocks_fp8, pack_blocks_nvfp4
+    from vdcores_b200.decode import quantize_fp8_rows, quantize_nvfp4_rows
+    w = seeded((M, K), seed, 0.05)
+    if fmt == "bf16":
+        return pack_blocks(w.to(dev), isa.STAGE_BLOCK), None, w.float()
+    if fmt == "fp8":
+        codes, sc = quantize_fp8_rows(w)
+        return (pack_blocks_fp8(codes.to(dev), isa.STAGE_BLOCK), sc.to(dev),
+                codes.view(torch.float8_e4m3fn).float() * sc[:, None])
+    rows, ts = quantize_nvfp4_rows(w)
+    grid = torch.tensor([0.0, 0.5, 1.0, 1.5, 2.0, 3.0, 4.0, 6.0])
+    grid = torch.cat((grid, -grid))
+    codes, bs = rows[:, :K // 2], rows[:, K // 2:].contiguous().view(torch.float8_e4m3fn).float()
+    vals = torch.stack((grid[(codes & 15).long()], grid[(codes >> 4).long()]), -1).view(M, K // 16, 16) * bs[..., None]
+    return (pack_blocks_nvfp4(rows.to(dev), K, isa.STAGE_BLOCK), ts.expand(M).contiguous().to(dev), vals.view(M, K) * ts)
+
+
+CASES = [(1, 256, 16, 4, "bf16"), (3, 512, 144, 8, "bf16"), (16, 4096, 256, 8, "bf16"), (40, 768, 400, 2, "bf16"),
+         (128, 1024, 128, 1, "bf16"), (100, 14336, 128, 8, "bf16"), (2, 512, 48, 1, "fp8"), (33, 1024, 272, 4, "fp8"),
+         (128, 4096, 128, 2, "fp8"), (5, 1024, 16, 8, "nvfp4"), (64, 2048, 272, 1, "nvfp4"), (128, 1024, 112, 2, "nvfp4")]
+
+
+def gemm(dev, fmt, B, M, K, splits, w, sc, x, **kw):
+    from vdcores_b200 import isa, runtime
+    return runtime.Stage(kind=isa.STAGE_GEMM, wfmt={"bf16": 0, "fp8": 1, "nvfp4": 2}[fmt], B=B, Bpad=bpad(B), M=M, K=K,
+                         splits=splits, w=w.data_ptr(), scales=sc.data_ptr() if sc is not None else 0, x=x.data_ptr(), **kw)
+
+
+@pytest.mark.parametrize("B,K,M,splits,fmt", CASES)
+def test_projection_with_residual(cuda_device, B, K, M, splits, fmt):
+    from vdcores_b200 import isa
+    from vdcores_b200.batch import unpack_kc
+    dev, Bp = cuda_device, bpad(B)
+    x, h = seeded((B, K), 1), seeded((B, M), 3)
+    w, sc, wf = weights(M, K, fmt, dev)
+    xd, hd = packed_rows(x, dev), packed_rows(h, dev)
+    stats = torch.zeros(128, device=dev)
+    run(dev, gemm(dev, fmt, B, M, K, splits, w, sc, xd, mode=isa.STAGE_RESID, hid=hd.data_ptr(), stats_out=stats.data_ptr()))
+    ref = h.float() + x.float() @ wf.t()
+    got = unpack_kc(hd.cpu(), Bp, M)
+    assert rel(got[:B], ref) < REL and float(got[B:].abs().max() if B < Bp else 0) == 0
+    assert torch.allclose(stats.cpu()[:B], got[:B].float().pow(2).sum(1), rtol=1e-4) and float(stats[B:].abs().sum()) == 0
+
+
+@pytest.mark.parametrize("B,K,M,splits,fmt", CASES)
+def test_projection_gate_up_and_argmax(cuda_device, B, K, M, splits, fmt):
+    from vdcores_b200 import isa
+    from vdcores_b200.batch import unpack_kc
+    dev, Bp = cuda_device, bpad(B)
+    x = seeded((B, K), 5)
+    w, sc, wf = weights(M, K, fmt, dev, seed=6)
+    stats = torch.zeros(128)
+    stats[:B] = seeded((B,), 7).float().abs() * K + 1
+    xd, sd, out = packed_rows(x, dev), stats.to(dev), torch.zeros(Bp * M // 2, dtype=BF16, device=dev)
+    keys = torch.zeros(B, dtype=torch.int64, device=dev)
+    nw = (1 + 0.1 * seeded((K,), 4).float()).to(BF16)
+    nwd = nw.to(dev)
+    common = dict(stats_in=sd.data_ptr(), norm_w=nwd.data_ptr(), eps=1e-5)
+    run(dev, gemm(dev, fmt, B, M, K, splits, w, sc, xd, mode=isa.STAGE_SILU, out=out.data_ptr(), **common))
+    xn = (x.float() * torch.rsqrt(stats[:B, None] / K + 1e-5)).to(BF16).float() * nw.float()
+    y = xn.to(BF16).float() @ wf.t()
+    yb = y.to(BF16).float()
+    ref = torch.nn.functional.silu(yb[:, 0::2]) * yb[:, 1::2]
+    assert rel(unpack_kc(out.cpu(), Bp, M // 2)[:B], ref) < 2 * REL
+    if fmt == "bf16":
+        run(dev, gemm(dev, fmt, B, M, K, splits, w, sc, xd, mode=isa.STAGE_ARGMAX, keys=keys.data_ptr(), **common))
+        rows = 0xFFFFFFFF - (keys.cpu() & 0xFFFFFFFF)
+        top = y.max(1).values
+        assert bool((y[torch.arange(B), rows] >= top - 2.0 ** -7 * top.abs()).all())
+
+
+@pytest.mark.parametrize("B,fmt,norm", [(3, "bf16", True), (16, "nvfp4", True), (128, "bf16", True), (16, "fp8", False)])
+def test_many_blocks_stream_in_order(cuda_device, B, fmt, norm):
+    """More CTAs than SMs, so that two stream side by side, and rings of 3 to 8 stages behind 64 chunks: every pass gives
+    the same bits (each CTA alone owns its block's sums), and the sums of the inputs."""
+    from vdcores_b200 import isa
+    from vdcores_b200.batch import unpack_kc
+    dev, Bp, K, M = cuda_device, bpad(B), 4096, 28672
+    x = seeded((B, K), 11)
+    w, sc, wf = weights(M, K, fmt, dev, seed=12)
+    stats = torch.zeros(128)
+    stats[:B] = x.float().pow(2).sum(1)
+    xd, sd, nwd = packed_rows(x, dev), stats.to(dev), torch.ones(K, dtype=BF16, device=dev)
+    outs = []
+    for _ in range(12):
+        out = torch.zeros(Bp * M // 2, dtype=BF16, device=dev)
+        kw = dict(stats_in=sd.data_ptr(), norm_w=nwd.data_ptr(), eps=1e-5) if norm else {}
+        run(dev, gemm(dev, fmt, B, M, K, 1, w, sc, xd, mode=isa.STAGE_SILU, out=out.data_ptr(), **kw))
+        outs.append(out)
+    assert all(torch.equal(o, outs[0]) for o in outs)
+    xn = (x.float() * torch.rsqrt(stats[:B, None] / K + 1e-5)).to(BF16).float() if norm else x.float()
+    yb = (xn.to(dev).double() @ wf.to(dev).double().t()).to(BF16).float()
+    ref = torch.nn.functional.silu(yb[:, 0::2]) * yb[:, 1::2]
+    assert rel(unpack_kc(outs[0].cpu(), Bp, M // 2)[:B], ref.cpu()) < 2 * REL
+
+
+@pytest.mark.parametrize("kind", ["decode", "prefill"])
+@pytest.mark.parametrize("G,n_kv,B,splits,lens", [(4, 2, 3, 8, [1, 64, 65]), (8, 1, 2, 2, [700, 129]), (4, 1, 17, 1, None),
+                                                  (8, 2, 9, 4, None), (4, 2, 128, 2, None)])
+def test_attention(cuda_device, kind, G, n_kv, B, splits, lens):
+    """decode: every row over its own pages (lengths of one row, whole pages, one row more; more CTAs than pages).
+    prefill: rows are consecutive positions of one sequence, the last ones repeated, tiles that end past the rows."""
+    from vdcores_b200 import isa, runtime
+    from vdcores_b200.batch import unpack_kc
+    from vdcores_b200.decode import kv_page_swizzle
+    dev, Bp, D = cuda_device, bpad(B), 128
+    if kind == "prefill":
+        pos = torch.arange(90, 90 + B).clamp_(max=90 + max(0, B - 3))
+        n_tab, tables = 5, torch.randperm(5, generator=torch.Generator().manual_seed(1))[None].expand(B, -1)
+    else:
+        pos = torch.tensor([l - 1 for l in lens]) if lens else torch.randint(0, 300, (B,), generator=torch.Generator().manual_seed(3))
+        n_tab = int(pos.max()) // 64 + 2
+        tables = torch.randperm(B * n_tab, generator=torch.Generator().manual_seed(2)).view(B, n_tab)
+    k, v = seeded((int(tables.max()) + 1, n_kv, 64, D), 8), seeded((int(tables.max()) + 1, n_kv, 64, D), 9)
+    for b in range(B):          # rows past a sequence's last position: whatever an earlier request left
+        last = int(pos.max()) if kind == "prefill" else int(pos[b])
+        for t in (k, v):
+            t[tables[b, last // 64], :, last % 64 + 1:] = float("nan")
+    q = seeded((B, n_kv * G, D), 10, 2.0)
+    state = torch.zeros(B, isa.ST_PAGETABLE + n_tab, dtype=torch.int32)
+    state[:, isa.ST_POS] = pos
+    state[:, isa.ST_PAGETABLE:] = tables
+    kd, vd, qd, sd = kv_page_swizzle(k).to(dev), kv_page_swizzle(v).to(dev), q.to(dev), state.to(dev)
+    out = torch.zeros(Bp * n_kv * G * D, dtype=BF16, device=dev)
+    run(dev, runtime.Stage(kind=isa.STAGE_ATTN if kind == "decode" else isa.STAGE_ATTN_PREFILL, B=B, Bpad=Bp, splits=splits,
+                           group=G, n_kv=n_kv, n_pages=n_tab, state_stride=state.shape[1], state=sd.data_ptr(),
+                           q=qd.data_ptr(), out=out.data_ptr(), kpool=kd.data_ptr(), vpool=vd.data_ptr()))
+    got = unpack_kc(out.cpu(), Bp, n_kv * G * D).view(Bp, n_kv, G, D)
+    for b in range(B):
+        T = int(pos[b]) + 1
+        kk = k[tables[b]].transpose(0, 1).reshape(n_kv, -1, D)[:, :T].float()
+        vv = v[tables[b]].transpose(0, 1).reshape(n_kv, -1, D)[:, :T].float()
+        p = torch.softmax(q[b].view(n_kv, G, D).float() @ kk.transpose(1, 2) / math.sqrt(D), -1)
+        assert rel(got[b], p @ vv) < REL, f"row {b}"
+    assert float(got[B:].abs().max() if B < Bp else 0) == 0
+
+
+def test_stages_refuse_bad_arguments(cuda_device):
+    from vdcores_b200 import isa, runtime
+    good = dict(kind=isa.STAGE_GEMM, mode=isa.STAGE_SILU, B=2, Bpad=16, M=64, K=128, splits=1, w=1 << 20, x=1 << 20, out=1 << 20)
+    for bad in (dict(K=96), dict(M=8), dict(splits=3), dict(splits=4), dict(Bpad=24), dict(B=17), dict(w=0), dict(x=8), dict(wfmt=1),
+                dict(kind=9), dict(mode=7)):
+        with pytest.raises(runtime.VdcError):
+            runtime.launch_stages((runtime.Stage * 1)(runtime.Stage(**{**good, **bad})))

@@ -2,24 +2,26 @@
 
 The reference pads every decode batch to 8 request slots and pushes it through
 its 64x8 WGMMA GEMV tile (reference include/task/gemv.cuh:13-128,
-python/dae/schedule.py:404-570).  Here the projections of a batch run on the
-tcgen05 tensor cores: the batch sits on the 128 lanes of the accumulator in
-tensor memory, each SM owns groups of 16 weight rows of every projection, and
-activations live in HBM in the k-chunk-major layout the tensor cores read
-without swizzling (csrc/isa.h).  Attention, RoPE, QK-norm and the KV cache are
-the batch-1 tasks, one unit per (sequence, KV head, split), each sequence with
-its own state block and page table.
+python/dae/schedule.py:404-570).  Here a step is a list of stage kernels
+(csrc/stage_kernels.cu), one per projection and attention, launched back to
+back with programmatic dependent launch: the batch sits on the 128 lanes of a
+tcgen05 accumulator in tensor memory, blocks of 128 weight rows on its columns,
+and activations live in HBM in the k-chunk-major layout the tensor cores read
+without swizzling (csrc/isa.h).  Every sequence has its own state block, page
+table and length.
+
+The helpers above the engine (`emit_projection` and the layouts it packs) emit
+the same projection as tasks of the megakernel.
 """
 from __future__ import annotations
 
-import math
 from typing import List
 
 import torch
 
 from . import isa, runtime
 from .decode import BF16, DecodeConfig, DecodeEngine, kv_page_swizzle
-from .program import Dst, Program, Src, slots_for
+from .program import Program, Src
 
 
 def pack_kc(x: torch.Tensor) -> torch.Tensor:
@@ -35,47 +37,50 @@ def unpack_kc(flat: torch.Tensor, R: int, K: int) -> torch.Tensor:
 BLOCK_ROWS = 256    # weight rows per projection block = accumulator columns of one tensor-core task
 
 
-def projection_blocks(M: int):
+def projection_blocks(M: int, rows: int = BLOCK_ROWS):
     """[(first row, rows)] of a projection with M output rows (a multiple of 16)."""
     assert M % 16 == 0
-    return [(r, min(BLOCK_ROWS, M - r)) for r in range(0, M, BLOCK_ROWS)]
+    return [(r, min(rows, M - r)) for r in range(0, M, rows)]
 
 
-def pack_blocks(w: torch.Tensor) -> torch.Tensor:
-    """[M, K] -> flat: every block of 256 rows (the last one may be smaller) k-chunk-major, so
+def _pack_blocks(rows_of, M: int, bytes_or_elems_per_row: int, out: torch.Tensor, rows: int) -> torch.Tensor:
+    """Fills `out` block by block; rows_of(r0, blocks, n) returns the packed rows r0 .. r0 + blocks * n - 1 as `blocks`
+    blocks of n rows: all full blocks at once, then the smaller last one."""
+    full = M // rows
+    if full:
+        out[:full * rows * bytes_or_elems_per_row] = rows_of(0, full, rows).reshape(-1)
+    if M % rows:
+        out[full * rows * bytes_or_elems_per_row:] = rows_of(full * rows, 1, M % rows).reshape(-1)
+    return out
+
+
+def pack_blocks(w: torch.Tensor, rows: int = BLOCK_ROWS) -> torch.Tensor:
+    """[M, K] -> flat: every block of `rows` rows (the last one may be smaller) k-chunk-major, so
     that any K-range of a block is one contiguous piece; block (r0, N) starts at element r0 * K."""
     M, K = w.shape
-    out = torch.empty(M * K, dtype=w.dtype, device=w.device)
-    full = M // BLOCK_ROWS
-    if full:
-        out[:full * BLOCK_ROWS * K] = (w[:full * BLOCK_ROWS].reshape(full, BLOCK_ROWS // 8, 8, K // 8, 8)
-                                       .permute(0, 3, 1, 2, 4).reshape(-1))
-    if M % BLOCK_ROWS:
-        out[full * BLOCK_ROWS * K:] = pack_kc(w[full * BLOCK_ROWS:])
-    return out
+    return _pack_blocks(lambda r0, nb, n: w[r0:r0 + nb * n].reshape(nb, n // 8, 8, K // 8, 8).permute(0, 3, 1, 2, 4),
+                        M, K, torch.empty(M * K, dtype=w.dtype, device=w.device), rows)
 
 
-def pack_blocks_fp8(codes: torch.Tensor) -> torch.Tensor:
-    """[M, K] e4m3 bytes -> flat: per block of 256 rows the layout [K/16][N/8][8 rows][16 k],
+def pack_blocks_fp8(codes: torch.Tensor, rows: int = BLOCK_ROWS) -> torch.Tensor:
+    """[M, K] e4m3 bytes -> flat: per block of `rows` rows the layout [K/16][N/8][8 rows][16 k],
     which a 16-byte load turns into two adjacent bf16 pieces of the tensor-core operand layout."""
     M, K = codes.shape
-    out = torch.empty(M * K, dtype=codes.dtype, device=codes.device)
-    for r0, n in projection_blocks(M):
-        out[r0 * K:(r0 + n) * K] = codes[r0:r0 + n].reshape(n // 8, 8, K // 16, 16).permute(2, 0, 1, 3).reshape(-1)
-    return out
+    return _pack_blocks(lambda r0, nb, n: codes[r0:r0 + nb * n].reshape(nb, n // 8, 8, K // 16, 16).permute(0, 3, 1, 2, 4),
+                        M, K, torch.empty(M * K, dtype=codes.dtype, device=codes.device), rows)
 
 
-def pack_blocks_nvfp4(rows: torch.Tensor, K: int) -> torch.Tensor:
-    """[M, K/2 + K/16] NVFP4 rows (e2m1 pairs, then the e4m3 block scales) -> flat: per block of 256 rows
+def pack_blocks_nvfp4(w: torch.Tensor, K: int, rows: int = BLOCK_ROWS) -> torch.Tensor:
+    """[M, K/2 + K/16] NVFP4 rows (e2m1 pairs, then the e4m3 block scales) -> flat: per block of `rows` rows
     and per 16 inputs, the rows' 8 code bytes followed by the rows' scale bytes ([K/16][N x 8 | N]), so that
     any K-range of a block is one contiguous piece of 9 N bytes per 16 inputs."""
-    M = rows.shape[0]
-    codes, bs = rows[:, :K // 2].reshape(M, K // 16, 8), rows[:, K // 2:]
-    out = torch.empty(M * K * 9 // 16, dtype=rows.dtype, device=rows.device)
-    for r0, n in projection_blocks(M):
-        blk = torch.cat((codes[r0:r0 + n].permute(1, 0, 2).reshape(K // 16, n * 8), bs[r0:r0 + n].t()), dim=1)
-        out[r0 * K * 9 // 16:(r0 + n) * K * 9 // 16] = blk.reshape(-1)
-    return out
+    M = w.shape[0]
+    codes, bs = w[:, :K // 2].reshape(M, K // 16, 8), w[:, K // 2:]
+
+    def rows_of(r0, nb, n):
+        c = codes[r0:r0 + nb * n].reshape(nb, n, K // 16, 8).transpose(1, 2).reshape(nb, K // 16, n * 8)
+        return torch.cat((c, bs[r0:r0 + nb * n].reshape(nb, n, K // 16).transpose(1, 2)), dim=2)
+    return _pack_blocks(rows_of, M, K * 9 // 16, torch.empty(M * K * 9 // 16, dtype=w.dtype, device=w.device), rows)
 
 
 def chunk_geometry(N: int, Bpad: int, K: int):
@@ -138,13 +143,11 @@ def emit_projection(P: Program, *, sms, load, w_addr, M, K, x_addr, B, Bpad, mod
 
 
 class BatchDecodeEngine(DecodeEngine):
-    """`batch` sequences decoded together, one kernel launch per step.  Dense models; the layer
+    """`batch` sequences decoded together, one list of stage kernels per step.  Dense models; the layer
     projections are bf16, e4m3 with per-row scales (wkind "fp8") or NVFP4 (wkind "nvfp4": e2m1 values, e4m3 block
     scales, fp32 tensor scale), everything else bf16."""
     GEMV_PROJECTIONS = False
-    FULL_KERNEL = True       # the attention variants for long page walks live in the full kernel only
     SHARED_CACHE = False     # True: the batch rows are consecutive positions of ONE sequence (prefill.PrefillEngine)
-    WITH_VOCAB_PROJECTION = True   # False: the program ends after the last layer (prefill chunks before the last)
 
     def __init__(self, cfg: DecodeConfig, batch: int, max_seq: int, device="cuda:0", num_sms=None, taps=False,
                  page_perm_seed=None, max_steps: int = 256, timeout_ns: int = 2_000_000_000, wkind: str = "bf16"):
@@ -158,7 +161,7 @@ class BatchDecodeEngine(DecodeEngine):
         self.hidden = z(Bp * H)                       # k-chunk-major [Bpad, H]
         self.attn_out = z(Bp * cfg.q_width)           # k-chunk-major [Bpad, q_width]
         self.act = z(Bp * F)                          # k-chunk-major [Bpad, F]
-        self.qkv = z(B, self.qkv_rows)                # per sequence: [G q heads | k | v] per KV head
+        self.q = z(B, cfg.q_width)                    # rotated query heads
         self.keys = z(B, dt=torch.int64)              # argmax keys (u64), zero between steps
         # per-sequence sums of squares of the hidden matrix after the embedding / each residual add
         # (the RMSNorm statistics of the projection that reads it); zero between steps
@@ -167,10 +170,7 @@ class BatchDecodeEngine(DecodeEngine):
         self.n_splits = 1 if units >= self.num_sms else max(1, min(self.num_sms // units, self.max_pages))
         self.pages_per_split = (self.max_pages + self.n_splits - 1) // self.n_splits
         self.n_splits = (self.max_pages + self.pages_per_split - 1) // self.pages_per_split
-        self.attn_part = z(B, cfg.n_kv_heads, self.n_splits, self.rec_floats, dt=torch.float32)
-        if self.SHARED_CACHE and cfg.group == 4:      # split records of two positions x four heads (eight query rows)
-            self.attn_part_pair = z((B + 1) // 2, cfg.n_kv_heads, self.n_splits, 8 * isa.HEAD_DIM + 16, dt=torch.float32)
-        self.attn_cnt = z(L, B, cfg.n_kv_heads, dt=torch.int32)
+        self.stages = None
         self.state_words = isa.ST_PAGETABLE + self.max_pages
         self.state = z(B, self.state_words, dt=torch.int32)
         self.state_host = torch.zeros(B, self.state_words, dtype=torch.int32).pin_memory()
@@ -219,155 +219,69 @@ class BatchDecodeEngine(DecodeEngine):
         return self.weight_bytes() + self.batch * (cfg.hidden * 2 + 2 * cfg.kv_width * 2 * (pos + 1) * cfg.n_layers)
 
     # ------------------------------------------------------------------ program
-    def _build_program(self):
-        cfg = self.cfg
-        L, H, F, V, G = cfg.n_layers, cfg.hidden, cfg.ffn, cfg.vocab, cfg.group
-        D, S, B, Bp = isa.HEAD_DIM, self.num_sms, self.batch, self.bpad
-        P = Program(S, insts_per_sm=isa.MAX_INSTS)
-        st, sw = self.state.data_ptr(), self.state_words
-        page_bytes = isa.KV_PAGE * D * 2
-        page_stride = cfg.n_kv_heads * page_bytes
-        page_shift = int(math.log2(page_stride))
-        assert 1 << page_shift == page_stride
-        hid, qkv, ao, act = (t.data_ptr() for t in (self.hidden, self.qkv, self.attn_out, self.act))
-        load = [0] * S
-        packed = {"wqkv": [], "wo": [], "wgu": [], "wd": []}
-        # fp32 scratch / counters per projection kind and the packed weights outlive a rebuild of the program
-        self.scratch = getattr(self, "scratch", None) or {}
-        self._pack_cache = getattr(self, "_pack_cache", None) or {}
+    def _splits(self, units: int, per_sm: int, most: int) -> int:
+        """CTAs (one cluster) that share a unit: the largest power of two with at most per_sm CTAs for every SM."""
+        s = 1
+        while s < 8 and units * s * 2 <= per_sm * self.num_sms and s * 2 <= most:
+            s *= 2
+        return s
 
+    def _gemm(self, name, l, w, x, mode, norm=None, **kw):
+        # norm: (index of the rows' sums of squares, norm weights) of a projection with a fused input RMSNorm
+        """Projection stage over layer l's matrix `name` ("lm": the vocabulary projection, bf16 in every engine)."""
+        wf = self.wkind if name != "lm" else "bf16"
+        K = {"wo": self.cfg.q_width, "wd": self.cfg.ffn}.get(name, self.cfg.hidden)
+        if (name, l) not in self._pack_cache:     # the programs of one engine share the packed copies
+            self._pack_cache[name, l] = {"bf16": lambda: pack_blocks(w, isa.STAGE_BLOCK),
+                                         "fp8": lambda: pack_blocks_fp8(w, isa.STAGE_BLOCK),
+                                         "nvfp4": lambda: pack_blocks_nvfp4(w, K, isa.STAGE_BLOCK)}[wf]()
+        blocks = -(-w.shape[0] // isa.STAGE_BLOCK)
+        return runtime.Stage(
+            kind=isa.STAGE_GEMM, mode=mode, wfmt={"bf16": 0, "fp8": 1, "nvfp4": 2}[wf], B=self.batch, Bpad=self.bpad,
+            M=w.shape[0], K=K, splits=self._splits(blocks, 2, K // 64), w=self._pack_cache[name, l].data_ptr(),
+            scales=self.scales[name][l].data_ptr() if wf != "bf16" else 0, x=x.data_ptr(),
+            stats_in=self.stats[norm[0]].data_ptr() if norm else 0, norm_w=norm[1].data_ptr() if norm else 0,
+            eps=self.cfg.eps, **kw)
+
+    def _plan(self, vocab: bool = True):
+        """The stages of one step; vocab False: it ends after the last layer (prefill chunks before the last)."""
+        cfg, B = self.cfg, self.batch
+        L, G = cfg.n_layers, cfg.group
+        hid = self.hidden.data_ptr()
         stat = lambda i: self.stats[i].data_ptr()
-
-        def gemm_stage(w, name, K, x_addr, x_wait, mode, out_addr, release, norm=None, ld=0, keys=0, stats=0):
-            M = w.shape[0]
-            wf = self.wkind if name is not None else "bf16"     # the vocabulary projection stays bf16
-            fp8 = wf != "bf16"
-            key = (name, len(packed[name]) if name is not None else 0)
-            if key not in self._pack_cache:     # a second program of the same engine (prefill) shares the packed copies
-                self._pack_cache[key] = (pack_blocks_fp8(w) if wf == "fp8" else pack_blocks_nvfp4(w, K) if wf == "nvfp4"
-                                         else pack_blocks(w))
-            pk = self._pack_cache[key]
-            if name is not None:
-                packed[name].append(pk)
-            kind = name or "lm"
-            n_blocks = len(projection_blocks(M))
-            if kind not in self.scratch:      # fp32 partial sums and arrival counters, zero between uses
-                self.scratch[kind] = (torch.zeros(n_blocks * B * BLOCK_ROWS, dtype=torch.float32, device=self.dev),
-                                      torch.zeros(n_blocks, dtype=torch.int32, device=self.dev))
-            scr, cnt = self.scratch[kind]
-            sms = sorted(range(S), key=lambda i: (load[i], i))
-            emit_projection(P, sms=sms, load=load, w_addr=pk.data_ptr(), M=M, K=K, x_addr=x_addr, B=B, Bpad=Bp,
-                            mode=mode, out_addr=out_addr, scratch_addr=scr.data_ptr(), counter_addr=cnt.data_ptr(),
-                            x_wait=x_wait, release=release, norm_addr=norm.data_ptr() if norm is not None else None,
-                            eps=cfg.eps, ld=ld, keys_addr=keys, stats_addr=stats, wfmt=wf,
-                            scales_addr=self.scales[name][len(packed[name]) - 1].data_ptr() if fp8 else 0)
-            return pk
-
-        def tap(l, wait, release):
-            sm = self._pick(load, 1)[0]
-            n = Bp * H * 2
-            P.copy(sm, Src(hid, n, wait=wait), Dst(self.taps[l].data_ptr(), n, release=release), n)
-
-        # ---- embedding rows into the hidden matrix
-        b_hid = P.new_barrier()
-        for b, sm in enumerate(self._pick(load, B)):
-            P.embed_pack(sm, b0=b, count=1, Bpad=Bp, state_addr=st, state_stride_words=sw, hidden=H,
-                         table_addr=self.embed.data_ptr(), out_addr=hid, stats_addr=stat(0), release=b_hid)
+        state = dict(state=self.state.data_ptr(), state_stride=self.state_words)
+        heads = dict(group=G, n_kv=cfg.n_kv_heads, **state)
+        out = [runtime.Stage(kind=isa.STAGE_EMBED, B=B, Bpad=self.bpad, K=cfg.hidden, w=self.embed.data_ptr(), hid=hid,
+                             stats_out=stat(0), n_stats=2 * L + 1, **state)]
+        tile = 64 // G      # rows of one prefill attention unit
+        units = cfg.n_kv_heads * (-(-B // tile) if self.SHARED_CACHE else B)
+        attn_kind = isa.STAGE_ATTN_PREFILL if self.SHARED_CACHE else isa.STAGE_ATTN
+        self.attn_splits = self._splits(units, 4, self.max_pages)
         for l in range(L):
-            # ---- QKV projection with fused input RMSNorm
-            b_qkv = P.new_barrier()
-            gemm_stage(self.wqkv[l], "wqkv", H, hid, b_hid, isa.GEMM_MODE_STORE_ROWS, qkv, b_qkv, norm=self.ln1[l],
-                       ld=self.qkv_rows, stats=stat(2 * l))
-            if self.taps_enabled and l > 0:
-                tap(l - 1, b_hid, b_qkv)
-            # ---- attention: one unit per (sequence, KV head, split)
-            b_merge = P.new_barrier()
-            P.add_releases(b_merge, (B // 2 if self.SHARED_CACHE and G == 4 and B % 2 == 0 else B) * cfg.n_kv_heads)
-            units = [(b, h, s) for s in range(self.n_splits) for b in range(B) for h in range(cfg.n_kv_heads)]
-            kp, vp = self.kpool[l].data_ptr(), self.vpool[l].data_ptr()
-            grp = (G + 2) * D * 2
-            b_rows = None
-            if self.SHARED_CACHE:
-                # the rows of all the chunk's positions go to the pools first: position p attends to rows the
-                # tasks of positions < p write in this same launch
-                b_rows = P.new_barrier()
-                P.add_releases(b_rows, B * cfg.n_kv_heads)
-                for (b, h), sm in zip([(b, h) for b in range(B) for h in range(cfg.n_kv_heads)],
-                                      self._pick(load, B * cfg.n_kv_heads)):
-                    sb = st + 4 * sw * b
-                    P.attn_decode(
-                        sm, G=G, state_addr=sb,
-                        rope=Src(self.rope.data_ptr(), D * 4, indirect=(sb + 4 * isa.ST_POS, 9, None)),
-                        norm_w=Src(self.qknorm[l].data_ptr(), 2 * D * 2) if cfg.qk_norm else None,
-                        qkv=Src(qkv + (b * self.qkv_rows) * 2 + h * grp, grp, wait=b_qkv),
-                        k_page_addr=kp + h * page_bytes, v_page_addr=vp + h * page_bytes, page_shift=page_shift,
-                        base_page=0, max_pages=0, records_addr=0, counter_addr=0, out_addr=0, split=0, n_splits=1,
-                        release=b_rows, qk_eps=cfg.qk_norm_eps, append=True)
-            pairs = self.SHARED_CACHE and G == 4 and B % 2 == 0
-            if pairs:
-                # two consecutive prompt positions per unit: half the units walk the same pages (prefill only)
-                units = [(b, h, s) for s in range(self.n_splits) for b in range(0, B, 2) for h in range(cfg.n_kv_heads)]
-            for (b, h, s), sm in zip(units, self._pick(load, len(units), 2 * page_bytes * self.pages_per_split)):
-                sb = st + 4 * sw * b
-                if pairs:
-                    P.attn_decode(
-                        sm, G=8, state_addr=sb, pair=(sw, self.qkv_rows),
-                        rope=Src(self.rope.data_ptr(), D * 4, indirect=(sb + 4 * isa.ST_POS, 9, None)),
-                        norm_w=Src(self.qknorm[l].data_ptr(), 2 * D * 2) if cfg.qk_norm else None,
-                        qkv=Src(qkv + (b * self.qkv_rows) * 2 + h * grp, grp, wait=b_rows), wait_issue=b_rows,
-                        k_page_addr=kp + h * page_bytes, v_page_addr=vp + h * page_bytes, page_shift=page_shift,
-                        base_page=s * self.pages_per_split, max_pages=self.pages_per_split,
-                        records_addr=self.attn_part_pair[b // 2, h].data_ptr(),
-                        counter_addr=self.attn_cnt[l, b, h].data_ptr(),
-                        out_addr=ao + (h * G * D) * Bp * 2, split=s, n_splits=self.n_splits, release=b_merge,
-                        qk_eps=cfg.qk_norm_eps, packed=(b, Bp))
-                    continue
-                P.attn_decode(
-                    sm, G=G, state_addr=sb,
-                    rope=Src(self.rope.data_ptr(), D * 4, indirect=(sb + 4 * isa.ST_POS, 9, None)),
-                    norm_w=Src(self.qknorm[l].data_ptr(), 2 * D * 2) if cfg.qk_norm else None,
-                    qkv=Src(qkv + (b * self.qkv_rows) * 2 + h * grp, grp, wait=b_qkv if b_rows is None else b_rows),
-                    wait_issue=b_rows,
-                    k_page_addr=kp + h * page_bytes, v_page_addr=vp + h * page_bytes, page_shift=page_shift,
-                    base_page=s * self.pages_per_split, max_pages=self.pages_per_split,
-                    records_addr=self.attn_part[b, h].data_ptr(), counter_addr=self.attn_cnt[l, b, h].data_ptr(),
-                    out_addr=ao + (h * G * D) * Bp * 2, split=s, n_splits=self.n_splits, release=b_merge,
-                    qk_eps=cfg.qk_norm_eps, packed=(b, Bp))
-            # ---- output projection, residual add into the hidden matrix
-            b_o = P.new_barrier()
-            gemm_stage(self.wo[l], "wo", cfg.q_width, ao, b_merge, isa.GEMM_MODE_ADD_PACKED, hid, b_o,
-                       stats=stat(2 * l + 1))
-            # ---- gate/up projection with fused post-attention RMSNorm and SiLU-mul
-            b_gu = P.new_barrier()
-            gemm_stage(self.wgu[l], "wgu", H, hid, b_o, isa.GEMM_MODE_SILU_PAIRS, act, b_gu, norm=self.ln2[l],
-                       stats=stat(2 * l + 1))
-            # ---- down projection, residual add
-            b_hid = P.new_barrier()
-            gemm_stage(self.wd[l], "wd", F, act, b_gu, isa.GEMM_MODE_ADD_PACKED, hid, b_hid, stats=stat(2 * l + 2))
-        # ---- final norm, vocabulary projection, per-sequence argmax
-        if self.WITH_VOCAB_PROJECTION:
-            b_lm = P.new_barrier()
-            self.lm_head_packed = gemm_stage(self.lm_head, None, H, hid, b_hid, isa.GEMM_MODE_ARGMAX, 0, b_lm,
-                                             norm=self.norm_w, keys=self.keys.data_ptr(), stats=stat(2 * L))
+            pools = dict(kpool=self.kpool[l].data_ptr(), vpool=self.vpool[l].data_ptr())
+            out.append(self._gemm("wqkv", l, self.wqkv[l], self.hidden, isa.STAGE_QKV, (2 * l, self.ln1[l]), out=self.q.data_ptr(),
+                                  rope=self.rope.data_ptr(), qk_norm=self.qknorm[l].data_ptr() if cfg.qk_norm else 0,
+                                  qk_eps=cfg.qk_norm_eps, **heads, **pools))
+            out.append(runtime.Stage(kind=attn_kind, B=B, Bpad=self.bpad, splits=self.attn_splits, n_pages=self.max_pages,
+                                     q=self.q.data_ptr(), out=self.attn_out.data_ptr(), **heads, **pools))
+            out.append(self._gemm("wo", l, self.wo[l], self.attn_out, isa.STAGE_RESID, hid=hid,
+                                  stats_out=stat(2 * l + 1)))
+            out.append(self._gemm("wgu", l, self.wgu[l], self.hidden, isa.STAGE_SILU, (2 * l + 1, self.ln2[l]),
+                                  out=self.act.data_ptr()))
+            out.append(self._gemm("wd", l, self.wd[l], self.act, isa.STAGE_RESID, hid=hid, stats_out=stat(2 * l + 2)))
             if self.taps_enabled:
-                tap(L - 1, b_hid, b_lm)
-        else:
-            b_lm = b_hid        # a prefill chunk that is not the prompt's last: nobody reads its logits
-        sm = self._pick(load, 1)[0]
-        P.batch_advance(sm, batch=B, state_addr=st, state_stride_words=sw, keys_addr=self.keys.data_ptr(),
-                        log_addr=self.token_log.data_ptr(), log_stride=self.max_steps, wait=b_lm,
-                        stats_addr=self.stats.data_ptr(), n_stats=self.stats.numel())
-        self.packed = {k: v for k, v in packed.items()}     # keeps the device copies alive
-        n = max(max(len(x) for x in P.m), max(len(x) for x in P.c)) + 2
-        P.insts_per_sm = ((n + 15) // 16) * 16
-        c, m, bars = P.finalize()
-        self.program = P
-        self.insts_per_sm = P.insts_per_sm
-        self.cinsts = torch.from_numpy(c).to(self.dev)
-        self.minsts = torch.from_numpy(m).to(self.dev)
-        self.bars_init = torch.from_numpy(bars).to(self.dev)
-        self.bars.copy_(self.bars_init)
-        self.launches_per_step = 1
+                out.append(runtime.Stage(kind=isa.STAGE_COPY, x=hid, out=self.taps[l].data_ptr(), M=self.hidden.numel(), K=2))
+        if vocab:
+            out.append(self._gemm("lm", 0, self.lm_head, self.hidden, isa.STAGE_ARGMAX, (2 * L, self.norm_w),
+                                  keys=self.keys.data_ptr()))
+            out.append(runtime.Stage(kind=isa.STAGE_ADVANCE, B=B, Bpad=self.bpad, keys=self.keys.data_ptr(),
+                                     log=self.token_log.data_ptr(), log_stride=self.max_steps, **state))
+        return (runtime.Stage * len(out))(*out)
+
+    def _build_program(self):
+        self._pack_cache = getattr(self, "_pack_cache", None) or {}
+        self.stages = self._plan()
+        self.launches_per_step = len(self.stages)
 
     # ------------------------------------------------------------------ state
     def set_state(self, pos: int, token: int, b: int = None):
@@ -386,7 +300,6 @@ class BatchDecodeEngine(DecodeEngine):
         s[isa.ST_MAXPAGES] = self.max_pages
         s[isa.ST_PAGETABLE:] = table
         self.state[b].copy_(s, non_blocking=True)
-        self.attn_cnt.zero_()
         self.keys.zero_()
         self.stats.zero_()
         self.positions[b] = pos
@@ -431,6 +344,15 @@ class BatchDecodeEngine(DecodeEngine):
         return out
 
     # ------------------------------------------------------------------ decode
+    def step_async(self):
+        """Enqueues one decode step (its stages, one kernel each); no synchronisation."""
+        assert self.stages is not None, "load weights first"
+        if self.pos >= self.max_seq or self.steps_done >= self.max_steps:
+            raise RuntimeError("out of KV pages or token-log space")
+        runtime.launch_stages(self.stages, self.stream.cuda_stream, self.timeout_ns)
+        self.pos += 1
+        self.steps_done += 1
+
     def generate(self, n_steps: int) -> List[List[int]]:
         """n_steps greedy steps, device resident; returns [n_steps][batch] token ids."""
         first = self.steps_done

@@ -16,6 +16,9 @@ extern "C" cudaError_t vdc_megakernel_launch(int num_sms, const void* cinsts, co
                                              int* bars, uint64_t* profile, vdc_status* status, int insts_per_sm,
                                              uint64_t timeout_ns, cudaStream_t stream, int ref_ops);
 
+extern "C" cudaError_t vdc_stage_prepare();
+extern "C" cudaError_t vdc_stage_launch(const vdc_stage* s, vdc_status* status, uint64_t timeout_ns, cudaStream_t stream);
+
 namespace {
 
 thread_local std::string g_err;
@@ -85,6 +88,8 @@ int vdc_init(void) {
   g_sm_count[dev] = prop.multiProcessorCount;
   e = vdc_megakernel_prepare();
   if (e != cudaSuccess) return fail_cuda(e, "cudaFuncSetAttribute(MaxDynamicSharedMemorySize)");
+  e = vdc_stage_prepare();
+  if (e != cudaSuccess) return fail_cuda(e, "cudaFuncSetAttribute(stage kernels)");
   vdc_status* st = nullptr;
   e = cudaMalloc(&st, sizeof(vdc_status));
   if (e != cudaSuccess) return fail_cuda(e, "cudaMalloc(status)");
@@ -132,6 +137,53 @@ int vdc_launch_async_full(int num_sms, int insts_per_sm, const void* compute_ins
                           uint64_t timeout_ns) {
   return launch_async_impl(num_sms, insts_per_sm, compute_insts, memory_insts, tma_descs, bars, bars_init, profile, stream,
                            timeout_ns, 1);
+}
+
+static const char* check_stage(const vdc_stage& s) {
+  auto pow2 = [](int v) { return v > 0 && (v & (v - 1)) == 0; };
+  auto al16 = [](uint64_t p) { return (p & 15) == 0; };
+  if (s.kind == VDC_STAGE_COPY) return s.x && s.out && s.M > 0 && s.K > 0 ? nullptr : "copy stage: null pointer or size";
+  if (s.B < 1 || s.B > 128 || s.Bpad < s.B || (s.Bpad != 16 && s.Bpad != 32 && s.Bpad != 64 && s.Bpad != 128))
+    return "stage: rows out of range";
+  if (s.kind == VDC_STAGE_EMBED)
+    return s.K % 8 == 0 && s.w && s.hid && s.state && s.stats_out ? nullptr : "embedding stage: bad argument";
+  if (s.kind == VDC_STAGE_ADVANCE) return s.state && s.keys && s.log ? nullptr : "advance stage: null pointer";
+  if (!pow2(s.splits) || s.splits > 8) return "stage: splits must be 1, 2, 4 or 8";
+  if (s.kind == VDC_STAGE_ATTN || s.kind == VDC_STAGE_ATTN_PREFILL) {
+    if ((s.group != 4 && s.group != 8) || s.n_kv < 1 || s.n_kv > 65535 || s.n_pages < 1) return "attention stage: bad shape";
+    return s.state && s.q && s.out && s.kpool && s.vpool && al16(s.q) && al16(s.out) && al16(s.kpool) && al16(s.vpool)
+               ? nullptr : "attention stage: null or misaligned pointer";
+  }
+  if (s.kind != VDC_STAGE_GEMM) return "stage: unknown kind";
+  if (s.wfmt < 0 || s.wfmt > 2 || s.M < 16 || s.M % 16 || s.K < 64 || s.K % 64 || s.splits > s.K / 64)
+    return "projection stage: bad shape";
+  if (!s.w || !s.x || !al16(s.w) || !al16(s.x) || !al16(s.scales) || (s.wfmt && !s.scales))
+    return "projection stage: null or misaligned pointer";
+  if (s.stats_in && (!s.norm_w || !al16(s.norm_w))) return "projection stage: norm weights missing or misaligned";
+  switch (s.mode) {
+    case VDC_STAGE_QKV:
+      if (s.group < 1 || s.n_kv < 1 || s.M != s.n_kv * (s.group + 2) * VDC_HEAD_DIM) return "QKV stage: rows do not match the heads";
+      return s.out && s.state && s.rope && s.kpool && s.vpool ? nullptr : "QKV stage: null pointer";
+    case VDC_STAGE_RESID: return s.hid && s.stats_out ? nullptr : "residual stage: null pointer";
+    case VDC_STAGE_SILU: return s.out ? nullptr : "gate/up stage: null pointer";
+    case VDC_STAGE_ARGMAX: return s.keys ? nullptr : "argmax stage: null pointer";
+    default: return "projection stage: unknown mode";
+  }
+}
+
+int vdc_launch_stages(const vdc_stage* stages, int n, uint64_t stream, uint64_t timeout_ns) {
+  int dev;
+  if (int r = current_device(&dev)) return r;
+  if (!g_status[dev]) return fail_arg("vdc_init was not called on this device");
+  if (!stages || n < 1) return fail_arg("no stages");
+  for (int i = 0; i < n; ++i)
+    if (const char* why = check_stage(stages[i])) return fail_arg(why);
+  if (timeout_ns == 0) timeout_ns = 2000000000ull;
+  for (int i = 0; i < n; ++i) {
+    cudaError_t e = vdc_stage_launch(&stages[i], g_status[dev], timeout_ns, reinterpret_cast<cudaStream_t>(stream));
+    if (e != cudaSuccess) return fail_cuda(e, "stage launch");
+  }
+  return VDC_OK;
 }
 
 int vdc_read_status(uint64_t stream, vdc_status* status, int clear) {

@@ -39,6 +39,20 @@
 #define VDC_FLAG_BITS 6
 #define VDC_MOP(id, flags) ((uint16_t)(((id) << VDC_FLAG_BITS) | (flags)))
 
+// Stage kernels (batched decode, chunked prefill): kinds of a vdc_stage, epilogues of a projection stage, weight rows
+// per projection block
+#define VDC_STAGE_GEMM 1
+#define VDC_STAGE_ATTN 2
+#define VDC_STAGE_ATTN_PREFILL 3
+#define VDC_STAGE_EMBED 4
+#define VDC_STAGE_ADVANCE 5
+#define VDC_STAGE_COPY 6
+#define VDC_STAGE_QKV 0
+#define VDC_STAGE_RESID 1
+#define VDC_STAGE_SILU 2
+#define VDC_STAGE_ARGMAX 3
+#define VDC_STAGE_BLOCK 128
+
 // X(name, value)
 #define VDC_MEMORY_OPS(X)                                                              \
   X(OP_TERMINATE, VDC_MOP(1, 0))                                                       \

@@ -233,7 +233,7 @@ struct Ctx {
 
 __device__ __forceinline__ void* slot_ptr(const Ctx& c, int slot) { return c.slots + (size_t)slot * VDC_SLOT_BYTES; }
 
-__device__ __noinline__ void raise_abort(const Ctx& c, int code, int role, int pc, int opcode, int bar, int aux) {
+static __device__ __noinline__ void raise_abort(const Ctx& c, int code, int role, int pc, int opcode, int bar, int aux) {
   if (atomicCAS(&c.status->abort, 0, 1) == 0) {
     c.status->code = code;
     c.status->sm = c.sm;

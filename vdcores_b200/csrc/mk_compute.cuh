@@ -1,9 +1,7 @@
 // Compute virtual core of the megakernel: queue access and the decode tasks.
 #pragma once
-#include <cuda_fp4.h>
-#include <cuda_fp8.h>
-
 #include "mk_common.cuh"
+#include "mk_umma.cuh"
 
 namespace vdc {
 
@@ -294,10 +292,6 @@ __device__ __forceinline__ void gemv_chunk_mixed(const uint8_t* w, const uint8_t
 // vector has been converted to fp16 in place (exact for normalised activations); 16 weights per lane and
 // step become fp16 pairs with one conversion per pair and go straight into the mixed-precision FMA
 // d(f32) = a(f16) * b(f16) + c(f32): half a conversion and one FMA per weight, nothing is widened.
-__device__ __forceinline__ float2 e4m3x2_to_float2(uint32_t pair16) {   // widened pair (batched path's conversion)
-  const __half2_raw h = __nv_cvt_fp8x2_to_halfraw2((__nv_fp8x2_storage_t)pair16, __NV_E4M3);
-  return __half22float2(*reinterpret_cast<const __half2*>(&h));
-}
 __device__ __forceinline__ uint32_t e4m3x2_to_f16x2(uint32_t pair16) {
   uint32_t d;
   asm("cvt.rn.f16x2.e4m3x2 %0, %1;" : "=r"(d) : "h"((unsigned short)pair16));
@@ -376,10 +370,6 @@ __device__ __forceinline__ void gemv_chunk_fp8(const uint8_t* w, const uint8_t* 
 // the 16 products of a block are accumulated with half2 FMAs, the block sum is
 // widened, multiplied by the block scale and accumulated in fp32.  The per-row
 // fp32 scale (the tensor scale) is applied by the caller.
-__device__ __forceinline__ __half2 e2m1x2_to_half2(uint32_t byte) {
-  const __half2_raw h = __nv_cvt_fp4x2_to_halfraw2((__nv_fp4x2_storage_t)byte, __NV_E2M1);
-  return *reinterpret_cast<const __half2*>(&h);
-}
 __device__ __forceinline__ float e4m3_to_float(uint32_t byte) {
   const __half_raw h = __nv_cvt_fp8_to_halfraw((__nv_fp8_storage_t)byte, __NV_E4M3);
   return __half2float(*reinterpret_cast<const __half*>(&h));

@@ -9,66 +9,11 @@
 // groups of 16 and each sequence's outputs land in one thread's registers.
 #pragma once
 #include "mk_compute.cuh"
+#include "mk_umma.cuh"
 
 namespace vdc {
 
 constexpr uint32_t kTmemCols = 512;
-
-// ------------------------------------------------------------------------- //
-// tcgen05 helpers
-// ------------------------------------------------------------------------- //
-__device__ __forceinline__ void tc_fence_before() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
-__device__ __forceinline__ void tc_fence_after() { asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); }
-// Warp-wide: allocates `ncols` columns of tensor memory, the base address lands in *dst (shared memory).
-__device__ __forceinline__ void tmem_alloc(uint32_t* dst, uint32_t ncols) {
-  asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(dst)), "r"(ncols)
-               : "memory");
-  asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
-}
-__device__ __forceinline__ void tmem_dealloc(uint32_t taddr, uint32_t ncols) {
-  asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(taddr), "r"(ncols) : "memory");
-}
-// Shared-memory operand descriptor, no swizzle, K-major: 8 rows x 16 bytes form one contiguous
-// 128-byte core matrix; `lbo` = byte distance between the two core matrices a 16-element k-step
-// spans, `sbo` = byte distance between consecutive 8-row groups.  Bit 46 marks the sm_100 format.
-__device__ __forceinline__ uint64_t umma_desc(uint32_t saddr, uint32_t lbo, uint32_t sbo) {
-  return (uint64_t)((saddr & 0x3FFFFu) >> 4) | ((uint64_t)(lbo >> 4) << 16) | ((uint64_t)(sbo >> 4) << 32) |
-         (1ull << 46);
-}
-// Instruction descriptor of kind::f16: fp32 accumulator, bf16 A and B, both K-major, M = 128.
-__device__ __forceinline__ uint32_t umma_idesc_bf16_m128(int n) {
-  return (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(n >> 3) << 17) | ((128u >> 4) << 24);
-}
-// One thread issues: D[tmem] (+)= A[smem] * B[smem]^T for one k-step of 16.
-__device__ __forceinline__ void umma_bf16(uint32_t d_tmem, uint64_t adesc, uint64_t bdesc, uint32_t idesc,
-                                          uint32_t accumulate) {
-  asm volatile(
-      "{\n\t.reg .pred p;\n\t"
-      "setp.ne.b32 p, %4, 0;\n\t"
-      "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}" ::"r"(d_tmem),
-      "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate)
-      : "memory");
-}
-// The mbarrier gets one arrival when every tensor-core operation this thread issued so far is done.
-__device__ __forceinline__ void umma_commit(uint64_t* bar) {
-  asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(smem_u32(bar))
-               : "memory");
-}
-// Warp-wide: 16 consecutive fp32 columns of this thread's lane.
-__device__ __forceinline__ void tmem_ld16(uint32_t taddr, uint32_t (&r)[16]) {
-  asm volatile(
-      "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];"
-      : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]),
-        "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
-      : "r"(taddr)
-      : "memory");
-  asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-}
-
-// Byte offset of the 16-byte piece holding (b, k..k+7) in a k-chunk-major [Bpad, K] matrix.
-__device__ __forceinline__ size_t kc_piece(int bpad, int b, int k) {
-  return ((size_t)(k >> 3) * (size_t)(bpad >> 3) + (size_t)(b >> 3)) * 128 + (size_t)(b & 7) * 16;
-}
 
 // Bounded wait on one of the tensor-core completion barriers (thread 0 only).
 __device__ __forceinline__ bool mma_wait(Compute& q, unsigned commit_index) {

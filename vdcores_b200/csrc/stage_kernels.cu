@@ -1,0 +1,1021 @@
+// Stage kernels: the batched decode step and the chunked prefill as one kernel per stage.
+//
+// A step of 2..128 rows runs, per layer: QKV projection (with per-head norm, rotation and the cache append in its
+// epilogue), attention, output projection, gate/up projection, down projection.  The rows sit on the 128 lanes of a
+// tcgen05 accumulator, a block of 128 weight rows on its columns.  Why kernels and not tasks of the megakernel: with
+// many rows a projection block needs a K-split whose partial sums meet (here through distributed shared memory inside
+// one cluster, in the megakernel through fp32 atomics in L2 and a last arrival that ran the block's epilogue alone), and
+// a stage boundary needs no spinning: programmatic dependent launch starts the next kernel's CTAs while this one drains,
+// and they fill their shared memory with weights before they wait for its results (427 -> 384 us for two layers and a
+// 128256-row vocabulary projection at 3 rows).
+//
+// Measured against the megakernel's program, two Llama-3.1-8B-shaped layers and a small vocabulary (B200): 3 rows at
+// 1000 positions 416 -> 252 us, 32 rows with e4m3 weights 758 -> 379, 64 rows at 2100 positions 932 -> 497, 128 rows
+// 1025 -> 577, a 2048-token prompt 15.8 -> 8.2 ms.
+#include "mk_umma.cuh"
+
+#include "../../include/vdcores.h"
+
+namespace vdc {
+
+constexpr int kBlk = VDC_STAGE_BLOCK;   // weight rows of a projection block: accumulator columns
+constexpr int kKc = 64;                 // inputs per chunk
+constexpr int kMaxRing = 8;
+constexpr int kGemmThreads = 320;       // producer warp, MMA warp, eight warps that convert weights and run the epilogue
+constexpr int kEpiThreads = 256;
+// Shared memory of one CTA.  Two CTAs fit an SM (the register budget allows it too), so that one streams while the
+// other is in its prologue or epilogue, and the next stage's CTAs move in while the last ones of this stage finish.
+constexpr int kGemmSmem = 110 * 1024;
+constexpr int kEpiLd = kBlk + 4;        // row stride of the fp32 exchange tile: eight rows start in eight bank groups
+
+// ------------------------------------------------------------------------- //
+// helpers
+// ------------------------------------------------------------------------- //
+__device__ __forceinline__ void grid_dep_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void grid_dep_launch() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+__device__ __forceinline__ void cluster_arrive() { asm volatile("barrier.cluster.arrive.release;" ::: "memory"); }
+__device__ __forceinline__ void cluster_wait() { asm volatile("barrier.cluster.wait.acquire;" ::: "memory"); }
+__device__ __forceinline__ uint32_t cluster_rank() {
+  uint32_t r;
+  asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
+  return r;
+}
+__device__ __forceinline__ uint32_t peer_smem(uint32_t saddr, uint32_t rank) {
+  uint32_t a;
+  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(a) : "r"(saddr), "r"(rank));
+  return a;
+}
+__device__ __forceinline__ float4 ld_cluster4(uint32_t a) {
+  float4 v;
+  asm volatile("ld.shared::cluster.v4.f32 {%0,%1,%2,%3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "r"(a) : "memory");
+  return v;
+}
+__device__ __forceinline__ float2 ld_cluster2(uint32_t a) {
+  float2 v;
+  asm volatile("ld.shared::cluster.v2.f32 {%0,%1}, [%2];" : "=f"(v.x), "=f"(v.y) : "r"(a) : "memory");
+  return v;
+}
+__device__ __forceinline__ float ld_cluster1(uint32_t a) {
+  float v;
+  asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(v) : "r"(a) : "memory");
+  return v;
+}
+
+// Bounded wait on an mbarrier of this CTA: after `timeout_ns` the status block says so, the CTA's `fail` word stops
+// every other role, and all of them leave through the ordinary exit (cluster barriers and tensor memory included).
+__device__ __noinline__ bool stage_wait_slow(uint64_t* bar, uint32_t parity, volatile int* fail, vdc_status* status,
+                                             uint64_t timeout_ns, int kind, int role, int at) {
+  const uint64_t t0 = globaltimer_ns();
+  for (uint32_t it = 1;; ++it) {
+    if (mbar_try_wait(bar, parity)) return true;
+    if ((it & 15u) != 0) continue;
+    if (*fail) return false;
+    if (globaltimer_ns() - t0 > timeout_ns) {
+      if (atomicCAS(&status->abort, 0, 1) == 0) {
+        status->code = VDC_ERR_TIMEOUT;
+        status->sm = (int)blockIdx.x;
+        status->role = role;
+        status->pc = at;
+        status->opcode = kind;
+        status->bar = -1;
+        status->aux = (int)it;
+        __threadfence();
+      }
+      *fail = 1;
+      return false;
+    }
+  }
+}
+
+struct Waiter {
+  volatile int* fail;
+  vdc_status* status;
+  uint64_t timeout_ns;
+  int kind;
+  __device__ __forceinline__ bool operator()(uint64_t* bar, uint32_t parity, int role, int at) const {
+    return mbar_try_wait(bar, parity) || stage_wait_slow(bar, parity, fail, status, timeout_ns, kind, role, at);
+  }
+  // copies that may still be in flight after a wait was given up get a bounded time to land
+  __device__ __forceinline__ void drain() const {
+    if (*fail) {
+      const uint64_t t0 = globaltimer_ns();
+      while (globaltimer_ns() - t0 < 200000ull) __nanosleep(1000);
+    }
+  }
+};
+
+// ------------------------------------------------------------------------- //
+// projection: D[b, n] = sum_k X[b, k] W[n, k] for one block of weight rows, K shared by the CTAs of a cluster
+// ------------------------------------------------------------------------- //
+struct GemmShared {
+  uint64_t full[kMaxRing], empty[kMaxRing];
+  uint64_t ready[kMaxRing];     // rows normalised and weights converted
+  uint64_t stg_empty[2];
+  uint64_t done;
+  uint32_t tmem;
+  volatile int fail;
+  float rstd[128];
+  float ssq[128];
+  unsigned long long key[128];
+};
+
+// Bytes of a chunk of n weight rows x 64 inputs as stored: bf16, e4m3, or e2m1 pairs with one e4m3 scale per 16.
+__host__ __device__ constexpr int chunk_bytes(int wfmt, int n) { return wfmt == 0 ? n * 128 : wfmt == 1 ? n * 64 : n * 36; }
+
+// One ring stage: the rows' chunk, the weights' chunk, the norm weights of the chunk's inputs.
+__host__ __device__ constexpr int stage_size(int wfmt, int bpad) {
+  return bpad * kKc * 2 + (chunk_bytes(wfmt, kBlk) + 127) / 128 * 128 + kKc * 2;
+}
+__host__ __device__ inline int ring_stages(int wfmt, int bpad) {
+  const int staging = wfmt ? 2 * kBlk * kKc * 2 : 0;
+  const int stage = stage_size(wfmt, bpad);
+  const int n = (kGemmSmem - 2048 - 128 - staging) / stage;
+  return n < kMaxRing ? n : kMaxRing;
+}
+
+// Eight fp32 sums (columns col .. col+7 of row b) over the cluster's K-ranges, in rank order.
+__device__ __forceinline__ void sum8(float (&v)[8], uint32_t tile, int splits, int b, int col) {
+  const uint32_t at = tile + (uint32_t)(b * kEpiLd + col) * 4u;
+#pragma unroll
+  for (int j = 0; j < 8; ++j) v[j] = 0.f;
+  for (int r = 0; r < splits; ++r) {
+    const uint32_t p = peer_smem(at, (uint32_t)r);
+    const float4 a = ld_cluster4(p), c = ld_cluster4(p + 16);
+    v[0] += a.x; v[1] += a.y; v[2] += a.z; v[3] += a.w;
+    v[4] += c.x; v[5] += c.y; v[6] += c.z; v[7] += c.w;
+  }
+}
+__device__ __forceinline__ uint4 pack8(const float (&v)[8]) {
+  return make_uint4(pack_bf16x2(v[0], v[1]), pack_bf16x2(v[2], v[3]), pack_bf16x2(v[4], v[5]), pack_bf16x2(v[6], v[7]));
+}
+__device__ __forceinline__ void scale8(float (&v)[8], const float* sc) {
+  if (sc != nullptr) {
+    const float4 a = __ldg(reinterpret_cast<const float4*>(sc)), c = __ldg(reinterpret_cast<const float4*>(sc) + 1);
+    v[0] *= a.x; v[1] *= a.y; v[2] *= a.z; v[3] *= a.w;
+    v[4] *= c.x; v[5] *= c.y; v[6] *= c.z; v[7] *= c.w;
+  }
+}
+
+// One head of the QKV projection, one warp per row: optional RMSNorm over the head, half-rotation, then a query row to
+// the query matrix or a key / value row to the row's cache page.  Every product is rounded as a bf16 tensor expression
+// rounds it.  Lane i holds dims 2i, 2i+1 and their rotation partners 64 further.
+__device__ __forceinline__ void qkv_head(const vdc_stage& s, uint32_t tile, int splits, int b, int block,
+                                         int lane) {
+  constexpr int D = VDC_HEAD_DIM;
+  const int G = s.group, kvh = block / (G + 2), part = block % (G + 2), n0 = block * kBlk;
+  const int i0 = lane * 2;
+  float x[4] = {0.f, 0.f, 0.f, 0.f};
+  const uint32_t at = tile + (uint32_t)(b * kEpiLd + i0) * 4u;
+  for (int r = 0; r < splits; ++r) {
+    const uint32_t p = peer_smem(at, (uint32_t)r);
+    const float2 lo = ld_cluster2(p), hi = ld_cluster2(p + 256);
+    x[0] += lo.x; x[1] += lo.y; x[2] += hi.x; x[3] += hi.y;
+  }
+  const float* scales = reinterpret_cast<const float*>(s.scales);
+  if (scales != nullptr) {
+    const float2 lo = __ldg(reinterpret_cast<const float2*>(scales + n0 + i0));
+    const float2 hi = __ldg(reinterpret_cast<const float2*>(scales + n0 + i0 + 64));
+    x[0] *= lo.x; x[1] *= lo.y; x[2] *= hi.x; x[3] *= hi.y;
+  }
+#pragma unroll
+  for (int j = 0; j < 4; ++j) x[j] = bf16_round(x[j]);
+  const int* st = reinterpret_cast<const int*>(s.state) + (size_t)b * s.state_stride;
+  const int pos = ld_relaxed_gpu(st + VDC_ST_POS);
+  if (part <= G) {   // a query head or the key head
+    if (s.qk_norm) {
+      const float ss = warp_sum(x[0] * x[0] + x[1] * x[1] + x[2] * x[2] + x[3] * x[3]);
+      const float rs = rsqrtf(ss / (float)D + s.qk_eps);
+      const __nv_bfloat16* w = reinterpret_cast<const __nv_bfloat16*>(s.qk_norm) + (part == G ? D : 0);
+      const uint32_t wl = *reinterpret_cast<const uint32_t*>(w + i0), wh = *reinterpret_cast<const uint32_t*>(w + i0 + 64);
+      x[0] = bf16_round(bf_lo(wl) * bf16_round(x[0] * rs));
+      x[1] = bf16_round(bf_hi(wl) * bf16_round(x[1] * rs));
+      x[2] = bf16_round(bf_lo(wh) * bf16_round(x[2] * rs));
+      x[3] = bf16_round(bf_hi(wh) * bf16_round(x[3] * rs));
+    }
+    const float* rope = reinterpret_cast<const float*>(s.rope) + (size_t)pos * D;
+    const float2 cs = __ldg(reinterpret_cast<const float2*>(rope + i0));
+    const float2 sn = __ldg(reinterpret_cast<const float2*>(rope + 64 + i0));
+    const float a0 = x[0], a1 = x[1], b0 = x[2], b1 = x[3];
+    x[0] = bf16_round(a0 * cs.x) - bf16_round(b0 * sn.x);
+    x[1] = bf16_round(a1 * cs.y) - bf16_round(b1 * sn.y);
+    x[2] = bf16_round(b0 * cs.x) + bf16_round(a0 * sn.x);
+    x[3] = bf16_round(b1 * cs.y) + bf16_round(a1 * sn.y);
+  }
+  const uint32_t lo = pack_bf16x2(x[0], x[1]), hi = pack_bf16x2(x[2], x[3]);
+  if (part < G) {
+    uint32_t* dst = reinterpret_cast<uint32_t*>(s.out) + ((size_t)b * s.n_kv * G + (size_t)kvh * G + part) * (D / 2) + lane;
+    dst[0] = lo;
+    dst[32] = hi;
+    return;
+  }
+  // the row's 16-byte pieces lie at (piece XOR (row mod 8)), the page-row order the attention reads
+  const int sw = pos & 7;
+  uint8_t* row = reinterpret_cast<uint8_t*>(part == G ? s.kpool : s.vpool) + (size_t)kvh * (VDC_KV_PAGE * D * 2) +
+                 (size_t)ld_relaxed_gpu(st + VDC_ST_NEWROW) * (D * 2);
+  *reinterpret_cast<uint32_t*>(row + (((i0 >> 3) ^ sw) << 4) + (i0 & 7) * 2) = lo;
+  *reinterpret_cast<uint32_t*>(row + (((8 + (i0 >> 3)) ^ sw) << 4) + (i0 & 7) * 2) = hi;
+}
+
+template <int kFmt>
+__global__ void __launch_bounds__(kGemmThreads, 2) stage_gemm(const __grid_constant__ vdc_stage s, int n_ring,
+                                                              vdc_status* status, uint64_t timeout_ns) {
+  extern __shared__ uint8_t dyn[];
+  __shared__ GemmShared sh;
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int splits = s.splits;
+  const int rank = splits > 1 ? (int)cluster_rank() : 0;
+  const int block = (int)blockIdx.x / splits;
+  const int n0 = block * kBlk, N = min(kBlk, s.M - n0);
+  const int chunks = s.K / kKc, c0 = chunks * rank / splits, n_ch = chunks * (rank + 1) / splits - c0;
+  const int xbytes = s.Bpad * kKc * 2, wbytes = chunk_bytes(kFmt, N);
+  const int stage_bytes = stage_size(kFmt, s.Bpad), nw_off = stage_bytes - kKc * 2;
+  const bool norm = s.stats_in != 0, prepare = kFmt != 0 || norm;
+  uint8_t* ring = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(dyn) + 127) & ~(uintptr_t)127);
+  uint8_t* staging = ring + n_ring * stage_bytes;
+  const Waiter wait{&sh.fail, status, timeout_ns, s.kind};
+
+  if (warp == 1) tmem_alloc(&sh.tmem, kBlk);
+  if (tid == 0) {
+    for (int i = 0; i < n_ring; ++i) {
+      mbar_init(&sh.full[i], 1);
+      mbar_init(&sh.empty[i], 1);
+      mbar_init(&sh.ready[i], kEpiThreads);
+    }
+    for (int i = 0; i < 2; ++i) mbar_init(&sh.stg_empty[i], 1);
+    mbar_init(&sh.done, 1);
+    sh.fail = 0;
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+  }
+  if (tid >= 64 && tid < 192) {
+    sh.ssq[tid - 64] = 0.f;
+    sh.key[tid - 64] = 0ull;
+  }
+  tc_fence_before();
+  __syncthreads();
+  tc_fence_after();
+  const uint32_t tmem = sh.tmem;
+
+  if (warp == 0) {
+    if (lane == 0) {
+      const uint8_t* w = reinterpret_cast<const uint8_t*>(s.w) + (size_t)n0 * s.K * (kFmt == 0 ? 32 : kFmt == 1 ? 16 : 9) / 16 +
+                         (size_t)c0 * wbytes;
+      const uint8_t* x = reinterpret_cast<const uint8_t*>(s.x) + (size_t)c0 * xbytes;
+      const uint8_t* nw = reinterpret_cast<const uint8_t*>(s.norm_w) + (size_t)c0 * kKc * 2;
+      const uint32_t tx = (uint32_t)(xbytes + wbytes + (norm ? kKc * 2 : 0));
+      auto load_weights = [&](int i, int st) {
+        mbar_arrive_expect_tx(&sh.full[st], tx);
+        bulk_load_1d(ring + st * stage_bytes + xbytes, w + (size_t)i * wbytes, (uint32_t)wbytes, &sh.full[st]);
+        if (norm) bulk_load_1d(ring + st * stage_bytes + nw_off, nw + (size_t)i * kKc * 2, kKc * 2, &sh.full[st]);
+      };
+      // the weights depend on nothing: they are on their way before the previous stage's results are waited for
+      const int first = min(n_ch, n_ring);
+      for (int i = 0; i < first; ++i) load_weights(i, i);
+      grid_dep_wait();
+      fence_proxy_async();
+      for (int i = 0; i < first; ++i) bulk_load_1d(ring + i * stage_bytes, x + (size_t)i * xbytes, (uint32_t)xbytes, &sh.full[i]);
+      for (int i = first; i < n_ch; ++i) {
+        const int st = i % n_ring;
+        if (!wait(&sh.empty[st], (uint32_t)(i / n_ring - 1) & 1u, 0, i)) break;
+        load_weights(i, st);
+        bulk_load_1d(ring + st * stage_bytes, x + (size_t)i * xbytes, (uint32_t)xbytes, &sh.full[st]);
+      }
+      grid_dep_launch();     // not earlier: waiting CTAs of the stages behind would hold the shared memory of this one's
+    }
+  } else if (warp == 1) {
+    if (lane == 0) {
+      const uint32_t idesc = umma_idesc_bf16_m128(N);
+      const uint32_t lbo_a = (uint32_t)s.Bpad * 16u, lbo_b = (uint32_t)N * 16u;
+      bool ok = true;
+      for (int i = 0; i < n_ch && ok; ++i) {
+        const int st = i % n_ring;
+        ok = wait(&sh.full[st], (uint32_t)(i / n_ring) & 1u, 1, i);
+        if (prepare && ok) ok = wait(&sh.ready[st], (uint32_t)(i / n_ring) & 1u, 1, i);
+        if (!ok) break;
+        tc_fence_after();
+        uint8_t* at = ring + st * stage_bytes;
+        uint64_t adesc = umma_desc(smem_u32(at), lbo_a, 128u);
+        uint64_t bdesc = umma_desc(smem_u32(kFmt != 0 ? staging + (i & 1) * (kBlk * kKc * 2) : at + xbytes), lbo_b, 128u);
+#pragma unroll
+        for (int k = 0; k < kKc / 16; ++k) {
+          umma_bf16(tmem, adesc, bdesc, idesc, (uint32_t)((i | k) != 0));
+          adesc += (2u * lbo_a) >> 4;
+          bdesc += (2u * lbo_b) >> 4;
+        }
+        umma_commit(&sh.empty[st]);
+        if (kFmt != 0) umma_commit(&sh.stg_empty[i & 1]);
+      }
+      umma_commit(&sh.done);
+      wait(&sh.done, 0u, 1, n_ch);
+    }
+  } else {
+    const int t = tid - 64;
+    if (prepare) {
+      // The eight warps normalise the rows in place, rounded like a bf16 tensor expression, bf16(w * bf16(x * rstd)), and
+      // turn quantised weights into bf16 pieces of the tensor cores' operand layout, 32 weights of one row per thread
+      // (exact for e4m3 and for e2m1 code times block scale).  Every thread takes part in every chunk: a warp that took
+      // only every other chunk could meet a ring stage two rounds ahead and read its barrier's parity the wrong way.
+      const int row = t & 127, g_lo = (t >> 7) * (kKc / 32);
+      if (norm) {
+        grid_dep_wait();
+        if (t < s.Bpad)
+          sh.rstd[t] = rsqrtf(__ldcg(reinterpret_cast<const float*>(s.stats_in) + t) / (float)s.K + s.eps);
+        asm volatile("bar.sync 1, %0;" ::"n"(kEpiThreads) : "memory");
+      }
+      const float rstd = norm ? sh.rstd[t & (s.Bpad - 1)] : 1.f;    // a thread's pieces belong to one row
+      for (int i = 0; i < n_ch; ++i) {
+        const int st = i % n_ring;
+        if (!wait(&sh.full[st], (uint32_t)(i / n_ring) & 1u, 2, i)) break;
+        if (norm) {
+          uint8_t* xs = ring + st * stage_bytes;
+          const uint8_t* nw = xs + nw_off;
+          for (int p = t; p < s.Bpad * (kKc / 8); p += kEpiThreads) {
+            const uint4 v = lds128(xs + p * 16), w = lds128(nw + p / s.Bpad * 16);
+            const uint32_t xv[4] = {v.x, v.y, v.z, v.w}, wv[4] = {w.x, w.y, w.z, w.w};
+            uint32_t o[4];
+#pragma unroll
+            for (int j = 0; j < 4; ++j)
+              o[j] = pack_bf16x2(bf16_round(bf_lo(xv[j]) * rstd) * bf_lo(wv[j]), bf16_round(bf_hi(xv[j]) * rstd) * bf_hi(wv[j]));
+            *reinterpret_cast<uint4*>(xs + p * 16) = make_uint4(o[0], o[1], o[2], o[3]);
+          }
+        }
+        if (kFmt != 0 && i >= 2 && !wait(&sh.stg_empty[i & 1], (uint32_t)((i >> 1) - 1) & 1u, 2, i)) break;
+        uint8_t* dst = staging + (i & 1) * (kBlk * kKc * 2);
+        const uint8_t* src = ring + st * stage_bytes + xbytes;
+        if (kFmt != 0 && row < N) {
+#pragma unroll
+          for (int gj = 0; gj < kKc / 32; ++gj) {
+            const int g16 = g_lo + gj;
+            uint32_t o[8];
+            if (kFmt == 1) {
+              const uint4 v = lds128(src + (g16 * N + row) * 16);
+              const uint32_t wv[4] = {v.x, v.y, v.z, v.w};
+#pragma unroll
+              for (int j = 0; j < 4; ++j) {
+                const float2 lo = e4m3x2_to_float2(wv[j] & 0xFFFFu), hi = e4m3x2_to_float2(wv[j] >> 16);
+                o[2 * j] = pack_bf16x2(lo.x, lo.y);
+                o[2 * j + 1] = pack_bf16x2(hi.x, hi.y);
+              }
+            } else {
+              const uint8_t* g = src + g16 * 9 * N;
+              const uint2 cv = *reinterpret_cast<const uint2*>(g + row * 8);
+              const __half_raw hr = __nv_cvt_fp8_to_halfraw((__nv_fp8_storage_t)g[8 * N + row], __NV_E4M3);
+              const __half2 sc = __half2half2(*reinterpret_cast<const __half*>(&hr));
+              const uint32_t cw[2] = {cv.x, cv.y};
+#pragma unroll
+              for (int j = 0; j < 8; ++j) {
+                const float2 f = __half22float2(__hmul2(e2m1x2_to_half2((cw[j >> 2] >> (8 * (j & 3))) & 0xFFu), sc));
+                o[j] = pack_bf16x2(f.x, f.y);
+              }
+            }
+            *reinterpret_cast<uint4*>(dst + ((2 * g16) * N + row) * 16) = make_uint4(o[0], o[1], o[2], o[3]);
+            *reinterpret_cast<uint4*>(dst + ((2 * g16 + 1) * N + row) * 16) = make_uint4(o[4], o[5], o[6], o[7]);
+          }
+        }
+        fence_proxy_async_smem();
+        mbar_arrive(&sh.ready[st]);
+      }
+    }
+    grid_dep_wait();
+  }
+  __syncthreads();   // lane 0 of warp 1 saw the last commit: the accumulator is complete, the ring is free
+  tc_fence_after();
+  const bool failed = sh.fail != 0;
+  float* tile_p = reinterpret_cast<float*>(ring);
+  const uint32_t tile = smem_u32(tile_p);
+  if (warp >= 2 && !failed) {
+    const int quarter = warp & 3, half = (warp - 2) >> 2;
+    const int b = quarter * 32 + lane, ng = N >> 4;
+    if (quarter * 32 < s.Bpad) {
+      for (int gi = half ? (ng + 1) / 2 : 0; gi < (half ? ng : (ng + 1) / 2); ++gi) {
+        uint32_t r[16];
+        tmem_ld16(tmem + ((uint32_t)(quarter * 32) << 16) + (uint32_t)(gi * 16), r);
+        if (b < s.Bpad) {
+          uint4* d = reinterpret_cast<uint4*>(tile_p + b * kEpiLd + gi * 16);
+#pragma unroll
+          for (int j = 0; j < 4; ++j) d[j] = make_uint4(r[4 * j], r[4 * j + 1], r[4 * j + 2], r[4 * j + 3]);
+        }
+      }
+    }
+    tc_fence_before();
+  }
+  if (splits > 1) {
+    cluster_arrive();
+    cluster_wait();
+  } else {
+    __syncthreads();
+  }
+
+  // ---- epilogue: this CTA finishes Bpad / splits of the rows, all columns of the block
+  if (warp >= 2 && !failed) {
+    const int t = tid - 64;
+    const int nb = s.Bpad / splits, b_lo = rank * nb;
+    const float* scales = reinterpret_cast<const float*>(s.scales);
+    if (s.mode == VDC_STAGE_QKV) {
+      for (int bl = warp - 2; bl < nb; bl += kEpiThreads / 32)
+        if (b_lo + bl < s.B) qkv_head(s, tile, splits, b_lo + bl, block, lane);
+    } else {
+      const int bl = t & (nb - 1), b = b_lo + bl;      // nb is a power of two, at most 128
+      const int f0 = t / nb, fstep = kEpiThreads / nb;
+      if (b < s.B) {
+        if (s.mode == VDC_STAGE_RESID) {
+          float ssq = 0.f;
+          for (int f = f0; f < N / 8; f += fstep) {
+            float v[8];
+            sum8(v, tile, splits, b, f * 8);
+            scale8(v, scales ? scales + n0 + f * 8 : nullptr);
+            uint4* hp = reinterpret_cast<uint4*>(reinterpret_cast<uint8_t*>(s.hid) + kc_piece(s.Bpad, b, n0 + f * 8));
+            const uint4 h = *hp;
+            const uint32_t hv[4] = {h.x, h.y, h.z, h.w};
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+              v[2 * j] = bf16_round(bf_lo(hv[j]) + bf16_round(v[2 * j]));
+              v[2 * j + 1] = bf16_round(bf_hi(hv[j]) + bf16_round(v[2 * j + 1]));
+              ssq = fmaf(v[2 * j], v[2 * j], fmaf(v[2 * j + 1], v[2 * j + 1], ssq));
+            }
+            *hp = pack8(v);
+          }
+          atomicAdd(&sh.ssq[bl], ssq);
+        } else if (s.mode == VDC_STAGE_SILU) {
+          for (int f = f0; f < N / 16; f += fstep) {
+            float o[8];
+#pragma unroll
+            for (int h = 0; h < 2; ++h) {
+              float v[8];
+              sum8(v, tile, splits, b, f * 16 + h * 8);
+              scale8(v, scales ? scales + n0 + f * 16 + h * 8 : nullptr);
+#pragma unroll
+              for (int j = 0; j < 4; ++j) {
+                const float g = bf16_round(v[2 * j]), u = bf16_round(v[2 * j + 1]);
+                o[4 * h + j] = bf16_round(g / (1.f + __expf(-g))) * u;
+              }
+            }
+            *reinterpret_cast<uint4*>(reinterpret_cast<uint8_t*>(s.out) + kc_piece(s.Bpad, b, (n0 >> 1) + f * 8)) = pack8(o);
+          }
+        } else {   // VDC_STAGE_ARGMAX over bf16 logits, the lowest row wins ties
+          float best = -INFINITY;
+          int row = 0x7fffffff;
+          for (int f = f0; f < N / 8; f += fstep) {
+            float v[8];
+            sum8(v, tile, splits, b, f * 8);
+#pragma unroll
+            for (int j = 0; j < 8; ++j) {
+              const float l = bf16_round(v[j]);
+              if (l > best) {
+                best = l;
+                row = n0 + f * 8 + j;
+              }
+            }
+          }
+          if (row != 0x7fffffff) {
+            uint32_t u = __float_as_uint(best);
+            u = (u & 0x80000000u) ? ~u : (u | 0x80000000u);   // order-preserving map of the float
+            atomicMax(&sh.key[bl], ((unsigned long long)u << 32) | (unsigned long long)(0xFFFFFFFFu - (uint32_t)row));
+          }
+        }
+      }
+      __syncwarp();
+      asm volatile("bar.sync 1, %0;" ::"n"(kEpiThreads) : "memory");
+      if (t < nb && b_lo + t < s.B) {
+        if (s.mode == VDC_STAGE_RESID) atomicAdd(reinterpret_cast<float*>(s.stats_out) + b_lo + t, sh.ssq[t]);
+        if (s.mode == VDC_STAGE_ARGMAX) atomicMax(reinterpret_cast<unsigned long long*>(s.keys) + b_lo + t, sh.key[t]);
+      }
+    }
+  }
+  wait.drain();
+  __syncwarp();
+  if (splits > 1) {
+    cluster_arrive();   // nobody leaves while another CTA of the cluster reads its tile
+    cluster_wait();
+  }
+  __syncthreads();
+  if (warp == 1) tmem_dealloc(tmem, kBlk);
+}
+
+// ------------------------------------------------------------------------- //
+// attention of a batched step: one row (sequence) and KV head per cluster, its pages shared by the cluster's CTAs
+// ------------------------------------------------------------------------- //
+// Bound by HBM: 6.1 TB/s at 64 rows and 6.5 TB/s at 128 rows of 2048 positions (the megakernel's units, each walking its
+// pages alone with 192 MMAs per page, were bound by the warps at 1.3 us per page and SM).  A page is two bulk copies;
+// three of them in flight in each of two CTAs keep 192 KB per SM on their way.
+constexpr int kPageBytes = VDC_KV_PAGE * VDC_HEAD_DIM * 2;
+constexpr int kAttnRing = 3;
+constexpr int kAttnThreads = 160;      // four consumer warps (16 positions of a page each), one producer warp
+constexpr int kAttnSmem = kAttnRing * 2 * kPageBytes + 128;
+constexpr int kRecLd = VDC_HEAD_DIM + 4;
+
+struct AttnShared {
+  uint64_t full[kAttnRing], empty[kAttnRing];
+  volatile int fail;
+  alignas(16) float m[64], l[64];            // a row's maximum and sum over this CTA's pages
+  alignas(16) uint4 zero[16];
+  float wm[4][8], wl[4][8];
+};
+
+__device__ __forceinline__ void mma_16816(float (&d)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0,
+                                          uint32_t b1) {
+  asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
+               : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3]) : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
+}
+__device__ __forceinline__ uint32_t transpose8x8(uint32_t v) {
+  uint32_t d;
+  asm volatile("movmatrix.sync.aligned.m8n8.trans.b16 %0, %1;" : "=r"(d) : "r"(v));
+  return d;
+}
+
+// Producer warp: streams the K and V pages first .. first + count - 1 of one KV head through the ring.
+__device__ __forceinline__ void stream_pages(AttnShared& sh, const Waiter& wait, uint8_t* ring, const int* table, int first,
+                                             int count, const uint8_t* k0, const uint8_t* v0, size_t page_stride, int lane) {
+  int ids = 0;
+  for (int i = 0; i < count; ++i) {
+    if ((i & 31) == 0) ids = i + lane < count ? ld_relaxed_gpu(table + first + i + lane) : 0;
+    const size_t off = (size_t)__shfl_sync(0xffffffffu, ids, i & 31) * page_stride;
+    int ok = 1;
+    if (lane == 0) {
+      const int st = i % kAttnRing;
+      if (i >= kAttnRing) ok = wait(&sh.empty[st], (uint32_t)(i / kAttnRing - 1) & 1u, 0, i);
+      if (ok) {
+        uint8_t* at = ring + st * 2 * kPageBytes;
+        mbar_arrive_expect_tx(&sh.full[st], 2 * kPageBytes);
+        bulk_load_1d(at, k0 + off, kPageBytes, &sh.full[st]);
+        bulk_load_1d(at + kPageBytes, v0 + off, kPageBytes, &sh.full[st]);
+      }
+    }
+    if (!__shfl_sync(0xffffffffu, ok, 0)) break;
+  }
+  grid_dep_launch();
+}
+
+__device__ __forceinline__ void attn_setup(AttnShared& sh, int tid) {
+  if (tid == 0) {
+    for (int i = 0; i < kAttnRing; ++i) {
+      mbar_init(&sh.full[i], 1);
+      mbar_init(&sh.empty[i], 4);
+    }
+    sh.fail = 0;
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+  }
+  if (tid >= 64 && tid < 80) sh.zero[tid - 64] = make_uint4(0u, 0u, 0u, 0u);
+  __syncthreads();
+}
+
+// The cluster's last step: output rows are sums of the CTAs' unnormalised rows, weighted by their maxima.
+// rows: query rows of the tile; row r of this tile is out row `row_b(r)`, head column `row_h(r)`.
+template <class Dst>
+__device__ __forceinline__ void attn_merge(AttnShared& sh, uint32_t tile, int splits, int rank, int rows, int t, int nt, Dst dst) {
+  const uint32_t m_at = smem_u32(sh.m), l_at = smem_u32(sh.l);
+  const int per = VDC_HEAD_DIM / 8;
+  for (int it = rank * nt + t; it < rows * per; it += splits * nt) {
+    const int r = it / per, d = (it % per) * 8;
+    float m = -INFINITY;
+    for (int k = 0; k < splits; ++k) m = fmaxf(m, ld_cluster1(peer_smem(m_at + r * 4, k)));
+    float den = 0.f, v[8];
+#pragma unroll
+    for (int j = 0; j < 8; ++j) v[j] = 0.f;
+    for (int k = 0; k < splits; ++k) {
+      const float mk = ld_cluster1(peer_smem(m_at + r * 4, k));
+      const float w = mk == -INFINITY ? 0.f : exp2f(mk - m);
+      den = fmaf(w, ld_cluster1(peer_smem(l_at + r * 4, k)), den);
+      const uint32_t p = peer_smem(tile + (uint32_t)(r * kRecLd + d) * 4u, k);
+      const float4 a = ld_cluster4(p), c = ld_cluster4(p + 16);
+      v[0] = fmaf(w, a.x, v[0]); v[1] = fmaf(w, a.y, v[1]); v[2] = fmaf(w, a.z, v[2]); v[3] = fmaf(w, a.w, v[3]);
+      v[4] = fmaf(w, c.x, v[4]); v[5] = fmaf(w, c.y, v[5]); v[6] = fmaf(w, c.z, v[6]); v[7] = fmaf(w, c.w, v[7]);
+    }
+    const float inv = den > 0.f ? 1.f / den : 0.f;
+#pragma unroll
+    for (int j = 0; j < 8; ++j) v[j] *= inv;
+    uint4* at = dst(r, d);
+    if (at != nullptr) *at = pack8(v);
+  }
+}
+
+__global__ void __launch_bounds__(kAttnThreads, 2) stage_attn(const __grid_constant__ vdc_stage s, vdc_status* status,
+                                                              uint64_t timeout_ns) {
+  extern __shared__ uint8_t dyn[];
+  __shared__ AttnShared sh;
+  constexpr int D = VDC_HEAD_DIM;
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int splits = s.splits, rank = splits > 1 ? (int)cluster_rank() : 0;
+  const int h = blockIdx.y, b = blockIdx.z, G = s.group;
+  uint8_t* ring = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(dyn) + 127) & ~(uintptr_t)127);
+  const Waiter wait{&sh.fail, status, timeout_ns, s.kind};
+  attn_setup(sh, tid);
+  grid_dep_wait();
+  const int* st = reinterpret_cast<const int*>(s.state) + (size_t)b * s.state_stride;
+  const int pos = ld_relaxed_gpu(st + VDC_ST_POS);
+  const int n_pages = min(pos / VDC_KV_PAGE + 1, s.n_pages);
+  const int per = (n_pages + splits - 1) / splits, first = rank * per;
+  const int count = max(0, min(per, n_pages - first));
+
+  const int gid = lane >> 2, t4 = lane & 3;
+  float m[2] = {-INFINITY, -INFINITY}, l[2] = {0.f, 0.f}, o[8][4];
+#pragma unroll
+  for (int i = 0; i < 8; ++i)
+#pragma unroll
+    for (int j = 0; j < 4; ++j) o[i][j] = 0.f;
+
+  if (warp == 4) {
+    fence_proxy_async();   // the new cache rows were written with ordinary stores by the projection in front
+    const size_t head_off = (size_t)h * kPageBytes;
+    stream_pages(sh, wait, ring, st + VDC_ST_PAGETABLE, first, count, reinterpret_cast<const uint8_t*>(s.kpool) + head_off,
+                 reinterpret_cast<const uint8_t*>(s.vpool) + head_off, (size_t)s.n_kv * kPageBytes, lane);
+  } else {
+    // S^T = K Q^T and O^T = V^T P^T: the warp's 16 positions (then 16 dims at a time) on the tile's rows, the query
+    // heads of the group on its 8 columns.  8 + 8 MMAs per warp and page, none of them on padding for a group of 8.
+    uint32_t q[8][2];
+    const uint32_t* qp = reinterpret_cast<const uint32_t*>(s.q) + ((size_t)b * s.n_kv * G + (size_t)h * G + gid) * (D / 2) + t4;
+#pragma unroll
+    for (int k = 0; k < 8; ++k) {
+      q[k][0] = gid < G ? ldcg32(qp + 8 * k) : 0u;
+      q[k][1] = gid < G ? ldcg32(qp + 8 * k + 4) : 0u;
+    }
+    const float scale_log2 = 1.4426950408889634f * rsqrtf((float)D);
+    const uint32_t zero = smem_u32(sh.zero), ring_s = smem_u32(ring);
+    const int lr = lane & 7, mi = lane >> 3;
+    const int pk = warp * 16 + lr + 8 * (mi & 1), hk = mi >> 1;      // ldmatrix rows of K: position, upper k half
+    const int pv = warp * 16 + lr + 8 * (mi >> 1), hv = mi & 1;      // of V (transposed): position, upper dim half
+    for (int i = 0; i < count; ++i) {
+      const int stg = i % kAttnRing;
+      if (!wait(&sh.full[stg], (uint32_t)(i / kAttnRing) & 1u, 1, i)) break;
+      const uint32_t kb = ring_s + (uint32_t)(stg * 2 * kPageBytes), vb = kb + kPageBytes;
+      const int valid = pos - (first + i) * VDC_KV_PAGE;             // last position that exists, within the page
+      float c[4] = {0.f, 0.f, 0.f, 0.f}, c2[4] = {0.f, 0.f, 0.f, 0.f};
+#pragma unroll
+      for (int k = 0; k < 8; k += 2) {
+        uint32_t a[4], a2[4];
+        ldsm_x4(a, kb + (uint32_t)(pk * 256 + (((2 * k + hk) ^ lr) << 4)));
+        ldsm_x4(a2, kb + (uint32_t)(pk * 256 + (((2 * k + 2 + hk) ^ lr) << 4)));
+        mma_16816(c, a[0], a[1], a[2], a[3], q[k][0], q[k][1]);
+        mma_16816(c2, a2[0], a2[1], a2[2], a2[3], q[k + 1][0], q[k + 1][1]);
+      }
+      const int p0 = warp * 16 + gid;
+      float e[4];
+#pragma unroll
+      for (int j = 0; j < 4; ++j) e[j] = p0 + 8 * (j >> 1) <= valid ? (c[j] + c2[j]) * scale_log2 : -INFINITY;
+      float mx[2] = {fmaxf(e[0], e[2]), fmaxf(e[1], e[3])};
+#pragma unroll
+      for (int x = 4; x < 32; x <<= 1) {
+        mx[0] = fmaxf(mx[0], __shfl_xor_sync(0xffffffffu, mx[0], x));
+        mx[1] = fmaxf(mx[1], __shfl_xor_sync(0xffffffffu, mx[1], x));
+      }
+      float al[2];
+#pragma unroll
+      for (int j = 0; j < 2; ++j) {
+        const float mn = fmaxf(m[j], mx[j]);
+        const bool none = mn == -INFINITY;
+        al[j] = none ? 1.f : exp2f(m[j] - mn);
+        e[j] = none ? 0.f : exp2f(e[j] - mn);
+        e[j + 2] = none ? 0.f : exp2f(e[j + 2] - mn);
+        m[j] = mn;
+        l[j] = l[j] * al[j] + e[j] + e[j + 2];       // this lane's positions only: summed over the lanes at the end
+      }
+      // probabilities enter P V rounded to bf16, as a bf16 attention module hands them over
+      const uint32_t b0 = transpose8x8(pack_bf16x2(e[0], e[1])), b1 = transpose8x8(pack_bf16x2(e[2], e[3]));
+      const uint32_t vrow = pv <= valid ? vb + (uint32_t)(pv * 256) : zero;
+#pragma unroll
+      for (int d = 0; d < 8; ++d) {
+        uint32_t a[4];
+        ldsm_x4_trans(a, vrow + (uint32_t)(((2 * d + hv) ^ lr) << 4));
+#pragma unroll
+        for (int j = 0; j < 4; ++j) o[d][j] *= al[j & 1];
+        mma_16816(o[d], a[0], a[1], a[2], a[3], b0, b1);
+      }
+      __syncwarp();
+      if (lane == 0) mbar_arrive(&sh.empty[stg]);
+    }
+#pragma unroll
+    for (int x = 4; x < 32; x <<= 1) {
+      l[0] += __shfl_xor_sync(0xffffffffu, l[0], x);
+      l[1] += __shfl_xor_sync(0xffffffffu, l[1], x);
+    }
+    if (gid == 0) {
+      sh.wm[warp][2 * t4] = m[0];
+      sh.wm[warp][2 * t4 + 1] = m[1];
+      sh.wl[warp][2 * t4] = l[0];
+      sh.wl[warp][2 * t4 + 1] = l[1];
+    }
+  }
+  __syncthreads();                       // pages are consumed: their shared memory takes the warps' partial outputs
+  const bool failed = sh.fail != 0;
+  float* part = reinterpret_cast<float*>(ring);                 // [warp][8 heads][kRecLd]
+  float* rec = part + 4 * 8 * kRecLd;                           // [head][kRecLd]: this CTA's sum
+  if (warp < 4 && !failed) {
+#pragma unroll
+    for (int d = 0; d < 8; ++d)
+#pragma unroll
+      for (int j = 0; j < 4; ++j)
+        part[(warp * 8 + 2 * t4 + (j & 1)) * kRecLd + d * 16 + gid + 8 * (j >> 1)] = o[d][j];
+  }
+  __syncthreads();
+  if (warp < 4 && !failed) {
+    for (int g = 0; g < G; ++g) {
+      float mm = -INFINITY;
+#pragma unroll
+      for (int w = 0; w < 4; ++w) mm = fmaxf(mm, sh.wm[w][g]);
+      float sum = 0.f, den = 0.f;
+#pragma unroll
+      for (int w = 0; w < 4; ++w) {
+        const float wt = sh.wm[w][g] == -INFINITY ? 0.f : exp2f(sh.wm[w][g] - mm);
+        sum = fmaf(wt, part[(w * 8 + g) * kRecLd + tid], sum);
+        den = fmaf(wt, sh.wl[w][g], den);
+      }
+      rec[g * kRecLd + tid] = sum;
+      if (tid == 0) {
+        sh.m[g] = mm;
+        sh.l[g] = den;
+      }
+    }
+  }
+  if (splits > 1) {
+    cluster_arrive();
+    cluster_wait();
+  } else {
+    __syncthreads();
+  }
+  if (warp < 4 && !failed)
+    attn_merge(sh, smem_u32(rec), splits, rank, G, tid, 128, [&](int r, int d) {
+      return reinterpret_cast<uint4*>(reinterpret_cast<uint8_t*>(s.out) + kc_piece(s.Bpad, b, (h * G + r) * D + d));
+    });
+  wait.drain();
+  if (splits > 1) {
+    cluster_arrive();
+    cluster_wait();
+  }
+}
+
+// ------------------------------------------------------------------------- //
+// attention of a prefill chunk: 64 query rows (64 / G consecutive positions x G heads) of one KV head per cluster
+// ------------------------------------------------------------------------- //
+constexpr int kRows = 64;
+
+__global__ void __launch_bounds__(kAttnThreads, 2) stage_attn_prefill(const __grid_constant__ vdc_stage s, vdc_status* status,
+                                                                      uint64_t timeout_ns) {
+  extern __shared__ uint8_t dyn[];
+  __shared__ AttnShared sh;
+  constexpr int D = VDC_HEAD_DIM;
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int splits = s.splits, rank = splits > 1 ? (int)cluster_rank() : 0;
+  const int h = blockIdx.y, G = s.group, per_tile = kRows / G, b0 = blockIdx.z * per_tile;
+  uint8_t* ring = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(dyn) + 127) & ~(uintptr_t)127);
+  const Waiter wait{&sh.fail, status, timeout_ns, s.kind};
+  attn_setup(sh, tid);
+  grid_dep_wait();
+  const int* st = reinterpret_cast<const int*>(s.state);
+  auto row_b = [&](int r) { return min(b0 + r / G, s.B - 1); };
+  auto pos_of = [&](int r) { return ld_relaxed_gpu(st + (size_t)row_b(r) * s.state_stride + VDC_ST_POS); };
+  const int pos_hi = pos_of(kRows - 1), pos_lo = pos_of(0);          // the rows' positions never decrease
+  const int n_pages = min(pos_hi / VDC_KV_PAGE + 1, s.n_pages);
+  const int per = (n_pages + splits - 1) / splits, first = rank * per;
+  const int count = max(0, min(per, n_pages - first));
+
+  const int gid = lane >> 2, t4 = lane & 3;
+  const int r0 = warp * 16 + gid;
+  float m[2] = {-INFINITY, -INFINITY}, l[2] = {0.f, 0.f}, o[16][4];
+#pragma unroll
+  for (int i = 0; i < 16; ++i)
+#pragma unroll
+    for (int j = 0; j < 4; ++j) o[i][j] = 0.f;
+
+  if (warp == 4) {
+    fence_proxy_async();
+    const size_t head_off = (size_t)h * kPageBytes;
+    stream_pages(sh, wait, ring, st + VDC_ST_PAGETABLE, first, count, reinterpret_cast<const uint8_t*>(s.kpool) + head_off,
+                 reinterpret_cast<const uint8_t*>(s.vpool) + head_off, (size_t)s.n_kv * kPageBytes, lane);
+  } else {
+    uint32_t q[8][4];
+    const int pos[2] = {pos_of(r0), pos_of(r0 + 8)};
+    const uint32_t* qa = reinterpret_cast<const uint32_t*>(s.q) + ((size_t)row_b(r0) * s.n_kv * G + (size_t)h * G + r0 % G) * (D / 2) + t4;
+    const uint32_t* qb = reinterpret_cast<const uint32_t*>(s.q) + ((size_t)row_b(r0 + 8) * s.n_kv * G + (size_t)h * G + (r0 + 8) % G) * (D / 2) + t4;
+#pragma unroll
+    for (int k = 0; k < 8; ++k) {
+      q[k][0] = ldcg32(qa + 8 * k);
+      q[k][1] = ldcg32(qb + 8 * k);
+      q[k][2] = ldcg32(qa + 8 * k + 4);
+      q[k][3] = ldcg32(qb + 8 * k + 4);
+    }
+    const float scale_log2 = 1.4426950408889634f * rsqrtf((float)D);
+    const uint32_t zero = smem_u32(sh.zero), ring_s = smem_u32(ring);
+    const int lr = lane & 7, mi = lane >> 3;
+    for (int i = 0; i < count; ++i) {
+      const int stg = i % kAttnRing;
+      if (!wait(&sh.full[stg], (uint32_t)(i / kAttnRing) & 1u, 1, i)) break;
+      const uint32_t kb = ring_s + (uint32_t)(stg * 2 * kPageBytes), vb = kb + kPageBytes;
+      const int page0 = (first + i) * VDC_KV_PAGE;
+      float c[8][4];
+#pragma unroll
+      for (int n = 0; n < 8; ++n) {
+#pragma unroll
+        for (int j = 0; j < 4; ++j) c[n][j] = 0.f;
+#pragma unroll
+        for (int k = 0; k < 8; k += 2) {      // one load: eight positions, dims 32 (k / 2) .. + 31
+          uint32_t a[4];
+          ldsm_x4(a, kb + (uint32_t)((n * 8 + lr) * 256 + (((2 * k + mi) ^ lr) << 4)));
+          mma_16816(c[n], q[k][0], q[k][1], q[k][2], q[k][3], a[0], a[1]);
+          mma_16816(c[n], q[k + 1][0], q[k + 1][1], q[k + 1][2], q[k + 1][3], a[2], a[3]);
+        }
+      }
+      float mx[2] = {-INFINITY, -INFINITY};
+      const bool edge = page0 + VDC_KV_PAGE - 1 > pos_lo;             // only pages at the diagonal need the mask
+#pragma unroll
+      for (int n = 0; n < 8; ++n)
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+          c[n][j] *= scale_log2;
+          if (edge && page0 + n * 8 + 2 * t4 + (j & 1) > pos[j >> 1]) c[n][j] = -INFINITY;
+          mx[j >> 1] = fmaxf(mx[j >> 1], c[n][j]);
+        }
+      float al[2];
+#pragma unroll
+      for (int j = 0; j < 2; ++j) {
+        mx[j] = fmaxf(mx[j], __shfl_xor_sync(0xffffffffu, mx[j], 1));
+        mx[j] = fmaxf(mx[j], __shfl_xor_sync(0xffffffffu, mx[j], 2));
+        const float mn = fmaxf(m[j], mx[j]);
+        al[j] = mn == -INFINITY ? 1.f : exp2f(m[j] - mn);
+        m[j] = mn;
+        l[j] *= al[j];
+        mx[j] = mn == -INFINITY ? 0.f : mn;                           // a row with no key here: every exponent is -inf
+      }
+      uint32_t p[8][2];
+#pragma unroll
+      for (int n = 0; n < 8; ++n) {
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+          c[n][j] = exp2f(c[n][j] - mx[j >> 1]);
+          l[j >> 1] += c[n][j];
+        }
+        p[n][0] = pack_bf16x2(c[n][0], c[n][1]);
+        p[n][1] = pack_bf16x2(c[n][2], c[n][3]);
+      }
+#pragma unroll
+      for (int d = 0; d < 16; ++d)
+#pragma unroll
+        for (int j = 0; j < 4; ++j) o[d][j] *= al[j >> 1];
+#pragma unroll
+      for (int k = 0; k < 4; ++k) {            // 16 positions at a time
+        const int pv = k * 16 + lr + 8 * (mi & 1);
+        const uint32_t vrow = page0 + pv <= pos_hi ? vb + (uint32_t)(pv * 256) : zero;
+#pragma unroll
+        for (int d = 0; d < 16; d += 2) {      // one load: the positions' dims 8 d .. 8 d + 15
+          uint32_t a[4];
+          ldsm_x4_trans(a, vrow + (uint32_t)(((d + (mi >> 1)) ^ lr) << 4));
+          mma_16816(o[d], p[2 * k][0], p[2 * k][1], p[2 * k + 1][0], p[2 * k + 1][1], a[0], a[1]);
+          mma_16816(o[d + 1], p[2 * k][0], p[2 * k][1], p[2 * k + 1][0], p[2 * k + 1][1], a[2], a[3]);
+        }
+      }
+      __syncwarp();
+      if (lane == 0) mbar_arrive(&sh.empty[stg]);
+    }
+  }
+  __syncthreads();
+  const bool failed = sh.fail != 0;
+  float* rec = reinterpret_cast<float*>(ring);     // [64 rows][kRecLd]
+  if (warp < 4 && !failed) {
+#pragma unroll
+    for (int j = 0; j < 2; ++j) {
+      l[j] += __shfl_xor_sync(0xffffffffu, l[j], 1);
+      l[j] += __shfl_xor_sync(0xffffffffu, l[j], 2);
+      if (t4 == 0) {
+        sh.m[r0 + 8 * j] = m[j];
+        sh.l[r0 + 8 * j] = l[j];
+      }
+#pragma unroll
+      for (int d = 0; d < 16; ++d)
+        *reinterpret_cast<float2*>(rec + (r0 + 8 * j) * kRecLd + d * 8 + 2 * t4) = make_float2(o[d][2 * j], o[d][2 * j + 1]);
+    }
+  }
+  if (splits > 1) {
+    cluster_arrive();
+    cluster_wait();
+  } else {
+    __syncthreads();
+  }
+  if (warp < 4 && !failed)
+    attn_merge(sh, smem_u32(rec), splits, rank, kRows, tid, 128, [&](int r, int d) -> uint4* {
+      const int b = b0 + r / G;
+      if (b >= s.B) return nullptr;
+      return reinterpret_cast<uint4*>(reinterpret_cast<uint8_t*>(s.out) + kc_piece(s.Bpad, b, (h * G + r % G) * D + d));
+    });
+  wait.drain();
+  if (splits > 1) {
+    cluster_arrive();
+    cluster_wait();
+  }
+}
+
+// ------------------------------------------------------------------------- //
+// first and last kernel of a step
+// ------------------------------------------------------------------------- //
+// Embedding row of one sequence: the hidden state and its sum of squares; and zeros for the sums that the step's residual
+// adds accumulate.
+__global__ void __launch_bounds__(256) stage_embed(const __grid_constant__ vdc_stage s) {
+  __shared__ float red[8];
+  const int b = blockIdx.x, tid = threadIdx.x;
+  grid_dep_wait();
+  grid_dep_launch();
+  const int token = ld_relaxed_gpu(reinterpret_cast<const int*>(s.state) + (size_t)b * s.state_stride + VDC_ST_TOKEN);
+  const uint8_t* row = reinterpret_cast<const uint8_t*>(s.w) + (size_t)token * s.K * 2;
+  float ssq = 0.f;
+  for (int p = tid; p < s.K / 8; p += 256) {
+    const uint4 v = __ldg(reinterpret_cast<const uint4*>(row) + p);
+    const uint32_t xv[4] = {v.x, v.y, v.z, v.w};
+#pragma unroll
+    for (int j = 0; j < 4; ++j) ssq = fmaf(bf_lo(xv[j]), bf_lo(xv[j]), fmaf(bf_hi(xv[j]), bf_hi(xv[j]), ssq));
+    *reinterpret_cast<uint4*>(reinterpret_cast<uint8_t*>(s.hid) + kc_piece(s.Bpad, b, p * 8)) = v;
+  }
+  ssq = warp_sum(ssq);
+  if ((tid & 31) == 0) red[tid >> 5] = ssq;
+  __syncthreads();
+  float* stats = reinterpret_cast<float*>(s.stats_out);
+  if (tid == 0) {
+    float t = 0.f;
+    for (int w = 0; w < 8; ++w) t += red[w];
+    stats[b] = t;
+  }
+  for (int i = 1 + tid; i < s.n_stats; i += 256) stats[(size_t)i * 128 + b] = 0.f;
+}
+
+// Next token, token log and state advance of every sequence.
+__global__ void __launch_bounds__(128) stage_advance(const __grid_constant__ vdc_stage s) {
+  grid_dep_wait();
+  grid_dep_launch();
+  const int b = threadIdx.x;
+  if (b >= s.B) return;
+  int* state = reinterpret_cast<int*>(s.state) + (size_t)b * s.state_stride;
+  unsigned long long* keys = reinterpret_cast<unsigned long long*>(s.keys);
+  const int token = (int)(0xFFFFFFFFu - (uint32_t)(__ldcg(keys + b) & 0xFFFFFFFFull));
+  keys[b] = 0ull;
+  const int step = state[VDC_ST_STEP], pos = state[VDC_ST_POS] + 1, page = pos / VDC_KV_PAGE;
+  reinterpret_cast<int*>(s.log)[(size_t)b * s.log_stride + step] = token;
+  state[VDC_ST_TOKEN] = token;
+  state[VDC_ST_STEP] = step + 1;
+  state[VDC_ST_POS] = pos;
+  state[VDC_ST_NPAGES] = page + 1;
+  if (page < state[VDC_ST_MAXPAGES])
+    state[VDC_ST_NEWROW] = state[VDC_ST_PAGETABLE + page] * VDC_KV_PAGE * state[VDC_ST_NKVH] + pos % VDC_KV_PAGE;
+  else
+    state[VDC_ST_ERR] = 1;   // out of KV pages: the host must not launch another step
+}
+
+}  // namespace vdc
+
+// ------------------------------------------------------------------------- //
+// host entry used by the C ABI
+// ------------------------------------------------------------------------- //
+extern "C" cudaError_t vdc_stage_prepare() {
+  const void* gemms[] = {(const void*)vdc::stage_gemm<0>, (const void*)vdc::stage_gemm<1>, (const void*)vdc::stage_gemm<2>};
+  for (const void* f : gemms)
+    if (cudaError_t e = cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, vdc::kGemmSmem)) return e;
+  const void* attns[] = {(const void*)vdc::stage_attn, (const void*)vdc::stage_attn_prefill};
+  for (const void* f : attns)
+    if (cudaError_t e = cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, vdc::kAttnSmem)) return e;
+  return cudaSuccess;
+}
+
+extern "C" cudaError_t vdc_stage_launch(const vdc_stage* s, vdc_status* status, uint64_t timeout_ns, cudaStream_t stream) {
+  if (s->kind == VDC_STAGE_COPY)
+    return cudaMemcpyAsync((void*)s->out, (const void*)s->x, (size_t)s->M * s->K, cudaMemcpyDeviceToDevice, stream);
+  cudaLaunchConfig_t cfg{};
+  cudaLaunchAttribute attr[2];
+  cfg.stream = stream;
+  cfg.attrs = attr;
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  cfg.numAttrs = 1;
+  if (s->splits > 1) {
+    attr[1].id = cudaLaunchAttributeClusterDimension;
+    attr[1].val.clusterDim.x = (unsigned)s->splits;
+    attr[1].val.clusterDim.y = attr[1].val.clusterDim.z = 1;
+    cfg.numAttrs = 2;
+  }
+  switch (s->kind) {
+    case VDC_STAGE_GEMM: {
+      cfg.gridDim = dim3((unsigned)((s->M + vdc::kBlk - 1) / vdc::kBlk * s->splits));
+      cfg.blockDim = dim3(vdc::kGemmThreads);
+      cfg.dynamicSmemBytes = vdc::kGemmSmem;
+      const int ring = vdc::ring_stages(s->wfmt, s->Bpad);
+      auto f = s->wfmt == 0 ? vdc::stage_gemm<0> : s->wfmt == 1 ? vdc::stage_gemm<1> : vdc::stage_gemm<2>;
+      return cudaLaunchKernelEx(&cfg, f, *s, ring, status, timeout_ns);
+    }
+    case VDC_STAGE_ATTN:
+      cfg.gridDim = dim3((unsigned)s->splits, (unsigned)s->n_kv, (unsigned)s->B);
+      cfg.blockDim = dim3(vdc::kAttnThreads);
+      cfg.dynamicSmemBytes = vdc::kAttnSmem;
+      return cudaLaunchKernelEx(&cfg, vdc::stage_attn, *s, status, timeout_ns);
+    case VDC_STAGE_ATTN_PREFILL: {
+      const int per = vdc::kRows / s->group;
+      cfg.gridDim = dim3((unsigned)s->splits, (unsigned)s->n_kv, (unsigned)((s->B + per - 1) / per));
+      cfg.blockDim = dim3(vdc::kAttnThreads);
+      cfg.dynamicSmemBytes = vdc::kAttnSmem;
+      return cudaLaunchKernelEx(&cfg, vdc::stage_attn_prefill, *s, status, timeout_ns);
+    }
+    case VDC_STAGE_EMBED:
+      cfg.gridDim = dim3((unsigned)s->B);
+      cfg.blockDim = dim3(256);
+      return cudaLaunchKernelEx(&cfg, vdc::stage_embed, *s);
+    case VDC_STAGE_ADVANCE:
+      cfg.gridDim = dim3(1);
+      cfg.blockDim = dim3(128);
+      return cudaLaunchKernelEx(&cfg, vdc::stage_advance, *s);
+    default:
+      return cudaErrorInvalidValue;
+  }
+}

@@ -51,6 +51,11 @@ GEMM_MODE_SILU_PAIRS = _defs["GEMM_MODE_SILU_PAIRS"]
 GEMM_MODE_ARGMAX = _defs["GEMM_MODE_ARGMAX"]
 GEMM_MODE_ADD_PACKED = _defs["GEMM_MODE_ADD_PACKED"]
 
+STAGE_GEMM, STAGE_ATTN, STAGE_ATTN_PREFILL, STAGE_EMBED, STAGE_ADVANCE, STAGE_COPY = (
+    _defs["STAGE_" + k] for k in ("GEMM", "ATTN", "ATTN_PREFILL", "EMBED", "ADVANCE", "COPY"))
+STAGE_QKV, STAGE_RESID, STAGE_SILU, STAGE_ARGMAX = (_defs["STAGE_" + k] for k in ("QKV", "RESID", "SILU", "ARGMAX"))
+STAGE_BLOCK = _defs["STAGE_BLOCK"]
+
 ST_POS, ST_NPAGES, ST_TOKEN, ST_STEP = _defs["ST_POS"], _defs["ST_NPAGES"], _defs["ST_TOKEN"], _defs["ST_STEP"]
 ST_NEWROW, ST_NKVH, ST_MAXPAGES, ST_ERR = _defs["ST_NEWROW"], _defs["ST_NKVH"], _defs["ST_MAXPAGES"], _defs["ST_ERR"]
 ST_PAGETABLE = _defs["ST_PAGETABLE"]

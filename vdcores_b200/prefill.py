@@ -1,14 +1,13 @@
-"""Prefill on the device: a chunk of consecutive prompt positions per launch of the megakernel.
+"""Prefill on the device: a chunk of consecutive prompt positions per list of stage kernels.
 
-The batched decode program (batch.BatchDecodeEngine: projections on the tensor cores, one attention unit per
-(row, KV head)) already computes, for every row of its batch, exactly what a prompt position needs; what differs
-in a prefill is that the rows are consecutive positions of ONE sequence.  PrefillEngine therefore gives every row
-the same page table and position pos0 + b, and adds one stage per layer in front of the attention: cache-append
-tasks (isa.ATTN_APPEND_BIT) write the normed, rotated key rows and the value rows of all the chunk's positions to
-the paged pools; the attention units start behind that stage's barrier (their page copies are held back by the
-same barrier), so position p finds the rows of every position < p of its own chunk in HBM, and its row limit
-(pos + 1 rows of the last page) is the causal mask.  The pools and the page table are those of the decode engine
-the prompt is prefilled for: nothing is copied when decode takes over.
+The batched decode step (batch.BatchDecodeEngine) already computes, for every row of its batch, exactly what a prompt
+position needs; what differs in a prefill is that the rows are consecutive positions of ONE sequence.  PrefillEngine
+therefore gives every row the same page table and position pos0 + b.  The QKV projection's epilogue writes the normed,
+rotated key rows and the value rows of all the chunk's positions to the paged pools, so the attention behind it finds
+the rows of every earlier position of its own chunk in HBM; its units are tiles of 64 query rows (64 / G positions times
+the G heads of a KV head) that share one walk over the pages, with the causal mask applied in the pages at the diagonal.
+The pools and the page table are those of the decode engine the prompt is prefilled for: nothing is copied when decode
+takes over.
 
 The reference has no prefill of its own on the device either side of its decode schedules: its correctness runs
 take the prompt's cache from a HuggingFace forward (app/python/llama3/sched.py:574-622 in the reference); this
@@ -50,14 +49,10 @@ class PrefillEngine(BatchDecodeEngine):
         return self
 
     def _build_program(self):
-        """Two programs over the same packed weights: chunks before the prompt's last end after the last layer,
+        """Two lists of stages over the same packed weights: chunks before the prompt's last end after the last layer,
         the last chunk adds the final norm, the vocabulary projection and the argmax (the first generated id)."""
-        self.WITH_VOCAB_PROJECTION = False
         super()._build_program()
-        self._body = (self.insts_per_sm, self.cinsts, self.minsts, self.bars_init)
-        self.WITH_VOCAB_PROJECTION = True
-        super()._build_program()
-        self._last = (self.insts_per_sm, self.cinsts, self.minsts, self.bars_init)
+        self._body = self._plan(vocab=False)
 
     # ------------------------------------------------------------------ chunks
     def _chunk_states(self, tokens: torch.Tensor) -> torch.Tensor:
@@ -82,18 +77,15 @@ class PrefillEngine(BatchDecodeEngine):
         """Runs the prompt, ceil(T / chunk) launches, and returns the first generated (greedy) id.  The only host
         work inside the loop is enqueueing, per chunk, the copy of its prepared state blocks and the launch."""
         T, B = int(tokens.numel()), self.batch
-        assert 1 <= T < self.max_seq and self.program is not None
+        assert 1 <= T < self.max_seq and self.stages is not None
         states = self._chunk_states(tokens.cpu()).to(self.dev)
-        self.attn_cnt.zero_()
         self.keys.zero_()
         self.stats.zero_()
         with torch.cuda.stream(self.stream):
             n = states.shape[0]
             for c in range(n):
                 self.state.copy_(states[c], non_blocking=True)
-                insts_per_sm, cinsts, minsts, bars_init = self._last if c == n - 1 else self._body
-                runtime.launch_async(self.num_sms, insts_per_sm, cinsts, minsts, None, self.bars, bars_init,
-                                     self.profile, self.stream.cuda_stream, self.timeout_ns, full=True)
+                runtime.launch_stages(self.stages if c == n - 1 else self._body, self.stream.cuda_stream, self.timeout_ns)
         runtime.read_status(self.stream.cuda_stream)
         first = int(self.token_log[(T - 1) % B, 0])
         if set_target_state:

@@ -32,6 +32,15 @@ class Status(ctypes.Structure):
         return {n: getattr(self, n) for n, _ in self._fields_}
 
 
+class Stage(ctypes.Structure):
+    """One kernel of a batched step or a prefill chunk (vdc_stage in include/vdcores.h, which documents the fields)."""
+    _fields_ = ([(n, ctypes.c_int32) for n in ("kind", "mode", "wfmt", "B", "Bpad", "M", "K", "splits", "group", "n_kv",
+                                               "n_pages", "state_stride", "log_stride", "n_stats")]
+                + [(n, ctypes.c_float) for n in ("eps", "qk_eps")]
+                + [(n, ctypes.c_uint64) for n in ("w", "scales", "x", "stats_in", "out", "hid", "norm_w", "stats_out", "keys",
+                                                  "state", "log", "rope", "qk_norm", "kpool", "vpool", "q")])
+
+
 _u64, _i32, _vp = ctypes.c_uint64, ctypes.c_int, ctypes.c_void_p
 _lib.vdc_version.restype = _i32
 _lib.vdc_init.restype = _i32
@@ -40,6 +49,7 @@ _lib.vdc_launch.argtypes = [_i32, _i32, _vp, _vp, _vp, _vp, _vp, _u64, _u64, cty
 _lib.vdc_launch_async.argtypes = [_i32, _i32, _vp, _vp, _vp, _vp, _vp, _vp, _u64, _u64]
 _lib.vdc_launch_async_full.argtypes = [_i32, _i32, _vp, _vp, _vp, _vp, _vp, _vp, _u64, _u64]
 _lib.vdc_launch_static.argtypes = [_i32, _i32, _vp, _vp, _vp, _vp, _u64, _u64, ctypes.POINTER(Status)]
+_lib.vdc_launch_stages.argtypes = [ctypes.POINTER(Stage), _i32, _u64, _u64]
 _lib.vdc_read_status.argtypes = [_u64, ctypes.POINTER(Status), _i32]
 _lib.vdc_build_tma_desc.argtypes = [_vp, _vp, _i32, _i32, ctypes.POINTER(_u64), ctypes.POINTER(_u64),
                                     ctypes.POINTER(ctypes.c_uint32), ctypes.POINTER(ctypes.c_uint32), _i32, _i32]
@@ -69,7 +79,7 @@ _lib.vdc_validate_streams.restype = _i32
 
 EXPORTED_SYMBOLS = [
     "vdc_version", "vdc_init", "vdc_set_smem_size", "vdc_launch", "vdc_launch_async", "vdc_launch_async_full",
-    "vdc_launch_static",
+    "vdc_launch_static", "vdc_launch_stages",
     "vdc_read_status",
     "vdc_build_tma_desc", "vdc_set_cache_policy", "vdc_enable_peer_access", "vdc_ipc_open", "vdc_ipc_close", "vdc_peer_alloc", "vdc_peer_free", "vdc_ipc_export", "vdc_opcode_count", "vdc_opcode_name", "vdc_opcode_value",
     "vdc_opcode_is_compute", "vdc_config", "vdc_family_specs", "vdc_last_error", "vdc_validate_streams",
@@ -176,6 +186,12 @@ def launch_async(num_sms, insts_per_sm, compute_insts, memory_insts, tma_descs, 
     fn = _lib.vdc_launch_async_full if full else _lib.vdc_launch_async
     _check(fn(num_sms, insts_per_sm, _ptr(compute_insts), _ptr(memory_insts), _ptr(tma_descs),
                                  _ptr(bars), _ptr(bars_init), _ptr(profile), int(stream), int(timeout_ns)))
+
+
+def launch_stages(stages, stream=0, timeout_ns=0):
+    """Enqueues the stages of one batched step (a ctypes array of Stage), in order, without synchronising."""
+    init()
+    _check(_lib.vdc_launch_stages(stages, len(stages), int(stream), int(timeout_ns)))
 
 
 def launch_static(num_sms, insts_per_sm, compute_insts, memory_insts, tma_descs, bars_init, stream=0, timeout_ns=0):

@@ -9,11 +9,10 @@ first and last SM started and ended it (i.e. the stage and its skew).
 
 With a library built by `python -m vdcores_b200.build --trace VDC_TRACE_ATTN` (or VDC_TRACE_GEMV) and selected
 through VDCORES_LIB, the stamps inside the attention task (barrier seen, prologue, page arrivals, arrival at the
-head's counter, merge) or inside the GEMV task are printed as well.  With --batch B > 1 the program is the batched
-one (projections on the tensor cores); a library built with --trace VDC_TC_PROFILE adds where the projection task's
-issuing warp and the task as a whole spend their cycles (sums per SM over one launch); one built with --trace
-VDC_TRACE_CHUNKS prints the life of SM 0's ring entries --entries LO:HI (published by the control warp, copy issued
-by the load port, seen by the consuming warp, slots given back)."""
+head's counter, merge) or inside the GEMV task are printed as well; one built with --trace VDC_TRACE_CHUNKS prints the
+life of SM 0's ring entries --entries LO:HI (published by the control warp, copy issued by the load port, seen by the
+consuming warp, slots given back).  With --batch B > 1 a step is a list of stage kernels: the program prints every
+stage's time by itself (CUDA events around it, so nothing overlaps) beside the whole step's."""
 import argparse
 import collections
 import dataclasses
@@ -31,23 +30,63 @@ GEMV_LABELS = ["task start", "pops done", "barrier open", "x ready", "phase begu
                "phase end", "released"]
 
 
+def trace_stages(eng, reps=20):
+    """Per stage: mean time alone, and the bytes of weights or cache it reads over that time; then the whole step."""
+    names = {isa.STAGE_ATTN: "attention", isa.STAGE_ATTN_PREFILL: "attention (prefill)", isa.STAGE_EMBED: "embedding",
+             isa.STAGE_ADVANCE: "advance", isa.STAGE_COPY: "copy"}
+    modes = {isa.STAGE_QKV: "qkv", isa.STAGE_RESID: "residual", isa.STAGE_SILU: "gate/up", isa.STAGE_ARGMAX: "vocabulary"}
+    state = eng.state.clone()
+    n = len(eng.stages)
+    ev = [[torch.cuda.Event(enable_timing=True) for _ in range(n + 1)] for _ in range(reps)]
+    one = [(runtime.Stage * 1)(s) for s in eng.stages]
+    whole = []
+    for r in range(reps):
+        for i in range(n):
+            ev[r][i].record(eng.stream)
+            runtime.launch_stages(one[i], eng.stream.cuda_stream, eng.timeout_ns)
+        ev[r][n].record(eng.stream)
+        eng.state.copy_(state)
+    for r in range(reps):
+        a, b = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+        a.record(eng.stream)
+        runtime.launch_stages(eng.stages, eng.stream.cuda_stream, eng.timeout_ns)
+        b.record(eng.stream)
+        eng.state.copy_(state)
+        whole.append((a, b))
+    runtime.read_status(eng.stream.cuda_stream)
+    wb = {0: 2.0, 1: 1.0, 2: 9 / 16}
+    total = 0.0
+    for i, s in enumerate(eng.stages):
+        us = float(np.median([ev[r][i].elapsed_time(ev[r][i + 1]) for r in range(reps)])) * 1e3
+        total += us
+        what = modes[s.mode] if s.kind == isa.STAGE_GEMM else names[s.kind]
+        nbytes = s.M * s.K * wb[s.wfmt] if s.kind == isa.STAGE_GEMM else 0
+        if s.kind == isa.STAGE_ATTN:
+            nbytes = int(state[:, isa.ST_POS].sum()) * s.n_kv * isa.HEAD_DIM * 4
+        print(f"   {i:3d} {what:20s} splits {s.splits}  {us:8.2f} us" + (f"  {nbytes / us / 1e3:8.1f} GB/s" if nbytes else ""))
+    print(f"   sum {total:.1f} us; whole step {float(np.median([a.elapsed_time(b) for a, b in whole])) * 1e3:.1f} us")
+
+
 def main():
     ap = argparse.ArgumentParser()
     ap.add_argument("--layers", type=int, default=4)
     ap.add_argument("--prompt", type=int, default=2048)
     ap.add_argument("--steps", type=int, default=5)
     ap.add_argument("--batch", type=int, default=1)
+    ap.add_argument("--wkind", default="bf16", choices=("bf16", "fp8", "nvfp4"), help="with --batch")
+    ap.add_argument("--stages", action="store_true", help="the stage kernels, at batch 1 too")
     ap.add_argument("--entries", default="60:120", help="ring entries of SM 0 to list (VDC_TRACE_CHUNKS library)")
     args = ap.parse_args()
     dev = torch.device("cuda", 0)
     cfg = dataclasses.replace(LLAMA31_8B, n_layers=args.layers)
     max_seq = ((args.prompt + 64 + 63) // 64) * 64
-    if args.batch > 1:
+    if args.batch != 1 or args.stages:
         from .batch import BatchDecodeEngine
-        eng = BatchDecodeEngine(cfg, args.batch, max_seq=max_seq, device=dev, max_steps=64)
+        eng = BatchDecodeEngine(cfg, args.batch, max_seq=max_seq, device=dev, max_steps=64, wkind=args.wkind)
         eng.init_random_weights(0)
         for b in range(args.batch):           # the cache contents do not matter for the timing: zero rows
             eng.set_state(args.prompt, 5 + b, b=b)
+        return trace_stages(eng)
     else:
         eng = DecodeEngine(cfg, max_seq=max_seq, device=dev, max_steps=64)
         eng.init_random_weights(0)
@@ -71,11 +110,6 @@ def main():
           f"CTA start skew {(pv[:, 0].max() - t0) / 1e3:.2f} us")
     rows = []
     n_traced = 24 if "trace_gemv" in trace else 56
-    if "tc_profile" in trace:
-        # the task stamps (rows 16 + 2 j) must stay clear of the projection task's sums in rows 100-106
-        n_tasks = max(sum(1 for w in eng.program.c[sm] if w[0] not in (isa.OP_EXT, isa.OP_TERMINATEC))
-                      for sm in range(eng.num_sms))
-        assert n_tasks <= 42, f"{n_tasks} tasks on one SM: use fewer layers (--layers 2) with the VDC_TC_PROFILE library"
     for sm in range(eng.num_sms):
         ops = [w[0] for w in eng.program.c[sm] if w[0] not in (isa.OP_EXT, isa.OP_TERMINATEC)]
         for j, o in enumerate(ops[:n_traced]):
@@ -123,16 +157,6 @@ def main():
                 d = [f"{(x - a[0]) / 1e3:6.2f}" if x else "     -" for x in a[1:]]
                 print(f"   {n:5d}  {(a[0] - t0) / 1e3:8.2f} (+{(a[0] - prev) / 1e3 if prev else 0:5.2f}) | {d[0]} | {d[1]} | {d[2]}")
             prev = a[0]
-    if "tc_profile" in trace:
-        clk = 1965.0      # SM cycles per microsecond at the clock the B200s of this pool run at
-        print("projection task, microseconds per SM in this launch (issuing warp, then the whole task):")
-        for row, label in ((8, "waiting for chunks (incl. the stage's input barrier)"), (14, "   of that, X chunks after a task's first"),
-                           (15, "   of that, W chunks after a task's first"), (9, "waiting for the normalised X chunk"),
-                           (10, "issuing MMAs"), (11, "waiting for the previous chunk's commit"), (100, "set-up"),
-                           (101, "streaming loop"), (102, "epilogue from tensor memory"), (103, "partial sums to scratch"),
-                           (104, "arrival at the block's counter"), (105, "last arrival's epilogue")):
-            print(f"   {label:56s} {pv[:, row].mean() / clk:8.1f}")
-        print(f"   weight chunks per SM {pv[:, 12].mean():.0f}, blocks finished per SM {pv[:, 106].mean():.1f}")
     if "trace_gemv" in trace:
         stage = ["qkv", "o", "gate/up", "down"]
         for o in range(8):
