@@ -72,8 +72,7 @@ int vdc_launch_async_full(int num_sms, int insts_per_sm, const void* compute_ins
 /* One stage of a batched decode step or of a prefill chunk (2..128 rows), run as a kernel of its own.
  *   kind VDC_STAGE_GEMM: projection of the k-chunk-major rows `x` [Bpad, K] with the M x K weights `w` (blocks of
  *     VDC_STAGE_BLOCK rows; wfmt 0 bf16, 1 e4m3, 2 NVFP4, fp32 per-row `scales` for the last two); every block's K is
- *     shared by `splits` CTAs of one cluster.  stats_in: sums of squares of the rows, which are
- *     then RMS-normalised with the weights norm_w on their way to the tensor cores (0: taken as they are).  `mode` says where the result goes:
+ *     shared by `splits` CTAs of one cluster.  `mode` says where the result goes:
  *       VDC_STAGE_QKV    heads: q/k norm (qk_norm, 0: none), rotation (`rope`), query rows to `out` [B, heads, 128], key
  *                        and value rows to the pages state.NEWROW names in kpool / vpool
  *       VDC_STAGE_RESID  hid += result; stats_out += squares of hid
@@ -83,6 +82,8 @@ int vdc_launch_async_full(int num_sms, int insts_per_sm, const void* compute_ins
  *   kind VDC_STAGE_ATTN_PREFILL: the same for rows that are consecutive positions of ONE sequence
  *   kind VDC_STAGE_EMBED: embedding rows (table `w`, width K) to hid, stats_out[0] = squares, the other n_stats - 1 rows
  *     of stats_out zeroed
+ *   kind VDC_STAGE_NORM: out = the rows x [Bpad, K], RMS-normalised with their sums of squares stats_in and the weights
+ *     norm_w
  *   kind VDC_STAGE_ADVANCE: keys -> next tokens, token log, state blocks moved on by one position
  *   kind VDC_STAGE_COPY: M bytes from x to out
  * Pointers are device addresses; 0 where a stage has no use for one. */

@@ -87,7 +87,7 @@ def test_projection_with_residual(cuda_device, B, K, M, splits, fmt):
 
 @pytest.mark.parametrize("B,K,M,splits,fmt", CASES)
 def test_projection_gate_up_and_argmax(cuda_device, B, K, M, splits, fmt):
-    from vdcores_b200 import isa
+    from vdcores_b200 import isa, runtime
     from vdcores_b200.batch import unpack_kc
     dev, Bp = cuda_device, bpad(B)
     x = seeded((B, K), 5)
@@ -98,22 +98,25 @@ def test_projection_gate_up_and_argmax(cuda_device, B, K, M, splits, fmt):
     keys = torch.zeros(B, dtype=torch.int64, device=dev)
     nw = (1 + 0.1 * seeded((K,), 4).float()).to(BF16)
     nwd = nw.to(dev)
-    common = dict(stats_in=sd.data_ptr(), norm_w=nwd.data_ptr(), eps=1e-5)
-    run(dev, gemm(dev, fmt, B, M, K, splits, w, sc, xd, mode=isa.STAGE_SILU, out=out.data_ptr(), **common))
+    xnd = torch.zeros_like(xd)
+    norm = runtime.Stage(kind=isa.STAGE_NORM, B=B, Bpad=Bp, K=K, x=xd.data_ptr(), out=xnd.data_ptr(), stats_in=sd.data_ptr(),
+                         norm_w=nwd.data_ptr(), eps=1e-5)
+    run(dev, norm, gemm(dev, fmt, B, M, K, splits, w, sc, xnd, mode=isa.STAGE_SILU, out=out.data_ptr()))
     xn = (x.float() * torch.rsqrt(stats[:B, None] / K + 1e-5)).to(BF16).float() * nw.float()
+    assert rel(unpack_kc(xnd.cpu(), Bp, K)[:B], xn) < REL
     y = xn.to(BF16).float() @ wf.t()
     yb = y.to(BF16).float()
     ref = torch.nn.functional.silu(yb[:, 0::2]) * yb[:, 1::2]
     assert rel(unpack_kc(out.cpu(), Bp, M // 2)[:B], ref) < 2 * REL
     if fmt == "bf16":
-        run(dev, gemm(dev, fmt, B, M, K, splits, w, sc, xd, mode=isa.STAGE_ARGMAX, keys=keys.data_ptr(), **common))
+        run(dev, gemm(dev, fmt, B, M, K, splits, w, sc, xnd, mode=isa.STAGE_ARGMAX, keys=keys.data_ptr()))
         rows = 0xFFFFFFFF - (keys.cpu() & 0xFFFFFFFF)
         top = y.max(1).values
         assert bool((y[torch.arange(B), rows] >= top - 2.0 ** -7 * top.abs()).all())
 
 
-@pytest.mark.parametrize("B,fmt,norm", [(3, "bf16", True), (16, "nvfp4", True), (128, "bf16", True), (16, "fp8", False)])
-def test_many_blocks_stream_in_order(cuda_device, B, fmt, norm):
+@pytest.mark.parametrize("B,fmt", [(3, "bf16"), (16, "nvfp4"), (128, "bf16"), (128, "fp8"), (16, "fp8")])
+def test_many_blocks_stream_in_order(cuda_device, B, fmt):
     """More CTAs than SMs, so that two stream side by side, and rings of 3 to 8 stages behind 64 chunks: every pass gives
     the same bits (each CTA alone owns its block's sums), and the sums of the inputs."""
     from vdcores_b200 import isa
@@ -121,18 +124,13 @@ def test_many_blocks_stream_in_order(cuda_device, B, fmt, norm):
     dev, Bp, K, M = cuda_device, bpad(B), 4096, 28672
     x = seeded((B, K), 11)
     w, sc, wf = weights(M, K, fmt, dev, seed=12)
-    stats = torch.zeros(128)
-    stats[:B] = x.float().pow(2).sum(1)
-    xd, sd, nwd = packed_rows(x, dev), stats.to(dev), torch.ones(K, dtype=BF16, device=dev)
-    outs = []
+    xd, outs = packed_rows(x, dev), []
     for _ in range(12):
         out = torch.zeros(Bp * M // 2, dtype=BF16, device=dev)
-        kw = dict(stats_in=sd.data_ptr(), norm_w=nwd.data_ptr(), eps=1e-5) if norm else {}
-        run(dev, gemm(dev, fmt, B, M, K, 1, w, sc, xd, mode=isa.STAGE_SILU, out=out.data_ptr(), **kw))
+        run(dev, gemm(dev, fmt, B, M, K, 1, w, sc, xd, mode=isa.STAGE_SILU, out=out.data_ptr()))
         outs.append(out)
     assert all(torch.equal(o, outs[0]) for o in outs)
-    xn = (x.float() * torch.rsqrt(stats[:B, None] / K + 1e-5)).to(BF16).float() if norm else x.float()
-    yb = (xn.to(dev).double() @ wf.to(dev).double().t()).to(BF16).float()
+    yb = (x.to(dev).double() @ wf.to(dev).double().t()).to(BF16).float()
     ref = torch.nn.functional.silu(yb[:, 0::2]) * yb[:, 1::2]
     assert rel(unpack_kc(outs[0].cpu(), Bp, M // 2)[:B], ref.cpu()) < 2 * REL
 

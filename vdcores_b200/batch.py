@@ -161,6 +161,7 @@ class BatchDecodeEngine(DecodeEngine):
         self.hidden = z(Bp * H)                       # k-chunk-major [Bpad, H]
         self.attn_out = z(Bp * cfg.q_width)           # k-chunk-major [Bpad, q_width]
         self.act = z(Bp * F)                          # k-chunk-major [Bpad, F]
+        self.normed = z(Bp * H)                       # k-chunk-major: normalised hidden rows
         self.q = z(B, cfg.q_width)                    # rotated query heads
         self.keys = z(B, dt=torch.int64)              # argmax keys (u64), zero between steps
         # per-sequence sums of squares of the hidden matrix after the embedding / each residual add
@@ -226,8 +227,7 @@ class BatchDecodeEngine(DecodeEngine):
             s *= 2
         return s
 
-    def _gemm(self, name, l, w, x, mode, norm=None, **kw):
-        # norm: (index of the rows' sums of squares, norm weights) of a projection with a fused input RMSNorm
+    def _gemm(self, name, l, w, x, mode, **kw):
         """Projection stage over layer l's matrix `name` ("lm": the vocabulary projection, bf16 in every engine)."""
         wf = self.wkind if name != "lm" else "bf16"
         K = {"wo": self.cfg.q_width, "wd": self.cfg.ffn}.get(name, self.cfg.hidden)
@@ -239,15 +239,15 @@ class BatchDecodeEngine(DecodeEngine):
         return runtime.Stage(
             kind=isa.STAGE_GEMM, mode=mode, wfmt={"bf16": 0, "fp8": 1, "nvfp4": 2}[wf], B=self.batch, Bpad=self.bpad,
             M=w.shape[0], K=K, splits=self._splits(blocks, 2, K // 64), w=self._pack_cache[name, l].data_ptr(),
-            scales=self.scales[name][l].data_ptr() if wf != "bf16" else 0, x=x.data_ptr(),
-            stats_in=self.stats[norm[0]].data_ptr() if norm else 0, norm_w=norm[1].data_ptr() if norm else 0,
-            eps=self.cfg.eps, **kw)
+            scales=self.scales[name][l].data_ptr() if wf != "bf16" else 0, x=x.data_ptr(), **kw)
 
     def _plan(self, vocab: bool = True):
         """The stages of one step; vocab False: it ends after the last layer (prefill chunks before the last)."""
         cfg, B = self.cfg, self.batch
         L, G = cfg.n_layers, cfg.group
         hid = self.hidden.data_ptr()
+        norm = lambda i, w: runtime.Stage(kind=isa.STAGE_NORM, B=B, Bpad=self.bpad, K=cfg.hidden, x=hid, out=self.normed.data_ptr(),
+                                          stats_in=stat(i), norm_w=w.data_ptr(), eps=cfg.eps)
         stat = lambda i: self.stats[i].data_ptr()
         state = dict(state=self.state.data_ptr(), state_stride=self.state_words)
         heads = dict(group=G, n_kv=cfg.n_kv_heads, **state)
@@ -259,21 +259,22 @@ class BatchDecodeEngine(DecodeEngine):
         self.attn_splits = self._splits(units, 4, self.max_pages)
         for l in range(L):
             pools = dict(kpool=self.kpool[l].data_ptr(), vpool=self.vpool[l].data_ptr())
-            out.append(self._gemm("wqkv", l, self.wqkv[l], self.hidden, isa.STAGE_QKV, (2 * l, self.ln1[l]), out=self.q.data_ptr(),
+            out.append(norm(2 * l, self.ln1[l]))
+            out.append(self._gemm("wqkv", l, self.wqkv[l], self.normed, isa.STAGE_QKV, out=self.q.data_ptr(),
                                   rope=self.rope.data_ptr(), qk_norm=self.qknorm[l].data_ptr() if cfg.qk_norm else 0,
                                   qk_eps=cfg.qk_norm_eps, **heads, **pools))
             out.append(runtime.Stage(kind=attn_kind, B=B, Bpad=self.bpad, splits=self.attn_splits, n_pages=self.max_pages,
                                      q=self.q.data_ptr(), out=self.attn_out.data_ptr(), **heads, **pools))
             out.append(self._gemm("wo", l, self.wo[l], self.attn_out, isa.STAGE_RESID, hid=hid,
                                   stats_out=stat(2 * l + 1)))
-            out.append(self._gemm("wgu", l, self.wgu[l], self.hidden, isa.STAGE_SILU, (2 * l + 1, self.ln2[l]),
-                                  out=self.act.data_ptr()))
+            out.append(norm(2 * l + 1, self.ln2[l]))
+            out.append(self._gemm("wgu", l, self.wgu[l], self.normed, isa.STAGE_SILU, out=self.act.data_ptr()))
             out.append(self._gemm("wd", l, self.wd[l], self.act, isa.STAGE_RESID, hid=hid, stats_out=stat(2 * l + 2)))
             if self.taps_enabled:
                 out.append(runtime.Stage(kind=isa.STAGE_COPY, x=hid, out=self.taps[l].data_ptr(), M=self.hidden.numel(), K=2))
         if vocab:
-            out.append(self._gemm("lm", 0, self.lm_head, self.hidden, isa.STAGE_ARGMAX, (2 * L, self.norm_w),
-                                  keys=self.keys.data_ptr()))
+            out.append(norm(2 * L, self.norm_w))
+            out.append(self._gemm("lm", 0, self.lm_head, self.normed, isa.STAGE_ARGMAX, keys=self.keys.data_ptr()))
             out.append(runtime.Stage(kind=isa.STAGE_ADVANCE, B=B, Bpad=self.bpad, keys=self.keys.data_ptr(),
                                      log=self.token_log.data_ptr(), log_stride=self.max_steps, **state))
         return (runtime.Stage * len(out))(*out)

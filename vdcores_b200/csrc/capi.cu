@@ -147,6 +147,9 @@ static const char* check_stage(const vdc_stage& s) {
     return "stage: rows out of range";
   if (s.kind == VDC_STAGE_EMBED)
     return s.K % 8 == 0 && s.w && s.hid && s.state && s.stats_out ? nullptr : "embedding stage: bad argument";
+  if (s.kind == VDC_STAGE_NORM)
+    return s.K > 0 && s.K % 8 == 0 && s.x && s.out && s.stats_in && s.norm_w && al16(s.x) && al16(s.out) && al16(s.norm_w)
+               ? nullptr : "norm stage: bad argument";
   if (s.kind == VDC_STAGE_ADVANCE) return s.state && s.keys && s.log ? nullptr : "advance stage: null pointer";
   if (!pow2(s.splits) || s.splits > 8) return "stage: splits must be 1, 2, 4 or 8";
   if (s.kind == VDC_STAGE_ATTN || s.kind == VDC_STAGE_ATTN_PREFILL) {
@@ -159,7 +162,6 @@ static const char* check_stage(const vdc_stage& s) {
     return "projection stage: bad shape";
   if (!s.w || !s.x || !al16(s.w) || !al16(s.x) || !al16(s.scales) || (s.wfmt && !s.scales))
     return "projection stage: null or misaligned pointer";
-  if (s.stats_in && (!s.norm_w || !al16(s.norm_w))) return "projection stage: norm weights missing or misaligned";
   switch (s.mode) {
     case VDC_STAGE_QKV:
       if (s.group < 1 || s.n_kv < 1 || s.M != s.n_kv * (s.group + 2) * VDC_HEAD_DIM) return "QKV stage: rows do not match the heads";

@@ -47,6 +47,7 @@
 #define VDC_STAGE_EMBED 4
 #define VDC_STAGE_ADVANCE 5
 #define VDC_STAGE_COPY 6
+#define VDC_STAGE_NORM 7
 #define VDC_STAGE_QKV 0
 #define VDC_STAGE_RESID 1
 #define VDC_STAGE_SILU 2

@@ -10,8 +10,8 @@
 // 128256-row vocabulary projection at 3 rows).
 //
 // Measured against the megakernel's program, two Llama-3.1-8B-shaped layers and a small vocabulary (B200): 3 rows at
-// 1000 positions 416 -> 252 us, 32 rows with e4m3 weights 758 -> 379, 64 rows at 2100 positions 932 -> 497, 128 rows
-// 1025 -> 577, a 2048-token prompt 15.8 -> 8.2 ms.
+// 1000 positions 416 -> 242 us, 32 rows with e4m3 weights 758 -> 324, 64 rows at 2100 positions 932 -> 436, 128 rows
+// 1025 -> 450, a 2048-token prompt 15.9 -> 6.5 ms.
 #include "mk_umma.cuh"
 
 #include "../../include/vdcores.h"
@@ -109,12 +109,11 @@ struct Waiter {
 // ------------------------------------------------------------------------- //
 struct GemmShared {
   uint64_t full[kMaxRing], empty[kMaxRing];
-  uint64_t ready[kMaxRing];     // rows normalised and weights converted
+  uint64_t ready[kMaxRing];     // weights converted
   uint64_t stg_empty[2];
   uint64_t done;
   uint32_t tmem;
   volatile int fail;
-  float rstd[128];
   float ssq[128];
   unsigned long long key[128];
 };
@@ -122,15 +121,15 @@ struct GemmShared {
 // Bytes of a chunk of n weight rows x 64 inputs as stored: bf16, e4m3, or e2m1 pairs with one e4m3 scale per 16.
 __host__ __device__ constexpr int chunk_bytes(int wfmt, int n) { return wfmt == 0 ? n * 128 : wfmt == 1 ? n * 64 : n * 36; }
 
-// One ring stage: the rows' chunk, the weights' chunk, the norm weights of the chunk's inputs.
+// One ring stage: the rows' chunk, then the weights' chunk.
 __host__ __device__ constexpr int stage_size(int wfmt, int bpad) {
-  return bpad * kKc * 2 + (chunk_bytes(wfmt, kBlk) + 127) / 128 * 128 + kKc * 2;
+  return bpad * kKc * 2 + (chunk_bytes(wfmt, kBlk) + 127) / 128 * 128;
 }
 __host__ __device__ inline int ring_stages(int wfmt, int bpad) {
   const int staging = wfmt ? 2 * kBlk * kKc * 2 : 0;
   const int stage = stage_size(wfmt, bpad);
   const int n = (kGemmSmem - 2048 - 128 - staging) / stage;
-  return n < kMaxRing ? n : kMaxRing;
+  return n >= kMaxRing ? kMaxRing : wfmt && n >= 4 ? n & ~1 : n;    // even where weights are converted, see `teams`
 }
 
 // Eight fp32 sums (columns col .. col+7 of row b) over the cluster's K-ranges, in rank order.
@@ -228,8 +227,12 @@ __global__ void __launch_bounds__(kGemmThreads, 2) stage_gemm(const __grid_const
   const int n0 = block * kBlk, N = min(kBlk, s.M - n0);
   const int chunks = s.K / kKc, c0 = chunks * rank / splits, n_ch = chunks * (rank + 1) / splits - c0;
   const int xbytes = s.Bpad * kKc * 2, wbytes = chunk_bytes(kFmt, N);
-  const int stage_bytes = stage_size(kFmt, s.Bpad), nw_off = stage_bytes - kKc * 2;
-  const bool norm = s.stats_in != 0, prepare = kFmt != 0 || norm;
+  const int stage_bytes = stage_size(kFmt, s.Bpad);
+  // Quantised weights are converted by two teams of warps that take the chunks in turn where the ring's length is even, so
+  // that a team sees every round of its stages; by all warps together where it is not (a team would then meet a stage two
+  // rounds on, and the barrier's parity cannot tell those apart).  Teams, because a team's wait for the tensor cores to
+  // leave its staging buffer then falls into the other's conversion: e4m3 gate/up at 32 rows 74.7 -> 65.6 us.
+  const int teams = n_ring & 1 ? 1 : 2;
   uint8_t* ring = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(dyn) + 127) & ~(uintptr_t)127);
   uint8_t* staging = ring + n_ring * stage_bytes;
   const Waiter wait{&sh.fail, status, timeout_ns, s.kind};
@@ -239,7 +242,7 @@ __global__ void __launch_bounds__(kGemmThreads, 2) stage_gemm(const __grid_const
     for (int i = 0; i < n_ring; ++i) {
       mbar_init(&sh.full[i], 1);
       mbar_init(&sh.empty[i], 1);
-      mbar_init(&sh.ready[i], kEpiThreads);
+      mbar_init(&sh.ready[i], kEpiThreads / 32 / teams);
     }
     for (int i = 0; i < 2; ++i) mbar_init(&sh.stg_empty[i], 1);
     mbar_init(&sh.done, 1);
@@ -260,12 +263,10 @@ __global__ void __launch_bounds__(kGemmThreads, 2) stage_gemm(const __grid_const
       const uint8_t* w = reinterpret_cast<const uint8_t*>(s.w) + (size_t)n0 * s.K * (kFmt == 0 ? 32 : kFmt == 1 ? 16 : 9) / 16 +
                          (size_t)c0 * wbytes;
       const uint8_t* x = reinterpret_cast<const uint8_t*>(s.x) + (size_t)c0 * xbytes;
-      const uint8_t* nw = reinterpret_cast<const uint8_t*>(s.norm_w) + (size_t)c0 * kKc * 2;
-      const uint32_t tx = (uint32_t)(xbytes + wbytes + (norm ? kKc * 2 : 0));
+      const uint32_t tx = (uint32_t)(xbytes + wbytes);
       auto load_weights = [&](int i, int st) {
         mbar_arrive_expect_tx(&sh.full[st], tx);
         bulk_load_1d(ring + st * stage_bytes + xbytes, w + (size_t)i * wbytes, (uint32_t)wbytes, &sh.full[st]);
-        if (norm) bulk_load_1d(ring + st * stage_bytes + nw_off, nw + (size_t)i * kKc * 2, kKc * 2, &sh.full[st]);
       };
       // the weights depend on nothing: they are on their way before the previous stage's results are waited for
       const int first = min(n_ch, n_ring);
@@ -289,7 +290,7 @@ __global__ void __launch_bounds__(kGemmThreads, 2) stage_gemm(const __grid_const
       for (int i = 0; i < n_ch && ok; ++i) {
         const int st = i % n_ring;
         ok = wait(&sh.full[st], (uint32_t)(i / n_ring) & 1u, 1, i);
-        if (prepare && ok) ok = wait(&sh.ready[st], (uint32_t)(i / n_ring) & 1u, 1, i);
+        if (kFmt != 0 && ok) ok = wait(&sh.ready[st], (uint32_t)(i / n_ring) & 1u, 1, i);
         if (!ok) break;
         tc_fence_after();
         uint8_t* at = ring + st * stage_bytes;
@@ -309,42 +310,19 @@ __global__ void __launch_bounds__(kGemmThreads, 2) stage_gemm(const __grid_const
     }
   } else {
     const int t = tid - 64;
-    if (prepare) {
-      // The eight warps normalise the rows in place, rounded like a bf16 tensor expression, bf16(w * bf16(x * rstd)), and
-      // turn quantised weights into bf16 pieces of the tensor cores' operand layout, 32 weights of one row per thread
-      // (exact for e4m3 and for e2m1 code times block scale).  Every thread takes part in every chunk: a warp that took
-      // only every other chunk could meet a ring stage two rounds ahead and read its barrier's parity the wrong way.
-      const int row = t & 127, g_lo = (t >> 7) * (kKc / 32);
-      if (norm) {
-        grid_dep_wait();
-        if (t < s.Bpad)
-          sh.rstd[t] = rsqrtf(__ldcg(reinterpret_cast<const float*>(s.stats_in) + t) / (float)s.K + s.eps);
-        asm volatile("bar.sync 1, %0;" ::"n"(kEpiThreads) : "memory");
-      }
-      const float rstd = norm ? sh.rstd[t & (s.Bpad - 1)] : 1.f;    // a thread's pieces belong to one row
-      for (int i = 0; i < n_ch; ++i) {
+    if (kFmt != 0) {
+      // bf16 pieces of the tensor cores' operand layout, 16 weights of a row at a time (exact for e4m3 and for e2m1 code
+      // times block scale)
+      const int team = kEpiThreads / teams, tt = t & (team - 1), row = t & 127;
+      for (int i = t / team; i < n_ch; i += teams) {
         const int st = i % n_ring;
         if (!wait(&sh.full[st], (uint32_t)(i / n_ring) & 1u, 2, i)) break;
-        if (norm) {
-          uint8_t* xs = ring + st * stage_bytes;
-          const uint8_t* nw = xs + nw_off;
-          for (int p = t; p < s.Bpad * (kKc / 8); p += kEpiThreads) {
-            const uint4 v = lds128(xs + p * 16), w = lds128(nw + p / s.Bpad * 16);
-            const uint32_t xv[4] = {v.x, v.y, v.z, v.w}, wv[4] = {w.x, w.y, w.z, w.w};
-            uint32_t o[4];
-#pragma unroll
-            for (int j = 0; j < 4; ++j)
-              o[j] = pack_bf16x2(bf16_round(bf_lo(xv[j]) * rstd) * bf_lo(wv[j]), bf16_round(bf_hi(xv[j]) * rstd) * bf_hi(wv[j]));
-            *reinterpret_cast<uint4*>(xs + p * 16) = make_uint4(o[0], o[1], o[2], o[3]);
-          }
-        }
-        if (kFmt != 0 && i >= 2 && !wait(&sh.stg_empty[i & 1], (uint32_t)((i >> 1) - 1) & 1u, 2, i)) break;
+        if (i >= 2 && !wait(&sh.stg_empty[i & 1], (uint32_t)((i >> 1) - 1) & 1u, 2, i)) break;
         uint8_t* dst = staging + (i & 1) * (kBlk * kKc * 2);
         const uint8_t* src = ring + st * stage_bytes + xbytes;
-        if (kFmt != 0 && row < N) {
-#pragma unroll
-          for (int gj = 0; gj < kKc / 32; ++gj) {
-            const int g16 = g_lo + gj;
+        if (row < N) {
+#pragma unroll 2
+          for (int g16 = tt >> 7; g16 < kKc / 16; g16 += team >> 7) {
             uint32_t o[8];
             if (kFmt == 1) {
               const uint4 v = lds128(src + (g16 * N + row) * 16);
@@ -372,7 +350,8 @@ __global__ void __launch_bounds__(kGemmThreads, 2) stage_gemm(const __grid_const
           }
         }
         fence_proxy_async_smem();
-        mbar_arrive(&sh.ready[st]);
+        __syncwarp();
+        if (lane == 0) mbar_arrive(&sh.ready[st]);   // one arrival per warp: one per thread would queue on the barrier's word
       }
     }
     grid_dep_wait();
@@ -933,6 +912,29 @@ __global__ void __launch_bounds__(256) stage_embed(const __grid_constant__ vdc_s
   for (int i = 1 + tid; i < s.n_stats; i += 256) stats[(size_t)i * 128 + b] = 0.f;
 }
 
+// RMSNorm of the hidden rows into a matrix of their own, rounded like a bf16 tensor expression: bf16(w * bf16(x * rstd)).
+// A stage of its own, once per projection, instead of in every block of the projection that reads the rows: two layers and
+// a 128256-row vocabulary projection 382 -> 374 us at 3 rows, 617 -> 574 at 64, 1070 -> 821 at 128 (normalising inside
+// the projection, a block's warps rewrote every chunk in shared memory between its arrival and the tensor cores).
+__global__ void __launch_bounds__(256) stage_norm(const __grid_constant__ vdc_stage s) {
+  const int p = (int)blockIdx.x * 256 + (int)threadIdx.x;      // 16-byte piece: eight inputs of one row
+  const int k8 = p / s.Bpad, b = p & (s.Bpad - 1);
+  const bool live = k8 < s.K / 8;
+  const uint4 w = live ? __ldg(reinterpret_cast<const uint4*>(s.norm_w) + k8) : make_uint4(0u, 0u, 0u, 0u);
+  grid_dep_wait();
+  grid_dep_launch();
+  if (!live) return;
+  // piece (k8, b) of a k-chunk-major matrix is its p-th piece
+  const uint4 v = ldcg128(reinterpret_cast<const uint8_t*>(s.x) + (size_t)p * 16);
+  const float rstd = rsqrtf(__ldcg(reinterpret_cast<const float*>(s.stats_in) + b) / (float)s.K + s.eps);
+  const uint32_t xv[4] = {v.x, v.y, v.z, v.w}, wv[4] = {w.x, w.y, w.z, w.w};
+  uint32_t o[4];
+#pragma unroll
+  for (int j = 0; j < 4; ++j)
+    o[j] = pack_bf16x2(bf16_round(bf_lo(xv[j]) * rstd) * bf_lo(wv[j]), bf16_round(bf_hi(xv[j]) * rstd) * bf_hi(wv[j]));
+  *reinterpret_cast<uint4*>(reinterpret_cast<uint8_t*>(s.out) + (size_t)p * 16) = make_uint4(o[0], o[1], o[2], o[3]);
+}
+
 // Next token, token log and state advance of every sequence.
 __global__ void __launch_bounds__(128) stage_advance(const __grid_constant__ vdc_stage s) {
   grid_dep_wait();
@@ -1007,6 +1009,10 @@ extern "C" cudaError_t vdc_stage_launch(const vdc_stage* s, vdc_status* status, 
       cfg.dynamicSmemBytes = vdc::kAttnSmem;
       return cudaLaunchKernelEx(&cfg, vdc::stage_attn_prefill, *s, status, timeout_ns);
     }
+    case VDC_STAGE_NORM:
+      cfg.gridDim = dim3((unsigned)((s->Bpad * (s->K / 8) + 255) / 256));
+      cfg.blockDim = dim3(256);
+      return cudaLaunchKernelEx(&cfg, vdc::stage_norm, *s);
     case VDC_STAGE_EMBED:
       cfg.gridDim = dim3((unsigned)s->B);
       cfg.blockDim = dim3(256);

@@ -51,8 +51,8 @@ GEMM_MODE_SILU_PAIRS = _defs["GEMM_MODE_SILU_PAIRS"]
 GEMM_MODE_ARGMAX = _defs["GEMM_MODE_ARGMAX"]
 GEMM_MODE_ADD_PACKED = _defs["GEMM_MODE_ADD_PACKED"]
 
-STAGE_GEMM, STAGE_ATTN, STAGE_ATTN_PREFILL, STAGE_EMBED, STAGE_ADVANCE, STAGE_COPY = (
-    _defs["STAGE_" + k] for k in ("GEMM", "ATTN", "ATTN_PREFILL", "EMBED", "ADVANCE", "COPY"))
+STAGE_GEMM, STAGE_ATTN, STAGE_ATTN_PREFILL, STAGE_EMBED, STAGE_ADVANCE, STAGE_COPY, STAGE_NORM = (
+    _defs["STAGE_" + k] for k in ("GEMM", "ATTN", "ATTN_PREFILL", "EMBED", "ADVANCE", "COPY", "NORM"))
 STAGE_QKV, STAGE_RESID, STAGE_SILU, STAGE_ARGMAX = (_defs["STAGE_" + k] for k in ("QKV", "RESID", "SILU", "ARGMAX"))
 STAGE_BLOCK = _defs["STAGE_BLOCK"]
 

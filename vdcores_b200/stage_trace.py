@@ -33,7 +33,7 @@ GEMV_LABELS = ["task start", "pops done", "barrier open", "x ready", "phase begu
 def trace_stages(eng, reps=20):
     """Per stage: mean time alone, and the bytes of weights or cache it reads over that time; then the whole step."""
     names = {isa.STAGE_ATTN: "attention", isa.STAGE_ATTN_PREFILL: "attention (prefill)", isa.STAGE_EMBED: "embedding",
-             isa.STAGE_ADVANCE: "advance", isa.STAGE_COPY: "copy"}
+             isa.STAGE_ADVANCE: "advance", isa.STAGE_COPY: "copy", isa.STAGE_NORM: "norm"}
     modes = {isa.STAGE_QKV: "qkv", isa.STAGE_RESID: "residual", isa.STAGE_SILU: "gate/up", isa.STAGE_ARGMAX: "vocabulary"}
     state = eng.state.clone()
     n = len(eng.stages)
