@@ -26,7 +26,7 @@ constexpr int kEpiThreads = 256;
 // Shared memory of one CTA.  Two CTAs fit an SM (the register budget allows it too), so that one streams while the
 // other is in its prologue or epilogue, and the next stage's CTAs move in while the last ones of this stage finish.
 constexpr int kGemmSmem = 110 * 1024;
-constexpr int kEpiLd = kBlk + 4;        // row stride of the fp32 exchange tile: eight rows start in eight bank groups
+constexpr int kCol4 = kBlk / 4;         // groups of four columns in the fp32 exchange tile
 
 // ------------------------------------------------------------------------- //
 // helpers
@@ -50,10 +50,11 @@ __device__ __forceinline__ float4 ld_cluster4(uint32_t a) {
   asm volatile("ld.shared::cluster.v4.f32 {%0,%1,%2,%3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "r"(a) : "memory");
   return v;
 }
-__device__ __forceinline__ float2 ld_cluster2(uint32_t a) {
-  float2 v;
-  asm volatile("ld.shared::cluster.v2.f32 {%0,%1}, [%2];" : "=f"(v.x), "=f"(v.y) : "r"(a) : "memory");
-  return v;
+__device__ __forceinline__ void st_cluster4(uint32_t a, uint32_t x, uint32_t y, uint32_t z, uint32_t w) {
+  asm volatile("st.shared::cluster.v4.b32 [%0], {%1,%2,%3,%4};" ::"r"(a), "r"(x), "r"(y), "r"(z), "r"(w) : "memory");
+}
+__device__ __forceinline__ void st_shared4(uint32_t a, uint32_t x, uint32_t y, uint32_t z, uint32_t w) {
+  asm volatile("st.shared.v4.b32 [%0], {%1,%2,%3,%4};" ::"r"(a), "r"(x), "r"(y), "r"(z), "r"(w) : "memory");
 }
 __device__ __forceinline__ float ld_cluster1(uint32_t a) {
   float v;
@@ -132,14 +133,20 @@ __host__ __device__ inline int ring_stages(int wfmt, int bpad) {
   return n >= kMaxRing ? kMaxRing : wfmt && n >= 4 ? n & ~1 : n;    // even where weights are converted, see `teams`
 }
 
-// Eight fp32 sums (columns col .. col+7 of row b) over the cluster's K-ranges, in rank order.
-__device__ __forceinline__ void sum8(float (&v)[8], uint32_t tile, int splits, int b, int col) {
-  const uint32_t at = tile + (uint32_t)(b * kEpiLd + col) * 4u;
+// The exchange tile of a CTA: [source CTA][four columns][its row, one spare][4] fp32.  Every CTA of the cluster writes the
+// sums of its K-range straight from tensor memory into the tile of the CTA that finishes the row (consecutive rows lie
+// side by side, so a warp's store is contiguous; the spare row spreads the column groups over the banks); what is then
+// read is local.  Pulling the sums instead cost one remote round trip per source and item.
+__device__ __forceinline__ uint32_t tile_at(uint32_t tile, int src, int nb, int col4, int row) {
+  return tile + (uint32_t)(((src * kCol4 + col4) * (nb + 1) + row) * 16);
+}
+// Eight fp32 sums (columns col .. col+7 of the CTA's row bl) over the cluster's K-ranges, in rank order.
+__device__ __forceinline__ void sum8(float (&v)[8], const uint8_t* tile, int splits, int nb, int bl, int col) {
 #pragma unroll
   for (int j = 0; j < 8; ++j) v[j] = 0.f;
   for (int r = 0; r < splits; ++r) {
-    const uint32_t p = peer_smem(at, (uint32_t)r);
-    const float4 a = ld_cluster4(p), c = ld_cluster4(p + 16);
+    const uint8_t* p = tile + (size_t)((r * kCol4 + (col >> 2)) * (nb + 1) + bl) * 16;
+    const float4 a = *reinterpret_cast<const float4*>(p), c = *reinterpret_cast<const float4*>(p + (nb + 1) * 16);
     v[0] += a.x; v[1] += a.y; v[2] += a.z; v[3] += a.w;
     v[4] += c.x; v[5] += c.y; v[6] += c.z; v[7] += c.w;
   }
@@ -158,16 +165,15 @@ __device__ __forceinline__ void scale8(float (&v)[8], const float* sc) {
 // One head of the QKV projection, one warp per row: optional RMSNorm over the head, half-rotation, then a query row to
 // the query matrix or a key / value row to the row's cache page.  Every product is rounded as a bf16 tensor expression
 // rounds it.  Lane i holds dims 2i, 2i+1 and their rotation partners 64 further.
-__device__ __forceinline__ void qkv_head(const vdc_stage& s, uint32_t tile, int splits, int b, int block,
+__device__ __forceinline__ void qkv_head(const vdc_stage& s, const uint8_t* tile, int splits, int nb, int bl, int b, int block,
                                          int lane) {
   constexpr int D = VDC_HEAD_DIM;
   const int G = s.group, kvh = block / (G + 2), part = block % (G + 2), n0 = block * kBlk;
   const int i0 = lane * 2;
   float x[4] = {0.f, 0.f, 0.f, 0.f};
-  const uint32_t at = tile + (uint32_t)(b * kEpiLd + i0) * 4u;
   for (int r = 0; r < splits; ++r) {
-    const uint32_t p = peer_smem(at, (uint32_t)r);
-    const float2 lo = ld_cluster2(p), hi = ld_cluster2(p + 256);
+    const uint8_t* p = tile + (size_t)((r * kCol4 + (i0 >> 2)) * (nb + 1) + bl) * 16 + (i0 & 3) * 4;
+    const float2 lo = *reinterpret_cast<const float2*>(p), hi = *reinterpret_cast<const float2*>(p + (size_t)(16 * (nb + 1)) * 16);
     x[0] += lo.x; x[1] += lo.y; x[2] += hi.x; x[3] += hi.y;
   }
   const float* scales = reinterpret_cast<const float*>(s.scales);
@@ -356,11 +362,18 @@ __global__ void __launch_bounds__(kGemmThreads, 2) stage_gemm(const __grid_const
     }
     grid_dep_wait();
   }
-  __syncthreads();   // lane 0 of warp 1 saw the last commit: the accumulator is complete, the ring is free
+  __syncwarp();
+  // lane 0 of warp 1 saw the last commit: the accumulators are complete, and the rings free, in every CTA of the cluster
+  if (splits > 1) {
+    cluster_arrive();
+    cluster_wait();
+  } else {
+    __syncthreads();
+  }
   tc_fence_after();
   const bool failed = sh.fail != 0;
-  float* tile_p = reinterpret_cast<float*>(ring);
-  const uint32_t tile = smem_u32(tile_p);
+  const uint32_t tile = smem_u32(ring);
+  const int nb = s.Bpad / splits;                    // rows this CTA finishes: a power of two
   if (warp >= 2 && !failed) {
     const int quarter = warp & 3, half = (warp - 2) >> 2;
     const int b = quarter * 32 + lane, ng = N >> 4;
@@ -368,10 +381,13 @@ __global__ void __launch_bounds__(kGemmThreads, 2) stage_gemm(const __grid_const
       for (int gi = half ? (ng + 1) / 2 : 0; gi < (half ? ng : (ng + 1) / 2); ++gi) {
         uint32_t r[16];
         tmem_ld16(tmem + ((uint32_t)(quarter * 32) << 16) + (uint32_t)(gi * 16), r);
-        if (b < s.Bpad) {
-          uint4* d = reinterpret_cast<uint4*>(tile_p + b * kEpiLd + gi * 16);
+        if (b >= s.Bpad) continue;
+        const uint32_t at = tile_at(tile, rank, nb, gi * 4, b & (nb - 1)), step = (uint32_t)(nb + 1) * 16u;
+        const uint32_t to = splits > 1 ? peer_smem(at, (uint32_t)(b / nb)) : at;
 #pragma unroll
-          for (int j = 0; j < 4; ++j) d[j] = make_uint4(r[4 * j], r[4 * j + 1], r[4 * j + 2], r[4 * j + 3]);
+        for (int j = 0; j < 4; ++j) {
+          if (splits > 1) st_cluster4(to + j * step, r[4 * j], r[4 * j + 1], r[4 * j + 2], r[4 * j + 3]);
+          else st_shared4(to + j * step, r[4 * j], r[4 * j + 1], r[4 * j + 2], r[4 * j + 3]);
         }
       }
     }
@@ -387,11 +403,11 @@ __global__ void __launch_bounds__(kGemmThreads, 2) stage_gemm(const __grid_const
   // ---- epilogue: this CTA finishes Bpad / splits of the rows, all columns of the block
   if (warp >= 2 && !failed) {
     const int t = tid - 64;
-    const int nb = s.Bpad / splits, b_lo = rank * nb;
+    const int b_lo = rank * nb;
     const float* scales = reinterpret_cast<const float*>(s.scales);
     if (s.mode == VDC_STAGE_QKV) {
       for (int bl = warp - 2; bl < nb; bl += kEpiThreads / 32)
-        if (b_lo + bl < s.B) qkv_head(s, tile, splits, b_lo + bl, block, lane);
+        if (b_lo + bl < s.B) qkv_head(s, ring, splits, nb, bl, b_lo + bl, block, lane);
     } else {
       const int bl = t & (nb - 1), b = b_lo + bl;      // nb is a power of two, at most 128
       const int f0 = t / nb, fstep = kEpiThreads / nb;
@@ -400,7 +416,7 @@ __global__ void __launch_bounds__(kGemmThreads, 2) stage_gemm(const __grid_const
           float ssq = 0.f;
           for (int f = f0; f < N / 8; f += fstep) {
             float v[8];
-            sum8(v, tile, splits, b, f * 8);
+            sum8(v, ring, splits, nb, bl, f * 8);
             scale8(v, scales ? scales + n0 + f * 8 : nullptr);
             uint4* hp = reinterpret_cast<uint4*>(reinterpret_cast<uint8_t*>(s.hid) + kc_piece(s.Bpad, b, n0 + f * 8));
             const uint4 h = *hp;
@@ -420,7 +436,7 @@ __global__ void __launch_bounds__(kGemmThreads, 2) stage_gemm(const __grid_const
 #pragma unroll
             for (int h = 0; h < 2; ++h) {
               float v[8];
-              sum8(v, tile, splits, b, f * 16 + h * 8);
+              sum8(v, ring, splits, nb, bl, f * 16 + h * 8);
               scale8(v, scales ? scales + n0 + f * 16 + h * 8 : nullptr);
 #pragma unroll
               for (int j = 0; j < 4; ++j) {
@@ -435,7 +451,7 @@ __global__ void __launch_bounds__(kGemmThreads, 2) stage_gemm(const __grid_const
           int row = 0x7fffffff;
           for (int f = f0; f < N / 8; f += fstep) {
             float v[8];
-            sum8(v, tile, splits, b, f * 8);
+            sum8(v, ring, splits, nb, bl, f * 8);
 #pragma unroll
             for (int j = 0; j < 8; ++j) {
               const float l = bf16_round(v[j]);
@@ -461,12 +477,6 @@ __global__ void __launch_bounds__(kGemmThreads, 2) stage_gemm(const __grid_const
     }
   }
   wait.drain();
-  __syncwarp();
-  if (splits > 1) {
-    cluster_arrive();   // nobody leaves while another CTA of the cluster reads its tile
-    cluster_wait();
-  }
-  __syncthreads();
   if (warp == 1) tmem_dealloc(tmem, kBlk);
 }
 
@@ -545,19 +555,33 @@ __device__ __forceinline__ void attn_merge(AttnShared& sh, uint32_t tile, int sp
   const int per = VDC_HEAD_DIM / 8;
   for (int it = rank * nt + t; it < rows * per; it += splits * nt) {
     const int r = it / per, d = (it % per) * 8;
-    float m = -INFINITY;
-    for (int k = 0; k < splits; ++k) m = fmaxf(m, ld_cluster1(peer_smem(m_at + r * 4, k)));
-    float den = 0.f, v[8];
+    // every CTA's share is requested before the first one is used: two remote round trips instead of two per CTA
+    float mk[8], m = -INFINITY, den = 0.f, v[8];
+    float4 a[8], c[8];
+    float lk[8];
+#pragma unroll
+    for (int k = 0; k < 8; ++k) {
+      mk[k] = -INFINITY;
+      lk[k] = 0.f;
+      a[k] = c[k] = make_float4(0.f, 0.f, 0.f, 0.f);
+      if (k < splits) {
+        mk[k] = ld_cluster1(peer_smem(m_at + r * 4, k));
+        lk[k] = ld_cluster1(peer_smem(l_at + r * 4, k));
+        const uint32_t p = peer_smem(tile + (uint32_t)(r * kRecLd + d) * 4u, k);
+        a[k] = ld_cluster4(p);
+        c[k] = ld_cluster4(p + 16);
+      }
+    }
+#pragma unroll
+    for (int k = 0; k < 8; ++k) m = fmaxf(m, mk[k]);
 #pragma unroll
     for (int j = 0; j < 8; ++j) v[j] = 0.f;
-    for (int k = 0; k < splits; ++k) {
-      const float mk = ld_cluster1(peer_smem(m_at + r * 4, k));
-      const float w = mk == -INFINITY ? 0.f : exp2f(mk - m);
-      den = fmaf(w, ld_cluster1(peer_smem(l_at + r * 4, k)), den);
-      const uint32_t p = peer_smem(tile + (uint32_t)(r * kRecLd + d) * 4u, k);
-      const float4 a = ld_cluster4(p), c = ld_cluster4(p + 16);
-      v[0] = fmaf(w, a.x, v[0]); v[1] = fmaf(w, a.y, v[1]); v[2] = fmaf(w, a.z, v[2]); v[3] = fmaf(w, a.w, v[3]);
-      v[4] = fmaf(w, c.x, v[4]); v[5] = fmaf(w, c.y, v[5]); v[6] = fmaf(w, c.z, v[6]); v[7] = fmaf(w, c.w, v[7]);
+#pragma unroll
+    for (int k = 0; k < 8; ++k) {
+      const float w = mk[k] == -INFINITY ? 0.f : exp2f(mk[k] - m);
+      den = fmaf(w, lk[k], den);
+      v[0] = fmaf(w, a[k].x, v[0]); v[1] = fmaf(w, a[k].y, v[1]); v[2] = fmaf(w, a[k].z, v[2]); v[3] = fmaf(w, a[k].w, v[3]);
+      v[4] = fmaf(w, c[k].x, v[4]); v[5] = fmaf(w, c[k].y, v[5]); v[6] = fmaf(w, c[k].z, v[6]); v[7] = fmaf(w, c[k].w, v[7]);
     }
     const float inv = den > 0.f ? 1.f / den : 0.f;
 #pragma unroll
