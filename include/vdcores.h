@@ -80,6 +80,8 @@ int vdc_launch_async_full(int num_sms, int insts_per_sm, const void* compute_ins
  *       VDC_STAGE_ARGMAX the rows' largest logit into keys
  *   kind VDC_STAGE_ATTN: attention of every row over its own pages (one row per sequence), queries `q`, result `out`
  *   kind VDC_STAGE_ATTN_PREFILL: the same for rows that are consecutive positions of ONE sequence
+ *     (both read the state blocks, and pages without a new row, while the stage directly in front still runs: that stage
+ *     may write the new cache rows and the queries, nothing else of these)
  *   kind VDC_STAGE_EMBED: embedding rows (table `w`, width K) to hid, stats_out[0] = squares, the other n_stats - 1 rows
  *     of stats_out zeroed
  *   kind VDC_STAGE_NORM: out = the rows x [Bpad, K], RMS-normalised with their sums of squares stats_in and the weights

@@ -135,6 +135,34 @@ def test_many_blocks_stream_in_order(cuda_device, B, fmt):
     assert rel(unpack_kc(outs[0].cpu(), Bp, M // 2)[:B], ref.cpu()) < 2 * REL
 
 
+def test_quantised_codes_widen_exactly(cuda_device):
+    """Every e4m3 code, and every e2m1 code under every block scale, against one-hot rows: the stored value itself, the
+    codes that are no numbers included."""
+    from vdcores_b200 import isa
+    from vdcores_b200.batch import pack_blocks_fp8, pack_blocks_nvfp4, unpack_kc
+    dev, K, M, B = cuda_device, 64, 256, 64
+    x = torch.eye(B, K).to(BF16)
+    codes = torch.zeros(M, K, dtype=torch.uint8)
+    codes[torch.arange(M), torch.arange(M) % K] = torch.arange(M, dtype=torch.uint8)
+    rows = torch.zeros(M, K // 2 + K // 16, dtype=torch.uint8)
+    pairs = torch.tensor([(2 * j) | ((2 * j + 1) << 4) for j in range(8)], dtype=torch.uint8)
+    rows[:, :8], rows[:, K // 2] = pairs, torch.arange(M, dtype=torch.uint8)
+    ones = torch.ones(M, device=dev)
+    grid = torch.tensor([0.0, 0.5, 1.0, 1.5, 2.0, 3.0, 4.0, 6.0])
+    e4m3 = torch.arange(256, dtype=torch.uint8).view(torch.float8_e4m3fn).float()
+    want8 = torch.zeros(B, M)
+    want8[torch.arange(M) % K, torch.arange(M)] = e4m3
+    want4 = torch.zeros(B, M)
+    want4[:16] = torch.cat((grid, -grid))[:, None] * e4m3[None]
+    for fmt, w, want in (("fp8", pack_blocks_fp8(codes.to(dev), isa.STAGE_BLOCK), want8),
+                         ("nvfp4", pack_blocks_nvfp4(rows.to(dev), K, isa.STAGE_BLOCK), want4)):
+        xd, hd, st = packed_rows(x, dev), torch.zeros(64 * M, dtype=BF16, device=dev), torch.zeros(128, device=dev)
+        run(dev, gemm(dev, fmt, B, M, K, 1, w, ones, xd, mode=isa.STAGE_RESID, hid=hd.data_ptr(), stats_out=st.data_ptr()))
+        got = unpack_kc(hd.cpu(), 64, M).float()
+        nan = torch.isnan(e4m3)[None].expand(B, -1)     # a row with a code that is no number is one in every sum
+        assert torch.equal(got[~nan], want[~nan]) and bool(torch.isnan(got[nan]).all())
+
+
 @pytest.mark.parametrize("kind", ["decode", "prefill"])
 @pytest.mark.parametrize("G,n_kv,B,splits,lens", [(4, 2, 3, 8, [1, 64, 65]), (8, 1, 2, 2, [700, 129]), (4, 1, 17, 1, None),
                                                   (8, 2, 9, 4, None), (4, 2, 128, 2, None)])
