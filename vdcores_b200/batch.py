@@ -256,7 +256,10 @@ class BatchDecodeEngine(DecodeEngine):
         tile = 64 // G      # rows of one prefill attention unit
         units = cfg.n_kv_heads * (-(-B // tile) if self.SHARED_CACHE else B)
         attn_kind = isa.STAGE_ATTN_PREFILL if self.SHARED_CACHE else isa.STAGE_ATTN
-        self.attn_splits = self._splits(units, 4, self.max_pages)
+        # a prefill tile's shares are 64 rows each to merge: no more CTAs than are resident at once (8 shares of 64 tiles
+        # took 31 us at four pages and 46 at 31 pages); a decode unit's are 4 or 8 rows, and two waves of CTAs even out
+        # sequences of different lengths
+        self.attn_splits = self._splits(units, 2 if self.SHARED_CACHE else 4, self.max_pages)
         for l in range(L):
             pools = dict(kpool=self.kpool[l].data_ptr(), vpool=self.vpool[l].data_ptr())
             out.append(norm(2 * l, self.ln1[l]))
