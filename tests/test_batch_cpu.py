@@ -133,3 +133,22 @@ def test_emitted_streams_read_every_weight_byte_once_and_the_right_activations()
     # compute side: one task per unit, eleven words each
     assert sum(1 for sm in range(S) for c in P.c[sm] if c[0] == isa.OP_GEMM_TC_BF16) == len(units)
     assert all(len(P.c[sm]) % 11 == 0 for sm in range(S))
+
+
+def test_prefill_state_blocks_of_a_chunk():
+    """Row b of chunk c: its position, page count, token, cache row and page table; rows past the prompt repeat the last."""
+    import types
+    import numpy as np
+    from vdcores_b200.prefill import PrefillEngine
+    table = torch.tensor([3, 0, 4, 1, 2], dtype=torch.int32)
+    e = types.SimpleNamespace(batch=48, page_table=table, max_pages=5, cfg=types.SimpleNamespace(n_kv_heads=2))
+    tokens = np.arange(1000, 1130, dtype=np.int32)      # 130 positions: chunks of 48, 48 and 34
+    for c in range(3):
+        s = np.full((48, isa.ST_PAGETABLE + 5), -7, dtype=np.int32)
+        PrefillEngine._fill_states(e, s, tokens, c)
+        for b in range(48):
+            pos = min(c * 48 + b, 129)
+            assert s[b, isa.ST_POS] == pos and s[b, isa.ST_TOKEN] == 1000 + pos and s[b, isa.ST_NPAGES] == pos // 64 + 1
+            assert s[b, isa.ST_NEWROW] == int(table[pos // 64]) * 64 * 2 + pos % 64
+            assert s[b, isa.ST_NKVH] == 2 and s[b, isa.ST_MAXPAGES] == 5 and s[b, isa.ST_STEP] == 0 and s[b, isa.ST_ERR] == 0
+            assert (s[b, isa.ST_PAGETABLE:] == table.numpy()).all()

@@ -12,6 +12,7 @@ takes over.
 The reference has no prefill of its own on the device either side of its decode schedules: its correctness runs
 take the prompt's cache from a HuggingFace forward (app/python/llama3/sched.py:574-622 in the reference); this
 engine replaces the PyTorch prefill of decode.DecodeEngine.prefill on the product path."""
+import numpy as np
 import torch
 
 from . import isa, runtime
@@ -55,35 +56,34 @@ class PrefillEngine(BatchDecodeEngine):
         self._body = self._plan(vocab=False)
 
     # ------------------------------------------------------------------ chunks
-    def _chunk_states(self, tokens: torch.Tensor) -> torch.Tensor:
-        """State blocks [n_chunks, chunk, state_words] of a prompt: row b of chunk c is position c * chunk + b
-        (rows past the prompt's end repeat its last position: same row, same bytes)."""
-        T, B = int(tokens.numel()), self.batch
-        n_chunks = (T + B - 1) // B
-        pos = torch.arange(n_chunks * B).clamp_(max=T - 1)
-        table = self.page_table.to(torch.int64)
-        s = torch.zeros(n_chunks * B, self.state_words, dtype=torch.int32)
-        s[:, isa.ST_POS] = pos.to(torch.int32)
-        s[:, isa.ST_NPAGES] = (pos // isa.KV_PAGE + 1).to(torch.int32)
-        s[:, isa.ST_TOKEN] = tokens.to(torch.int32)[pos]
-        s[:, isa.ST_NEWROW] = (table[pos // isa.KV_PAGE] * isa.KV_PAGE * self.cfg.n_kv_heads + pos % isa.KV_PAGE).to(torch.int32)
+    def _fill_states(self, s, tokens, c: int):
+        """State blocks of chunk c into the int32 array s [chunk, state_words]: row b is position c * chunk + b (rows past
+        the prompt's end repeat its last position: same row, same bytes)."""
+        pos = np.minimum(np.arange(c * self.batch, (c + 1) * self.batch), len(tokens) - 1)
+        page = pos // isa.KV_PAGE
+        table = self.page_table.numpy()
+        s[:, :isa.ST_PAGETABLE] = 0
+        s[:, isa.ST_POS] = pos
+        s[:, isa.ST_NPAGES] = page + 1
+        s[:, isa.ST_TOKEN] = tokens[pos]
+        s[:, isa.ST_NEWROW] = table[page] * (isa.KV_PAGE * self.cfg.n_kv_heads) + pos % isa.KV_PAGE
         s[:, isa.ST_NKVH] = self.cfg.n_kv_heads
         s[:, isa.ST_MAXPAGES] = self.max_pages
-        s[:, isa.ST_PAGETABLE:] = self.page_table
-        return s.view(n_chunks, B, self.state_words)
+        s[:, isa.ST_PAGETABLE:] = table
 
     @torch.no_grad()
     def prefill(self, tokens: torch.Tensor, set_target_state: bool = True) -> int:
-        """Runs the prompt, ceil(T / chunk) launches, and returns the first generated (greedy) id.  The only host
-        work inside the loop is enqueueing, per chunk, the copy of its prepared state blocks and the launch."""
+        """Runs the prompt, ceil(T / chunk) lists of stages, and returns the first generated (greedy) id.  A chunk's state
+        blocks are prepared in pinned memory while the GPU runs the chunk before it."""
         T, B = int(tokens.numel()), self.batch
         assert 1 <= T < self.max_seq and self.stages is not None
-        states = self._chunk_states(tokens.cpu()).to(self.dev)
+        n = (T + B - 1) // B
+        ids = tokens.cpu().to(torch.int32).numpy().reshape(-1)
+        states = torch.empty(n, B, self.state_words, dtype=torch.int32, pin_memory=True)    # one block per chunk: none is rewritten
         self.keys.zero_()
-        self.stats.zero_()
         with torch.cuda.stream(self.stream):
-            n = states.shape[0]
             for c in range(n):
+                self._fill_states(states[c].numpy(), ids, c)
                 self.state.copy_(states[c], non_blocking=True)
                 runtime.launch_stages(self.stages if c == n - 1 else self._body, self.stream.cuda_stream, self.timeout_ns)
         runtime.read_status(self.stream.cuda_stream)
