@@ -10,8 +10,8 @@
 // 128256-row vocabulary projection at 3 rows).
 //
 // Measured against the megakernel's program, two Llama-3.1-8B-shaped layers and a small vocabulary (B200): 3 rows at
-// 1000 positions 416 -> 242 us, 32 rows with e4m3 weights 758 -> 324, 64 rows at 2100 positions 932 -> 436, 128 rows
-// 1025 -> 450, a 2048-token prompt 15.9 -> 6.5 ms.
+// 1000 positions 416 -> 244 us, 32 rows with e4m3 weights 759 -> 327, 64 rows at 2100 positions 929 -> 418, 128 rows
+// 1024 -> 396, a 2048-token prompt 15.9 -> 4.8 ms.
 #include "mk_umma.cuh"
 
 #include "../../include/vdcores.h"
