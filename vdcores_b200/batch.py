@@ -145,7 +145,8 @@ def emit_projection(P: Program, *, sms, load, w_addr, M, K, x_addr, B, Bpad, mod
 class BatchDecodeEngine(DecodeEngine):
     """`batch` sequences decoded together, one list of stage kernels per step.  Dense models; the layer
     projections are bf16, e4m3 with per-row scales (wkind "fp8") or NVFP4 (wkind "nvfp4": e2m1 values, e4m3 block
-    scales, fp32 tensor scale), everything else bf16."""
+    scales, fp32 tensor scale), everything else bf16.  num_sms sizes the K-splits of the projections and the page shares of
+    the attention; the stages' CTAs are not pinned to SMs."""
     GEMV_PROJECTIONS = False
     SHARED_CACHE = False     # True: the batch rows are consecutive positions of ONE sequence (prefill.PrefillEngine)
 
