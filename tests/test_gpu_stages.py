@@ -204,6 +204,48 @@ def test_attention(cuda_device, kind, G, n_kv, B, splits, lens):
     assert float(got[B:].abs().max() if B < Bp else 0) == 0
 
 
+@pytest.mark.parametrize("fmt", ["bf16", "fp8", "nvfp4"])
+def test_a_budget_of_one_nanosecond_ends_every_wait(cuda_device, fmt):
+    """Waits that may give up at their first look at the clock: the launch ends, either with the right result (nothing had
+    to wait that long) or with the timeout in the status block; the context stays usable and the next launch is right."""
+    from vdcores_b200 import isa, runtime
+    dev, B, K, M, G, n_kv, n_tab = cuda_device, 40, 4096, 4096, 4, 2, 16
+    x = seeded((B, K), 1)
+    w, sc, _ = weights(M, K, fmt, dev)
+    xd = packed_rows(x, dev)
+    pools = [torch.randn(B * n_tab, n_kv, 64, 128, device=dev).to(BF16) for _ in range(2)]
+    state = torch.zeros(B, isa.ST_PAGETABLE + n_tab, dtype=torch.int32)
+    state[:, isa.ST_POS] = 64 * n_tab - 1
+    state[:, isa.ST_PAGETABLE:] = torch.arange(B * n_tab).view(B, n_tab)
+    sd, q = state.to(dev), seeded((B, n_kv * G, 128), 10, 2.0).to(dev)
+    stream = torch.cuda.current_stream(dev).cuda_stream
+
+    def both(timeout_ns):
+        act = torch.zeros(bpad(B) * M // 2, dtype=BF16, device=dev)
+        out = torch.zeros(bpad(B) * n_kv * G * 128, dtype=BF16, device=dev)
+        stages = [gemm(dev, fmt, B, M, K, 2, w, sc, xd, mode=isa.STAGE_SILU, out=act.data_ptr()),
+                  runtime.Stage(kind=isa.STAGE_ATTN, B=B, Bpad=bpad(B), splits=2, group=G, n_kv=n_kv, n_pages=n_tab,
+                                state_stride=state.shape[1], state=sd.data_ptr(), q=q.data_ptr(), out=out.data_ptr(),
+                                kpool=pools[0].data_ptr(), vpool=pools[1].data_ptr())]
+        for s in stages:
+            runtime.launch_stages((runtime.Stage * 1)(s), stream, timeout_ns)
+        try:
+            runtime.read_status(stream)
+            ok = True
+        except runtime.VdcError as e:
+            assert e.code == 1 and e.status["opcode"] in (isa.STAGE_GEMM, isa.STAGE_ATTN)
+            ok = False
+        return ok, act, out
+
+    ok, act, out = both(500_000_000)
+    assert ok
+    for _ in range(20):
+        ok, a, o = both(1)
+        assert not ok or (torch.equal(a, act) and torch.equal(o, out))
+    ok, a, o = both(500_000_000)
+    assert ok and torch.equal(a, act) and torch.equal(o, out)
+
+
 def test_stages_refuse_bad_arguments(cuda_device):
     from vdcores_b200 import isa, runtime
     good = dict(kind=isa.STAGE_GEMM, mode=isa.STAGE_SILU, B=2, Bpad=16, M=64, K=128, splits=1, w=1 << 20, x=1 << 20, out=1 << 20)

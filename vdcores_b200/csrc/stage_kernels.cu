@@ -96,6 +96,11 @@ struct Waiter {
   __device__ __forceinline__ bool operator()(uint64_t* bar, uint32_t parity, int role, int at) const {
     return mbar_try_wait(bar, parity) || stage_wait_slow(bar, parity, fail, status, timeout_ns, kind, role, at);
   }
+  // The same for a whole warp: all 32 lanes leave together and with one answer, true only if every lane saw the barrier.
+  // What follows such a wait (ldmatrix, mma, full-mask shuffles, one arrival for the warp) needs all lanes.
+  __device__ __forceinline__ bool warp_wait(uint64_t* bar, uint32_t parity, int role, int at) const {
+    return __all_sync(0xffffffffu, (*this)(bar, parity, role, at));
+  }
   // copies that may still be in flight after a wait was given up get a bounded time to land
   __device__ __forceinline__ void drain() const {
     if (*fail) {
@@ -322,8 +327,8 @@ __global__ void __launch_bounds__(kGemmThreads, 2) stage_gemm(const __grid_const
       const int team = kEpiThreads / teams, tt = t & (team - 1), row = t & 127;
       for (int i = t / team; i < n_ch; i += teams) {
         const int st = i % n_ring;
-        if (!wait(&sh.full[st], (uint32_t)(i / n_ring) & 1u, 2, i)) break;
-        if (i >= 2 && !wait(&sh.stg_empty[i & 1], (uint32_t)((i >> 1) - 1) & 1u, 2, i)) break;
+        if (!wait.warp_wait(&sh.full[st], (uint32_t)(i / n_ring) & 1u, 2, i)) break;
+        if (i >= 2 && !wait.warp_wait(&sh.stg_empty[i & 1], (uint32_t)((i >> 1) - 1) & 1u, 2, i)) break;
         uint8_t* dst = staging + (i & 1) * (kBlk * kKc * 2);
         const uint8_t* src = ring + st * stage_bytes + xbytes;
         if (row < N) {
@@ -381,14 +386,16 @@ __global__ void __launch_bounds__(kGemmThreads, 2) stage_gemm(const __grid_const
       for (int gi = half ? (ng + 1) / 2 : 0; gi < (half ? ng : (ng + 1) / 2); ++gi) {
         uint32_t r[16];
         tmem_ld16(tmem + ((uint32_t)(quarter * 32) << 16) + (uint32_t)(gi * 16), r);
-        if (b >= s.Bpad) continue;
-        const uint32_t at = tile_at(tile, rank, nb, gi * 4, b & (nb - 1)), step = (uint32_t)(nb + 1) * 16u;
-        const uint32_t to = splits > 1 ? peer_smem(at, (uint32_t)(b / nb)) : at;
+        if (b < s.Bpad) {
+          const uint32_t at = tile_at(tile, rank, nb, gi * 4, b & (nb - 1)), step = (uint32_t)(nb + 1) * 16u;
+          const uint32_t to = splits > 1 ? peer_smem(at, (uint32_t)(b / nb)) : at;
 #pragma unroll
-        for (int j = 0; j < 4; ++j) {
-          if (splits > 1) st_cluster4(to + j * step, r[4 * j], r[4 * j + 1], r[4 * j + 2], r[4 * j + 3]);
-          else st_shared4(to + j * step, r[4 * j], r[4 * j + 1], r[4 * j + 2], r[4 * j + 3]);
+          for (int j = 0; j < 4; ++j) {
+            if (splits > 1) st_cluster4(to + j * step, r[4 * j], r[4 * j + 1], r[4 * j + 2], r[4 * j + 3]);
+            else st_shared4(to + j * step, r[4 * j], r[4 * j + 1], r[4 * j + 2], r[4 * j + 3]);
+          }
         }
+        __syncwarp();      // at 16 rows half a warp has none: it comes back before the next load of all lanes
       }
     }
     tc_fence_before();
@@ -648,7 +655,7 @@ __global__ void __launch_bounds__(kAttnThreads, 2) stage_attn(const __grid_const
     const int pv = warp * 16 + lr + 8 * (mi >> 1), hv = mi & 1;      // of V (transposed): position, upper dim half
     for (int i = 0; i < count; ++i) {
       const int stg = i % kAttnRing;
-      if (!wait(&sh.full[stg], (uint32_t)(i / kAttnRing) & 1u, 1, i)) break;
+      if (!wait.warp_wait(&sh.full[stg], (uint32_t)(i / kAttnRing) & 1u, 1, i)) break;
       const uint32_t kb = ring_s + (uint32_t)(stg * 2 * kPageBytes), vb = kb + kPageBytes;
       const int valid = pos - (first + i) * VDC_KV_PAGE;             // last position that exists, within the page
       float c[4] = {0.f, 0.f, 0.f, 0.f}, c2[4] = {0.f, 0.f, 0.f, 0.f};
@@ -809,7 +816,7 @@ __global__ void __launch_bounds__(kAttnThreads, 2) stage_attn_prefill(const __gr
     const int lr = lane & 7, mi = lane >> 3;
     for (int i = 0; i < count; ++i) {
       const int stg = i % kAttnRing;
-      if (!wait(&sh.full[stg], (uint32_t)(i / kAttnRing) & 1u, 1, i)) break;
+      if (!wait.warp_wait(&sh.full[stg], (uint32_t)(i / kAttnRing) & 1u, 1, i)) break;
       const uint32_t kb = ring_s + (uint32_t)(stg * 2 * kPageBytes), vb = kb + kPageBytes;
       const int page0 = (first + i) * VDC_KV_PAGE;
       float c[8][4];
