@@ -318,6 +318,7 @@ __global__ void __launch_bounds__(kGemmThreads, 2) stage_gemm(const __grid_const
       }
       umma_commit(&sh.done);
       wait(&sh.done, 0u, 1, n_ch);
+      tc_fence_before();     // the warps that read the accumulators learn of their completion from this thread's next barrier
     }
   } else {
     const int t = tid - 64;
