@@ -204,6 +204,94 @@ def test_attention(cuda_device, kind, G, n_kv, B, splits, lens):
     assert float(got[B:].abs().max() if B < Bp else 0) == 0
 
 
+def _walk(dev, kind, B, n_kv, G, splits, pos, seed):
+    """One attention stage over random pages: (run() -> fresh output rows [B, heads, 128], the same in fp32)."""
+    from vdcores_b200 import isa, runtime
+    from vdcores_b200.batch import unpack_kc
+    from vdcores_b200.decode import kv_page_swizzle
+    g = torch.Generator(device=dev).manual_seed(seed)
+    rnd = lambda *s: torch.empty(*s, device=dev).normal_(generator=g).to(BF16)
+    n_tab, seqs, D = int(max(pos)) // 64 + 1, (B if kind == "decode" else 1), 128
+    tables = torch.randperm(seqs * n_tab, generator=torch.Generator().manual_seed(seed)).view(seqs, n_tab).expand(B, -1)
+    k, v, q = rnd(seqs * n_tab, n_kv, 64, D), rnd(seqs * n_tab, n_kv, 64, D), rnd(B, n_kv * G, D)
+    state = torch.zeros(B, isa.ST_PAGETABLE + n_tab, dtype=torch.int32)
+    state[:, isa.ST_POS] = torch.tensor(pos, dtype=torch.int32)
+    state[:, isa.ST_PAGETABLE:] = tables
+    kd, vd, sd = kv_page_swizzle(k), kv_page_swizzle(v), state.to(dev)
+
+    def once():
+        out = torch.full((bpad(B) * n_kv * G * D,), float("nan"), dtype=BF16, device=dev)
+        run(dev, runtime.Stage(kind=isa.STAGE_ATTN if kind == "decode" else isa.STAGE_ATTN_PREFILL, B=B, Bpad=bpad(B),
+                               splits=splits, group=G, n_kv=n_kv, n_pages=n_tab, state_stride=state.shape[1],
+                               state=sd.data_ptr(), q=q.data_ptr(), out=out.data_ptr(), kpool=kd.data_ptr(),
+                               vpool=vd.data_ptr()))
+        return unpack_kc(out, bpad(B), n_kv * G * D)[:B].view(B, n_kv * G, D)
+
+    ref = torch.empty(B, n_kv, G, D, device=dev)
+    for b in range(B):
+        T, rows = int(pos[b]) + 1, tables[b].to(dev)
+        kk, vv = (t[rows].transpose(0, 1).reshape(n_kv, -1, D)[:, :T].float() for t in (k, v))
+        ref[b] = torch.softmax(q[b].view(n_kv, G, D).float() @ kk.transpose(1, 2) / math.sqrt(D), -1) @ vv
+    return once, ref.view(B, n_kv * G, D)
+
+
+@pytest.mark.parametrize("kind,B,n_kv,G,splits,lo,hi", [
+    ("decode", 128, 8, 4, 1, 351, 700), ("decode", 64, 8, 4, 1, 1051, 2100), ("decode", 24, 4, 8, 1, 2050, 2300),
+    ("decode", 32, 8, 4, 2, 751, 1500), ("prefill", 128, 8, 4, 1, 1037, 1164), ("prefill", 40, 2, 8, 2, 2100, 2139)])
+def test_long_walks_give_the_same_bits_every_time(cuda_device, kind, B, n_kv, G, splits, lo, hi):
+    """Up to 36 pages per CTA (the ring many times over, a second read of the page ids), more units than fit the GPU at
+    once, with one CTA per unit and with several: the sums are ordered, so that every head of every row has the same bits
+    in every pass, and each is the fp32 softmax's within the bound of the attention."""
+    dev = cuda_device
+    pos = list(range(lo, lo + B)) if kind == "prefill" else [hi - (b * 37) % (hi - lo + 1) for b in range(B)]
+    once, ref = _walk(dev, kind, B, n_kv, G, splits, pos, seed=B + G)
+    first = once()
+    err = (first.float() - ref).norm(dim=2) / ref.norm(dim=2)
+    assert float(err.max()) < 2 * REL, f"(row, head) {divmod(int(err.argmax()), n_kv * G)}"
+    for i in range(150):
+        differs = (once() != first).any(2).nonzero()
+        assert not len(differs), f"pass {i}: (row, head) {differs[:8].tolist()}"
+
+
+@pytest.mark.parametrize("batch,ctx", [(128, 700), (64, 2100)])
+def test_every_step_of_a_large_batch_has_the_same_bits(cuda_device, batch, ctx):
+    """One layer, one step from the same state again and again: queries, appended cache rows and attention outputs depend on
+    ordered sums only and repeat bit for bit; the hidden rows behind them repeat within the rounding of their statistics'
+    order."""
+    from vdcores_b200.batch import BatchDecodeEngine
+    from vdcores_b200.decode import DecodeConfig
+    cfg = DecodeConfig(hidden=1024, n_heads=32, n_kv_heads=8, ffn=2048, vocab=2048, n_layers=1)
+    eng = BatchDecodeEngine(cfg, batch, max_seq=ctx + 64, device=cuda_device, page_perm_seed=3)
+    eng.init_random_weights(1)
+    assert eng.attn_splits == 1
+    g = torch.Generator(device=cuda_device).manual_seed(2)
+    for t in (eng.kpool, eng.vpool):
+        t.normal_(generator=g)
+    for b in range(batch):
+        eng.set_state(ctx - (b * 37) % (ctx // 2), (b * 29) % cfg.vocab, b=b)
+    torch.cuda.synchronize()
+    state, pos, first = eng.state.clone(), eng.pos, None
+    k_rows, v_rows = (t.view(-1, 128) for t in (eng.kpool, eng.vpool))
+    from vdcores_b200 import isa
+    new = (state[:, isa.ST_NEWROW, None] + 64 * torch.arange(8, device=cuda_device)).long()     # [batch, kv heads]
+    for i in range(200):
+        for t in (k_rows, v_rows):
+            t[new] = 0
+        eng.q.zero_()
+        eng.attn_out.zero_()
+        eng.state.copy_(state)
+        eng.pos, eng.steps_done = pos, 0
+        eng.generate(1)
+        got = [eng.q.clone(), k_rows[new], v_rows[new], eng.attn_out.clone(), eng.read_hidden(eng.hidden).float()]
+        if first is None:
+            first = got
+            continue
+        for name, a, b in zip(("q", "k", "v", "attention"), got, first):
+            assert torch.equal(a, b), f"pass {i}: {name} differs at {(a != b).nonzero()[:8].tolist()}"
+        rows = (got[4] - first[4]).norm(dim=1) / first[4].norm(dim=1)
+        assert float(rows.max()) < 1e-2, f"pass {i}: hidden row {int(rows.argmax())}"
+
+
 @pytest.mark.parametrize("fmt", ["bf16", "fp8", "nvfp4"])
 def test_a_budget_of_one_nanosecond_ends_every_wait(cuda_device, fmt):
     """Waits that may give up at their first look at the clock: the launch ends, either with the right result (nothing had

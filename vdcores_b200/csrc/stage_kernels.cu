@@ -553,6 +553,16 @@ __device__ __forceinline__ void stream_pages(AttnShared& sh, const Waiter& wait,
   grid_dep_launch();
 }
 
+// A warp is done with a page.  Its loads (generic proxy) have to be complete before the next bulk copy (async proxy) may
+// write there: without the fence the last loads of V, dims 64 and up, could still be on their way when the warp had arrived,
+// and when page i + 3 then came in before page i + 1 they read it (a unit in some thousands, 5 % off in the step's hidden
+// row).  Fenced by every lane, since each has read for itself, then one arrival for the warp.
+__device__ __forceinline__ void page_consumed(uint64_t* empty, int lane) {
+  fence_proxy_async_smem();
+  __syncwarp();
+  if (lane == 0) mbar_arrive(empty);
+}
+
 __device__ __forceinline__ void attn_setup(AttnShared& sh, int tid) {
   if (tid == 0) {
     for (int i = 0; i < kAttnRing; ++i) {
@@ -700,8 +710,7 @@ __global__ void __launch_bounds__(kAttnThreads, 2) stage_attn(const __grid_const
         for (int j = 0; j < 4; ++j) o[d][j] *= al[j & 1];
         mma_16816(o[d], a[0], a[1], a[2], a[3], b0, b1);
       }
-      __syncwarp();
-      if (lane == 0) mbar_arrive(&sh.empty[stg]);
+      page_consumed(&sh.empty[stg], lane);
     }
 #pragma unroll
     for (int x = 4; x < 32; x <<= 1) {
@@ -881,8 +890,7 @@ __global__ void __launch_bounds__(kAttnThreads, 2) stage_attn_prefill(const __gr
           mma_16816(o[d + 1], p[2 * k][0], p[2 * k][1], p[2 * k + 1][0], p[2 * k + 1][1], a[2], a[3]);
         }
       }
-      __syncwarp();
-      if (lane == 0) mbar_arrive(&sh.empty[stg]);
+      page_consumed(&sh.empty[stg], lane);
     }
   }
   __syncthreads();
