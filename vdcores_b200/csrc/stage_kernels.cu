@@ -678,6 +678,12 @@ __global__ void __launch_bounds__(kAttnThreads, 2) stage_attn(const __grid_const
         mma_16816(c, a[0], a[1], a[2], a[3], q[k][0], q[k][1]);
         mma_16816(c2, a2[0], a2[1], a2[2], a2[3], q[k + 1][0], q[k + 1][1]);
       }
+      // V goes to registers before the softmax, which hides the loads, and the page's place is free that much sooner
+      const uint32_t vrow = pv <= valid ? vb + (uint32_t)(pv * 256) : zero;
+      uint32_t va[8][4];
+#pragma unroll
+      for (int d = 0; d < 8; ++d) ldsm_x4_trans(va[d], vrow + (uint32_t)(((2 * d + hv) ^ lr) << 4));
+      page_consumed(&sh.empty[stg], lane);
       const int p0 = warp * 16 + gid;
       float e[4];
 #pragma unroll
@@ -701,16 +707,12 @@ __global__ void __launch_bounds__(kAttnThreads, 2) stage_attn(const __grid_const
       }
       // probabilities enter P V rounded to bf16, as a bf16 attention module hands them over
       const uint32_t b0 = transpose8x8(pack_bf16x2(e[0], e[1])), b1 = transpose8x8(pack_bf16x2(e[2], e[3]));
-      const uint32_t vrow = pv <= valid ? vb + (uint32_t)(pv * 256) : zero;
 #pragma unroll
       for (int d = 0; d < 8; ++d) {
-        uint32_t a[4];
-        ldsm_x4_trans(a, vrow + (uint32_t)(((2 * d + hv) ^ lr) << 4));
 #pragma unroll
         for (int j = 0; j < 4; ++j) o[d][j] *= al[j & 1];
-        mma_16816(o[d], a[0], a[1], a[2], a[3], b0, b1);
+        mma_16816(o[d], va[d][0], va[d][1], va[d][2], va[d][3], b0, b1);
       }
-      page_consumed(&sh.empty[stg], lane);
     }
 #pragma unroll
     for (int x = 4; x < 32; x <<= 1) {
