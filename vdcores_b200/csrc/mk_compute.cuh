@@ -1004,6 +1004,7 @@ VDC_TASK void task_attn_decode(Compute& q, const AttnArgs& a) {
 #pragma unroll
         for (int mi = 0; mi < 4; ++mi) mma_rows8(acc[4 * j + mi][0], acc[4 * j + mi][1], z0, z1, pa, pb, vr[mi], vs2[mi]);
       }
+      fence_proxy_async_smem();   // the pages' loads are complete before a bulk copy may take their slots
       __syncwarp();
       if (q.lane == 0) {
         // counters 0..3 serve the trips (the slot pool holds three trips, so a warp is at most two trips ahead
@@ -1079,7 +1080,9 @@ VDC_TASK void task_attn_decode(Compute& q, const AttnArgs& a) {
 #pragma unroll
       for (int mi = 0; mi < 4; ++mi) mma_rows8(acc[4 * j + mi][0], acc[4 * j + mi][1], z0, z1, pa, 0u, vr[mi], 0u);
     }
-    // ---- the warp is done with this page pair; the last of the eight gives the slots back
+    // ---- the warp is done with this page pair; the last of the eight gives the slots back.  Fenced first: V's loads are
+    // complete before a bulk copy may take the slots
+    fence_proxy_async_smem();
     __syncwarp();
     if (q.lane == 0) {
       const int di = kTwo ? 4 : (blk & 7);

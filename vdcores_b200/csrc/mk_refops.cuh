@@ -421,6 +421,7 @@ VDC_TASK void task_ref_attn_decode(Compute& q, int num_kv_blocks, int last_len, 
 #pragma unroll
       for (int mi = 0; mi < 4; ++mi) mma_rows8(acc[4 * j + mi][0], acc[4 * j + mi][1], z0, z1, pa, 0u, vr[mi], 0u);
     }
+    fence_proxy_async_smem();   // the tiles' loads are complete before a bulk copy may take their slots
     compute_sync();  // every warp is done with the block's tiles
     q.free_slots(k_mask | v_mask);
   }
