@@ -82,12 +82,14 @@ int vdc_launch_async_full(int num_sms, int insts_per_sm, const void* compute_ins
  *   kind VDC_STAGE_ATTN_PREFILL: the same for rows that are consecutive positions of ONE sequence
  *     (both read the state blocks, and pages without a new row, while the stage directly in front still runs: that stage
  *     may write the new cache rows and the queries, nothing else of these)
- *   kind VDC_STAGE_EMBED: embedding rows (table `w`, width K) to hid, stats_out[0] = squares, the other n_stats - 1 rows
- *     of stats_out zeroed
+ *   kind VDC_STAGE_EMBED: embedding rows (table `w`, M rows of width K; M 0: their number is not checked) to hid,
+ *     stats_out[0] = squares, the other n_stats - 1 rows of stats_out zeroed
  *   kind VDC_STAGE_NORM: out = the rows x [Bpad, K], RMS-normalised with their sums of squares stats_in and the weights
  *     norm_w
  *   kind VDC_STAGE_ADVANCE: keys -> next tokens, token log, state blocks moved on by one position
- *   kind VDC_STAGE_COPY: M bytes from x to out
+ *   kind VDC_STAGE_COPY: M * K bytes from x to out
+ * A token id outside the table, and a row without a key (none of its logits is a number), are reported as VDC_ERR_TOKEN and
+ * id 0 is taken.  While an error is unread, EMBED, GEMM and ADVANCE stages write nothing.
  * Pointers are device addresses; 0 where a stage has no use for one. */
 typedef struct {
   int32_t kind, mode, wfmt, B, Bpad, M, K, splits;

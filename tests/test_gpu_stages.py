@@ -334,6 +334,77 @@ def test_a_budget_of_one_nanosecond_ends_every_wait(cuda_device, fmt):
     assert ok and torch.equal(a, act) and torch.equal(o, out)
 
 
+def test_a_row_without_a_token_is_reported_and_nothing_runs_on(cuda_device):
+    """A key of 0 (no number among the logits) at the advance, ids outside the table at the embedding: an error in the status
+    block, a valid id in the state; stages behind an unread error leave hidden rows, keys and states as they were."""
+    from vdcores_b200 import isa, runtime
+    from vdcores_b200.batch import unpack_kc
+    dev, B, H, V = cuda_device, 3, 256, 32
+    stream = torch.cuda.current_stream(dev).cuda_stream
+    state = torch.zeros(B, isa.ST_PAGETABLE + 2, dtype=torch.int32, device=dev)
+    state[:, isa.ST_POS], state[:, isa.ST_MAXPAGES], state[:, isa.ST_NKVH] = 5, 2, 1
+    log = torch.full((B, 4), -9, dtype=torch.int32, device=dev)
+    keys = torch.tensor([(1 << 40) | (0xFFFFFFFF - 7), 0, (1 << 40) | (0xFFFFFFFF - 9)], device=dev)
+    advance = runtime.Stage(kind=isa.STAGE_ADVANCE, B=B, Bpad=16, keys=keys.data_ptr(), log=log.data_ptr(), log_stride=4,
+                            state=state.data_ptr(), state_stride=state.shape[1])
+    table = seeded((V, H), 1).to(dev)
+    hid, stats = torch.zeros(16 * H, dtype=BF16, device=dev), torch.zeros(128, device=dev)
+    embed = runtime.Stage(kind=isa.STAGE_EMBED, B=B, Bpad=16, M=V, K=H, w=table.data_ptr(), hid=hid.data_ptr(),
+                          stats_out=stats.data_ptr(), n_stats=1, state=state.data_ptr(), state_stride=state.shape[1])
+    w, sc, _ = weights(H, H, "bf16", dev)
+    xd = packed_rows(seeded((B, H), 2), dev)
+    add = gemm(dev, "bf16", B, H, H, 2, w, sc, xd, mode=isa.STAGE_RESID, hid=hid.data_ptr(), stats_out=stats.data_ptr())
+
+    def launch(*stages):
+        runtime.launch_stages((runtime.Stage * len(stages))(*stages), stream, 500_000_000)
+
+    launch(advance)
+    kept = state.clone(), log.clone(), keys.clone(), hid.clone(), stats.clone()
+    launch(embed, add, advance)
+    with pytest.raises(runtime.VdcError) as e:
+        runtime.read_status(stream)
+    assert e.value.code == 5 and e.value.status["pc"] == 1 and e.value.status["opcode"] == isa.STAGE_ADVANCE
+    assert all(torch.equal(a, b) for a, b in zip(kept, (state, log, keys, hid, stats)))
+    assert state[:, isa.ST_TOKEN].tolist() == [7, 0, 9] and state[:, isa.ST_ERR].tolist() == [0, 1, 0]
+    assert log[:, 0].tolist() == [7, 0, 9] and state[:, isa.ST_POS].tolist() == [6, 6, 6] and not keys.any()
+    for bad in (-1, V, 2 ** 31 - 1, -2 ** 31):
+        state[1, isa.ST_TOKEN] = bad
+        launch(embed)
+        with pytest.raises(runtime.VdcError) as e:
+            runtime.read_status(stream)
+        assert e.value.code == 5 and e.value.status["aux"] == bad
+        assert torch.equal(unpack_kc(hid, 16, H)[1], table[0])
+    state[1, isa.ST_TOKEN] = V - 1
+    run(dev, embed)
+    assert torch.equal(unpack_kc(hid, 16, H)[:B], table[[7, V - 1, 9]])
+
+
+def test_logits_without_a_number_end_a_generation_with_an_error(cuda_device):
+    """Weights with a NaN: the steps already enqueued behind the first one stop at it, and the engine can be used again."""
+    from vdcores_b200 import isa, runtime
+    from vdcores_b200.batch import BatchDecodeEngine
+    from vdcores_b200.decode import DecodeConfig
+    cfg = DecodeConfig(hidden=512, n_heads=8, n_kv_heads=2, ffn=1024, vocab=256, n_layers=1)
+    eng = BatchDecodeEngine(cfg, 3, max_seq=128, device=cuda_device)
+    eng.init_random_weights(1)
+
+    def start():
+        for b in range(3):
+            eng.set_state(4, 10 + b, b=b)
+        torch.cuda.synchronize()
+    start()
+    good = eng.generate(4)
+    eng.norm_w.fill_(float("nan"))
+    start()
+    with pytest.raises(runtime.VdcError) as e:
+        eng.generate(4)
+    assert e.value.code == 5
+    assert eng.state[:, isa.ST_POS].tolist() == [5, 5, 5] and eng.state[:, isa.ST_TOKEN].tolist() == [0, 0, 0]
+    eng.norm_w.fill_(1.0)
+    start()
+    assert eng.generate(4) == good
+
+
 def test_stages_refuse_bad_arguments(cuda_device):
     from vdcores_b200 import isa, runtime
     good = dict(kind=isa.STAGE_GEMM, mode=isa.STAGE_SILU, B=2, Bpad=16, M=64, K=128, splits=1, w=1 << 20, x=1 << 20, out=1 << 20)

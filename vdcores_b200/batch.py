@@ -252,7 +252,7 @@ class BatchDecodeEngine(DecodeEngine):
         stat = lambda i: self.stats[i].data_ptr()
         state = dict(state=self.state.data_ptr(), state_stride=self.state_words)
         heads = dict(group=G, n_kv=cfg.n_kv_heads, **state)
-        out = [runtime.Stage(kind=isa.STAGE_EMBED, B=B, Bpad=self.bpad, K=cfg.hidden, w=self.embed.data_ptr(), hid=hid,
+        out = [runtime.Stage(kind=isa.STAGE_EMBED, B=B, Bpad=self.bpad, M=cfg.vocab, K=cfg.hidden, w=self.embed.data_ptr(), hid=hid,
                              stats_out=stat(0), n_stats=2 * L + 1, **state)]
         tile = 64 // G      # rows of one prefill attention unit
         units = cfg.n_kv_heads * (-(-B // tile) if self.SHARED_CACHE else B)

@@ -205,8 +205,12 @@ int vdc_read_status(uint64_t stream, vdc_status* status, int clear) {
   if (status) *status = h;
   if (h.abort) {
     char buf[256];
-    snprintf(buf, sizeof buf, "megakernel gave up: code=%d sm=%d role=%d pc=%d opcode=0x%x bar=%d aux=%d", h.code, h.sm,
-             h.role, h.pc, h.opcode, h.bar, h.aux);
+    if (h.code == VDC_ERR_TOKEN)
+      snprintf(buf, sizeof buf, "row %d: %s (%d)", h.pc, h.opcode == VDC_STAGE_EMBED ? "token id outside the vocabulary"
+               : "no number among its logits, no next token", h.aux);
+    else
+      snprintf(buf, sizeof buf, "megakernel gave up: code=%d sm=%d role=%d pc=%d opcode=0x%x bar=%d aux=%d", h.code, h.sm,
+               h.role, h.pc, h.opcode, h.bar, h.aux);
     g_err = buf;
     return h.code ? h.code : VDC_ERR_TIMEOUT;
   }
@@ -564,8 +568,12 @@ int vdc_launch_static(int num_sms, int insts_per_sm, const void* compute_insts, 
   if (status) *status = h;
   if (h.abort) {
     char buf[256];
-    snprintf(buf, sizeof buf, "megakernel gave up: code=%d sm=%d role=%d pc=%d opcode=0x%x bar=%d aux=%d", h.code, h.sm,
-             h.role, h.pc, h.opcode, h.bar, h.aux);
+    if (h.code == VDC_ERR_TOKEN)
+      snprintf(buf, sizeof buf, "row %d: %s (%d)", h.pc, h.opcode == VDC_STAGE_EMBED ? "token id outside the vocabulary"
+               : "no number among its logits, no next token", h.aux);
+    else
+      snprintf(buf, sizeof buf, "megakernel gave up: code=%d sm=%d role=%d pc=%d opcode=0x%x bar=%d aux=%d", h.code, h.sm,
+               h.role, h.pc, h.opcode, h.bar, h.aux);
     g_err = buf;
     return h.code ? h.code : VDC_ERR_TIMEOUT;
   }

@@ -300,9 +300,10 @@
 #define VDC_ERR_BAD_OPCODE 2
 #define VDC_ERR_CUDA 3
 #define VDC_ERR_ARG 4
+#define VDC_ERR_TOKEN 5   // a row without a next token (no number among its logits), or a token id outside the vocabulary
 
 typedef struct vdc_status {
-  int32_t abort;    // non-zero once any wait gave up; every other wait then returns
+  int32_t abort;    // non-zero once any wait gave up (every other wait then returns) or a token was refused
   int32_t code;     // VDC_ERR_*
   int32_t sm;       // CTA that raised it
   int32_t role;     // 0 compute, 1 control warp, 2 store warp, 3/4 load port 0/1

@@ -62,6 +62,20 @@ __device__ __forceinline__ float ld_cluster1(uint32_t a) {
   return v;
 }
 
+// The first error since the host last looked goes to the status block.
+static __device__ void report(vdc_status* status, int code, int kind, int role, int at, int aux) {
+  if (atomicCAS(&status->abort, 0, 1) == 0) {
+    status->code = code;
+    status->sm = (int)blockIdx.x;
+    status->role = role;
+    status->pc = at;
+    status->opcode = kind;
+    status->bar = -1;
+    status->aux = aux;
+    __threadfence();
+  }
+}
+
 // Bounded wait on an mbarrier of this CTA: after `timeout_ns` the status block says so, the CTA's `fail` word stops
 // every other role, and all of them leave through the ordinary exit (cluster barriers and tensor memory included).
 __device__ __noinline__ bool stage_wait_slow(uint64_t* bar, uint32_t parity, volatile int* fail, vdc_status* status,
@@ -72,16 +86,7 @@ __device__ __noinline__ bool stage_wait_slow(uint64_t* bar, uint32_t parity, vol
     if ((it & 15u) != 0) continue;
     if (*fail) return false;
     if (globaltimer_ns() - t0 > timeout_ns) {
-      if (atomicCAS(&status->abort, 0, 1) == 0) {
-        status->code = VDC_ERR_TIMEOUT;
-        status->sm = (int)blockIdx.x;
-        status->role = role;
-        status->pc = at;
-        status->opcode = kind;
-        status->bar = -1;
-        status->aux = (int)it;
-        __threadfence();
-      }
+      report(status, VDC_ERR_TIMEOUT, kind, role, at, (int)it);
       *fail = 1;
       return false;
     }
@@ -120,6 +125,7 @@ struct GemmShared {
   uint64_t done;
   uint32_t tmem;
   volatile int fail;
+  int skip;                     // an earlier stage failed: what this one computes is not written
   float ssq[128];
   unsigned long long key[128];
 };
@@ -285,12 +291,14 @@ __global__ void __launch_bounds__(kGemmThreads, 2) stage_gemm(const __grid_const
       grid_dep_wait();
       fence_proxy_async();
       for (int i = 0; i < first; ++i) bulk_load_1d(ring + i * stage_bytes, x + (size_t)i * xbytes, (uint32_t)xbytes, &sh.full[i]);
+      const int aborted = ld_relaxed_gpu(&status->abort);    // looked at below, when it has long arrived
       for (int i = first; i < n_ch; ++i) {
         const int st = i % n_ring;
         if (!wait(&sh.empty[st], (uint32_t)(i / n_ring - 1) & 1u, 0, i)) break;
         load_weights(i, st);
         bulk_load_1d(ring + st * stage_bytes, x + (size_t)i * xbytes, (uint32_t)xbytes, &sh.full[st]);
       }
+      sh.skip = aborted;
       grid_dep_launch();     // not earlier: waiting CTAs of the stages behind would hold the shared memory of this one's
     }
   } else if (warp == 1) {
@@ -377,7 +385,7 @@ __global__ void __launch_bounds__(kGemmThreads, 2) stage_gemm(const __grid_const
     __syncthreads();
   }
   tc_fence_after();
-  const bool failed = sh.fail != 0;
+  const bool failed = sh.fail != 0 || sh.skip != 0;
   const uint32_t tile = smem_u32(ring);
   const int nb = s.Bpad / splits;                    // rows this CTA finishes: a power of two
   if (warp >= 2 && !failed) {
@@ -934,14 +942,22 @@ __global__ void __launch_bounds__(kAttnThreads, 2) stage_attn_prefill(const __gr
 // ------------------------------------------------------------------------- //
 // first and last kernel of a step
 // ------------------------------------------------------------------------- //
+// Behind an error that the host has not read yet a step writes nothing that outlives it: the embedding, the projections'
+// epilogues and the advance return, so that no state moves on past the failed step.
+
 // Embedding row of one sequence: the hidden state and its sum of squares; and zeros for the sums that the step's residual
-// adds accumulate.
-__global__ void __launch_bounds__(256) stage_embed(const __grid_constant__ vdc_stage s) {
+// adds accumulate.  An id outside the table (M rows, 0: only its sign is known) is reported and row 0 taken in its place.
+__global__ void __launch_bounds__(256) stage_embed(const __grid_constant__ vdc_stage s, vdc_status* status) {
   __shared__ float red[8];
   const int b = blockIdx.x, tid = threadIdx.x;
   grid_dep_wait();
   grid_dep_launch();
-  const int token = ld_relaxed_gpu(reinterpret_cast<const int*>(s.state) + (size_t)b * s.state_stride + VDC_ST_TOKEN);
+  int token = ld_relaxed_gpu(reinterpret_cast<const int*>(s.state) + (size_t)b * s.state_stride + VDC_ST_TOKEN);
+  if (__syncthreads_or(ld_relaxed_gpu(&status->abort))) return;
+  if (token < 0 || (s.M > 0 && token >= s.M)) {
+    if (tid == 0) report(status, VDC_ERR_TOKEN, s.kind, 0, b, token);
+    token = 0;
+  }
   const uint8_t* row = reinterpret_cast<const uint8_t*>(s.w) + (size_t)token * s.K * 2;
   float ssq = 0.f;
   for (int p = tid; p < s.K / 8; p += 256) {
@@ -986,17 +1002,20 @@ __global__ void __launch_bounds__(256) stage_norm(const __grid_constant__ vdc_st
   *reinterpret_cast<uint4*>(reinterpret_cast<uint8_t*>(s.out) + (size_t)p * 16) = make_uint4(o[0], o[1], o[2], o[3]);
 }
 
-// Next token, token log and state advance of every sequence.
-__global__ void __launch_bounds__(128) stage_advance(const __grid_constant__ vdc_stage s) {
+// Next token, token log and state advance of every sequence.  A row whose logits held no number has no key: that is
+// reported, its block marked, and id 0 stored.
+__global__ void __launch_bounds__(128) stage_advance(const __grid_constant__ vdc_stage s, vdc_status* status) {
   grid_dep_wait();
   grid_dep_launch();
   const int b = threadIdx.x;
-  if (b >= s.B) return;
-  int* state = reinterpret_cast<int*>(s.state) + (size_t)b * s.state_stride;
+  const bool live = b < s.B;
+  int* state = reinterpret_cast<int*>(s.state) + (size_t)(live ? b : 0) * s.state_stride;
   unsigned long long* keys = reinterpret_cast<unsigned long long*>(s.keys);
-  const int token = (int)(0xFFFFFFFFu - (uint32_t)(__ldcg(keys + b) & 0xFFFFFFFFull));
-  keys[b] = 0ull;
+  const unsigned long long key = live ? __ldcg(keys + b) : 0ull;
   const int step = state[VDC_ST_STEP], pos = state[VDC_ST_POS] + 1, page = pos / VDC_KV_PAGE;
+  if (__syncthreads_or(ld_relaxed_gpu(&status->abort)) || !live) return;
+  const int token = key != 0ull ? (int)(0xFFFFFFFFu - (uint32_t)(key & 0xFFFFFFFFull)) : 0;
+  keys[b] = 0ull;
   reinterpret_cast<int*>(s.log)[(size_t)b * s.log_stride + step] = token;
   state[VDC_ST_TOKEN] = token;
   state[VDC_ST_STEP] = step + 1;
@@ -1006,6 +1025,10 @@ __global__ void __launch_bounds__(128) stage_advance(const __grid_constant__ vdc
     state[VDC_ST_NEWROW] = state[VDC_ST_PAGETABLE + page] * VDC_KV_PAGE * state[VDC_ST_NKVH] + pos % VDC_KV_PAGE;
   else
     state[VDC_ST_ERR] = 1;   // out of KV pages: the host must not launch another step
+  if (key == 0ull) {
+    state[VDC_ST_ERR] = 1;
+    report(status, VDC_ERR_TOKEN, s.kind, 0, b, -1);
+  }
 }
 
 }  // namespace vdc
@@ -1067,11 +1090,11 @@ extern "C" cudaError_t vdc_stage_launch(const vdc_stage* s, vdc_status* status, 
     case VDC_STAGE_EMBED:
       cfg.gridDim = dim3((unsigned)s->B);
       cfg.blockDim = dim3(256);
-      return cudaLaunchKernelEx(&cfg, vdc::stage_embed, *s);
+      return cudaLaunchKernelEx(&cfg, vdc::stage_embed, *s, status);
     case VDC_STAGE_ADVANCE:
       cfg.gridDim = dim3(1);
       cfg.blockDim = dim3(128);
-      return cudaLaunchKernelEx(&cfg, vdc::stage_advance, *s);
+      return cudaLaunchKernelEx(&cfg, vdc::stage_advance, *s, status);
     default:
       return cudaErrorInvalidValue;
   }
