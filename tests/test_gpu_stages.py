@@ -108,11 +108,13 @@ def test_projection_gate_up_and_argmax(cuda_device, B, K, M, splits, fmt):
     yb = y.to(BF16).float()
     ref = torch.nn.functional.silu(yb[:, 0::2]) * yb[:, 1::2]
     assert rel(unpack_kc(out.cpu(), Bp, M // 2)[:B], ref) < 2 * REL
-    if fmt == "bf16":
-        run(dev, gemm(dev, fmt, B, M, K, splits, w, sc, xnd, mode=isa.STAGE_ARGMAX, keys=keys.data_ptr()))
-        rows = 0xFFFFFFFF - (keys.cpu() & 0xFFFFFFFF)
-        top = y.max(1).values
-        assert bool((y[torch.arange(B), rows] >= top - 2.0 ** -7 * top.abs()).all())
+    if sc is not None:      # rows whose scales differ by more than their logits: the winner is the scaled one
+        f = torch.where(torch.arange(M) % 3 == 0, 8.0, 1.0)
+        sc, y = (sc.cpu() * f).to(dev), y * f
+    run(dev, gemm(dev, fmt, B, M, K, splits, w, sc, xnd, mode=isa.STAGE_ARGMAX, keys=keys.data_ptr()))
+    rows = 0xFFFFFFFF - (keys.cpu() & 0xFFFFFFFF)
+    top = y.max(1).values
+    assert bool((y[torch.arange(B), rows] >= top - 2.0 ** -7 * top.abs()).all())
 
 
 @pytest.mark.parametrize("B,fmt", [(3, "bf16"), (16, "nvfp4"), (128, "bf16"), (128, "fp8"), (16, "fp8")])

@@ -468,6 +468,7 @@ __global__ void __launch_bounds__(kGemmThreads, 2) stage_gemm(const __grid_const
           for (int f = f0; f < N / 8; f += fstep) {
             float v[8];
             sum8(v, ring, splits, nb, bl, f * 8);
+            scale8(v, scales ? scales + n0 + f * 8 : nullptr);
 #pragma unroll
             for (int j = 0; j < 8; ++j) {
               const float l = bf16_round(v[j]);
