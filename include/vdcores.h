@@ -72,7 +72,8 @@ int vdc_launch_async_full(int num_sms, int insts_per_sm, const void* compute_ins
 /* One stage of a batched decode step or of a prefill chunk (2..128 rows), run as a kernel of its own.
  *   kind VDC_STAGE_GEMM: projection of the k-chunk-major rows `x` [Bpad, K] with the M x K weights `w` (blocks of
  *     VDC_STAGE_BLOCK rows; wfmt 0 bf16, 1 e4m3, 2 NVFP4, fp32 per-row `scales` for the last two); every block's K is
- *     shared by `splits` CTAs of one cluster.  `mode` says where the result goes:
+ *     shared by `splits` CTAs of one cluster.  `w` is read while the stage in front still runs (and while what the stream
+ *     holds in front of the list finishes): it has to be complete before that one starts.  `mode` says where the result goes:
  *       VDC_STAGE_QKV    heads: q/k norm (qk_norm, 0: none), rotation (`rope`), query rows to `out` [B, heads, 128], key
  *                        and value rows to the pages state.NEWROW names in kpool / vpool
  *       VDC_STAGE_RESID  hid += result; stats_out += squares of hid

@@ -408,9 +408,34 @@ def test_logits_without_a_number_end_a_generation_with_an_error(cuda_device):
 
 
 def test_stages_refuse_bad_arguments(cuda_device):
+    """Nothing is launched: the check of the whole list comes first."""
     from vdcores_b200 import isa, runtime
-    good = dict(kind=isa.STAGE_GEMM, mode=isa.STAGE_SILU, B=2, Bpad=16, M=64, K=128, splits=1, w=1 << 20, x=1 << 20, out=1 << 20)
-    for bad in (dict(K=96), dict(M=8), dict(splits=3), dict(splits=4), dict(Bpad=24), dict(B=17), dict(w=0), dict(x=8), dict(wfmt=1),
-                dict(kind=9), dict(mode=7)):
-        with pytest.raises(runtime.VdcError):
-            runtime.launch_stages((runtime.Stage * 1)(runtime.Stage(**{**good, **bad})))
+    a = 1 << 20         # aligned; never read
+    heads = dict(group=4, n_kv=1, state=a, state_stride=isa.ST_PAGETABLE + 3, kpool=a, vpool=a)
+    proj = dict(kind=isa.STAGE_GEMM, B=2, Bpad=16, K=128, splits=1, w=a, x=a)
+    kinds = [
+        (dict(proj, mode=isa.STAGE_SILU, M=64, out=a),
+         [dict(K=96), dict(M=8), dict(splits=3), dict(splits=4), dict(Bpad=24), dict(B=17), dict(w=0), dict(x=a + 8), dict(wfmt=1),
+          dict(kind=9), dict(mode=7), dict(out=a + 8), dict(wfmt=1, scales=a + 4)]),
+        (dict(proj, mode=isa.STAGE_RESID, M=64, hid=a, stats_out=a), [dict(hid=a + 8), dict(hid=0), dict(stats_out=a + 2)]),
+        (dict(proj, mode=isa.STAGE_ARGMAX, M=64, keys=a), [dict(keys=a + 4), dict(keys=0)]),
+        (dict(proj, mode=isa.STAGE_QKV, M=768, out=a, rope=a, **heads),
+         [dict(M=896), dict(out=a + 2), dict(rope=a + 4), dict(qk_norm=a + 2), dict(kpool=a + 8), dict(vpool=a + 8), dict(state=0),
+          dict(state=a + 2), dict(state_stride=4)]),
+        (dict(kind=isa.STAGE_ATTN, B=2, Bpad=16, splits=1, n_pages=3, q=a, out=a, **heads),
+         [dict(group=5), dict(q=a + 8), dict(out=a + 8), dict(kpool=0), dict(vpool=a + 8), dict(n_pages=0), dict(n_pages=4), dict(splits=16)]),
+        (dict(kind=isa.STAGE_ATTN_PREFILL, B=2, Bpad=16, splits=1, n_pages=3, q=a, out=a, **heads), [dict(n_pages=4), dict(group=2)]),
+        (dict(kind=isa.STAGE_EMBED, B=2, Bpad=16, M=8, K=64, w=a, hid=a, stats_out=a, n_stats=1, state=a, state_stride=64),
+         [dict(K=0), dict(K=60), dict(w=a + 8), dict(hid=a + 8), dict(n_stats=0), dict(M=-1), dict(state=0), dict(state_stride=1)]),
+        (dict(kind=isa.STAGE_NORM, B=2, Bpad=16, K=64, x=a, out=a, stats_in=a, norm_w=a),
+         [dict(K=0), dict(x=a + 8), dict(out=0), dict(norm_w=a + 2), dict(stats_in=a + 1)]),
+        (dict(kind=isa.STAGE_ADVANCE, B=2, Bpad=16, keys=a, log=a, state=a, state_stride=64),
+         [dict(keys=a + 4), dict(log=a + 2), dict(state=0), dict(state_stride=isa.ST_PAGETABLE)])]
+    refused = runtime.Stage(kind=9, B=1, Bpad=16)
+    for good, bads in kinds:
+        for bad in bads:
+            with pytest.raises(runtime.VdcError):
+                runtime.launch_stages((runtime.Stage * 1)(runtime.Stage(**{**good, **bad})))
+        # the good one passes its own check: what is refused is the stage behind it
+        with pytest.raises(runtime.VdcError, match="unknown kind|splits"):
+            runtime.launch_stages((runtime.Stage * 2)(runtime.Stage(**good), refused))

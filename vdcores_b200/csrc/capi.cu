@@ -139,23 +139,34 @@ int vdc_launch_async_full(int num_sms, int insts_per_sm, const void* compute_ins
                            timeout_ns, 1);
 }
 
+// Everything a stage's kernel takes for granted.  Alignments are those of its widest access: 16 bytes for rows, pages and
+// hidden or output pieces, 8 for the rotation table and the keys, 4 for the rest.
 static const char* check_stage(const vdc_stage& s) {
   auto pow2 = [](int v) { return v > 0 && (v & (v - 1)) == 0; };
   auto al16 = [](uint64_t p) { return (p & 15) == 0; };
+  auto al8 = [](uint64_t p) { return (p & 7) == 0; };
+  auto al4 = [](uint64_t p) { return (p & 3) == 0; };
   if (s.kind == VDC_STAGE_COPY) return s.x && s.out && s.M > 0 && s.K > 0 ? nullptr : "copy stage: null pointer or size";
   if (s.B < 1 || s.B > 128 || s.Bpad < s.B || (s.Bpad != 16 && s.Bpad != 32 && s.Bpad != 64 && s.Bpad != 128))
     return "stage: rows out of range";
+  // a row's state block: the words in front of its page table, and with `pages` the table too
+  auto state_ok = [&](int pages) {
+    return s.state && al4(s.state) && (s.B == 1 || s.state_stride >= VDC_ST_PAGETABLE + pages);
+  };
   if (s.kind == VDC_STAGE_EMBED)
-    return s.K % 8 == 0 && s.w && s.hid && s.state && s.stats_out ? nullptr : "embedding stage: bad argument";
+    return s.K > 0 && s.K % 8 == 0 && s.M >= 0 && s.n_stats >= 1 && s.w && s.hid && s.stats_out && al16(s.w) && al16(s.hid) &&
+                   al4(s.stats_out) && state_ok(0) ? nullptr : "embedding stage: bad argument";
   if (s.kind == VDC_STAGE_NORM)
-    return s.K > 0 && s.K % 8 == 0 && s.x && s.out && s.stats_in && s.norm_w && al16(s.x) && al16(s.out) && al16(s.norm_w)
-               ? nullptr : "norm stage: bad argument";
-  if (s.kind == VDC_STAGE_ADVANCE) return s.state && s.keys && s.log ? nullptr : "advance stage: null pointer";
+    return s.K > 0 && s.K % 8 == 0 && s.x && s.out && s.stats_in && s.norm_w && al16(s.x) && al16(s.out) && al16(s.norm_w) &&
+                   al4(s.stats_in) ? nullptr : "norm stage: bad argument";
+  if (s.kind == VDC_STAGE_ADVANCE)
+    return s.keys && s.log && al8(s.keys) && al4(s.log) && state_ok(1) ? nullptr : "advance stage: bad argument";
   if (!pow2(s.splits) || s.splits > 8) return "stage: splits must be 1, 2, 4 or 8";
   if (s.kind == VDC_STAGE_ATTN || s.kind == VDC_STAGE_ATTN_PREFILL) {
     if ((s.group != 4 && s.group != 8) || s.n_kv < 1 || s.n_kv > 65535 || s.n_pages < 1) return "attention stage: bad shape";
-    return s.state && s.q && s.out && s.kpool && s.vpool && al16(s.q) && al16(s.out) && al16(s.kpool) && al16(s.vpool)
-               ? nullptr : "attention stage: null or misaligned pointer";
+    // a prefill stage reads the page table of its first row only, but the row behind it has to lie beyond that
+    return state_ok(s.n_pages) && s.q && s.out && s.kpool && s.vpool && al16(s.q) && al16(s.out) && al16(s.kpool) &&
+                   al16(s.vpool) ? nullptr : "attention stage: bad state stride, null or misaligned pointer";
   }
   if (s.kind != VDC_STAGE_GEMM) return "stage: unknown kind";
   if (s.wfmt < 0 || s.wfmt > 2 || s.M < 16 || s.M % 16 || s.K < 64 || s.K % 64 || s.splits > s.K / 64)
@@ -165,10 +176,12 @@ static const char* check_stage(const vdc_stage& s) {
   switch (s.mode) {
     case VDC_STAGE_QKV:
       if (s.group < 1 || s.n_kv < 1 || s.M != s.n_kv * (s.group + 2) * VDC_HEAD_DIM) return "QKV stage: rows do not match the heads";
-      return s.out && s.state && s.rope && s.kpool && s.vpool ? nullptr : "QKV stage: null pointer";
-    case VDC_STAGE_RESID: return s.hid && s.stats_out ? nullptr : "residual stage: null pointer";
-    case VDC_STAGE_SILU: return s.out ? nullptr : "gate/up stage: null pointer";
-    case VDC_STAGE_ARGMAX: return s.keys ? nullptr : "argmax stage: null pointer";
+      return s.out && s.rope && s.kpool && s.vpool && state_ok(0) && al4(s.out) && al8(s.rope) && al4(s.qk_norm) &&
+                     al16(s.kpool) && al16(s.vpool) ? nullptr : "QKV stage: bad state stride, null or misaligned pointer";
+    case VDC_STAGE_RESID:
+      return s.hid && s.stats_out && al16(s.hid) && al4(s.stats_out) ? nullptr : "residual stage: null or misaligned pointer";
+    case VDC_STAGE_SILU: return s.out && al16(s.out) ? nullptr : "gate/up stage: null or misaligned pointer";
+    case VDC_STAGE_ARGMAX: return s.keys && al8(s.keys) ? nullptr : "argmax stage: null or misaligned pointer";
     default: return "projection stage: unknown mode";
   }
 }
