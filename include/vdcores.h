@@ -106,6 +106,15 @@ typedef struct {
  * vdc_read_status.  The stages are checked before anything is enqueued.  No counterpart in the reference. */
 int vdc_launch_stages(const vdc_stage* stages, int n, uint64_t stream, uint64_t timeout_ns);
 
+/* The same with at most max_ctas CTAs running at any time (0: no limit), so that no more than that many SMs are taken:
+ * a stage's grid goes in slices, and a launch starts before the one in front of it has ended only where both fit the limit.
+ * max_ctas must not be smaller than a stage's splits. */
+int vdc_launch_stages_limited(const vdc_stage* stages, int n, int max_ctas, uint64_t stream, uint64_t timeout_ns);
+
+/* Checks the stages as a launch does, needs no GPU: *launches = what vdc_launch_stages_limited enqueues (a copy counts as
+ * one), *largest = the most CTAs of one launch. */
+int vdc_count_stage_launches(const vdc_stage* stages, int n, int max_ctas, int* launches, int* largest);
+
 /* Synchronises `stream` and copies the device status block to *status; returns
  * its code.  Clears the block when `clear` is non-zero. */
 int vdc_read_status(uint64_t stream, vdc_status* status, int clear);

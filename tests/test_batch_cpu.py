@@ -1,6 +1,7 @@
 """Host-side logic of the batched (tensor-core) decode path, without a GPU: operand layouts,
 the dealing of projection work to SMs, and the memory streams the program builder emits
 (expanded here by a small interpreter of REPEAT loops)."""
+import pytest
 import torch
 
 from vdcores_b200 import isa
@@ -152,3 +153,56 @@ def test_prefill_state_blocks_of_a_chunk():
             assert s[b, isa.ST_NEWROW] == int(table[pos // 64]) * 64 * 2 + pos % 64
             assert s[b, isa.ST_NKVH] == 2 and s[b, isa.ST_MAXPAGES] == 5 and s[b, isa.ST_STEP] == 0 and s[b, isa.ST_ERR] == 0
             assert (s[b, isa.ST_PAGETABLE:] == table.numpy()).all()
+
+
+def test_stages_refuse_bad_arguments():
+    """The check that a launch runs over its whole list first; no GPU is needed for it."""
+    from vdcores_b200 import isa, runtime
+    a = 1 << 20         # aligned; never read
+    heads = dict(group=4, n_kv=1, state=a, state_stride=isa.ST_PAGETABLE + 3, kpool=a, vpool=a)
+    proj = dict(kind=isa.STAGE_GEMM, B=2, Bpad=16, K=128, splits=1, w=a, x=a)
+    kinds = [
+        (dict(proj, mode=isa.STAGE_SILU, M=64, out=a),
+         [dict(K=96), dict(M=8), dict(splits=3), dict(splits=4), dict(Bpad=24), dict(B=17), dict(w=0), dict(x=a + 8), dict(wfmt=1),
+          dict(kind=9), dict(mode=7), dict(out=a + 8), dict(wfmt=1, scales=a + 4)]),
+        (dict(proj, mode=isa.STAGE_RESID, M=64, hid=a, stats_out=a), [dict(hid=a + 8), dict(hid=0), dict(stats_out=a + 2)]),
+        (dict(proj, mode=isa.STAGE_ARGMAX, M=64, keys=a), [dict(keys=a + 4), dict(keys=0)]),
+        (dict(proj, mode=isa.STAGE_QKV, M=768, out=a, rope=a, **heads),
+         [dict(M=896), dict(out=a + 2), dict(rope=a + 4), dict(qk_norm=a + 2), dict(kpool=a + 8), dict(vpool=a + 8), dict(state=0),
+          dict(state=a + 2), dict(state_stride=4)]),
+        (dict(kind=isa.STAGE_ATTN, B=2, Bpad=16, splits=1, n_pages=3, q=a, out=a, **heads),
+         [dict(group=5), dict(q=a + 8), dict(out=a + 8), dict(kpool=0), dict(vpool=a + 8), dict(n_pages=0), dict(n_pages=4), dict(splits=16)]),
+        (dict(kind=isa.STAGE_ATTN_PREFILL, B=2, Bpad=16, splits=1, n_pages=3, q=a, out=a, **heads), [dict(n_pages=4), dict(group=2)]),
+        (dict(kind=isa.STAGE_EMBED, B=2, Bpad=16, M=8, K=64, w=a, hid=a, stats_out=a, n_stats=1, state=a, state_stride=64),
+         [dict(K=0), dict(K=60), dict(w=a + 8), dict(hid=a + 8), dict(n_stats=0), dict(M=-1), dict(state=0), dict(state_stride=1)]),
+        (dict(kind=isa.STAGE_NORM, B=2, Bpad=16, K=64, x=a, out=a, stats_in=a, norm_w=a),
+         [dict(K=0), dict(x=a + 8), dict(out=0), dict(norm_w=a + 2), dict(stats_in=a + 1)]),
+        (dict(kind=isa.STAGE_ADVANCE, B=2, Bpad=16, keys=a, log=a, state=a, state_stride=64),
+         [dict(keys=a + 4), dict(log=a + 2), dict(state=0), dict(state_stride=isa.ST_PAGETABLE)])]
+    for good, bads in kinds:
+        runtime.count_stage_launches((runtime.Stage * 1)(runtime.Stage(**good)))
+        for bad in bads:
+            with pytest.raises(runtime.VdcError):
+                runtime.count_stage_launches((runtime.Stage * 1)(runtime.Stage(**{**good, **bad})))
+
+
+@pytest.mark.parametrize("limit", [1, 7, 61, 147])
+def test_slices_of_a_limited_launch(limit):
+    """Whole clusters, never more than the limit, all units once: per kind the number of launches and the largest."""
+    from vdcores_b200 import isa, runtime
+    a = 1 << 20
+    common = dict(B=100, Bpad=128, w=a, x=a, out=a, hid=a, stats_out=a, stats_in=a, norm_w=a, keys=a, log=a, state=a, q=a, kpool=a,
+                  vpool=a, n_stats=1, state_stride=64, group=4, n_kv=8, n_pages=9, K=4096)
+    for kind, units, splits, more in ((isa.STAGE_GEMM, 113, 4, dict(M=14400, mode=isa.STAGE_SILU)),
+                                      (isa.STAGE_GEMM, 32, 1, dict(M=4096, mode=isa.STAGE_RESID)), (isa.STAGE_ATTN, 800, 1, {}),
+                                      (isa.STAGE_ATTN_PREFILL, 56, 2, {}), (isa.STAGE_NORM, 256, 1, {}), (isa.STAGE_EMBED, 100, 1, {}),
+                                      (isa.STAGE_ADVANCE, 1, 1, {})):
+        st = (runtime.Stage * 1)(runtime.Stage(kind=kind, splits=splits, **{**common, **more}))
+        assert runtime.count_stage_launches(st) == (1, units * splits)
+        if splits > limit:
+            with pytest.raises(runtime.VdcError, match="splits"):
+                runtime.count_stage_launches(st, limit)
+            continue
+        launches, largest = runtime.count_stage_launches(st, limit)
+        per = limit // splits
+        assert launches == -(-units // per) and largest == min(units, per) * splits <= limit

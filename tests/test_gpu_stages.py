@@ -294,6 +294,36 @@ def test_every_step_of_a_large_batch_has_the_same_bits(cuda_device, batch, ctx):
         assert float(rows.max()) < 1e-2, f"pass {i}: hidden row {int(rows.argmax())}"
 
 
+@pytest.mark.parametrize("num_sms", [1, 7, 61, 140])
+def test_a_step_and_a_prompt_on_fewer_sms(cuda_device, num_sms):
+    """num_sms below the device's count: slices of at most that many CTAs, and the results of the whole device."""
+    from vdcores_b200 import runtime
+    from vdcores_b200.batch import BatchDecodeEngine
+    from vdcores_b200.decode import DecodeConfig, DecodeEngine
+    from vdcores_b200.prefill import PrefillEngine
+    cfg = DecodeConfig(hidden=512, n_heads=8, n_kv_heads=2, ffn=1024, vocab=512, n_layers=2)
+    prompt = torch.randint(0, cfg.vocab, (100,), generator=torch.Generator().manual_seed(4))
+    got = {}
+    for n in (None, num_sms):
+        eng = BatchDecodeEngine(cfg, 20, max_seq=192, device=cuda_device, num_sms=n)
+        eng.init_random_weights(1)
+        g = torch.Generator(device=cuda_device).manual_seed(2)
+        for t in (eng.kpool, eng.vpool):
+            t.normal_(generator=g)
+        for b in range(20):
+            eng.set_state(150 - 7 * b, 10 + b, b=b)
+        torch.cuda.synchronize()
+        eng.generate(1)
+        dec = DecodeEngine(cfg, 192, device=cuda_device, num_sms=n)
+        dec.init_random_weights(1)
+        pre = PrefillEngine(dec, chunk=64).adopt_weights()
+        pre.prefill(prompt)
+        got[n] = eng.read_hidden(eng.hidden), pre.read_hidden(pre.hidden), dec.kpool[:, :2]
+        assert n is None or all(runtime.count_stage_launches(e.stages, e.max_ctas)[1] <= n for e in (eng, pre))
+    for a, b in zip(got[None], got[num_sms]):
+        assert rel(a, b) < 2e-2          # other K-splits: other orders of the sums, in bf16 through two layers
+
+
 @pytest.mark.parametrize("fmt", ["bf16", "fp8", "nvfp4"])
 def test_a_budget_of_one_nanosecond_ends_every_wait(cuda_device, fmt):
     """Waits that may give up at their first look at the clock: the launch ends, either with the right result (nothing had
@@ -405,37 +435,3 @@ def test_logits_without_a_number_end_a_generation_with_an_error(cuda_device):
     eng.norm_w.fill_(1.0)
     start()
     assert eng.generate(4) == good
-
-
-def test_stages_refuse_bad_arguments(cuda_device):
-    """Nothing is launched: the check of the whole list comes first."""
-    from vdcores_b200 import isa, runtime
-    a = 1 << 20         # aligned; never read
-    heads = dict(group=4, n_kv=1, state=a, state_stride=isa.ST_PAGETABLE + 3, kpool=a, vpool=a)
-    proj = dict(kind=isa.STAGE_GEMM, B=2, Bpad=16, K=128, splits=1, w=a, x=a)
-    kinds = [
-        (dict(proj, mode=isa.STAGE_SILU, M=64, out=a),
-         [dict(K=96), dict(M=8), dict(splits=3), dict(splits=4), dict(Bpad=24), dict(B=17), dict(w=0), dict(x=a + 8), dict(wfmt=1),
-          dict(kind=9), dict(mode=7), dict(out=a + 8), dict(wfmt=1, scales=a + 4)]),
-        (dict(proj, mode=isa.STAGE_RESID, M=64, hid=a, stats_out=a), [dict(hid=a + 8), dict(hid=0), dict(stats_out=a + 2)]),
-        (dict(proj, mode=isa.STAGE_ARGMAX, M=64, keys=a), [dict(keys=a + 4), dict(keys=0)]),
-        (dict(proj, mode=isa.STAGE_QKV, M=768, out=a, rope=a, **heads),
-         [dict(M=896), dict(out=a + 2), dict(rope=a + 4), dict(qk_norm=a + 2), dict(kpool=a + 8), dict(vpool=a + 8), dict(state=0),
-          dict(state=a + 2), dict(state_stride=4)]),
-        (dict(kind=isa.STAGE_ATTN, B=2, Bpad=16, splits=1, n_pages=3, q=a, out=a, **heads),
-         [dict(group=5), dict(q=a + 8), dict(out=a + 8), dict(kpool=0), dict(vpool=a + 8), dict(n_pages=0), dict(n_pages=4), dict(splits=16)]),
-        (dict(kind=isa.STAGE_ATTN_PREFILL, B=2, Bpad=16, splits=1, n_pages=3, q=a, out=a, **heads), [dict(n_pages=4), dict(group=2)]),
-        (dict(kind=isa.STAGE_EMBED, B=2, Bpad=16, M=8, K=64, w=a, hid=a, stats_out=a, n_stats=1, state=a, state_stride=64),
-         [dict(K=0), dict(K=60), dict(w=a + 8), dict(hid=a + 8), dict(n_stats=0), dict(M=-1), dict(state=0), dict(state_stride=1)]),
-        (dict(kind=isa.STAGE_NORM, B=2, Bpad=16, K=64, x=a, out=a, stats_in=a, norm_w=a),
-         [dict(K=0), dict(x=a + 8), dict(out=0), dict(norm_w=a + 2), dict(stats_in=a + 1)]),
-        (dict(kind=isa.STAGE_ADVANCE, B=2, Bpad=16, keys=a, log=a, state=a, state_stride=64),
-         [dict(keys=a + 4), dict(log=a + 2), dict(state=0), dict(state_stride=isa.ST_PAGETABLE)])]
-    refused = runtime.Stage(kind=9, B=1, Bpad=16)
-    for good, bads in kinds:
-        for bad in bads:
-            with pytest.raises(runtime.VdcError):
-                runtime.launch_stages((runtime.Stage * 1)(runtime.Stage(**{**good, **bad})))
-        # the good one passes its own check: what is refused is the stage behind it
-        with pytest.raises(runtime.VdcError, match="unknown kind|splits"):
-            runtime.launch_stages((runtime.Stage * 2)(runtime.Stage(**good), refused))

@@ -146,7 +146,8 @@ class BatchDecodeEngine(DecodeEngine):
     """`batch` sequences decoded together, one list of stage kernels per step.  Dense models; the layer
     projections are bf16, e4m3 with per-row scales (wkind "fp8") or NVFP4 (wkind "nvfp4": e2m1 values, e4m3 block
     scales, fp32 tensor scale), everything else bf16.  num_sms sizes the K-splits of the projections and the page shares of
-    the attention; the stages' CTAs are not pinned to SMs."""
+    the attention; below the device's count it also bounds the CTAs of a step that run at any time, and so the SMs it
+    takes."""
     GEMV_PROJECTIONS = False
     SHARED_CACHE = False     # True: the batch rows are consecutive positions of ONE sequence (prefill.PrefillEngine)
 
@@ -173,6 +174,7 @@ class BatchDecodeEngine(DecodeEngine):
         self.pages_per_split = (self.max_pages + self.n_splits - 1) // self.n_splits
         self.n_splits = (self.max_pages + self.pages_per_split - 1) // self.pages_per_split
         self.stages = None
+        self.max_ctas = self.num_sms if self.num_sms < torch.cuda.get_device_properties(self.dev).multi_processor_count else 0
         self.state_words = isa.ST_PAGETABLE + self.max_pages
         self.state = z(B, self.state_words, dt=torch.int32)
         self.state_host = torch.zeros(B, self.state_words, dtype=torch.int32).pin_memory()
@@ -222,8 +224,9 @@ class BatchDecodeEngine(DecodeEngine):
 
     # ------------------------------------------------------------------ program
     def _splits(self, units: int, per_sm: int, most: int) -> int:
-        """CTAs (one cluster) that share a unit: the largest power of two with at most per_sm CTAs for every SM."""
-        s = 1
+        """CTAs (one cluster) that share a unit: the largest power of two with at most per_sm CTAs for every SM (one where
+        no more CTAs than SMs may run at a time)."""
+        s, per_sm = 1, 1 if self.max_ctas else per_sm
         while s < 8 and units * s * 2 <= per_sm * self.num_sms and s * 2 <= most:
             s *= 2
         return s
@@ -286,7 +289,7 @@ class BatchDecodeEngine(DecodeEngine):
     def _build_program(self):
         self._pack_cache = getattr(self, "_pack_cache", None) or {}
         self.stages = self._plan()
-        self.launches_per_step = len(self.stages)
+        self.launches_per_step = runtime.count_stage_launches(self.stages, self.max_ctas)[0]
 
     # ------------------------------------------------------------------ state
     def set_state(self, pos: int, token: int, b: int = None):
@@ -354,7 +357,7 @@ class BatchDecodeEngine(DecodeEngine):
         assert self.stages is not None, "load weights first"
         if self.pos >= self.max_seq or self.steps_done >= self.max_steps:
             raise RuntimeError("out of KV pages or token-log space")
-        runtime.launch_stages(self.stages, self.stream.cuda_stream, self.timeout_ns)
+        runtime.launch_stages(self.stages, self.stream.cuda_stream, self.timeout_ns, self.max_ctas)
         self.pos += 1
         self.steps_done += 1
 

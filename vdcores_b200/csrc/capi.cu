@@ -17,7 +17,9 @@ extern "C" cudaError_t vdc_megakernel_launch(int num_sms, const void* cinsts, co
                                              uint64_t timeout_ns, cudaStream_t stream, int ref_ops);
 
 extern "C" cudaError_t vdc_stage_prepare();
-extern "C" cudaError_t vdc_stage_launch(const vdc_stage* s, vdc_status* status, uint64_t timeout_ns, cudaStream_t stream);
+extern "C" cudaError_t vdc_stage_launch(const vdc_stage* s, int max_ctas, int* front, vdc_status* status,
+                                        uint64_t timeout_ns, cudaStream_t stream);
+extern "C" void vdc_stage_slices(const vdc_stage* s, int max_ctas, int* launches, int* largest);
 
 namespace {
 
@@ -186,19 +188,46 @@ static const char* check_stage(const vdc_stage& s) {
   }
 }
 
-int vdc_launch_stages(const vdc_stage* stages, int n, uint64_t stream, uint64_t timeout_ns) {
+static const char* check_stages(const vdc_stage* stages, int n, int max_ctas) {
+  if (!stages || n < 1) return "no stages";
+  if (max_ctas < 0) return "the number of CTAs must not be negative";
+  for (int i = 0; i < n; ++i) {
+    if (const char* why = check_stage(stages[i])) return why;
+    const bool shared = stages[i].kind == VDC_STAGE_GEMM || stages[i].kind == VDC_STAGE_ATTN || stages[i].kind == VDC_STAGE_ATTN_PREFILL;
+    if (max_ctas && shared && stages[i].splits > max_ctas) return "stage: more splits than CTAs are allowed";
+  }
+  return nullptr;
+}
+
+int vdc_launch_stages_limited(const vdc_stage* stages, int n, int max_ctas, uint64_t stream, uint64_t timeout_ns) {
   int dev;
   if (int r = current_device(&dev)) return r;
   if (!g_status[dev]) return fail_arg("vdc_init was not called on this device");
-  if (!stages || n < 1) return fail_arg("no stages");
-  for (int i = 0; i < n; ++i)
-    if (const char* why = check_stage(stages[i])) return fail_arg(why);
+  if (const char* why = check_stages(stages, n, max_ctas)) return fail_arg(why);
   if (timeout_ns == 0) timeout_ns = 2000000000ull;
+  int front = -1;      // CTAs of the launch in front of the next one
   for (int i = 0; i < n; ++i) {
-    cudaError_t e = vdc_stage_launch(&stages[i], g_status[dev], timeout_ns, reinterpret_cast<cudaStream_t>(stream));
+    cudaError_t e = vdc_stage_launch(&stages[i], max_ctas, &front, g_status[dev], timeout_ns, reinterpret_cast<cudaStream_t>(stream));
     if (e != cudaSuccess) return fail_cuda(e, "stage launch");
   }
   return VDC_OK;
+}
+
+int vdc_count_stage_launches(const vdc_stage* stages, int n, int max_ctas, int* launches, int* largest) {
+  if (!launches || !largest) return fail_arg("null argument");
+  if (const char* why = check_stages(stages, n, max_ctas)) return fail_arg(why);
+  *launches = *largest = 0;
+  for (int i = 0; i < n; ++i) {
+    int k, c;
+    vdc_stage_slices(&stages[i], max_ctas, &k, &c);
+    *launches += k;
+    if (c > *largest) *largest = c;
+  }
+  return VDC_OK;
+}
+
+int vdc_launch_stages(const vdc_stage* stages, int n, uint64_t stream, uint64_t timeout_ns) {
+  return vdc_launch_stages_limited(stages, n, 0, stream, timeout_ns);
 }
 
 int vdc_read_status(uint64_t stream, vdc_status* status, int clear) {

@@ -233,14 +233,14 @@ __device__ __forceinline__ void qkv_head(const vdc_stage& s, const uint8_t* tile
 }
 
 template <int kFmt>
-__global__ void __launch_bounds__(kGemmThreads, 2) stage_gemm(const __grid_constant__ vdc_stage s, int n_ring,
+__global__ void __launch_bounds__(kGemmThreads, 2) stage_gemm(const __grid_constant__ vdc_stage s, int first_block, int n_ring,
                                                               vdc_status* status, uint64_t timeout_ns) {
   extern __shared__ uint8_t dyn[];
   __shared__ GemmShared sh;
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int splits = s.splits;
   const int rank = splits > 1 ? (int)cluster_rank() : 0;
-  const int block = (int)blockIdx.x / splits;
+  const int block = first_block + (int)blockIdx.x / splits;
   const int n0 = block * kBlk, N = min(kBlk, s.M - n0);
   const int chunks = s.K / kKc, c0 = chunks * rank / splits, n_ch = chunks * (rank + 1) / splits - c0;
   const int xbytes = s.Bpad * kKc * 2, wbytes = chunk_bytes(kFmt, N);
@@ -629,14 +629,14 @@ __device__ __forceinline__ void attn_merge(AttnShared& sh, uint32_t tile, int sp
   }
 }
 
-__global__ void __launch_bounds__(kAttnThreads, 2) stage_attn(const __grid_constant__ vdc_stage s, vdc_status* status,
+__global__ void __launch_bounds__(kAttnThreads, 2) stage_attn(const __grid_constant__ vdc_stage s, int first_unit, vdc_status* status,
                                                               uint64_t timeout_ns) {
   extern __shared__ uint8_t dyn[];
   __shared__ AttnShared sh;
   constexpr int D = VDC_HEAD_DIM;
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int splits = s.splits, rank = splits > 1 ? (int)cluster_rank() : 0;
-  const int h = blockIdx.y, b = blockIdx.z, G = s.group;
+  const int unit = first_unit + (int)blockIdx.x / splits, h = unit % s.n_kv, b = unit / s.n_kv, G = s.group;
   uint8_t* ring = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(dyn) + 127) & ~(uintptr_t)127);
   const Waiter wait{&sh.fail, status, timeout_ns, s.kind};
   attn_setup(sh, tid);
@@ -788,14 +788,14 @@ __global__ void __launch_bounds__(kAttnThreads, 2) stage_attn(const __grid_const
 // ------------------------------------------------------------------------- //
 constexpr int kRows = 64;
 
-__global__ void __launch_bounds__(kAttnThreads, 2) stage_attn_prefill(const __grid_constant__ vdc_stage s, vdc_status* status,
+__global__ void __launch_bounds__(kAttnThreads, 2) stage_attn_prefill(const __grid_constant__ vdc_stage s, int first_unit, vdc_status* status,
                                                                       uint64_t timeout_ns) {
   extern __shared__ uint8_t dyn[];
   __shared__ AttnShared sh;
   constexpr int D = VDC_HEAD_DIM;
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int splits = s.splits, rank = splits > 1 ? (int)cluster_rank() : 0;
-  const int h = blockIdx.y, G = s.group, per_tile = kRows / G, b0 = blockIdx.z * per_tile;
+  const int unit = first_unit + (int)blockIdx.x / splits, h = unit % s.n_kv, G = s.group, b0 = unit / s.n_kv * (kRows / G);
   uint8_t* ring = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(dyn) + 127) & ~(uintptr_t)127);
   const Waiter wait{&sh.fail, status, timeout_ns, s.kind};
   attn_setup(sh, tid);
@@ -948,9 +948,9 @@ __global__ void __launch_bounds__(kAttnThreads, 2) stage_attn_prefill(const __gr
 
 // Embedding row of one sequence: the hidden state and its sum of squares; and zeros for the sums that the step's residual
 // adds accumulate.  An id outside the table (M rows, 0: only its sign is known) is reported and row 0 taken in its place.
-__global__ void __launch_bounds__(256) stage_embed(const __grid_constant__ vdc_stage s, vdc_status* status) {
+__global__ void __launch_bounds__(256) stage_embed(const __grid_constant__ vdc_stage s, int first_row, vdc_status* status) {
   __shared__ float red[8];
-  const int b = blockIdx.x, tid = threadIdx.x;
+  const int b = first_row + (int)blockIdx.x, tid = threadIdx.x;
   grid_dep_wait();
   grid_dep_launch();
   int token = ld_relaxed_gpu(reinterpret_cast<const int*>(s.state) + (size_t)b * s.state_stride + VDC_ST_TOKEN);
@@ -984,8 +984,8 @@ __global__ void __launch_bounds__(256) stage_embed(const __grid_constant__ vdc_s
 // A stage of its own, once per projection, instead of in every block of the projection that reads the rows: two layers and
 // a 128256-row vocabulary projection 382 -> 374 us at 3 rows, 617 -> 574 at 64, 1070 -> 821 at 128 (normalising inside
 // the projection, a block's warps rewrote every chunk in shared memory between its arrival and the tensor cores).
-__global__ void __launch_bounds__(256) stage_norm(const __grid_constant__ vdc_stage s) {
-  const int p = (int)blockIdx.x * 256 + (int)threadIdx.x;      // 16-byte piece: eight inputs of one row
+__global__ void __launch_bounds__(256) stage_norm(const __grid_constant__ vdc_stage s, int first_block) {
+  const int p = (first_block + (int)blockIdx.x) * 256 + (int)threadIdx.x;      // 16-byte piece: eight inputs of one row
   const int k8 = p / s.Bpad, b = p & (s.Bpad - 1);
   const bool live = k8 < s.K / 8;
   const uint4 w = live ? __ldg(reinterpret_cast<const uint4*>(s.norm_w) + k8) : make_uint4(0u, 0u, 0u, 0u);
@@ -1047,56 +1047,77 @@ extern "C" cudaError_t vdc_stage_prepare() {
   return cudaSuccess;
 }
 
-extern "C" cudaError_t vdc_stage_launch(const vdc_stage* s, vdc_status* status, uint64_t timeout_ns, cudaStream_t stream) {
+// A stage's grid: `units` of `splits` CTAs each, and how many units one launch takes.
+struct Grid {
+  int units, splits, slice;
+};
+static Grid stage_grid(const vdc_stage* s, int max_ctas) {
+  const bool attn = s->kind == VDC_STAGE_ATTN || s->kind == VDC_STAGE_ATTN_PREFILL;
+  const int tile = attn ? vdc::kRows / s->group : 1;       // rows of a prefill unit
+  Grid g{1, s->kind == VDC_STAGE_GEMM || attn ? s->splits : 1, 0};
+  switch (s->kind) {
+    case VDC_STAGE_GEMM: g.units = (s->M + vdc::kBlk - 1) / vdc::kBlk; break;
+    case VDC_STAGE_ATTN: g.units = s->n_kv * s->B; break;
+    case VDC_STAGE_ATTN_PREFILL: g.units = s->n_kv * ((s->B + tile - 1) / tile); break;
+    case VDC_STAGE_NORM: g.units = (s->Bpad * (s->K / 8) + 255) / 256; break;
+    case VDC_STAGE_EMBED: g.units = s->B; break;
+  }
+  g.slice = max_ctas ? max_ctas / g.splits : g.units;
+  return g;
+}
+
+extern "C" void vdc_stage_slices(const vdc_stage* s, int max_ctas, int* launches, int* largest) {
+  const Grid g = stage_grid(s, max_ctas);
+  *launches = (g.units + g.slice - 1) / g.slice;
+  *largest = (g.units < g.slice ? g.units : g.slice) * g.splits;
+}
+
+// max_ctas 0: the stage's grid in one launch, with programmatic stream serialisation.  Otherwise at most that many CTAs run
+// at any time: the grid goes in slices of whole clusters, and a launch starts early only where it and the one in front of it
+// (*front CTAs, -1: not known) fit the limit together.  No third launch joins them: each lets the next one start behind its
+// own wait, when the one in front of it has ended.  24 layers of width 512, two rows, on 132 SMs: 1319 us with every launch
+// behind the end of the last, 878 us so.
+extern "C" cudaError_t vdc_stage_launch(const vdc_stage* s, int max_ctas, int* front, vdc_status* status, uint64_t timeout_ns,
+                                        cudaStream_t stream) {
+  if (s->kind == VDC_STAGE_COPY) *front = -1;
   if (s->kind == VDC_STAGE_COPY)
     return cudaMemcpyAsync((void*)s->out, (const void*)s->x, (size_t)s->M * s->K, cudaMemcpyDeviceToDevice, stream);
   cudaLaunchConfig_t cfg{};
   cudaLaunchAttribute attr[2];
   cfg.stream = stream;
   cfg.attrs = attr;
-  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  attr[0].val.programmaticStreamSerializationAllowed = 1;
-  cfg.numAttrs = 1;
-  if (s->splits > 1) {
-    attr[1].id = cudaLaunchAttributeClusterDimension;
-    attr[1].val.clusterDim.x = (unsigned)s->splits;
-    attr[1].val.clusterDim.y = attr[1].val.clusterDim.z = 1;
-    cfg.numAttrs = 2;
+  const bool gemm = s->kind == VDC_STAGE_GEMM, attn = s->kind == VDC_STAGE_ATTN || s->kind == VDC_STAGE_ATTN_PREFILL;
+  const Grid g = stage_grid(s, max_ctas);
+  if (g.splits > 1) {
+    attr[cfg.numAttrs].id = cudaLaunchAttributeClusterDimension;
+    attr[cfg.numAttrs].val.clusterDim.x = (unsigned)g.splits;
+    attr[cfg.numAttrs].val.clusterDim.y = attr[cfg.numAttrs].val.clusterDim.z = 1;
+    ++cfg.numAttrs;
   }
-  switch (s->kind) {
-    case VDC_STAGE_GEMM: {
-      cfg.gridDim = dim3((unsigned)((s->M + vdc::kBlk - 1) / vdc::kBlk * s->splits));
-      cfg.blockDim = dim3(vdc::kGemmThreads);
-      cfg.dynamicSmemBytes = vdc::kGemmSmem;
-      const int ring = vdc::ring_stages(s->wfmt, s->Bpad);
-      auto f = s->wfmt == 0 ? vdc::stage_gemm<0> : s->wfmt == 1 ? vdc::stage_gemm<1> : vdc::stage_gemm<2>;
-      return cudaLaunchKernelEx(&cfg, f, *s, ring, status, timeout_ns);
+  cudaLaunchAttribute& early = attr[cfg.numAttrs++];
+  early.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  cfg.blockDim = dim3(gemm ? vdc::kGemmThreads : attn ? vdc::kAttnThreads : s->kind == VDC_STAGE_ADVANCE ? 128 : 256);
+  cfg.dynamicSmemBytes = gemm ? vdc::kGemmSmem : attn ? vdc::kAttnSmem : 0;
+  for (int first = 0; first < g.units; first += g.slice) {
+    const int ctas = (g.units - first < g.slice ? g.units - first : g.slice) * g.splits;
+    cfg.gridDim = dim3((unsigned)ctas);
+    early.val.programmaticStreamSerializationAllowed = max_ctas == 0 || (*front >= 0 && *front + ctas <= max_ctas);
+    *front = ctas;
+    cudaError_t e;
+    switch (s->kind) {
+      case VDC_STAGE_GEMM: {
+        auto f = s->wfmt == 0 ? vdc::stage_gemm<0> : s->wfmt == 1 ? vdc::stage_gemm<1> : vdc::stage_gemm<2>;
+        e = cudaLaunchKernelEx(&cfg, f, *s, first, vdc::ring_stages(s->wfmt, s->Bpad), status, timeout_ns);
+        break;
+      }
+      case VDC_STAGE_ATTN: e = cudaLaunchKernelEx(&cfg, vdc::stage_attn, *s, first, status, timeout_ns); break;
+      case VDC_STAGE_ATTN_PREFILL: e = cudaLaunchKernelEx(&cfg, vdc::stage_attn_prefill, *s, first, status, timeout_ns); break;
+      case VDC_STAGE_NORM: e = cudaLaunchKernelEx(&cfg, vdc::stage_norm, *s, first); break;
+      case VDC_STAGE_EMBED: e = cudaLaunchKernelEx(&cfg, vdc::stage_embed, *s, first, status); break;
+      case VDC_STAGE_ADVANCE: e = cudaLaunchKernelEx(&cfg, vdc::stage_advance, *s, status); break;
+      default: e = cudaErrorInvalidValue;
     }
-    case VDC_STAGE_ATTN:
-      cfg.gridDim = dim3((unsigned)s->splits, (unsigned)s->n_kv, (unsigned)s->B);
-      cfg.blockDim = dim3(vdc::kAttnThreads);
-      cfg.dynamicSmemBytes = vdc::kAttnSmem;
-      return cudaLaunchKernelEx(&cfg, vdc::stage_attn, *s, status, timeout_ns);
-    case VDC_STAGE_ATTN_PREFILL: {
-      const int per = vdc::kRows / s->group;
-      cfg.gridDim = dim3((unsigned)s->splits, (unsigned)s->n_kv, (unsigned)((s->B + per - 1) / per));
-      cfg.blockDim = dim3(vdc::kAttnThreads);
-      cfg.dynamicSmemBytes = vdc::kAttnSmem;
-      return cudaLaunchKernelEx(&cfg, vdc::stage_attn_prefill, *s, status, timeout_ns);
-    }
-    case VDC_STAGE_NORM:
-      cfg.gridDim = dim3((unsigned)((s->Bpad * (s->K / 8) + 255) / 256));
-      cfg.blockDim = dim3(256);
-      return cudaLaunchKernelEx(&cfg, vdc::stage_norm, *s);
-    case VDC_STAGE_EMBED:
-      cfg.gridDim = dim3((unsigned)s->B);
-      cfg.blockDim = dim3(256);
-      return cudaLaunchKernelEx(&cfg, vdc::stage_embed, *s, status);
-    case VDC_STAGE_ADVANCE:
-      cfg.gridDim = dim3(1);
-      cfg.blockDim = dim3(128);
-      return cudaLaunchKernelEx(&cfg, vdc::stage_advance, *s, status);
-    default:
-      return cudaErrorInvalidValue;
+    if (e != cudaSuccess) return e;
   }
+  return cudaSuccess;
 }

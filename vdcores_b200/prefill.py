@@ -85,7 +85,8 @@ class PrefillEngine(BatchDecodeEngine):
             for c in range(n):
                 self._fill_states(states[c].numpy(), ids, c)
                 self.state.copy_(states[c], non_blocking=True)
-                runtime.launch_stages(self.stages if c == n - 1 else self._body, self.stream.cuda_stream, self.timeout_ns)
+                runtime.launch_stages(self.stages if c == n - 1 else self._body, self.stream.cuda_stream, self.timeout_ns,
+                                      self.max_ctas)
         runtime.read_status(self.stream.cuda_stream)
         first = int(self.token_log[(T - 1) % B, 0])
         if set_target_state:
