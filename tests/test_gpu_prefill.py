@@ -148,3 +148,36 @@ def test_long_walks_agree_with_the_decode_program(cuda_device):
         assert float(((kd - ko).norm(dim=1) / ko.norm(dim=1)).max()) < 4 * REL_L2_BF16, f"a K row of layer {l}"
     if float((top2[0] - top2[1]) / top2[0].abs()) > 5 * GAP:
         assert first == first_ref
+
+
+def test_host_memory_of_a_prompt_does_not_grow_with_its_chunks(cuda_device, monkeypatch):
+    """60 chunks through a bounded number of pinned state blocks, with the cache rows of one chunk after another's block."""
+    from vdcores_b200.decode import DecodeEngine
+    from vdcores_b200.prefill import PrefillEngine
+    cfg = small_cfg("llama")
+    w = perturb_norms(O.ModelWeights.random(cfg, seed=27))
+    T, chunk = 950, 16
+    prompt = torch.randint(0, cfg.vocab, (T,), generator=torch.Generator().manual_seed(28))
+    eng = DecodeEngine(engine_config(cfg), max_seq=1088, device=cuda_device, timeout_ns=500_000_000)
+    eng.load_weights(dense_weights(w))
+    wide = PrefillEngine(eng, chunk=128, timeout_ns=500_000_000).adopt_weights()
+    wide.prefill(prompt)
+    ref = [[t.clone() for t in eng.read_kv(l, T)] for l in range(cfg.n_layers)]
+    eng.kpool.zero_()
+    eng.vpool.zero_()
+    pre = PrefillEngine(eng, chunk=chunk, timeout_ns=500_000_000).adopt_weights()
+    pinned, empty = [], torch.empty
+
+    def counted(*a, **kw):
+        t = empty(*a, **kw)
+        if kw.get("pin_memory"):
+            pinned.append(t.numel() * t.element_size())
+        return t
+    monkeypatch.setattr(torch, "empty", counted)
+    pre.prefill(prompt)
+    monkeypatch.undo()
+    assert sum(pinned) == 4 * chunk * pre.state_words * 4
+    for l in range(cfg.n_layers):
+        for got, want in zip(eng.read_kv(l, T), ref[l]):
+            rows = (got.float() - want.float()).flatten(1).norm(dim=1) / want.float().flatten(1).norm(dim=1)
+            assert float(rows.max()) < 4 * REL_L2_BF16, f"layer {l} position {int(rows.argmax())}"

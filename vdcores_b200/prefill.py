@@ -23,6 +23,7 @@ from .decode import DecodeEngine
 class PrefillEngine(BatchDecodeEngine):
     """`chunk` prompt positions per launch into the KV pools of `target` (a DecodeEngine of the same model)."""
     SHARED_CACHE = True
+    BLOCKS = 4          # chunks whose state blocks may wait in host memory
 
     def __init__(self, target: DecodeEngine, chunk: int = 64, timeout_ns: int = 2_000_000_000):
         assert not isinstance(target, BatchDecodeEngine) and not target.cfg.n_experts
@@ -74,17 +75,24 @@ class PrefillEngine(BatchDecodeEngine):
     @torch.no_grad()
     def prefill(self, tokens: torch.Tensor, set_target_state: bool = True) -> int:
         """Runs the prompt, ceil(T / chunk) lists of stages, and returns the first generated (greedy) id.  A chunk's state
-        blocks are prepared in pinned memory while the GPU runs the chunk before it."""
+        blocks are prepared in pinned memory while the GPU runs the chunks before it, BLOCKS of them at most: every row of a
+        block carries the page table, and a place per chunk would grow with the square of the prompt."""
         T, B = int(tokens.numel()), self.batch
         assert 1 <= T < self.max_seq and self.stages is not None
         n = (T + B - 1) // B
         ids = tokens.cpu().to(torch.int32).numpy().reshape(-1)
-        states = torch.empty(n, B, self.state_words, dtype=torch.int32, pin_memory=True)    # one block per chunk: none is rewritten
+        blocks = torch.empty(min(n, self.BLOCKS), B, self.state_words, dtype=torch.int32, pin_memory=True)
+        k = len(blocks)
+        copied = [torch.cuda.Event() for _ in blocks] if n > k else None
         self.keys.zero_()
         with torch.cuda.stream(self.stream):
             for c in range(n):
-                self._fill_states(states[c].numpy(), ids, c)
-                self.state.copy_(states[c], non_blocking=True)
+                if c >= k:
+                    copied[c % k].synchronize()         # the chunk that had this block has been copied
+                self._fill_states(blocks[c % k].numpy(), ids, c)
+                self.state.copy_(blocks[c % k], non_blocking=True)
+                if copied:
+                    copied[c % k].record(self.stream)
                 runtime.launch_stages(self.stages if c == n - 1 else self._body, self.stream.cuda_stream, self.timeout_ns,
                                       self.max_ctas)
         runtime.read_status(self.stream.cuda_stream)
