@@ -294,6 +294,41 @@ def test_every_step_of_a_large_batch_has_the_same_bits(cuda_device, batch, ctx):
         assert float(rows.max()) < 1e-2, f"pass {i}: hidden row {int(rows.argmax())}"
 
 
+@pytest.mark.parametrize("splits", [1, 8])
+def test_qkv_stage_writes_a_repeated_position_once(cuda_device, splits):
+    """Query rows and cache rows against plain matmuls (no rotation at position 0's angles); rows with the cache row of the
+    row in front of them leave it to that one, whatever their own values are."""
+    from vdcores_b200 import isa, runtime
+    from vdcores_b200.decode import kv_page_swizzle
+    dev, B, G, n_kv, K, D = cuda_device, 24, 4, 2, 1024, 128
+    M = n_kv * (G + 2) * D
+    x = seeded((B, K), 31)
+    w, _, wf = weights(M, K, "bf16", dev, seed=32)
+    xd = packed_rows(x, dev)
+    rope = torch.cat((torch.ones(128, 64), torch.zeros(128, 64)), 1).to(dev)
+    pos = torch.arange(60, 60 + B).clamp_(max=60 + 9)
+    table = torch.tensor([2, 0])
+    state = torch.zeros(B, isa.ST_PAGETABLE + 2, dtype=torch.int32)
+    state[:, isa.ST_POS] = pos
+    state[:, isa.ST_NEWROW] = table[pos // 64] * 64 * n_kv + pos % 64
+    sd, q = state.to(dev), torch.zeros(B, n_kv * G, D, dtype=BF16, device=dev)
+    for _ in range(20):
+        pools = [torch.zeros(3, n_kv, 64, D, dtype=BF16, device=dev) for _ in range(2)]
+        run(dev, gemm(dev, "bf16", B, M, K, splits, w, None, xd, mode=isa.STAGE_QKV, out=q.data_ptr(), rope=rope.data_ptr(),
+                      kpool=pools[0].data_ptr(), vpool=pools[1].data_ptr(), group=G, n_kv=n_kv, state=sd.data_ptr(),
+                      state_stride=state.shape[1]))
+        y = (x.float() @ wf.t()).view(B, n_kv, G + 2, D)
+        assert rel(q.cpu().view(B, n_kv, G, D), y[:, :, :G]) < REL
+        for i, pool in enumerate(pools):
+            rows = kv_page_swizzle(pool.cpu()).float()
+            want = torch.zeros_like(rows)
+            for b in range(10):
+                want[table[pos[b] // 64], :, pos[b] % 64] = y[b, :, G + i]
+            assert rel(rows, want) < REL and bool((rows[want.abs().sum(-1) == 0] == 0).all())
+            last = rows[table[pos[9] // 64], :, pos[9] % 64]
+            assert rel(last, y[9, :, G + i]) < REL
+
+
 @pytest.mark.parametrize("num_sms", [1, 7, 61, 140])
 def test_a_step_and_a_prompt_on_fewer_sms(cuda_device, num_sms):
     """num_sms below the device's count: slices of at most that many CTAs, and the results of the whole device."""

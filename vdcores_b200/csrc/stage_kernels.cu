@@ -224,10 +224,14 @@ __device__ __forceinline__ void qkv_head(const vdc_stage& s, const uint8_t* tile
     dst[32] = hi;
     return;
   }
+  // rows past a prompt's end repeat its last position: the first of them writes the cache row, since their sums of squares
+  // (atomics) may differ in the last bit
+  const int new_row = ld_relaxed_gpu(st + VDC_ST_NEWROW);
+  if (b > 0 && ld_relaxed_gpu(st - s.state_stride + VDC_ST_NEWROW) == new_row) return;
   // the row's 16-byte pieces lie at (piece XOR (row mod 8)), the page-row order the attention reads
   const int sw = pos & 7;
   uint8_t* row = reinterpret_cast<uint8_t*>(part == G ? s.kpool : s.vpool) + (size_t)kvh * (VDC_KV_PAGE * D * 2) +
-                 (size_t)ld_relaxed_gpu(st + VDC_ST_NEWROW) * (D * 2);
+                 (size_t)new_row * (D * 2);
   *reinterpret_cast<uint32_t*>(row + (((i0 >> 3) ^ sw) << 4) + (i0 & 7) * 2) = lo;
   *reinterpret_cast<uint32_t*>(row + (((8 + (i0 >> 3)) ^ sw) << 4) + (i0 & 7) * 2) = hi;
 }

@@ -59,7 +59,7 @@ class PrefillEngine(BatchDecodeEngine):
     # ------------------------------------------------------------------ chunks
     def _fill_states(self, s, tokens, c: int):
         """State blocks of chunk c into the int32 array s [chunk, state_words]: row b is position c * chunk + b (rows past
-        the prompt's end repeat its last position: same row, same bytes)."""
+        the prompt's end repeat its last position; the first of them writes the cache row)."""
         pos = np.minimum(np.arange(c * self.batch, (c + 1) * self.batch), len(tokens) - 1)
         page = pos // isa.KV_PAGE
         table = self.page_table.numpy()
