@@ -384,7 +384,7 @@ def run_gpu(args):
                                 f"batch {args.batch}, {PROMPT_LEN}-token prompt{'s' if args.batch > 1 else ''} prefilled, greedy decode"),
                    "l2": f"inputs larger than L2: every step streams {bytes_per_launch / 1e9:.2f} GB per GPU through a 126 MB L2",
                    "parallelism": parallelism,
-                   "num_sms": eng.num_sms, "kv_splits": getattr(eng, "attn_splits", eng.n_splits), "first_tokens": tokens[:4],
+                   "num_sms": eng.num_sms, "kv_splits": eng.n_splits, "first_tokens": tokens[:4],
                    **({"layers": args.layers, "note": "reduced-depth profiling case, not a benchmark result"}
                       if args.layers != 32 else {})},
         "roofline": {"bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s", "frac": achieved / peak,

@@ -158,25 +158,27 @@ def test_gemm_tc_argmax_keys(cuda_device):
         assert float(ref[b, got[b]]) >= float(ref[b].max()) - 1e-2 * float(ref[b].abs().max())
 
 
-@pytest.mark.parametrize("kind,batch,num_sms", [("llama", 3, None), ("qwen3", 20, None), ("llama", 20, 32)])
+@pytest.mark.parametrize("kind,batch,num_sms", [("llama", 3, None), ("qwen3", 20, None), ("llama", 20, 32), ("llama", 64, 100),
+                                                ("qwen3", 128, None), ("llama", 128, 100)])
 def test_batch_decode_matches_oracle(cuda_device, kind, batch, num_sms):
-    """20 sequences x 2 KV heads on 32 SMs: more attention units than SMs, so a unit walks all four pages of its
-    sequence alone, two pages per trip (contexts of 4, 3 and 2 pages: last page second in a trip, odd tail page,
-    single trip)."""
+    """20 and more sequences x 2 KV heads on 32 or 100 SMs: more attention units than SMs, so a unit's CTA walks all four
+    pages of its sequence alone (contexts of 4, 3, 2 and 1 pages); with all SMs several CTAs share them."""
+    from vdcores_b200 import isa
     from vdcores_b200.batch import BatchDecodeEngine
     cfg = small_cfg(kind)
     w = perturb_norms(O.ModelWeights.random(cfg, seed=3))
     g = torch.Generator().manual_seed(31)
     lens = [int(v) for v in torch.randint(2, 150, (batch,), generator=g)]
     if batch > 4:       # the oracle prefill is the slow part: keep most prompts short
-        lens = [l if b < 3 else 2 + l % 20 for b, l in enumerate(lens)]
+        lens = [l if b < 3 else 2 + l % (20 if batch <= 20 else 5) for b, l in enumerate(lens)]
     if num_sms is not None:
         lens[:3] = [200, 131, 100]
     prompts = [torch.randint(0, cfg.vocab, (n,), generator=g) for n in lens]
     eng = BatchDecodeEngine(engine_config(cfg), batch, max_seq=256, device=cuda_device, taps=True, page_perm_seed=5,
                             timeout_ns=500_000_000, num_sms=num_sms)
-    assert num_sms is None or (eng.n_splits == 1 and eng.pages_per_split == 4)
     eng.load_weights(dense_weights(w))
+    walks = {s.splits for s in eng.stages if s.kind == isa.STAGE_ATTN}
+    assert walks == {eng.n_splits} and (eng.n_splits == 1) == (num_sms is not None)
     orcs, toks = [], []
     for b in range(batch):
         orc = O.DecodeOracle(w, 256)
@@ -186,7 +188,7 @@ def test_batch_decode_matches_oracle(cuda_device, kind, batch, num_sms):
         eng.set_state(n, int(prompts[b][-1]), b=b)
         orcs.append(orc)
         toks.append(int(prompts[b][-1]))
-    for step in range(3):
+    for step in range(3 if batch <= 20 else 2):
         got = eng.generate(1)[0]
         taps = [eng.read_hidden(eng.taps[l]).cpu() for l in range(cfg.n_layers)]
         fix = {}

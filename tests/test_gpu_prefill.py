@@ -52,8 +52,8 @@ def _check_cache_and_continue(cfg, T, orc, nxt, gap, eng, first, n_steps=4):
                                                         ("llama", 200, 128, 9), ("qwen3", 150, 128, None)])
 def test_chunked_prefill_matches_oracle(cuda_device, kind, prompt_len, chunk, perm):
     """Chunks that end inside a page, a ragged last chunk, a prompt shorter than one chunk, shuffled page ids,
-    per-head q/k norms; with 128 positions per launch there are more attention units than SMs and a unit walks
-    its pages alone, two per trip (with and without two positions per unit)."""
+    per-head q/k norms; chunks of 16 to 128 positions (one to eight tiles of query rows per KV head, a last one that ends past
+    the rows)."""
     from vdcores_b200.prefill import PrefillEngine
     cfg, prompt, orc, nxt, gap, eng = _setup(kind, prompt_len, cuda_device, seed=21, page_perm_seed=perm)
     pre = PrefillEngine(eng, chunk=chunk, timeout_ns=500_000_000).adopt_weights()
@@ -120,18 +120,19 @@ def test_chunked_prefill_with_quantised_projections(cuda_device, wkind, tol, bas
         assert first == nxt
 
 
-def test_long_walks_agree_with_the_decode_program(cuda_device):
-    """A 1000-token prompt, 128 positions per launch: units walk up to 16 pages two at a time, through every page
-    count whose odd tail page once shared an arrival counter with the trip before it (15 pages: positions 896..959).
-    Checked against the same prompt run position by position through the decode program (itself checked against the
+@pytest.mark.parametrize("num_sms,n_splits", [(16, 1), (None, 8)])
+def test_long_walks_agree_with_the_decode_program(cuda_device, num_sms, n_splits):
+    """A 1000-token prompt, 128 positions per chunk: on 16 SMs a tile's CTA walks all its pages alone, up to 16 of them;
+    with all SMs eight CTAs share them.  Checked against the same prompt run position by position through the decode program (itself checked against the
     oracle above): cache rows of every layer, first generated id."""
+    from vdcores_b200 import isa
     from vdcores_b200.decode import DecodeEngine
     from vdcores_b200.prefill import PrefillEngine
     cfg = small_cfg("llama")
     w = perturb_norms(O.ModelWeights.random(cfg, seed=27))
     T = 1000
     prompt = torch.randint(0, cfg.vocab, (T,), generator=torch.Generator().manual_seed(28))
-    eng = DecodeEngine(engine_config(cfg), max_seq=1088, device=cuda_device, timeout_ns=500_000_000)
+    eng = DecodeEngine(engine_config(cfg), max_seq=1088, device=cuda_device, timeout_ns=500_000_000, num_sms=num_sms)
     eng.load_weights(dense_weights(w))
     first_ref = eng.prefill_device(prompt)
     ref = [[t.clone() for t in eng.read_kv(l, T)] for l in range(cfg.n_layers)]
@@ -139,7 +140,8 @@ def test_long_walks_agree_with_the_decode_program(cuda_device):
     eng.kpool.zero_()
     eng.vpool.zero_()
     pre = PrefillEngine(eng, chunk=128, timeout_ns=500_000_000).adopt_weights()
-    assert pre.n_splits == 1 and pre.pages_per_split == 17
+    assert {s.splits for s in pre.stages if s.kind == isa.STAGE_ATTN_PREFILL} == {n_splits}
+    assert pre.n_splits == n_splits and pre.pages_per_split == -(-17 // n_splits)
     first = pre.prefill(prompt)
     for l in range(cfg.n_layers):
         k_dev, v_dev = eng.read_kv(l, T)

@@ -265,7 +265,7 @@ def test_every_step_of_a_large_batch_has_the_same_bits(cuda_device, batch, ctx):
     cfg = DecodeConfig(hidden=1024, n_heads=32, n_kv_heads=8, ffn=2048, vocab=2048, n_layers=1)
     eng = BatchDecodeEngine(cfg, batch, max_seq=ctx + 64, device=cuda_device, page_perm_seed=3)
     eng.init_random_weights(1)
-    assert eng.attn_splits == 1
+    assert eng.n_splits == 1
     g = torch.Generator(device=cuda_device).manual_seed(2)
     for t in (eng.kpool, eng.vpool):
         t.normal_(generator=g)

@@ -169,12 +169,15 @@ class BatchDecodeEngine(DecodeEngine):
         # per-sequence sums of squares of the hidden matrix after the embedding / each residual add
         # (the RMSNorm statistics of the projection that reads it); zero between steps
         self.stats = z(2 * L + 1, 128, dt=torch.float32)
-        units = B * cfg.n_kv_heads
-        self.n_splits = 1 if units >= self.num_sms else max(1, min(self.num_sms // units, self.max_pages))
-        self.pages_per_split = (self.max_pages + self.n_splits - 1) // self.n_splits
-        self.n_splits = (self.max_pages + self.pages_per_split - 1) // self.pages_per_split
         self.stages = None
         self.max_ctas = self.num_sms if self.num_sms < torch.cuda.get_device_properties(self.dev).multi_processor_count else 0
+        # CTAs that share an attention unit's pages.  A prefill tile's shares are 64 rows each to merge: no more CTAs than are
+        # resident at once (8 shares of 64 tiles took 31 us at four pages and 46 at 31 pages); a decode unit's are 4 or 8
+        # rows, and two waves of CTAs even out sequences of different lengths
+        tile = 64 // cfg.group          # rows of one prefill attention unit
+        units = cfg.n_kv_heads * (-(-B // tile) if self.SHARED_CACHE else B)
+        self.n_splits = self._splits(units, 2 if self.SHARED_CACHE else 4, self.max_pages)
+        self.pages_per_split = -(-self.max_pages // self.n_splits)
         self.state_words = isa.ST_PAGETABLE + self.max_pages
         self.state = z(B, self.state_words, dt=torch.int32)
         self.state_host = torch.zeros(B, self.state_words, dtype=torch.int32).pin_memory()
@@ -182,7 +185,6 @@ class BatchDecodeEngine(DecodeEngine):
         self._alloc_cache(page_perm_seed)
         self.taps_enabled = taps
         if taps:
-            assert Bp * H * 2 <= 32768, "taps copy the hidden matrix with one bulk load"
             self.taps = z(L, Bp * H)
         self._cur = 0
         self.positions = [0] * B
@@ -257,20 +259,14 @@ class BatchDecodeEngine(DecodeEngine):
         heads = dict(group=G, n_kv=cfg.n_kv_heads, **state)
         out = [runtime.Stage(kind=isa.STAGE_EMBED, B=B, Bpad=self.bpad, M=cfg.vocab, K=cfg.hidden, w=self.embed.data_ptr(), hid=hid,
                              stats_out=stat(0), n_stats=2 * L + 1, **state)]
-        tile = 64 // G      # rows of one prefill attention unit
-        units = cfg.n_kv_heads * (-(-B // tile) if self.SHARED_CACHE else B)
         attn_kind = isa.STAGE_ATTN_PREFILL if self.SHARED_CACHE else isa.STAGE_ATTN
-        # a prefill tile's shares are 64 rows each to merge: no more CTAs than are resident at once (8 shares of 64 tiles
-        # took 31 us at four pages and 46 at 31 pages); a decode unit's are 4 or 8 rows, and two waves of CTAs even out
-        # sequences of different lengths
-        self.attn_splits = self._splits(units, 2 if self.SHARED_CACHE else 4, self.max_pages)
         for l in range(L):
             pools = dict(kpool=self.kpool[l].data_ptr(), vpool=self.vpool[l].data_ptr())
             out.append(norm(2 * l, self.ln1[l]))
             out.append(self._gemm("wqkv", l, self.wqkv[l], self.normed, isa.STAGE_QKV, out=self.q.data_ptr(),
                                   rope=self.rope.data_ptr(), qk_norm=self.qknorm[l].data_ptr() if cfg.qk_norm else 0,
                                   qk_eps=cfg.qk_norm_eps, **heads, **pools))
-            out.append(runtime.Stage(kind=attn_kind, B=B, Bpad=self.bpad, splits=self.attn_splits, n_pages=self.max_pages,
+            out.append(runtime.Stage(kind=attn_kind, B=B, Bpad=self.bpad, splits=self.n_splits, n_pages=self.max_pages,
                                      q=self.q.data_ptr(), out=self.attn_out.data_ptr(), **heads, **pools))
             out.append(self._gemm("wo", l, self.wo[l], self.attn_out, isa.STAGE_RESID, hid=hid,
                                   stats_out=stat(2 * l + 1)))
