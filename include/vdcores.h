@@ -62,8 +62,7 @@ int vdc_launch_async(int num_sms, int insts_per_sm, const void* compute_insts, c
                      const void* tma_descs, int* bars, const int* bars_init, uint64_t* profile, uint64_t stream,
                      uint64_t timeout_ns);
 
-/* vdc_launch_async for the FULL kernel (every operator vdc_launch has, no synchronisation): what the batched decode
- * engine and the prefill launch.  The batch-1 engines stay on vdc_launch_async, whose kernel is smaller and, measured,
+/* vdc_launch_async for the FULL kernel (every operator vdc_launch has, no synchronisation).  The batch-1 engines stay on vdc_launch_async, whose kernel is smaller and, measured,
  * 1.7-1.8 % faster on their step.  No counterpart in the reference. */
 int vdc_launch_async_full(int num_sms, int insts_per_sm, const void* compute_insts, const void* memory_insts,
                           const void* tma_descs, int* bars, const int* bars_init, uint64_t* profile, uint64_t stream,

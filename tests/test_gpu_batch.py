@@ -291,3 +291,139 @@ def test_batch_decode_quantised_matches_oracle(cuda_device, wkind, tol):
             toks[b] = nxt_ref
         for b, t in fix.items():
             eng.state[b, 2:3].copy_(torch.tensor([t], dtype=torch.int32))
+
+
+def _step_program(eng, n_sms, splits):
+    """The step of a one-layer batched engine (or the chunk of a prefill engine) as one program of the megakernel: embedding
+    rows, projections, cache append, attention units (two positions each where they can be paired), advance."""
+    import math
+    from vdcores_b200 import isa
+    from vdcores_b200.batch import BLOCK_ROWS, emit_projection, pack_blocks, projection_blocks
+    from vdcores_b200.program import Program, Src
+    cfg, B, Bp, D, G, n_kv, dev = eng.cfg, eng.batch, eng.bpad, 128, eng.cfg.group, eng.cfg.n_kv_heads, eng.dev
+    H, F, V, W = cfg.hidden, cfg.ffn, cfg.vocab, eng.state_words
+    P, load, keep = Program(n_sms, insts_per_sm=isa.MAX_INSTS), [0] * n_sms, []
+    z = lambda *n, dt=torch.int32: keep.append(torch.zeros(*n, dtype=dt, device=dev)) or keep[-1]
+    st, stat = eng.state.data_ptr(), lambda i: eng.stats[i].data_ptr()
+    qkv, sms, at = z(B, eng.qkv_rows, dt=BF16), list(range(n_sms)), [0]
+
+    def sm():
+        at[0] += 1
+        return at[0] % n_sms
+
+    def project(w, K, x, wait, mode, release, out=0, **kw):
+        keep.append(pack_blocks(w))
+        n = len(projection_blocks(w.shape[0]))
+        emit_projection(P, sms=sms, load=load, w_addr=keep[-1].data_ptr(), M=w.shape[0], K=K, x_addr=x, B=B, Bpad=Bp, mode=mode,
+                        out_addr=out, scratch_addr=z(n * B * BLOCK_ROWS, dt=torch.float32).data_ptr(),
+                        counter_addr=z(n).data_ptr(), x_wait=wait, release=release, eps=cfg.eps, **kw)
+
+    b_hid, b_qkv, b_att, b_o, b_gu, b_d, b_lm = (P.new_barrier() for _ in range(7))
+    for b in range(B):
+        P.embed_pack(sm(), b0=b, count=1, Bpad=Bp, state_addr=st, state_stride_words=W, hidden=H, table_addr=eng.embed.data_ptr(),
+                     out_addr=eng.hidden.data_ptr(), stats_addr=stat(0), release=b_hid)
+    project(eng.wqkv[0], H, eng.hidden.data_ptr(), b_hid, isa.GEMM_MODE_STORE_ROWS, b_qkv, out=qkv.data_ptr(), ld=eng.qkv_rows,
+            norm_addr=eng.ln1[0].data_ptr(), stats_addr=stat(0))
+    page, pages, grp = 64 * D * 2, -(-eng.max_pages // splits), (G + 2) * D * 2
+    pair = eng.SHARED_CACHE and G == 4 and B % 2 == 0
+
+    def unit(b, h, **kw):
+        sb = st + 4 * W * b
+        return dict(state_addr=sb, rope=Src(eng.rope.data_ptr(), D * 4, indirect=(sb + 4 * isa.ST_POS, 9, None)),
+                    norm_w=Src(eng.qknorm[0].data_ptr(), 2 * D * 2) if cfg.qk_norm else None, qk_eps=cfg.qk_norm_eps,
+                    k_page_addr=eng.kpool[0].data_ptr() + h * page, v_page_addr=eng.vpool[0].data_ptr() + h * page,
+                    page_shift=int(math.log2(n_kv * page)), **kw)
+    rows = lambda b, h, wait: Src(qkv.data_ptr() + b * eng.qkv_rows * 2 + h * grp, grp, wait=wait)
+    b_rows = P.new_barrier() if eng.SHARED_CACHE else None
+    if eng.SHARED_CACHE:
+        P.add_releases(b_rows, B * n_kv)
+        for b in range(B):
+            for h in range(n_kv):
+                P.attn_decode(sm(), G=G, qkv=rows(b, h, b_qkv), base_page=0, max_pages=0, records_addr=0, counter_addr=0, out_addr=0,
+                              split=0, n_splits=1, release=b_rows, append=True, **unit(b, h))
+    step, GG = (2, 8) if pair else (1, G)
+    part, cnt = z(B, n_kv, splits, GG * D + 16, dt=torch.float32), z(B, n_kv)
+    P.add_releases(b_att, B // step * n_kv)
+    for b in range(0, B, step):
+        for h in range(n_kv):
+            for s in range(splits):
+                P.attn_decode(sm(), G=GG, qkv=rows(b, h, b_qkv if b_rows is None else b_rows), wait_issue=b_rows, base_page=s * pages,
+                              max_pages=pages, records_addr=part[b, h].data_ptr(), counter_addr=cnt[b, h].data_ptr(),
+                              out_addr=eng.attn_out.data_ptr() + h * G * D * Bp * 2, split=s, n_splits=splits, release=b_att,
+                              packed=(b, Bp), pair=(W, eng.qkv_rows) if pair else None, **unit(b, h))
+    project(eng.wo[0], cfg.q_width, eng.attn_out.data_ptr(), b_att, isa.GEMM_MODE_ADD_PACKED, b_o, out=eng.hidden.data_ptr(),
+            stats_addr=stat(1))
+    project(eng.wgu[0], H, eng.hidden.data_ptr(), b_o, isa.GEMM_MODE_SILU_PAIRS, b_gu, out=eng.act.data_ptr(),
+            norm_addr=eng.ln2[0].data_ptr(), stats_addr=stat(1))
+    project(eng.wd[0], F, eng.act.data_ptr(), b_gu, isa.GEMM_MODE_ADD_PACKED, b_d, out=eng.hidden.data_ptr(), stats_addr=stat(2))
+    project(eng.lm_head, H, eng.hidden.data_ptr(), b_d, isa.GEMM_MODE_ARGMAX, b_lm, keys_addr=eng.keys.data_ptr(),
+            norm_addr=eng.norm_w.data_ptr(), stats_addr=stat(2))
+    P.batch_advance(0, batch=B, state_addr=st, state_stride_words=W, keys_addr=eng.keys.data_ptr(), log_addr=eng.token_log.data_ptr(),
+                    log_stride=eng.max_steps, wait=b_lm, stats_addr=eng.stats.data_ptr(), n_stats=eng.stats.numel())
+    return P, keep
+
+
+@pytest.mark.parametrize("kind,shared,batch,splits", [("llama", False, 9, 2), ("qwen3", False, 20, 1), ("llama", True, 48, 1),
+                                                      ("llama", True, 32, 2), ("llama", True, 17, 1), ("qwen3", True, 16, 1)])
+def test_megakernel_tasks_of_a_batched_step(cuda_device, kind, shared, batch, splits):
+    """The batched tasks of the megakernel (embedding rows, packed, appending and paired attention, advance) put together to a
+    step and to a prompt's chunk, against the stage kernels' step over the same engine's weights and caches."""
+    import dataclasses
+    import numpy as np
+    from vdcores_b200 import isa
+    from vdcores_b200.batch import BatchDecodeEngine
+    from vdcores_b200.decode import DecodeEngine
+    from vdcores_b200.prefill import PrefillEngine
+    cfg = dataclasses.replace(engine_config(small_cfg(kind)), n_layers=1)
+    dev = cuda_device
+    if shared:
+        target = DecodeEngine(cfg, 320, device=dev, page_perm_seed=4)
+        target.init_random_weights(3)
+        eng = PrefillEngine(target, chunk=batch).adopt_weights()
+    else:
+        eng = BatchDecodeEngine(cfg, batch, max_seq=320, device=dev, page_perm_seed=4)
+        eng.init_random_weights(3)
+    g = torch.Generator(device=dev).manual_seed(5)
+    caches = [torch.empty_like(t).normal_(generator=g) for t in (eng.kpool, eng.vpool)]
+    state = np.zeros((batch, eng.state_words), dtype=np.int32)
+    if shared:      # positions 230 .. : the chunk's second page behind cached ones
+        eng._fill_states(state, np.arange(300, dtype=np.int32) % cfg.vocab, 0)
+        pos = 230 + np.arange(batch)
+        state[:, isa.ST_POS], state[:, isa.ST_NPAGES] = pos, pos // 64 + 1
+        state[:, isa.ST_NEWROW] = eng.page_table.numpy()[pos // 64] * 64 * cfg.n_kv_heads + pos % 64
+    else:
+        for b in range(batch):
+            eng.set_state(250 - 13 * b, b + 1, b=b)
+        state = eng.state.cpu().numpy()
+    before = torch.from_numpy(state).to(dev)
+    program, keep = _step_program(eng, 24, splits)
+
+    def results(launch):
+        eng.kpool.copy_(caches[0])
+        eng.vpool.copy_(caches[1])
+        eng.state.copy_(before)
+        eng.stats.zero_()
+        eng.keys.zero_()
+        eng.token_log.zero_()
+        launch()
+        return [t.clone() for t in (eng.state, eng.token_log[:, 0], eng.read_hidden(eng.hidden), eng.kpool, eng.vpool)]
+
+    from vdcores_b200 import runtime
+
+    def stages():
+        runtime.launch_stages(eng.stages, eng.stream.cuda_stream, 500_000_000)
+        runtime.read_status(eng.stream.cuda_stream)
+    got, want = results(lambda: run_program(program, dev)), results(stages)
+    same = got[1] == want[1]
+    assert float(same.float().mean()) > 0.8         # near-ties of random logits may fall either way
+    moved = got[0].clone()
+    moved[~same, isa.ST_TOKEN] = want[0][~same, isa.ST_TOKEN]
+    assert torch.equal(moved, want[0])
+    rows = (got[2].float() - want[2].float()).norm(dim=1) / want[2].float().norm(dim=1)
+    assert float(rows.max()) < 1e-2, f"hidden row {int(rows.argmax())}"
+    for a, b in zip(got[3:], want[3:]):
+        assert O.rel_l2(a, b) < 4e-3
+        rows = (a.float() - b.float()).flatten(0, 3).norm(dim=1) / b.float().flatten(0, 3).norm(dim=1)
+        assert float(rows.max()) < 2e-2
+    assert int(eng.keys.abs().max()) == 0
+    del keep

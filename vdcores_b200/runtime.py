@@ -184,7 +184,7 @@ def validate_streams(num_sms, insts_per_sm, compute_insts, memory_insts):
 
 def launch_async(num_sms, insts_per_sm, compute_insts, memory_insts, tma_descs, bars, bars_init, profile,
                  stream=0, timeout_ns=0, full=False):
-    """Enqueues one launch; full=True selects the kernel with every operator (batched engines, prefill)."""
+    """Enqueues one launch; full=True selects the kernel with every operator of launch_dae."""
     init()
     fn = _lib.vdc_launch_async_full if full else _lib.vdc_launch_async
     _check(fn(num_sms, insts_per_sm, _ptr(compute_insts), _ptr(memory_insts), _ptr(tma_descs),
