@@ -121,17 +121,9 @@ __device__ __forceinline__ void gemm_epilogue_flush(const GemmTc& g, int b, EpiA
   acc.best_row = 0x7fffffff;
 }
 
-#ifdef VDC_TC_PROFILE
-#define TCS(i) if (q.tid == 0) { const long long _n = clock64(); c.profile[c.sm * VDC_NUM_PROFILE_EVENTS + 100 + (i)] += _n - tcs_mark; tcs_mark = _n; }
-#else
-#define TCS(i)
-#endif
 VDC_TASK void task_gemm_tc(Compute& q, const GemmTc& g) {
   Shared* sh = q.sh;
   const Ctx& c = q.c;
-#ifdef VDC_TC_PROFILE
-  long long tcs_mark = clock64();
-#endif
   // Tensor memory is taken the first time a program needs it and given back when the kernel ends.
   if (!sh->tmem_ready) {
     if (q.warp == 0) tmem_alloc(&sh->tmem_base, kTmemCols);
@@ -167,7 +159,6 @@ VDC_TASK void task_gemm_tc(Compute& q, const GemmTc& g) {
   // order: it waits for the chunks, one lane issues the tensor-core work and, once the
   // previous chunk's reads are done, recycles its slots.  With norm the other seven warps
   // run ahead of it, normalising the X chunks in place and signalling each chunk's barrier.
-  TCS(0);
   q.warp_phase_begin(n_ent, q.warp == 0 ? 0u : n_ent);
   if (q.warp > 0 && (g.norm || g.wfmt != 0)) {
     // The seven warps work as a team of 224 threads, ahead of the issuer: they normalise each X
@@ -278,32 +269,16 @@ VDC_TASK void task_gemm_tc(Compute& q, const GemmTc& g) {
   if (q.warp == 0) {
     int w_prev = 0, x_prev = 0;  // lane 0: slots whose tensor-core reads may still be in flight
     int xm = 0;
-#ifdef VDC_TC_PROFILE
-    long long t_data = 0, t_xr = 0, t_mma = 0, t_wait = 0, t_xw = 0, t_ww = 0;
-#endif
     for (int j = 0; j < g.n_w; ++j) {
       const int grp = j / g.G, jj = j % g.G;
-#ifdef VDC_TC_PROFILE
-      const long long td0 = clock64();
-#endif
       int x_done = 0;
       if (jj == 0) x_done = xm;  // the previous group's X chunk: its last W chunk is the previous chunk
-#ifdef VDC_TC_PROFILE
-      const long long tq0 = clock64();
-#endif
       if (jj == 0) {
         xm = q.warp_wait(x_entry(grp));
         if (xm == kPopAbort) break;
         if (q.lane == 0) CHUNK_STAMP(c, q.head + x_entry(grp), 2);
       }
-#ifdef VDC_TC_PROFILE
-      if (j > 0) t_xw += clock64() - tq0;
-      const long long tq1 = clock64();
-#endif
       const int wm = q.warp_wait(w_entry(j));
-#ifdef VDC_TC_PROFILE
-      if (j > 0) t_ww += clock64() - tq1;
-#endif
       if (wm == kPopAbort) break;
       if (q.lane == 0) CHUNK_STAMP(c, q.head + w_entry(j), 2);
       if (g.wfmt != 0) {
@@ -320,10 +295,6 @@ VDC_TASK void task_gemm_tc(Compute& q, const GemmTc& g) {
         }
         if (!__shfl_sync(0xffffffffu, ok, 0)) break;
       }
-#ifdef VDC_TC_PROFILE
-      t_data += clock64() - td0;
-      const long long tx0 = clock64();
-#endif
       if (g.norm && jj == 0) {
         int ok = 1;
         if (q.lane == 0) {
@@ -337,10 +308,6 @@ VDC_TASK void task_gemm_tc(Compute& q, const GemmTc& g) {
         }
         if (!__shfl_sync(0xffffffffu, ok, 0)) break;
       }
-#ifdef VDC_TC_PROFILE
-      t_xr += clock64() - tx0;
-      const long long tm0 = clock64();
-#endif
       if (q.lane == 0) {
         tc_fence_after();
         uint64_t adesc = umma_desc(smem_u32(slot_ptr(c, first_slot(xm))) + (uint32_t)(jj * g.KS) * 2u * lbo_a, lbo_a, 128u);
@@ -355,10 +322,6 @@ VDC_TASK void task_gemm_tc(Compute& q, const GemmTc& g) {
           umma_bf16(tmem, adesc, bdesc, idesc, 1u);
         }
         umma_commit(&sh->mma_bar[q.mma_count & 3u]);
-#ifdef VDC_TC_PROFILE
-        t_mma += clock64() - tm0;
-        const long long tw0 = clock64();
-#endif
         // the previous chunk's reads are certainly done once its commit arrived
         if (j > 0) {
           int done = (g.wfmt != 0 ? 0 : w_prev) | x_done;  // e4m3 chunks were freed by the converting team
@@ -369,9 +332,6 @@ VDC_TASK void task_gemm_tc(Compute& q, const GemmTc& g) {
         }
         w_prev = wm & (int)kSlotMaskAll;
         q.mma_count++;
-#ifdef VDC_TC_PROFILE
-        t_wait += clock64() - tw0;
-#endif
       }
       __syncwarp();
     }
@@ -381,12 +341,6 @@ VDC_TASK void task_gemm_tc(Compute& q, const GemmTc& g) {
       if (q.mma_count > 0 && mma_wait(q, q.mma_count - 1) && (w_prev | x_prev))
         atomicOr(&sh->slot_avail, (uint32_t)(w_prev | x_prev) & kSlotMaskAll);
       sh->warp_next[0] = 0xFFFFFFFFu;
-#ifdef VDC_TC_PROFILE
-      uint64_t* pr = c.profile + c.sm * VDC_NUM_PROFILE_EVENTS;
-      pr[8] += t_data; pr[9] += t_xr; pr[10] += t_mma; pr[11] += t_wait; pr[12] += g.n_w;
-      pr[13] += (uint64_t)g.n_w * g.KS;
-      pr[14] += t_xw; pr[15] += t_ww;   // waits for X / W chunks after a task's first chunk
-#endif
     }
   }
   tc_fence_before();
@@ -402,7 +356,6 @@ VDC_TASK void task_gemm_tc(Compute& q, const GemmTc& g) {
     for (int st = 0; st < kStages; ++st) all |= stage_mask[st];
     q.free_slots(all);
   }
-  TCS(1);
 
   // Lane b of the accumulator belongs to sequence b; warps w and w+4 share the lane quarter
   // w % 4 and split the columns.
@@ -429,7 +382,6 @@ VDC_TASK void task_gemm_tc(Compute& q, const GemmTc& g) {
     compute_sync();  // every lane read its columns: the next task may overwrite the accumulator
     if (q.tid == 0 && g.bar != 0xFFFF) red_release_gpu_add(c.bars + g.bar, -1);
     q.free_slots(normw_mask);
-    TCS(2);
     return;
   }
   // ---- a K-slice: add the partial sums to the block's fp32 scratch area
@@ -448,7 +400,6 @@ VDC_TASK void task_gemm_tc(Compute& q, const GemmTc& g) {
   }
   tc_fence_before();
   compute_sync();
-  TCS(3);
   if (q.tid == 0) {
     // The sums are complete once every unit of the block arrived.  The bump releases this CTA's
     // adds (ordered before it by the CTA barrier; a release is cumulative) and acquires the
@@ -459,7 +410,6 @@ VDC_TASK void task_gemm_tc(Compute& q, const GemmTc& g) {
   }
   compute_sync();
   q.free_slots(normw_mask);
-  TCS(4);
   if (sh->misc[35] == 0.f) return;
   // ---- last arrival for this block: epilogue from the scratch area (read past L1), cleared for its next use
   const int items = g.B * ng;
@@ -483,10 +433,6 @@ VDC_TASK void task_gemm_tc(Compute& q, const GemmTc& g) {
     // the releasing count-down is cumulative: it publishes what the CTA barrier ordered before it
     if (g.bar != 0xFFFF) red_release_gpu_add(c.bars + g.bar, -1);
   }
-  TCS(5);
-#ifdef VDC_TC_PROFILE
-  if (q.tid == 0) c.profile[c.sm * VDC_NUM_PROFILE_EVENTS + 106] += 1;
-#endif
 }
 
 // ------------------------------------------------------------------------- //
