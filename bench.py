@@ -3,8 +3,9 @@
 
     python bench.py [--gpus N] [--steps K] [--warmup W] [--impl reference]
 
-One step = one greedy decode step (one megakernel launch) after a 2048-token
-prompt has been prefilled into the paged KV cache.  Weights are random
+One step = one greedy decode step (batch 1: one megakernel launch; larger
+batches: a list of stage kernels) after a 2048-token prompt has been prefilled
+into the paged KV cache.  Weights are random
 N(0, 0.02) bf16 of the named shape, the prompt is uniform random ids (synthetic
 stand-ins for a checkpoint and a dataset; there is no network).  Prints ONE
 JSON line.  `value` is timed with the state resident on the device; `e2e` goes
@@ -222,7 +223,7 @@ def run_gpu(args):
         full.init_random_weights(seed=0)
         first, prefill_info = run_prefill(full, prompt, args.prefill == "device")
         if "ms" in prefill_info:
-            # The megakernel prefill adds the K-slices of a projection block with fp32 atomics: the cache is not
+            # The device prefill adds a row's sums of squares with fp32 atomics: the cache is not
             # bit-identical from one GPU to the next, and a random-init model turns the last bits into other greedy
             # ids.  Every rank's shard and every rank's single-GPU trajectory must come from one cache: rank 0's.
             t = torch.tensor([first], dtype=torch.int64, device=dev)
@@ -390,7 +391,8 @@ def run_gpu(args):
         "roofline": {"bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s", "frac": achieved / peak,
                      # dram__bytes_read+write per launch: ncu measured 1.006 x the algorithmic bytes on a
                      # 4-layer case of the same program (profiles/), scaled here by the bytes of this launch
-                     "traffic": bytes_per_launch * 1.006 / 1e9, "traffic_unit": "GB", "peak_kind": f"of {peak_kind}", "frac_of_8TBs": achieved / 8000.0,
+                     # (one launch per step, batch 1; the stage kernels of larger batches were not captured at that size)
+                     "traffic": bytes_per_launch * 1.006 / 1e9 if args.batch == 1 else None, "traffic_unit": "GB", "peak_kind": f"of {peak_kind}", "frac_of_8TBs": achieved / 8000.0,
                      "bytes_per_launch": bytes_per_launch},
         "e2e": ({"value": tokens_per_step * K / (e2e_ms * 1e-3), "unit": "tokens/s",
                  "h2d_bytes_per_step": 4 * tokens_per_step, "d2h_bytes_per_step": 4 * tokens_per_step}
@@ -424,7 +426,7 @@ def run_prefill(eng, prompt, on_device):
         dt = time.perf_counter() - t0
         return first, {"impl": "megakernel, one prompt position per launch (the decode program)", "prompt_tokens": T,
                        "ms": dt * 1e3, "tokens_per_s": T / dt, "launches": T}
-    # the prompt goes through the megakernel too: 128 positions per launch into this engine's own pools
+    # the prompt goes through the stage kernels: 128 positions per list of stages into this engine's own pools
     from vdcores_b200.prefill import PrefillEngine
     pre = PrefillEngine(eng, chunk=128).adopt_weights()
     pre.prefill(prompt)                          # first call: one-time set-up of the kernel
@@ -433,10 +435,11 @@ def run_prefill(eng, prompt, on_device):
     first = pre.prefill(prompt)
     torch.cuda.synchronize()
     dt = time.perf_counter() - t0
+    launches = pre.launches(T)
     del pre
     torch.cuda.empty_cache()
-    return first, {"impl": "megakernel, 128 prompt positions per launch", "prompt_tokens": T, "ms": dt * 1e3,
-                   "tokens_per_s": T / dt, "launches": (T + 127) // 128}
+    return first, {"impl": "stage kernels, 128 prompt positions per list of stages", "prompt_tokens": T, "ms": dt * 1e3,
+                   "tokens_per_s": T / dt, "launches": launches}
 
 
 def main():
@@ -456,7 +459,7 @@ def main():
     ap.add_argument("--tp-impl", default="fused", choices=["fused", "nccl"],
                     help="N > 1, dense models: exchange inside the kernel (peer stores) or NCCL collectives between launches")
     ap.add_argument("--prefill", default="device", choices=["device", "torch"],
-                    help="batch 1: prompt through the megakernel (device) or PyTorch ops (torch)")
+                    help="batch 1: prompt through the device engine (device) or PyTorch ops (torch)")
     ap.add_argument("--layers", type=int, default=32,
                     help="profiling only: a model with fewer layers of the same shape (the JSON line says so)")
     args = ap.parse_args()

@@ -1,6 +1,6 @@
 """A Hugging Face checkpoint directory straight into the engines, checked against the Hugging Face model itself:
 tiny random LlamaForCausalLM / Qwen3ForCausalLM saved with save_pretrained, read by vdcores_b200.checkpoint, the
-prompt prefilled through the megakernel, then greedy decode; logits within the bf16 bar of the Hugging Face forward
+prompt prefilled on the device, then greedy decode; logits within the bf16 bar of the Hugging Face forward
 (bf16 on the host CPU), ids equal wherever its two best logits are more than a near-tie apart."""
 import pytest
 import torch

@@ -1,6 +1,6 @@
 """Prefill on the device against the CPU oracle: the prompt's cache rows (every layer) within the hidden-state bar,
 the first generated id equal wherever the oracle's top-2 logit gap exceeds 1e-2, and decode continuing from the
-prefilled pools on the oracle's trajectory.  Two paths: a chunk of positions per launch (prefill.PrefillEngine)
+prefilled pools on the oracle's trajectory.  Two paths: a chunk of positions per list of stages (prefill.PrefillEngine)
 and one position per launch through the decode program (DecodeEngine.prefill_device)."""
 import pytest
 import torch
@@ -63,7 +63,7 @@ def test_chunked_prefill_matches_oracle(cuda_device, kind, prompt_len, chunk, pe
 
 
 def test_chunked_prefill_agrees_with_the_pytorch_prefill(cuda_device):
-    """Same prompt through the library-GEMM prefill and the megakernel prefill: same first id (outside near-ties),
+    """Same prompt through the library-GEMM prefill and the device prefill: same first id (outside near-ties),
     cache rows within the bf16 bar of each other."""
     from vdcores_b200.prefill import PrefillEngine
     cfg, prompt, orc, nxt, gap, eng = _setup("llama", 200, cuda_device, seed=23)

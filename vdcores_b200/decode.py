@@ -822,8 +822,8 @@ class DecodeEngine:
         decode step, with the next prompt id written over the step's own argmax before the next launch (an 8-byte
         device-to-device copy on the engine's stream: {next id, step counter 0}).  No PyTorch arithmetic and no
         host round trip inside the loop; the KV rows and the returned first generated id have exactly the decode
-        path's numerics.  Cost: one decode step per prompt position (PrefillEngine in prefill.py does 64
-        positions per launch)."""
+        path's numerics.  Cost: one decode step per prompt position (PrefillEngine in prefill.py does up to 128
+        positions per list of stage kernels)."""
         T = int(tokens.numel())
         assert 1 <= T < self.max_seq
         forced = torch.zeros(T, 2, dtype=torch.int32)

@@ -21,7 +21,7 @@ from .decode import DecodeEngine
 
 
 class PrefillEngine(BatchDecodeEngine):
-    """`chunk` prompt positions per launch into the KV pools of `target` (a DecodeEngine of the same model)."""
+    """`chunk` prompt positions per list of stages into the KV pools of `target` (a DecodeEngine of the same model)."""
     SHARED_CACHE = True
     BLOCKS = 4          # chunks whose state blocks may wait in host memory
 
@@ -55,6 +55,11 @@ class PrefillEngine(BatchDecodeEngine):
         the last chunk adds the final norm, the vocabulary projection and the argmax (the first generated id)."""
         super()._build_program()
         self._body = self._plan(vocab=False)
+
+    def launches(self, T: int) -> int:
+        """Kernels a prompt of T tokens takes."""
+        body, last = (runtime.count_stage_launches(s, self.max_ctas)[0] for s in (self._body, self.stages))
+        return (T - 1) // self.batch * body + last
 
     # ------------------------------------------------------------------ chunks
     def _fill_states(self, s, tokens, c: int):

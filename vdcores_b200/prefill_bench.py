@@ -1,11 +1,11 @@
-"""Time to first token: the prompt through the megakernel, next to the PyTorch (library GEMM) prefill.
+"""Time to first token: the prompt through the stage kernels, next to the PyTorch (library GEMM) prefill.
 
     python -m vdcores_b200.prefill_bench [--layers 32] [--prompt 2048] [--chunks 64,128] [--reps 2]
 
 A Llama-3.1-8B-shaped model with `--layers` layers and random weights; for every chunk size the prompt is
 prefilled `--reps` times (best wall-clock time between two synchronisations, first call untimed) into the decode
 engine's own pools, then the last layer's cached key rows are compared with the PyTorch prefill's and a few decode
-steps run from the prefilled cache.  Prints one line per path: time, prompt tokens/s, time per launch.  The two
+steps run from the prefilled cache.  Prints one line per path: time, prompt tokens/s, time per chunk.  The two
 paths round at different points, and a random-weight network amplifies that from layer to layer (rel-L2 of the key
 rows between any two bf16 implementations: 2e-4 at layer 0, 5e-2 at layer 31); parity is what the tests check
 against the oracle on small models, this program measures time."""
@@ -57,8 +57,8 @@ def main():
         eng.vpool.zero_()
         first, dt = timed(lambda: pre.prefill(prompt), args.reps)
         n = (T + chunk - 1) // chunk
-        line = (f"megakernel, chunk {chunk:3d}: {dt * 1e3:8.1f} ms  {T / dt:9.0f} prompt tokens/s  first id {first}  "
-                f"{n} launches, {dt * 1e3 / n:.2f} ms each")
+        line = (f"stages, chunk {chunk:3d}    : {dt * 1e3:8.1f} ms  {T / dt:9.0f} prompt tokens/s  first id {first}  "
+                f"{n} chunks, {dt * 1e3 / n:.2f} ms each, {pre.launches(T)} launches")
         if k_ref is not None:
             line += f"  last layer's key rows vs PyTorch: rel-L2 {rel(eng.read_kv(cfg.n_layers - 1, T)[0], k_ref):.1e}"
         print(line, flush=True)
