@@ -340,8 +340,9 @@ __global__ void __launch_bounds__(kGemmThreads, 2) stage_gemm(const __grid_const
       const int team = kEpiThreads / teams, tt = t & (team - 1), row = t & 127;
       for (int i = t / team; i < n_ch; i += teams) {
         const int st = i % n_ring;
-        if (!wait.warp_wait(&sh.full[st], (uint32_t)(i / n_ring) & 1u, 2, i)) break;
-        if (i >= 2 && !wait.warp_wait(&sh.stg_empty[i & 1], (uint32_t)((i >> 1) - 1) & 1u, 2, i)) break;
+        const bool seen = wait(&sh.full[st], (uint32_t)(i / n_ring) & 1u, 2, i) &&
+                          (i < 2 || wait(&sh.stg_empty[i & 1], (uint32_t)((i >> 1) - 1) & 1u, 2, i));
+        if (!__all_sync(0xffffffffu, seen)) break;      // as in warp_wait, one vote for both
         uint8_t* dst = staging + (i & 1) * (kBlk * kKc * 2);
         const uint8_t* src = ring + st * stage_bytes + xbytes;
         if (row < N) {
