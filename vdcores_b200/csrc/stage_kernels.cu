@@ -10,8 +10,8 @@
 // 128256-row vocabulary projection at 3 rows).
 //
 // Measured against the megakernel's program, two Llama-3.1-8B-shaped layers and a small vocabulary (B200): 3 rows at
-// 1000 positions 416 -> 244 us, 32 rows with e4m3 weights 759 -> 327, 64 rows at 2100 positions 929 -> 418, 128 rows
-// 1024 -> 396, a 2048-token prompt 15.9 -> 4.8 ms.
+// 1000 positions 416 -> 247 us, 32 rows with e4m3 weights 759 -> 336, 64 rows at 2100 positions 929 -> 427, 128 rows
+// 1024 -> 405, a 2048-token prompt 15.9 -> 5.1 ms (up to 4 % less from one GPU to another).
 #include "mk_umma.cuh"
 
 #include "../../include/vdcores.h"
