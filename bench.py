@@ -426,7 +426,7 @@ def run_prefill(eng, prompt, on_device):
         dt = time.perf_counter() - t0
         return first, {"impl": "megakernel, one prompt position per launch (the decode program)", "prompt_tokens": T,
                        "ms": dt * 1e3, "tokens_per_s": T / dt, "launches": T}
-    # the prompt goes through the stage kernels: 128 positions per list of stages into this engine's own pools
+    # the prompt goes through the stage kernels into this engine's own pools
     from vdcores_b200.prefill import PrefillEngine
     pre = PrefillEngine(eng, chunk=128).adopt_weights()
     pre.prefill(prompt)                          # first call: one-time set-up of the kernel
@@ -438,7 +438,7 @@ def run_prefill(eng, prompt, on_device):
     launches = pre.launches(T)
     del pre
     torch.cuda.empty_cache()
-    return first, {"impl": "stage kernels, 128 prompt positions per list of stages", "prompt_tokens": T, "ms": dt * 1e3,
+    return first, {"impl": "stage kernels, a prompt's positions through a layer together (up to 2048)", "prompt_tokens": T, "ms": dt * 1e3,
                    "tokens_per_s": T / dt, "launches": launches}
 
 

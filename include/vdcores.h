@@ -68,7 +68,7 @@ int vdc_launch_async_full(int num_sms, int insts_per_sm, const void* compute_ins
                           const void* tma_descs, int* bars, const int* bars_init, uint64_t* profile, uint64_t stream,
                           uint64_t timeout_ns);
 
-/* One stage of a batched decode step or of a prefill chunk (2..128 rows), run as a kernel of its own.
+/* One stage of a batched decode step or of a prefill chunk (2..128 rows) or of a whole prompt, run as a kernel of its own.
  *   kind VDC_STAGE_GEMM: projection of the k-chunk-major rows `x` [Bpad, K] with the M x K weights `w` (blocks of
  *     VDC_STAGE_BLOCK rows; wfmt 0 bf16, 1 e4m3, 2 NVFP4, fp32 per-row `scales` for the last two); every block's K is
  *     shared by `splits` CTAs of one cluster.  `w` is read while the stage in front still runs (and while what the stream
@@ -88,8 +88,20 @@ int vdc_launch_async_full(int num_sms, int insts_per_sm, const void* compute_ins
  *     norm_w
  *   kind VDC_STAGE_ADVANCE: keys -> next tokens, token log, state blocks moved on by one position
  *   kind VDC_STAGE_COPY: M * K bytes from x to out
+ * The stages of a prompt whose rows (Bpad of them, a multiple of 128 up to VDC_WIDE_ROWS) go through a layer together read
+ * one block `state` of int32 words: VDC_WIDE_POS the first row's position, VDC_WIDE_N the rows that exist, and at
+ * VDC_ST_PAGETABLE the page table.  Their rows lie in sub-matrices of 128, each k-chunk-major.
+ *   kind VDC_STAGE_WIDE_EMBED: rows of the table `w` (M x K) for the ids `log` to hid
+ *   kind VDC_STAGE_WIDE_GEMM: projection of x [Bpad, K]; tiles of `group` (1, 2) sub-matrices by `n_kv` weight rows (16..256),
+ *     K shared by `splits` tiles (vdc_wide_tiles chooses all three).  mode VDC_STAGE_SUMS: fp32 sums to
+ *     out [splits][M / 4][Bpad][4]; VDC_STAGE_SILU: as above, splits 1
+ *   kind VDC_STAGE_WIDE_HEADS: what VDC_STAGE_QKV does, from the sums `x` of `splits` splits
+ *   kind VDC_STAGE_WIDE_ATTN: as VDC_STAGE_ATTN_PREFILL
+ *   kind VDC_STAGE_WIDE_NORM: hid += the sums x (0: none), then out (0: not wanted) = hid RMS-normalised with norm_w
+ *   kind VDC_STAGE_WIDE_TAIL: rows M .. M + B - 1 of x, the last one repeated, to hid [Bpad 16..128, K], squares to stats_out
  * A token id outside the table, and a row without a key (none of its logits is a number), are reported as VDC_ERR_TOKEN and
- * id 0 is taken.  While an error is unread, EMBED, GEMM and ADVANCE stages write nothing.
+ * id 0 is taken.  While an error is unread, EMBED, GEMM and ADVANCE stages (and the prompt's HEADS, NORM and TAIL) write
+ * nothing.
  * Pointers are device addresses; 0 where a stage has no use for one. */
 typedef struct {
   int32_t kind, mode, wfmt, B, Bpad, M, K, splits;
@@ -113,6 +125,11 @@ int vdc_launch_stages_limited(const vdc_stage* stages, int n, int max_ctas, uint
 /* Checks the stages as a launch does, needs no GPU: *launches = what vdc_launch_stages_limited enqueues (a copy counts as
  * one), *largest = the most CTAs of one launch. */
 int vdc_count_stage_launches(const vdc_stage* stages, int n, int max_ctas, int* launches, int* largest);
+
+/* Tile of the wide projection of `rows` rows (a multiple of 128) by an M x K matrix of format wfmt on `sms` SMs, the one with
+ * the least estimated time: out = {sub-matrices of rows (stage field group), weight rows (n_kv), K-splits (splits)}; whole
+ * non-zero: K is not split.  Needs no GPU. */
+int vdc_wide_tiles(int rows, int M, int K, int wfmt, int sms, int whole, int* out);
 
 /* Synchronises `stream` and copies the device status block to *status; returns
  * its code.  Clears the block when `clear` is non-zero. */

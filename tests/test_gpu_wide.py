@@ -1,0 +1,84 @@
+"""The stages of a whole prompt (csrc/wide_kernels.cu): the projection at the edges of its tiles against an fp32 matmul, and
+prompts whose rows go through a layer together against the same prompts chunk by chunk."""
+import pytest
+import torch
+
+from tests.test_gpu_stages import rel, seeded, weights
+
+pytestmark = pytest.mark.gpu
+BF16 = torch.bfloat16
+
+
+def _rows(x):
+    """[R, K] -> sub-matrices of 128 rows, each k-chunk-major"""
+    from vdcores_b200.batch import pack_kc
+    return torch.cat([pack_kc(x[r:r + 128]) for r in range(0, x.shape[0], 128)])
+
+
+@pytest.mark.parametrize("fmt", ["bf16", "fp8", "nvfp4"])
+@pytest.mark.parametrize("R,M,K,subs,cols,splits", [
+    (128, 16, 64, 1, 16, 1),            # the smallest tile, one chunk
+    (128, 272, 1024, 1, 48, 3),         # tiles across a block's edge, the last block and tile smaller, uneven K ranges
+    (384, 400, 512, 2, 240, 2),         # a last row tile of one sub-matrix; tiles over three blocks
+    (256, 4096, 1024, 2, 256, 1),
+    (640, 6144, 2048, 2, 176, 1),       # several tiles per CTA
+    (2048, 1024, 4096, 1, 80, 8)])      # both accumulators of one-sub-matrix tiles in turn, many times
+def test_prompt_projection(cuda_device, fmt, R, M, K, subs, cols, splits):
+    from vdcores_b200 import isa, runtime
+    dev = cuda_device
+    x = seeded((R, K), 1).to(dev)
+    w, sc, ref = weights(M, K, fmt, dev)
+    xd = _rows(x)
+    sums = torch.full((splits, M // 4, R, 4), float("nan"), device=dev)
+    act = torch.full((R * M // 2,), float("nan"), device=dev, dtype=BF16)
+    kw = dict(kind=isa.STAGE_WIDE_GEMM, wfmt={"bf16": 0, "fp8": 1, "nvfp4": 2}[fmt], Bpad=R, M=M, K=K, group=subs, n_kv=cols,
+              w=w.data_ptr(), scales=sc.data_ptr() if sc is not None else 0, x=xd.data_ptr())
+    arr = (runtime.Stage * 2)(runtime.Stage(mode=isa.STAGE_SUMS, splits=splits, out=sums.data_ptr(), **kw),
+                              runtime.Stage(mode=isa.STAGE_SILU, splits=1, out=act.data_ptr(), **kw))
+    s = torch.cuda.current_stream(dev).cuda_stream
+    runtime.launch_stages(arr, s, 500_000_000)
+    runtime.read_status(s)
+    y = x.double() @ ref.to(dev).double().t()
+    got = sums.sum(0).permute(1, 0, 2).reshape(R, M)
+    # the tensor cores add K / 16 products of 16 to an fp32 sum, each addition exact to 2^-23 of it (twice that where cut off)
+    assert rel(got, y) < 2 * K / 16 * 2.0 ** -23 + 1e-6
+    g, u = y[:, 0::2].float().to(BF16).float(), y[:, 1::2].float().to(BF16).float()
+    want = torch.nn.functional.silu(g).to(BF16).float() * u
+    rows = torch.cat([a.view(M // 16, 16, 8, 8).permute(1, 2, 0, 3).reshape(128, M // 2) for a in act.view(R // 128, -1)])
+    assert rel(rows, want) < 4e-3       # three bf16 roundings of 2^-9 each
+
+
+@pytest.mark.parametrize("kind,fmt,T,chunk,perm", [("llama", "bf16", 77, 64, 3), ("llama", "bf16", 129, 128, None),
+                                                   ("qwen3", "bf16", 300, 48, 5), ("llama", "fp8", 257, 16, None),
+                                                   ("qwen3_1k", "nvfp4", 515, 128, 1), ("llama", "bf16", 2200, 120, 2)])
+def test_prompt_in_one_pass_agrees_with_its_chunks(cuda_device, kind, fmt, T, chunk, perm):
+    """Ragged prompts, shuffled pages, chunks that do not divide 128, prompts of two passes: cache rows of every layer, the last
+    chunk's hidden rows (its repeated ones too) and the first id."""
+    from tests.helpers import engine_config, small_cfg
+    from vdcores_b200.decode import DecodeEngine
+    from vdcores_b200.prefill import PrefillEngine
+    dev = cuda_device
+    cfg = engine_config(small_cfg(kind))
+    eng = DecodeEngine(cfg, (T + 70) // 64 * 64, device=dev, wkind=fmt, page_perm_seed=perm)
+    eng.init_random_weights(3)
+    prompt = torch.randint(0, cfg.vocab, (T,), generator=torch.Generator().manual_seed(T))
+    pre = PrefillEngine(eng, chunk=chunk, timeout_ns=500_000_000).adopt_weights()
+    got = []
+    for wide in (True, False):
+        if not wide:
+            pre._wide = None
+        assert pre._goes_wide(T) == wide
+        eng.kpool.zero_()
+        eng.vpool.zero_()
+        first = pre.prefill(prompt)
+        top = torch.topk(pre.read_hidden(pre.hidden)[(T - 1) % chunk].float(), 1)
+        got.append((first, pre.read_hidden(pre.hidden).clone(), eng.kpool.clone(), eng.vpool.clone(), top))
+    (f1, h1, k1, v1, _), (f0, h0, k0, v0, _) = got
+    assert bool(torch.isfinite(h1.float()).all())
+    for a, b in ((h1, h0), (k1[1:], k0[1:]), (v1[1:], v0[1:])):
+        assert rel(a, b) < 1e-2          # sums in other orders, rounded to bf16 through two or three layers
+    for a, b in ((k1[0], k0[0]), (v1[0], v0[0])):
+        assert rel(a, b) < 2e-3          # one projection behind exact inputs: a rounding here and there
+        rows = (a.float() - b.float()).flatten(0, 2).norm(dim=1) / b.float().flatten(0, 2).norm(dim=1).clamp_min(1e-6)
+        assert float(rows.max()) < 1e-2
+    assert bool(((k1 == 0) == (k0 == 0)).float().mean() > 0.999)     # nothing written past the prompt

@@ -19,6 +19,10 @@ extern "C" cudaError_t vdc_megakernel_launch(int num_sms, const void* cinsts, co
 extern "C" cudaError_t vdc_stage_prepare();
 extern "C" cudaError_t vdc_stage_launch(const vdc_stage* s, int max_ctas, int* front, vdc_status* status,
                                         uint64_t timeout_ns, cudaStream_t stream);
+extern "C" cudaError_t vdc_wide_prepare();
+extern "C" void vdc_wide_choose(int rows, int M, int K, int wfmt, int sms, int whole, int* out);
+extern "C" int vdc_wide_grid(const vdc_stage* s, int sms, int* tiles);
+extern "C" cudaError_t vdc_wide_launch(const vdc_stage* s, int sms, vdc_status* status, uint64_t timeout_ns, cudaStream_t stream);
 extern "C" void vdc_stage_slices(const vdc_stage* s, int max_ctas, int* launches, int* largest);
 
 namespace {
@@ -91,6 +95,7 @@ int vdc_init(void) {
   e = vdc_megakernel_prepare();
   if (e != cudaSuccess) return fail_cuda(e, "cudaFuncSetAttribute(MaxDynamicSharedMemorySize)");
   e = vdc_stage_prepare();
+  if (e == cudaSuccess) e = vdc_wide_prepare();
   if (e != cudaSuccess) return fail_cuda(e, "cudaFuncSetAttribute(stage kernels)");
   vdc_status* st = nullptr;
   e = cudaMalloc(&st, sizeof(vdc_status));
@@ -142,7 +147,43 @@ int vdc_launch_async_full(int num_sms, int insts_per_sm, const void* compute_ins
 
 // Everything a stage's kernel takes for granted.  Alignments are those of its widest access: 16 bytes for rows, pages and
 // hidden or output pieces, 8 for the rotation table and the keys, 4 for the rest.
+static bool is_wide(const vdc_stage& s) { return s.kind >= VDC_STAGE_WIDE_EMBED && s.kind <= VDC_STAGE_WIDE_TAIL; }
+
+// The same for the stages of a whole prompt: Bpad rows in sub-matrices of 128.
+static const char* check_wide(const vdc_stage& s) {
+  auto al16 = [](uint64_t p) { return (p & 15) == 0; };
+  auto al4 = [](uint64_t p) { return (p & 3) == 0; };
+  if (s.kind == VDC_STAGE_WIDE_TAIL)
+    return s.B >= 1 && s.B <= 128 && s.Bpad >= s.B && s.Bpad <= 128 && s.Bpad % 16 == 0 && s.M >= 0 && s.K > 0 && s.K % 8 == 0 && s.x &&
+                   s.hid && s.stats_out && s.state && al16(s.x) && al16(s.hid) && al4(s.stats_out) && al4(s.state) ? nullptr : "tail stage: bad argument";
+  if (s.Bpad < 128 || s.Bpad > VDC_WIDE_ROWS || s.Bpad % 128) return "prompt stage: rows out of range";
+  switch (s.kind) {
+    case VDC_STAGE_WIDE_EMBED:
+      return s.K > 0 && s.K % 8 == 0 && s.M >= 0 && s.w && s.hid && s.state && s.log && al16(s.w) && al16(s.hid) && al4(s.state) &&
+                     al4(s.log) ? nullptr : "prompt embedding stage: bad argument";
+    case VDC_STAGE_WIDE_NORM:
+      return s.K > 0 && s.K % 8 == 0 && s.hid && al16(s.hid) && al16(s.x) && (!s.x || s.splits >= 1) && al16(s.out) &&
+                     (!s.out || (s.norm_w && al16(s.norm_w))) ? nullptr : "prompt norm stage: bad argument";
+    case VDC_STAGE_WIDE_HEADS:
+      return s.group >= 1 && s.n_kv >= 1 && s.M == s.n_kv * (s.group + 2) * VDC_HEAD_DIM && s.splits >= 1 && s.x && s.out && s.state &&
+                     s.rope && s.kpool && s.vpool && al16(s.x) && al4(s.out) && al4(s.state) && (s.rope & 7) == 0 && al4(s.qk_norm) &&
+                     al16(s.kpool) && al16(s.vpool) ? nullptr : "prompt heads stage: bad argument";
+    case VDC_STAGE_WIDE_ATTN:
+      return (s.group == 4 || s.group == 8) && s.n_kv >= 1 && s.n_kv <= 65535 && s.n_pages >= 1 && s.state && s.q && s.out && s.kpool &&
+                     s.vpool && al4(s.state) && al16(s.q) && al16(s.out) && al16(s.kpool) && al16(s.vpool) &&
+                     (s.splits == 1 || s.splits == 2 || s.splits == 4 || s.splits == 8) ? nullptr : "prompt attention stage: bad argument";
+    default: break;
+  }
+  if (s.wfmt < 0 || s.wfmt > 2 || s.M < 16 || s.M % 16 || s.K < 64 || s.K % 64 || s.splits < 1 || s.splits > s.K / 64 ||
+      (s.group != 1 && s.group != 2) || s.n_kv < 16 || s.n_kv > 256 || s.n_kv % 16)
+    return "prompt projection stage: bad shape";
+  if (s.mode != VDC_STAGE_SUMS && (s.mode != VDC_STAGE_SILU || s.splits != 1)) return "prompt projection stage: unknown mode";
+  return s.w && s.x && s.out && al16(s.w) && al16(s.x) && al16(s.out) && al16(s.scales) && (!s.wfmt || s.scales)
+             ? nullptr : "prompt projection stage: null or misaligned pointer";
+}
+
 static const char* check_stage(const vdc_stage& s) {
+  if (is_wide(s)) return check_wide(s);
   auto pow2 = [](int v) { return v > 0 && (v & (v - 1)) == 0; };
   auto al16 = [](uint64_t p) { return (p & 15) == 0; };
   auto al8 = [](uint64_t p) { return (p & 7) == 0; };
@@ -192,6 +233,7 @@ static const char* check_stages(const vdc_stage* stages, int n, int max_ctas) {
   if (max_ctas < 0) return "the number of CTAs must not be negative";
   for (int i = 0; i < n; ++i) {
     if (const char* why = check_stage(stages[i])) return why;
+    if (max_ctas && is_wide(stages[i])) return "prompt stage: takes all SMs";
     const bool shared = stages[i].kind == VDC_STAGE_GEMM || stages[i].kind == VDC_STAGE_ATTN || stages[i].kind == VDC_STAGE_ATTN_PREFILL;
     if (max_ctas && shared && stages[i].splits > max_ctas) return "stage: more splits than CTAs are allowed";
   }
@@ -206,7 +248,9 @@ int vdc_launch_stages_limited(const vdc_stage* stages, int n, int max_ctas, uint
   if (timeout_ns == 0) timeout_ns = 2000000000ull;
   int front = -1;      // CTAs of the launch in front of the next one
   for (int i = 0; i < n; ++i) {
-    cudaError_t e = vdc_stage_launch(&stages[i], max_ctas, &front, g_status[dev], timeout_ns, reinterpret_cast<cudaStream_t>(stream));
+    cudaError_t e = is_wide(stages[i]) && stages[i].kind != VDC_STAGE_WIDE_ATTN
+                        ? vdc_wide_launch(&stages[i], g_sm_count[dev], g_status[dev], timeout_ns, reinterpret_cast<cudaStream_t>(stream))
+                        : vdc_stage_launch(&stages[i], max_ctas, &front, g_status[dev], timeout_ns, reinterpret_cast<cudaStream_t>(stream));
     if (e != cudaSuccess) return fail_cuda(e, "stage launch");
   }
   return VDC_OK;
@@ -217,11 +261,23 @@ int vdc_count_stage_launches(const vdc_stage* stages, int n, int max_ctas, int* 
   if (const char* why = check_stages(stages, n, max_ctas)) return fail_arg(why);
   *launches = *largest = 0;
   for (int i = 0; i < n; ++i) {
-    int k, c;
-    vdc_stage_slices(&stages[i], max_ctas, &k, &c);
+    int k, c, tiles;
+    if (is_wide(stages[i]) && stages[i].kind != VDC_STAGE_WIDE_ATTN) {
+      k = 1;
+      c = vdc_wide_grid(&stages[i], VDC_MAX_SMS, &tiles);
+    } else {
+      vdc_stage_slices(&stages[i], max_ctas, &k, &c);
+    }
     *launches += k;
     if (c > *largest) *largest = c;
   }
+  return VDC_OK;
+}
+
+int vdc_wide_tiles(int rows, int M, int K, int wfmt, int sms, int whole, int* out) {
+  if (!out || rows < 128 || rows > VDC_WIDE_ROWS || rows % 128 || M < 16 || K < 64 || wfmt < 0 || wfmt > 2 || sms < 1)
+    return fail_arg("wide tile: bad shape");
+  vdc_wide_choose(rows, M, K, wfmt, sms, whole, out);
   return VDC_OK;
 }
 

@@ -52,7 +52,17 @@
 #define VDC_STAGE_RESID 1
 #define VDC_STAGE_SILU 2
 #define VDC_STAGE_ARGMAX 3
+#define VDC_STAGE_SUMS 4
 #define VDC_STAGE_BLOCK 128
+#define VDC_STAGE_WIDE_EMBED 8   // the stages of a prompt whose rows go through a layer together
+#define VDC_STAGE_WIDE_GEMM 9
+#define VDC_STAGE_WIDE_HEADS 10
+#define VDC_STAGE_WIDE_ATTN 11
+#define VDC_STAGE_WIDE_NORM 12
+#define VDC_STAGE_WIDE_TAIL 13
+#define VDC_WIDE_ROWS 2048       // most rows of one pass
+#define VDC_WIDE_POS 0           // words of the block those stages read: first position, rows; page table at VDC_ST_PAGETABLE
+#define VDC_WIDE_N 1
 
 // X(name, value)
 #define VDC_MEMORY_OPS(X)                                                              \

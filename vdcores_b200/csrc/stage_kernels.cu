@@ -11,10 +11,8 @@
 //
 // Measured against the megakernel's program, two Llama-3.1-8B-shaped layers and a small vocabulary (B200): 3 rows at
 // 1000 positions 416 -> 247 us, 32 rows with e4m3 weights 759 -> 336, 64 rows at 2100 positions 929 -> 427, 128 rows
-// 1024 -> 405, a 2048-token prompt 15.9 -> 5.1 ms (up to 4 % less from one GPU to another).
-#include "mk_umma.cuh"
-
-#include "../../include/vdcores.h"
+// 1024 -> 405 (up to 4 % less from one GPU to another).
+#include "mk_stage.cuh"
 
 namespace vdc {
 
@@ -27,93 +25,6 @@ constexpr int kEpiThreads = 256;
 // other is in its prologue or epilogue, and the next stage's CTAs move in while the last ones of this stage finish.
 constexpr int kGemmSmem = 110 * 1024;
 constexpr int kCol4 = kBlk / 4;         // groups of four columns in the fp32 exchange tile
-
-// ------------------------------------------------------------------------- //
-// helpers
-// ------------------------------------------------------------------------- //
-__device__ __forceinline__ void grid_dep_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
-__device__ __forceinline__ void grid_dep_launch() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
-__device__ __forceinline__ void cluster_arrive() { asm volatile("barrier.cluster.arrive.release;" ::: "memory"); }
-__device__ __forceinline__ void cluster_wait() { asm volatile("barrier.cluster.wait.acquire;" ::: "memory"); }
-__device__ __forceinline__ uint32_t cluster_rank() {
-  uint32_t r;
-  asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
-  return r;
-}
-__device__ __forceinline__ uint32_t peer_smem(uint32_t saddr, uint32_t rank) {
-  uint32_t a;
-  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(a) : "r"(saddr), "r"(rank));
-  return a;
-}
-__device__ __forceinline__ float4 ld_cluster4(uint32_t a) {
-  float4 v;
-  asm volatile("ld.shared::cluster.v4.f32 {%0,%1,%2,%3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "r"(a) : "memory");
-  return v;
-}
-__device__ __forceinline__ void st_cluster4(uint32_t a, uint32_t x, uint32_t y, uint32_t z, uint32_t w) {
-  asm volatile("st.shared::cluster.v4.b32 [%0], {%1,%2,%3,%4};" ::"r"(a), "r"(x), "r"(y), "r"(z), "r"(w) : "memory");
-}
-__device__ __forceinline__ void st_shared4(uint32_t a, uint32_t x, uint32_t y, uint32_t z, uint32_t w) {
-  asm volatile("st.shared.v4.b32 [%0], {%1,%2,%3,%4};" ::"r"(a), "r"(x), "r"(y), "r"(z), "r"(w) : "memory");
-}
-__device__ __forceinline__ float ld_cluster1(uint32_t a) {
-  float v;
-  asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(v) : "r"(a) : "memory");
-  return v;
-}
-
-// The first error since the host last looked goes to the status block.
-static __device__ void report(vdc_status* status, int code, int kind, int role, int at, int aux) {
-  if (atomicCAS(&status->abort, 0, 1) == 0) {
-    status->code = code;
-    status->sm = (int)blockIdx.x;
-    status->role = role;
-    status->pc = at;
-    status->opcode = kind;
-    status->bar = -1;
-    status->aux = aux;
-    __threadfence();
-  }
-}
-
-// Bounded wait on an mbarrier of this CTA: after `timeout_ns` the status block says so, the CTA's `fail` word stops
-// every other role, and all of them leave through the ordinary exit (cluster barriers and tensor memory included).
-__device__ __noinline__ bool stage_wait_slow(uint64_t* bar, uint32_t parity, volatile int* fail, vdc_status* status,
-                                             uint64_t timeout_ns, int kind, int role, int at) {
-  const uint64_t t0 = globaltimer_ns();
-  for (uint32_t it = 1;; ++it) {
-    if (mbar_try_wait(bar, parity)) return true;
-    if ((it & 15u) != 0) continue;
-    if (*fail) return false;
-    if (globaltimer_ns() - t0 > timeout_ns) {
-      report(status, VDC_ERR_TIMEOUT, kind, role, at, (int)it);
-      *fail = 1;
-      return false;
-    }
-  }
-}
-
-struct Waiter {
-  volatile int* fail;
-  vdc_status* status;
-  uint64_t timeout_ns;
-  int kind;
-  __device__ __forceinline__ bool operator()(uint64_t* bar, uint32_t parity, int role, int at) const {
-    return mbar_try_wait(bar, parity) || stage_wait_slow(bar, parity, fail, status, timeout_ns, kind, role, at);
-  }
-  // The same for a whole warp: all 32 lanes leave together and with one answer, true only if every lane saw the barrier.
-  // What follows such a wait (ldmatrix, mma, full-mask shuffles, one arrival for the warp) needs all lanes.
-  __device__ __forceinline__ bool warp_wait(uint64_t* bar, uint32_t parity, int role, int at) const {
-    return __all_sync(0xffffffffu, (*this)(bar, parity, role, at));
-  }
-  // copies that may still be in flight after a wait was given up get a bounded time to land
-  __device__ __forceinline__ void drain() const {
-    if (*fail) {
-      const uint64_t t0 = globaltimer_ns();
-      while (globaltimer_ns() - t0 < 200000ull) __nanosleep(1000);
-    }
-  }
-};
 
 // ------------------------------------------------------------------------- //
 // projection: D[b, n] = sum_k X[b, k] W[n, k] for one block of weight rows, K shared by the CTAs of a cluster
@@ -129,9 +40,6 @@ struct GemmShared {
   float ssq[128];
   unsigned long long key[128];
 };
-
-// Bytes of a chunk of n weight rows x 64 inputs as stored: bf16, e4m3, or e2m1 pairs with one e4m3 scale per 16.
-__host__ __device__ constexpr int chunk_bytes(int wfmt, int n) { return wfmt == 0 ? n * 128 : wfmt == 1 ? n * 64 : n * 36; }
 
 // One ring stage: the rows' chunk, then the weights' chunk.
 __host__ __device__ constexpr int stage_size(int wfmt, int bpad) {
@@ -162,25 +70,10 @@ __device__ __forceinline__ void sum8(float (&v)[8], const uint8_t* tile, int spl
     v[4] += c.x; v[5] += c.y; v[6] += c.z; v[7] += c.w;
   }
 }
-__device__ __forceinline__ uint4 pack8(const float (&v)[8]) {
-  return make_uint4(pack_bf16x2(v[0], v[1]), pack_bf16x2(v[2], v[3]), pack_bf16x2(v[4], v[5]), pack_bf16x2(v[6], v[7]));
-}
-__device__ __forceinline__ void scale8(float (&v)[8], const float* sc) {
-  if (sc != nullptr) {
-    const float4 a = __ldg(reinterpret_cast<const float4*>(sc)), c = __ldg(reinterpret_cast<const float4*>(sc) + 1);
-    v[0] *= a.x; v[1] *= a.y; v[2] *= a.z; v[3] *= a.w;
-    v[4] *= c.x; v[5] *= c.y; v[6] *= c.z; v[7] *= c.w;
-  }
-}
-
-// One head of the QKV projection, one warp per row: optional RMSNorm over the head, half-rotation, then a query row to
-// the query matrix or a key / value row to the row's cache page.  Every product is rounded as a bf16 tensor expression
-// rounds it.  Lane i holds dims 2i, 2i+1 and their rotation partners 64 further.
+// One head of the QKV projection, one warp per row: the sums over the cluster's K-ranges, then the rest of the head.
 __device__ __forceinline__ void qkv_head(const vdc_stage& s, const uint8_t* tile, int splits, int nb, int bl, int b, int block,
                                          int lane) {
-  constexpr int D = VDC_HEAD_DIM;
-  const int G = s.group, kvh = block / (G + 2), part = block % (G + 2), n0 = block * kBlk;
-  const int i0 = lane * 2;
+  const int n0 = block * kBlk, i0 = lane * 2;
   float x[4] = {0.f, 0.f, 0.f, 0.f};
   for (int r = 0; r < splits; ++r) {
     const uint8_t* p = tile + (size_t)((r * kCol4 + (i0 >> 2)) * (nb + 1) + bl) * 16 + (i0 & 3) * 4;
@@ -193,47 +86,12 @@ __device__ __forceinline__ void qkv_head(const vdc_stage& s, const uint8_t* tile
     const float2 hi = __ldg(reinterpret_cast<const float2*>(scales + n0 + i0 + 64));
     x[0] *= lo.x; x[1] *= lo.y; x[2] *= hi.x; x[3] *= hi.y;
   }
-#pragma unroll
-  for (int j = 0; j < 4; ++j) x[j] = bf16_round(x[j]);
   const int* st = reinterpret_cast<const int*>(s.state) + (size_t)b * s.state_stride;
-  const int pos = ld_relaxed_gpu(st + VDC_ST_POS);
-  if (part <= G) {   // a query head or the key head
-    if (s.qk_norm) {
-      const float ss = warp_sum(x[0] * x[0] + x[1] * x[1] + x[2] * x[2] + x[3] * x[3]);
-      const float rs = rsqrtf(ss / (float)D + s.qk_eps);
-      const __nv_bfloat16* w = reinterpret_cast<const __nv_bfloat16*>(s.qk_norm) + (part == G ? D : 0);
-      const uint32_t wl = *reinterpret_cast<const uint32_t*>(w + i0), wh = *reinterpret_cast<const uint32_t*>(w + i0 + 64);
-      x[0] = bf16_round(bf_lo(wl) * bf16_round(x[0] * rs));
-      x[1] = bf16_round(bf_hi(wl) * bf16_round(x[1] * rs));
-      x[2] = bf16_round(bf_lo(wh) * bf16_round(x[2] * rs));
-      x[3] = bf16_round(bf_hi(wh) * bf16_round(x[3] * rs));
-    }
-    const float* rope = reinterpret_cast<const float*>(s.rope) + (size_t)pos * D;
-    const float2 cs = __ldg(reinterpret_cast<const float2*>(rope + i0));
-    const float2 sn = __ldg(reinterpret_cast<const float2*>(rope + 64 + i0));
-    const float a0 = x[0], a1 = x[1], b0 = x[2], b1 = x[3];
-    x[0] = bf16_round(a0 * cs.x) - bf16_round(b0 * sn.x);
-    x[1] = bf16_round(a1 * cs.y) - bf16_round(b1 * sn.y);
-    x[2] = bf16_round(b0 * cs.x) + bf16_round(a0 * sn.x);
-    x[3] = bf16_round(b1 * cs.y) + bf16_round(a1 * sn.y);
-  }
-  const uint32_t lo = pack_bf16x2(x[0], x[1]), hi = pack_bf16x2(x[2], x[3]);
-  if (part < G) {
-    uint32_t* dst = reinterpret_cast<uint32_t*>(s.out) + ((size_t)b * s.n_kv * G + (size_t)kvh * G + part) * (D / 2) + lane;
-    dst[0] = lo;
-    dst[32] = hi;
-    return;
-  }
   // rows past a prompt's end repeat its last position: the first of them writes the cache row, since their sums of squares
   // (atomics) may differ in the last bit
   const int new_row = ld_relaxed_gpu(st + VDC_ST_NEWROW);
-  if (b > 0 && ld_relaxed_gpu(st - s.state_stride + VDC_ST_NEWROW) == new_row) return;
-  // the row's 16-byte pieces lie at (piece XOR (row mod 8)), the page-row order the attention reads
-  const int sw = pos & 7;
-  uint8_t* row = reinterpret_cast<uint8_t*>(part == G ? s.kpool : s.vpool) + (size_t)kvh * (VDC_KV_PAGE * D * 2) +
-                 (size_t)new_row * (D * 2);
-  *reinterpret_cast<uint32_t*>(row + (((i0 >> 3) ^ sw) << 4) + (i0 & 7) * 2) = lo;
-  *reinterpret_cast<uint32_t*>(row + (((8 + (i0 >> 3)) ^ sw) << 4) + (i0 & 7) * 2) = hi;
+  const bool first = b == 0 || ld_relaxed_gpu(st - s.state_stride + VDC_ST_NEWROW) != new_row;
+  head_row(s, x, b, block, lane, ld_relaxed_gpu(st + VDC_ST_POS), new_row, first);
 }
 
 template <int kFmt>
@@ -335,8 +193,6 @@ __global__ void __launch_bounds__(kGemmThreads, 2) stage_gemm(const __grid_const
   } else {
     const int t = tid - 64;
     if (kFmt != 0) {
-      // bf16 pieces of the tensor cores' operand layout, 16 weights of a row at a time (exact for e4m3 and for e2m1 code
-      // times block scale)
       const int team = kEpiThreads / teams, tt = t & (team - 1), row = t & 127;
       for (int i = t / team; i < n_ch; i += teams) {
         const int st = i % n_ring;
@@ -348,30 +204,7 @@ __global__ void __launch_bounds__(kGemmThreads, 2) stage_gemm(const __grid_const
         if (row < N) {
 #pragma unroll 2
           for (int g16 = tt >> 7; g16 < kKc / 16; g16 += team >> 7) {
-            uint32_t o[8];
-            if (kFmt == 1) {
-              const uint4 v = lds128(src + (g16 * N + row) * 16);
-              const uint32_t wv[4] = {v.x, v.y, v.z, v.w};
-#pragma unroll
-              for (int j = 0; j < 4; ++j) {
-                const float2 lo = e4m3x2_to_float2(wv[j] & 0xFFFFu), hi = e4m3x2_to_float2(wv[j] >> 16);
-                o[2 * j] = pack_bf16x2(lo.x, lo.y);
-                o[2 * j + 1] = pack_bf16x2(hi.x, hi.y);
-              }
-            } else {
-              const uint8_t* g = src + g16 * 9 * N;
-              const uint2 cv = *reinterpret_cast<const uint2*>(g + row * 8);
-              const __half_raw hr = __nv_cvt_fp8_to_halfraw((__nv_fp8_storage_t)g[8 * N + row], __NV_E4M3);
-              const __half2 sc = __half2half2(*reinterpret_cast<const __half*>(&hr));
-              const uint32_t cw[2] = {cv.x, cv.y};
-#pragma unroll
-              for (int j = 0; j < 8; ++j) {
-                const float2 f = __half22float2(__hmul2(e2m1x2_to_half2((cw[j >> 2] >> (8 * (j & 3))) & 0xFFu), sc));
-                o[j] = pack_bf16x2(f.x, f.y);
-              }
-            }
-            *reinterpret_cast<uint4*>(dst + ((2 * g16) * N + row) * 16) = make_uint4(o[0], o[1], o[2], o[3]);
-            *reinterpret_cast<uint4*>(dst + ((2 * g16 + 1) * N + row) * 16) = make_uint4(o[4], o[5], o[6], o[7]);
+            widen16<kFmt>(dst, src, N, row, g16);
           }
         }
         fence_proxy_async_smem();
@@ -526,6 +359,12 @@ __device__ __forceinline__ void mma_16816(float (&d)[4], uint32_t a0, uint32_t a
                                           uint32_t b1) {
   asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
                : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3]) : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
+}
+// 2^x as one instruction: results below the smallest normal number become zero.
+__device__ __forceinline__ float exp2_ftz(float x) {
+  float y;
+  asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+  return y;
 }
 __device__ __forceinline__ uint32_t transpose8x8(uint32_t v) {
   uint32_t d;
@@ -793,6 +632,9 @@ __global__ void __launch_bounds__(kAttnThreads, 2) stage_attn(const __grid_const
 // ------------------------------------------------------------------------- //
 constexpr int kRows = 64;
 
+// kWide: the rows are a whole prompt's (up to VDC_WIDE_ROWS), their number and first position in the block `state`; the tiles
+// with the longest walks start first.
+template <bool kWide>
 __global__ void __launch_bounds__(kAttnThreads, 2) stage_attn_prefill(const __grid_constant__ vdc_stage s, int first_unit, vdc_status* status,
                                                                       uint64_t timeout_ns) {
   extern __shared__ uint8_t dyn[];
@@ -800,13 +642,17 @@ __global__ void __launch_bounds__(kAttnThreads, 2) stage_attn_prefill(const __gr
   constexpr int D = VDC_HEAD_DIM;
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int splits = s.splits, rank = splits > 1 ? (int)cluster_rank() : 0;
-  const int unit = first_unit + (int)blockIdx.x / splits, h = unit % s.n_kv, G = s.group, b0 = unit / s.n_kv * (kRows / G);
+  const int* st = reinterpret_cast<const int*>(s.state);
+  const int unit = first_unit + (int)blockIdx.x / splits, h = unit % s.n_kv, G = s.group, per_tile = kRows / G;
+  const int rows = kWide ? ld_relaxed_gpu(st + VDC_WIDE_N) : s.B;
+  const int b0 = (kWide ? s.Bpad / per_tile - 1 - unit / s.n_kv : unit / s.n_kv) * per_tile;
+  if (kWide && b0 >= rows) return;
   uint8_t* ring = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(dyn) + 127) & ~(uintptr_t)127);
   const Waiter wait{&sh.fail, status, timeout_ns, s.kind};
   attn_setup(sh, tid);
-  const int* st = reinterpret_cast<const int*>(s.state);
-  auto row_b = [&](int r) { return min(b0 + r / G, s.B - 1); };
-  auto pos_of = [&](int r) { return ld_relaxed_gpu(st + (size_t)row_b(r) * s.state_stride + VDC_ST_POS); };
+  const int pos0 = ld_relaxed_gpu(st + (kWide ? VDC_WIDE_POS : VDC_ST_POS));
+  auto row_b = [&](int r) { return min(b0 + r / G, rows - 1); };
+  auto pos_of = [&](int r) { return kWide ? pos0 + row_b(r) : ld_relaxed_gpu(st + (size_t)row_b(r) * s.state_stride + VDC_ST_POS); };
   const int pos_hi = pos_of(kRows - 1), pos_lo = pos_of(0);          // the rows' positions never decrease
   const int n_pages = min(pos_hi / VDC_KV_PAGE + 1, s.n_pages);
   const int per = (n_pages + splits - 1) / splits, first = rank * per;
@@ -823,7 +669,7 @@ __global__ void __launch_bounds__(kAttnThreads, 2) stage_attn_prefill(const __gr
   if (warp == 4) {
     const size_t head_off = (size_t)h * kPageBytes;
     stream_pages(sh, wait, ring, st + VDC_ST_PAGETABLE, first, count, reinterpret_cast<const uint8_t*>(s.kpool) + head_off,
-                 reinterpret_cast<const uint8_t*>(s.vpool) + head_off, (size_t)s.n_kv * kPageBytes, ld_relaxed_gpu(st + VDC_ST_POS) / VDC_KV_PAGE, lane);
+                 reinterpret_cast<const uint8_t*>(s.vpool) + head_off, (size_t)s.n_kv * kPageBytes, pos0 / VDC_KV_PAGE, lane);
   } else {
     grid_dep_wait();
     uint32_t q[8][4];
@@ -847,53 +693,62 @@ __global__ void __launch_bounds__(kAttnThreads, 2) stage_attn_prefill(const __gr
       const int page0 = (first + i) * VDC_KV_PAGE;
       float c[8][4];
 #pragma unroll
-      for (int n = 0; n < 8; ++n) {
+      for (int n = 0; n < 8; ++n)
 #pragma unroll
         for (int j = 0; j < 4; ++j) c[n][j] = 0.f;
 #pragma unroll
-        for (int k = 0; k < 8; k += 2) {      // one load: eight positions, dims 32 (k / 2) .. + 31
+      for (int k = 0; k < 8; k += 2)
+#pragma unroll
+        for (int n = 0; n < 8; ++n) {         // one load: eight positions, dims 32 (k / 2) .. + 31
           uint32_t a[4];
           ldsm_x4(a, kb + (uint32_t)((n * 8 + lr) * 256 + (((2 * k + mi) ^ lr) << 4)));
           mma_16816(c[n], q[k][0], q[k][1], q[k][2], q[k][3], a[0], a[1]);
           mma_16816(c[n], q[k + 1][0], q[k + 1][1], q[k + 1][2], q[k + 1][3], a[2], a[3]);
         }
-      }
+      // Four instructions per score (maximum, fused scale and subtraction, exponential, sum) and nothing that only some pages
+      // need: the mask at the diagonal, the rows' rescaling when a maximum moved.  The walk is bound by instructions issued
+      // (two warps per scheduler): 2048 positions 178 -> 167 us with 1065 -> 840 per warp and page.
       float mx[2] = {-INFINITY, -INFINITY};
-      const bool edge = page0 + VDC_KV_PAGE - 1 > pos_lo;             // only pages at the diagonal need the mask
+      if (page0 + VDC_KV_PAGE - 1 > pos_lo) {
+#pragma unroll
+        for (int n = 0; n < 8; ++n)
+#pragma unroll
+          for (int j = 0; j < 4; ++j)
+            if (page0 + n * 8 + 2 * t4 + (j & 1) > pos[j >> 1]) c[n][j] = -INFINITY;
+      }
 #pragma unroll
       for (int n = 0; n < 8; ++n)
 #pragma unroll
-        for (int j = 0; j < 4; ++j) {
-          c[n][j] *= scale_log2;
-          if (edge && page0 + n * 8 + 2 * t4 + (j & 1) > pos[j >> 1]) c[n][j] = -INFINITY;
-          mx[j >> 1] = fmaxf(mx[j >> 1], c[n][j]);
-        }
+        for (int j = 0; j < 4; ++j) mx[j >> 1] = fmaxf(mx[j >> 1], c[n][j]);
       float al[2];
 #pragma unroll
       for (int j = 0; j < 2; ++j) {
         mx[j] = fmaxf(mx[j], __shfl_xor_sync(0xffffffffu, mx[j], 1));
         mx[j] = fmaxf(mx[j], __shfl_xor_sync(0xffffffffu, mx[j], 2));
-        const float mn = fmaxf(m[j], mx[j]);
-        al[j] = mn == -INFINITY ? 1.f : exp2f(m[j] - mn);
+        const float mn = fmaxf(m[j], mx[j] * scale_log2);
+        al[j] = mn == -INFINITY ? 1.f : exp2_ftz(m[j] - mn);
         m[j] = mn;
-        l[j] *= al[j];
         mx[j] = mn == -INFINITY ? 0.f : mn;                           // a row with no key here: every exponent is -inf
+      }
+      if (__any_sync(0xffffffffu, al[0] != 1.f || al[1] != 1.f)) {
+#pragma unroll
+        for (int j = 0; j < 2; ++j) l[j] *= al[j];
+#pragma unroll
+        for (int d = 0; d < 16; ++d)
+#pragma unroll
+          for (int j = 0; j < 4; ++j) o[d][j] *= al[j >> 1];
       }
       uint32_t p[8][2];
 #pragma unroll
       for (int n = 0; n < 8; ++n) {
 #pragma unroll
         for (int j = 0; j < 4; ++j) {
-          c[n][j] = exp2f(c[n][j] - mx[j >> 1]);
+          c[n][j] = exp2_ftz(fmaf(c[n][j], scale_log2, -mx[j >> 1]));
           l[j >> 1] += c[n][j];
         }
         p[n][0] = pack_bf16x2(c[n][0], c[n][1]);
         p[n][1] = pack_bf16x2(c[n][2], c[n][3]);
       }
-#pragma unroll
-      for (int d = 0; d < 16; ++d)
-#pragma unroll
-        for (int j = 0; j < 4; ++j) o[d][j] *= al[j >> 1];
 #pragma unroll
       for (int k = 0; k < 4; ++k) {            // 16 positions at a time
         const int pv = k * 16 + lr + 8 * (mi & 1);
@@ -934,9 +789,10 @@ __global__ void __launch_bounds__(kAttnThreads, 2) stage_attn_prefill(const __gr
   }
   if (warp < 4 && !failed)
     attn_merge(sh, smem_u32(rec), splits, rank, kRows, tid, 128, [&](int r, int d) -> uint4* {
-      const int b = b0 + r / G;
-      if (b >= s.B) return nullptr;
-      return reinterpret_cast<uint4*>(reinterpret_cast<uint8_t*>(s.out) + kc_piece(s.Bpad, b, (h * G + r % G) * D + d));
+      const int b = b0 + r / G, col = (h * G + r % G) * D + d;
+      if (b >= rows) return nullptr;
+      const size_t at = kWide ? (size_t)(b / 128) * 128 * s.n_kv * G * D * 2 + kc_piece(128, b % 128, col) : kc_piece(s.Bpad, b, col);
+      return reinterpret_cast<uint4*>(reinterpret_cast<uint8_t*>(s.out) + at);
     });
   wait.drain();
   if (splits > 1) {
@@ -1046,7 +902,7 @@ extern "C" cudaError_t vdc_stage_prepare() {
   const void* gemms[] = {(const void*)vdc::stage_gemm<0>, (const void*)vdc::stage_gemm<1>, (const void*)vdc::stage_gemm<2>};
   for (const void* f : gemms)
     if (cudaError_t e = cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, vdc::kGemmSmem)) return e;
-  const void* attns[] = {(const void*)vdc::stage_attn, (const void*)vdc::stage_attn_prefill};
+  const void* attns[] = {(const void*)vdc::stage_attn, (const void*)vdc::stage_attn_prefill<false>, (const void*)vdc::stage_attn_prefill<true>};
   for (const void* f : attns)
     if (cudaError_t e = cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, vdc::kAttnSmem)) return e;
   return cudaSuccess;
@@ -1057,13 +913,14 @@ struct Grid {
   int units, splits, slice;
 };
 static Grid stage_grid(const vdc_stage* s, int max_ctas) {
-  const bool attn = s->kind == VDC_STAGE_ATTN || s->kind == VDC_STAGE_ATTN_PREFILL;
+  const bool attn = s->kind == VDC_STAGE_ATTN || s->kind == VDC_STAGE_ATTN_PREFILL || s->kind == VDC_STAGE_WIDE_ATTN;
   const int tile = attn ? vdc::kRows / s->group : 1;       // rows of a prefill unit
   Grid g{1, s->kind == VDC_STAGE_GEMM || attn ? s->splits : 1, 0};
   switch (s->kind) {
     case VDC_STAGE_GEMM: g.units = (s->M + vdc::kBlk - 1) / vdc::kBlk; break;
     case VDC_STAGE_ATTN: g.units = s->n_kv * s->B; break;
     case VDC_STAGE_ATTN_PREFILL: g.units = s->n_kv * ((s->B + tile - 1) / tile); break;
+    case VDC_STAGE_WIDE_ATTN: g.units = s->n_kv * (s->Bpad / tile); break;
     case VDC_STAGE_NORM: g.units = (s->Bpad * (s->K / 8) + 255) / 256; break;
     case VDC_STAGE_EMBED: g.units = s->B; break;
   }
@@ -1091,7 +948,7 @@ extern "C" cudaError_t vdc_stage_launch(const vdc_stage* s, int max_ctas, int* f
   cudaLaunchAttribute attr[2];
   cfg.stream = stream;
   cfg.attrs = attr;
-  const bool gemm = s->kind == VDC_STAGE_GEMM, attn = s->kind == VDC_STAGE_ATTN || s->kind == VDC_STAGE_ATTN_PREFILL;
+  const bool gemm = s->kind == VDC_STAGE_GEMM, attn = s->kind == VDC_STAGE_ATTN || s->kind == VDC_STAGE_ATTN_PREFILL || s->kind == VDC_STAGE_WIDE_ATTN;
   const Grid g = stage_grid(s, max_ctas);
   if (g.splits > 1) {
     attr[cfg.numAttrs].id = cudaLaunchAttributeClusterDimension;
@@ -1116,7 +973,8 @@ extern "C" cudaError_t vdc_stage_launch(const vdc_stage* s, int max_ctas, int* f
         break;
       }
       case VDC_STAGE_ATTN: e = cudaLaunchKernelEx(&cfg, vdc::stage_attn, *s, first, status, timeout_ns); break;
-      case VDC_STAGE_ATTN_PREFILL: e = cudaLaunchKernelEx(&cfg, vdc::stage_attn_prefill, *s, first, status, timeout_ns); break;
+      case VDC_STAGE_WIDE_ATTN: e = cudaLaunchKernelEx(&cfg, vdc::stage_attn_prefill<true>, *s, first, status, timeout_ns); break;
+      case VDC_STAGE_ATTN_PREFILL: e = cudaLaunchKernelEx(&cfg, vdc::stage_attn_prefill<false>, *s, first, status, timeout_ns); break;
       case VDC_STAGE_NORM: e = cudaLaunchKernelEx(&cfg, vdc::stage_norm, *s, first); break;
       case VDC_STAGE_EMBED: e = cudaLaunchKernelEx(&cfg, vdc::stage_embed, *s, first, status); break;
       case VDC_STAGE_ADVANCE: e = cudaLaunchKernelEx(&cfg, vdc::stage_advance, *s, status); break;

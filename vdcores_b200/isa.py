@@ -54,7 +54,11 @@ GEMM_MODE_ADD_PACKED = _defs["GEMM_MODE_ADD_PACKED"]
 STAGE_GEMM, STAGE_ATTN, STAGE_ATTN_PREFILL, STAGE_EMBED, STAGE_ADVANCE, STAGE_COPY, STAGE_NORM = (
     _defs["STAGE_" + k] for k in ("GEMM", "ATTN", "ATTN_PREFILL", "EMBED", "ADVANCE", "COPY", "NORM"))
 STAGE_QKV, STAGE_RESID, STAGE_SILU, STAGE_ARGMAX = (_defs["STAGE_" + k] for k in ("QKV", "RESID", "SILU", "ARGMAX"))
+STAGE_WIDE_EMBED, STAGE_WIDE_GEMM, STAGE_WIDE_HEADS, STAGE_WIDE_ATTN, STAGE_WIDE_NORM, STAGE_WIDE_TAIL = (
+    _defs["STAGE_WIDE_" + k] for k in ("EMBED", "GEMM", "HEADS", "ATTN", "NORM", "TAIL"))
+STAGE_SUMS = _defs["STAGE_SUMS"]
 STAGE_BLOCK = _defs["STAGE_BLOCK"]
+WIDE_ROWS, WIDE_POS, WIDE_N = _defs["WIDE_ROWS"], _defs["WIDE_POS"], _defs["WIDE_N"]
 
 ST_POS, ST_NPAGES, ST_TOKEN, ST_STEP = _defs["ST_POS"], _defs["ST_NPAGES"], _defs["ST_TOKEN"], _defs["ST_STEP"]
 ST_NEWROW, ST_NKVH, ST_MAXPAGES, ST_ERR = _defs["ST_NEWROW"], _defs["ST_NKVH"], _defs["ST_MAXPAGES"], _defs["ST_ERR"]

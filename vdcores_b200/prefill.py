@@ -1,6 +1,10 @@
-"""Prefill on the device: a chunk of consecutive prompt positions per list of stage kernels.
+"""Prefill on the device: the prompt's positions as rows of stage kernels.
 
-The batched decode step (batch.BatchDecodeEngine) already computes, for every row of its batch, exactly what a prompt
+A prompt goes through a layer with all its rows together, up to isa.WIDE_ROWS of them (csrc/wide_kernels.cu): the weights are
+read once and the tensor cores are the bound.  On a part of the SMs (num_sms below the device's) it goes chunk by chunk
+through the batched step's stages instead.
+
+The chunks: the batched decode step (batch.BatchDecodeEngine) already computes, for every row of its batch, exactly what a prompt
 position needs; what differs in a prefill is that the rows are consecutive positions of ONE sequence.  PrefillEngine
 therefore gives every row the same page table and position pos0 + b.  The QKV projection's epilogue writes the normed,
 rotated key rows and the value rows of all the chunk's positions to the paged pools, so the attention behind it finds
@@ -17,7 +21,7 @@ import torch
 
 from . import isa, runtime
 from .batch import BatchDecodeEngine
-from .decode import DecodeEngine
+from .decode import BF16, DecodeEngine
 
 
 class PrefillEngine(BatchDecodeEngine):
@@ -55,9 +59,12 @@ class PrefillEngine(BatchDecodeEngine):
         the last chunk adds the final norm, the vocabulary projection and the argmax (the first generated id)."""
         super()._build_program()
         self._body = self._plan(vocab=False)
+        self._wide = None if self.max_ctas else WideStages(self)
 
     def launches(self, T: int) -> int:
         """Kernels a prompt of T tokens takes."""
+        if self._goes_wide(T):
+            return self._wide.launches(T)
         body, last = (runtime.count_stage_launches(s, self.max_ctas)[0] for s in (self._body, self.stages))
         return (T - 1) // self.batch * body + last
 
@@ -77,31 +84,143 @@ class PrefillEngine(BatchDecodeEngine):
         s[:, isa.ST_MAXPAGES] = self.max_pages
         s[:, isa.ST_PAGETABLE:] = table
 
+    def _goes_wide(self, T: int) -> bool:
+        return self._wide is not None and T > self.batch
+
     @torch.no_grad()
     def prefill(self, tokens: torch.Tensor, set_target_state: bool = True) -> int:
-        """Runs the prompt, ceil(T / chunk) lists of stages, and returns the first generated (greedy) id.  A chunk's state
-        blocks are prepared in pinned memory while the GPU runs the chunks before it, BLOCKS of them at most: every row of a
-        block carries the page table, and a place per chunk would grow with the square of the prompt."""
+        """Runs the prompt and returns the first generated (greedy) id.  What the host sends (ids, state blocks) is prepared in
+        pinned memory while the GPU runs what was sent before it, in BLOCKS blocks at most: every row of a chunk's block carries
+        the page table, and a place per chunk would grow with the square of the prompt."""
         T, B = int(tokens.numel()), self.batch
         assert 1 <= T < self.max_seq and self.stages is not None
         n = (T + B - 1) // B
         ids = tokens.cpu().to(torch.int32).numpy().reshape(-1)
         blocks = torch.empty(min(n, self.BLOCKS), B, self.state_words, dtype=torch.int32, pin_memory=True)
-        k = len(blocks)
-        copied = [torch.cuda.Event() for _ in blocks] if n > k else None
+        k, sent = len(blocks), 0
+        copied = [torch.cuda.Event() for _ in blocks]
+
+        def send(fill, dst):
+            """The next block, filled by fill(numpy view), into dst; its place is free again when it has been copied."""
+            nonlocal sent
+            if sent >= k:
+                copied[sent % k].synchronize()
+            block = blocks[sent % k]
+            fill(block.numpy())
+            dst.copy_(block.view(-1)[:dst.numel()].view(dst.shape), non_blocking=True)
+            copied[sent % k].record(self.stream)
+            sent += 1
         self.keys.zero_()
+        launch = lambda stages: runtime.launch_stages(stages, self.stream.cuda_stream, self.timeout_ns, self.max_ctas)
         with torch.cuda.stream(self.stream):
-            for c in range(n):
-                if c >= k:
-                    copied[c % k].synchronize()         # the chunk that had this block has been copied
-                self._fill_states(blocks[c % k].numpy(), ids, c)
-                self.state.copy_(blocks[c % k], non_blocking=True)
-                if copied:
-                    copied[c % k].record(self.stream)
-                runtime.launch_stages(self.stages if c == n - 1 else self._body, self.stream.cuda_stream, self.timeout_ns,
-                                      self.max_ctas)
+            if self._goes_wide(T):
+                self._wide.run(ids, send, launch)
+                send(lambda s: self._fill_states(s, ids, n - 1), self.state)
+                launch(self._wide.last)
+            else:
+                for c in range(n):
+                    send(lambda s: self._fill_states(s, ids, c), self.state)
+                    launch(self.stages if c == n - 1 else self._body)
         runtime.read_status(self.stream.cuda_stream)
         first = int(self.token_log[(T - 1) % B, 0])
         if set_target_state:
             self.target.set_state(T, first)
         return first
+
+
+class WideStages:
+    """Buffers and stages of a prompt whose rows go through a layer together.  Rows are taken in passes of `rows` (whole chunks
+    of the engine, at most isa.WIDE_ROWS); a pass over R rows (a multiple of 128) has a list of stages of its own."""
+    HEADER = isa.ST_PAGETABLE       # words in front of the page table
+
+    def __init__(self, e: PrefillEngine):
+        self.e, cfg, dev = e, e.cfg, e.dev
+        B, H, F, Q = e.batch, cfg.hidden, cfg.ffn, cfg.q_width
+        self.rows = min(isa.WIDE_ROWS, -(-e.max_seq // B) * B) // B * B
+        self.sms = torch.cuda.get_device_properties(dev).multi_processor_count
+        self.fmt = {"bf16": 0, "fp8": 1, "nvfp4": 2}[e.wkind]
+        R = -(-self.rows // 128) * 128
+        z = lambda n, dt=BF16: torch.empty(n, dtype=dt, device=dev)
+        self.hidden, self.normed, self.attn, self.act, self.q = z(R * H), z(R * H), z(R * Q), z(R * F), z(R * Q)
+        # every K-split leaves sums of its own: at most 8, and no more than make 2048 rows of them (runtime.wide_tiles)
+        self.sums = z(max(R, min(8 * R, 2048)) * max(e.qkv_rows, H), torch.float32)
+        self.block = z(self.HEADER + e.max_pages + self.rows, torch.int32)       # header, page table, ids
+        self.table = e.page_table.numpy()
+        self.lists = {}
+        self.template, self.places = self._plan()
+        # what follows the last layer: the last chunk's rows, then the chunk's own final stages
+        tail = runtime.Stage(kind=isa.STAGE_WIDE_TAIL, B=B, Bpad=e.bpad, K=H, x=self.hidden.data_ptr(), hid=e.hidden.data_ptr(),
+                             stats_out=e.stats[2 * cfg.n_layers].data_ptr(), state=self.block.data_ptr())
+        final = list(e.stages)[-3:]
+        self.last = (runtime.Stage * 4)(tail, *final)
+
+    def launches(self, T: int) -> int:
+        passes = -(-T // self.rows)
+        return passes * len(self.template) + len(self.last)
+
+    def _plan(self):
+        """The stages of a pass without what depends on its rows, and the places of each projection and of its sums' reader."""
+        e, cfg = self.e, self.e.cfg
+        H, F, Q = cfg.hidden, cfg.ffn, cfg.q_width
+        hid, normed, sums, state, attn, act = (t.data_ptr() for t in (self.hidden, self.normed, self.sums, self.block, self.attn, self.act))
+        S = runtime.Stage
+        heads = dict(group=cfg.group, n_kv=cfg.n_kv_heads, state=state)
+
+        def gemm(name, l, M, K, x, out):
+            return S(kind=isa.STAGE_WIDE_GEMM, mode=isa.STAGE_SILU if name == "wgu" else isa.STAGE_SUMS, wfmt=self.fmt, M=M, K=K,
+                     w=e._pack_cache[name, l].data_ptr(), x=x, out=out, scales=e.scales[name][l].data_ptr() if self.fmt else 0)
+        norm = lambda w, out, x: S(kind=isa.STAGE_WIDE_NORM, K=H, hid=hid, out=out, norm_w=w.data_ptr(), eps=cfg.eps, x=x, splits=1)
+        out = [S(kind=isa.STAGE_WIDE_EMBED, M=cfg.vocab, K=H, w=e.embed.data_ptr(), hid=hid, state=state,
+                 log=state + 4 * (self.HEADER + e.max_pages))]
+        for l in range(cfg.n_layers):
+            pools = dict(kpool=e.kpool[l].data_ptr(), vpool=e.vpool[l].data_ptr())
+            out += [norm(e.ln1[l], normed, sums if l else 0),
+                    gemm("wqkv", l, e.qkv_rows, H, normed, sums),
+                    S(kind=isa.STAGE_WIDE_HEADS, M=e.qkv_rows, x=sums, out=self.q.data_ptr(), rope=e.rope.data_ptr(),
+                      qk_norm=e.qknorm[l].data_ptr() if cfg.qk_norm else 0, qk_eps=cfg.qk_norm_eps, **heads, **pools),
+                    S(kind=isa.STAGE_WIDE_ATTN, n_pages=e.max_pages, q=self.q.data_ptr(), out=attn, **heads, **pools),
+                    gemm("wo", l, H, Q, attn, sums),
+                    norm(e.ln2[l], normed, sums),
+                    gemm("wgu", l, 2 * F, H, normed, act),
+                    gemm("wd", l, H, F, act, sums)]
+        out.append(norm(e.norm_w, 0, sums))
+        # place of a layer's first stage, then of the projection and the reader of its sums (0: none) from there
+        places = {"wqkv": (1, 2, e.qkv_rows, H), "wo": (4, 5, H, Q), "wgu": (6, 0, 2 * F, H), "wd": (7, 8, H, F)}
+        return (S * len(out))(*out), places
+
+    def stages(self, R: int):
+        """The stages of a pass over R rows."""
+        if R not in self.lists:
+            e, cfg = self.e, self.e.cfg
+            arr = type(self.template).from_buffer_copy(self.template)
+            v = np.ctypeslib.as_array(arr)
+            v["Bpad"] = R
+            n = 8 * cfg.n_layers
+            v["splits"][1 + 3:1 + n:8] = e._splits(cfg.n_kv_heads * (R // (64 // cfg.group)), 2, e.max_pages)
+            for name, (at, reader, M, K) in self.places.items():
+                subs, cols, ks = runtime.wide_tiles(R, M, K, self.fmt, self.sms, name == "wgu")
+                v["group"][1 + at:1 + n:8], v["n_kv"][1 + at:1 + n:8], v["splits"][1 + at:1 + n:8] = subs, cols, ks
+                if reader:
+                    v["splits"][1 + reader:2 + n:8] = ks
+            self.lists[R] = arr
+        return self.lists[R]
+
+    def run(self, ids, send, launch):
+        """All layers over the prompt's ids; send and launch are PrefillEngine.prefill's."""
+        at = self.HEADER + self.e.max_pages
+        for p0 in range(0, len(ids), self.rows):
+            part = ids[p0:p0 + self.rows]
+            words = np.zeros(at + len(part), dtype=np.int32)
+            words[isa.WIDE_POS], words[isa.WIDE_N] = p0, len(part)
+            words[isa.ST_PAGETABLE:at] = self.table
+            words[at:] = part
+            piece = self.e.batch * self.e.state_words       # a block of the engine's pinned memory
+            for w0 in range(0, len(words), piece):
+                w = words[w0:w0 + piece]
+
+                def fill(s, w=w):
+                    s.reshape(-1)[:len(w)] = w
+                send(fill, self.block[w0:w0 + len(w)])
+            launch(self.stages(-(-len(part) // 128) * 128))
+        n = len(ids)
+        self.last[0].M = (n - 1) // self.e.batch * self.e.batch % self.rows      # the last chunk's first row in its pass

@@ -56,9 +56,8 @@ def main():
         eng.kpool.zero_()
         eng.vpool.zero_()
         first, dt = timed(lambda: pre.prefill(prompt), args.reps)
-        n = (T + chunk - 1) // chunk
         line = (f"stages, chunk {chunk:3d}    : {dt * 1e3:8.1f} ms  {T / dt:9.0f} prompt tokens/s  first id {first}  "
-                f"{n} chunks, {dt * 1e3 / n:.2f} ms each, {pre.launches(T)} launches")
+                f"{pre.launches(T)} launches")
         if k_ref is not None:
             line += f"  last layer's key rows vs PyTorch: rel-L2 {rel(eng.read_kv(cfg.n_layers - 1, T)[0], k_ref):.1e}"
         print(line, flush=True)

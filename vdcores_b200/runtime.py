@@ -52,6 +52,7 @@ _lib.vdc_launch_static.argtypes = [_i32, _i32, _vp, _vp, _vp, _vp, _u64, _u64, c
 _lib.vdc_launch_stages.argtypes = [ctypes.POINTER(Stage), _i32, _u64, _u64]
 _lib.vdc_launch_stages_limited.argtypes = [ctypes.POINTER(Stage), _i32, _i32, _u64, _u64]
 _lib.vdc_count_stage_launches.argtypes = [ctypes.POINTER(Stage), _i32, _i32, ctypes.POINTER(_i32), ctypes.POINTER(_i32)]
+_lib.vdc_wide_tiles.argtypes = [_i32] * 6 + [ctypes.POINTER(_i32)]
 _lib.vdc_read_status.argtypes = [_u64, ctypes.POINTER(Status), _i32]
 _lib.vdc_build_tma_desc.argtypes = [_vp, _vp, _i32, _i32, ctypes.POINTER(_u64), ctypes.POINTER(_u64),
                                     ctypes.POINTER(ctypes.c_uint32), ctypes.POINTER(ctypes.c_uint32), _i32, _i32]
@@ -82,7 +83,7 @@ _lib.vdc_validate_streams.restype = _i32
 EXPORTED_SYMBOLS = [
     "vdc_version", "vdc_init", "vdc_set_smem_size", "vdc_launch", "vdc_launch_async", "vdc_launch_async_full",
     "vdc_launch_static", "vdc_launch_stages", "vdc_launch_stages_limited",
-    "vdc_count_stage_launches",
+    "vdc_count_stage_launches", "vdc_wide_tiles",
     "vdc_read_status",
     "vdc_build_tma_desc", "vdc_set_cache_policy", "vdc_enable_peer_access", "vdc_ipc_open", "vdc_ipc_close", "vdc_peer_alloc", "vdc_peer_free", "vdc_ipc_export", "vdc_opcode_count", "vdc_opcode_name", "vdc_opcode_value",
     "vdc_opcode_is_compute", "vdc_config", "vdc_family_specs", "vdc_last_error", "vdc_validate_streams",
@@ -203,6 +204,14 @@ def count_stage_launches(stages, max_ctas=0):
     launches, largest = _i32(), _i32()
     _check(_lib.vdc_count_stage_launches(stages, len(stages), int(max_ctas), ctypes.byref(launches), ctypes.byref(largest)))
     return launches.value, largest.value
+
+
+def wide_tiles(rows, M, K, wfmt, sms, whole=False):
+    """(128-row sub-matrices, columns, K-splits) of a tile of the projection of `rows` rows by an M x K matrix (whole: K is
+    not split); needs no GPU."""
+    out = (_i32 * 3)()
+    _check(_lib.vdc_wide_tiles(int(rows), int(M), int(K), int(wfmt), int(sms), int(whole), out))
+    return tuple(out)
 
 
 def launch_static(num_sms, insts_per_sm, compute_insts, memory_insts, tma_descs, bars_init, stream=0, timeout_ns=0):
