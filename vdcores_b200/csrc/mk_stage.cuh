@@ -90,6 +90,18 @@ struct Waiter {
   }
 };
 
+// Place in the ring and parity of the phase a role is at.
+struct RingAt {
+  int n, st = 0;
+  uint32_t parity = 0u;
+  __device__ __forceinline__ void next() {
+    if (++st == n) {
+      st = 0;
+      parity ^= 1u;
+    }
+  }
+};
+
 __device__ __forceinline__ uint4 pack8(const float (&v)[8]) {
   return make_uint4(pack_bf16x2(v[0], v[1]), pack_bf16x2(v[2], v[3]), pack_bf16x2(v[4], v[5]), pack_bf16x2(v[6], v[7]));
 }

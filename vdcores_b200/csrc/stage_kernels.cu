@@ -154,9 +154,10 @@ __global__ void __launch_bounds__(kGemmThreads, 2) stage_gemm(const __grid_const
       fence_proxy_async();
       for (int i = 0; i < first; ++i) bulk_load_1d(ring + i * stage_bytes, x + (size_t)i * xbytes, (uint32_t)xbytes, &sh.full[i]);
       const int aborted = ld_relaxed_gpu(&status->abort);    // looked at below, when it has long arrived
-      for (int i = first; i < n_ch; ++i) {
-        const int st = i % n_ring;
-        if (!wait(&sh.empty[st], (uint32_t)(i / n_ring - 1) & 1u, 0, i)) break;
+      RingAt at{n_ring};
+      for (int i = first; i < n_ch; ++i, at.next()) {       // chunk i takes the place of chunk i - n_ring
+        const int st = at.st;
+        if (!wait(&sh.empty[st], at.parity, 0, i)) break;
         load_weights(i, st);
         bulk_load_1d(ring + st * stage_bytes, x + (size_t)i * xbytes, (uint32_t)xbytes, &sh.full[st]);
       }
@@ -167,22 +168,22 @@ __global__ void __launch_bounds__(kGemmThreads, 2) stage_gemm(const __grid_const
     if (lane == 0) {
       const uint32_t idesc = umma_idesc_bf16_m128(N);
       const uint32_t lbo_a = (uint32_t)s.Bpad * 16u, lbo_b = (uint32_t)N * 16u;
-      bool ok = true;
-      for (int i = 0; i < n_ch && ok; ++i) {
-        const int st = i % n_ring;
-        ok = wait(&sh.full[st], (uint32_t)(i / n_ring) & 1u, 1, i);
-        if (kFmt != 0 && ok) ok = wait(&sh.ready[st], (uint32_t)(i / n_ring) & 1u, 1, i);
+      // No divisions per chunk and descriptors advanced by constants, here and in the other roles: what this thread does beside
+      // its MMAs the tensor cores wait for.  A step of 32 rows with e4m3 weights 338 -> 319 us, 16 rows NVFP4 364 -> 358, 3 rows
+      // bf16 245 -> 242.
+      const uint64_t a0 = umma_desc(smem_u32(ring), lbo_a, 128u);
+      const uint64_t b0 = umma_desc(smem_u32(kFmt != 0 ? staging : ring + xbytes), lbo_b, 128u);
+      const uint32_t stage16 = (uint32_t)stage_bytes >> 4, step_a = (2u * lbo_a) >> 4, step_b = (2u * lbo_b) >> 4;
+      RingAt at{n_ring};
+      for (int i = 0; i < n_ch; ++i, at.next()) {
+        const int st = at.st;
+        bool ok = wait(&sh.full[st], at.parity, 1, i);
+        if (kFmt != 0 && ok) ok = wait(&sh.ready[st], at.parity, 1, i);
         if (!ok) break;
         tc_fence_after();
-        uint8_t* at = ring + st * stage_bytes;
-        uint64_t adesc = umma_desc(smem_u32(at), lbo_a, 128u);
-        uint64_t bdesc = umma_desc(smem_u32(kFmt != 0 ? staging + (i & 1) * (kBlk * kKc * 2) : at + xbytes), lbo_b, 128u);
+        const uint64_t ad = a0 + st * stage16, bd = b0 + (kFmt != 0 ? (i & 1) * (uint32_t)(kBlk * kKc * 2 >> 4) : st * stage16);
 #pragma unroll
-        for (int k = 0; k < kKc / 16; ++k) {
-          umma_bf16(tmem, adesc, bdesc, idesc, (uint32_t)((i | k) != 0));
-          adesc += (2u * lbo_a) >> 4;
-          bdesc += (2u * lbo_b) >> 4;
-        }
+        for (int k = 0; k < kKc / 16; ++k) umma_bf16(tmem, ad + k * step_a, bd + k * step_b, idesc, (uint32_t)((i | k) != 0));
         umma_commit(&sh.empty[st]);
         if (kFmt != 0) umma_commit(&sh.stg_empty[i & 1]);
       }
@@ -194,9 +195,11 @@ __global__ void __launch_bounds__(kGemmThreads, 2) stage_gemm(const __grid_const
     const int t = tid - 64;
     if (kFmt != 0) {
       const int team = kEpiThreads / teams, tt = t & (team - 1), row = t & 127;
+      RingAt at{n_ring};
+      if (t >= team) at.next();
       for (int i = t / team; i < n_ch; i += teams) {
-        const int st = i % n_ring;
-        const bool seen = wait(&sh.full[st], (uint32_t)(i / n_ring) & 1u, 2, i) &&
+        const int st = at.st;
+        const bool seen = wait(&sh.full[st], at.parity, 2, i) &&
                           (i < 2 || wait(&sh.stg_empty[i & 1], (uint32_t)((i >> 1) - 1) & 1u, 2, i));
         if (!__all_sync(0xffffffffu, seen)) break;      // as in warp_wait, one vote for both
         uint8_t* dst = staging + (i & 1) * (kBlk * kKc * 2);
@@ -210,6 +213,8 @@ __global__ void __launch_bounds__(kGemmThreads, 2) stage_gemm(const __grid_const
         fence_proxy_async_smem();
         __syncwarp();
         if (lane == 0) mbar_arrive(&sh.ready[st]);   // one arrival per warp: one per thread would queue on the barrier's word
+        at.next();
+        if (teams == 2) at.next();
       }
     }
     grid_dep_wait();

@@ -44,18 +44,6 @@ __host__ __device__ inline int wide_ring(int wfmt, int subs, int n) {
   return r < kWideRing ? r : kWideRing;
 }
 
-// Place in the ring and parity of the phase a role is at.
-struct RingAt {
-  int n, st = 0;
-  uint32_t parity = 0u;
-  __device__ __forceinline__ void next() {
-    if (++st == n) {
-      st = 0;
-      parity ^= 1u;
-    }
-  }
-};
-
 struct WideTile {
   int m, n0, N, c0, n_ch, subs, split;
 };
