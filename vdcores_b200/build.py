@@ -5,7 +5,7 @@ import sys
 
 HERE = os.path.dirname(os.path.abspath(__file__))
 LIB = os.path.join(HERE, "libvdcores_b200.so")
-SOURCES = [os.path.join(HERE, "csrc", f) for f in ("megakernel.cu", "stage_kernels.cu", "wide_kernels.cu", "capi.cu")]
+SOURCES = [os.path.join(HERE, "csrc", f) for f in ("megakernel.cu", "stage_kernels.cu", "wide_kernels.cu", "step_kernel.cu", "capi.cu")]
 # VDC_NO_STREAMER: the optional HBM->L2 streamer warp stays out of the build (it did not pay for
 # the registers it costs: 13 warps cap the kernel at 128 registers per thread instead of 168).
 FLAGS = ["-gencode", "arch=compute_100a,code=sm_100a", "-lineinfo", "-O3", "-std=c++17", "-shared",

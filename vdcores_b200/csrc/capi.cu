@@ -19,6 +19,10 @@ extern "C" cudaError_t vdc_megakernel_launch(int num_sms, const void* cinsts, co
 extern "C" cudaError_t vdc_stage_prepare();
 extern "C" cudaError_t vdc_stage_launch(const vdc_stage* s, int max_ctas, int* front, vdc_status* status,
                                         uint64_t timeout_ns, cudaStream_t stream);
+extern "C" const char* vdc_step_refuses(const vdc_step* s, bool pointers);
+extern "C" long long vdc_step_words(const vdc_step* s);
+extern "C" cudaError_t vdc_step_prepare();
+extern "C" cudaError_t vdc_step_launch(const vdc_step* s, vdc_status* status, uint64_t timeout_ns, cudaStream_t stream);
 extern "C" cudaError_t vdc_wide_prepare();
 extern "C" void vdc_wide_choose(int rows, int M, int K, int wfmt, int sms, int whole, int* out);
 extern "C" int vdc_wide_grid(const vdc_stage* s, int sms, int* tiles);
@@ -96,6 +100,7 @@ int vdc_init(void) {
   if (e != cudaSuccess) return fail_cuda(e, "cudaFuncSetAttribute(MaxDynamicSharedMemorySize)");
   e = vdc_stage_prepare();
   if (e == cudaSuccess) e = vdc_wide_prepare();
+  if (e == cudaSuccess) e = vdc_step_prepare();
   if (e != cudaSuccess) return fail_cuda(e, "cudaFuncSetAttribute(stage kernels)");
   vdc_status* st = nullptr;
   e = cudaMalloc(&st, sizeof(vdc_status));
@@ -272,6 +277,24 @@ int vdc_count_stage_launches(const vdc_stage* stages, int n, int max_ctas, int* 
     if (c > *largest) *largest = c;
   }
   return VDC_OK;
+}
+
+int vdc_step_workspace(const vdc_step* step, uint64_t* bytes) {
+  if (!step || !bytes) return fail_arg("null argument");
+  if (const char* why = vdc_step_refuses(step, false)) return fail_arg(why);
+  *bytes = (uint64_t)vdc_step_words(step) * 8;
+  return VDC_OK;
+}
+
+int vdc_launch_step(const vdc_step* step, uint64_t stream, uint64_t timeout_ns) {
+  int dev;
+  if (int r = current_device(&dev)) return r;
+  if (!g_status[dev]) return fail_arg("vdc_init was not called on this device");
+  if (!step) return fail_arg("null argument");
+  if (const char* why = vdc_step_refuses(step, true)) return fail_arg(why);
+  if (step->num_sms > g_sm_count[dev]) return fail_arg("num_sms must be in [1, SM count of the device]");
+  cudaError_t e = vdc_step_launch(step, g_status[dev], timeout_ns ? timeout_ns : 2000000000ull, reinterpret_cast<cudaStream_t>(stream));
+  return e == cudaSuccess ? VDC_OK : fail_cuda(e, "step launch");
 }
 
 int vdc_wide_tiles(int rows, int M, int K, int wfmt, int sms, int whole, int* out) {

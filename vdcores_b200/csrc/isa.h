@@ -60,6 +60,7 @@
 #define VDC_STAGE_WIDE_ATTN 11
 #define VDC_STAGE_WIDE_NORM 12
 #define VDC_STAGE_WIDE_TAIL 13
+#define VDC_STEP_KIND 14          // what a step kernel's errors carry in the status block's opcode
 #define VDC_WIDE_ROWS 2048       // most rows of one pass
 #define VDC_WIDE_POS 0           // words of the block those stages read: first position, rows; page table at VDC_ST_PAGETABLE
 #define VDC_WIDE_N 1

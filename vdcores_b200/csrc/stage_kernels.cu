@@ -360,23 +360,6 @@ struct AttnShared {
   float wm[4][8], wl[4][8];
 };
 
-__device__ __forceinline__ void mma_16816(float (&d)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0,
-                                          uint32_t b1) {
-  asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
-               : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3]) : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
-}
-// 2^x as one instruction: results below the smallest normal number become zero.
-__device__ __forceinline__ float exp2_ftz(float x) {
-  float y;
-  asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
-  return y;
-}
-__device__ __forceinline__ uint32_t transpose8x8(uint32_t v) {
-  uint32_t d;
-  asm volatile("movmatrix.sync.aligned.m8n8.trans.b16 %0, %1;" : "=r"(d) : "r"(v));
-  return d;
-}
-
 // Producer warp: streams the K and V pages first .. first + count - 1 of one KV head through the ring.  Pages in front of
 // `settled` hold no row that the projection in front of this stage writes: their copies start before its end is waited
 // for.  (Reading the state blocks that early is safe for the same reason: the stage in front triggers this launch only

@@ -1,0 +1,1134 @@
+// One token of a model at batch 1, as one persistent kernel.
+//
+// A step streams every weight once (1 FLOP per byte), so HBM is the floor; what a step costs beyond it are the places where
+// every SM needs what all SMs have just computed, five per layer.  Two things make those short here:
+//   * The producer warp of a CTA knows every weight row and cache page of the whole step beforehand and copies them through a
+//     ring of ~170 KB without looking at the stages: HBM keeps streaming while the other warps wait for activations.
+//   * Activations travel as 8-byte entries {payload, tag}.  A consumer polls the entries themselves; no fence, counter or flag
+//     stands between a result and the SMs that wait for it.
+// The same step as a program of the megakernel (csrc/megakernel.cu) counts barriers down: fence, atomic, poll, then a copy,
+// about 7 us per boundary.
+//
+// An entry buffer is written again one layer later, when everything that read it must have been read: whoever polls a buffer
+// has rows in the same or the following stage, and those rows go into what the next writer of the buffer waits for.
+#include "mk_stage.cuh"
+
+namespace vdc {
+
+constexpr int kStepWarps = 16;                       // consumer warps; one more warp produces
+constexpr int kStepThreads = 32 * kStepWarps;
+constexpr int kItems = 16;                           // copies in the ring, at most
+constexpr int kItemBytes = 32 * 1024;                // bytes of one, at most
+constexpr int kPageBytes = VDC_KV_PAGE * VDC_HEAD_DIM * 2;
+constexpr int kGroups = 4;                           // of four warps: a page of the cache each
+constexpr int kOutLd = VDC_HEAD_DIM + 4;
+constexpr int kPartFloats = kGroups * 8 * kOutLd;    // partial sums of rows; also the groups' partial heads
+constexpr int kQLd = VDC_HEAD_DIM / 2 + 4;           // words of a query row in shared memory
+constexpr int kPLd = VDC_KV_PAGE / 2 + 4;            // words of a row of probabilities
+constexpr int kMaxSplits = 32;
+constexpr int kMaxTopK = 16, kMaxExperts = 256;
+constexpr int kStepSmem = 227 * 1024 - 1024;         // dynamic; the rest is StepShared's barriers
+
+enum { kQkv, kOut, kRouter, kGateUp, kDown, kVocab, kStages };
+
+struct StepShared {
+  uint64_t full[kItems], empty[kItems], routed;
+  int start[kItems];                                 // offset of an item in the ring
+  volatile int fail;
+  float red[kStepWarps];
+  float best[kStepWarps];
+  int best_row[kStepWarps];
+  int share[kStages][2];                             // first row and rows of this SM, stage by stage
+};
+// Behind the ring: what the consumers share.
+struct StepLayout {
+  int ring, x, h, part, raw, q, rows, p, gm, wl, route;
+  int total;
+};
+__host__ __device__ inline StepLayout step_layout(const vdc_step& s) {
+  const int q = s.n_kv * s.group * VDC_HEAD_DIM, act = s.ffn * (s.n_experts ? s.top_k : 1);
+  int xw = s.hidden > q ? s.hidden : q;
+  if (act > xw) xw = act;
+  StepLayout l;
+  int at = 0;
+  auto take = [&](int bytes) {
+    const int r = at;
+    at += (bytes + 127) / 128 * 128;
+    return r;
+  };
+  l.x = take(xw * 2);
+  l.h = take(s.hidden * 2);
+  l.part = take(kPartFloats * 4);
+  l.raw = take(10 * VDC_HEAD_DIM * 2);
+  l.q = take(8 * kQLd * 4);
+  l.rows = take(2 * VDC_HEAD_DIM * 2 + VDC_HEAD_DIM * 2);       // new key and value row; zeros
+  l.p = take(kGroups * 8 * kPLd * 4);
+  l.gm = take(kGroups * 4 * 8 * 4);
+  l.wl = take(kGroups * 5 * 8 * 4);
+  l.route = take(kMaxExperts * 4 + 2 * kMaxTopK * 4);
+  l.ring = at;
+  l.total = kStepSmem - 128;
+  return l;
+}
+
+// Entry buffers in the workspace, in 8-byte words; word 0 counts the launches.
+struct StepWork {
+  size_t h, qkv, rec, ml, attn, act, router, best, words;
+};
+__host__ __device__ inline StepWork step_work(const vdc_step& s) {
+  StepWork w;
+  size_t at = 16;
+  auto take = [&](size_t n) {
+    const size_t r = at;
+    at += (n + 15) / 16 * 16;
+    return r;
+  };
+  const size_t heads = (size_t)s.n_kv * s.group;
+  w.h = take(s.hidden);                                        // two versions of hidden / 2 entries
+  w.qkv = take((heads + 2 * (size_t)s.n_kv) * VDC_HEAD_DIM / 2);
+  w.rec = take((size_t)s.n_kv * s.n_splits * s.group * VDC_HEAD_DIM);
+  w.ml = take((size_t)s.n_kv * s.n_splits * s.group * 2);
+  w.attn = take(heads * VDC_HEAD_DIM / 2);
+  w.act = take((size_t)s.ffn * (s.n_experts ? s.top_k : 1) / 2);
+  w.router = take(s.n_experts ? s.n_experts : 1);
+  w.best = take(2 * (size_t)s.num_sms);
+  w.words = at;
+  return w;
+}
+
+// What a launch passes: the step, and where its shared memory and its entries lie.  From the constant bank these cost no
+// registers.
+struct StepArgs {
+  vdc_step s;
+  StepLayout lay;
+  StepWork wk;
+};
+// Rows of a stage that one SM takes.
+struct Share {
+  int r0, n;
+};
+
+// ------------------------------------------------------------------------- //
+// entries
+// ------------------------------------------------------------------------- //
+__device__ __forceinline__ void put(uint64_t* p, uint32_t payload, uint32_t tag) {
+  asm volatile("st.relaxed.gpu.global.u64 [%0], %1;" ::"l"(p), "l"(((uint64_t)tag << 32) | payload) : "memory");
+}
+__device__ __forceinline__ void put2(uint64_t* p, uint32_t a, uint32_t b, uint32_t tag) {
+  asm volatile("st.relaxed.gpu.global.v2.u64 [%0], {%1,%2};" ::"l"(p), "l"(((uint64_t)tag << 32) | a),
+               "l"(((uint64_t)tag << 32) | b)
+               : "memory");
+}
+struct Two {
+  uint64_t a, b;
+  __device__ __forceinline__ bool are(uint32_t tag) const { return (uint32_t)(a >> 32) == tag && (uint32_t)(b >> 32) == tag; }
+};
+__device__ __forceinline__ Two get2(const uint64_t* p) {
+  Two v;
+  asm volatile("ld.relaxed.gpu.global.v2.u64 {%0,%1}, [%2];" : "=l"(v.a), "=l"(v.b) : "l"(p) : "memory");
+  return v;
+}
+
+// ------------------------------------------------------------------------- //
+// dot products of a chunk's rows
+// ------------------------------------------------------------------------- //
+__device__ __forceinline__ void mma_f16(float (&d)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0, uint32_t b1) {
+  asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
+               : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3]) : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
+}
+__device__ __forceinline__ uint32_t e4m3_pair(uint32_t pair) {
+  uint32_t d;
+  asm("cvt.rn.f16x2.e4m3x2 %0, %1;" : "=r"(d) : "h"((unsigned short)pair));
+  return d;
+}
+__host__ __device__ constexpr int row_bytes(int fmt, int K) { return fmt == 0 ? 2 * K : fmt == 1 ? K : K / 2 + K / 16; }
+__host__ __device__ constexpr int unit_of(int fmt) { return fmt == 0 ? 256 : fmt == 1 ? 512 : 1024; }     // inputs of a warp's step
+
+// Weights as the tensor cores take them: four (bf16), four (e4m3) or eight (NVFP4) of a lane's 16 bytes, which is two, one or
+// one word of them, as bf16 or f16 pairs.  An NVFP4 weight times its block's scale is exact in f16.
+template <int kFmt>
+__device__ __forceinline__ void expand(uint32_t (&o)[kFmt == 2 ? 4 : 2], const uint32_t (&c)[4], int part, uint32_t scales) {
+  if (kFmt == 0) {
+    o[0] = c[2 * part];
+    o[1] = c[2 * part + 1];
+  } else if (kFmt == 1) {
+    o[0] = e4m3_pair(c[part] & 0xFFFFu);
+    o[1] = e4m3_pair(c[part] >> 16);
+  } else {
+    const uint32_t sc = __byte_perm(scales, 0, part < 2 ? 0x1010 : 0x3232);
+#pragma unroll
+    for (int j = 0; j < (kFmt == 2 ? 4 : 2); ++j) {
+      const __half2 p = __hmul2(e2m1x2_to_half2((c[part] >> (8 * j)) & 0xFFu), *reinterpret_cast<const __half2*>(&sc));
+      o[j] = *reinterpret_cast<const uint32_t*>(&p);
+    }
+  }
+}
+
+// One step of a warp: 16 bytes per lane of kPairs pairs of rows times the same inputs, as products of 16 x 16 by 16 x 8 tiles.
+// Row g of a tile is what the four lanes 4g .. 4g + 3 hold of the pair's first row (8 + g: of its second), column g what they
+// hold of the inputs: the tile's element (g, g) is the sum of the four lanes' products, the other elements mean nothing.  An
+// FMA per product would do the same, but fma with 16-bit operands runs at 16 a clock and SM (measured: 0.8 us for 32 KB of
+// bf16, where HBM takes 0.73).
+template <int kFmt, int kPairs>
+__device__ __forceinline__ void dot_unit(float (&d)[kPairs][4], const uint8_t* w, const int (&row)[4], bool single, const uint8_t* x,
+                                         int u, int lane, int K) {
+  constexpr int kParts = kFmt == 0 ? 2 : 4, kWords = kFmt == 2 ? 4 : 2;       // of a lane's 16 bytes; expanded words of one
+  uint32_t c[2 * kPairs][4], sc[2 * kPairs];
+#pragma unroll
+  for (int i = 0; i < 2 * kPairs; ++i) {
+    const uint8_t* r = w + row[i];
+    const bool none = (i & 1) && single;
+    const uint4 v = none ? make_uint4(0u, 0u, 0u, 0u) : lds128(r + u * 512 + lane * 16);
+    c[i][0] = v.x; c[i][1] = v.y; c[i][2] = v.z; c[i][3] = v.w;
+    sc[i] = kFmt == 2 && !none ? e4m3_pair(*reinterpret_cast<const uint16_t*>(r + (K >> 1) + u * 64 + lane * 2)) : 0u;
+  }
+  const uint8_t* xp = x + u * unit_of(kFmt) * 2 + lane * 16;
+  uint32_t xv[4];
+#pragma unroll
+  for (int part = 0; part < kParts; ++part) {
+    const int at = part * kWords;                                               // first expanded word; four of them are 16 bytes of x
+    if ((at & 3) == 0) {
+      const uint4 v = lds128(xp + (at >> 2) * 512);
+      xv[0] = v.x; xv[1] = v.y; xv[2] = v.z; xv[3] = v.w;
+    }
+#pragma unroll
+    for (int p = 0; p < kPairs; ++p) {
+      uint32_t a[kWords], b[kWords];
+      expand<kFmt>(a, c[2 * p], part, sc[2 * p]);
+      expand<kFmt>(b, c[2 * p + 1], part, sc[2 * p + 1]);
+#pragma unroll
+      for (int j = 0; j < kWords; j += 2) {
+        if (kFmt == 0) mma_16816(d[p], a[j], b[j], a[j + 1], b[j + 1], xv[(at & 3) + j], xv[(at & 3) + j + 1]);
+        else mma_f16(d[p], a[j], b[j], a[j + 1], b[j + 1], xv[(at & 3) + j], xv[(at & 3) + j + 1]);
+      }
+    }
+  }
+}
+
+// Units of q rows; the first SMs' shares are never empty while there are any.
+__device__ __forceinline__ Share share_of(int rows, int q, int sm, int sms) {
+  const int units = rows / q;
+  const int a = (int)(((long long)units * sm + sms - 1) / sms), b = (int)(((long long)units * (sm + 1) + sms - 1) / sms);
+  return {a * q, (b - a) * q};
+}
+__host__ __device__ constexpr int chunk_rows(int rb) {        // an even number where more than one
+  const int n = kItemBytes / rb < 32 ? kItemBytes / rb : 32;
+  return n > 1 ? n & ~1 : 1;
+}
+
+// ------------------------------------------------------------------------- //
+// producer
+// ------------------------------------------------------------------------- //
+struct Producer {
+  StepShared& sh;
+  const Waiter& wait;
+  uint8_t* ring;
+  int cap;
+  RingAt at{kItems};       // next item
+  int oldest = 0, live = 0, wr = 0, count = 0;
+  uint32_t oldest_parity = 0u;
+  bool wrapped = false, ok = true;
+
+  // Room for one more item of `bytes`, freeing the oldest ones as they are consumed.
+  __device__ __forceinline__ uint8_t* room(int bytes) {
+    bytes = (bytes + 127) & ~127;
+    while (ok) {
+      if (live < kItems) {
+        if (live == 0) {
+          wr = 0;
+          wrapped = false;
+        }
+        if (!wrapped && wr + bytes > cap && bytes <= sh.start[oldest]) {
+          wr = 0;
+          wrapped = true;
+        }
+        if (wr + bytes <= (wrapped ? sh.start[oldest] : cap)) break;
+      }
+      ok = wait(&sh.empty[oldest], oldest_parity, 0, count);
+      const int was = sh.start[oldest];
+      if (++oldest == kItems) {
+        oldest = 0;
+        oldest_parity ^= 1u;
+      }
+      --live;
+      if (live > 0 && sh.start[oldest] < was) wrapped = false;
+    }
+    uint8_t* p = ring + wr;
+    sh.start[at.st] = wr;
+    wr += bytes;
+    ++live;
+    return p;
+  }
+  __device__ __forceinline__ void copy(const uint8_t* src, int bytes) {
+    uint8_t* p = room(bytes);
+    if (!ok) return;
+    mbar_arrive_expect_tx(&sh.full[at.st], (uint32_t)bytes);
+    bulk_load_1d(p, src, (uint32_t)bytes, &sh.full[at.st]);
+    at.next();
+    ++count;
+  }
+  __device__ __forceinline__ void rows(const uint8_t* w, int rb, int n) {
+    const int per = chunk_rows(rb);
+    for (int r = 0; r < n && ok; r += per) copy(w + (size_t)r * rb, min(per, n - r) * rb);
+  }
+  __device__ __forceinline__ void page(const uint8_t* k, const uint8_t* v) {
+    uint8_t* p = room(2 * kPageBytes);
+    if (!ok) return;
+    mbar_arrive_expect_tx(&sh.full[at.st], 2 * kPageBytes);
+    bulk_load_1d(p, k, kPageBytes, &sh.full[at.st]);
+    bulk_load_1d(p + kPageBytes, v, kPageBytes, &sh.full[at.st]);
+    at.next();
+    ++count;
+  }
+};
+
+// An SM's share of the attention: one KV head's pages first .. first + count - 1; `live` splits of the head have pages.  Up to
+// four pages, one per group of warps, stay with one SM: there is nothing to merge then.
+struct Pages {
+  int h, split, live, first, count;
+};
+__device__ __forceinline__ Pages pages_of(const vdc_step& s, int pos, int sm) {
+  Pages p{sm % s.n_kv, sm / s.n_kv, 0, 0, 0};
+  const int n = min(pos / VDC_KV_PAGE + 1, s.max_pages), per = n <= kGroups ? n : (n + s.n_splits - 1) / s.n_splits;
+  p.live = (n + per - 1) / per;
+  if (p.split < p.live) {
+    p.first = p.split * per;
+    p.count = min(per, n - p.first);
+  }
+  return p;
+}
+
+// ------------------------------------------------------------------------- //
+// consumers
+// ------------------------------------------------------------------------- //
+__device__ __forceinline__ void consumers_sync() { asm volatile("bar.sync 1, %0;" ::"n"(kStepThreads) : "memory"); }
+
+struct Consumer {
+  const StepArgs& args;
+  const vdc_step& s;
+  const StepLayout& lay;
+  StepShared& sh;
+  const Waiter& wait;
+  uint8_t* base;
+  int tid, warp, lane, sm;
+  RingAt at{kItems};
+  int kw, kg, rw, rg, ld;        // warps along the inputs, this warp's place there; along the rows; rows there is room for
+
+  __device__ __forceinline__ float* part() const { return reinterpret_cast<float*>(base + lay.part); }
+  __device__ __forceinline__ uint32_t* hs() const { return reinterpret_cast<uint32_t*>(base + lay.h); }
+  __device__ __forceinline__ uint8_t* x() const { return base + lay.x; }
+
+  // Whether to look again for entries that are not there yet (it: looks so far); false when the wait was given up.
+  __device__ __forceinline__ bool again(const uint64_t* p, uint32_t it, uint64_t& t0) const {
+    if ((it & 63u) != 0) return true;
+    if (*wait.fail) return false;
+    if (ld_relaxed_gpu(&wait.status->abort) == 0) {
+      const uint64_t now = globaltimer_ns();
+      if (t0 == 0) t0 = now;
+      if (now - t0 <= wait.timeout_ns) return true;
+      report(wait.status, VDC_ERR_TIMEOUT, VDC_STEP_KIND, 1, (int)(p - reinterpret_cast<const uint64_t*>(s.work)), (int)it);
+    }
+    *wait.fail = 1;
+    return false;
+  }
+  __device__ __forceinline__ bool poll2(const uint64_t* p, uint32_t tag, Two& v) const {
+    uint64_t t0 = 0;
+    for (uint32_t it = 1; !v.are(tag); ++it) {
+      if (!again(p, it, t0)) return false;
+      v = get2(p);
+    }
+    return true;
+  }
+  // n 2-byte values (a multiple of 4) of an entry buffer: f(i, values 4i .. 4i + 3 as two words) for this thread's i.  All that
+  // a thread still misses is looked for at the same time: one after another, each look is a round trip of its own.
+  template <int kBatch, class F>
+  __device__ __forceinline__ void collect(const uint64_t* buf, int n, uint32_t tag, F f) const {
+    for (int i0 = tid; i0 < n / 4; i0 += kBatch * kStepThreads) {
+      Two v[kBatch];
+#pragma unroll
+      for (int j = 0; j < kBatch; ++j)
+        if (i0 + j * kStepThreads < n / 4) v[j] = get2(buf + 2 * (i0 + j * kStepThreads));
+      uint64_t t0 = 0;
+      for (uint32_t it = 1;; ++it) {
+        bool all = true;
+#pragma unroll
+        for (int j = 0; j < kBatch; ++j)
+          if (i0 + j * kStepThreads < n / 4) all = all && v[j].are(tag);
+        if (all) break;
+        if (!again(buf + 2 * i0, it, t0)) return;
+#pragma unroll
+        for (int j = 0; j < kBatch; ++j)
+          if (i0 + j * kStepThreads < n / 4 && !v[j].are(tag)) v[j] = get2(buf + 2 * (i0 + j * kStepThreads));
+      }
+#pragma unroll
+      for (int j = 0; j < kBatch; ++j)
+        if (i0 + j * kStepThreads < n / 4) f(i0 + j * kStepThreads, (uint32_t)v[j].a, (uint32_t)v[j].b);
+    }
+  }
+  // Inputs 4i .. 4i + 3 (two bf16 pairs) as the dot products take them: bf16 in order; f16 for quantised rows, a lane's 16-byte
+  // pieces of a step 512 bytes apart, so that neighbouring lanes read neighbouring pieces.
+  template <int kFmt>
+  __device__ __forceinline__ void set_input(int i, uint32_t a, uint32_t b, bool plain) const {
+    if (kFmt == 0 || plain) {
+      *reinterpret_cast<uint2*>(x() + i * 8) = make_uint2(a, b);
+      return;
+    }
+    constexpr int kLane = unit_of(kFmt) / 32;
+    const int e = i * 4, u = e / unit_of(kFmt), in = e % unit_of(kFmt);
+    const __half2 ha = __floats2half2_rn(bf_lo(a), bf_hi(a)), hb = __floats2half2_rn(bf_lo(b), bf_hi(b));
+    *reinterpret_cast<uint2*>(x() + u * unit_of(kFmt) * 2 + (in % kLane) / 8 * 512 + in / kLane * 16 + (i & 1) * 8) =
+        make_uint2(*reinterpret_cast<const uint32_t*>(&ha), *reinterpret_cast<const uint32_t*>(&hb));
+  }
+  // The hidden state (entries, or a row of the embedding table) into shared memory and, RMS-normalised with the weights w,
+  // into the input vector.  Rounded like a bf16 tensor expression.
+  template <int kFmt>
+  __device__ __forceinline__ void hidden(const uint64_t* buf, uint32_t tag, const uint8_t* row, uint64_t w, bool plain) const {
+    const int H = s.hidden;
+    constexpr int kMost = 4;                                      // hidden <= 8192
+    uint2 wv[kMost];
+#pragma unroll
+    for (int j = 0; j < kMost; ++j) {
+      const int i = tid + j * kStepThreads;
+      if (i < H / 4) wv[j] = __ldg(reinterpret_cast<const uint2*>(w) + i);
+    }
+    float ssq = 0.f;
+    auto keep = [&](int i, uint32_t a, uint32_t b) {
+      *reinterpret_cast<uint2*>(hs() + 2 * i) = make_uint2(a, b);
+      ssq = fmaf(bf_lo(a), bf_lo(a), fmaf(bf_hi(a), bf_hi(a), fmaf(bf_lo(b), bf_lo(b), fmaf(bf_hi(b), bf_hi(b), ssq))));
+    };
+    if (row != nullptr) {
+      for (int i = tid; i < H / 4; i += kStepThreads) {
+        const uint2 v = __ldg(reinterpret_cast<const uint2*>(row) + i);
+        keep(i, v.x, v.y);
+      }
+    } else {
+      collect<kMost>(buf, H, tag, keep);
+    }
+    ssq = warp_sum(ssq);
+    if (lane == 0) sh.red[warp] = ssq;
+    consumers_sync();
+    float tot = 0.f;
+#pragma unroll
+    for (int k = 0; k < kStepWarps; ++k) tot += sh.red[k];
+    const float rstd = rsqrtf(tot / (float)H + s.eps);
+#pragma unroll
+    for (int j = 0; j < kMost; ++j) {
+      const int i = tid + j * kStepThreads;
+      if (i < H / 4) {
+        const uint2 v = *reinterpret_cast<const uint2*>(hs() + 2 * i);
+        const uint32_t a = pack_bf16x2(bf16_round(bf_lo(v.x) * rstd) * bf_lo(wv[j].x), bf16_round(bf_hi(v.x) * rstd) * bf_hi(wv[j].x));
+        const uint32_t b = pack_bf16x2(bf16_round(bf_lo(v.y) * rstd) * bf_lo(wv[j].y), bf16_round(bf_hi(v.y) * rstd) * bf_hi(wv[j].y));
+        set_input<kFmt>(i, a, b, plain);
+      }
+    }
+    consumers_sync();
+  }
+
+  // How the warps share rows of K inputs: along K as far as that has steps for them, the rest along the rows.
+  template <int kFmt>
+  __device__ __forceinline__ void split(int K) {
+    const int units = K / unit_of(kFmt);
+    kw = units >= 16 ? 16 : units >= 8 ? 8 : units >= 4 ? 4 : units >= 2 ? 2 : 1;
+    rw = kStepWarps / kw;
+    kg = warp & (kw - 1);
+    rg = warp / kw;
+    ld = kPartFloats / kw;
+  }
+  // n rows from the ring times the inputs xp: every warp's share of row r to part[kg][row0 + r], rows side by side for the
+  // threads that add the shares up.
+  template <int kFmt>
+  __device__ __forceinline__ void rows(int K, int n, const uint8_t* xp, int row0) {
+    const int rb = row_bytes(kFmt, K), per = chunk_rows(rb), units = K / unit_of(kFmt);
+    for (int r0 = 0; r0 < n; r0 += per, at.next()) {
+      if (!wait.warp_wait(&sh.full[at.st], at.parity, 2, r0)) return;
+      const uint8_t* w = base + lay.ring + sh.start[at.st];
+      const int nr = min(per, n - r0);
+      for (int r = rg; r < nr; r += 4 * rw) {
+        int off[4];
+#pragma unroll
+        for (int i = 0; i < 4; ++i) off[i] = min(r + i * rw, nr - 1) * rb;
+        float d[2][4] = {{0.f, 0.f, 0.f, 0.f}, {0.f, 0.f, 0.f, 0.f}};
+        if (r + 2 * rw < nr) {
+          for (int u = kg; u < units; u += kw) dot_unit<kFmt, 2>(d, w, off, false, xp, u, lane, K);
+        } else {
+          float one[1][4] = {{0.f, 0.f, 0.f, 0.f}};
+          for (int u = kg; u < units; u += kw) dot_unit<kFmt, 1>(one, w, off, r + rw >= nr, xp, u, lane, K);
+#pragma unroll
+          for (int j = 0; j < 4; ++j) d[0][j] = one[0][j];
+        }
+        // the lanes that hold a tile's diagonal, four sums over the lanes at once: lanes 8i .. 8i + 7 end up with row i
+        const bool diag = (lane >> 3) == (lane & 3), odd = lane & 4;
+        const float a = diag ? (odd ? d[0][1] : d[0][0]) : 0.f, b = diag ? (odd ? d[0][3] : d[0][2]) : 0.f;
+        const float c = diag ? (odd ? d[1][1] : d[1][0]) : 0.f, e = diag ? (odd ? d[1][3] : d[1][2]) : 0.f;
+        const bool up = lane & 16, right = lane & 8;
+        float p = up ? c : a, q = up ? e : b;
+        p += __shfl_xor_sync(0xffffffffu, up ? a : c, 16);
+        q += __shfl_xor_sync(0xffffffffu, up ? b : e, 16);
+        float v = (right ? q : p) + __shfl_xor_sync(0xffffffffu, right ? p : q, 8);
+#pragma unroll
+        for (int o = 4; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+        const int mine = r + (lane >> 3) * rw;
+        if ((lane & 7) == 0 && mine < nr) part()[kg * ld + row0 + r0 + mine] = v;
+      }
+      // every value read went into the sums stored above, so the reads are complete when the place is given back
+      __syncwarp();
+      if (lane == 0) mbar_arrive(&sh.empty[at.st]);
+    }
+  }
+  __device__ __forceinline__ float sum1(int row) const {
+    float v = 0.f;
+    for (int j = 0; j < kw; ++j) v += part()[j * ld + row];
+    return v;
+  }
+  __device__ __forceinline__ float2 sum2(int row) const {      // rows row, row + 1 (row even)
+    float2 v = make_float2(0.f, 0.f);
+#pragma unroll 4
+    for (int j = 0; j < kw; ++j) {
+      const float2 a = *reinterpret_cast<const float2*>(part() + j * ld + row);
+      v.x += a.x; v.y += a.y;
+    }
+    return v;
+  }
+  __device__ __forceinline__ float4 sum4(int row) const {      // four rows (row a multiple of 4)
+    float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll 4
+    for (int j = 0; j < kw; ++j) {
+      const float4 a = *reinterpret_cast<const float4*>(part() + j * ld + row);
+      v.x += a.x; v.y += a.y; v.z += a.z; v.w += a.w;
+    }
+    return v;
+  }
+  __device__ __forceinline__ bool failed() const { return *wait.fail != 0; }
+
+  // Attention of this SM's unit: queries and the new rows from the QKV entries, its pages from the ring, its share of the
+  // head's output to the entries `out`.
+  __device__ __forceinline__ void attention(int layer, int pos, const Pages& pg, const uint64_t* qkv, uint64_t* rec, uint64_t* ml,
+                                            uint64_t* out, uint32_t tag_in, uint32_t tag_rec, uint32_t tag_out) {
+    constexpr int D = VDC_HEAD_DIM;
+    const int G = s.group;
+    uint32_t* raw = reinterpret_cast<uint32_t*>(base + lay.raw);
+    uint32_t* qs = reinterpret_cast<uint32_t*>(base + lay.q);
+    uint32_t* krow = reinterpret_cast<uint32_t*>(base + lay.rows);
+    uint32_t* vrow = krow + D / 2;
+    const bool owner = pg.first + pg.count == min(pos / VDC_KV_PAGE + 1, s.max_pages);
+    // what the heads' prologue needs besides the entries is on its way before they are waited for
+    float2 cs = make_float2(0.f, 0.f), sn = cs;
+    uint32_t nlo = 0u, nhi = 0u;
+    const int i0 = lane * 2;
+    if (warp <= G) {
+      const float* rope = reinterpret_cast<const float*>(s.rope) + (size_t)pos * D;
+      cs = __ldg(reinterpret_cast<const float2*>(rope + i0));
+      sn = __ldg(reinterpret_cast<const float2*>(rope + 64 + i0));
+      if (s.qk_norm) {
+        const uint32_t* w = reinterpret_cast<const uint32_t*>(s.qk_norm) + (size_t)layer * D + (warp == G ? D / 2 : 0);
+        nlo = __ldg(w + lane);
+        nhi = __ldg(w + lane + 32);
+      }
+    }
+    collect<1>(qkv + (size_t)pg.h * (G + 2) * (D / 2), (G + 2) * D, tag_in,
+            [&](int i, uint32_t a, uint32_t b) { *reinterpret_cast<uint2*>(raw + 2 * i) = make_uint2(a, b); });
+    consumers_sync();
+    if (warp <= G) {
+      const uint32_t lo = raw[warp * (D / 2) + lane], hi = raw[warp * (D / 2) + lane + 32];
+      float a0 = bf_lo(lo), a1 = bf_hi(lo), b0 = bf_lo(hi), b1 = bf_hi(hi);
+      if (s.qk_norm) {
+        const float rs = rsqrtf(warp_sum(a0 * a0 + a1 * a1 + b0 * b0 + b1 * b1) / (float)D + s.qk_eps);
+        a0 = bf16_round(bf_lo(nlo) * bf16_round(a0 * rs));
+        a1 = bf16_round(bf_hi(nlo) * bf16_round(a1 * rs));
+        b0 = bf16_round(bf_lo(nhi) * bf16_round(b0 * rs));
+        b1 = bf16_round(bf_hi(nhi) * bf16_round(b1 * rs));
+      }
+      const uint32_t rlo = pack_bf16x2(bf16_round(a0 * cs.x) - bf16_round(b0 * sn.x), bf16_round(a1 * cs.y) - bf16_round(b1 * sn.y));
+      const uint32_t rhi = pack_bf16x2(bf16_round(b0 * cs.x) + bf16_round(a0 * sn.x), bf16_round(b1 * cs.y) + bf16_round(a1 * sn.y));
+      uint32_t* dst = warp < G ? qs + warp * kQLd : krow;
+      dst[lane] = rlo;
+      dst[lane + 32] = rhi;
+    } else if (warp == G + 1) {
+      vrow[lane] = raw[(G + 1) * (D / 2) + lane];
+      vrow[lane + 32] = raw[(G + 1) * (D / 2) + lane + 32];
+    }
+    consumers_sync();
+
+    const int group = warp >> 2, wq = warp & 3, gid = lane >> 2, t4 = lane & 3;
+    uint32_t q[8][2];
+#pragma unroll
+    for (int k = 0; k < 8; ++k) {
+      q[k][0] = gid < G ? qs[gid * kQLd + 8 * k + t4] : 0u;
+      q[k][1] = gid < G ? qs[gid * kQLd + 8 * k + 4 + t4] : 0u;
+    }
+    float* gm = reinterpret_cast<float*>(base + lay.gm) + group * 32;
+    float* wl = reinterpret_cast<float*>(base + lay.wl) + group * 40;
+    uint32_t* ps = reinterpret_cast<uint32_t*>(base + lay.p) + group * 8 * kPLd;
+    const uint32_t zero = smem_u32(vrow + D / 2);
+    const float scale_log2 = 1.4426950408889634f * rsqrtf((float)D);
+    const int lr = lane & 7, mi = lane >> 3;
+    float m[2] = {-INFINITY, -INFINITY}, l[2] = {0.f, 0.f}, o[2][4];
+#pragma unroll
+    for (int i = 0; i < 2; ++i)
+#pragma unroll
+      for (int j = 0; j < 4; ++j) o[i][j] = 0.f;
+    auto group_sync = [&] { asm volatile("bar.sync %0, 128;" ::"r"(2 + group) : "memory"); };
+    for (int i = 0; i < pg.count; ++i, at.next()) {
+      // every warp sees every page arrive (so that no phase of the ring passes unseen); one group of four works on it
+      const bool there = wait.warp_wait(&sh.full[at.st], at.parity, 3, i);
+      if ((i & (kGroups - 1)) == group) {      // all of a group's warps meet at its barriers, page or no page
+        uint8_t* page = base + lay.ring + (there ? sh.start[at.st] : 0);
+        const int valid = pos - (pg.first + i) * VDC_KV_PAGE;
+        const bool tail = owner && i == pg.count - 1;
+        if (tail && there && wq == 0) {
+          // the new position's rows, here and in the cache
+          const int r = pos % VDC_KV_PAGE, piece = lane & 15;
+          const uint4 v = reinterpret_cast<const uint4*>(krow)[lane];
+          *reinterpret_cast<uint4*>(page + (lane < 16 ? 0 : kPageBytes) + r * (D * 2) + ((piece ^ (r & 7)) << 4)) = v;
+          const size_t row = (size_t)ld_relaxed_gpu(reinterpret_cast<const int*>(s.state) + VDC_ST_NEWROW) * (D * 2);
+          const size_t pool = (size_t)layer * s.max_pages * s.n_kv * kPageBytes + (size_t)pg.h * kPageBytes;
+          uint8_t* to = reinterpret_cast<uint8_t*>(lane < 16 ? s.kpool : s.vpool) + pool + row;
+          if (!failed()) *reinterpret_cast<uint4*>(to + ((piece ^ (r & 7)) << 4)) = v;
+        }
+        if (tail) group_sync();
+        const uint32_t kb = smem_u32(page), vb = kb + kPageBytes;
+        // S^T = K Q^T: this warp's 16 positions on the tile's rows, the query heads on its columns
+        float c[4] = {0.f, 0.f, 0.f, 0.f}, c2[4] = {0.f, 0.f, 0.f, 0.f};
+        const int pk = wq * 16 + lr + 8 * (mi & 1), hk = mi >> 1;
+#pragma unroll
+        for (int k = 0; k < 8; k += 2) {
+          uint32_t a[4], a2[4];
+          ldsm_x4(a, kb + (uint32_t)(pk * 256 + (((2 * k + hk) ^ lr) << 4)));
+          ldsm_x4(a2, kb + (uint32_t)(pk * 256 + (((2 * k + 2 + hk) ^ lr) << 4)));
+          mma_16816(c, a[0], a[1], a[2], a[3], q[k][0], q[k][1]);
+          mma_16816(c2, a2[0], a2[1], a2[2], a2[3], q[k + 1][0], q[k + 1][1]);
+        }
+        const int p0 = wq * 16 + gid;
+        float e[4];
+#pragma unroll
+        for (int j = 0; j < 4; ++j) e[j] = p0 + 8 * (j >> 1) <= valid ? (c[j] + c2[j]) * scale_log2 : -INFINITY;
+        float mx[2] = {fmaxf(e[0], e[2]), fmaxf(e[1], e[3])};
+#pragma unroll
+        for (int z = 4; z < 32; z <<= 1) {
+          mx[0] = fmaxf(mx[0], __shfl_xor_sync(0xffffffffu, mx[0], z));
+          mx[1] = fmaxf(mx[1], __shfl_xor_sync(0xffffffffu, mx[1], z));
+        }
+        if (gid == 0) *reinterpret_cast<float2*>(gm + wq * 8 + 2 * t4) = make_float2(mx[0], mx[1]);
+        group_sync();
+        float al[2];
+#pragma unroll
+        for (int j = 0; j < 2; ++j) {
+          float mn = m[j];
+#pragma unroll
+          for (int w = 0; w < 4; ++w) mn = fmaxf(mn, gm[w * 8 + 2 * t4 + j]);
+          const bool none = mn == -INFINITY;
+          al[j] = none ? 1.f : exp2f(m[j] - mn);
+          e[j] = none ? 0.f : exp2f(e[j] - mn);
+          e[j + 2] = none ? 0.f : exp2f(e[j + 2] - mn);
+          m[j] = mn;
+          l[j] = l[j] * al[j] + e[j] + e[j + 2];      // this warp's positions only
+        }
+        // probabilities enter P V rounded to bf16, as a bf16 attention module hands them over
+        ps[gid * kPLd + wq * 8 + t4] = transpose8x8(pack_bf16x2(e[0], e[1]));
+        ps[gid * kPLd + wq * 8 + 4 + t4] = transpose8x8(pack_bf16x2(e[2], e[3]));
+        group_sync();
+        // O^T = V^T P^T: 32 of the head's dims per warp, all positions of the page
+#pragma unroll
+        for (int d = 0; d < 2; ++d)
+#pragma unroll
+          for (int j = 0; j < 4; ++j) o[d][j] *= al[j & 1];
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+          const int pv = k * 16 + lr + 8 * (mi >> 1), hv = mi & 1;
+          const uint32_t vr = pv <= valid ? vb + (uint32_t)(pv * 256) : zero;
+          const uint32_t b0 = ps[gid * kPLd + k * 8 + t4], b1 = ps[gid * kPLd + k * 8 + 4 + t4];
+#pragma unroll
+          for (int d = 0; d < 2; ++d) {
+            uint32_t va[4];
+            ldsm_x4_trans(va, vr + (uint32_t)(((2 * (2 * wq + d) + hv) ^ lr) << 4));
+            mma_16816(o[d], va[0], va[1], va[2], va[3], b0, b1);
+          }
+        }
+      }
+      fence_proxy_async_smem();
+      __syncwarp();
+      if (lane == 0) mbar_arrive(&sh.empty[at.st]);
+    }
+#pragma unroll
+    for (int z = 4; z < 32; z <<= 1) {
+      l[0] += __shfl_xor_sync(0xffffffffu, l[0], z);
+      l[1] += __shfl_xor_sync(0xffffffffu, l[1], z);
+    }
+    if (gid == 0) {
+      *reinterpret_cast<float2*>(wl + wq * 8 + 2 * t4) = make_float2(l[0], l[1]);
+      if (wq == 0) *reinterpret_cast<float2*>(wl + 32 + 2 * t4) = make_float2(m[0], m[1]);
+    }
+    float* po = part() + group * 8 * kOutLd;
+#pragma unroll
+    for (int d = 0; d < 2; ++d)
+#pragma unroll
+      for (int j = 0; j < 4; ++j) po[(2 * t4 + (j & 1)) * kOutLd + (2 * wq + d) * 16 + gid + 8 * (j >> 1)] = o[d][j];
+    consumers_sync();
+    if (failed()) return;
+
+    // the groups' sums: two dims of a head per thread
+    if (tid < G * (D / 2)) {
+      const int g = tid / (D / 2), d2 = tid % (D / 2);
+      const float* w0 = reinterpret_cast<const float*>(base + lay.wl);
+      float mm = -INFINITY;
+#pragma unroll
+      for (int k = 0; k < kGroups; ++k) mm = fmaxf(mm, w0[k * 40 + 32 + g]);
+      float n0 = 0.f, n1 = 0.f, den = 0.f;
+#pragma unroll
+      for (int k = 0; k < kGroups; ++k) {
+        const float mk = w0[k * 40 + 32 + g], wt = mk == -INFINITY ? 0.f : exp2f(mk - mm);
+        const float2 v = *reinterpret_cast<const float2*>(part() + (k * 8 + g) * kOutLd + 2 * d2);
+        n0 = fmaf(wt, v.x, n0);
+        n1 = fmaf(wt, v.y, n1);
+        den = fmaf(wt, w0[k * 40 + g] + w0[k * 40 + 8 + g] + w0[k * 40 + 16 + g] + w0[k * 40 + 24 + g], den);
+      }
+      if (pg.live == 1) {
+        const float inv = 1.f / den;
+        put(out + (size_t)pg.h * G * (D / 2) + tid, pack_bf16x2(n0 * inv, n1 * inv), tag_out);
+      } else {
+        const size_t u = (size_t)pg.h * s.n_splits + pg.split;
+        put2(rec + (u * G * (D / 2) + tid) * 2, __float_as_uint(n0), __float_as_uint(n1), tag_rec);
+        if (d2 == 0) put2(ml + (u * G + g) * 2, __float_as_uint(mm), __float_as_uint(den), tag_rec);
+      }
+    }
+    if (pg.live == 1) return;
+    // the head's pairs of dims are shared by its units: a lane per split
+    const int pairs = G * (D / 2), lo = pairs * pg.split / pg.live, hi = pairs * (pg.split + 1) / pg.live;
+    for (int i = lo + warp; i < hi; i += kStepWarps) {
+      float mk = -INFINITY, lk = 0.f, n0 = 0.f, n1 = 0.f;
+      bool ok = true;
+      if (lane < pg.live) {
+        const size_t u = (size_t)pg.h * s.n_splits + lane;
+        const uint64_t *rp = rec + (u * pairs + i) * 2, *mp = ml + (u * G + i / (D / 2)) * 2;
+        Two r = get2(rp), z = get2(mp);
+        ok = poll2(rp, tag_rec, r) && poll2(mp, tag_rec, z);
+        n0 = __uint_as_float((uint32_t)r.a);
+        n1 = __uint_as_float((uint32_t)r.b);
+        mk = __uint_as_float((uint32_t)z.a);
+        lk = __uint_as_float((uint32_t)z.b);
+      }
+      if (!__all_sync(0xffffffffu, ok)) break;
+      float mm = mk;
+#pragma unroll
+      for (int z = 16; z > 0; z >>= 1) mm = fmaxf(mm, __shfl_xor_sync(0xffffffffu, mm, z));
+      const float wt = mk == -INFINITY ? 0.f : exp2f(mk - mm);
+      const float den = warp_sum(wt * lk), a = warp_sum(wt * n0), b = warp_sum(wt * n1);
+      const float inv = 1.f / den;
+      if (lane == 0) put(out + (size_t)pg.h * pairs + i, pack_bf16x2(a * inv, b * inv), tag_out);
+    }
+  }
+
+  // The router's logits from their entries; every SM selects the experts for itself and tells its producer.
+  __device__ __forceinline__ void route(const uint64_t* buf, uint32_t tag) {
+    const int E = s.n_experts;
+    float* lg = reinterpret_cast<float*>(base + lay.route);
+    int* ids = reinterpret_cast<int*>(lg + kMaxExperts);
+    float* weights = reinterpret_cast<float*>(ids + kMaxTopK);
+    collect<1>(buf, 2 * E, tag, [&](int i, uint32_t a, uint32_t b) {
+      lg[2 * i] = __uint_as_float(a);
+      lg[2 * i + 1] = __uint_as_float(b);
+    });
+    consumers_sync();
+    if (warp == 0) {
+      constexpr int kMost = kMaxExperts / 32;
+      float v[kMost], mx = -INFINITY, sum = 0.f;
+#pragma unroll
+      for (int j = 0; j < kMost; ++j) {
+        v[j] = lane + 32 * j < E ? lg[lane + 32 * j] : -INFINITY;
+        mx = fmaxf(mx, v[j]);
+      }
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, o));
+#pragma unroll
+      for (int j = 0; j < kMost; ++j) {
+        v[j] = v[j] == -INFINITY ? 0.f : __expf(v[j] - mx);
+        sum += v[j];
+      }
+      sum = warp_sum(sum);
+      float all = 0.f, mine = 0.f;
+      int id = 0;
+      for (int k = 0; k < s.top_k; ++k) {
+        float bv = -1.f;
+        int bi = 0x7fffffff;
+#pragma unroll
+        for (int j = 0; j < kMost; ++j)
+          if (lane + 32 * j < E && v[j] > bv) {
+            bv = v[j];
+            bi = lane + 32 * j;
+          }
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) {
+          const float ov = __shfl_xor_sync(0xffffffffu, bv, o);
+          const int oi = __shfl_xor_sync(0xffffffffu, bi, o);
+          if (ov > bv || (ov == bv && oi < bi)) {
+            bv = ov;
+            bi = oi;
+          }
+        }
+        bi = min(bi, E - 1);               // logits without a number select nothing: any expert will do
+#pragma unroll
+        for (int j = 0; j < kMost; ++j)
+          if (bi == lane + 32 * j) v[j] = -1.f;
+        all += bv / sum;
+        if (lane == k) {
+          mine = bv / sum;
+          id = bi;
+        }
+      }
+      if (lane < s.top_k) {
+        ids[lane] = id;
+        weights[lane] = bf16_round(mine / all);
+        if (sm == 0) {
+          reinterpret_cast<int*>(s.route)[lane] = id;
+          reinterpret_cast<float*>(s.route)[16 + lane] = bf16_round(mine / all);
+        }
+      }
+      __syncwarp();
+      if (lane == 0 && !failed()) mbar_arrive(&sh.routed);
+    }
+    consumers_sync();
+  }
+};
+
+// ------------------------------------------------------------------------- //
+// the step
+// ------------------------------------------------------------------------- //
+template <int kFmt>
+__global__ void __launch_bounds__(kStepThreads + 32, 1) decode_step(const __grid_constant__ StepArgs args, vdc_status* status,
+                                                                    uint64_t timeout_ns) {
+  extern __shared__ uint8_t dyn[];
+  __shared__ StepShared sh;
+  const vdc_step& s = args.s;
+  const StepLayout& lay = args.lay;
+  const StepWork& wk = args.wk;
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, sm = blockIdx.x, sms = gridDim.x;
+  uint8_t* base = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(dyn) + 127) & ~(uintptr_t)127);
+  const Waiter wait{&sh.fail, status, timeout_ns, VDC_STEP_KIND};
+  constexpr int D = VDC_HEAD_DIM;
+  if (tid < kStages) {
+    const int k = s.n_experts ? s.top_k : 1, q = s.n_kv * s.group * D;
+    const int rows[kStages] = {q + 2 * s.n_kv * D, s.hidden, s.n_experts, 2 * s.ffn * k, s.hidden, s.vocab};
+    const Share r = share_of(rows[tid], tid == kGateUp ? 4 : tid == kRouter ? 1 : 2, sm, sms);
+    sh.share[tid][0] = r.r0;
+    sh.share[tid][1] = r.n;
+  }
+  if (tid == 0) {
+    for (int i = 0; i < kItems; ++i) {
+      mbar_init(&sh.full[i], 1);
+      mbar_init(&sh.empty[i], kStepWarps);
+    }
+    mbar_init(&sh.routed, 1);
+    sh.fail = 0;
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+  }
+  if (tid >= 64 && tid < 64 + D / 2) reinterpret_cast<uint32_t*>(base + lay.rows)[D + tid - 64] = 0u;     // a value row of zeros
+  grid_dep_wait();
+  grid_dep_launch();
+  if (__syncthreads_or(ld_relaxed_gpu(&status->abort))) {      // behind an unread error nothing runs
+    if (sm == 0 && tid == 0) *reinterpret_cast<int*>(s.work) += 1;
+    return;
+  }
+
+  const int H = s.hidden, F = s.ffn, G = s.group, Q = s.n_kv * G * D, QKV = Q + 2 * s.n_kv * D, L = s.n_layers, E = s.n_experts;
+  const int* state = reinterpret_cast<const int*>(s.state);
+  const int pos = ld_relaxed_gpu(state + VDC_ST_POS);
+  const Pages pg = pages_of(s, pos, sm);
+  const int slots = E ? s.top_k : 1;
+  const int rbH = row_bytes(kFmt, H), rbQ = row_bytes(kFmt, Q), rbF = row_bytes(kFmt, F);
+  int* ids = reinterpret_cast<int*>(base + lay.route + kMaxExperts * 4);
+  float* weights = reinterpret_cast<float*>(ids + kMaxTopK);
+
+  if (warp == kStepWarps) {
+    if (lane == 0) {
+      Producer p{sh, wait, base + lay.ring, lay.total - lay.ring};
+      const int* table = state + VDC_ST_PAGETABLE;
+      auto mine = [&](int stage, uint64_t w, size_t first, int rb) {      // this SM's rows of the matrix that begins at row `first`
+        p.rows(reinterpret_cast<const uint8_t*>(w) + (first + sh.share[stage][0]) * rb, rb, sh.share[stage][1]);
+      };
+      for (int l = 0; l < L && p.ok; ++l) {
+        mine(kQkv, s.wqkv, (size_t)l * QKV, rbH);
+        for (int i = 0; i < pg.count && p.ok; ++i) {
+          const size_t off = ((size_t)l * s.max_pages + ld_relaxed_gpu(table + pg.first + i)) * s.n_kv * kPageBytes + (size_t)pg.h * kPageBytes;
+          p.page(reinterpret_cast<const uint8_t*>(s.kpool) + off, reinterpret_cast<const uint8_t*>(s.vpool) + off);
+        }
+        mine(kOut, s.wo, (size_t)l * H, rbQ);
+        if (E == 0) {
+          mine(kGateUp, s.wgu, (size_t)l * 2 * F, rbH);
+          mine(kDown, s.wd, (size_t)l * H, rbF);
+          continue;
+        }
+        mine(kRouter, s.router, (size_t)l * E, rbH);
+        if (sh.share[kGateUp][1] || sh.share[kDown][1]) p.ok = p.ok && wait(&sh.routed, (uint32_t)l & 1u, 0, l);
+        if (!p.ok) break;
+        const int end = sh.share[kGateUp][0] + sh.share[kGateUp][1];
+        for (int r = sh.share[kGateUp][0]; r < end && p.ok;) {        // a slot's rows end where the next slot's begin
+          const int in = r % (2 * F), n = min(end - r, 2 * F - in);
+          p.rows(reinterpret_cast<const uint8_t*>(s.wgu) + (((size_t)l * E + ids[r / (2 * F)]) * 2 * F + in) * rbH, rbH, n);
+          r += n;
+        }
+        for (int e = 0; e < slots && p.ok; ++e) mine(kDown, s.wd, ((size_t)l * E + ids[e]) * H, rbF);
+      }
+      if (p.ok) mine(kVocab, s.lm_head, 0, H * 2);
+    }
+    __syncwarp();
+  } else {
+    uint64_t* work = reinterpret_cast<uint64_t*>(s.work);
+    const uint32_t tag0 = ((uint32_t)ld_relaxed_gpu(reinterpret_cast<const int*>(work)) * (uint32_t)(L + 1) + 1u) * 8u;
+    Consumer c{args, s, lay, sh, wait, base, tid, warp, lane, sm};
+    auto scaled2 = [&](int row, uint64_t sc, size_t at) {
+      float2 v = c.sum2(row);
+      if (kFmt) {
+        const float2 k = __ldg(reinterpret_cast<const float2*>(reinterpret_cast<const float*>(sc) + at));
+        v.x *= k.x; v.y *= k.y;
+      }
+      return v;
+    };
+    // a residual row pair: this SM's rows of a projection added to the hidden state it has in shared memory
+    auto residual = [&](int pair, float y0, float y1, uint64_t* out, uint32_t tag) {
+      const uint32_t h = c.hs()[pair];
+      put(out + pair, pack_bf16x2(bf_lo(h) + bf16_round(y0), bf_hi(h) + bf16_round(y1)), tag);
+    };
+    auto silu = [&](float g, float u) {
+      g = bf16_round(g);
+      return bf16_round(g / (1.f + __expf(-g))) * bf16_round(u);
+    };
+    auto keep_hidden = [&](uint64_t to) {        // SM 0: the hidden state as it came in, for whoever asks
+      if (sm == 0 && to && !c.failed())
+        for (int i = tid; i < H / 2; i += kStepThreads) reinterpret_cast<uint32_t*>(to)[i] = c.hs()[i];
+    };
+    const uint8_t* row = nullptr;
+    {
+      int token = ld_relaxed_gpu(state + VDC_ST_TOKEN);
+      if (token < 0 || token >= s.vocab) {
+        if (sm == 0 && tid == 0) report(status, VDC_ERR_TOKEN, VDC_STEP_KIND, 0, 0, token);
+        token = 0;
+      }
+      row = reinterpret_cast<const uint8_t*>(s.embed) + (size_t)token * H * 2;
+    }
+    float best = -INFINITY;
+    int best_row = 0x7fffffff;
+    // One loop over the layers' stages, with the vocabulary projection as the first stage behind the last layer: each piece of
+    // code is there once, since what falls out of the instruction caches between two stages costs as much as the stage.
+    for (int l = 0, stage = kQkv; l < L || stage == kQkv;) {
+      const uint32_t tag = tag0 + (uint32_t)l * 8u;
+      const bool lm = l == L;
+      const int K = stage == kOut ? Q : stage == kDown ? F : H;
+      const Share r{sh.share[lm ? kVocab : stage][0], sh.share[lm ? kVocab : stage][1]};
+      // ---- inputs
+      bool skip = false;
+      if (stage == kQkv || stage == (E ? kRouter : kGateUp)) {
+        // whoever has rows of this stage, or of the one that adds to the hidden state, reads it
+        skip = !r.n && (lm ? sm != 0 : !sh.share[kOut][1] && (stage == kQkv || !sh.share[kGateUp][1]));
+        if (!skip) {
+          const uint64_t w = lm ? s.norm_w : (stage == kQkv ? s.ln1 : s.ln2) + (size_t)l * H * 2;
+          c.template hidden<kFmt>(work + wk.h + (stage == kQkv ? H / 2 : 0), stage == kQkv ? tag - 8u + 5u : tag + 4u, l == 0 && stage == kQkv ? row : nullptr, w, lm);
+          if (stage == kQkv && l > 0 && s.taps) keep_hidden(s.taps + (size_t)(l - 1) * H * 2);
+          if (lm) keep_hidden(s.hidden_out);
+        }
+      } else if (stage == kOut || stage == kDown) {
+        skip = !r.n;
+        if (!skip) {
+          c.template collect<7>(work + (stage == kOut ? wk.attn : wk.act), stage == kOut ? Q : F * slots, tag + (stage == kOut ? 3u : 6u),
+                    [&](int i, uint32_t a, uint32_t b) { c.template set_input<kFmt>(i, a, b, false); });
+          consumers_sync();
+        }
+      } else if (r.n || sh.share[kDown][1]) {      // kGateUp behind a router: its inputs are there, the experts are not
+        c.route(work + wk.router, tag + 7u);
+      }
+      // ---- rows, as many at a time as their partial sums have room for
+      if (lm && kFmt != 0) c.template split<0>(K);
+      else c.template split<kFmt>(K);
+      const int per = chunk_rows(2 * H), most = lm ? kPartFloats / c.kw / per * per : r.n;
+      for (int r0 = 0; r0 < r.n && !skip; r0 += most) {
+        const int n = min(most, r.n - r0);
+        if (lm && kFmt != 0) {
+          c.template rows<0>(K, n, c.x(), 0);
+        } else {
+          // experts: a slot's gate/up rows end where the next slot's begin; every slot's down rows have inputs of their own
+          const int segs = E && stage == kDown ? slots : 1;
+          for (int e = 0, done = 0; E && stage == kGateUp ? done < n : e < segs; ++e) {
+            const int take = E && stage == kGateUp ? min(n - done, 2 * F - (r.r0 + done) % (2 * F)) : n;
+            c.template rows<kFmt>(K, take, c.x() + (segs > 1 ? (size_t)e * F * 2 : 0), segs > 1 ? e * n : done);
+            done += take;
+          }
+        }
+        consumers_sync();
+        if (!c.failed()) {
+          const size_t row_at = (size_t)l * (stage == kQkv ? QKV : stage == kGateUp ? 2 * F : H) + r.r0;      // of the scales
+          if (lm) {
+            for (int i = tid; i < n / 2; i += kStepThreads) {
+              const int rr = r.r0 + r0 + 2 * i;
+              const float2 y = c.sum2(2 * i);
+              const uint32_t v = pack_bf16x2(y.x, y.y);
+              reinterpret_cast<uint32_t*>(s.logits)[rr >> 1] = v;
+              if (bf_lo(v) > best) {
+                best = bf_lo(v);
+                best_row = rr;
+              }
+              if (bf_hi(v) > best) {
+                best = bf_hi(v);
+                best_row = rr + 1;
+              }
+            }
+          } else if (stage == kQkv) {
+            for (int i = tid; i < n / 2; i += kStepThreads) {
+              const float2 y = scaled2(2 * i, s.s_qkv, row_at + 2 * i);
+              put(work + wk.qkv + (r.r0 >> 1) + i, pack_bf16x2(y.x, y.y), tag + 1u);
+            }
+          } else if (stage == kRouter) {
+            if (tid < n) put(work + wk.router + r.r0 + tid, __float_as_uint(c.sum1(tid)), tag + 7u);
+          } else if (stage == kGateUp) {
+            for (int i = tid; i < n / 4; i += kStepThreads) {
+              float4 y = c.sum4(4 * i);
+              if (kFmt) {
+                const float4 k = __ldg(reinterpret_cast<const float4*>(reinterpret_cast<const float*>(s.s_gu) + row_at) + i);
+                y.x *= k.x; y.y *= k.y; y.z *= k.z; y.w *= k.w;
+              }
+              put(work + wk.act + (r.r0 >> 2) + i, pack_bf16x2(silu(y.x, y.y), silu(y.z, y.w)), tag + 6u);
+            }
+          } else {
+            for (int i = tid; i < n / 2; i += kStepThreads) {
+              float2 y = make_float2(0.f, 0.f);
+              if (E && stage == kDown) {
+                for (int e = 0; e < slots; ++e) {
+                  const float2 v = c.sum2(e * n + 2 * i);
+                  y.x = fmaf(weights[e], bf16_round(v.x), y.x);
+                  y.y = fmaf(weights[e], bf16_round(v.y), y.y);
+                }
+              } else {
+                y = scaled2(2 * i, stage == kOut ? s.s_o : s.s_d, row_at + 2 * i);
+              }
+              residual((r.r0 >> 1) + i, y.x, y.y, work + wk.h + (stage == kDown ? H / 2 : 0), tag + (stage == kDown ? 5u : 4u));
+            }
+          }
+        }
+        if (lm) consumers_sync();
+      }
+      if (lm) break;
+      if (stage == kQkv && pg.count > 0)
+        c.attention(l, pos, pg, work + wk.qkv, work + wk.rec, work + wk.ml, work + wk.attn, tag + 1u, tag + 2u, tag + 3u);
+      if (stage == kDown) ++l;
+      stage = stage == kDown ? kQkv : stage == kOut ? (E ? kRouter : kGateUp) : stage + 1;
+    }
+    const uint32_t tag = tag0 + (uint32_t)L * 8u;
+    if (s.taps) keep_hidden(s.taps + (size_t)(L - 1) * H * 2);
+    auto better = [](float v, int r, float& bv, int& br) {      // the lowest row wins ties
+      if (v > bv || (v == bv && r < br)) {
+        bv = v;
+        br = r;
+      }
+    };
+    auto warp_best = [&](float& bv, int& br) {
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1) {
+        const float ov = __shfl_xor_sync(0xffffffffu, bv, o);
+        const int orow = __shfl_xor_sync(0xffffffffu, br, o);
+        better(ov, orow, bv, br);
+      }
+    };
+    warp_best(best, best_row);
+    if (lane == 0) {
+      sh.best[warp] = best;
+      sh.best_row[warp] = best_row;
+    }
+    consumers_sync();
+    if (warp == 0) {
+      best = lane < kStepWarps ? sh.best[lane] : -INFINITY;
+      best_row = lane < kStepWarps ? sh.best_row[lane] : 0x7fffffff;
+      warp_best(best, best_row);
+      if (lane == 0 && !c.failed()) put2(work + wk.best + 2 * sm, __float_as_uint(best), (uint32_t)best_row, tag + 1u);
+      if (sm == 0) {
+        best = -INFINITY;
+        best_row = 0x7fffffff;
+        bool ok = true;
+        for (int i = lane; i < sms && ok; i += 32) {
+          Two v = get2(work + wk.best + 2 * i);
+          ok = c.poll2(work + wk.best + 2 * i, tag + 1u, v);
+          if (ok) better(__uint_as_float((uint32_t)v.a), (int)(uint32_t)v.b, best, best_row);
+        }
+        warp_best(best, best_row);
+        ok = __all_sync(0xffffffffu, ok);
+        if (lane == 0) {
+          *reinterpret_cast<int*>(work) += 1;        // the next launch's tags are others, whatever became of this one
+          int* st = reinterpret_cast<int*>(s.state);
+          if (ok && !c.failed() && !ld_relaxed_gpu(&status->abort)) {
+            const int step = st[VDC_ST_STEP], next = pos + 1, page = next / VDC_KV_PAGE;
+            reinterpret_cast<int*>(s.log)[step] = best_row;
+            st[VDC_ST_TOKEN] = best_row;
+            st[VDC_ST_STEP] = step + 1;
+            st[VDC_ST_POS] = next;
+            st[VDC_ST_NPAGES] = page + 1;
+            if (page < st[VDC_ST_MAXPAGES])
+              st[VDC_ST_NEWROW] = st[VDC_ST_PAGETABLE + page] * VDC_KV_PAGE * st[VDC_ST_NKVH] + next % VDC_KV_PAGE;
+            else
+              st[VDC_ST_ERR] = 1;      // out of KV pages: the host must not launch another step
+          }
+        }
+      }
+    }
+  }
+  wait.drain();
+}
+
+}  // namespace vdc
+
+// 0 when the kernel can run this step, otherwise why not.
+extern "C" const char* vdc_step_refuses(const vdc_step* s, bool pointers) {
+  using namespace vdc;
+  auto al16 = [](uint64_t p) { return p != 0 && (p & 15) == 0; };
+  if (s->num_sms < 1 || s->num_sms > VDC_MAX_SMS || s->n_layers < 1 || s->wfmt < 0 || s->wfmt > 2) return "step: bad shape";
+  if ((s->group != 4 && s->group != 8) || s->n_kv < 1 || s->max_pages < 1 || s->max_seq < 1) return "step: bad heads or pages";
+  if (s->n_splits < 1 || s->n_splits > kMaxSplits || s->n_splits * s->n_kv > s->num_sms) return "step: more attention units than SMs";
+  const int u = unit_of(s->wfmt), Q = s->n_kv * s->group * VDC_HEAD_DIM;
+  if (s->hidden < 512 && s->hidden != 256) return "step: hidden too small";
+  if (s->hidden > 8192 || s->hidden % u || s->hidden % 256 || s->ffn < u || s->ffn % u || Q % u || s->vocab < 2 || s->vocab % 2)
+    return "step: widths not supported";
+  if (row_bytes(0, s->hidden) > kItemBytes || row_bytes(s->wfmt, s->ffn) > kItemBytes || row_bytes(s->wfmt, Q) > kItemBytes)
+    return "step: a weight row is longer than a copy";
+  if (s->n_experts && (s->wfmt || s->n_experts > kMaxExperts || s->n_experts % 2 || s->top_k < 1 || s->top_k > kMaxTopK || s->top_k > s->n_experts))
+    return "step: experts not supported";
+  const StepLayout l = step_layout(*s);
+  if (l.total - l.ring < 3 * kItemBytes) return "step: no room for the ring";
+  // the partial sums of an SM's rows
+  auto fits = [&](long long rows, int K, int fmt) {
+    const int units = K / unit_of(fmt), kw = units >= 16 ? 16 : units >= 8 ? 8 : units >= 4 ? 4 : units >= 2 ? 2 : 1;
+    return ((rows + s->num_sms - 1) / s->num_sms + 4) * kw <= kPartFloats;
+  };
+  const int k = s->n_experts ? s->top_k : 1;
+  if (!fits(Q + 2 * s->n_kv * VDC_HEAD_DIM, s->hidden, s->wfmt) || !fits(s->hidden, Q, s->wfmt) ||
+      !fits(2ll * s->ffn * k, s->hidden, s->wfmt) || !fits((long long)s->hidden * k, s->ffn, s->wfmt))
+    return "step: more rows per SM than partial sums have room for";
+  if (!pointers) return nullptr;
+  if (!al16(s->embed) || !al16(s->lm_head) || !al16(s->norm_w) || !al16(s->ln1) || !al16(s->ln2) || !al16(s->wqkv) || !al16(s->wo) ||
+      !al16(s->wgu) || !al16(s->wd) || !al16(s->kpool) || !al16(s->vpool) || !al16(s->rope) || !al16(s->logits) || !al16(s->hidden_out) ||
+      !al16(s->work) || !s->state || (s->state & 3) || !s->log || (s->log & 3) || (s->taps & 15) || (s->qk_norm & 15))
+    return "step: null or misaligned pointer";
+  if (s->wfmt && (!al16(s->s_qkv) || !al16(s->s_o) || !al16(s->s_gu) || !al16(s->s_d))) return "step: null or misaligned scales";
+  if (s->n_experts && (!al16(s->router) || !al16(s->route))) return "step: null or misaligned router";
+  return nullptr;
+}
+
+extern "C" long long vdc_step_words(const vdc_step* s) { return (long long)vdc::step_work(*s).words; }
+
+extern "C" cudaError_t vdc_step_prepare() {
+  const void* fs[] = {(const void*)vdc::decode_step<0>, (const void*)vdc::decode_step<1>, (const void*)vdc::decode_step<2>};
+  for (const void* f : fs)
+    if (cudaError_t e = cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, vdc::kStepSmem)) return e;
+  return cudaSuccess;
+}
+
+extern "C" cudaError_t vdc_step_launch(const vdc_step* s, vdc_status* status, uint64_t timeout_ns, cudaStream_t stream) {
+  cudaLaunchConfig_t cfg{};
+  cudaLaunchAttribute attr{};
+  attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr.val.programmaticStreamSerializationAllowed = 1;
+  cfg.stream = stream;
+  cfg.attrs = &attr;
+  cfg.numAttrs = 1;
+  cfg.gridDim = dim3((unsigned)s->num_sms);
+  cfg.blockDim = dim3(vdc::kStepThreads + 32);
+  cfg.dynamicSmemBytes = vdc::kStepSmem;
+  auto f = s->wfmt == 0 ? vdc::decode_step<0> : s->wfmt == 1 ? vdc::decode_step<1> : vdc::decode_step<2>;
+  const vdc::StepArgs args{*s, vdc::step_layout(*s), vdc::step_work(*s)};
+  return cudaLaunchKernelEx(&cfg, f, args, status, timeout_ns);
+}

@@ -651,6 +651,40 @@ class DecodeEngine:
         self.minsts = torch.from_numpy(m).to(self.dev)
         self.bars_init = torch.from_numpy(bars).to(self.dev)
         self.launches_per_step = 1
+        self.step_kernel = None
+
+    def _plan_step(self):
+        """The step as one persistent kernel (csrc/step_kernel.cu), or None where the program of the megakernel runs it: for
+        the options that describe that program, and for shapes the kernel refuses (rows longer than 32 KB, fewer SMs than KV
+        heads)."""
+        cfg = self.cfg
+        if self.shared_counters or self.split_down_wanted or self.l2_prefetch_bytes or not self.interleave:
+            return None
+        s = runtime.Step(num_sms=self.num_sms, n_layers=cfg.n_layers, hidden=cfg.hidden, ffn=cfg.ffn, vocab=cfg.vocab,
+                         n_kv=cfg.n_kv_heads, group=cfg.group, wfmt={"bf16": 0, "fp8": 1, "nvfp4": 2}[self.wkind],
+                         max_pages=self.max_pages, max_seq=self.max_seq, n_experts=cfg.n_experts,
+                         n_splits=min(self.num_sms // cfg.n_kv_heads, self.max_pages, 32),
+                         top_k=cfg.top_k if cfg.n_experts else 0, eps=cfg.eps, qk_eps=cfg.qk_norm_eps)
+        nbytes = runtime.step_workspace(s)
+        if nbytes is None:
+            return None
+        self.step_work = torch.zeros(nbytes // 8, dtype=torch.int64, device=self.dev)
+        for name, t in dict(embed=self.embed, lm_head=self.lm_head, norm_w=self.norm_w, ln1=self.ln1, ln2=self.ln2, wqkv=self.wqkv,
+                            wo=self.wo, wgu=self.wgu, wd=self.wd, s_qkv=self.scales.get("wqkv"), s_o=self.scales.get("wo"),
+                            s_gu=self.scales.get("wgu"), s_d=self.scales.get("wd"), qk_norm=self.qknorm, router=self.router,
+                            kpool=self.kpool, vpool=self.vpool, state=self.state, rope=self.rope, log=self.token_log,
+                            logits=self.logits, hidden_out=self.hidden, taps=self.taps,
+                            route=self.route if cfg.n_experts else None, work=self.step_work).items():
+            setattr(s, name, t.data_ptr() if t is not None else 0)
+        return s
+
+    def _launch(self):
+        """Enqueues one token."""
+        if self.step_kernel is not None:
+            runtime.launch_step(self.step_kernel, self.stream.cuda_stream, self.timeout_ns)
+        else:
+            runtime.launch_async(self.num_sms, self.insts_per_sm, self.cinsts, self.minsts, None, self.bars,
+                                 self.bars_init, self.profile, self.stream.cuda_stream, self.timeout_ns)
 
     def _plan_moe(self, P, plan, load, l, b_o, add_gemv):
         """Router, top-k routing and the selected experts' gate/up and down projections of layer l."""
@@ -834,8 +868,7 @@ class DecodeEngine:
         assert isa.ST_STEP == isa.ST_TOKEN + 1
         with torch.cuda.stream(self.stream):
             for t in range(T):
-                runtime.launch_async(self.num_sms, self.insts_per_sm, self.cinsts, self.minsts, None, self.bars,
-                                     self.bars_init, self.profile, self.stream.cuda_stream, self.timeout_ns)
+                self._launch()
                 if t + 1 < T:
                     word.copy_(forced[t], non_blocking=True)
         runtime.read_status(self.stream.cuda_stream)
@@ -849,8 +882,7 @@ class DecodeEngine:
         assert self.program is not None, "load weights first"
         if self.pos >= self.max_seq or self.steps_done >= self.max_steps:
             raise RuntimeError("out of KV pages or token-log space")
-        runtime.launch_async(self.num_sms, self.insts_per_sm, self.cinsts, self.minsts, None, self.bars,
-                             self.bars_init, self.profile, self.stream.cuda_stream, self.timeout_ns)
+        self._launch()
         self.pos += 1
         self.steps_done += 1
 

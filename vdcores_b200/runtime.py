@@ -41,6 +41,16 @@ class Stage(ctypes.Structure):
                                                   "state", "log", "rope", "qk_norm", "kpool", "vpool", "q")])
 
 
+class Step(ctypes.Structure):
+    """One token at batch 1 (vdc_step in include/vdcores.h, which documents the fields)."""
+    _fields_ = ([(n, ctypes.c_int32) for n in ("num_sms", "n_layers", "hidden", "ffn", "vocab", "n_kv", "group", "wfmt", "max_pages",
+                                               "max_seq", "n_splits", "n_experts", "top_k", "reserved")]
+                + [(n, ctypes.c_float) for n in ("eps", "qk_eps")]
+                + [(n, ctypes.c_uint64) for n in ("embed", "lm_head", "norm_w", "ln1", "ln2", "wqkv", "wo", "wgu", "wd", "s_qkv",
+                                                  "s_o", "s_gu", "s_d", "qk_norm", "router", "kpool", "vpool", "state", "rope", "log",
+                                                  "logits", "hidden_out", "taps", "route", "work")])
+
+
 _u64, _i32, _vp = ctypes.c_uint64, ctypes.c_int, ctypes.c_void_p
 _lib.vdc_version.restype = _i32
 _lib.vdc_init.restype = _i32
@@ -52,6 +62,8 @@ _lib.vdc_launch_static.argtypes = [_i32, _i32, _vp, _vp, _vp, _vp, _u64, _u64, c
 _lib.vdc_launch_stages.argtypes = [ctypes.POINTER(Stage), _i32, _u64, _u64]
 _lib.vdc_launch_stages_limited.argtypes = [ctypes.POINTER(Stage), _i32, _i32, _u64, _u64]
 _lib.vdc_count_stage_launches.argtypes = [ctypes.POINTER(Stage), _i32, _i32, ctypes.POINTER(_i32), ctypes.POINTER(_i32)]
+_lib.vdc_step_workspace.argtypes = [ctypes.POINTER(Step), ctypes.POINTER(_u64)]
+_lib.vdc_launch_step.argtypes = [ctypes.POINTER(Step), _u64, _u64]
 _lib.vdc_wide_tiles.argtypes = [_i32] * 6 + [ctypes.POINTER(_i32)]
 _lib.vdc_read_status.argtypes = [_u64, ctypes.POINTER(Status), _i32]
 _lib.vdc_build_tma_desc.argtypes = [_vp, _vp, _i32, _i32, ctypes.POINTER(_u64), ctypes.POINTER(_u64),
@@ -83,7 +95,7 @@ _lib.vdc_validate_streams.restype = _i32
 EXPORTED_SYMBOLS = [
     "vdc_version", "vdc_init", "vdc_set_smem_size", "vdc_launch", "vdc_launch_async", "vdc_launch_async_full",
     "vdc_launch_static", "vdc_launch_stages", "vdc_launch_stages_limited",
-    "vdc_count_stage_launches", "vdc_wide_tiles",
+    "vdc_count_stage_launches", "vdc_wide_tiles", "vdc_step_workspace", "vdc_launch_step",
     "vdc_read_status",
     "vdc_build_tma_desc", "vdc_set_cache_policy", "vdc_enable_peer_access", "vdc_ipc_open", "vdc_ipc_close", "vdc_peer_alloc", "vdc_peer_free", "vdc_ipc_export", "vdc_opcode_count", "vdc_opcode_name", "vdc_opcode_value",
     "vdc_opcode_is_compute", "vdc_config", "vdc_family_specs", "vdc_last_error", "vdc_validate_streams",
@@ -204,6 +216,18 @@ def count_stage_launches(stages, max_ctas=0):
     launches, largest = _i32(), _i32()
     _check(_lib.vdc_count_stage_launches(stages, len(stages), int(max_ctas), ctypes.byref(launches), ctypes.byref(largest)))
     return launches.value, largest.value
+
+
+def step_workspace(step):
+    """Bytes of the workspace a Step needs, or None where the step kernel cannot run it; needs no GPU."""
+    n = _u64()
+    return int(n.value) if _lib.vdc_step_workspace(ctypes.byref(step), ctypes.byref(n)) == 0 else None
+
+
+def launch_step(step, stream=0, timeout_ns=0):
+    """Enqueues one token of a model at batch 1; no synchronisation."""
+    init()
+    _check(_lib.vdc_launch_step(ctypes.byref(step), int(stream), int(timeout_ns)))
 
 
 def wide_tiles(rows, M, K, wfmt, sms, whole=False):
