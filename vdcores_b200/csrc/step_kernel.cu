@@ -164,6 +164,23 @@ __device__ __forceinline__ void expand(uint32_t (&o)[kFmt == 2 ? 4 : 2], const u
   }
 }
 
+// bf16 rows: packed fp32 FMAs of the widened pairs, per row one sum of the even and one of the odd weights (which are as many
+// instructions as the tensor cores' products below would take away again in picking sums out of their tiles).
+template <int kPairs>
+__device__ __forceinline__ void dot_bf16(float2 (&d)[2 * kPairs], const uint8_t* w, const int (&row)[4], const uint8_t* x, int u, int lane) {
+  auto pair = [](uint32_t v) { return make_float2(bf_lo(v), bf_hi(v)); };
+  const uint4 xv = lds128(x + u * 512 + lane * 16);
+  const float2 xf[4] = {pair(xv.x), pair(xv.y), pair(xv.z), pair(xv.w)};
+#pragma unroll
+  for (int i = 0; i < 2 * kPairs; ++i) {
+    const uint4 v = lds128(w + row[i] + u * 512 + lane * 16);
+    d[i] = __ffma2_rn(pair(v.x), xf[0], d[i]);
+    d[i] = __ffma2_rn(pair(v.y), xf[1], d[i]);
+    d[i] = __ffma2_rn(pair(v.z), xf[2], d[i]);
+    d[i] = __ffma2_rn(pair(v.w), xf[3], d[i]);
+  }
+}
+
 // One step of a warp: 16 bytes per lane of kPairs pairs of rows times the same inputs, as products of 16 x 16 by 16 x 8 tiles.
 // Row g of a tile is what the four lanes 4g .. 4g + 3 hold of the pair's first row (8 + g: of its second), column g what they
 // hold of the inputs: the tile's element (g, g) is the sum of the four lanes' products, the other elements mean nothing.  An
@@ -208,8 +225,8 @@ __device__ __forceinline__ void dot_unit(float (&d)[kPairs][4], const uint8_t* w
 // Units of q rows; the first SMs' shares are never empty while there are any.
 __device__ __forceinline__ Share share_of(int rows, int q, int sm, int sms) {
   const int units = rows / q;
-  const int a = (int)(((long long)units * sm + sms - 1) / sms), b = (int)(((long long)units * (sm + 1) + sms - 1) / sms);
-  return {a * q, (b - a) * q};
+  const int each = units / sms, more = units % sms;             // the first `more` SMs take one unit more
+  return {(sm * each + min(sm, more)) * q, (each + (sm < more ? 1 : 0)) * q};
 }
 __host__ __device__ constexpr int chunk_rows(int rb) {        // an even number where more than one
   const int n = kItemBytes / rb < 32 ? kItemBytes / rb : 32;
@@ -232,6 +249,7 @@ struct Producer {
   // Room for one more item of `bytes`, freeing the oldest ones as they are consumed.
   __device__ __forceinline__ uint8_t* room(int bytes) {
     bytes = (bytes + 127) & ~127;
+#pragma unroll 1
     while (ok) {
       if (live < kItems) {
         if (live == 0) {
@@ -259,26 +277,20 @@ struct Producer {
     ++live;
     return p;
   }
-  __device__ __forceinline__ void copy(const uint8_t* src, int bytes) {
-    uint8_t* p = room(bytes);
-    if (!ok) return;
-    mbar_arrive_expect_tx(&sh.full[at.st], (uint32_t)bytes);
-    bulk_load_1d(p, src, (uint32_t)bytes, &sh.full[at.st]);
-    at.next();
-    ++count;
-  }
-  __device__ __forceinline__ void rows(const uint8_t* w, int rb, int n) {
-    const int per = chunk_rows(rb);
-    for (int r = 0; r < n && ok; r += per) copy(w + (size_t)r * rb, min(per, n - r) * rb);
-  }
-  __device__ __forceinline__ void page(const uint8_t* k, const uint8_t* v) {
-    uint8_t* p = room(2 * kPageBytes);
-    if (!ok) return;
-    mbar_arrive_expect_tx(&sh.full[at.st], 2 * kPageBytes);
-    bulk_load_1d(p, k, kPageBytes, &sh.full[at.st]);
-    bulk_load_1d(p + kPageBytes, v, kPageBytes, &sh.full[at.st]);
-    at.next();
-    ++count;
+  // n pieces of at most `bytes` (the last one `last`), one behind the other from src; with `second` a piece of the same size from
+  // there joins each one's item.
+  __device__ __forceinline__ void copy(const uint8_t* src, const uint8_t* second, int n, int bytes, int last) {
+#pragma unroll 1
+    for (int i = 0; i < n; ++i) {
+      const int size = i + 1 < n ? bytes : last;
+      uint8_t* p = room(second ? 2 * size : size);
+      if (!ok) return;
+      mbar_arrive_expect_tx(&sh.full[at.st], (uint32_t)(second ? 2 * size : size));
+      bulk_load_1d(p, src + (size_t)i * bytes, (uint32_t)size, &sh.full[at.st]);
+      if (second) bulk_load_1d(p + size, second, (uint32_t)size, &sh.full[at.st]);
+      at.next();
+      ++count;
+    }
   }
 };
 
@@ -319,8 +331,7 @@ struct Consumer {
   __device__ __forceinline__ uint8_t* x() const { return base + lay.x; }
 
   // Whether to look again for entries that are not there yet (it: looks so far); false when the wait was given up.
-  __device__ __forceinline__ bool again(const uint64_t* p, uint32_t it, uint64_t& t0) const {
-    if ((it & 63u) != 0) return true;
+  __device__ __noinline__ bool again(const uint64_t* p, uint32_t it, uint64_t& t0) const {
     if (*wait.fail) return false;
     if (ld_relaxed_gpu(&wait.status->abort) == 0) {
       const uint64_t now = globaltimer_ns();
@@ -333,8 +344,9 @@ struct Consumer {
   }
   __device__ __forceinline__ bool poll2(const uint64_t* p, uint32_t tag, Two& v) const {
     uint64_t t0 = 0;
+#pragma unroll 1
     for (uint32_t it = 1; !v.are(tag); ++it) {
-      if (!again(p, it, t0)) return false;
+      if ((it & 63u) == 0 && !again(p, it, t0)) return false;
       v = get2(p);
     }
     return true;
@@ -343,19 +355,21 @@ struct Consumer {
   // a thread still misses is looked for at the same time: one after another, each look is a round trip of its own.
   template <int kBatch, class F>
   __device__ __forceinline__ void collect(const uint64_t* buf, int n, uint32_t tag, F f) const {
+#pragma unroll 1
     for (int i0 = tid; i0 < n / 4; i0 += kBatch * kStepThreads) {
       Two v[kBatch];
 #pragma unroll
       for (int j = 0; j < kBatch; ++j)
         if (i0 + j * kStepThreads < n / 4) v[j] = get2(buf + 2 * (i0 + j * kStepThreads));
       uint64_t t0 = 0;
+#pragma unroll 1
       for (uint32_t it = 1;; ++it) {
         bool all = true;
 #pragma unroll
         for (int j = 0; j < kBatch; ++j)
           if (i0 + j * kStepThreads < n / 4) all = all && v[j].are(tag);
         if (all) break;
-        if (!again(buf + 2 * i0, it, t0)) return;
+        if ((it & 63u) == 0 && !again(buf + 2 * i0, it, t0)) return;
 #pragma unroll
         for (int j = 0; j < kBatch; ++j)
           if (i0 + j * kStepThreads < n / 4 && !v[j].are(tag)) v[j] = get2(buf + 2 * (i0 + j * kStepThreads));
@@ -397,6 +411,7 @@ struct Consumer {
       ssq = fmaf(bf_lo(a), bf_lo(a), fmaf(bf_hi(a), bf_hi(a), fmaf(bf_lo(b), bf_lo(b), fmaf(bf_hi(b), bf_hi(b), ssq))));
     };
     if (row != nullptr) {
+#pragma unroll 1
       for (int i = tid; i < H / 4; i += kStepThreads) {
         const uint2 v = __ldg(reinterpret_cast<const uint2*>(row) + i);
         keep(i, v.x, v.y);
@@ -439,27 +454,50 @@ struct Consumer {
   template <int kFmt>
   __device__ __forceinline__ void rows(int K, int n, const uint8_t* xp, int row0) {
     const int rb = row_bytes(kFmt, K), per = chunk_rows(rb), units = K / unit_of(kFmt);
+#pragma unroll 1
     for (int r0 = 0; r0 < n; r0 += per, at.next()) {
       if (!wait.warp_wait(&sh.full[at.st], at.parity, 2, r0)) return;
       const uint8_t* w = base + lay.ring + sh.start[at.st];
       const int nr = min(per, n - r0);
+#pragma unroll 1
       for (int r = rg; r < nr; r += 4 * rw) {
         int off[4];
 #pragma unroll
         for (int i = 0; i < 4; ++i) off[i] = min(r + i * rw, nr - 1) * rb;
-        float d[2][4] = {{0.f, 0.f, 0.f, 0.f}, {0.f, 0.f, 0.f, 0.f}};
-        if (r + 2 * rw < nr) {
-          for (int u = kg; u < units; u += kw) dot_unit<kFmt, 2>(d, w, off, false, xp, u, lane, K);
+        float a, b, c = 0.f, e = 0.f;          // the lane's share of the four rows
+        if (kFmt == 0) {
+          if (r + 2 * rw < nr) {
+            float2 d[4] = {};
+#pragma unroll 1
+            for (int u = kg; u < units; u += kw) dot_bf16<2>(d, w, off, xp, u, lane);
+            a = d[0].x + d[0].y; b = d[1].x + d[1].y; c = d[2].x + d[2].y; e = d[3].x + d[3].y;
+          } else {
+            float2 d[2] = {};
+#pragma unroll 1
+            for (int u = kg; u < units; u += kw) dot_bf16<1>(d, w, off, xp, u, lane);
+            a = d[0].x + d[0].y; b = d[1].x + d[1].y;
+          }
         } else {
-          float one[1][4] = {{0.f, 0.f, 0.f, 0.f}};
-          for (int u = kg; u < units; u += kw) dot_unit<kFmt, 1>(one, w, off, r + rw >= nr, xp, u, lane, K);
-#pragma unroll
-          for (int j = 0; j < 4; ++j) d[0][j] = one[0][j];
+          // of a tile the lanes that hold its diagonal
+          const bool diag = (lane >> 3) == (lane & 3), odd = lane & 4;
+          auto share = [&](const float (&d)[4], float& first, float& second) {
+            first = diag ? (odd ? d[1] : d[0]) : 0.f;
+            second = diag ? (odd ? d[3] : d[2]) : 0.f;
+          };
+          if (r + 2 * rw < nr) {
+            float d[2][4] = {};
+#pragma unroll 1
+            for (int u = kg; u < units; u += kw) dot_unit<kFmt, 2>(d, w, off, false, xp, u, lane, K);
+            share(d[0], a, b);
+            share(d[1], c, e);
+          } else {
+            float d[1][4] = {};
+#pragma unroll 1
+            for (int u = kg; u < units; u += kw) dot_unit<kFmt, 1>(d, w, off, r + rw >= nr, xp, u, lane, K);
+            share(d[0], a, b);
+          }
         }
-        // the lanes that hold a tile's diagonal, four sums over the lanes at once: lanes 8i .. 8i + 7 end up with row i
-        const bool diag = (lane >> 3) == (lane & 3), odd = lane & 4;
-        const float a = diag ? (odd ? d[0][1] : d[0][0]) : 0.f, b = diag ? (odd ? d[0][3] : d[0][2]) : 0.f;
-        const float c = diag ? (odd ? d[1][1] : d[1][0]) : 0.f, e = diag ? (odd ? d[1][3] : d[1][2]) : 0.f;
+        // four sums over the lanes at once: lanes 8i .. 8i + 7 end up with row i
         const bool up = lane & 16, right = lane & 8;
         float p = up ? c : a, q = up ? e : b;
         p += __shfl_xor_sync(0xffffffffu, up ? a : c, 16);
@@ -477,6 +515,7 @@ struct Consumer {
   }
   __device__ __forceinline__ float sum1(int row) const {
     float v = 0.f;
+#pragma unroll 4
     for (int j = 0; j < kw; ++j) v += part()[j * ld + row];
     return v;
   }
@@ -568,6 +607,7 @@ struct Consumer {
 #pragma unroll
       for (int j = 0; j < 4; ++j) o[i][j] = 0.f;
     auto group_sync = [&] { asm volatile("bar.sync %0, 128;" ::"r"(2 + group) : "memory"); };
+#pragma unroll 1
     for (int i = 0; i < pg.count; ++i, at.next()) {
       // every warp sees every page arrive (so that no phase of the ring passes unseen); one group of four works on it
       const bool there = wait.warp_wait(&sh.full[at.st], at.parity, 3, i);
@@ -694,6 +734,7 @@ struct Consumer {
     if (pg.live == 1) return;
     // the head's pairs of dims are shared by its units: a lane per split
     const int pairs = G * (D / 2), lo = pairs * pg.split / pg.live, hi = pairs * (pg.split + 1) / pg.live;
+#pragma unroll 1
     for (int i = lo + warp; i < hi; i += kStepWarps) {
       float mk = -INFINITY, lk = 0.f, n0 = 0.f, n1 = 0.f;
       bool ok = true;
@@ -747,6 +788,7 @@ struct Consumer {
       sum = warp_sum(sum);
       float all = 0.f, mine = 0.f;
       int id = 0;
+#pragma unroll 1
       for (int k = 0; k < s.top_k; ++k) {
         float bv = -1.f;
         int bi = 0x7fffffff;
@@ -842,33 +884,67 @@ __global__ void __launch_bounds__(kStepThreads + 32, 1) decode_step(const __grid
     if (lane == 0) {
       Producer p{sh, wait, base + lay.ring, lay.total - lay.ring};
       const int* table = state + VDC_ST_PAGETABLE;
-      auto mine = [&](int stage, uint64_t w, size_t first, int rb) {      // this SM's rows of the matrix that begins at row `first`
-        p.rows(reinterpret_cast<const uint8_t*>(w) + (first + sh.share[stage][0]) * rb, rb, sh.share[stage][1]);
-      };
-      for (int l = 0; l < L && p.ok; ++l) {
-        mine(kQkv, s.wqkv, (size_t)l * QKV, rbH);
-        for (int i = 0; i < pg.count && p.ok; ++i) {
-          const size_t off = ((size_t)l * s.max_pages + ld_relaxed_gpu(table + pg.first + i)) * s.n_kv * kPageBytes + (size_t)pg.h * kPageBytes;
-          p.page(reinterpret_cast<const uint8_t*>(s.kpool) + off, reinterpret_cast<const uint8_t*>(s.vpool) + off);
+      // stage after stage; a stage is one run of rows or several (experts), the attention one run per page
+      int l = 0, stage = kQkv, sub = 0;
+#pragma unroll 1
+      while (p.ok) {
+        asm volatile("" : "+r"(stage), "+r"(sub));
+        const uint8_t *src = nullptr, *second = nullptr;
+        int n = 0, rb = rbH, r0 = sh.share[stage][0], rows = sh.share[stage][1];
+        bool more = false;                     // the stage goes on
+        if (stage == kQkv) {
+          src = reinterpret_cast<const uint8_t*>(s.wqkv) + (size_t)l * QKV * rbH;
+          if (sub > 0) {                       // page sub - 1
+            rows = 0;
+            if (sub <= pg.count) {
+              const size_t off = ((size_t)l * s.max_pages + ld_relaxed_gpu(table + pg.first + sub - 1)) * s.n_kv * kPageBytes + (size_t)pg.h * kPageBytes;
+              src = reinterpret_cast<const uint8_t*>(s.kpool) + off;
+              second = reinterpret_cast<const uint8_t*>(s.vpool) + off;
+              rows = 1;
+              r0 = 0;
+              rb = kPageBytes;
+            }
+          }
+          more = sub < pg.count;
+        } else if (stage == kOut) {
+          rb = rbQ;
+          src = reinterpret_cast<const uint8_t*>(s.wo) + (size_t)l * H * rbQ;
+        } else if (stage == kRouter) {
+          src = reinterpret_cast<const uint8_t*>(s.router) + (size_t)l * E * rbH;
+        } else if (stage == kGateUp) {
+          src = reinterpret_cast<const uint8_t*>(s.wgu);
+          size_t first = (size_t)l * 2 * F;
+          if (E) {                             // a slot's rows end where the next slot's begin
+            if (sub == 0 && (rows || sh.share[kDown][1]) && !(p.ok = wait(&sh.routed, (uint32_t)l & 1u, 0, l))) break;
+            const int end = r0 + rows, slot = r0 / (2 * F) + sub;
+            r0 = max(r0, slot * 2 * F);
+            rows = min(end, (slot + 1) * 2 * F) - r0;
+            more = r0 + rows < end;
+            first = rows > 0 ? ((size_t)l * E + ids[slot]) * 2 * F : 0;
+            r0 -= slot * 2 * F;
+          }
+          src += first * rbH;
+        } else if (stage == kDown) {
+          rb = rbF;
+          more = sub + 1 < slots;
+          src = reinterpret_cast<const uint8_t*>(s.wd) + (E ? ((size_t)l * E + ids[sub]) * H : (size_t)l * H) * rbF;
+          if (!rows) more = false;
+        } else {
+          rb = H * 2;
+          src = reinterpret_cast<const uint8_t*>(s.lm_head);
         }
-        mine(kOut, s.wo, (size_t)l * H, rbQ);
-        if (E == 0) {
-          mine(kGateUp, s.wgu, (size_t)l * 2 * F, rbH);
-          mine(kDown, s.wd, (size_t)l * H, rbF);
-          continue;
+        if (rows > 0) {
+          const int per = second ? 1 : chunk_rows(rb);
+          n = (rows + per - 1) / per;
+          p.copy(src + (size_t)r0 * rb, second, n, per * rb, (rows - (n - 1) * per) * rb);
         }
-        mine(kRouter, s.router, (size_t)l * E, rbH);
-        if (sh.share[kGateUp][1] || sh.share[kDown][1]) p.ok = p.ok && wait(&sh.routed, (uint32_t)l & 1u, 0, l);
-        if (!p.ok) break;
-        const int end = sh.share[kGateUp][0] + sh.share[kGateUp][1];
-        for (int r = sh.share[kGateUp][0]; r < end && p.ok;) {        // a slot's rows end where the next slot's begin
-          const int in = r % (2 * F), n = min(end - r, 2 * F - in);
-          p.rows(reinterpret_cast<const uint8_t*>(s.wgu) + (((size_t)l * E + ids[r / (2 * F)]) * 2 * F + in) * rbH, rbH, n);
-          r += n;
-        }
-        for (int e = 0; e < slots && p.ok; ++e) mine(kDown, s.wd, ((size_t)l * E + ids[e]) * H, rbF);
+        if (stage == kVocab) break;
+        ++sub;
+        if (more) continue;
+        sub = 0;
+        if (stage == kDown) stage = ++l == L ? kVocab : kQkv;
+        else stage = stage == kOut && !E ? kGateUp : stage + 1;
       }
-      if (p.ok) mine(kVocab, s.lm_head, 0, H * 2);
     }
     __syncwarp();
   } else {
@@ -894,6 +970,7 @@ __global__ void __launch_bounds__(kStepThreads + 32, 1) decode_step(const __grid
     };
     auto keep_hidden = [&](uint64_t to) {        // SM 0: the hidden state as it came in, for whoever asks
       if (sm == 0 && to && !c.failed())
+#pragma unroll 1
         for (int i = tid; i < H / 2; i += kStepThreads) reinterpret_cast<uint32_t*>(to)[i] = c.hs()[i];
     };
     const uint8_t* row = nullptr;
@@ -909,7 +986,9 @@ __global__ void __launch_bounds__(kStepThreads + 32, 1) decode_step(const __grid
     int best_row = 0x7fffffff;
     // One loop over the layers' stages, with the vocabulary projection as the first stage behind the last layer: each piece of
     // code is there once, since what falls out of the instruction caches between two stages costs as much as the stage.
+#pragma unroll 1
     for (int l = 0, stage = kQkv; l < L || stage == kQkv;) {
+      asm volatile("" : "+r"(stage), "+r"(l));      // the compiler would otherwise make a copy of the loop for every stage
       const uint32_t tag = tag0 + (uint32_t)l * 8u;
       const bool lm = l == L;
       const int K = stage == kOut ? Q : stage == kDown ? F : H;
@@ -939,6 +1018,7 @@ __global__ void __launch_bounds__(kStepThreads + 32, 1) decode_step(const __grid
       if (lm && kFmt != 0) c.template split<0>(K);
       else c.template split<kFmt>(K);
       const int per = chunk_rows(2 * H), most = lm ? kPartFloats / c.kw / per * per : r.n;
+#pragma unroll 1
       for (int r0 = 0; r0 < r.n && !skip; r0 += most) {
         const int n = min(most, r.n - r0);
         if (lm && kFmt != 0) {
@@ -946,6 +1026,7 @@ __global__ void __launch_bounds__(kStepThreads + 32, 1) decode_step(const __grid
         } else {
           // experts: a slot's gate/up rows end where the next slot's begin; every slot's down rows have inputs of their own
           const int segs = E && stage == kDown ? slots : 1;
+#pragma unroll 1
           for (int e = 0, done = 0; E && stage == kGateUp ? done < n : e < segs; ++e) {
             const int take = E && stage == kGateUp ? min(n - done, 2 * F - (r.r0 + done) % (2 * F)) : n;
             c.template rows<kFmt>(K, take, c.x() + (segs > 1 ? (size_t)e * F * 2 : 0), segs > 1 ? e * n : done);
@@ -956,6 +1037,7 @@ __global__ void __launch_bounds__(kStepThreads + 32, 1) decode_step(const __grid
         if (!c.failed()) {
           const size_t row_at = (size_t)l * (stage == kQkv ? QKV : stage == kGateUp ? 2 * F : H) + r.r0;      // of the scales
           if (lm) {
+#pragma unroll 1
             for (int i = tid; i < n / 2; i += kStepThreads) {
               const int rr = r.r0 + r0 + 2 * i;
               const float2 y = c.sum2(2 * i);
@@ -971,6 +1053,7 @@ __global__ void __launch_bounds__(kStepThreads + 32, 1) decode_step(const __grid
               }
             }
           } else if (stage == kQkv) {
+#pragma unroll 1
             for (int i = tid; i < n / 2; i += kStepThreads) {
               const float2 y = scaled2(2 * i, s.s_qkv, row_at + 2 * i);
               put(work + wk.qkv + (r.r0 >> 1) + i, pack_bf16x2(y.x, y.y), tag + 1u);
@@ -978,6 +1061,7 @@ __global__ void __launch_bounds__(kStepThreads + 32, 1) decode_step(const __grid
           } else if (stage == kRouter) {
             if (tid < n) put(work + wk.router + r.r0 + tid, __float_as_uint(c.sum1(tid)), tag + 7u);
           } else if (stage == kGateUp) {
+#pragma unroll 1
             for (int i = tid; i < n / 4; i += kStepThreads) {
               float4 y = c.sum4(4 * i);
               if (kFmt) {
@@ -987,9 +1071,11 @@ __global__ void __launch_bounds__(kStepThreads + 32, 1) decode_step(const __grid
               put(work + wk.act + (r.r0 >> 2) + i, pack_bf16x2(silu(y.x, y.y), silu(y.z, y.w)), tag + 6u);
             }
           } else {
+#pragma unroll 1
             for (int i = tid; i < n / 2; i += kStepThreads) {
               float2 y = make_float2(0.f, 0.f);
               if (E && stage == kDown) {
+#pragma unroll 1
                 for (int e = 0; e < slots; ++e) {
                   const float2 v = c.sum2(e * n + 2 * i);
                   y.x = fmaf(weights[e], bf16_round(v.x), y.x);
@@ -1041,6 +1127,7 @@ __global__ void __launch_bounds__(kStepThreads + 32, 1) decode_step(const __grid
         best = -INFINITY;
         best_row = 0x7fffffff;
         bool ok = true;
+#pragma unroll 1
         for (int i = lane; i < sms && ok; i += 32) {
           Two v = get2(work + wk.best + 2 * i);
           ok = c.poll2(work + wk.best + 2 * i, tag + 1u, v);
