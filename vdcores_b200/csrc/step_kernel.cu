@@ -324,6 +324,7 @@ struct Consumer {
   uint8_t* base;
   int tid, warp, lane, sm;
   RingAt at{kItems};
+  int teams, turn;               // and the chunks until this warp's team is on
   int kw, kg, rw, rg, ld;        // warps along the inputs, this warp's place there; along the rows; rows there is room for
 
   __device__ __forceinline__ float* part() const { return reinterpret_cast<float*>(base + lay.part); }
@@ -439,15 +440,21 @@ struct Consumer {
     consumers_sync();
   }
 
-  // How the warps share rows of K inputs: along K as far as that has steps for them, the rest along the rows.
+  // How the warps share a stage's n rows of K inputs: teams of them take the chunks in turn, so that one's way through a chunk
+  // (a few hundred cycles of latency) falls into the others'; a team's warps divide K as far as that has steps for them, and
+  // the rows.
   template <int kFmt>
-  __device__ __forceinline__ void split(int K) {
-    const int units = K / unit_of(kFmt);
-    kw = units >= 16 ? 16 : units >= 8 ? 8 : units >= 4 ? 4 : units >= 2 ? 2 : 1;
-    rw = kStepWarps / kw;
+  __device__ __forceinline__ void split(int K, int n) {
+    const int units = K / unit_of(kFmt), chunks = n / chunk_rows(row_bytes(kFmt, K));
+    teams = chunks >= 4 ? 4 : chunks >= 2 ? 2 : 1;
+    const int warps = kStepWarps / teams;
+    kw = 1;
+    while (kw < warps && 2 * kw <= units) kw *= 2;
+    rw = warps / kw;
     kg = warp & (kw - 1);
-    rg = warp / kw;
+    rg = (warp & (warps - 1)) / kw;
     ld = kPartFloats / kw;
+    turn = warp / warps;
   }
   // n rows from the ring times the inputs xp: every warp's share of row r to part[kg][row0 + r], rows side by side for the
   // threads that add the shares up.
@@ -458,7 +465,9 @@ struct Consumer {
     for (int r0 = 0; r0 < n; r0 += per, at.next()) {
       if (!wait.warp_wait(&sh.full[at.st], at.parity, 2, r0)) return;
       const uint8_t* w = base + lay.ring + sh.start[at.st];
-      const int nr = min(per, n - r0);
+      const bool mine_now = turn == 0;
+      turn = mine_now ? teams - 1 : turn - 1;
+      const int nr = mine_now ? min(per, n - r0) : 0;      // every warp sees every chunk arrive, one team works on it
 #pragma unroll 1
       for (int r = rg; r < nr; r += 4 * rw) {
         int off[4];
@@ -468,12 +477,12 @@ struct Consumer {
         if (kFmt == 0) {
           if (r + 2 * rw < nr) {
             float2 d[4] = {};
-#pragma unroll 1
+#pragma unroll 2
             for (int u = kg; u < units; u += kw) dot_bf16<2>(d, w, off, xp, u, lane);
             a = d[0].x + d[0].y; b = d[1].x + d[1].y; c = d[2].x + d[2].y; e = d[3].x + d[3].y;
           } else {
             float2 d[2] = {};
-#pragma unroll 1
+#pragma unroll 2
             for (int u = kg; u < units; u += kw) dot_bf16<1>(d, w, off, xp, u, lane);
             a = d[0].x + d[0].y; b = d[1].x + d[1].y;
           }
@@ -1015,8 +1024,8 @@ __global__ void __launch_bounds__(kStepThreads + 32, 1) decode_step(const __grid
         c.route(work + wk.router, tag + 7u);
       }
       // ---- rows, as many at a time as their partial sums have room for
-      if (lm && kFmt != 0) c.template split<0>(K);
-      else c.template split<kFmt>(K);
+      if (lm && kFmt != 0) c.template split<0>(K, r.n);
+      else c.template split<kFmt>(K, r.n * (E && stage == kDown ? slots : 1));
       const int per = chunk_rows(2 * H), most = lm ? kPartFloats / c.kw / per * per : r.n;
 #pragma unroll 1
       for (int r0 = 0; r0 < r.n && !skip; r0 += most) {
@@ -1178,7 +1187,7 @@ extern "C" const char* vdc_step_refuses(const vdc_step* s, bool pointers) {
   if (l.total - l.ring < 3 * kItemBytes) return "step: no room for the ring";
   // the partial sums of an SM's rows
   auto fits = [&](long long rows, int K, int fmt) {
-    const int units = K / unit_of(fmt), kw = units >= 16 ? 16 : units >= 8 ? 8 : units >= 4 ? 4 : units >= 2 ? 2 : 1;
+    const int units = K / unit_of(fmt), kw = units >= 16 ? 16 : units >= 8 ? 8 : units >= 4 ? 4 : units >= 2 ? 2 : 1;      // at most
     return ((rows + s->num_sms - 1) / s->num_sms + 4) * kw <= kPartFloats;
   };
   const int k = s->n_experts ? s->top_k : 1;
