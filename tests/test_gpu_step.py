@@ -65,9 +65,9 @@ def test_step_kernel_against_the_megakernels_program(cuda_device, kw, positions,
         assert torch.equal(sa, sb)
         for (ta, la, ha, na), (tb, lb, hb, nb) in zip(a, b):
             assert bool(torch.isfinite(ta.float()).all()) and torch.equal(ta[-1], ha)
-            # two orders of fp32 sums, rounded to bf16 at the same places through up to three layers; random experts' weights
-            # hang on logits that those roundings move
-            bound = 2e-2 if kw.get("n_experts") else 1e-2
+            # each is within the oracle tests' 1e-2 of the exact result, so the two are within sqrt(2) of that of each other;
+            # random experts' weights hang on logits that the roundings move
+            bound = 2e-2 if kw.get("n_experts") else 1.5e-2
             assert rel(ta, tb) < bound, pos
             # the logits of this hidden state (the program's own cover whole chunks of rows only): one bf16 rounding, 2^-9
             x = ha.float() * torch.rsqrt(ha.float().pow(2).mean() + eng.cfg.eps)

@@ -15,14 +15,17 @@
 
 namespace vdc {
 
-constexpr int kStepWarps = 16;                       // consumer warps; one more warp produces
+// Consumer warps; one more warp produces.  What every warp executes at a stage's boundaries (some 500 instructions, 1400 around
+// the attention) is bound by instructions issued: eight warps, not sixteen.
+constexpr int kStepWarps = 8;
 constexpr int kStepThreads = 32 * kStepWarps;
 constexpr int kItems = 16;                           // copies in the ring, at most
 constexpr int kItemBytes = 32 * 1024;                // bytes of one, at most
 constexpr int kPageBytes = VDC_KV_PAGE * VDC_HEAD_DIM * 2;
-constexpr int kGroups = 4;                           // of four warps: a page of the cache each
+constexpr int kGroups = kStepWarps / 4;              // of four warps: a page of the cache each
+constexpr int kAlone = 4;                            // pages that one SM walks without splitting them
 constexpr int kOutLd = VDC_HEAD_DIM + 4;
-constexpr int kPartFloats = kGroups * 8 * kOutLd;    // partial sums of rows; also the groups' partial heads
+constexpr int kPartFloats = 4 * 8 * kOutLd;          // partial sums of rows; also the groups' partial heads
 constexpr int kQLd = VDC_HEAD_DIM / 2 + 4;           // words of a query row in shared memory
 constexpr int kPLd = VDC_KV_PAGE / 2 + 4;            // words of a row of probabilities
 constexpr int kMaxSplits = 32;
@@ -164,28 +167,11 @@ __device__ __forceinline__ void expand(uint32_t (&o)[kFmt == 2 ? 4 : 2], const u
   }
 }
 
-// bf16 rows: packed fp32 FMAs of the widened pairs, per row one sum of the even and one of the odd weights (which are as many
-// instructions as the tensor cores' products below would take away again in picking sums out of their tiles).
-template <int kPairs>
-__device__ __forceinline__ void dot_bf16(float2 (&d)[2 * kPairs], const uint8_t* w, const int (&row)[4], const uint8_t* x, int u, int lane) {
-  auto pair = [](uint32_t v) { return make_float2(bf_lo(v), bf_hi(v)); };
-  const uint4 xv = lds128(x + u * 512 + lane * 16);
-  const float2 xf[4] = {pair(xv.x), pair(xv.y), pair(xv.z), pair(xv.w)};
-#pragma unroll
-  for (int i = 0; i < 2 * kPairs; ++i) {
-    const uint4 v = lds128(w + row[i] + u * 512 + lane * 16);
-    d[i] = __ffma2_rn(pair(v.x), xf[0], d[i]);
-    d[i] = __ffma2_rn(pair(v.y), xf[1], d[i]);
-    d[i] = __ffma2_rn(pair(v.z), xf[2], d[i]);
-    d[i] = __ffma2_rn(pair(v.w), xf[3], d[i]);
-  }
-}
-
 // One step of a warp: 16 bytes per lane of kPairs pairs of rows times the same inputs, as products of 16 x 16 by 16 x 8 tiles.
 // Row g of a tile is what the four lanes 4g .. 4g + 3 hold of the pair's first row (8 + g: of its second), column g what they
-// hold of the inputs: the tile's element (g, g) is the sum of the four lanes' products, the other elements mean nothing.  An
-// FMA per product would do the same, but fma with 16-bit operands runs at 16 a clock and SM (measured: 0.8 us for 32 KB of
-// bf16, where HBM takes 0.73).
+// hold of the inputs: the tile's element (g, g) is the sum of the four lanes' products, the other elements mean nothing.  The
+// loop is bound by instructions issued: a product of tiles is one where FMAs of four rows are 12 (32 KB of bf16 took 0.8 us,
+// HBM 0.73).
 template <int kFmt, int kPairs>
 __device__ __forceinline__ void dot_unit(float (&d)[kPairs][4], const uint8_t* w, const int (&row)[4], bool single, const uint8_t* x,
                                          int u, int lane, int K) {
@@ -295,13 +281,13 @@ struct Producer {
 };
 
 // An SM's share of the attention: one KV head's pages first .. first + count - 1; `live` splits of the head have pages.  Up to
-// four pages, one per group of warps, stay with one SM: there is nothing to merge then.
+// kAlone pages stay with one SM: there is nothing to merge then.
 struct Pages {
   int h, split, live, first, count;
 };
 __device__ __forceinline__ Pages pages_of(const vdc_step& s, int pos, int sm) {
   Pages p{sm % s.n_kv, sm / s.n_kv, 0, 0, 0};
-  const int n = min(pos / VDC_KV_PAGE + 1, s.max_pages), per = n <= kGroups ? n : (n + s.n_splits - 1) / s.n_splits;
+  const int n = min(pos / VDC_KV_PAGE + 1, s.max_pages), per = n <= kAlone ? n : (n + s.n_splits - 1) / s.n_splits;
   p.live = (n + per - 1) / per;
   if (p.split < p.live) {
     p.first = p.split * per;
@@ -399,7 +385,7 @@ struct Consumer {
   template <int kFmt>
   __device__ __forceinline__ void hidden(const uint64_t* buf, uint32_t tag, const uint8_t* row, uint64_t w, bool plain) const {
     const int H = s.hidden;
-    constexpr int kMost = 4;                                      // hidden <= 8192
+    constexpr int kMost = 8;                                      // hidden <= 8192
     uint2 wv[kMost];
 #pragma unroll
     for (int j = 0; j < kMost; ++j) {
@@ -418,7 +404,7 @@ struct Consumer {
         keep(i, v.x, v.y);
       }
     } else {
-      collect<kMost>(buf, H, tag, keep);
+      collect<4>(buf, H, tag, keep);
     }
     ssq = warp_sum(ssq);
     if (lane == 0) sh.red[warp] = ssq;
@@ -474,37 +460,23 @@ struct Consumer {
 #pragma unroll
         for (int i = 0; i < 4; ++i) off[i] = min(r + i * rw, nr - 1) * rb;
         float a, b, c = 0.f, e = 0.f;          // the lane's share of the four rows
-        if (kFmt == 0) {
-          if (r + 2 * rw < nr) {
-            float2 d[4] = {};
-#pragma unroll 2
-            for (int u = kg; u < units; u += kw) dot_bf16<2>(d, w, off, xp, u, lane);
-            a = d[0].x + d[0].y; b = d[1].x + d[1].y; c = d[2].x + d[2].y; e = d[3].x + d[3].y;
-          } else {
-            float2 d[2] = {};
-#pragma unroll 2
-            for (int u = kg; u < units; u += kw) dot_bf16<1>(d, w, off, xp, u, lane);
-            a = d[0].x + d[0].y; b = d[1].x + d[1].y;
-          }
+        // of a tile the lanes that hold its diagonal
+        const bool diag = (lane >> 3) == (lane & 3), odd = lane & 4;
+        auto share = [&](const float (&d)[4], float& first, float& second) {
+          first = diag ? (odd ? d[1] : d[0]) : 0.f;
+          second = diag ? (odd ? d[3] : d[2]) : 0.f;
+        };
+        if (r + 2 * rw < nr) {
+          float d[2][4] = {};
+#pragma unroll 1
+          for (int u = kg; u < units; u += kw) dot_unit<kFmt, 2>(d, w, off, false, xp, u, lane, K);
+          share(d[0], a, b);
+          share(d[1], c, e);
         } else {
-          // of a tile the lanes that hold its diagonal
-          const bool diag = (lane >> 3) == (lane & 3), odd = lane & 4;
-          auto share = [&](const float (&d)[4], float& first, float& second) {
-            first = diag ? (odd ? d[1] : d[0]) : 0.f;
-            second = diag ? (odd ? d[3] : d[2]) : 0.f;
-          };
-          if (r + 2 * rw < nr) {
-            float d[2][4] = {};
+          float d[1][4] = {};
 #pragma unroll 1
-            for (int u = kg; u < units; u += kw) dot_unit<kFmt, 2>(d, w, off, false, xp, u, lane, K);
-            share(d[0], a, b);
-            share(d[1], c, e);
-          } else {
-            float d[1][4] = {};
-#pragma unroll 1
-            for (int u = kg; u < units; u += kw) dot_unit<kFmt, 1>(d, w, off, r + rw >= nr, xp, u, lane, K);
-            share(d[0], a, b);
-          }
+          for (int u = kg; u < units; u += kw) dot_unit<kFmt, 1>(d, w, off, r + rw >= nr, xp, u, lane, K);
+          share(d[0], a, b);
         }
         // four sums over the lanes at once: lanes 8i .. 8i + 7 end up with row i
         const bool up = lane & 16, right = lane & 8;
@@ -560,40 +532,37 @@ struct Consumer {
     uint32_t* vrow = krow + D / 2;
     const bool owner = pg.first + pg.count == min(pos / VDC_KV_PAGE + 1, s.max_pages);
     // what the heads' prologue needs besides the entries is on its way before they are waited for
-    float2 cs = make_float2(0.f, 0.f), sn = cs;
-    uint32_t nlo = 0u, nhi = 0u;
     const int i0 = lane * 2;
-    if (warp <= G) {
-      const float* rope = reinterpret_cast<const float*>(s.rope) + (size_t)pos * D;
-      cs = __ldg(reinterpret_cast<const float2*>(rope + i0));
-      sn = __ldg(reinterpret_cast<const float2*>(rope + 64 + i0));
-      if (s.qk_norm) {
-        const uint32_t* w = reinterpret_cast<const uint32_t*>(s.qk_norm) + (size_t)layer * D + (warp == G ? D / 2 : 0);
-        nlo = __ldg(w + lane);
-        nhi = __ldg(w + lane + 32);
-      }
+    const float* rope = reinterpret_cast<const float*>(s.rope) + (size_t)pos * D;
+    const float2 cs = __ldg(reinterpret_cast<const float2*>(rope + i0)), sn = __ldg(reinterpret_cast<const float2*>(rope + 64 + i0));
+    uint32_t nw[4] = {0u, 0u, 0u, 0u};            // norm weights of the queries, of the key
+    if (s.qk_norm) {
+      const uint32_t* w = reinterpret_cast<const uint32_t*>(s.qk_norm) + (size_t)layer * D + lane;
+#pragma unroll
+      for (int j = 0; j < 4; ++j) nw[j] = __ldg(w + 32 * j);
     }
-    collect<1>(qkv + (size_t)pg.h * (G + 2) * (D / 2), (G + 2) * D, tag_in,
-            [&](int i, uint32_t a, uint32_t b) { *reinterpret_cast<uint2*>(raw + 2 * i) = make_uint2(a, b); });
+    collect<2>(qkv + (size_t)pg.h * (G + 2) * (D / 2), (G + 2) * D, tag_in,
+               [&](int i, uint32_t a, uint32_t b) { *reinterpret_cast<uint2*>(raw + 2 * i) = make_uint2(a, b); });
     consumers_sync();
-    if (warp <= G) {
-      const uint32_t lo = raw[warp * (D / 2) + lane], hi = raw[warp * (D / 2) + lane + 32];
-      float a0 = bf_lo(lo), a1 = bf_hi(lo), b0 = bf_lo(hi), b1 = bf_hi(hi);
-      if (s.qk_norm) {
-        const float rs = rsqrtf(warp_sum(a0 * a0 + a1 * a1 + b0 * b0 + b1 * b1) / (float)D + s.qk_eps);
-        a0 = bf16_round(bf_lo(nlo) * bf16_round(a0 * rs));
-        a1 = bf16_round(bf_hi(nlo) * bf16_round(a1 * rs));
-        b0 = bf16_round(bf_lo(nhi) * bf16_round(b0 * rs));
-        b1 = bf16_round(bf_hi(nhi) * bf16_round(b1 * rs));
+#pragma unroll 1
+    for (int hd = warp; hd < G + 2; hd += kStepWarps) {      // queries, key, value
+      uint32_t lo = raw[hd * (D / 2) + lane], hi = raw[hd * (D / 2) + lane + 32];
+      if (hd <= G) {
+        float a0 = bf_lo(lo), a1 = bf_hi(lo), b0 = bf_lo(hi), b1 = bf_hi(hi);
+        if (s.qk_norm) {
+          const float rs = rsqrtf(warp_sum(a0 * a0 + a1 * a1 + b0 * b0 + b1 * b1) / (float)D + s.qk_eps);
+          const uint32_t nlo = hd < G ? nw[0] : nw[2], nhi = hd < G ? nw[1] : nw[3];
+          a0 = bf16_round(bf_lo(nlo) * bf16_round(a0 * rs));
+          a1 = bf16_round(bf_hi(nlo) * bf16_round(a1 * rs));
+          b0 = bf16_round(bf_lo(nhi) * bf16_round(b0 * rs));
+          b1 = bf16_round(bf_hi(nhi) * bf16_round(b1 * rs));
+        }
+        lo = pack_bf16x2(bf16_round(a0 * cs.x) - bf16_round(b0 * sn.x), bf16_round(a1 * cs.y) - bf16_round(b1 * sn.y));
+        hi = pack_bf16x2(bf16_round(b0 * cs.x) + bf16_round(a0 * sn.x), bf16_round(b1 * cs.y) + bf16_round(a1 * sn.y));
       }
-      const uint32_t rlo = pack_bf16x2(bf16_round(a0 * cs.x) - bf16_round(b0 * sn.x), bf16_round(a1 * cs.y) - bf16_round(b1 * sn.y));
-      const uint32_t rhi = pack_bf16x2(bf16_round(b0 * cs.x) + bf16_round(a0 * sn.x), bf16_round(b1 * cs.y) + bf16_round(a1 * sn.y));
-      uint32_t* dst = warp < G ? qs + warp * kQLd : krow;
-      dst[lane] = rlo;
-      dst[lane + 32] = rhi;
-    } else if (warp == G + 1) {
-      vrow[lane] = raw[(G + 1) * (D / 2) + lane];
-      vrow[lane + 32] = raw[(G + 1) * (D / 2) + lane + 32];
+      uint32_t* dst = hd < G ? qs + hd * kQLd : hd == G ? krow : vrow;
+      dst[lane] = lo;
+      dst[lane + 32] = hi;
     }
     consumers_sync();
 
@@ -716,8 +685,9 @@ struct Consumer {
     if (failed()) return;
 
     // the groups' sums: two dims of a head per thread
-    if (tid < G * (D / 2)) {
-      const int g = tid / (D / 2), d2 = tid % (D / 2);
+#pragma unroll 1
+    for (int t = tid; t < G * (D / 2); t += kStepThreads) {
+      const int g = t / (D / 2), d2 = t % (D / 2);
       const float* w0 = reinterpret_cast<const float*>(base + lay.wl);
       float mm = -INFINITY;
 #pragma unroll
@@ -733,10 +703,10 @@ struct Consumer {
       }
       if (pg.live == 1) {
         const float inv = 1.f / den;
-        put(out + (size_t)pg.h * G * (D / 2) + tid, pack_bf16x2(n0 * inv, n1 * inv), tag_out);
+        put(out + (size_t)pg.h * G * (D / 2) + t, pack_bf16x2(n0 * inv, n1 * inv), tag_out);
       } else {
         const size_t u = (size_t)pg.h * s.n_splits + pg.split;
-        put2(rec + (u * G * (D / 2) + tid) * 2, __float_as_uint(n0), __float_as_uint(n1), tag_rec);
+        put2(rec + (u * G * (D / 2) + t) * 2, __float_as_uint(n0), __float_as_uint(n1), tag_rec);
         if (d2 == 0) put2(ml + (u * G + g) * 2, __float_as_uint(mm), __float_as_uint(den), tag_rec);
       }
     }
@@ -1187,7 +1157,7 @@ extern "C" const char* vdc_step_refuses(const vdc_step* s, bool pointers) {
   if (l.total - l.ring < 3 * kItemBytes) return "step: no room for the ring";
   // the partial sums of an SM's rows
   auto fits = [&](long long rows, int K, int fmt) {
-    const int units = K / unit_of(fmt), kw = units >= 16 ? 16 : units >= 8 ? 8 : units >= 4 ? 4 : units >= 2 ? 2 : 1;      // at most
+    const int units = K / unit_of(fmt), kw = units >= 8 ? 8 : units >= 4 ? 4 : units >= 2 ? 2 : 1;      // at most
     return ((rows + s->num_sms - 1) / s->num_sms + 4) * kw <= kPartFloats;
   };
   const int k = s->n_experts ? s->top_k : 1;
