@@ -747,18 +747,18 @@ class DecodeEngine:
     def set_state(self, pos: int, token: int):
         """Positions [0, pos) are cached; `token` is decoded next at position pos."""
         assert pos < self.max_seq
-        s = self.state_host
-        s.zero_()
+        s = self.state_host.numpy()
         page = pos // isa.KV_PAGE
+        table = self.page_table.numpy()
+        s[:isa.ST_PAGETABLE] = 0
         s[isa.ST_POS] = pos
         s[isa.ST_NPAGES] = page + 1
         s[isa.ST_TOKEN] = token
-        s[isa.ST_STEP] = 0
-        s[isa.ST_NEWROW] = int(self.page_table[page]) * isa.KV_PAGE * self.cfg.n_kv_heads + pos % isa.KV_PAGE
+        s[isa.ST_NEWROW] = int(table[page]) * isa.KV_PAGE * self.cfg.n_kv_heads + pos % isa.KV_PAGE
         s[isa.ST_NKVH] = self.cfg.n_kv_heads
         s[isa.ST_MAXPAGES] = self.max_pages
-        s[isa.ST_PAGETABLE:] = self.page_table
-        self.state.copy_(s, non_blocking=True)
+        s[isa.ST_PAGETABLE:] = table
+        self.state.copy_(self.state_host, non_blocking=True)
         self.attn_cnt.zero_()
         if self.cfg.n_experts:
             self.moe_acc.zero_()

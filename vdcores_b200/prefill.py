@@ -60,6 +60,7 @@ class PrefillEngine(BatchDecodeEngine):
         super()._build_program()
         self._body = self._plan(vocab=False)
         self._wide = None if self.max_ctas else WideStages(self)
+        self._first = torch.zeros(1, dtype=torch.int32).pin_memory()
 
     def launches(self, T: int) -> int:
         """Kernels a prompt of T tokens takes."""
@@ -95,10 +96,12 @@ class PrefillEngine(BatchDecodeEngine):
         T, B = int(tokens.numel()), self.batch
         assert 1 <= T < self.max_seq and self.stages is not None
         n = (T + B - 1) // B
+        wide = self._goes_wide(T)
         ids = tokens.cpu().to(torch.int32).numpy().reshape(-1)
         blocks = torch.empty(min(n, self.BLOCKS), B, self.state_words, dtype=torch.int32, pin_memory=True)
         k, sent = len(blocks), 0
-        copied = [torch.cuda.Event() for _ in blocks]
+        # a block's place is waited for only where it is used a second time
+        copied = [torch.cuda.Event() for _ in blocks] if (self._wide.sends(T) + 1 if wide else n) > k else None
 
         def send(fill, dst):
             """The next block, filled by fill(numpy view), into dst; its place is free again when it has been copied."""
@@ -108,21 +111,20 @@ class PrefillEngine(BatchDecodeEngine):
             block = blocks[sent % k]
             fill(block.numpy())
             dst.copy_(block.view(-1)[:dst.numel()].view(dst.shape), non_blocking=True)
-            copied[sent % k].record(self.stream)
+            if copied:
+                copied[sent % k].record(self.stream)
             sent += 1
-        self.keys.zero_()
         launch = lambda stages: runtime.launch_stages(stages, self.stream.cuda_stream, self.timeout_ns, self.max_ctas)
         with torch.cuda.stream(self.stream):
-            if self._goes_wide(T):
+            if wide:
                 self._wide.run(ids, send, launch)
-                send(lambda s: self._fill_states(s, ids, n - 1), self.state)
-                launch(self._wide.last)
-            else:
-                for c in range(n):
-                    send(lambda s: self._fill_states(s, ids, c), self.state)
-                    launch(self.stages if c == n - 1 else self._body)
+            self.keys.zero_()
+            for c in range(n - 1 if wide else 0, n):
+                send(lambda s: self._fill_states(s, ids, c), self.state)
+                launch(self._wide.last if wide else self.stages if c == n - 1 else self._body)
+            self._first.copy_(self.token_log[(T - 1) % B, :1], non_blocking=True)
         runtime.read_status(self.stream.cuda_stream)
-        first = int(self.token_log[(T - 1) % B, 0])
+        first = int(self._first)
         if set_target_state:
             self.target.set_state(T, first)
         return first
@@ -204,6 +206,11 @@ class WideStages:
                     v["splits"][1 + reader:2 + n:8] = ks
             self.lists[R] = arr
         return self.lists[R]
+
+    def sends(self, T: int) -> int:
+        """Blocks of the engine's pinned memory that a prompt's ids and page tables take."""
+        at, piece = self.HEADER + self.e.max_pages, self.e.batch * self.e.state_words
+        return sum(-(-(at + min(self.rows, T - p0)) // piece) for p0 in range(0, T, self.rows))
 
     def run(self, ids, send, launch):
         """All layers over the prompt's ids; send and launch are PrefillEngine.prefill's."""
