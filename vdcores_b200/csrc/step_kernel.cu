@@ -167,6 +167,23 @@ __device__ __forceinline__ void expand(uint32_t (&o)[kFmt == 2 ? 4 : 2], const u
   }
 }
 
+// Models with experts: packed fp32 FMAs of the widened pairs, sums rounded to nearest at every product.  The router's softmax
+// is steep enough that the last bits of what stands in front of it can be seen behind it (the tensor cores cut theirs off).
+template <int kPairs>
+__device__ __forceinline__ void dot_fma(float2 (&d)[2 * kPairs], const uint8_t* w, const int (&row)[4], const uint8_t* x, int u, int lane) {
+  auto pair = [](uint32_t v) { return make_float2(bf_lo(v), bf_hi(v)); };
+  const uint4 xv = lds128(x + u * 512 + lane * 16);
+  const float2 xf[4] = {pair(xv.x), pair(xv.y), pair(xv.z), pair(xv.w)};
+#pragma unroll
+  for (int i = 0; i < 2 * kPairs; ++i) {
+    const uint4 v = lds128(w + row[i] + u * 512 + lane * 16);
+    d[i] = __ffma2_rn(pair(v.x), xf[0], d[i]);
+    d[i] = __ffma2_rn(pair(v.y), xf[1], d[i]);
+    d[i] = __ffma2_rn(pair(v.z), xf[2], d[i]);
+    d[i] = __ffma2_rn(pair(v.w), xf[3], d[i]);
+  }
+}
+
 // One step of a warp: 16 bytes per lane of kPairs pairs of rows times the same inputs, as products of 16 x 16 by 16 x 8 tiles.
 // Row g of a tile is what the four lanes 4g .. 4g + 3 hold of the pair's first row (8 + g: of its second), column g what they
 // hold of the inputs: the tile's element (g, g) is the sum of the four lanes' products, the other elements mean nothing.  The
@@ -444,7 +461,7 @@ struct Consumer {
   }
   // n rows from the ring times the inputs xp: every warp's share of row r to part[kg][row0 + r], rows side by side for the
   // threads that add the shares up.
-  template <int kFmt>
+  template <int kFmt, bool kFma>
   __device__ __forceinline__ void rows(int K, int n, const uint8_t* xp, int row0) {
     const int rb = row_bytes(kFmt, K), per = chunk_rows(rb), units = K / unit_of(kFmt);
 #pragma unroll 1
@@ -466,7 +483,17 @@ struct Consumer {
           first = diag ? (odd ? d[1] : d[0]) : 0.f;
           second = diag ? (odd ? d[3] : d[2]) : 0.f;
         };
-        if (r + 2 * rw < nr) {
+        if (kFma && r + 2 * rw < nr) {
+          float2 d[4] = {};
+#pragma unroll 2
+          for (int u = kg; u < units; u += kw) dot_fma<2>(d, w, off, xp, u, lane);
+          a = d[0].x + d[0].y; b = d[1].x + d[1].y; c = d[2].x + d[2].y; e = d[3].x + d[3].y;
+        } else if (kFma) {
+          float2 d[2] = {};
+#pragma unroll 2
+          for (int u = kg; u < units; u += kw) dot_fma<1>(d, w, off, xp, u, lane);
+          a = d[0].x + d[0].y; b = d[1].x + d[1].y;
+        } else if (r + 2 * rw < nr) {
           float d[2][4] = {};
 #pragma unroll 1
           for (int u = kg; u < units; u += kw) dot_unit<kFmt, 2>(d, w, off, false, xp, u, lane, K);
@@ -814,7 +841,7 @@ struct Consumer {
 // ------------------------------------------------------------------------- //
 // the step
 // ------------------------------------------------------------------------- //
-template <int kFmt>
+template <int kFmt, bool kExperts>
 __global__ void __launch_bounds__(kStepThreads + 32, 1) decode_step(const __grid_constant__ StepArgs args, vdc_status* status,
                                                                     uint64_t timeout_ns) {
   extern __shared__ uint8_t dyn[];
@@ -850,7 +877,7 @@ __global__ void __launch_bounds__(kStepThreads + 32, 1) decode_step(const __grid
     return;
   }
 
-  const int H = s.hidden, F = s.ffn, G = s.group, Q = s.n_kv * G * D, QKV = Q + 2 * s.n_kv * D, L = s.n_layers, E = s.n_experts;
+  const int H = s.hidden, F = s.ffn, G = s.group, Q = s.n_kv * G * D, QKV = Q + 2 * s.n_kv * D, L = s.n_layers, E = kExperts ? s.n_experts : 0;
   const int* state = reinterpret_cast<const int*>(s.state);
   const int pos = ld_relaxed_gpu(state + VDC_ST_POS);
   const Pages pg = pages_of(s, pos, sm);
@@ -1001,14 +1028,14 @@ __global__ void __launch_bounds__(kStepThreads + 32, 1) decode_step(const __grid
       for (int r0 = 0; r0 < r.n && !skip; r0 += most) {
         const int n = min(most, r.n - r0);
         if (lm && kFmt != 0) {
-          c.template rows<0>(K, n, c.x(), 0);
+          c.template rows<0, false>(K, n, c.x(), 0);
         } else {
           // experts: a slot's gate/up rows end where the next slot's begin; every slot's down rows have inputs of their own
           const int segs = E && stage == kDown ? slots : 1;
 #pragma unroll 1
           for (int e = 0, done = 0; E && stage == kGateUp ? done < n : e < segs; ++e) {
             const int take = E && stage == kGateUp ? min(n - done, 2 * F - (r.r0 + done) % (2 * F)) : n;
-            c.template rows<kFmt>(K, take, c.x() + (segs > 1 ? (size_t)e * F * 2 : 0), segs > 1 ? e * n : done);
+            c.template rows<kFmt, kExperts>(K, take, c.x() + (segs > 1 ? (size_t)e * F * 2 : 0), segs > 1 ? e * n : done);
             done += take;
           }
         }
@@ -1177,7 +1204,8 @@ extern "C" const char* vdc_step_refuses(const vdc_step* s, bool pointers) {
 extern "C" long long vdc_step_words(const vdc_step* s) { return (long long)vdc::step_work(*s).words; }
 
 extern "C" cudaError_t vdc_step_prepare() {
-  const void* fs[] = {(const void*)vdc::decode_step<0>, (const void*)vdc::decode_step<1>, (const void*)vdc::decode_step<2>};
+  const void* fs[] = {(const void*)vdc::decode_step<0, false>, (const void*)vdc::decode_step<0, true>,
+                      (const void*)vdc::decode_step<1, false>, (const void*)vdc::decode_step<2, false>};
   for (const void* f : fs)
     if (cudaError_t e = cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, vdc::kStepSmem)) return e;
   return cudaSuccess;
@@ -1194,7 +1222,8 @@ extern "C" cudaError_t vdc_step_launch(const vdc_step* s, vdc_status* status, ui
   cfg.gridDim = dim3((unsigned)s->num_sms);
   cfg.blockDim = dim3(vdc::kStepThreads + 32);
   cfg.dynamicSmemBytes = vdc::kStepSmem;
-  auto f = s->wfmt == 0 ? vdc::decode_step<0> : s->wfmt == 1 ? vdc::decode_step<1> : vdc::decode_step<2>;
+  auto f = s->n_experts ? vdc::decode_step<0, true> : s->wfmt == 0 ? vdc::decode_step<0, false>
+           : s->wfmt == 1 ? vdc::decode_step<1, false> : vdc::decode_step<2, false>;
   const vdc::StepArgs args{*s, vdc::step_layout(*s), vdc::step_work(*s)};
   return cudaLaunchKernelEx(&cfg, f, args, status, timeout_ns);
 }
