@@ -9,6 +9,10 @@
 // The same step as a program of the megakernel (csrc/megakernel.cu) counts barriers down: fence, atomic, poll, then a copy,
 // about 7 us per boundary.
 //
+// Measured against that program (B200): three layers of width 512 109 -> 69 us, eight 8B-shaped bf16 layers and a 128256-row
+// vocabulary projection 1013 -> 990, four such layers e4m3 390 -> 336, NVFP4 392 -> 330, four layers of a 30B mixture of experts
+// 437 -> 264.
+//
 // An entry buffer is written again one layer later, when everything that read it must have been read: whoever polls a buffer
 // has rows in the same or the following stage, and those rows go into what the next writer of the buffer waits for.
 #include "mk_stage.cuh"

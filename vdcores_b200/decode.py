@@ -1,6 +1,7 @@
-"""Batch-1 decode engine: packs a Llama / Qwen3 style model for the megakernel,
-builds the per-SM instruction program once, and runs one kernel launch per
-generated token.
+"""Batch-1 decode engine: packs a Llama / Qwen3 style model and runs one kernel
+launch per generated token: the step kernel (csrc/step_kernel.cu), or the
+per-SM instruction program built here for the megakernel where an option asks
+for it or a shape does not fit the step kernel.
 
 The program plays the role of the reference's model schedule scripts
 (reference app/python/llama3/sched.py:255-571, app/python/qwen3/sched.py): the
@@ -651,7 +652,7 @@ class DecodeEngine:
         self.minsts = torch.from_numpy(m).to(self.dev)
         self.bars_init = torch.from_numpy(bars).to(self.dev)
         self.launches_per_step = 1
-        self.step_kernel = None
+        self.step_kernel = self._plan_step()
 
     def _plan_step(self):
         """The step as one persistent kernel (csrc/step_kernel.cu), or None where the program of the megakernel runs it: for

@@ -90,6 +90,7 @@ def main():
     else:
         eng = DecodeEngine(cfg, max_seq=max_seq, device=dev, max_steps=64)
         eng.init_random_weights(0)
+        eng.step_kernel = None                # the program of the megakernel is what is traced
         g = torch.Generator().manual_seed(0)
         first = eng.prefill(torch.randint(0, cfg.vocab, (args.prompt,), generator=g))
         eng.set_state(args.prompt, first)
