@@ -10,7 +10,7 @@
 // about 7 us per boundary.
 //
 // Measured against that program (B200): three layers of width 512 109 -> 69 us, eight 8B-shaped bf16 layers and a 128256-row
-// vocabulary projection 1013 -> 990, four such layers e4m3 390 -> 336, NVFP4 392 -> 330, four layers of a 30B mixture of experts
+// vocabulary projection 1012 -> 977, four such layers e4m3 387 -> 325, NVFP4 388 -> 329, four layers of a 30B mixture of experts
 // 437 -> 264.
 //
 // An entry buffer is written again one layer later, when everything that read it must have been read: whoever polls a buffer
@@ -453,7 +453,11 @@ struct Consumer {
   template <int kFmt>
   __device__ __forceinline__ void split(int K, int n) {
     const int units = K / unit_of(kFmt), chunks = n / chunk_rows(row_bytes(kFmt, K));
-    teams = chunks >= 4 ? 4 : chunks >= 2 ? 2 : 1;
+    // Two teams, since a chunk's place in the ring is held for as long as its team works on it; four where there is more work per
+    // byte.  Four 8B-shaped layers with 1 / 2 / 4 teams: bf16 459 / 447 / 456 us, e4m3 358 / 328 / 335, NVFP4 348 / 339 / 334,
+    // the 30B mixture of experts 273 / 261 / 260.
+    const bool four = kFmt == 2 || s.n_experts;
+    teams = four && chunks >= 4 ? 4 : chunks >= 2 ? 2 : 1;
     const int warps = kStepWarps / teams;
     kw = 1;
     while (kw < warps && 2 * kw <= units) kw *= 2;
@@ -499,13 +503,13 @@ struct Consumer {
           a = d[0].x + d[0].y; b = d[1].x + d[1].y;
         } else if (r + 2 * rw < nr) {
           float d[2][4] = {};
-#pragma unroll 1
+#pragma unroll 2
           for (int u = kg; u < units; u += kw) dot_unit<kFmt, 2>(d, w, off, false, xp, u, lane, K);
           share(d[0], a, b);
           share(d[1], c, e);
         } else {
           float d[1][4] = {};
-#pragma unroll 1
+#pragma unroll 2
           for (int u = kg; u < units; u += kw) dot_unit<kFmt, 1>(d, w, off, r + rw >= nr, xp, u, lane, K);
           share(d[0], a, b);
         }
