@@ -127,3 +127,48 @@ def test_a_token_outside_the_vocabulary_is_reported(cuda_device):
     assert torch.equal(eng.state, before) and bool((eng.token_log == -7).all())
     eng.set_state(20, 5)
     assert eng.generate(1)[0] == want[3] and torch.equal(eng.logits, want[1])
+
+
+@pytest.mark.parametrize("wkind", ["bf16", "fp8"])
+def test_sums_lose_no_more_bits_than_fp32_fmas(cuda_device, wkind):
+    """Sums of 8192 products, two of them large and cancelling, so that every addition's rounding shows in the result: values of
+    the cache rows (a layer's projection) and logits that are not the bf16 rounding of the sum in 64 bits.  The program adds with
+    FMAs; the step kernel may miss no more of them than it, up to five standard deviations of the two counts."""
+    from vdcores_b200.decode import DecodeConfig, DecodeEngine
+    H, L = 8192, 4
+    cfg = DecodeConfig(hidden=H, n_heads=32, n_kv_heads=8, ffn=512, vocab=16384, n_layers=L, eps=0.0, theta=1e4)
+    eng = DecodeEngine(cfg, 64, device=cuda_device, wkind=wkind, timeout_ns=500_000_000)
+    eng.init_random_weights(1)
+    g = torch.Generator(device=cuda_device).manual_seed(2)
+    # a hidden state of ones that no layer adds to: the norms' weights are the inputs
+    eng.embed.fill_(1.0)
+    for n in ("wo", "wd"):
+        (eng.scales[n] if wkind == "fp8" else getattr(eng, n)).zero_()
+    x = torch.randn(L + 1, H, generator=g, device=cuda_device).to(torch.bfloat16)
+    x[:, 0] = x[:, -1] = 2.0 ** 14
+    eng.ln1.copy_(x[:L])
+    eng.norm_w.copy_(x[L])
+
+    def matrix(rows):
+        w = 0.02 * torch.randn(rows, H, generator=g, device=cuda_device)
+        w[:, 0], w[:, -1] = 0.02, -0.02
+        return w.to(torch.bfloat16)
+    eng.lm_head.copy_(matrix(cfg.vocab))
+    exact_l, exact_v = eng.lm_head.double() @ x[L].double(), []
+    for l in range(L):
+        rows, sc = eng._encode(matrix(eng.qkv_rows))
+        eng.wqkv[l].copy_(rows)
+        if sc is not None:
+            eng.scales["wqkv"][l].copy_(sc)
+            rows = rows.view(torch.float8_e4m3fn).double() * sc.double()[:, None]
+        exact_v.append((rows.double() @ x[l].double()).view(cfg.n_kv_heads, cfg.group + 2, 128)[:, -1].reshape(-1))
+    missed = []
+    for step in (eng.step_kernel, None):
+        eng.step_kernel = step
+        eng.set_state(0, 3)
+        eng.generate(1)
+        v = torch.stack([eng.read_kv(l, 1)[1][0].reshape(-1) for l in range(L)])
+        missed.append([int((got != want.float().to(torch.bfloat16)).sum())
+                       for got, want in ((v, torch.stack(exact_v)), (eng.logits, exact_l))])
+    for a, b in zip(*missed):
+        assert a <= b + 5 * (a + b) ** 0.5, missed
