@@ -1,0 +1,41 @@
+"""Which steps the step kernel takes (csrc/step_kernel.cu): its limits are checked on the host, without a GPU."""
+import pytest
+
+
+def step(hidden, ffn, num_sms, n_kv=1, group=4, vocab=64, experts=0, top_k=0, wfmt=0, splits=1):
+    from vdcores_b200 import runtime
+    return runtime.Step(num_sms=num_sms, n_layers=1, hidden=hidden, ffn=ffn, vocab=vocab, n_kv=n_kv, group=group, wfmt=wfmt,
+                        max_pages=4, max_seq=256, n_splits=splits, n_experts=experts, top_k=top_k, eps=1e-5, qk_eps=1e-5)
+
+
+def sums_and_room(rows, unit, K, num_sms, slots, experts):
+    """Partial sums of the SMs with the most rows and of those with a unit less, and the room for them: 4224 floats shared by the
+    warps that divide K (bf16: steps of 256 inputs; eight warps in one, two or, with experts, four teams)."""
+    most = -(-(rows // unit) // num_sms) * unit
+    out = []
+    for n in (most, most - unit):
+        per = max(1, min(32, 32768 // (2 * K)) // 2 * 2)
+        chunks = n * slots // per
+        teams = 4 if experts and chunks >= 4 else 2 if chunks >= 2 else 1
+        kw = 1
+        while kw < 8 // teams and 2 * kw <= K // 256:
+            kw *= 2
+        out.append((n * slots, 4224 // kw))
+    return out
+
+
+@pytest.mark.parametrize("hidden,ffn,num_sms,experts,top_k,taken", [
+    (6912, 512, 23, 8, 7, False),        # the down projection of 7 experts: 302 rows of 7 sums, room for 2112
+    (6912, 512, 24, 8, 7, True),
+    (2560, 768, 79, 64, 16, True),       # 34 rows of 16 sums
+    (1024, 4096, 8, 0, 0, True),         # gate and up: 1024 rows, room for 1056
+    (1024, 4352, 8, 0, 0, False),
+    (1024, 4096, 7, 0, 0, False)])
+def test_partial_sums_of_a_taken_step_fit(hidden, ffn, num_sms, experts, top_k, taken):
+    from vdcores_b200 import runtime
+    k = top_k or 1
+    stages = [(768, 2, hidden, 1), (hidden, 2, 512, 1), (2 * ffn * k, 4, hidden, 1), (hidden, 2, ffn, k)]
+    room = all(need <= have for rows, unit, K, slots in stages
+               for need, have in sums_and_room(rows, unit, K, num_sms, slots, experts > 0))
+    assert room == taken
+    assert (runtime.step_workspace(step(hidden, ffn, num_sms, experts=experts, top_k=top_k)) is not None) == taken

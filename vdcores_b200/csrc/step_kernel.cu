@@ -200,10 +200,10 @@ __device__ __forceinline__ void add2(float& a, float& b, float x, float y) {
 // loop is bound by instructions issued: a product of tiles is one where FMAs of four rows are 12 (32 KB of bf16 took 0.8 us,
 // HBM 0.73).
 // The tensor cores cut off what an fp32 sum cannot hold.  So bf16 and e4m3 rows have only two products of tiles (8 of a lane's
-// inputs) added up by them, from zero; those sums meet in rounded additions.  Of 32768
-// sums of 8192 products around two large ones that cancel, 2.0 % miss their bf16 rounding (FMAs 2.1 %, all products in one sum
-// of the tensor cores 7.2 %).  Four 8B-shaped layers e4m3 325 -> 329 us, eight bf16 the same.  NVFP4 rows keep the one sum:
-// the megakernel's program adds 16 of their products up in f16.
+// inputs) added up by them, from zero; those sums meet in rounded additions.  Of 32768 sums of 8192 products around two large
+// ones that cancel, 2.0 % miss their bf16 rounding (FMAs 2.1 %, all products in one sum of the tensor cores 7.2 %).  Four
+// 8B-shaped layers e4m3 325 -> 329 us, eight bf16 the same.  NVFP4 rows keep the one sum: the megakernel's program adds 16 of
+// their products up in f16.
 template <int kFmt, int kPairs>
 __device__ __forceinline__ void dot_unit(float (&d)[kPairs][4], const uint8_t* w, const int (&row)[4], bool single, const uint8_t* x,
                                          int u, int lane, int K) {
@@ -248,14 +248,31 @@ __device__ __forceinline__ void dot_unit(float (&d)[kPairs][4], const uint8_t* w
 }
 
 // Units of q rows; the first SMs' shares are never empty while there are any.
-__device__ __forceinline__ Share share_of(int rows, int q, int sm, int sms) {
+__host__ __device__ inline Share share_of(int rows, int q, int sm, int sms) {
   const int units = rows / q;
   const int each = units / sms, more = units % sms;             // the first `more` SMs take one unit more
-  return {(sm * each + min(sm, more)) * q, (each + (sm < more ? 1 : 0)) * q};
+  return {(sm * each + (sm < more ? sm : more)) * q, (each + (sm < more ? 1 : 0)) * q};
 }
 __host__ __device__ constexpr int chunk_rows(int rb) {        // an even number where more than one
   const int n = kItemBytes / rb < 32 ? kItemBytes / rb : 32;
   return n > 1 ? n & ~1 : 1;
+}
+
+// How the warps share n rows of K inputs: teams of them take the chunks in turn, so that one's way through a chunk (a few
+// hundred cycles of latency) falls into the others'; a team's warps divide K as far as that has steps for them (kw of them), and
+// the rows.
+struct Split {
+  int teams, kw;
+};
+__host__ __device__ inline Split split_of(int fmt, bool experts, int K, int n) {
+  const int units = K / unit_of(fmt), chunks = n / chunk_rows(row_bytes(fmt, K));
+  // Two teams, since a chunk's place in the ring is held for as long as its team works on it; four where there is more work per
+  // byte.  Four 8B-shaped layers with 1 / 2 / 4 teams: bf16 459 / 447 / 456 us, e4m3 358 / 328 / 335, NVFP4 348 / 339 / 334,
+  // the 30B mixture of experts 273 / 261 / 260.
+  const bool four = fmt == 2 || experts;
+  Split s{four && chunks >= 4 ? 4 : chunks >= 2 ? 2 : 1, 1};
+  while (s.kw < kStepWarps / s.teams && 2 * s.kw <= units) s.kw *= 2;
+  return s;
 }
 
 // ------------------------------------------------------------------------- //
@@ -465,20 +482,12 @@ struct Consumer {
     consumers_sync();
   }
 
-  // How the warps share a stage's n rows of K inputs: teams of them take the chunks in turn, so that one's way through a chunk
-  // (a few hundred cycles of latency) falls into the others'; a team's warps divide K as far as that has steps for them, and
-  // the rows.
   template <int kFmt>
   __device__ __forceinline__ void split(int K, int n) {
-    const int units = K / unit_of(kFmt), chunks = n / chunk_rows(row_bytes(kFmt, K));
-    // Two teams, since a chunk's place in the ring is held for as long as its team works on it; four where there is more work per
-    // byte.  Four 8B-shaped layers with 1 / 2 / 4 teams: bf16 459 / 447 / 456 us, e4m3 358 / 328 / 335, NVFP4 348 / 339 / 334,
-    // the 30B mixture of experts 273 / 261 / 260.
-    const bool four = kFmt == 2 || s.n_experts;
-    teams = four && chunks >= 4 ? 4 : chunks >= 2 ? 2 : 1;
-    const int warps = kStepWarps / teams;
-    kw = 1;
-    while (kw < warps && 2 * kw <= units) kw *= 2;
+    const Split sp = split_of(kFmt, s.n_experts != 0, K, n);
+    const int warps = kStepWarps / sp.teams;
+    teams = sp.teams;
+    kw = sp.kw;
     rw = warps / kw;
     kg = warp & (kw - 1);
     rg = (warp & (warps - 1)) / kw;
@@ -1208,14 +1217,16 @@ extern "C" const char* vdc_step_refuses(const vdc_step* s, bool pointers) {
     return "step: experts not supported";
   const StepLayout l = step_layout(*s);
   if (l.total - l.ring < 3 * kItemBytes) return "step: no room for the ring";
-  // the partial sums of an SM's rows
-  auto fits = [&](long long rows, int K, int fmt) {
-    const int units = K / unit_of(fmt), kw = units >= 8 ? 8 : units >= 4 ? 4 : units >= 2 ? 2 : 1;      // at most
-    return ((rows + s->num_sms - 1) / s->num_sms + 4) * kw <= kPartFloats;
+  // the partial sums of an SM's rows: of those SMs with the most, and of those with a unit less
+  auto fits = [&](int rows, int q, int K, int slots) {
+    const int most = share_of(rows, q, 0, s->num_sms).n;
+    for (int n = most; n > 0 && n >= most - q; n -= q)
+      if (n * slots > kPartFloats / split_of(s->wfmt, s->n_experts != 0, K, n * slots).kw) return false;
+    return true;
   };
   const int k = s->n_experts ? s->top_k : 1;
-  if (!fits(Q + 2 * s->n_kv * VDC_HEAD_DIM, s->hidden, s->wfmt) || !fits(s->hidden, Q, s->wfmt) ||
-      !fits(2ll * s->ffn * k, s->hidden, s->wfmt) || !fits((long long)s->hidden * k, s->ffn, s->wfmt))
+  if (!fits(Q + 2 * s->n_kv * VDC_HEAD_DIM, 2, s->hidden, 1) || !fits(s->hidden, 2, Q, 1) ||
+      !fits(2 * s->ffn * k, 4, s->hidden, 1) || !fits(s->hidden, 2, s->ffn, k))
     return "step: more rows per SM than partial sums have room for";
   if (!pointers) return nullptr;
   if (!al16(s->embed) || !al16(s->lm_head) || !al16(s->norm_w) || !al16(s->ln1) || !al16(s->ln2) || !al16(s->wqkv) || !al16(s->wo) ||
