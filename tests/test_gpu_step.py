@@ -129,6 +129,28 @@ def test_a_token_outside_the_vocabulary_is_reported(cuda_device):
     assert eng.generate(1)[0] == want[3] and torch.equal(eng.logits, want[1])
 
 
+def test_logits_without_a_number_are_reported(cuda_device):
+    """The step itself ends with the error and leaves state and log; one logit that is a number is enough for a token."""
+    from vdcores_b200 import runtime
+    eng = _engine(cuda_device, 128, hidden=512, n_heads=8, n_kv_heads=2, ffn=512, vocab=640, n_layers=1)
+    head = eng.lm_head.clone()
+    eng.set_state(20, 5)
+    want = eng.generate(1)[0]
+    eng.lm_head.fill_(float("nan"))
+    eng.set_state(20, 5)
+    eng.token_log.fill_(-7)
+    before = eng.state.clone()
+    with pytest.raises(runtime.VdcError, match="no number among"):
+        eng.generate(1)
+    assert torch.equal(eng.state, before) and bool((eng.token_log == -7).all())
+    eng.lm_head[601] = head[601]
+    eng.set_state(20, 5)
+    assert eng.generate(1) == [601]
+    eng.lm_head.copy_(head)
+    eng.set_state(20, 5)
+    assert eng.generate(1)[0] == want
+
+
 @pytest.mark.parametrize("wkind", ["bf16", "fp8"])
 def test_sums_lose_no_more_bits_than_fp32_fmas(cuda_device, wkind):
     """Sums of 8192 products, two of them large and cancelling, so that every addition's rounding shows in the result: values of

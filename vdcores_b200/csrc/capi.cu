@@ -326,7 +326,8 @@ int vdc_read_status(uint64_t stream, vdc_status* status, int clear) {
   if (h.abort) {
     char buf[256];
     if (h.code == VDC_ERR_TOKEN)
-      snprintf(buf, sizeof buf, "row %d: %s (%d)", h.pc, h.opcode == VDC_STAGE_EMBED || h.opcode == VDC_STAGE_WIDE_EMBED || h.opcode == VDC_STEP_KIND ? "token id outside the vocabulary"
+      snprintf(buf, sizeof buf, "row %d: %s (%d)", h.pc, h.opcode == VDC_STAGE_EMBED || h.opcode == VDC_STAGE_WIDE_EMBED ||
+               (h.opcode == VDC_STEP_KIND && h.role == 0) ? "token id outside the vocabulary"
                : "no number among its logits, no next token", h.aux);
     else
       snprintf(buf, sizeof buf, "megakernel gave up: code=%d sm=%d role=%d pc=%d opcode=0x%x bar=%d aux=%d", h.code, h.sm,

@@ -1179,7 +1179,9 @@ __global__ void __launch_bounds__(kStepThreads + 32, 1) decode_step(const __grid
         if (lane == 0) {
           *reinterpret_cast<int*>(work) += 1;        // the next launch's tags are others, whatever became of this one
           int* st = reinterpret_cast<int*>(s.state);
-          if (ok && !c.failed() && !ld_relaxed_gpu(&status->abort)) {
+          if (ok && best_row == 0x7fffffff) {         // no logit is a number: no next token, the state stays
+            report(status, VDC_ERR_TOKEN, VDC_STEP_KIND, 1, 0, -1);
+          } else if (ok && !c.failed() && !ld_relaxed_gpu(&status->abort)) {
             const int step = st[VDC_ST_STEP], next = pos + 1, page = next / VDC_KV_PAGE;
             reinterpret_cast<int*>(s.log)[step] = best_row;
             st[VDC_ST_TOKEN] = best_row;
