@@ -129,6 +129,16 @@ def test_a_token_outside_the_vocabulary_is_reported(cuda_device):
     assert eng.generate(1)[0] == want[3] and torch.equal(eng.logits, want[1])
 
 
+@pytest.mark.parametrize("pos", [100, 1500])         # one SM walks a head's pages; several do, and merge
+def test_queries_without_a_number_attend_to_nothing(cuda_device, pos):
+    eng = _engine(cuda_device, 1600, hidden=512, n_heads=8, n_kv_heads=2, ffn=512, vocab=640, n_layers=1, qk_norm=True)
+    eng.qknorm[:, :128] = float("nan")
+    caches = eng.kpool.clone(), eng.vpool.clone()
+    (a, la, _, _), = _steps(eng, pos, 1, True, caches)[0]
+    (b, _, _, _), = _steps(eng, pos, 1, False, caches)[0]
+    assert bool(torch.isfinite(la.float()).all()) and rel(a, b) < 1.5e-2
+
+
 def test_logits_without_a_number_are_reported(cuda_device):
     """The step itself ends with the error and leaves state and log; one logit that is a number is enough for a token."""
     from vdcores_b200 import runtime
