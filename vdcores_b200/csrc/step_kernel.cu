@@ -924,6 +924,7 @@ __global__ void __launch_bounds__(kStepThreads + 32, 1) decode_step(const __grid
 
   if (warp == kStepWarps) {
     if (lane == 0) {
+      fence_proxy_async();      // the cache rows of the steps before were written with ordinary stores
       Producer p{sh, wait, base + lay.ring, lay.total - lay.ring};
       const int* table = state + VDC_ST_PAGETABLE;
       // stage after stage; a stage is one run of rows or several (experts), the attention one run per page
