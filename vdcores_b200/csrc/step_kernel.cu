@@ -357,9 +357,6 @@ __device__ __forceinline__ Pages pages_of(const vdc_step& s, int pos, int sm) {
 // ------------------------------------------------------------------------- //
 __device__ __forceinline__ void consumers_sync() { asm volatile("bar.sync 1, %0;" ::"n"(kStepThreads) : "memory"); }
 
-// A head's output; 0 where no score was a number, as in the other attention kernels.
-__device__ __forceinline__ float over(float num, float den) { return den > 0.f ? num / den : 0.f; }
-
 struct Consumer {
   const StepArgs& args;
   const vdc_step& s;
@@ -767,7 +764,8 @@ struct Consumer {
         den = fmaf(wt, w0[k * 40 + g] + w0[k * 40 + 8 + g] + w0[k * 40 + 16 + g] + w0[k * 40 + 24 + g], den);
       }
       if (pg.live == 1) {
-        put(out + (size_t)pg.h * G * (D / 2) + t, pack_bf16x2(over(n0, den), over(n1, den)), tag_out);
+        const float inv = den > 0.f ? 1.f / den : 0.f;       // 0 where no score was a number
+        put(out + (size_t)pg.h * G * (D / 2) + t, pack_bf16x2(n0 * inv, n1 * inv), tag_out);
       } else {
         const size_t u = (size_t)pg.h * s.n_splits + pg.split;
         put2(rec + (u * G * (D / 2) + t) * 2, __float_as_uint(n0), __float_as_uint(n1), tag_rec);
@@ -797,7 +795,8 @@ struct Consumer {
       for (int z = 16; z > 0; z >>= 1) mm = fmaxf(mm, __shfl_xor_sync(0xffffffffu, mm, z));
       const float wt = mk == -INFINITY ? 0.f : exp2f(mk - mm);
       const float den = warp_sum(wt * lk), a = warp_sum(wt * n0), b = warp_sum(wt * n1);
-      if (lane == 0) put(out + (size_t)pg.h * pairs + i, pack_bf16x2(over(a, den), over(b, den)), tag_out);
+      const float inv = den > 0.f ? 1.f / den : 0.f;
+      if (lane == 0) put(out + (size_t)pg.h * pairs + i, pack_bf16x2(a * inv, b * inv), tag_out);
     }
   }
 
