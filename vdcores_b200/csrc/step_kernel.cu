@@ -907,8 +907,11 @@ __global__ void __launch_bounds__(kStepThreads + 32, 1) decode_step(const __grid
   if (tid >= 64 && tid < 64 + D / 2) reinterpret_cast<uint32_t*>(base + lay.rows)[D + tid - 64] = 0u;     // a value row of zeros
   grid_dep_wait();
   grid_dep_launch();
+  // Read before the error is looked for: in a launch that fails, SM 0 counts the launch behind the error.  An SM that starts late
+  // and took the number from there would leave entries that the next launch takes for its own.
+  const uint32_t launches = (uint32_t)ld_acquire_gpu(reinterpret_cast<const int*>(s.work));
   if (__syncthreads_or(ld_relaxed_gpu(&status->abort))) {      // behind an unread error nothing runs
-    if (sm == 0 && tid == 0) *reinterpret_cast<int*>(s.work) += 1;
+    if (sm == 0 && tid == 0) red_release_gpu_add(reinterpret_cast<int*>(s.work), 1);
     return;
   }
 
@@ -991,7 +994,7 @@ __global__ void __launch_bounds__(kStepThreads + 32, 1) decode_step(const __grid
     __syncwarp();
   } else {
     uint64_t* work = reinterpret_cast<uint64_t*>(s.work);
-    const uint32_t tag0 = ((uint32_t)ld_relaxed_gpu(reinterpret_cast<const int*>(work)) * (uint32_t)(L + 1) + 1u) * 8u;
+    const uint32_t tag0 = (launches * (uint32_t)(L + 1) + 1u) * 8u;
     Consumer c{args, s, lay, sh, wait, base, tid, warp, lane, sm};
     auto scaled2 = [&](int row, uint64_t sc, size_t at) {
       float2 v = c.sum2(row);
@@ -1178,7 +1181,7 @@ __global__ void __launch_bounds__(kStepThreads + 32, 1) decode_step(const __grid
         warp_best(best, best_row);
         ok = __all_sync(0xffffffffu, ok);
         if (lane == 0) {
-          *reinterpret_cast<int*>(work) += 1;        // the next launch's tags are others, whatever became of this one
+          red_release_gpu_add(reinterpret_cast<int*>(s.work), 1);      // the next launch's tags are others, whatever became of this one
           int* st = reinterpret_cast<int*>(s.state);
           if (ok && best_row == 0x7fffffff) {         // no logit is a number: no next token, the state stays
             report(status, VDC_ERR_TOKEN, VDC_STEP_KIND, 1, 0, -1);
