@@ -42,6 +42,9 @@ CASES = [
     (dict(hidden=512, n_heads=8, n_kv_heads=2, ffn=1024, vocab=2048, n_layers=3), (199, 255, 256, 257), None),
     # splits of several pages, the last ones empty; a head group of 8; q/k norms
     (dict(hidden=1024, n_heads=16, n_kv_heads=2, ffn=1280, vocab=530, n_layers=2, qk_norm=True), (1200, 4095), None),
+    # more splits of a head than a warp has lanes: 32 of four pages, 33, 119 of five, the last one smaller
+    (dict(hidden=512, n_heads=4, n_kv_heads=1, ffn=512, vocab=64, n_layers=1), (8191, 8192, 37900), None),
+    (dict(hidden=512, n_heads=16, n_kv_heads=2, ffn=512, vocab=64, n_layers=1), (9000, 23000), 132),
     # K ranges that do not divide among the warps (7, 5 and 3 steps), rows over 28 KB, an odd number of SMs
     (dict(hidden=1280, n_heads=8, n_kv_heads=2, ffn=14336, vocab=1000, n_layers=1), (300,), 61),
     (dict(hidden=1792, n_heads=16, n_kv_heads=4, ffn=768, vocab=4096, n_layers=2), (70,), 17),
@@ -57,6 +60,7 @@ CASES = [
 def test_step_kernel_against_the_megakernels_program(cuda_device, kw, positions, num_sms):
     eng = _engine(cuda_device, (max(positions) + 70) // 64 * 64, num_sms=num_sms, **dict(kw))
     assert eng.step_kernel is not None
+    assert eng.step_kernel.n_splits == min(eng.num_sms // eng.cfg.n_kv_heads, eng.max_pages)
     caches = eng.kpool.clone(), eng.vpool.clone()
     for pos in positions:
         n = 1 if pos + 3 > eng.max_seq else 3

@@ -28,11 +28,11 @@ constexpr int kItemBytes = 32 * 1024;                // bytes of one, at most
 constexpr int kPageBytes = VDC_KV_PAGE * VDC_HEAD_DIM * 2;
 constexpr int kGroups = kStepWarps / 4;              // of four warps: a page of the cache each
 constexpr int kAlone = 4;                            // pages that one SM walks without splitting them
+constexpr int kFewSplits = 32;                       // of a head, while that leaves each kAlone pages at most
 constexpr int kOutLd = VDC_HEAD_DIM + 4;
 constexpr int kPartFloats = 4 * 8 * kOutLd;          // partial sums of rows; also the groups' partial heads
 constexpr int kQLd = VDC_HEAD_DIM / 2 + 4;           // words of a query row in shared memory
 constexpr int kPLd = VDC_KV_PAGE / 2 + 4;            // words of a row of probabilities
-constexpr int kMaxSplits = 32;
 constexpr int kMaxTopK = 16, kMaxExperts = 256;
 constexpr int kStepSmem = 227 * 1024 - 1024;         // dynamic; the rest is StepShared's barriers
 
@@ -337,13 +337,17 @@ struct Producer {
 };
 
 // An SM's share of the attention: one KV head's pages first .. first + count - 1; `live` splits of the head have pages.  Up to
-// kAlone pages stay with one SM: there is nothing to merge then.
+// kAlone pages stay with one SM: there is nothing to merge then.  Few KV heads leave a head more splits than a warp has lanes;
+// they are used once 32 splits would walk more than kAlone pages each.  Eight layers of width 1024 with one KV head at 32000 /
+// 128000 positions 373 -> 274 and 839 -> 396 us, two 382 -> 315 and 876 -> 533 (with 8 or 16 pages in place of kAlone one head
+// at 32000 positions takes 309 and 386).
 struct Pages {
   int h, split, live, first, count;
 };
 __device__ __forceinline__ Pages pages_of(const vdc_step& s, int pos, int sm) {
   Pages p{sm % s.n_kv, sm / s.n_kv, 0, 0, 0};
-  const int n = min(pos / VDC_KV_PAGE + 1, s.max_pages), per = n <= kAlone ? n : (n + s.n_splits - 1) / s.n_splits;
+  const int n = min(pos / VDC_KV_PAGE + 1, s.max_pages);
+  const int per = n <= kAlone ? n : max((n + s.n_splits - 1) / s.n_splits, min((n + kFewSplits - 1) / kFewSplits, kAlone));
   p.live = (n + per - 1) / per;
   if (p.split < p.live) {
     p.first = p.split * per;
@@ -773,14 +777,15 @@ struct Consumer {
       }
     }
     if (pg.live == 1) return;
-    // the head's pairs of dims are shared by its units: a lane per split
+    // the head's pairs of dims are shared by its units: a lane takes every 32nd split.  The first one by itself: a loop over all
+    // of them lets the lanes drift apart while they poll (four 8B-shaped e4m3 layers 330 -> 368 us).
     const int pairs = G * (D / 2), lo = pairs * pg.split / pg.live, hi = pairs * (pg.split + 1) / pg.live;
 #pragma unroll 1
     for (int i = lo + warp; i < hi; i += kStepWarps) {
       float mk = -INFINITY, lk = 0.f, n0 = 0.f, n1 = 0.f;
       bool ok = true;
-      if (lane < pg.live) {
-        const size_t u = (size_t)pg.h * s.n_splits + lane;
+      auto take = [&](int sp, float& n0, float& n1, float& mk, float& lk) {
+        const size_t u = (size_t)pg.h * s.n_splits + sp;
         const uint64_t *rp = rec + (u * pairs + i) * 2, *mp = ml + (u * G + i / (D / 2)) * 2;
         Two r = get2(rp), z = get2(mp);
         ok = poll2(rp, tag_rec, r) && poll2(mp, tag_rec, z);
@@ -788,6 +793,18 @@ struct Consumer {
         n1 = __uint_as_float((uint32_t)r.b);
         mk = __uint_as_float((uint32_t)z.a);
         lk = __uint_as_float((uint32_t)z.b);
+      };
+      if (lane < pg.live) take(lane, n0, n1, mk, lk);
+#pragma unroll 1
+      for (int sp = lane + 32; sp - lane < pg.live; sp += 32) {
+        if (sp >= pg.live || !ok) continue;
+        float a0, a1, m1, l1;
+        take(sp, a0, a1, m1, l1);
+        const float m2 = fmaxf(mk, m1), w0 = mk == -INFINITY ? 0.f : exp2f(mk - m2), w1 = m1 == -INFINITY ? 0.f : exp2f(m1 - m2);
+        n0 = fmaf(w0, n0, w1 * a0);
+        n1 = fmaf(w0, n1, w1 * a1);
+        lk = fmaf(w0, lk, w1 * l1);
+        mk = m2;
       }
       if (!__all_sync(0xffffffffu, ok)) break;
       float mm = mk;
@@ -1212,7 +1229,7 @@ extern "C" const char* vdc_step_refuses(const vdc_step* s, bool pointers) {
   auto al16 = [](uint64_t p) { return p != 0 && (p & 15) == 0; };
   if (s->num_sms < 1 || s->num_sms > VDC_MAX_SMS || s->n_layers < 1 || s->wfmt < 0 || s->wfmt > 2) return "step: bad shape";
   if ((s->group != 4 && s->group != 8) || s->n_kv < 1 || s->max_pages < 1 || s->max_seq < 1) return "step: bad heads or pages";
-  if (s->n_splits < 1 || s->n_splits > kMaxSplits || s->n_splits * s->n_kv > s->num_sms) return "step: more attention units than SMs";
+  if (s->n_splits < 1 || s->n_splits > s->num_sms / s->n_kv) return "step: more attention units than SMs";
   const int u = unit_of(s->wfmt), Q = s->n_kv * s->group * VDC_HEAD_DIM;
   if (s->hidden < 512 && s->hidden != 256) return "step: hidden too small";
   if (s->hidden > 8192 || s->hidden % u || s->hidden % 256 || s->ffn < u || s->ffn % u || Q % u || s->vocab < 2 || s->vocab % 2)

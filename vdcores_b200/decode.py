@@ -664,7 +664,7 @@ class DecodeEngine:
         s = runtime.Step(num_sms=self.num_sms, n_layers=cfg.n_layers, hidden=cfg.hidden, ffn=cfg.ffn, vocab=cfg.vocab,
                          n_kv=cfg.n_kv_heads, group=cfg.group, wfmt={"bf16": 0, "fp8": 1, "nvfp4": 2}[self.wkind],
                          max_pages=self.max_pages, max_seq=self.max_seq, n_experts=cfg.n_experts,
-                         n_splits=min(self.num_sms // cfg.n_kv_heads, self.max_pages, 32),
+                         n_splits=min(self.num_sms // cfg.n_kv_heads, self.max_pages),
                          top_k=cfg.top_k if cfg.n_experts else 0, eps=cfg.eps, qk_eps=cfg.qk_norm_eps)
         nbytes = runtime.step_workspace(s)
         if nbytes is None:
