@@ -80,7 +80,8 @@ __global__ void __launch_bounds__(kWideThreads, 1) wide_gemm(const __grid_consta
   if (tid == 0) {
     for (int i = 0; i < kWideRing; ++i) {
       mbar_init(&sh.full[i], 1);
-      mbar_init(&sh.empty[i], 1);
+      // the MMAs have read it; and the team that does not widen it has seen it come (the one that does has, for them)
+      mbar_init(&sh.empty[i], kFmt != 0 ? 1 + kWideWorkers / 2 : 1);
       mbar_init(&sh.ready[i], kWideWorkers / 2);
     }
     for (int i = 0; i < 2; ++i) {
@@ -216,7 +217,10 @@ __global__ void __launch_bounds__(kWideThreads, 1) wide_gemm(const __grid_consta
           seen = wait(&sh.full[st], at_ring.parity, 3, it) &&
                  (!mine || it < 2 || wait(&sh.stg_empty[it & 1], (uint32_t)((it >> 1) - 1) & 1u, 3, it));
           if (!(seen = __all_sync(0xffffffffu, seen))) break;
-          if (!mine) continue;
+          if (!mine) {
+            if (lane == 0) mbar_arrive(&sh.empty[st]);
+            continue;
+          }
           uint8_t* dst = staging + (it & 1) * (NT * kKc * 2);
           const uint8_t* src = ring + st * stage_bytes + per * kSub;
           for (int g = 0, row = t512 & 255; g < 4; row += 256) {       // consecutive threads take consecutive rows
