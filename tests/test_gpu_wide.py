@@ -63,6 +63,7 @@ def test_prompt_in_one_pass_agrees_with_its_chunks(cuda_device, kind, fmt, T, ch
     eng.init_random_weights(3)
     prompt = torch.randint(0, cfg.vocab, (T,), generator=torch.Generator().manual_seed(T))
     pre = PrefillEngine(eng, chunk=chunk, timeout_ns=500_000_000).adopt_weights()
+    lists = dict(pre._wide.lists)
     got = []
     for wide in (True, False):
         if not wide:
@@ -71,6 +72,7 @@ def test_prompt_in_one_pass_agrees_with_its_chunks(cuda_device, kind, fmt, T, ch
         eng.kpool.zero_()
         eng.vpool.zero_()
         first = pre.prefill(prompt)
+        assert not wide or pre._wide.lists == lists          # the first prompt of a length plans nothing
         top = torch.topk(pre.read_hidden(pre.hidden)[(T - 1) % chunk].float(), 1)
         got.append((first, pre.read_hidden(pre.hidden).clone(), eng.kpool.clone(), eng.vpool.clone(), top))
     (f1, h1, k1, v1, _), (f0, h0, k0, v0, _) = got

@@ -23,6 +23,8 @@ from . import isa, runtime
 from .batch import BatchDecodeEngine
 from .decode import BF16, DecodeEngine
 
+STAGE = np.dtype(runtime.Stage)
+
 
 class PrefillEngine(BatchDecodeEngine):
     """`chunk` prompt positions per list of stages into the KV pools of `target` (a DecodeEngine of the same model)."""
@@ -148,8 +150,8 @@ class WideStages:
         self.sums = z(max(R, min(8 * R, 2048)) * max(e.qkv_rows, H), torch.float32)
         self.block = z(self.HEADER + e.max_pages + self.rows, torch.int32)       # header, page table, ids
         self.table = e.page_table.numpy()
-        self.lists = {}
         self.template, self.places = self._plan()
+        self.lists = {r: self._stages(r) for r in range(128, R + 1, 128)}
         # what follows the last layer: the last chunk's rows, then the chunk's own final stages
         tail = runtime.Stage(kind=isa.STAGE_WIDE_TAIL, B=B, Bpad=e.bpad, K=H, x=self.hidden.data_ptr(), hid=e.hidden.data_ptr(),
                              stats_out=e.stats[2 * cfg.n_layers].data_ptr(), state=self.block.data_ptr())
@@ -190,22 +192,20 @@ class WideStages:
         places = {"wqkv": (1, 2, e.qkv_rows, H), "wo": (4, 5, H, Q), "wgu": (6, 0, 2 * F, H), "wd": (7, 8, H, F)}
         return (S * len(out))(*out), places
 
-    def stages(self, R: int):
+    def _stages(self, R: int):
         """The stages of a pass over R rows."""
-        if R not in self.lists:
-            e, cfg = self.e, self.e.cfg
-            arr = type(self.template).from_buffer_copy(self.template)
-            v = np.ctypeslib.as_array(arr)
-            v["Bpad"] = R
-            n = 8 * cfg.n_layers
-            v["splits"][1 + 3:1 + n:8] = e._splits(cfg.n_kv_heads * (R // (64 // cfg.group)), 2, e.max_pages)
-            for name, (at, reader, M, K) in self.places.items():
-                subs, cols, ks = runtime.wide_tiles(R, M, K, self.fmt, self.sms, name == "wgu")
-                v["group"][1 + at:1 + n:8], v["n_kv"][1 + at:1 + n:8], v["splits"][1 + at:1 + n:8] = subs, cols, ks
-                if reader:
-                    v["splits"][1 + reader:2 + n:8] = ks
-            self.lists[R] = arr
-        return self.lists[R]
+        e, cfg = self.e, self.e.cfg
+        arr = type(self.template).from_buffer_copy(self.template)
+        v = np.frombuffer(arr, dtype=STAGE)
+        v["Bpad"] = R
+        n = 8 * cfg.n_layers
+        v["splits"][1 + 3:1 + n:8] = e._splits(cfg.n_kv_heads * (R // (64 // cfg.group)), 2, e.max_pages)
+        for name, (at, reader, M, K) in self.places.items():
+            subs, cols, ks = runtime.wide_tiles(R, M, K, self.fmt, self.sms, name == "wgu")
+            v["group"][1 + at:1 + n:8], v["n_kv"][1 + at:1 + n:8], v["splits"][1 + at:1 + n:8] = subs, cols, ks
+            if reader:
+                v["splits"][1 + reader:2 + n:8] = ks
+        return arr
 
     def sends(self, T: int) -> int:
         """Blocks of the engine's pinned memory that a prompt's ids and page tables take."""
@@ -228,6 +228,6 @@ class WideStages:
                 def fill(s, w=w):
                     s.reshape(-1)[:len(w)] = w
                 send(fill, self.block[w0:w0 + len(w)])
-            launch(self.stages(-(-len(part) // 128) * 128))
+            launch(self.lists[-(-len(part) // 128) * 128])
         n = len(ids)
         self.last[0].M = (n - 1) // self.e.batch * self.e.batch % self.rows      # the last chunk's first row in its pass
