@@ -84,3 +84,26 @@ def test_prompt_in_one_pass_agrees_with_its_chunks(cuda_device, kind, fmt, T, ch
         rows = (a.float() - b.float()).flatten(0, 2).norm(dim=1) / b.float().flatten(0, 2).norm(dim=1).clamp_min(1e-6)
         assert float(rows.max()) < 1e-2
     assert bool(((k1 == 0) == (k0 == 0)).float().mean() > 0.999)     # nothing written past the prompt
+
+
+def test_prompts_go_chunk_by_chunk_without_the_wide_buffers(cuda_device, monkeypatch):
+    """No buffers are taken where no prompt is longer than a chunk, and none are needed where there is no room for them."""
+    from tests.helpers import engine_config, small_cfg
+    from vdcores_b200 import prefill
+    from vdcores_b200.decode import DecodeEngine
+    eng = DecodeEngine(engine_config(small_cfg("llama")), 65, device=cuda_device)
+    eng.init_random_weights(3)
+    prompt = torch.arange(3, 53)
+    assert prefill.PrefillEngine(eng, chunk=64).adopt_weights()._wide is None
+    wide = prefill.PrefillEngine(eng, chunk=32).adopt_weights()
+    assert wide._goes_wide(50)
+    want = wide.prefill(prompt), eng.kpool.clone()
+
+    def no_room(self, e):
+        raise torch.cuda.OutOfMemoryError
+    monkeypatch.setattr(prefill.WideStages, "__init__", no_room)
+    pre = prefill.PrefillEngine(eng, chunk=32).adopt_weights()
+    assert not pre._goes_wide(50)
+    eng.kpool.zero_()
+    pre.prefill(prompt)
+    assert rel(eng.kpool, want[1]) < 1e-2

@@ -1,8 +1,8 @@
 """Prefill on the device: the prompt's positions as rows of stage kernels.
 
-A prompt goes through a layer with all its rows together, up to isa.WIDE_ROWS of them (csrc/wide_kernels.cu): the weights are
-read once and the tensor cores are the bound.  On a part of the SMs (num_sms below the device's) it goes chunk by chunk
-through the batched step's stages instead.
+A prompt longer than a chunk goes through a layer with all its rows together, up to isa.WIDE_ROWS of them
+(csrc/wide_kernels.cu): the weights are read once and the tensor cores are the bound.  On a part of the SMs (num_sms below the
+device's), or without room for those rows' buffers, it goes chunk by chunk through the batched step's stages instead.
 
 The chunks: the batched decode step (batch.BatchDecodeEngine) already computes, for every row of its batch, exactly what a prompt
 position needs; what differs in a prefill is that the rows are consecutive positions of ONE sequence.  PrefillEngine
@@ -27,7 +27,9 @@ STAGE = np.dtype(runtime.Stage)
 
 
 class PrefillEngine(BatchDecodeEngine):
-    """`chunk` prompt positions per list of stages into the KV pools of `target` (a DecodeEngine of the same model)."""
+    """Prompts into the KV pools of `target` (a DecodeEngine of the same model).  `chunk` rows at most go through the batched
+    step's stages at a time; it bounds neither the rows of a longer prompt's launches nor what the engine holds for them, which
+    is the buffers of WideStages: for an 8B shape 176 MB, when max_seq is 2048 or more."""
     SHARED_CACHE = True
     BLOCKS = 4          # chunks whose state blocks may wait in host memory
 
@@ -61,7 +63,12 @@ class PrefillEngine(BatchDecodeEngine):
         the last chunk adds the final norm, the vocabulary projection and the argmax (the first generated id)."""
         super()._build_program()
         self._body = self._plan(vocab=False)
-        self._wide = None if self.max_ctas else WideStages(self)
+        self._wide = None
+        if not self.max_ctas and self.max_seq - 1 > self.batch:      # otherwise no prompt is longer than a chunk
+            try:
+                self._wide = WideStages(self)
+            except torch.cuda.OutOfMemoryError:
+                pass                                                 # prompts go chunk by chunk
         self._first = torch.zeros(1, dtype=torch.int32).pin_memory()
 
     def launches(self, T: int) -> int:
