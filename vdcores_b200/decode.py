@@ -570,10 +570,11 @@ class DecodeEngine:
                         x = Src(act + half * Kh * 2, Kh * 2, wait=b_half)
                         if half == 0:
                             add_gemv(sm, (wa, n * rb(Kh)), w_addr=wa, n_rows=n, K=Kh, R=R, x=x, **sk('wd', l, r0),
-                                     out=Dst(part + r0 * 4, n * 4, "store"), mode=isa.GEMV_MODE_STORE_F32)
+                                     out=Dst(part + r0 * 4, n * 4, "store"), mode=isa.GEMV_MODE_STORE_F32, **(ctr or {}))
                         else:
                             add_gemv(sm, (wa, n * rb(Kh)), w_addr=wa, n_rows=n, K=Kh, R=R, x=x, **sk('wd', l, r0),
-                                     out=Dst(hid + r0 * 2, n * 2, "add_bf16", release=b_hid), partial_in=part + r0 * 4)
+                                     out=Dst(hid + r0 * 2, n * 2, "add_bf16", release=b_hid), partial_in=part + r0 * 4,
+                                     **(ctr or {}))
             else:
                 b_gu = halves[0][0]
                 R = rpc(F)
