@@ -73,9 +73,17 @@ def test_prompt_in_one_pass_agrees_with_its_chunks(cuda_device, kind, fmt, T, ch
         eng.vpool.zero_()
         first = pre.prefill(prompt)
         assert not wide or pre._wide.lists == lists          # the first prompt of a length plans nothing
-        top = torch.topk(pre.read_hidden(pre.hidden)[(T - 1) % chunk].float(), 1)
-        got.append((first, pre.read_hidden(pre.hidden).clone(), eng.kpool.clone(), eng.vpool.clone(), top))
-    (f1, h1, k1, v1, _), (f0, h0, k0, v0, _) = got
+        hidden = pre.read_hidden(pre.hidden)
+        # the id: the largest logit of the last row, where the next one is further off than roundings (2^-9 of the row's size)
+        x = hidden[(T - 1) % chunk].float()
+        x = (x * torch.rsqrt(x.pow(2).mean() + cfg.eps)).to(BF16) * eng.norm_w
+        logits = x.float() @ eng.lm_head.float().t()
+        top = torch.topk(logits, 2)
+        clear = float(top.values[0] - top.values[1]) > 2.0 ** -7 * float(top.values[0].abs())
+        assert first == int(top.indices[0]) or not clear
+        got.append((first, hidden.clone(), eng.kpool.clone(), eng.vpool.clone(), clear))
+    (f1, h1, k1, v1, clear1), (f0, h0, k0, v0, clear0) = got
+    assert f1 == f0 or not (clear1 and clear0)
     assert bool(torch.isfinite(h1.float()).all())
     for a, b in ((h1, h0), (k1[1:], k0[1:]), (v1[1:], v0[1:])):
         assert rel(a, b) < 1e-2          # sums in other orders, rounded to bf16 through two or three layers
@@ -107,3 +115,50 @@ def test_prompts_go_chunk_by_chunk_without_the_wide_buffers(cuda_device, monkeyp
     eng.kpool.zero_()
     pre.prefill(prompt)
     assert rel(eng.kpool, want[1]) < 1e-2
+
+
+def test_an_id_outside_the_vocabulary_ends_a_prompt_with_an_error(cuda_device):
+    from tests.helpers import engine_config, small_cfg
+    from vdcores_b200 import isa, runtime
+    from vdcores_b200.decode import DecodeEngine
+    from vdcores_b200.prefill import PrefillEngine
+    eng = DecodeEngine(engine_config(small_cfg("llama")), 320, device=cuda_device)
+    eng.init_random_weights(3)
+    pre = PrefillEngine(eng, chunk=64, timeout_ns=500_000_000).adopt_weights()
+    prompt = torch.randint(0, eng.cfg.vocab, (200,), generator=torch.Generator().manual_seed(5))
+    first, keys = pre.prefill(prompt), eng.kpool.clone()
+    for bad in (-1, eng.cfg.vocab, 2 ** 31 - 1):
+        wrong = prompt.clone()
+        wrong[130] = bad
+        eng.set_state(7, 3)
+        state = eng.state.clone()
+        with pytest.raises(runtime.VdcError) as e:
+            pre.prefill(wrong)
+        assert e.value.code == 5 and e.value.status["pc"] == 130 and e.value.status["opcode"] == isa.STAGE_WIDE_EMBED
+        assert e.value.status["aux"] == bad and torch.equal(eng.state, state)
+    eng.kpool.zero_()
+    assert pre.prefill(prompt) == first and torch.equal(eng.kpool, keys)
+
+
+@pytest.mark.parametrize("fmt", ["bf16", "fp8"])
+def test_a_wait_that_runs_out_ends_with_an_error(cuda_device, fmt):
+    """Waits limited to a nanosecond: a projection ends as it should or with the timeout in the status block; the next launch
+    with a proper limit is right."""
+    from vdcores_b200 import isa, runtime
+    dev, R, M, K = cuda_device, 256, 4096, 2048
+    w, sc, _ = weights(M, K, fmt, dev)
+    xd = _rows(seeded((R, K), 1).to(dev))
+    out = torch.zeros(M // 4, R, 4, device=dev)
+    s = runtime.Stage(kind=isa.STAGE_WIDE_GEMM, mode=isa.STAGE_SUMS, wfmt=int(fmt == "fp8"), Bpad=R, M=M, K=K, group=2, n_kv=128,
+                      splits=1, w=w.data_ptr(), scales=sc.data_ptr() if sc is not None else 0, x=xd.data_ptr(), out=out.data_ptr())
+    stream, want = torch.cuda.current_stream(dev).cuda_stream, None
+    for i in range(21):
+        out.zero_()
+        runtime.launch_stages((runtime.Stage * 1)(s), stream, 1 if i % 2 else 500_000_000)
+        try:
+            runtime.read_status(stream)
+        except runtime.VdcError as e:
+            assert i % 2 and e.code == 1 and e.status["opcode"] == isa.STAGE_WIDE_GEMM
+            continue
+        want = out.clone() if want is None else want
+        assert torch.equal(out, want)

@@ -58,6 +58,7 @@ STAGE_WIDE_EMBED, STAGE_WIDE_GEMM, STAGE_WIDE_HEADS, STAGE_WIDE_ATTN, STAGE_WIDE
     _defs["STAGE_WIDE_" + k] for k in ("EMBED", "GEMM", "HEADS", "ATTN", "NORM", "TAIL"))
 STAGE_SUMS = _defs["STAGE_SUMS"]
 STAGE_BLOCK = _defs["STAGE_BLOCK"]
+STEP_KIND = _defs["STEP_KIND"]
 WIDE_ROWS, WIDE_POS, WIDE_N = _defs["WIDE_ROWS"], _defs["WIDE_POS"], _defs["WIDE_N"]
 
 ST_POS, ST_NPAGES, ST_TOKEN, ST_STEP = _defs["ST_POS"], _defs["ST_NPAGES"], _defs["ST_TOKEN"], _defs["ST_STEP"]
