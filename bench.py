@@ -3,7 +3,7 @@
 
     python bench.py [--gpus N] [--steps K] [--warmup W] [--impl reference]
 
-One step = one greedy decode step (batch 1: one megakernel launch; larger
+One step = one greedy decode step (batch 1: one kernel launch; larger
 batches: a list of stage kernels) after a 2048-token prompt has been prefilled
 into the paged KV cache.  Weights are random
 N(0, 0.02) bf16 of the named shape, the prompt is uniform random ids (synthetic
@@ -418,14 +418,14 @@ def run_prefill(eng, prompt, on_device):
     if not on_device:
         return eng.prefill(prompt), {"impl": "PyTorch ops (library GEMMs)", "prompt_tokens": T}
     if eng.cfg.n_experts:
-        # mixture-of-experts models: the decode program itself over the prompt, one position per launch
+        # mixture-of-experts models: the decode step itself over the prompt, one position per launch
         torch.cuda.synchronize()
         t0 = time.perf_counter()
         first = eng.prefill_device(prompt)
         torch.cuda.synchronize()
         dt = time.perf_counter() - t0
-        return first, {"impl": "megakernel, one prompt position per launch (the decode program)", "prompt_tokens": T,
-                       "ms": dt * 1e3, "tokens_per_s": T / dt, "launches": T}
+        return first, {"impl": f"{'step kernel' if eng.step_kernel else 'megakernel program'}, one prompt position per launch",
+                       "prompt_tokens": T, "ms": dt * 1e3, "tokens_per_s": T / dt, "launches": T}
     # the prompt goes through the stage kernels into this engine's own pools
     from vdcores_b200.prefill import PrefillEngine
     pre = PrefillEngine(eng, chunk=128).adopt_weights()

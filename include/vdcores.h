@@ -134,12 +134,12 @@ int vdc_wide_tiles(int rows, int M, int K, int wfmt, int sms, int whole, int* ou
 /* One token of a model at batch 1 as one persistent kernel on num_sms SMs (csrc/step_kernel.cu): weights row-major as the
  * decode engine stores them, layer after layer (wqkv: per KV head `group` query heads, key, value; wgu: gate and up rows
  * alternate, with experts [layer][expert]), caches [layer][page][kv head][64][128], `state` the engine's state block.  wfmt 0
- * bf16, 1 e4m3 rows, 2 NVFP4 rows, the last two with fp32 row scales s_*.  The kernel appends the cache row, writes the final
- * hidden state, the logits, the next token to log, and moves the state on; taps (0: none) gets every layer's hidden state,
- * route the expert ids and weights of the last layer.  work: vdc_step_workspace bytes, zeroed once, one per engine.
- * Pointers are device addresses. */
+ * bf16, 1 e4m3 rows, 2 NVFP4 rows, the last two with fp32 row scales s_*.  n_splits: SMs that share a head's pages, num_sms /
+ * n_kv at most.  The kernel appends the cache row, writes the final hidden state, the logits, the next token to log, and moves
+ * the state on; taps (0: none) gets every layer's hidden state, route the expert ids and weights of the last layer.  work:
+ * vdc_step_workspace bytes, zeroed once, one per engine.  Pointers are device addresses. */
 typedef struct {
-  int32_t num_sms, n_layers, hidden, ffn, vocab, n_kv, group, wfmt, max_pages, max_seq, n_splits, n_experts, top_k, reserved;
+  int32_t num_sms, n_layers, hidden, ffn, vocab, n_kv, group, wfmt, max_pages, n_splits, n_experts, top_k;
   float eps, qk_eps;
   uint64_t embed, lm_head, norm_w, ln1, ln2, wqkv, wo, wgu, wd, s_qkv, s_o, s_gu, s_d, qk_norm, router;
   uint64_t kpool, vpool, state, rope, log, logits, hidden_out, taps, route, work;

@@ -5,7 +5,7 @@ import pytest
 def step(hidden, ffn, num_sms, n_kv=1, group=4, vocab=64, experts=0, top_k=0, wfmt=0, splits=1):
     from vdcores_b200 import runtime
     return runtime.Step(num_sms=num_sms, n_layers=1, hidden=hidden, ffn=ffn, vocab=vocab, n_kv=n_kv, group=group, wfmt=wfmt,
-                        max_pages=4, max_seq=256, n_splits=splits, n_experts=experts, top_k=top_k, eps=1e-5, qk_eps=1e-5)
+                        max_pages=4, n_splits=splits, n_experts=experts, top_k=top_k, eps=1e-5, qk_eps=1e-5)
 
 
 def sums_and_room(rows, unit, K, num_sms, slots, experts):

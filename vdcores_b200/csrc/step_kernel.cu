@@ -1228,7 +1228,7 @@ extern "C" const char* vdc_step_refuses(const vdc_step* s, bool pointers) {
   using namespace vdc;
   auto al16 = [](uint64_t p) { return p != 0 && (p & 15) == 0; };
   if (s->num_sms < 1 || s->num_sms > VDC_MAX_SMS || s->n_layers < 1 || s->wfmt < 0 || s->wfmt > 2) return "step: bad shape";
-  if ((s->group != 4 && s->group != 8) || s->n_kv < 1 || s->max_pages < 1 || s->max_seq < 1) return "step: bad heads or pages";
+  if ((s->group != 4 && s->group != 8) || s->n_kv < 1 || s->max_pages < 1) return "step: bad heads or pages";
   if (s->n_splits < 1 || s->n_splits > s->num_sms / s->n_kv) return "step: more attention units than SMs";
   const int u = unit_of(s->wfmt), Q = s->n_kv * s->group * VDC_HEAD_DIM;
   if (s->hidden < 512 && s->hidden != 256) return "step: hidden too small";

@@ -664,7 +664,7 @@ class DecodeEngine:
             return None
         s = runtime.Step(num_sms=self.num_sms, n_layers=cfg.n_layers, hidden=cfg.hidden, ffn=cfg.ffn, vocab=cfg.vocab,
                          n_kv=cfg.n_kv_heads, group=cfg.group, wfmt={"bf16": 0, "fp8": 1, "nvfp4": 2}[self.wkind],
-                         max_pages=self.max_pages, max_seq=self.max_seq, n_experts=cfg.n_experts,
+                         max_pages=self.max_pages, n_experts=cfg.n_experts,
                          n_splits=min(self.num_sms // cfg.n_kv_heads, self.max_pages),
                          top_k=cfg.top_k if cfg.n_experts else 0, eps=cfg.eps, qk_eps=cfg.qk_norm_eps)
         nbytes = runtime.step_workspace(s)
@@ -854,12 +854,12 @@ class DecodeEngine:
         return tok
 
     def prefill_device(self, tokens: torch.Tensor) -> int:
-        """The prompt goes through the decode megakernel itself, one position per launch: the same program as a
+        """The prompt goes through the decode step itself, one position per launch: the same kernel as a
         decode step, with the next prompt id written over the step's own argmax before the next launch (an 8-byte
         device-to-device copy on the engine's stream: {next id, step counter 0}).  No PyTorch arithmetic and no
         host round trip inside the loop; the KV rows and the returned first generated id have exactly the decode
-        path's numerics.  Cost: one decode step per prompt position (PrefillEngine in prefill.py does up to 128
-        positions per list of stage kernels)."""
+        path's numerics.  Cost: one decode step per prompt position (PrefillEngine in prefill.py takes up to 2048
+        positions through a layer together)."""
         T = int(tokens.numel())
         assert 1 <= T < self.max_seq
         forced = torch.zeros(T, 2, dtype=torch.int32)

@@ -44,7 +44,7 @@ class Stage(ctypes.Structure):
 class Step(ctypes.Structure):
     """One token at batch 1 (vdc_step in include/vdcores.h, which documents the fields)."""
     _fields_ = ([(n, ctypes.c_int32) for n in ("num_sms", "n_layers", "hidden", "ffn", "vocab", "n_kv", "group", "wfmt", "max_pages",
-                                               "max_seq", "n_splits", "n_experts", "top_k", "reserved")]
+                                               "n_splits", "n_experts", "top_k")]
                 + [(n, ctypes.c_float) for n in ("eps", "qk_eps")]
                 + [(n, ctypes.c_uint64) for n in ("embed", "lm_head", "norm_w", "ln1", "ln2", "wqkv", "wo", "wgu", "wd", "s_qkv",
                                                   "s_o", "s_gu", "s_d", "qk_norm", "router", "kpool", "vpool", "state", "rope", "log",
