@@ -10,8 +10,8 @@
 // about 7 us per boundary.
 //
 // Measured against that program (B200): three layers of width 512 109 -> 69 us, eight 8B-shaped bf16 layers and a 128256-row
-// vocabulary projection 1012 -> 977, four such layers e4m3 387 -> 325, NVFP4 388 -> 329, four layers of a 30B mixture of experts
-// 437 -> 264.
+// vocabulary projection 1012 -> 981, four such layers e4m3 387 -> 331, NVFP4 388 -> 326, four layers of a 30B mixture of experts
+// 437 -> 260.
 //
 // An entry buffer is written again one layer later, when everything that read it must have been read: whoever polls a buffer
 // has rows in the same or the following stage, and those rows go into what the next writer of the buffer waits for.
@@ -19,8 +19,9 @@
 
 namespace vdc {
 
-// Consumer warps; one more warp produces.  What every warp executes at a stage's boundaries (some 500 instructions, 1400 around
-// the attention) is bound by instructions issued: eight warps, not sixteen.
+// Consumer warps; one more warp produces.  All of them execute what a stage's boundary needs, each an instruction every ten
+// cycles (it waits for entries in L2, and for the instruction before): eight warps, not sixteen, which took 515 us for four
+// 8B-shaped layers where eight took 451.
 constexpr int kStepWarps = 8;
 constexpr int kStepThreads = 32 * kStepWarps;
 constexpr int kItems = 16;                           // copies in the ring, at most
@@ -196,9 +197,8 @@ __device__ __forceinline__ void add2(float& a, float& b, float x, float y) {
 
 // One step of a warp: 16 bytes per lane of kPairs pairs of rows times the same inputs, as products of 16 x 16 by 16 x 8 tiles.
 // Row g of a tile is what the four lanes 4g .. 4g + 3 hold of the pair's first row (8 + g: of its second), column g what they
-// hold of the inputs: the tile's element (g, g) is the sum of the four lanes' products, the other elements mean nothing.  The
-// loop is bound by instructions issued: a product of tiles is one where FMAs of four rows are 12 (32 KB of bf16 took 0.8 us,
-// HBM 0.73).
+// hold of the inputs: the tile's element (g, g) is the sum of the four lanes' products, the other elements mean nothing.  A
+// product of tiles is one instruction where FMAs of four rows are 12 (32 KB of bf16 took 0.8 us with those, HBM 0.73).
 // The tensor cores cut off what an fp32 sum cannot hold.  So bf16 and e4m3 rows have only two products of tiles (8 of a lane's
 // inputs) added up by them, from zero; those sums meet in rounded additions.  Of 32768 sums of 8192 products around two large
 // ones that cancel, 2.0 % miss their bf16 rounding (FMAs 2.1 %, all products in one sum of the tensor cores 7.2 %).  Four

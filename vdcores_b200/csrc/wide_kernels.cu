@@ -10,7 +10,7 @@
 // adds the splits up in order: no atomics, the same bits every time.
 //
 // Measured (B200): two such layers and a small vocabulary, 2048 tokens 5.1 -> 2.2 ms, 77 tokens (two chunks of 64 before)
-// 660 -> 540 us.  Gate/up of 2048 rows 352 us (1.37 PFLOP/s; cuBLAS 331), down 166 us (1.45; 155).
+// 667 -> 495 us.  Gate/up of 2048 rows 352 us (1.37 PFLOP/s; cuBLAS 331), down 166 us (1.45; 155).
 #include "mk_stage.cuh"
 
 namespace vdc {
@@ -100,8 +100,8 @@ __global__ void __launch_bounds__(kWideThreads, 1) wide_gemm(const __grid_consta
   if (warp < kWideProducers) {
     // A chunk of a tile's weights is cut from at most three blocks of packed rows: per block one piece per eight (bf16) or
     // sixteen inputs, NVFP4 one more for the scales.  Lane i of the producers copies piece i of the chunk, the last two lanes
-    // the rows.  Four warps, because a warp's lanes issue their copies one after another, at 47 ns each (one warp: gate/up of 2048
-    // rows 507 us instead of 420).
+    // the rows.  Four warps, because a warp's lanes issue their copies one after another (one warp: gate/up of 2048 rows 507 us
+    // instead of 420).
     constexpr int kPieces = kFmt == 1 ? 4 : 8;
     const int item = lane * kWideProducers + warp;
     bool ok = true;
