@@ -39,6 +39,12 @@ constexpr int kStepSmem = 227 * 1024 - 1024;         // dynamic; the rest is Ste
 
 enum { kQkv, kOut, kRouter, kGateUp, kDown, kVocab, kStages };
 
+// How an SM's consumers take a stage's rows: first row and rows; rows of a chunk; a warp's steps along the inputs; the teams and
+// the warps along the inputs (log2); a warp's room for partial sums; and the rows between two sums of them.
+struct Plan {
+  int r0, n, per, units, lt, lk, ld, most;
+};
+
 struct StepShared {
   uint64_t full[kItems], empty[kItems], routed;
   int start[kItems];                                 // offset of an item in the ring
@@ -46,7 +52,9 @@ struct StepShared {
   float red[kStepWarps];
   float best[kStepWarps];
   int best_row[kStepWarps];
-  int share[kStages][2];                             // first row and rows of this SM, stage by stage
+  alignas(16) Plan plan[kStages];
+  int slot0, head;                                   // experts: the slot of this SM's first gate/up row, its rows there are
+  int pair0, pair1;                                  // pairs of a head's dims that this SM merges
 };
 // Behind the ring: what the consumers share.
 struct StepLayout {
@@ -106,10 +114,17 @@ __host__ __device__ inline StepWork step_work(const vdc_step& s) {
 
 // What a launch passes: the step, and where its shared memory and its entries lie.  From the constant bank these cost no
 // registers.
+// A stage as the host divides it: the first `more` SMs take each + 1 units of q rows, the others `each`; lt, lk and most for
+// either.  A stage's boundary on the device had 1000 to 2300 cycles of integer divisions for this (of 8000 to 11000).
+struct Deal {
+  int q, each, more, per, units;
+  int lt[2], lk[2], most[2];
+};
 struct StepArgs {
   vdc_step s;
   StepLayout lay;
   StepWork wk;
+  Deal deal[kStages];
 };
 // Rows of a stage that one SM takes.
 struct Share {
@@ -275,6 +290,26 @@ __host__ __device__ inline Split split_of(int fmt, bool experts, int K, int n) {
   return s;
 }
 
+__host__ inline Deal deal_of(const vdc_step& s, int stage) {
+  const int k = s.n_experts ? s.top_k : 1, Q = s.n_kv * s.group * VDC_HEAD_DIM;
+  const int rows[kStages] = {Q + 2 * s.n_kv * VDC_HEAD_DIM, s.hidden, s.n_experts, 2 * s.ffn * k, s.hidden, s.vocab};
+  const int K = stage == kOut ? Q : stage == kDown ? s.ffn : s.hidden, fmt = stage == kVocab ? 0 : s.wfmt;
+  Deal d{};
+  d.q = stage == kGateUp ? 4 : stage == kRouter ? 1 : 2;
+  d.each = rows[stage] / d.q / s.num_sms;
+  d.more = rows[stage] / d.q % s.num_sms;
+  d.per = chunk_rows(row_bytes(fmt, K));
+  d.units = K / unit_of(fmt);
+  for (int i = 0; i < 2; ++i) {
+    const int n = (d.each + (i == 0)) * d.q;
+    const Split sp = split_of(fmt, s.n_experts != 0, K, stage == kDown ? n * k : n);
+    while (1 << d.lt[i] < sp.teams) ++d.lt[i];
+    while (1 << d.lk[i] < sp.kw) ++d.lk[i];
+    d.most[i] = stage == kVocab ? kPartFloats / sp.kw / d.per * d.per : n;
+  }
+  return d;
+}
+
 // ------------------------------------------------------------------------- //
 // producer
 // ------------------------------------------------------------------------- //
@@ -372,6 +407,7 @@ struct Consumer {
   RingAt at{kItems};
   int teams, turn;               // and the chunks until this warp's team is on
   int kw, kg, rw, rg, ld;        // warps along the inputs, this warp's place there; along the rows; rows there is room for
+  int per, units;                // rows of a chunk; steps along the inputs
 
   __device__ __forceinline__ float* part() const { return reinterpret_cast<float*>(base + lay.part); }
   __device__ __forceinline__ uint32_t* hs() const { return reinterpret_cast<uint32_t*>(base + lay.h); }
@@ -486,23 +522,24 @@ struct Consumer {
     consumers_sync();
   }
 
-  template <int kFmt>
-  __device__ __forceinline__ void split(int K, int n) {
-    const Split sp = split_of(kFmt, s.n_experts != 0, K, n);
-    const int warps = kStepWarps / sp.teams;
-    teams = sp.teams;
-    kw = sp.kw;
-    rw = warps / kw;
+  __device__ __forceinline__ void split(const Plan& p) {
+    const int lw = 3 - p.lt;                                   // log2 of a team's warps
+    static_assert(kStepWarps == 8, "log2");
+    teams = 1 << p.lt;
+    kw = 1 << p.lk;
+    rw = 1 << (lw - p.lk);
     kg = warp & (kw - 1);
-    rg = (warp & (warps - 1)) / kw;
-    ld = kPartFloats / kw;
-    turn = warp / warps;
+    rg = (warp & ((1 << lw) - 1)) >> p.lk;
+    turn = warp >> lw;
+    ld = p.ld;
+    per = p.per;
+    units = p.units;
   }
   // n rows from the ring times the inputs xp: every warp's share of row r to part[kg][row0 + r], rows side by side for the
   // threads that add the shares up.
   template <int kFmt, bool kFma>
   __device__ __forceinline__ void rows(int K, int n, const uint8_t* xp, int row0) {
-    const int rb = row_bytes(kFmt, K), per = chunk_rows(rb), units = K / unit_of(kFmt);
+    const int rb = row_bytes(kFmt, K);
 #pragma unroll 1
     for (int r0 = 0; r0 < n; r0 += per, at.next()) {
       if (!wait.warp_wait(&sh.full[at.st], at.parity, 2, r0)) return;
@@ -779,7 +816,7 @@ struct Consumer {
     if (pg.live == 1) return;
     // the head's pairs of dims are shared by its units: a lane takes every 32nd split.  The first one by itself: a loop over all
     // of them lets the lanes drift apart while they poll (four 8B-shaped e4m3 layers 330 -> 368 us).
-    const int pairs = G * (D / 2), lo = pairs * pg.split / pg.live, hi = pairs * (pg.split + 1) / pg.live;
+    const int pairs = G * (D / 2), lo = sh.pair0, hi = sh.pair1;
 #pragma unroll 1
     for (int i = lo + warp; i < hi; i += kStepWarps) {
       float mk = -INFINITY, lk = 0.f, n0 = 0.f, n1 = 0.f;
@@ -906,11 +943,13 @@ __global__ void __launch_bounds__(kStepThreads + 32, 1) decode_step(const __grid
   const Waiter wait{&sh.fail, status, timeout_ns, VDC_STEP_KIND};
   constexpr int D = VDC_HEAD_DIM;
   if (tid < kStages) {
-    const int k = s.n_experts ? s.top_k : 1, q = s.n_kv * s.group * D;
-    const int rows[kStages] = {q + 2 * s.n_kv * D, s.hidden, s.n_experts, 2 * s.ffn * k, s.hidden, s.vocab};
-    const Share r = share_of(rows[tid], tid == kGateUp ? 4 : tid == kRouter ? 1 : 2, sm, sms);
-    sh.share[tid][0] = r.r0;
-    sh.share[tid][1] = r.n;
+    const Deal& d = args.deal[tid];
+    const int i = sm < d.more ? 0 : 1;
+    sh.plan[tid] = Plan{(sm * d.each + min(sm, d.more)) * d.q, (d.each + 1 - i) * d.q, d.per, d.units, d.lt[i], d.lk[i], kPartFloats >> d.lk[i], d.most[i]};
+    if (kExperts && tid == kGateUp) {
+      sh.slot0 = sh.plan[tid].r0 / (2 * s.ffn);
+      sh.head = (sh.slot0 + 1) * 2 * s.ffn - sh.plan[tid].r0;
+    }
   }
   if (tid == 0) {
     for (int i = 0; i < kItems; ++i) {
@@ -937,6 +976,10 @@ __global__ void __launch_bounds__(kStepThreads + 32, 1) decode_step(const __grid
   const int pos = ld_relaxed_gpu(state + VDC_ST_POS);
   const Pages pg = pages_of(s, pos, sm);
   const int slots = E ? s.top_k : 1;
+  if (tid == 0 && pg.count > 0) {      // read behind the attention's barriers
+    sh.pair0 = G * (D / 2) * pg.split / pg.live;
+    sh.pair1 = G * (D / 2) * (pg.split + 1) / pg.live;
+  }
   const int rbH = row_bytes(kFmt, H), rbQ = row_bytes(kFmt, Q), rbF = row_bytes(kFmt, F);
   int* ids = reinterpret_cast<int*>(base + lay.route + kMaxExperts * 4);
   float* weights = reinterpret_cast<float*>(ids + kMaxTopK);
@@ -952,7 +995,7 @@ __global__ void __launch_bounds__(kStepThreads + 32, 1) decode_step(const __grid
       while (p.ok) {
         asm volatile("" : "+r"(stage), "+r"(sub));
         const uint8_t *src = nullptr, *second = nullptr;
-        int n = 0, rb = rbH, r0 = sh.share[stage][0], rows = sh.share[stage][1];
+        int n = 0, rb = rbH, r0 = sh.plan[stage].r0, rows = sh.plan[stage].n;
         bool more = false;                     // the stage goes on
         if (stage == kQkv) {
           src = reinterpret_cast<const uint8_t*>(s.wqkv) + (size_t)l * QKV * rbH;
@@ -977,8 +1020,8 @@ __global__ void __launch_bounds__(kStepThreads + 32, 1) decode_step(const __grid
           src = reinterpret_cast<const uint8_t*>(s.wgu);
           size_t first = (size_t)l * 2 * F;
           if (E) {                             // a slot's rows end where the next slot's begin
-            if (sub == 0 && (rows || sh.share[kDown][1]) && !(p.ok = wait(&sh.routed, (uint32_t)l & 1u, 0, l))) break;
-            const int end = r0 + rows, slot = r0 / (2 * F) + sub;
+            if (sub == 0 && (rows || sh.plan[kDown].n) && !(p.ok = wait(&sh.routed, (uint32_t)l & 1u, 0, l))) break;
+            const int end = r0 + rows, slot = sh.slot0 + sub;
             r0 = max(r0, slot * 2 * F);
             rows = min(end, (slot + 1) * 2 * F) - r0;
             more = r0 + rows < end;
@@ -996,7 +1039,7 @@ __global__ void __launch_bounds__(kStepThreads + 32, 1) decode_step(const __grid
           src = reinterpret_cast<const uint8_t*>(s.lm_head);
         }
         if (rows > 0) {
-          const int per = second ? 1 : chunk_rows(rb);
+          const int per = second ? 1 : sh.plan[stage].per;
           n = (rows + per - 1) / per;
           p.copy(src + (size_t)r0 * rb, second, n, per * rb, (rows - (n - 1) * per) * rb);
         }
@@ -1054,12 +1097,13 @@ __global__ void __launch_bounds__(kStepThreads + 32, 1) decode_step(const __grid
       const uint32_t tag = tag0 + (uint32_t)l * 8u;
       const bool lm = l == L;
       const int K = stage == kOut ? Q : stage == kDown ? F : H;
-      const Share r{sh.share[lm ? kVocab : stage][0], sh.share[lm ? kVocab : stage][1]};
+      const Plan r = sh.plan[lm ? kVocab : stage];
+      c.split(r);
       // ---- inputs
       bool skip = false;
       if (stage == kQkv || stage == (E ? kRouter : kGateUp)) {
         // whoever has rows of this stage, or of the one that adds to the hidden state, reads it
-        skip = !r.n && (lm ? sm != 0 : !sh.share[kOut][1] && (stage == kQkv || !sh.share[kGateUp][1]));
+        skip = !r.n && (lm ? sm != 0 : !sh.plan[kOut].n && (stage == kQkv || !sh.plan[kGateUp].n));
         if (!skip) {
           const uint64_t w = lm ? s.norm_w : (stage == kQkv ? s.ln1 : s.ln2) + (size_t)l * H * 2;
           c.template hidden<kFmt>(work + wk.h + (stage == kQkv ? H / 2 : 0), stage == kQkv ? tag - 8u + 5u : tag + 4u, l == 0 && stage == kQkv ? row : nullptr, w, lm);
@@ -1073,16 +1117,13 @@ __global__ void __launch_bounds__(kStepThreads + 32, 1) decode_step(const __grid
                     [&](int i, uint32_t a, uint32_t b) { c.template set_input<kFmt>(i, a, b, false); });
           consumers_sync();
         }
-      } else if (r.n || sh.share[kDown][1]) {      // kGateUp behind a router: its inputs are there, the experts are not
+      } else if (r.n || sh.plan[kDown].n) {      // kGateUp behind a router: its inputs are there, the experts are not
         c.route(work + wk.router, tag + 7u);
       }
       // ---- rows, as many at a time as their partial sums have room for
-      if (lm && kFmt != 0) c.template split<0>(K, r.n);
-      else c.template split<kFmt>(K, r.n * (E && stage == kDown ? slots : 1));
-      const int per = chunk_rows(2 * H), most = lm ? kPartFloats / c.kw / per * per : r.n;
 #pragma unroll 1
-      for (int r0 = 0; r0 < r.n && !skip; r0 += most) {
-        const int n = min(most, r.n - r0);
+      for (int r0 = 0; r0 < r.n && !skip; r0 += r.most) {
+        const int n = min(r.most, r.n - r0);
         if (lm && kFmt != 0) {
           c.template rows<0, false>(K, n, c.x(), 0);
         } else {
@@ -1090,7 +1131,7 @@ __global__ void __launch_bounds__(kStepThreads + 32, 1) decode_step(const __grid
           const int segs = E && stage == kDown ? slots : 1;
 #pragma unroll 1
           for (int e = 0, done = 0; E && stage == kGateUp ? done < n : e < segs; ++e) {
-            const int take = E && stage == kGateUp ? min(n - done, 2 * F - (r.r0 + done) % (2 * F)) : n;
+            const int take = E && stage == kGateUp ? min(n - done, done ? 2 * F : sh.head) : n;
             c.template rows<kFmt, kExperts>(K, take, c.x() + (segs > 1 ? (size_t)e * F * 2 : 0), segs > 1 ? e * n : done);
             done += take;
           }
@@ -1284,6 +1325,7 @@ extern "C" cudaError_t vdc_step_launch(const vdc_step* s, vdc_status* status, ui
   cfg.dynamicSmemBytes = vdc::kStepSmem;
   auto f = s->n_experts ? vdc::decode_step<0, true> : s->wfmt == 0 ? vdc::decode_step<0, false>
            : s->wfmt == 1 ? vdc::decode_step<1, false> : vdc::decode_step<2, false>;
-  const vdc::StepArgs args{*s, vdc::step_layout(*s), vdc::step_work(*s)};
+  vdc::StepArgs args{*s, vdc::step_layout(*s), vdc::step_work(*s), {}};
+  for (int i = 0; i < vdc::kStages; ++i) args.deal[i] = vdc::deal_of(*s, i);
   return cudaLaunchKernelEx(&cfg, f, args, status, timeout_ns);
 }
