@@ -49,12 +49,12 @@ struct StepShared {
   uint64_t full[kItems], empty[kItems], routed;
   int start[kItems];                                 // offset of an item in the ring
   volatile int fail;
-  float red[kStepWarps];
+  alignas(16) float red[kStepWarps];
   float best[kStepWarps];
   int best_row[kStepWarps];
   alignas(16) Plan plan[kStages];
   int slot0, head;                                   // experts: the slot of this SM's first gate/up row, its rows there are
-  int pair0, pair1;                                  // pairs of a head's dims that this SM merges
+  int four0, four1;                                  // fours of a head's dims that this SM merges
 };
 // Behind the ring: what the consumers share.
 struct StepLayout {
@@ -156,8 +156,12 @@ __device__ __forceinline__ Two get2(const uint64_t* p) {
 // dot products of a chunk's rows
 // ------------------------------------------------------------------------- //
 __device__ __forceinline__ void mma_f16(float (&d)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0, uint32_t b1) {
-  asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
-               : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3]) : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
+  asm("mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
+      : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3]) : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
+}
+__device__ __forceinline__ void mma_bf16(float (&d)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0, uint32_t b1) {
+  asm("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
+      : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3]) : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
 }
 __device__ __forceinline__ uint32_t e4m3_pair(uint32_t pair) {
   uint32_t d;
@@ -170,7 +174,8 @@ __host__ __device__ constexpr int unit_of(int fmt) { return fmt == 0 ? 256 : fmt
 // Weights as the tensor cores take them: four (bf16), four (e4m3) or eight (NVFP4) of a lane's 16 bytes, which is two, one or
 // one word of them, as bf16 or f16 pairs.  An NVFP4 weight times its block's scale is exact in f16.
 template <int kFmt>
-__device__ __forceinline__ void expand(uint32_t (&o)[kFmt == 2 ? 4 : 2], const uint32_t (&c)[4], int part, uint32_t scales) {
+__device__ __forceinline__ void expand(uint32_t (&o)[kFmt == 2 ? 4 : 2], const uint4& v, int part, uint32_t scales) {
+  const uint32_t c[4] = {v.x, v.y, v.z, v.w};
   if (kFmt == 0) {
     o[0] = c[2 * part];
     o[1] = c[2 * part + 1];
@@ -189,18 +194,27 @@ __device__ __forceinline__ void expand(uint32_t (&o)[kFmt == 2 ? 4 : 2], const u
 
 // Models with experts: packed fp32 FMAs of the widened pairs, sums rounded to nearest at every product.  The router's softmax
 // is steep enough that the last bits of what stands in front of it can be seen behind it.
-template <int kPairs>
-__device__ __forceinline__ void dot_fma(float2 (&d)[2 * kPairs], const uint8_t* w, const int (&row)[4], const uint8_t* x, int u, int lane) {
+template <int kPairs, int kSteps>
+__device__ __forceinline__ void dot_fma(float2 (&d)[2 * kPairs], const uint8_t* w, const int (&row)[4], const uint8_t* x, int u, int kw, int lane) {
   auto pair = [](uint32_t v) { return make_float2(bf_lo(v), bf_hi(v)); };
-  const uint4 xv = lds128(x + u * 512 + lane * 16);
-  const float2 xf[4] = {pair(xv.x), pair(xv.y), pair(xv.z), pair(xv.w)};
+  uint4 xs[kSteps], c[kSteps][2 * kPairs];
 #pragma unroll
-  for (int i = 0; i < 2 * kPairs; ++i) {
-    const uint4 v = lds128(w + row[i] + u * 512 + lane * 16);
-    d[i] = __ffma2_rn(pair(v.x), xf[0], d[i]);
-    d[i] = __ffma2_rn(pair(v.y), xf[1], d[i]);
-    d[i] = __ffma2_rn(pair(v.z), xf[2], d[i]);
-    d[i] = __ffma2_rn(pair(v.w), xf[3], d[i]);
+  for (int j = 0; j < kSteps; ++j) {
+    const int at = (u + j * kw) * 512 + lane * 16;
+    xs[j] = lds128(x + at);
+#pragma unroll
+    for (int i = 0; i < 2 * kPairs; ++i) c[j][i] = lds128(w + row[i] + at);
+  }
+#pragma unroll
+  for (int j = 0; j < kSteps; ++j) {
+    const float2 xf[4] = {pair(xs[j].x), pair(xs[j].y), pair(xs[j].z), pair(xs[j].w)};
+#pragma unroll
+    for (int i = 0; i < 2 * kPairs; ++i) {
+      d[i] = __ffma2_rn(pair(c[j][i].x), xf[0], d[i]);
+      d[i] = __ffma2_rn(pair(c[j][i].y), xf[1], d[i]);
+      d[i] = __ffma2_rn(pair(c[j][i].z), xf[2], d[i]);
+      d[i] = __ffma2_rn(pair(c[j][i].w), xf[3], d[i]);
+    }
   }
 }
 
@@ -210,57 +224,71 @@ __device__ __forceinline__ void add2(float& a, float& b, float x, float y) {
   b = v.y;
 }
 
-// One step of a warp: 16 bytes per lane of kPairs pairs of rows times the same inputs, as products of 16 x 16 by 16 x 8 tiles.
-// Row g of a tile is what the four lanes 4g .. 4g + 3 hold of the pair's first row (8 + g: of its second), column g what they
-// hold of the inputs: the tile's element (g, g) is the sum of the four lanes' products, the other elements mean nothing.  A
-// product of tiles is one instruction where FMAs of four rows are 12 (32 KB of bf16 took 0.8 us with those, HBM 0.73).
+// kSteps steps of a warp (u, u + kw, ...): 16 bytes per lane of kPairs pairs of rows times the same inputs, as products of 16 x 16
+// by 16 x 8 tiles.  Row g of a tile is what the four lanes 4g .. 4g + 3 hold of the pair's first row (8 + g: of its second), column
+// g what they hold of the inputs: the tile's element (g, g) is the sum of the four lanes' products, the other elements mean nothing.
+// A product of tiles is one instruction where FMAs of four rows are 12 (32 KB of bf16 took 0.8 us with those, HBM 0.73).
+// All loads of the steps are issued before the first product waits for one: see kStepsOf.
 // The tensor cores cut off what an fp32 sum cannot hold.  So bf16 and e4m3 rows have only two products of tiles (8 of a lane's
 // inputs) added up by them, from zero; those sums meet in rounded additions.  Of 32768 sums of 8192 products around two large
 // ones that cancel, 2.0 % miss their bf16 rounding (FMAs 2.1 %, all products in one sum of the tensor cores 7.2 %).  Four
-// 8B-shaped layers e4m3 325 -> 329 us, eight bf16 the same.  NVFP4 rows keep the one sum: the megakernel's program adds 16 of
-// their products up in f16.
-template <int kFmt, int kPairs>
-__device__ __forceinline__ void dot_unit(float (&d)[kPairs][4], const uint8_t* w, const int (&row)[4], bool single, const uint8_t* x,
-                                         int u, int lane, int K) {
+// 8B-shaped layers e4m3 325 -> 329 us, eight bf16 the same.  NVFP4 rows keep long sums, two of them in turn: the megakernel's
+// program adds 16 of their products up in f16.
+template <int kFmt, int kPairs, int kSteps>
+__device__ __forceinline__ void dot_steps(float (&d)[kFmt == 2 ? 2 : 1][kPairs][4], const uint8_t* w, const int (&row)[4], bool single, const uint8_t* x,
+                                          int u, int kw, int lane, int K) {
   constexpr int kParts = kFmt == 0 ? 2 : 4, kWords = kFmt == 2 ? 4 : 2;       // of a lane's 16 bytes; expanded words of one
-  uint32_t c[2 * kPairs][4], sc[2 * kPairs];
+  constexpr int kXs = kParts * kWords / 4;                                    // 16-byte pieces of a lane's inputs
+  uint4 xs[kSteps][kXs], c[kSteps][2 * kPairs];
+  uint32_t sc[kSteps][2 * kPairs];
 #pragma unroll
-  for (int i = 0; i < 2 * kPairs; ++i) {
-    const uint8_t* r = w + row[i];
-    const bool none = (i & 1) && single;
-    const uint4 v = none ? make_uint4(0u, 0u, 0u, 0u) : lds128(r + u * 512 + lane * 16);
-    c[i][0] = v.x; c[i][1] = v.y; c[i][2] = v.z; c[i][3] = v.w;
-    sc[i] = kFmt == 2 && !none ? e4m3_pair(*reinterpret_cast<const uint16_t*>(r + (K >> 1) + u * 64 + lane * 2)) : 0u;
-  }
-  const uint8_t* xp = x + u * unit_of(kFmt) * 2 + lane * 16;
-  uint32_t xv[4];
-  float t[kPairs][4] = {};
+  for (int j = 0; j < kSteps; ++j) {
+    const int v = u + j * kw;
 #pragma unroll
-  for (int part = 0; part < kParts; ++part) {
-    const int at = part * kWords;                                               // first expanded word; four of them are 16 bytes of x
-    if ((at & 3) == 0) {
-      const uint4 v = lds128(xp + (at >> 2) * 512);
-      xv[0] = v.x; xv[1] = v.y; xv[2] = v.z; xv[3] = v.w;
+    for (int i = 0; i < 2 * kPairs; ++i) {
+      const uint8_t* r = w + row[i];
+      const bool none = (i & 1) && single;
+      c[j][i] = none ? make_uint4(0u, 0u, 0u, 0u) : lds128(r + v * 512 + lane * 16);
+      sc[j][i] = kFmt == 2 && !none ? *reinterpret_cast<const uint16_t*>(r + (K >> 1) + v * 64 + lane * 2) : 0u;
     }
 #pragma unroll
-    for (int p = 0; p < kPairs; ++p) {
-      uint32_t a[kWords], b[kWords];
-      expand<kFmt>(a, c[2 * p], part, sc[2 * p]);
-      expand<kFmt>(b, c[2 * p + 1], part, sc[2 * p + 1]);
-      float(&sum)[4] = kFmt == 2 ? d[p] : t[p];
+    for (int i = 0; i < kXs; ++i) xs[j][i] = lds128(x + v * unit_of(kFmt) * 2 + lane * 16 + i * 512);
+  }
 #pragma unroll
-      for (int j = 0; j < kWords; j += 2) {
-        if (kFmt == 0) mma_16816(sum, a[j], b[j], a[j + 1], b[j + 1], xv[(at & 3) + j], xv[(at & 3) + j + 1]);
-        else mma_f16(sum, a[j], b[j], a[j + 1], b[j + 1], xv[(at & 3) + j], xv[(at & 3) + j + 1]);
-      }
-      if (kFmt != 2 && (part & 1) != 0) {
-        add2(d[p][0], d[p][1], t[p][0], t[p][1]);
-        add2(d[p][2], d[p][3], t[p][2], t[p][3]);
-        t[p][0] = t[p][1] = t[p][2] = t[p][3] = 0.f;
+  for (int j = 0; j < kSteps; ++j) {
+    float t[kPairs][4];
+    if (kFmt == 2) {
+#pragma unroll
+      for (int i = 0; i < 2 * kPairs; ++i) sc[j][i] = e4m3_pair(sc[j][i]);
+    }
+#pragma unroll
+    for (int part = 0; part < kParts; ++part) {
+      const int at = part * kWords;                                             // first expanded word
+      const uint4 xq = xs[j][at >> 2];
+      const uint32_t xv[4] = {xq.x, xq.y, xq.z, xq.w};
+#pragma unroll
+      for (int p = 0; p < kPairs; ++p) {
+        uint32_t a[kWords], b[kWords];
+        expand<kFmt>(a, c[j][2 * p], part, sc[j][2 * p]);
+        expand<kFmt>(b, c[j][2 * p + 1], part, sc[j][2 * p + 1]);
+        if (kFmt != 2 && (part & 1) == 0) t[p][0] = t[p][1] = t[p][2] = t[p][3] = 0.f;
+        float(&sum)[4] = kFmt == 2 ? d[kFmt == 2 ? part & 1 : 0][p] : t[p];
+#pragma unroll
+        for (int k = 0; k < kWords; k += 2) {
+          if (kFmt == 0) mma_bf16(sum, a[k], b[k], a[k + 1], b[k + 1], xv[(at & 3) + k], xv[(at & 3) + k + 1]);
+          else mma_f16(sum, a[k], b[k], a[k + 1], b[k + 1], xv[(at & 3) + k], xv[(at & 3) + k + 1]);
+        }
+        if (kFmt != 2 && (part & 1) != 0) {
+          add2(d[0][p][0], d[0][p][1], t[p][0], t[p][1]);
+          add2(d[0][p][2], d[0][p][3], t[p][2], t[p][3]);
+        }
       }
     }
   }
 }
+// Steps of a warp whose loads are on their way together.  With one (and the products in the order of the source) a warp took 290
+// cycles for a step of four bf16 rows, a chain of a load, two products and an addition.
+__host__ __device__ constexpr int steps_of(int fmt, int pairs) { return fmt == 0 ? 4 : 2; }
 
 // Units of q rows; the first SMs' shares are never empty while there are any.
 __host__ __device__ inline Share share_of(int rows, int q, int sm, int sms) {
@@ -396,6 +424,11 @@ __device__ __forceinline__ Pages pages_of(const vdc_step& s, int pos, int sm) {
 // ------------------------------------------------------------------------- //
 __device__ __forceinline__ void consumers_sync() { asm volatile("bar.sync 1, %0;" ::"n"(kStepThreads) : "memory"); }
 
+template <int n>
+struct Steps {
+  static constexpr int value = n;
+};
+
 struct Consumer {
   const StepArgs& args;
   const vdc_step& s;
@@ -434,32 +467,42 @@ struct Consumer {
     }
     return true;
   }
-  // n 2-byte values (a multiple of 4) of an entry buffer: f(i, values 4i .. 4i + 3 as two words) for this thread's i.  All that
-  // a thread still misses is looked for at the same time: one after another, each look is a round trip of its own.
+  // Fours j0 .. j0 + kBatch - 1 of this thread (its j-th is number tid + j * kStepThreads of n) from an entry buffer.  All that a
+  // thread still misses is looked for at the same time: one after another, each look is a round trip of its own.
+  template <int kBatch>
+  __device__ __forceinline__ bool take(const uint64_t* buf, int n, int j0, uint32_t tag, uint2* out) const {
+    const int i0 = tid + j0 * kStepThreads;
+    Two v[kBatch];
+#pragma unroll
+    for (int j = 0; j < kBatch; ++j)
+      if (i0 + j * kStepThreads < n) v[j] = get2(buf + 2 * (i0 + j * kStepThreads));
+    uint64_t t0 = 0;
+#pragma unroll 1
+    for (uint32_t it = 1;; ++it) {
+      bool all = true;
+#pragma unroll
+      for (int j = 0; j < kBatch; ++j)
+        if (i0 + j * kStepThreads < n) all = all && v[j].are(tag);
+      if (all) break;
+      if ((it & 63u) == 0 && !again(buf + 2 * i0, it, t0)) return false;
+#pragma unroll
+      for (int j = 0; j < kBatch; ++j)
+        if (i0 + j * kStepThreads < n && !v[j].are(tag)) v[j] = get2(buf + 2 * (i0 + j * kStepThreads));
+    }
+#pragma unroll
+    for (int j = 0; j < kBatch; ++j) out[j] = make_uint2((uint32_t)v[j].a, (uint32_t)v[j].b);
+    return true;
+  }
+  // n 2-byte values (a multiple of 4) of an entry buffer: f(i, values 4i .. 4i + 3 as two words) for this thread's i.
   template <int kBatch, class F>
   __device__ __forceinline__ void collect(const uint64_t* buf, int n, uint32_t tag, F f) const {
 #pragma unroll 1
-    for (int i0 = tid; i0 < n / 4; i0 += kBatch * kStepThreads) {
-      Two v[kBatch];
+    for (int j0 = 0; tid + j0 * kStepThreads < n / 4; j0 += kBatch) {
+      uint2 v[kBatch];
+      if (!take<kBatch>(buf, n / 4, j0, tag, v)) return;
 #pragma unroll
       for (int j = 0; j < kBatch; ++j)
-        if (i0 + j * kStepThreads < n / 4) v[j] = get2(buf + 2 * (i0 + j * kStepThreads));
-      uint64_t t0 = 0;
-#pragma unroll 1
-      for (uint32_t it = 1;; ++it) {
-        bool all = true;
-#pragma unroll
-        for (int j = 0; j < kBatch; ++j)
-          if (i0 + j * kStepThreads < n / 4) all = all && v[j].are(tag);
-        if (all) break;
-        if ((it & 63u) == 0 && !again(buf + 2 * i0, it, t0)) return;
-#pragma unroll
-        for (int j = 0; j < kBatch; ++j)
-          if (i0 + j * kStepThreads < n / 4 && !v[j].are(tag)) v[j] = get2(buf + 2 * (i0 + j * kStepThreads));
-      }
-#pragma unroll
-      for (int j = 0; j < kBatch; ++j)
-        if (i0 + j * kStepThreads < n / 4) f(i0 + j * kStepThreads, (uint32_t)v[j].a, (uint32_t)v[j].b);
+        if (tid + (j0 + j) * kStepThreads < n / 4) f(tid + (j0 + j) * kStepThreads, v[j].x, v[j].y);
     }
   }
   // Inputs 4i .. 4i + 3 (two bf16 pairs) as the dot products take them: bf16 in order; f16 for quantised rows, a lane's 16-byte
@@ -481,45 +524,61 @@ struct Consumer {
   template <int kFmt>
   __device__ __forceinline__ void hidden(const uint64_t* buf, uint32_t tag, const uint8_t* row, uint64_t w, bool plain) const {
     const int H = s.hidden;
-    constexpr int kMost = 8;                                      // hidden <= 8192
-    uint2 wv[kMost];
+    constexpr int kMost = 8, kHalf = kMost / 2;                   // hidden <= 8192; its first half stays in registers
+    uint2 wv[kMost], v[kHalf];
 #pragma unroll
     for (int j = 0; j < kMost; ++j) {
       const int i = tid + j * kStepThreads;
       if (i < H / 4) wv[j] = __ldg(reinterpret_cast<const uint2*>(w) + i);
     }
     float ssq = 0.f;
-    auto keep = [&](int i, uint32_t a, uint32_t b) {
-      *reinterpret_cast<uint2*>(hs() + 2 * i) = make_uint2(a, b);
-      ssq = fmaf(bf_lo(a), bf_lo(a), fmaf(bf_hi(a), bf_hi(a), fmaf(bf_lo(b), bf_lo(b), fmaf(bf_hi(b), bf_hi(b), ssq))));
-    };
-    if (row != nullptr) {
 #pragma unroll 1
-      for (int i = tid; i < H / 4; i += kStepThreads) {
-        const uint2 v = __ldg(reinterpret_cast<const uint2*>(row) + i);
-        keep(i, v.x, v.y);
+    for (int j0 = kHalf * (H > kHalf * 4 * kStepThreads); j0 >= 0; j0 -= kHalf) {
+      if (row != nullptr) {
+#pragma unroll
+        for (int j = 0; j < kHalf; ++j) {
+          const int i = tid + (j0 + j) * kStepThreads;
+          if (i < H / 4) v[j] = __ldg(reinterpret_cast<const uint2*>(row) + i);
+        }
+      } else if (!take<kHalf>(buf, H / 4, j0, tag, v)) {
+        break;
       }
-    } else {
-      collect<4>(buf, H, tag, keep);
+#pragma unroll
+      for (int j = 0; j < kHalf; ++j) {
+        const int i = tid + (j0 + j) * kStepThreads;
+        if (i < H / 4) {
+          const uint32_t a = v[j].x, b = v[j].y;
+          *reinterpret_cast<uint2*>(hs() + 2 * i) = v[j];
+          ssq = fmaf(bf_lo(a), bf_lo(a), fmaf(bf_hi(a), bf_hi(a), fmaf(bf_lo(b), bf_lo(b), fmaf(bf_hi(b), bf_hi(b), ssq))));
+        }
+      }
     }
     ssq = warp_sum(ssq);
     if (lane == 0) sh.red[warp] = ssq;
     consumers_sync();
     float tot = 0.f;
 #pragma unroll
-    for (int k = 0; k < kStepWarps; ++k) tot += sh.red[k];
+    for (int k = 0; k < kStepWarps; k += 4) {
+      const float4 r = *reinterpret_cast<const float4*>(sh.red + k);
+      tot += r.x; tot += r.y; tot += r.z; tot += r.w;
+    }
     const float rstd = rsqrtf(tot / (float)H + s.eps);
 #pragma unroll
     for (int j = 0; j < kMost; ++j) {
       const int i = tid + j * kStepThreads;
       if (i < H / 4) {
-        const uint2 v = *reinterpret_cast<const uint2*>(hs() + 2 * i);
-        const uint32_t a = pack_bf16x2(bf16_round(bf_lo(v.x) * rstd) * bf_lo(wv[j].x), bf16_round(bf_hi(v.x) * rstd) * bf_hi(wv[j].x));
-        const uint32_t b = pack_bf16x2(bf16_round(bf_lo(v.y) * rstd) * bf_lo(wv[j].y), bf16_round(bf_hi(v.y) * rstd) * bf_hi(wv[j].y));
-        set_input<kFmt>(i, a, b, plain);
+        const uint2 h = j < kHalf ? v[j < kHalf ? j : 0] : *reinterpret_cast<const uint2*>(hs() + 2 * i);
+        set_input<kFmt>(i, scaled(h.x, rstd, wv[j].x), scaled(h.y, rstd, wv[j].y), plain);
       }
     }
     consumers_sync();
+  }
+  // bf16(bf16(x * rstd) * w) of a pair: the product of two bf16 numbers is exact in fp32, so one rounding in the packed product
+  // is the same.
+  static __device__ __forceinline__ uint32_t scaled(uint32_t x, float rstd, uint32_t w) {
+    const __nv_bfloat162 n = __floats2bfloat162_rn(bf_lo(x) * rstd, bf_hi(x) * rstd);
+    const __nv_bfloat162 p = __hmul2(n, *reinterpret_cast<const __nv_bfloat162*>(&w));
+    return *reinterpret_cast<const uint32_t*>(&p);
   }
 
   __device__ __forceinline__ void split(const Plan& p) {
@@ -534,6 +593,15 @@ struct Consumer {
     ld = p.ld;
     per = p.per;
     units = p.units;
+  }
+  // This warp's steps along the inputs, kSteps at a time while there are as many.
+  template <int kSteps, class F>
+  __device__ __forceinline__ void walk(F f) const {
+    int u = kg;
+#pragma unroll 1
+    for (; u + (kSteps - 1) * kw < units; u += kSteps * kw) f(Steps<kSteps>{}, u);
+#pragma unroll 1
+    for (; u < units; u += kw) f(Steps<1>{}, u);
   }
   // n rows from the ring times the inputs xp: every warp's share of row r to part[kg][row0 + r], rows side by side for the
   // threads that add the shares up.
@@ -555,31 +623,32 @@ struct Consumer {
         float a, b, c = 0.f, e = 0.f;          // the lane's share of the four rows
         // of a tile the lanes that hold its diagonal
         const bool diag = (lane >> 3) == (lane & 3), odd = lane & 4;
-        auto share = [&](const float (&d)[4], float& first, float& second) {
-          first = diag ? (odd ? d[1] : d[0]) : 0.f;
-          second = diag ? (odd ? d[3] : d[2]) : 0.f;
+        auto share = [&](auto& d, int p, float& first, float& second) {
+          first = diag ? (odd ? d[0][p][1] : d[0][p][0]) : 0.f;
+          second = diag ? (odd ? d[0][p][3] : d[0][p][2]) : 0.f;
+          if (kFmt == 2) {
+            constexpr int k = kFmt == 2 ? 1 : 0;
+            first += diag ? (odd ? d[k][p][1] : d[k][p][0]) : 0.f;
+            second += diag ? (odd ? d[k][p][3] : d[k][p][2]) : 0.f;
+          }
         };
         if (kFma && r + 2 * rw < nr) {
           float2 d[4] = {};
-#pragma unroll 2
-          for (int u = kg; u < units; u += kw) dot_fma<2>(d, w, off, xp, u, lane);
+          walk<2>([&](auto steps, int u) { dot_fma<2, decltype(steps)::value>(d, w, off, xp, u, kw, lane); });
           a = d[0].x + d[0].y; b = d[1].x + d[1].y; c = d[2].x + d[2].y; e = d[3].x + d[3].y;
         } else if (kFma) {
           float2 d[2] = {};
-#pragma unroll 2
-          for (int u = kg; u < units; u += kw) dot_fma<1>(d, w, off, xp, u, lane);
+          walk<2>([&](auto steps, int u) { dot_fma<1, decltype(steps)::value>(d, w, off, xp, u, kw, lane); });
           a = d[0].x + d[0].y; b = d[1].x + d[1].y;
         } else if (r + 2 * rw < nr) {
-          float d[2][4] = {};
-#pragma unroll 2
-          for (int u = kg; u < units; u += kw) dot_unit<kFmt, 2>(d, w, off, false, xp, u, lane, K);
-          share(d[0], a, b);
-          share(d[1], c, e);
+          float d[kFmt == 2 ? 2 : 1][2][4] = {};
+          walk<steps_of(kFmt, 2)>([&](auto steps, int u) { dot_steps<kFmt, 2, decltype(steps)::value>(d, w, off, false, xp, u, kw, lane, K); });
+          share(d, 0, a, b);
+          share(d, 1, c, e);
         } else {
-          float d[1][4] = {};
-#pragma unroll 2
-          for (int u = kg; u < units; u += kw) dot_unit<kFmt, 1>(d, w, off, r + rw >= nr, xp, u, lane, K);
-          share(d[0], a, b);
+          float d[kFmt == 2 ? 2 : 1][1][4] = {};
+          walk<steps_of(kFmt, 1)>([&](auto steps, int u) { dot_steps<kFmt, 1, decltype(steps)::value>(d, w, off, r + rw >= nr, xp, u, kw, lane, K); });
+          share(d, 0, a, b);
         }
         // four sums over the lanes at once: lanes 8i .. 8i + 7 end up with row i
         const bool up = lane & 16, right = lane & 8;
@@ -814,43 +883,66 @@ struct Consumer {
       }
     }
     if (pg.live == 1) return;
-    // the head's pairs of dims are shared by its units: a lane takes every 32nd split.  The first one by itself: a loop over all
-    // of them lets the lanes drift apart while they poll (four 8B-shaped e4m3 layers 330 -> 368 us).
-    const int pairs = G * (D / 2), lo = sh.pair0, hi = sh.pair1;
+    // Four of the head's dims at a time are shared by its units: a lane per split (of 8, 16 or 32 lanes), so that an SM's share is
+    // one pass of the warps, as a rule.  Beyond 32 splits a lane takes every 32nd.  The first one by itself: a loop over all of
+    // them lets the lanes drift apart while they poll (four 8B-shaped e4m3 layers 330 -> 368 us).
+    const int fours = G * (D / 4), lo = sh.four0, hi = sh.four1;
+    const int lg = pg.live <= 8 ? 3 : pg.live <= 16 ? 4 : 5, lanes = 1 << lg, mine = lane & (lanes - 1), step = 32 >> lg;
 #pragma unroll 1
-    for (int i = lo + warp; i < hi; i += kStepWarps) {
-      float mk = -INFINITY, lk = 0.f, n0 = 0.f, n1 = 0.f;
+    for (int i0 = lo + warp * step; i0 < hi; i0 += kStepWarps * step) {
+      const int i = i0 + (lane >> lg);
+      float mk = -INFINITY, lk = 0.f;
+      float4 n = make_float4(0.f, 0.f, 0.f, 0.f);
       bool ok = true;
-      auto take = [&](int sp, float& n0, float& n1, float& mk, float& lk) {
+      auto take = [&](int sp, float4& n, float& mk, float& lk) {
         const size_t u = (size_t)pg.h * s.n_splits + sp;
-        const uint64_t *rp = rec + (u * pairs + i) * 2, *mp = ml + (u * G + i / (D / 2)) * 2;
-        Two r = get2(rp), z = get2(mp);
-        ok = poll2(rp, tag_rec, r) && poll2(mp, tag_rec, z);
-        n0 = __uint_as_float((uint32_t)r.a);
-        n1 = __uint_as_float((uint32_t)r.b);
+        const uint64_t *rp = rec + (u * fours + i) * 4, *mp = ml + (u * G + i / (D / 4)) * 2;
+        Two a = get2(rp), b = get2(rp + 2), z = get2(mp);
+        uint64_t t0 = 0;
+#pragma unroll 1
+        for (uint32_t it = 1; !(a.are(tag_rec) && b.are(tag_rec) && z.are(tag_rec)); ++it) {
+          if ((it & 63u) == 0 && !again(rp, it, t0)) {
+            ok = false;
+            return;
+          }
+          a = get2(rp);
+          b = get2(rp + 2);
+          z = get2(mp);
+        }
+        n = make_float4(__uint_as_float((uint32_t)a.a), __uint_as_float((uint32_t)a.b), __uint_as_float((uint32_t)b.a), __uint_as_float((uint32_t)b.b));
         mk = __uint_as_float((uint32_t)z.a);
         lk = __uint_as_float((uint32_t)z.b);
       };
-      if (lane < pg.live) take(lane, n0, n1, mk, lk);
+      if (i < hi && mine < pg.live) take(mine, n, mk, lk);
 #pragma unroll 1
-      for (int sp = lane + 32; sp - lane < pg.live; sp += 32) {
+      for (int sp = mine + 32; sp - mine < pg.live; sp += 32) {
         if (sp >= pg.live || !ok) continue;
-        float a0, a1, m1, l1;
-        take(sp, a0, a1, m1, l1);
+        float4 n1;
+        float m1, l1;
+        take(sp, n1, m1, l1);
+        if (!ok) continue;
         const float m2 = fmaxf(mk, m1), w0 = mk == -INFINITY ? 0.f : exp2f(mk - m2), w1 = m1 == -INFINITY ? 0.f : exp2f(m1 - m2);
-        n0 = fmaf(w0, n0, w1 * a0);
-        n1 = fmaf(w0, n1, w1 * a1);
+        n = make_float4(fmaf(w0, n.x, w1 * n1.x), fmaf(w0, n.y, w1 * n1.y), fmaf(w0, n.z, w1 * n1.z), fmaf(w0, n.w, w1 * n1.w));
         lk = fmaf(w0, lk, w1 * l1);
         mk = m2;
       }
       if (!__all_sync(0xffffffffu, ok)) break;
       float mm = mk;
-#pragma unroll
-      for (int z = 16; z > 0; z >>= 1) mm = fmaxf(mm, __shfl_xor_sync(0xffffffffu, mm, z));
+#pragma unroll 1
+      for (int z = lanes >> 1; z > 0; z >>= 1) mm = fmaxf(mm, __shfl_xor_sync(0xffffffffu, mm, z));
       const float wt = mk == -INFINITY ? 0.f : exp2f(mk - mm);
-      const float den = warp_sum(wt * lk), a = warp_sum(wt * n0), b = warp_sum(wt * n1);
+      n = make_float4(wt * n.x, wt * n.y, wt * n.z, wt * n.w);
+      float den = wt * lk;
+#pragma unroll 1
+      for (int z = lanes >> 1; z > 0; z >>= 1) {
+        n.x += __shfl_xor_sync(0xffffffffu, n.x, z);
+        n.y += __shfl_xor_sync(0xffffffffu, n.y, z);
+        n.z += __shfl_xor_sync(0xffffffffu, n.z, z);
+        n.w += __shfl_xor_sync(0xffffffffu, n.w, z);
+        den += __shfl_xor_sync(0xffffffffu, den, z);
+      }
       const float inv = den > 0.f ? 1.f / den : 0.f;
-      if (lane == 0) put(out + (size_t)pg.h * pairs + i, pack_bf16x2(a * inv, b * inv), tag_out);
+      if (mine == 0 && i < hi) put2(out + ((size_t)pg.h * fours + i) * 2, pack_bf16x2(n.x * inv, n.y * inv), pack_bf16x2(n.z * inv, n.w * inv), tag_out);
     }
   }
 
@@ -977,8 +1069,8 @@ __global__ void __launch_bounds__(kStepThreads + 32, 1) decode_step(const __grid
   const Pages pg = pages_of(s, pos, sm);
   const int slots = E ? s.top_k : 1;
   if (tid == 0 && pg.count > 0) {      // read behind the attention's barriers
-    sh.pair0 = G * (D / 2) * pg.split / pg.live;
-    sh.pair1 = G * (D / 2) * (pg.split + 1) / pg.live;
+    sh.four0 = G * (D / 4) * pg.split / pg.live;
+    sh.four1 = G * (D / 4) * (pg.split + 1) / pg.live;
   }
   const int rbH = row_bytes(kFmt, H), rbQ = row_bytes(kFmt, Q), rbF = row_bytes(kFmt, F);
   int* ids = reinterpret_cast<int*>(base + lay.route + kMaxExperts * 4);
@@ -1056,14 +1148,6 @@ __global__ void __launch_bounds__(kStepThreads + 32, 1) decode_step(const __grid
     uint64_t* work = reinterpret_cast<uint64_t*>(s.work);
     const uint32_t tag0 = (launches * (uint32_t)(L + 1) + 1u) * 8u;
     Consumer c{args, s, lay, sh, wait, base, tid, warp, lane, sm};
-    auto scaled2 = [&](int row, uint64_t sc, size_t at) {
-      float2 v = c.sum2(row);
-      if (kFmt) {
-        const float2 k = __ldg(reinterpret_cast<const float2*>(reinterpret_cast<const float*>(sc) + at));
-        v.x *= k.x; v.y *= k.y;
-      }
-      return v;
-    };
     // a residual row pair: this SM's rows of a projection added to the hidden state it has in shared memory
     auto residual = [&](int pair, float y0, float y1, uint64_t* out, uint32_t tag) {
       const uint32_t h = c.hs()[pair];
@@ -1099,6 +1183,27 @@ __global__ void __launch_bounds__(kStepThreads + 32, 1) decode_step(const __grid
       const int K = stage == kOut ? Q : stage == kDown ? F : H;
       const Plan r = sh.plan[lm ? kVocab : stage];
       c.split(r);
+      // the scales of this thread's first rows: from HBM while the inputs are waited for
+      const float* scales = nullptr;
+      float4 sc = make_float4(1.f, 1.f, 1.f, 1.f);
+      if (kFmt != 0 && !lm) {
+        const uint64_t of = stage == kQkv ? s.s_qkv : stage == kOut ? s.s_o : stage == kGateUp ? s.s_gu : s.s_d;
+        scales = reinterpret_cast<const float*>(of) + (size_t)l * (stage == kQkv ? QKV : stage == kGateUp ? 2 * F : H) + r.r0;
+        if (stage == kGateUp && tid < r.n / 4) {
+          sc = __ldg(reinterpret_cast<const float4*>(scales) + tid);
+        } else if (stage != kGateUp && tid < r.n / 2) {
+          const float2 k = __ldg(reinterpret_cast<const float2*>(scales) + tid);
+          sc.x = k.x; sc.y = k.y;
+        }
+      }
+      auto scaled2 = [&](int i) {         // rows 2i, 2i + 1 of this SM
+        float2 v = c.sum2(2 * i);
+        if (kFmt != 0) {
+          const float2 k = i == tid ? make_float2(sc.x, sc.y) : __ldg(reinterpret_cast<const float2*>(scales) + i);
+          v.x *= k.x; v.y *= k.y;
+        }
+        return v;
+      };
       // ---- inputs
       bool skip = false;
       if (stage == kQkv || stage == (E ? kRouter : kGateUp)) {
@@ -1138,7 +1243,6 @@ __global__ void __launch_bounds__(kStepThreads + 32, 1) decode_step(const __grid
         }
         consumers_sync();
         if (!c.failed()) {
-          const size_t row_at = (size_t)l * (stage == kQkv ? QKV : stage == kGateUp ? 2 * F : H) + r.r0;      // of the scales
           if (lm) {
 #pragma unroll 1
             for (int i = tid; i < n / 2; i += kStepThreads) {
@@ -1158,7 +1262,7 @@ __global__ void __launch_bounds__(kStepThreads + 32, 1) decode_step(const __grid
           } else if (stage == kQkv) {
 #pragma unroll 1
             for (int i = tid; i < n / 2; i += kStepThreads) {
-              const float2 y = scaled2(2 * i, s.s_qkv, row_at + 2 * i);
+              const float2 y = scaled2(i);
               put(work + wk.qkv + (r.r0 >> 1) + i, pack_bf16x2(y.x, y.y), tag + 1u);
             }
           } else if (stage == kRouter) {
@@ -1168,7 +1272,7 @@ __global__ void __launch_bounds__(kStepThreads + 32, 1) decode_step(const __grid
             for (int i = tid; i < n / 4; i += kStepThreads) {
               float4 y = c.sum4(4 * i);
               if (kFmt) {
-                const float4 k = __ldg(reinterpret_cast<const float4*>(reinterpret_cast<const float*>(s.s_gu) + row_at) + i);
+                const float4 k = i == tid ? sc : __ldg(reinterpret_cast<const float4*>(scales) + i);
                 y.x *= k.x; y.y *= k.y; y.z *= k.z; y.w *= k.w;
               }
               put(work + wk.act + (r.r0 >> 2) + i, pack_bf16x2(silu(y.x, y.y), silu(y.z, y.w)), tag + 6u);
@@ -1185,7 +1289,7 @@ __global__ void __launch_bounds__(kStepThreads + 32, 1) decode_step(const __grid
                   y.y = fmaf(weights[e], bf16_round(v.y), y.y);
                 }
               } else {
-                y = scaled2(2 * i, stage == kOut ? s.s_o : s.s_d, row_at + 2 * i);
+                y = scaled2(i);
               }
               residual((r.r0 >> 1) + i, y.x, y.y, work + wk.h + (stage == kDown ? H / 2 : 0), tag + (stage == kDown ? 5u : 4u));
             }
