@@ -58,7 +58,7 @@ struct StepShared {
 };
 // Behind the ring: what the consumers share.
 struct StepLayout {
-  int ring, x, h, part, raw, q, rows, p, gm, wl, route;
+  int ring, x, h, part, raw, q, rows, p, gm, wl, route, scales;
   int total;
 };
 __host__ __device__ inline StepLayout step_layout(const vdc_step& s) {
@@ -82,6 +82,7 @@ __host__ __device__ inline StepLayout step_layout(const vdc_step& s) {
   l.gm = take(kGroups * 4 * 8 * 4);
   l.wl = take(kGroups * 5 * 8 * 4);
   l.route = take(kMaxExperts * 4 + 2 * kMaxTopK * 4);
+  l.scales = take(s.wfmt ? kStepThreads * 16 : 0);
   l.ring = at;
   l.total = kStepSmem - 128;
   return l;
@@ -152,6 +153,13 @@ __device__ __forceinline__ Two get2(const uint64_t* p) {
   return v;
 }
 
+// A thread's own copies of 8 bytes to shared memory, waited for by the thread itself: loads that hold no registers while they are
+// on their way.
+__device__ __forceinline__ void copy8_async(void* to, uint64_t from) {
+  asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(smem_u32(to)), "l"(from) : "memory");
+}
+__device__ __forceinline__ void copies_wait() { asm volatile("cp.async.wait_all;" ::: "memory"); }
+
 // ------------------------------------------------------------------------- //
 // dot products of a chunk's rows
 // ------------------------------------------------------------------------- //
@@ -194,27 +202,18 @@ __device__ __forceinline__ void expand(uint32_t (&o)[kFmt == 2 ? 4 : 2], const u
 
 // Models with experts: packed fp32 FMAs of the widened pairs, sums rounded to nearest at every product.  The router's softmax
 // is steep enough that the last bits of what stands in front of it can be seen behind it.
-template <int kPairs, int kSteps>
-__device__ __forceinline__ void dot_fma(float2 (&d)[2 * kPairs], const uint8_t* w, const int (&row)[4], const uint8_t* x, int u, int kw, int lane) {
+template <int kPairs>
+__device__ __forceinline__ void dot_fma(float2 (&d)[2 * kPairs], const uint8_t* w, const int (&row)[4], const uint8_t* x, int u, int lane) {
   auto pair = [](uint32_t v) { return make_float2(bf_lo(v), bf_hi(v)); };
-  uint4 xs[kSteps], c[kSteps][2 * kPairs];
+  const uint4 xv = lds128(x + u * 512 + lane * 16);
+  const float2 xf[4] = {pair(xv.x), pair(xv.y), pair(xv.z), pair(xv.w)};
 #pragma unroll
-  for (int j = 0; j < kSteps; ++j) {
-    const int at = (u + j * kw) * 512 + lane * 16;
-    xs[j] = lds128(x + at);
-#pragma unroll
-    for (int i = 0; i < 2 * kPairs; ++i) c[j][i] = lds128(w + row[i] + at);
-  }
-#pragma unroll
-  for (int j = 0; j < kSteps; ++j) {
-    const float2 xf[4] = {pair(xs[j].x), pair(xs[j].y), pair(xs[j].z), pair(xs[j].w)};
-#pragma unroll
-    for (int i = 0; i < 2 * kPairs; ++i) {
-      d[i] = __ffma2_rn(pair(c[j][i].x), xf[0], d[i]);
-      d[i] = __ffma2_rn(pair(c[j][i].y), xf[1], d[i]);
-      d[i] = __ffma2_rn(pair(c[j][i].z), xf[2], d[i]);
-      d[i] = __ffma2_rn(pair(c[j][i].w), xf[3], d[i]);
-    }
+  for (int i = 0; i < 2 * kPairs; ++i) {
+    const uint4 v = lds128(w + row[i] + u * 512 + lane * 16);
+    d[i] = __ffma2_rn(pair(v.x), xf[0], d[i]);
+    d[i] = __ffma2_rn(pair(v.y), xf[1], d[i]);
+    d[i] = __ffma2_rn(pair(v.z), xf[2], d[i]);
+    d[i] = __ffma2_rn(pair(v.w), xf[3], d[i]);
   }
 }
 
@@ -508,16 +507,21 @@ struct Consumer {
   // Inputs 4i .. 4i + 3 (two bf16 pairs) as the dot products take them: bf16 in order; f16 for quantised rows, a lane's 16-byte
   // pieces of a step 512 bytes apart, so that neighbouring lanes read neighbouring pieces.
   template <int kFmt>
-  __device__ __forceinline__ void set_input(int i, uint32_t a, uint32_t b, bool plain) const {
-    if (kFmt == 0 || plain) {
-      *reinterpret_cast<uint2*>(x() + i * 8) = make_uint2(a, b);
-      return;
-    }
+  static __device__ __forceinline__ int input_at(int i, bool plain) {
+    if (kFmt == 0 || plain) return i * 8;
     constexpr int kLane = unit_of(kFmt) / 32;
     const int e = i * 4, u = e / unit_of(kFmt), in = e % unit_of(kFmt);
+    return u * unit_of(kFmt) * 2 + (in % kLane) / 8 * 512 + in / kLane * 16 + (i & 1) * 8;
+  }
+  template <int kFmt>
+  __device__ __forceinline__ void set_input(int i, uint32_t a, uint32_t b, bool plain) const {
+    uint2* to = reinterpret_cast<uint2*>(x() + input_at<kFmt>(i, plain));
+    if (kFmt == 0 || plain) {
+      *to = make_uint2(a, b);
+      return;
+    }
     const __half2 ha = __floats2half2_rn(bf_lo(a), bf_hi(a)), hb = __floats2half2_rn(bf_lo(b), bf_hi(b));
-    *reinterpret_cast<uint2*>(x() + u * unit_of(kFmt) * 2 + (in % kLane) / 8 * 512 + in / kLane * 16 + (i & 1) * 8) =
-        make_uint2(*reinterpret_cast<const uint32_t*>(&ha), *reinterpret_cast<const uint32_t*>(&hb));
+    *to = make_uint2(*reinterpret_cast<const uint32_t*>(&ha), *reinterpret_cast<const uint32_t*>(&hb));
   }
   // The hidden state (entries, or a row of the embedding table) into shared memory and, RMS-normalised with the weights w,
   // into the input vector.  Rounded like a bf16 tensor expression.
@@ -525,12 +529,11 @@ struct Consumer {
   __device__ __forceinline__ void hidden(const uint64_t* buf, uint32_t tag, const uint8_t* row, uint64_t w, bool plain) const {
     const int H = s.hidden;
     constexpr int kMost = 8, kHalf = kMost / 2;                   // hidden <= 8192; its first half stays in registers
-    uint2 wv[kMost], v[kHalf];
-#pragma unroll
-    for (int j = 0; j < kMost; ++j) {
-      const int i = tid + j * kStepThreads;
-      if (i < H / 4) wv[j] = __ldg(reinterpret_cast<const uint2*>(w) + i);
-    }
+    uint2 v[kHalf];
+    // The weights are on their way while the entries are waited for, to the places of the inputs that they make.  The last stage's
+    // inputs there have been read: its partial sums are complete.
+#pragma unroll 2
+    for (int i = tid; i < H / 4; i += kStepThreads) copy8_async(x() + input_at<kFmt>(i, plain), w + (size_t)i * 8);
     float ssq = 0.f;
 #pragma unroll 1
     for (int j0 = kHalf * (H > kHalf * 4 * kStepThreads); j0 >= 0; j0 -= kHalf) {
@@ -563,12 +566,15 @@ struct Consumer {
       tot += r.x; tot += r.y; tot += r.z; tot += r.w;
     }
     const float rstd = rsqrtf(tot / (float)H + s.eps);
+    copies_wait();
 #pragma unroll
     for (int j = 0; j < kMost; ++j) {
       const int i = tid + j * kStepThreads;
+      if (j == kHalf && H <= kHalf * 4 * kStepThreads) break;
       if (i < H / 4) {
         const uint2 h = j < kHalf ? v[j < kHalf ? j : 0] : *reinterpret_cast<const uint2*>(hs() + 2 * i);
-        set_input<kFmt>(i, scaled(h.x, rstd, wv[j].x), scaled(h.y, rstd, wv[j].y), plain);
+        const uint2 wv = *reinterpret_cast<const uint2*>(x() + input_at<kFmt>(i, plain));
+        set_input<kFmt>(i, scaled(h.x, rstd, wv.x), scaled(h.y, rstd, wv.y), plain);
       }
     }
     consumers_sync();
@@ -634,11 +640,13 @@ struct Consumer {
         };
         if (kFma && r + 2 * rw < nr) {
           float2 d[4] = {};
-          walk<2>([&](auto steps, int u) { dot_fma<2, decltype(steps)::value>(d, w, off, xp, u, kw, lane); });
+#pragma unroll 2
+          for (int u = kg; u < units; u += kw) dot_fma<2>(d, w, off, xp, u, lane);
           a = d[0].x + d[0].y; b = d[1].x + d[1].y; c = d[2].x + d[2].y; e = d[3].x + d[3].y;
         } else if (kFma) {
           float2 d[2] = {};
-          walk<2>([&](auto steps, int u) { dot_fma<1, decltype(steps)::value>(d, w, off, xp, u, kw, lane); });
+#pragma unroll 2
+          for (int u = kg; u < units; u += kw) dot_fma<1>(d, w, off, xp, u, lane);
           a = d[0].x + d[0].y; b = d[1].x + d[1].y;
         } else if (r + 2 * rw < nr) {
           float d[kFmt == 2 ? 2 : 1][2][4] = {};
@@ -1183,23 +1191,22 @@ __global__ void __launch_bounds__(kStepThreads + 32, 1) decode_step(const __grid
       const int K = stage == kOut ? Q : stage == kDown ? F : H;
       const Plan r = sh.plan[lm ? kVocab : stage];
       c.split(r);
-      // the scales of this thread's first rows: from HBM while the inputs are waited for
+      // the scales of this thread's first rows come from HBM while the inputs are waited for
       const float* scales = nullptr;
-      float4 sc = make_float4(1.f, 1.f, 1.f, 1.f);
+      const float2* mine = reinterpret_cast<const float2*>(base + lay.scales + tid * 16);
       if (kFmt != 0 && !lm) {
         const uint64_t of = stage == kQkv ? s.s_qkv : stage == kOut ? s.s_o : stage == kGateUp ? s.s_gu : s.s_d;
         scales = reinterpret_cast<const float*>(of) + (size_t)l * (stage == kQkv ? QKV : stage == kGateUp ? 2 * F : H) + r.r0;
-        if (stage == kGateUp && tid < r.n / 4) {
-          sc = __ldg(reinterpret_cast<const float4*>(scales) + tid);
-        } else if (stage != kGateUp && tid < r.n / 2) {
-          const float2 k = __ldg(reinterpret_cast<const float2*>(scales) + tid);
-          sc.x = k.x; sc.y = k.y;
+        const int each = stage == kGateUp ? 4 : 2;
+        if (tid < r.n / each) {
+          copy8_async(base + lay.scales + tid * 16, reinterpret_cast<uint64_t>(scales + tid * each));
+          if (each == 4) copy8_async(base + lay.scales + tid * 16 + 8, reinterpret_cast<uint64_t>(scales + tid * 4 + 2));
         }
       }
       auto scaled2 = [&](int i) {         // rows 2i, 2i + 1 of this SM
         float2 v = c.sum2(2 * i);
         if (kFmt != 0) {
-          const float2 k = i == tid ? make_float2(sc.x, sc.y) : __ldg(reinterpret_cast<const float2*>(scales) + i);
+          const float2 k = i == tid ? *mine : __ldg(reinterpret_cast<const float2*>(scales) + i);
           v.x *= k.x; v.y *= k.y;
         }
         return v;
@@ -1241,6 +1248,7 @@ __global__ void __launch_bounds__(kStepThreads + 32, 1) decode_step(const __grid
             done += take;
           }
         }
+        if (kFmt != 0) copies_wait();
         consumers_sync();
         if (!c.failed()) {
           if (lm) {
@@ -1272,7 +1280,7 @@ __global__ void __launch_bounds__(kStepThreads + 32, 1) decode_step(const __grid
             for (int i = tid; i < n / 4; i += kStepThreads) {
               float4 y = c.sum4(4 * i);
               if (kFmt) {
-                const float4 k = i == tid ? sc : __ldg(reinterpret_cast<const float4*>(scales) + i);
+                const float4 k = i == tid ? *reinterpret_cast<const float4*>(mine) : __ldg(reinterpret_cast<const float4*>(scales) + i);
                 y.x *= k.x; y.y *= k.y; y.z *= k.z; y.w *= k.w;
               }
               put(work + wk.act + (r.r0 >> 2) + i, pack_bf16x2(silu(y.x, y.y), silu(y.z, y.w)), tag + 6u);
