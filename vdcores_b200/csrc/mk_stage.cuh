@@ -154,9 +154,14 @@ __device__ __forceinline__ void widen16(uint8_t* dst, const uint8_t* src, int N,
     const __half2 sc = __half2half2(*reinterpret_cast<const __half*>(&hr));
     const uint32_t cw[2] = {cv.x, cv.y};
 #pragma unroll
-    for (int j = 0; j < 8; ++j) {
-      const float2 f = __half22float2(__hmul2(e2m1x2_to_half2((cw[j >> 2] >> (8 * (j & 3))) & 0xFFu), sc));
-      o[j] = pack_bf16x2(f.x, f.y);
+    for (int j = 0; j < 2; ++j) {
+      uint32_t h[4];
+      e2m1x8_to_half2(cw[j], h);
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        const float2 f = __half22float2(__hmul2(*reinterpret_cast<const __half2*>(&h[i]), sc));
+        o[4 * j + i] = pack_bf16x2(f.x, f.y);
+      }
     }
   }
   *reinterpret_cast<uint4*>(dst + ((2 * g16) * N + row) * 16) = make_uint4(o[0], o[1], o[2], o[3]);

@@ -17,6 +17,22 @@ __device__ __forceinline__ __half2 e2m1x2_to_half2(uint32_t byte) {
   return *reinterpret_cast<const __half2*>(&h);
 }
 
+// A word of eight e2m1 codes (four e4m3 codes) as f16 pairs.  The word is taken apart by the conversions' own operands: with a
+// shift and a mask per byte in front of them, conversion, scale and product of two rows of a warp's step took 58 cycles where
+// these take 37.
+__device__ __forceinline__ void e2m1x8_to_half2(uint32_t w, uint32_t (&o)[4]) {
+  asm("{.reg .b8 a, b, c, d;\n\t"
+      "mov.b32 {a, b, c, d}, %4;\n\t"
+      "cvt.rn.f16x2.e2m1x2 %0, a;\n\tcvt.rn.f16x2.e2m1x2 %1, b;\n\tcvt.rn.f16x2.e2m1x2 %2, c;\n\tcvt.rn.f16x2.e2m1x2 %3, d;}"
+      : "=r"(o[0]), "=r"(o[1]), "=r"(o[2]), "=r"(o[3]) : "r"(w));
+}
+__device__ __forceinline__ void e4m3x4_to_half2(uint32_t w, uint32_t (&o)[2]) {
+  asm("{.reg .b16 a, b;\n\t"
+      "mov.b32 {a, b}, %2;\n\t"
+      "cvt.rn.f16x2.e4m3x2 %0, a;\n\tcvt.rn.f16x2.e4m3x2 %1, b;}"
+      : "=r"(o[0]), "=r"(o[1]) : "r"(w));
+}
+
 // ------------------------------------------------------------------------- //
 // tcgen05 helpers
 // ------------------------------------------------------------------------- //

@@ -184,17 +184,17 @@ __host__ __device__ constexpr int unit_of(int fmt) { return fmt == 0 ? 256 : fmt
 template <int kFmt>
 __device__ __forceinline__ void expand(uint32_t (&o)[kFmt == 2 ? 4 : 2], const uint4& v, int part, uint32_t scales) {
   const uint32_t c[4] = {v.x, v.y, v.z, v.w};
-  if (kFmt == 0) {
+  if constexpr (kFmt == 0) {
     o[0] = c[2 * part];
     o[1] = c[2 * part + 1];
-  } else if (kFmt == 1) {
-    o[0] = e4m3_pair(c[part] & 0xFFFFu);
-    o[1] = e4m3_pair(c[part] >> 16);
+  } else if constexpr (kFmt == 1) {
+    e4m3x4_to_half2(c[part], o);
   } else {
     const uint32_t sc = __byte_perm(scales, 0, part < 2 ? 0x1010 : 0x3232);
+    e2m1x8_to_half2(c[part], o);
 #pragma unroll
-    for (int j = 0; j < (kFmt == 2 ? 4 : 2); ++j) {
-      const __half2 p = __hmul2(e2m1x2_to_half2((c[part] >> (8 * j)) & 0xFFu), *reinterpret_cast<const __half2*>(&sc));
+    for (int j = 0; j < 4; ++j) {
+      const __half2 p = __hmul2(*reinterpret_cast<const __half2*>(&o[j]), *reinterpret_cast<const __half2*>(&sc));
       o[j] = *reinterpret_cast<const uint32_t*>(&p);
     }
   }
