@@ -40,9 +40,9 @@ constexpr int kStepSmem = 227 * 1024 - 1024;         // dynamic; the rest is Ste
 enum { kQkv, kOut, kRouter, kGateUp, kDown, kVocab, kStages };
 
 // How an SM's consumers take a stage's rows: first row and rows; rows of a chunk; a warp's steps along the inputs; the teams and
-// the warps along the inputs (log2); a warp's room for partial sums; and the rows between two sums of them.
+// the warps along the inputs (log2); the steps of a slice (0: rows whole); and the rows between two sums of them.
 struct Plan {
-  int r0, n, per, units, lt, lk, ld, most;
+  int r0, n, per, units, lt, lk, slice, most;
 };
 
 struct StepShared {
@@ -119,7 +119,7 @@ __host__ __device__ inline StepWork step_work(const vdc_step& s) {
 // either.  A stage's boundary on the device had 1000 to 2300 cycles of integer divisions for this (of 8000 to 11000).
 struct Deal {
   int q, each, more, per, units;
-  int lt[2], lk[2], most[2];
+  int lt[2], lk[2], slice[2], most[2];
 };
 struct StepArgs {
   vdc_step s;
@@ -303,16 +303,23 @@ __host__ __device__ constexpr int chunk_rows(int rb) {        // an even number 
 // How the warps share n rows of K inputs: teams of them take the chunks in turn, so that one's way through a chunk (a few
 // hundred cycles of latency) falls into the others'; a team's warps divide K as far as that has steps for them (kw of them), and
 // the rows.
+// Dense bf16 rows of which four make more than one copy are cut along the inputs: a copy is `slice` steps of four rows,
+// the teams take a group's slices in turn and every warp keeps its sums of the four rows until the group ends.  Four rows read
+// the inputs from shared memory once instead of four times, and their sums meet once: a row of 28 KB took a team 2500 cycles,
+// 1.15 of what HBM takes to bring it.  Eight 8B-shaped layers 905 -> 887 us (four with e4m3 rows, two of which are a copy, 296 ->
+// 306: those stay whole).
 struct Split {
-  int teams, kw;
+  int teams, kw, slice;
 };
-__host__ __device__ inline Split split_of(int fmt, bool experts, int K, int n) {
+__host__ __device__ inline Split split_of(int fmt, bool experts, bool vocab, int K, int n) {
+  const int steps = K / unit_of(fmt), most = kItemBytes / (4 * 512);
+  if (fmt == 0 && !experts && steps > most && n >= 4 && (vocab || n <= kPartFloats / kStepWarps)) return {2, kStepWarps, most};
   const int units = K / unit_of(fmt), chunks = n / chunk_rows(row_bytes(fmt, K));
   // Two teams, since a chunk's place in the ring is held for as long as its team works on it; four where there is more work per
   // byte.  Four 8B-shaped layers with 1 / 2 / 4 teams: bf16 459 / 447 / 456 us, e4m3 358 / 328 / 335, NVFP4 348 / 339 / 334,
   // the 30B mixture of experts 273 / 261 / 260.
   const bool four = fmt == 2 || experts;
-  Split s{four && chunks >= 4 ? 4 : chunks >= 2 ? 2 : 1, 1};
+  Split s{four && chunks >= 4 ? 4 : chunks >= 2 ? 2 : 1, 1, 0};
   while (s.kw < kStepWarps / s.teams && 2 * s.kw <= units) s.kw *= 2;
   return s;
 }
@@ -329,10 +336,12 @@ __host__ inline Deal deal_of(const vdc_step& s, int stage) {
   d.units = K / unit_of(fmt);
   for (int i = 0; i < 2; ++i) {
     const int n = (d.each + (i == 0)) * d.q;
-    const Split sp = split_of(fmt, s.n_experts != 0, K, stage == kDown ? n * k : n);
+    const Split sp = split_of(fmt, s.n_experts != 0, stage == kVocab, K, stage == kDown ? n * k : n);
     while (1 << d.lt[i] < sp.teams) ++d.lt[i];
     while (1 << d.lk[i] < sp.kw) ++d.lk[i];
-    d.most[i] = stage == kVocab ? kPartFloats / sp.kw / d.per * d.per : n;
+    d.slice[i] = sp.slice;
+    const int per = sp.slice ? 4 : d.per;
+    d.most[i] = stage == kVocab ? kPartFloats / sp.kw / per * per : n;
   }
   return d;
 }
@@ -340,19 +349,23 @@ __host__ inline Deal deal_of(const vdc_step& s, int stage) {
 // ------------------------------------------------------------------------- //
 // producer
 // ------------------------------------------------------------------------- //
+// A whole warp: its lanes decide the same and an item's pieces are copied by a lane each.  (One lane alone takes 300 to 400 cycles
+// per piece: with four pieces to an item it took longer to ask for a row of 28 KB than HBM to bring it.)
 struct Producer {
   StepShared& sh;
   const Waiter& wait;
   uint8_t* ring;
-  int cap;
+  int cap, lane;
   RingAt at{kItems};       // next item
   int oldest = 0, live = 0, wr = 0, count = 0;
+  int mine = 0;            // offset in the ring of item `lane`
   uint32_t oldest_parity = 0u;
   bool wrapped = false, ok = true;
 
   // Room for one more item of `bytes`, freeing the oldest ones as they are consumed.
   __device__ __forceinline__ uint8_t* room(int bytes) {
     bytes = (bytes + 127) & ~127;
+    int first = __shfl_sync(0xffffffffu, mine, oldest);
 #pragma unroll 1
     while (ok) {
       if (live < kItems) {
@@ -360,41 +373,38 @@ struct Producer {
           wr = 0;
           wrapped = false;
         }
-        if (!wrapped && wr + bytes > cap && bytes <= sh.start[oldest]) {
+        if (!wrapped && wr + bytes > cap && bytes <= first) {
           wr = 0;
           wrapped = true;
         }
-        if (wr + bytes <= (wrapped ? sh.start[oldest] : cap)) break;
+        if (wr + bytes <= (wrapped ? first : cap)) break;
       }
-      ok = wait(&sh.empty[oldest], oldest_parity, 0, count);
-      const int was = sh.start[oldest];
+      ok = wait.warp_wait(&sh.empty[oldest], oldest_parity, 0, count);
+      const int was = first;
       if (++oldest == kItems) {
         oldest = 0;
         oldest_parity ^= 1u;
       }
+      first = __shfl_sync(0xffffffffu, mine, oldest);
       --live;
-      if (live > 0 && sh.start[oldest] < was) wrapped = false;
+      if (live > 0 && first < was) wrapped = false;
     }
     uint8_t* p = ring + wr;
-    sh.start[at.st] = wr;
+    if (lane == at.st) mine = wr;
+    if (lane == 0) sh.start[at.st] = wr;
     wr += bytes;
     ++live;
     return p;
   }
-  // n pieces of at most `bytes` (the last one `last`), one behind the other from src; with `second` a piece of the same size from
-  // there joins each one's item.
-  __device__ __forceinline__ void copy(const uint8_t* src, const uint8_t* second, int n, int bytes, int last) {
-#pragma unroll 1
-    for (int i = 0; i < n; ++i) {
-      const int size = i + 1 < n ? bytes : last;
-      uint8_t* p = room(second ? 2 * size : size);
-      if (!ok) return;
-      mbar_arrive_expect_tx(&sh.full[at.st], (uint32_t)(second ? 2 * size : size));
-      bulk_load_1d(p, src + (size_t)i * bytes, (uint32_t)size, &sh.full[at.st]);
-      if (second) bulk_load_1d(p + size, second, (uint32_t)size, &sh.full[at.st]);
-      at.next();
-      ++count;
-    }
+  // One item of n pieces of `bytes`, the i-th from this lane's src in lane i.
+  __device__ __forceinline__ void item(const uint8_t* src, int n, int bytes) {
+    uint8_t* p = room(n * bytes);
+    if (!ok) return;
+    if (lane == 0) mbar_arrive_expect_tx(&sh.full[at.st], (uint32_t)(n * bytes));
+    if (lane < n) bulk_load_1d(p + lane * bytes, src, (uint32_t)bytes, &sh.full[at.st]);
+    __syncwarp();
+    at.next();
+    ++count;
   }
 };
 
@@ -439,7 +449,7 @@ struct Consumer {
   RingAt at{kItems};
   int teams, turn;               // and the chunks until this warp's team is on
   int kw, kg, rw, rg, ld;        // warps along the inputs, this warp's place there; along the rows; rows there is room for
-  int per, units;                // rows of a chunk; steps along the inputs
+  int per, units, slice;         // rows of a chunk; steps along the inputs, of a slice of them
 
   __device__ __forceinline__ float* part() const { return reinterpret_cast<float*>(base + lay.part); }
   __device__ __forceinline__ uint32_t* hs() const { return reinterpret_cast<uint32_t*>(base + lay.h); }
@@ -596,23 +606,79 @@ struct Consumer {
     kg = warp & (kw - 1);
     rg = (warp & ((1 << lw) - 1)) >> p.lk;
     turn = warp >> lw;
-    ld = p.ld;
+    ld = kPartFloats >> p.lk;
+    slice = p.slice;
     per = p.per;
     units = p.units;
   }
   // This warp's steps along the inputs, kSteps at a time while there are as many.
   template <int kSteps, class F>
-  __device__ __forceinline__ void walk(F f) const {
-    int u = kg;
+  static __device__ __forceinline__ void walk(int u, int kw, int units, F f) {
 #pragma unroll 1
     for (; u + (kSteps - 1) * kw < units; u += kSteps * kw) f(Steps<kSteps>{}, u);
 #pragma unroll 1
     for (; u < units; u += kw) f(Steps<1>{}, u);
   }
+  // The four lanes 4g + t that hold the diagonal of a product of tiles: of lane l's sums the one of row g, and of row 8 + g.
+  template <int kFmt, int kPairs>
+  __device__ __forceinline__ void diagonal(const float (&d)[kFmt == 2 ? 2 : 1][kPairs][4], int p, float& first, float& second) const {
+    const bool diag = (lane >> 3) == (lane & 3), odd = lane & 4;
+    first = diag ? (odd ? d[0][p][1] : d[0][p][0]) : 0.f;
+    second = diag ? (odd ? d[0][p][3] : d[0][p][2]) : 0.f;
+    if constexpr (kFmt == 2) {
+      first += diag ? (odd ? d[1][p][1] : d[1][p][0]) : 0.f;
+      second += diag ? (odd ? d[1][p][3] : d[1][p][2]) : 0.f;
+    }
+  }
+  // Four sums over the lanes at once: lanes 8i .. 8i + 7 end up with the i-th.
+  __device__ __forceinline__ float sum_lanes(float a, float b, float c, float e) const {
+    const bool up = lane & 16, right = lane & 8;
+    float p = up ? c : a, q = up ? e : b;
+    p += __shfl_xor_sync(0xffffffffu, up ? a : c, 16);
+    q += __shfl_xor_sync(0xffffffffu, up ? b : e, 16);
+    float v = (right ? q : p) + __shfl_xor_sync(0xffffffffu, right ? p : q, 8);
+#pragma unroll
+    for (int o = 4; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+    return v;
+  }
+  // n rows in slices: every warp's share of row r to part[warp][row0 + r].
+  template <int kFmt>
+  __device__ __forceinline__ void sliced(int n, const uint8_t* xp) {
+#pragma unroll 1
+    for (int r0 = 0; r0 < n; r0 += 4) {
+      const int nr = min(4, n - r0);
+      float d[1][2][4] = {};
+#pragma unroll 1
+      for (int u0 = 0; u0 < units; u0 += slice, at.next(), turn ^= 1) {
+        if (!wait.warp_wait(&sh.full[at.st], at.parity, 2, r0)) return;
+        if (turn == 0) {
+          const uint8_t* w = base + lay.ring + sh.start[at.st];
+          const int nu = min(slice, units - u0);
+          int off[4];
+#pragma unroll
+          for (int i = 0; i < 4; ++i) off[i] = min(i, nr - 1) * nu * 512;
+          const uint8_t* xs = xp + u0 * (unit_of(kFmt) * 2);
+          walk<steps_of(kFmt, 2)>(warp & 3, 4, nu, [&](auto steps, int u) { dot_steps<kFmt, 2, decltype(steps)::value>(d, w, off, false, xs, u, 4, lane, 0); });
+          // the place's next bytes come through the other proxy, and nothing that depends on these reads is stored before
+          fence_proxy_async_smem();
+        }
+        __syncwarp();
+        if (lane == 0) mbar_arrive(&sh.empty[at.st]);
+      }
+      float a, b, c, e;
+      diagonal<kFmt, 2>(d, 0, a, b);
+      diagonal<kFmt, 2>(d, 1, c, e);
+      const float v = sum_lanes(a, b, c, e);
+      if ((lane & 7) == 0 && (lane >> 3) < nr) part()[warp * ld + r0 + (lane >> 3)] = v;
+    }
+  }
   // n rows from the ring times the inputs xp: every warp's share of row r to part[kg][row0 + r], rows side by side for the
   // threads that add the shares up.
   template <int kFmt, bool kFma>
   __device__ __forceinline__ void rows(int K, int n, const uint8_t* xp, int row0) {
+    if constexpr (kFmt == 0 && !kFma) {
+      if (slice) return sliced<kFmt>(n, xp);
+    }
     const int rb = row_bytes(kFmt, K);
 #pragma unroll 1
     for (int r0 = 0; r0 < n; r0 += per, at.next()) {
@@ -627,17 +693,6 @@ struct Consumer {
 #pragma unroll
         for (int i = 0; i < 4; ++i) off[i] = min(r + i * rw, nr - 1) * rb;
         float a, b, c = 0.f, e = 0.f;          // the lane's share of the four rows
-        // of a tile the lanes that hold its diagonal
-        const bool diag = (lane >> 3) == (lane & 3), odd = lane & 4;
-        auto share = [&](auto& d, int p, float& first, float& second) {
-          first = diag ? (odd ? d[0][p][1] : d[0][p][0]) : 0.f;
-          second = diag ? (odd ? d[0][p][3] : d[0][p][2]) : 0.f;
-          if (kFmt == 2) {
-            constexpr int k = kFmt == 2 ? 1 : 0;
-            first += diag ? (odd ? d[k][p][1] : d[k][p][0]) : 0.f;
-            second += diag ? (odd ? d[k][p][3] : d[k][p][2]) : 0.f;
-          }
-        };
         if (kFma && r + 2 * rw < nr) {
           float2 d[4] = {};
 #pragma unroll 2
@@ -650,22 +705,15 @@ struct Consumer {
           a = d[0].x + d[0].y; b = d[1].x + d[1].y;
         } else if (r + 2 * rw < nr) {
           float d[kFmt == 2 ? 2 : 1][2][4] = {};
-          walk<steps_of(kFmt, 2)>([&](auto steps, int u) { dot_steps<kFmt, 2, decltype(steps)::value>(d, w, off, false, xp, u, kw, lane, K); });
-          share(d, 0, a, b);
-          share(d, 1, c, e);
+          walk<steps_of(kFmt, 2)>(kg, kw, units, [&](auto steps, int u) { dot_steps<kFmt, 2, decltype(steps)::value>(d, w, off, false, xp, u, kw, lane, K); });
+          diagonal<kFmt, 2>(d, 0, a, b);
+          diagonal<kFmt, 2>(d, 1, c, e);
         } else {
           float d[kFmt == 2 ? 2 : 1][1][4] = {};
-          walk<steps_of(kFmt, 1)>([&](auto steps, int u) { dot_steps<kFmt, 1, decltype(steps)::value>(d, w, off, r + rw >= nr, xp, u, kw, lane, K); });
-          share(d, 0, a, b);
+          walk<steps_of(kFmt, 1)>(kg, kw, units, [&](auto steps, int u) { dot_steps<kFmt, 1, decltype(steps)::value>(d, w, off, r + rw >= nr, xp, u, kw, lane, K); });
+          diagonal<kFmt, 1>(d, 0, a, b);
         }
-        // four sums over the lanes at once: lanes 8i .. 8i + 7 end up with row i
-        const bool up = lane & 16, right = lane & 8;
-        float p = up ? c : a, q = up ? e : b;
-        p += __shfl_xor_sync(0xffffffffu, up ? a : c, 16);
-        q += __shfl_xor_sync(0xffffffffu, up ? b : e, 16);
-        float v = (right ? q : p) + __shfl_xor_sync(0xffffffffu, right ? p : q, 8);
-#pragma unroll
-        for (int o = 4; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+        const float v = sum_lanes(a, b, c, e);
         const int mine = r + (lane >> 3) * rw;
         if ((lane & 7) == 0 && mine < nr) part()[kg * ld + row0 + r0 + mine] = v;
       }
@@ -1045,7 +1093,7 @@ __global__ void __launch_bounds__(kStepThreads + 32, 1) decode_step(const __grid
   if (tid < kStages) {
     const Deal& d = args.deal[tid];
     const int i = sm < d.more ? 0 : 1;
-    sh.plan[tid] = Plan{(sm * d.each + min(sm, d.more)) * d.q, (d.each + 1 - i) * d.q, d.per, d.units, d.lt[i], d.lk[i], kPartFloats >> d.lk[i], d.most[i]};
+    sh.plan[tid] = Plan{(sm * d.each + min(sm, d.more)) * d.q, (d.each + 1 - i) * d.q, d.per, d.units, d.lt[i], d.lk[i], d.slice[i], d.most[i]};
     if (kExperts && tid == kGateUp) {
       sh.slot0 = sh.plan[tid].r0 / (2 * s.ffn);
       sh.head = (sh.slot0 + 1) * 2 * s.ffn - sh.plan[tid].r0;
@@ -1085,9 +1133,9 @@ __global__ void __launch_bounds__(kStepThreads + 32, 1) decode_step(const __grid
   float* weights = reinterpret_cast<float*>(ids + kMaxTopK);
 
   if (warp == kStepWarps) {
-    if (lane == 0) {
+    {
       fence_proxy_async();      // the cache rows of the steps before were written with ordinary stores
-      Producer p{sh, wait, base + lay.ring, lay.total - lay.ring};
+      Producer p{sh, wait, base + lay.ring, lay.total - lay.ring, lane};
       const int* table = state + VDC_ST_PAGETABLE;
       // stage after stage; a stage is one run of rows or several (experts), the attention one run per page
       int l = 0, stage = kQkv, sub = 0;
@@ -1095,7 +1143,7 @@ __global__ void __launch_bounds__(kStepThreads + 32, 1) decode_step(const __grid
       while (p.ok) {
         asm volatile("" : "+r"(stage), "+r"(sub));
         const uint8_t *src = nullptr, *second = nullptr;
-        int n = 0, rb = rbH, r0 = sh.plan[stage].r0, rows = sh.plan[stage].n;
+        int rb = rbH, r0 = sh.plan[stage].r0, rows = sh.plan[stage].n;
         bool more = false;                     // the stage goes on
         if (stage == kQkv) {
           src = reinterpret_cast<const uint8_t*>(s.wqkv) + (size_t)l * QKV * rbH;
@@ -1120,7 +1168,7 @@ __global__ void __launch_bounds__(kStepThreads + 32, 1) decode_step(const __grid
           src = reinterpret_cast<const uint8_t*>(s.wgu);
           size_t first = (size_t)l * 2 * F;
           if (E) {                             // a slot's rows end where the next slot's begin
-            if (sub == 0 && (rows || sh.plan[kDown].n) && !(p.ok = wait(&sh.routed, (uint32_t)l & 1u, 0, l))) break;
+            if (sub == 0 && (rows || sh.plan[kDown].n) && !(p.ok = wait.warp_wait(&sh.routed, (uint32_t)l & 1u, 0, l))) break;
             const int end = r0 + rows, slot = sh.slot0 + sub;
             r0 = max(r0, slot * 2 * F);
             rows = min(end, (slot + 1) * 2 * F) - r0;
@@ -1138,10 +1186,16 @@ __global__ void __launch_bounds__(kStepThreads + 32, 1) decode_step(const __grid
           rb = H * 2;
           src = reinterpret_cast<const uint8_t*>(s.lm_head);
         }
-        if (rows > 0) {
-          const int per = second ? 1 : sh.plan[stage].per;
-          n = (rows + per - 1) / per;
-          p.copy(src + (size_t)r0 * rb, second, n, per * rb, (rows - (n - 1) * per) * rb);
+        const int slice = kExperts || second ? 0 : sh.plan[stage].slice, units = sh.plan[stage].units, per = second ? 1 : sh.plan[stage].per;
+        src += (size_t)r0 * rb;
+        if (slice) {
+#pragma unroll 1
+          for (int g = 0; g < rows && p.ok; g += 4, src += 4 * rb)
+#pragma unroll 1
+            for (int u0 = 0; u0 < units; u0 += slice) p.item(src + lane * rb + u0 * 512, min(4, rows - g), min(slice, units - u0) * 512);
+        } else {
+#pragma unroll 1
+          for (int g = 0; g < rows && p.ok; g += per) p.item(second && lane ? second : src + (size_t)g * rb, second ? 2 : 1, min(per, rows - g) * rb);
         }
         if (stage == kVocab) break;
         ++sub;
@@ -1397,7 +1451,7 @@ extern "C" const char* vdc_step_refuses(const vdc_step* s, bool pointers) {
   auto fits = [&](int rows, int q, int K, int slots) {
     const int most = share_of(rows, q, 0, s->num_sms).n;
     for (int n = most; n > 0 && n >= most - q; n -= q)
-      if (n * slots > kPartFloats / split_of(s->wfmt, s->n_experts != 0, K, n * slots).kw) return false;
+      if (n * slots > kPartFloats / split_of(s->wfmt, s->n_experts != 0, false, K, n * slots).kw) return false;
     return true;
   };
   const int k = s->n_experts ? s->top_k : 1;
