@@ -31,6 +31,8 @@ __device__ __forceinline__ void st_cluster4(uint32_t a, uint32_t x, uint32_t y, 
 __device__ __forceinline__ void st_shared4(uint32_t a, uint32_t x, uint32_t y, uint32_t z, uint32_t w) {
   asm volatile("st.shared.v4.b32 [%0], {%1,%2,%3,%4};" ::"r"(a), "r"(x), "r"(y), "r"(z), "r"(w) : "memory");
 }
+__device__ __forceinline__ void st_cluster1(uint32_t a, uint32_t x) { asm volatile("st.shared::cluster.b32 [%0], %1;" ::"r"(a), "r"(x) : "memory"); }
+__device__ __forceinline__ void st_shared1(uint32_t a, uint32_t x) { asm volatile("st.shared.b32 [%0], %1;" ::"r"(a), "r"(x) : "memory"); }
 __device__ __forceinline__ float ld_cluster1(uint32_t a) {
   float v;
   asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(v) : "r"(a) : "memory");
@@ -133,11 +135,10 @@ __device__ __forceinline__ void scale8(float (&v)[8], const float* sc) {
 // Bytes of a chunk of n weight rows x 64 inputs as stored: bf16, e4m3, or e2m1 pairs with one e4m3 scale per 16.
 __host__ __device__ constexpr int chunk_bytes(int wfmt, int n) { return wfmt == 0 ? n * 128 : wfmt == 1 ? n * 64 : n * 36; }
 
-// 16 weights of a row (inputs 16 g16 .. + 15 of a chunk of N rows) from their stored form to bf16 pieces of the tensor cores'
-// operand layout (exact for e4m3 and for e2m1 code times block scale).
+// 16 weights of a row (inputs 16 g16 .. + 15 of a chunk of N rows) from their stored form to bf16 (exact for e4m3 and for e2m1
+// code times block scale).
 template <int kFmt>
-__device__ __forceinline__ void widen16(uint8_t* dst, const uint8_t* src, int N, int row, int g16) {
-  uint32_t o[8];
+__device__ __forceinline__ void widen16(uint32_t (&o)[8], const uint8_t* src, int N, int row, int g16) {
   if (kFmt == 1) {
     const uint4 v = lds128(src + (g16 * N + row) * 16);
     const uint32_t wv[4] = {v.x, v.y, v.z, v.w};
@@ -164,6 +165,12 @@ __device__ __forceinline__ void widen16(uint8_t* dst, const uint8_t* src, int N,
       }
     }
   }
+}
+// The same as pieces of the tensor cores' operand layout in shared memory.
+template <int kFmt>
+__device__ __forceinline__ void widen16(uint8_t* dst, const uint8_t* src, int N, int row, int g16) {
+  uint32_t o[8];
+  widen16<kFmt>(o, src, N, row, g16);
   *reinterpret_cast<uint4*>(dst + ((2 * g16) * N + row) * 16) = make_uint4(o[0], o[1], o[2], o[3]);
   *reinterpret_cast<uint4*>(dst + ((2 * g16 + 1) * N + row) * 16) = make_uint4(o[4], o[5], o[6], o[7]);
 }

@@ -18,7 +18,9 @@ namespace vdc {
 
 constexpr int kBlk = VDC_STAGE_BLOCK;   // weight rows of a projection block: accumulator columns
 constexpr int kKc = 64;                 // inputs per chunk
-constexpr int kMaxRing = 8;
+constexpr int kMaxRing = 16;
+constexpr int kBufs = 4;                // of widened weights
+constexpr int kRowCols = 128;           // tensor memory: sums in columns 0 .. 127, widened weights behind them
 constexpr int kGemmThreads = 320;       // producer warp, MMA warp, eight warps that convert weights and run the epilogue
 constexpr int kEpiThreads = 256;
 // Shared memory of one CTA.  Two CTAs fit an SM (the register budget allows it too), so that one streams while the
@@ -32,7 +34,7 @@ constexpr int kCol4 = kBlk / 4;         // groups of four columns in the fp32 ex
 struct GemmShared {
   uint64_t full[kMaxRing], empty[kMaxRing];
   uint64_t ready[kMaxRing];     // weights converted
-  uint64_t stg_empty[2];
+  uint64_t stg_empty[kBufs];
   uint64_t done;
   uint32_t tmem;
   volatile int fail;
@@ -46,10 +48,8 @@ __host__ __device__ constexpr int stage_size(int wfmt, int bpad) {
   return bpad * kKc * 2 + (chunk_bytes(wfmt, kBlk) + 127) / 128 * 128;
 }
 __host__ __device__ inline int ring_stages(int wfmt, int bpad) {
-  const int staging = wfmt ? 2 * kBlk * kKc * 2 : 0;
-  const int stage = stage_size(wfmt, bpad);
-  const int n = (kGemmSmem - 2048 - 128 - staging) / stage;
-  return n >= kMaxRing ? kMaxRing : wfmt && n >= 4 ? n & ~1 : n;    // even where weights are converted, see `teams`
+  const int n = (kGemmSmem - 2048 - 128) / stage_size(wfmt, bpad), most = wfmt ? kMaxRing : 8;
+  return n >= most ? most : wfmt && n >= 4 ? n & ~1 : n;    // even where weights are converted, see `teams`
 }
 
 // The exchange tile of a CTA: [source CTA][four columns][its row, one spare][4] fp32.  Every CTA of the cluster writes the
@@ -99,6 +99,8 @@ __global__ void __launch_bounds__(kGemmThreads, 2) stage_gemm(const __grid_const
                                                               vdc_status* status, uint64_t timeout_ns) {
   extern __shared__ uint8_t dyn[];
   __shared__ GemmShared sh;
+  constexpr int kTmem = kFmt != 0 ? kRowCols + kBufs * kKc / 2 : kBlk;
+  static_assert(kTmem == 128 || kTmem == 256, "a power of two");
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int splits = s.splits;
   const int rank = splits > 1 ? (int)cluster_rank() : 0;
@@ -113,17 +115,16 @@ __global__ void __launch_bounds__(kGemmThreads, 2) stage_gemm(const __grid_const
   // leave its staging buffer then falls into the other's conversion: e4m3 gate/up at 32 rows 74.7 -> 65.6 us.
   const int teams = n_ring & 1 ? 1 : 2;
   uint8_t* ring = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(dyn) + 127) & ~(uintptr_t)127);
-  uint8_t* staging = ring + n_ring * stage_bytes;
   const Waiter wait{&sh.fail, status, timeout_ns, s.kind};
 
-  if (warp == 1) tmem_alloc(&sh.tmem, kBlk);
+  if (warp == 1) tmem_alloc(&sh.tmem, kTmem);
   if (tid == 0) {
     for (int i = 0; i < n_ring; ++i) {
       mbar_init(&sh.full[i], 1);
       mbar_init(&sh.empty[i], 1);
       mbar_init(&sh.ready[i], kEpiThreads / 32 / teams);
     }
-    for (int i = 0; i < 2; ++i) mbar_init(&sh.stg_empty[i], 1);
+    for (int i = 0; i < kBufs; ++i) mbar_init(&sh.stg_empty[i], 1);
     mbar_init(&sh.done, 1);
     sh.fail = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
@@ -166,14 +167,13 @@ __global__ void __launch_bounds__(kGemmThreads, 2) stage_gemm(const __grid_const
     }
   } else if (warp == 1) {
     if (lane == 0) {
-      const uint32_t idesc = umma_idesc_bf16_m128(N);
-      const uint32_t lbo_a = (uint32_t)s.Bpad * 16u, lbo_b = (uint32_t)N * 16u;
+      const uint32_t idesc = umma_idesc_bf16_m128(kFmt != 0 ? s.Bpad : N);
+      const uint32_t lbo_x = (uint32_t)s.Bpad * 16u, lbo_w = (uint32_t)N * 16u;
       // No divisions per chunk and descriptors advanced by constants, here and in the other roles: what this thread does beside
       // its MMAs the tensor cores wait for.  A step of 32 rows with e4m3 weights 338 -> 319 us, 16 rows NVFP4 364 -> 358, 3 rows
       // bf16 245 -> 242.
-      const uint64_t a0 = umma_desc(smem_u32(ring), lbo_a, 128u);
-      const uint64_t b0 = umma_desc(smem_u32(kFmt != 0 ? staging : ring + xbytes), lbo_b, 128u);
-      const uint32_t stage16 = (uint32_t)stage_bytes >> 4, step_a = (2u * lbo_a) >> 4, step_b = (2u * lbo_b) >> 4;
+      const uint64_t x0 = umma_desc(smem_u32(ring), lbo_x, 128u), w0 = umma_desc(smem_u32(ring + xbytes), lbo_w, 128u);
+      const uint32_t stage16 = (uint32_t)stage_bytes >> 4, step_x = (2u * lbo_x) >> 4, step_w = (2u * lbo_w) >> 4;
       RingAt at{n_ring};
       for (int i = 0; i < n_ch; ++i, at.next()) {
         const int st = at.st;
@@ -181,11 +181,15 @@ __global__ void __launch_bounds__(kGemmThreads, 2) stage_gemm(const __grid_const
         if (kFmt != 0 && ok) ok = wait(&sh.ready[st], at.parity, 1, i);
         if (!ok) break;
         tc_fence_after();
-        const uint64_t ad = a0 + st * stage16, bd = b0 + (kFmt != 0 ? (i & 1) * (uint32_t)(kBlk * kKc * 2 >> 4) : st * stage16);
+        const uint64_t xd = x0 + st * stage16, wd = w0 + st * stage16;
+        const uint32_t wt = tmem + kRowCols + (i & (kBufs - 1)) * (kKc / 2);
 #pragma unroll
-        for (int k = 0; k < kKc / 16; ++k) umma_bf16(tmem, ad + k * step_a, bd + k * step_b, idesc, (uint32_t)((i | k) != 0));
+        for (int k = 0; k < kKc / 16; ++k) {
+          if (kFmt != 0) umma_bf16_ta(tmem, wt + k * 8, xd + k * step_x, idesc, (uint32_t)((i | k) != 0));
+          else umma_bf16(tmem, xd + k * step_x, wd + k * step_w, idesc, (uint32_t)((i | k) != 0));
+        }
         umma_commit(&sh.empty[st]);
-        if (kFmt != 0) umma_commit(&sh.stg_empty[i & 1]);
+        if (kFmt != 0) umma_commit(&sh.stg_empty[i & (kBufs - 1)]);
       }
       umma_commit(&sh.done);
       wait(&sh.done, 0u, 1, n_ch);
@@ -194,23 +198,28 @@ __global__ void __launch_bounds__(kGemmThreads, 2) stage_gemm(const __grid_const
   } else {
     const int t = tid - 64;
     if (kFmt != 0) {
-      const int team = kEpiThreads / teams, tt = t & (team - 1), row = t & 127;
+      // A warp widens the rows whose lanes of tensor memory it reaches; rows past N are whatever lies there, for sums that nobody
+      // reads.
+      const int team = kEpiThreads / teams, tt = t & (team - 1), quarter = warp & 3, row = quarter * 32 + lane;
+      const uint32_t to = tmem + ((uint32_t)(quarter * 32) << 16) + kRowCols;
       RingAt at{n_ring};
       if (t >= team) at.next();
       for (int i = t / team; i < n_ch; i += teams) {
-        const int st = at.st;
+        const int st = at.st, buf = i & (kBufs - 1);
         const bool seen = wait(&sh.full[st], at.parity, 2, i) &&
-                          (i < 2 || wait(&sh.stg_empty[i & 1], (uint32_t)((i >> 1) - 1) & 1u, 2, i));
+                          (i < kBufs || wait(&sh.stg_empty[buf], (uint32_t)(i / kBufs - 1) & 1u, 2, i));
         if (!__all_sync(0xffffffffu, seen)) break;      // as in warp_wait, one vote for both
-        uint8_t* dst = staging + (i & 1) * (kBlk * kKc * 2);
+        tc_fence_after();
         const uint8_t* src = ring + st * stage_bytes + xbytes;
-        if (row < N) {
 #pragma unroll 2
-          for (int g16 = tt >> 7; g16 < kKc / 16; g16 += team >> 7) {
-            widen16<kFmt>(dst, src, N, row, g16);
-          }
+        for (int g16 = tt >> 7; g16 < kKc / 16; g16 += team >> 7) {
+          uint32_t o[8];
+          widen16<kFmt == 0 ? 1 : kFmt>(o, src, N, min(row, N - 1), g16);
+          tmem_st8(to + buf * (kKc / 2) + g16 * 8, o);
         }
-        fence_proxy_async_smem();
+        tmem_st_wait();
+        tc_fence_before();
+        fence_proxy_async_smem();      // the place's next weights come through the other proxy
         __syncwarp();
         if (lane == 0) mbar_arrive(&sh.ready[st]);   // one arrival per warp: one per thread would queue on the barrier's word
         at.next();
@@ -234,7 +243,24 @@ __global__ void __launch_bounds__(kGemmThreads, 2) stage_gemm(const __grid_const
   if (warp >= 2 && !failed) {
     const int quarter = warp & 3, half = (warp - 2) >> 2;
     const int b = quarter * 32 + lane, ng = N >> 4;
-    if (quarter * 32 < s.Bpad) {
+    if (kFmt != 0) {
+      // a lane has a weight row, its columns the rows: four lanes make up four columns of the tile
+      const int n = quarter * 32 + lane, lg = 31 - __clz(nb);
+      for (int g = half; g < s.Bpad / 16; g += 2) {
+        uint32_t r[16];
+        tmem_ld16(tmem + ((uint32_t)(quarter * 32) << 16) + (uint32_t)(g * 16), r);
+        if (n < N) {
+#pragma unroll
+          for (int j = 0; j < 16; ++j) {
+            const int row = g * 16 + j;
+            const uint32_t at = tile_at(tile, rank, nb, n >> 2, row & (nb - 1)) + (uint32_t)(n & 3) * 4u;
+            if (splits > 1) st_cluster1(peer_smem(at, (uint32_t)(row >> lg)), r[j]);
+            else st_shared1(at, r[j]);
+          }
+        }
+        __syncwarp();
+      }
+    } else if (quarter * 32 < s.Bpad) {
       for (int gi = half ? (ng + 1) / 2 : 0; gi < (half ? ng : (ng + 1) / 2); ++gi) {
         uint32_t r[16];
         tmem_ld16(tmem + ((uint32_t)(quarter * 32) << 16) + (uint32_t)(gi * 16), r);
@@ -337,7 +363,7 @@ __global__ void __launch_bounds__(kGemmThreads, 2) stage_gemm(const __grid_const
     }
   }
   wait.drain();
-  if (warp == 1) tmem_dealloc(tmem, kBlk);
+  if (warp == 1) tmem_dealloc(tmem, kTmem);
 }
 
 // ------------------------------------------------------------------------- //
