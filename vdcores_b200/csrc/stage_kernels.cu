@@ -34,7 +34,6 @@ constexpr int kCol4 = kBlk / 4;         // groups of four columns in the fp32 ex
 struct GemmShared {
   uint64_t full[kMaxRing], empty[kMaxRing];
   uint64_t ready[kMaxRing];     // weights converted
-  uint64_t stg_empty[kBufs];
   uint64_t done;
   uint32_t tmem;
   volatile int fail;
@@ -51,6 +50,8 @@ __host__ __device__ inline int ring_stages(int wfmt, int bpad) {
   const int n = (kGemmSmem - 2048 - 128) / stage_size(wfmt, bpad), most = wfmt ? kMaxRing : 8;
   return n >= most ? most : wfmt && n >= 4 ? n & ~1 : n;    // even where weights are converted, see `teams`
 }
+
+static_assert((kGemmSmem - 2048 - 128) / stage_size(1, 128) >= kBufs, "a place for every buffer of widened weights");
 
 // The exchange tile of a CTA: [source CTA][four columns][its row, one spare][4] fp32.  Every CTA of the cluster writes the
 // sums of its K-range straight from tensor memory into the tile of the CTA that finishes the row (consecutive rows lie
@@ -124,7 +125,6 @@ __global__ void __launch_bounds__(kGemmThreads, 2) stage_gemm(const __grid_const
       mbar_init(&sh.empty[i], 1);
       mbar_init(&sh.ready[i], kEpiThreads / 32 / teams);
     }
-    for (int i = 0; i < kBufs; ++i) mbar_init(&sh.stg_empty[i], 1);
     mbar_init(&sh.done, 1);
     sh.fail = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
@@ -174,22 +174,27 @@ __global__ void __launch_bounds__(kGemmThreads, 2) stage_gemm(const __grid_const
       // bf16 245 -> 242.
       const uint64_t x0 = umma_desc(smem_u32(ring), lbo_x, 128u), w0 = umma_desc(smem_u32(ring + xbytes), lbo_w, 128u);
       const uint32_t stage16 = (uint32_t)stage_bytes >> 4, step_x = (2u * lbo_x) >> 4, step_w = (2u * lbo_w) >> 4;
+      // A finished wait is 145 cycles here, a commit 140 and an MMA 75, more than the tensor cores take for it: the descriptors are
+      // made in front of the wait, converted weights stand for the chunk's arrival too (the warps that converted them have seen
+      // it), and one commit gives back the chunk's place and the buffer.
       RingAt at{n_ring};
       for (int i = 0; i < n_ch; ++i, at.next()) {
         const int st = at.st;
-        bool ok = wait(&sh.full[st], at.parity, 1, i);
-        if (kFmt != 0 && ok) ok = wait(&sh.ready[st], at.parity, 1, i);
-        if (!ok) break;
-        tc_fence_after();
-        const uint64_t xd = x0 + st * stage16, wd = w0 + st * stage16;
-        const uint32_t wt = tmem + kRowCols + (i & (kBufs - 1)) * (kKc / 2);
+        uint64_t xd[kKc / 16], wd[kKc / 16];
 #pragma unroll
         for (int k = 0; k < kKc / 16; ++k) {
-          if (kFmt != 0) umma_bf16_ta(tmem, wt + k * 8, xd + k * step_x, idesc, (uint32_t)((i | k) != 0));
-          else umma_bf16(tmem, xd + k * step_x, wd + k * step_w, idesc, (uint32_t)((i | k) != 0));
+          xd[k] = x0 + st * stage16 + k * step_x;
+          wd[k] = kFmt != 0 ? tmem + kRowCols + (i & (kBufs - 1)) * (kKc / 2) + k * 8 : w0 + st * stage16 + k * step_w;
+          asm volatile("" : "+l"(xd[k]), "+l"(wd[k]));
+        }
+        if (!wait(kFmt != 0 ? &sh.ready[st] : &sh.full[st], at.parity, 1, i)) break;
+        tc_fence_after();
+#pragma unroll
+        for (int k = 0; k < kKc / 16; ++k) {
+          if (kFmt != 0) umma_bf16_ta(tmem, (uint32_t)wd[k], xd[k], idesc, (uint32_t)((i | k) != 0));
+          else umma_bf16(tmem, xd[k], wd[k], idesc, (uint32_t)((i | k) != 0));
         }
         umma_commit(&sh.empty[st]);
-        if (kFmt != 0) umma_commit(&sh.stg_empty[i & (kBufs - 1)]);
       }
       umma_commit(&sh.done);
       wait(&sh.done, 0u, 1, n_ch);
@@ -202,12 +207,16 @@ __global__ void __launch_bounds__(kGemmThreads, 2) stage_gemm(const __grid_const
       // reads.
       const int team = kEpiThreads / teams, tt = t & (team - 1), quarter = warp & 3, row = quarter * 32 + lane;
       const uint32_t to = tmem + ((uint32_t)(quarter * 32) << 16) + kRowCols;
-      RingAt at{n_ring};
-      if (t >= team) at.next();
+      // `old`: the place of the chunk whose buffer chunk i takes, kBufs chunks back.  It cannot be given back a second time before
+      // chunk i is converted, since the ring has kBufs places at least.
+      RingAt at{n_ring}, old{n_ring};
+      if (t >= team) {
+        at.next();
+        old.next();
+      }
       for (int i = t / team; i < n_ch; i += teams) {
         const int st = at.st, buf = i & (kBufs - 1);
-        const bool seen = wait(&sh.full[st], at.parity, 2, i) &&
-                          (i < kBufs || wait(&sh.stg_empty[buf], (uint32_t)(i / kBufs - 1) & 1u, 2, i));
+        const bool seen = wait(&sh.full[st], at.parity, 2, i) && (i < kBufs || wait(&sh.empty[old.st], old.parity, 2, i));
         if (!__all_sync(0xffffffffu, seen)) break;      // as in warp_wait, one vote for both
         tc_fence_after();
         const uint8_t* src = ring + st * stage_bytes + xbytes;
@@ -224,6 +233,10 @@ __global__ void __launch_bounds__(kGemmThreads, 2) stage_gemm(const __grid_const
         if (lane == 0) mbar_arrive(&sh.ready[st]);   // one arrival per warp: one per thread would queue on the barrier's word
         at.next();
         if (teams == 2) at.next();
+        if (i >= kBufs) {
+          old.next();
+          if (teams == 2) old.next();
+        }
       }
     }
     grid_dep_wait();
