@@ -135,42 +135,63 @@ __device__ __forceinline__ void scale8(float (&v)[8], const float* sc) {
 // Bytes of a chunk of n weight rows x 64 inputs as stored: bf16, e4m3, or e2m1 pairs with one e4m3 scale per 16.
 __host__ __device__ constexpr int chunk_bytes(int wfmt, int n) { return wfmt == 0 ? n * 128 : wfmt == 1 ? n * 64 : n * 36; }
 
-// 16 weights of a row (inputs 16 g16 .. + 15 of a chunk of N rows) from their stored form to bf16 (exact for e4m3 and for e2m1
-// code times block scale).
+// What a sum of products with widened weights is to be multiplied by.
 template <int kFmt>
-__device__ __forceinline__ void widen16(uint32_t (&o)[8], const uint8_t* src, int N, int row, int g16) {
-  if (kFmt == 1) {
-    const uint4 v = lds128(src + (g16 * N + row) * 16);
-    const uint32_t wv[4] = {v.x, v.y, v.z, v.w};
-#pragma unroll
-    for (int j = 0; j < 4; ++j) {
-      const float2 lo = e4m3x2_to_float2(wv[j] & 0xFFFFu), hi = e4m3x2_to_float2(wv[j] >> 16);
-      o[2 * j] = pack_bf16x2(lo.x, lo.y);
-      o[2 * j + 1] = pack_bf16x2(hi.x, hi.y);
-    }
-  } else {
-    const uint8_t* g = src + g16 * 9 * N;
-    const uint2 cv = *reinterpret_cast<const uint2*>(g + row * 8);
-    const __half_raw hr = __nv_cvt_fp8_to_halfraw((__nv_fp8_storage_t)g[8 * N + row], __NV_E4M3);
-    const __half2 sc = __half2half2(*reinterpret_cast<const __half*>(&hr));
-    const uint32_t cw[2] = {cv.x, cv.y};
-#pragma unroll
-    for (int j = 0; j < 2; ++j) {
-      uint32_t h[4];
-      e2m1x8_to_half2(cw[j], h);
-#pragma unroll
-      for (int i = 0; i < 4; ++i) {
-        const float2 f = __half22float2(__hmul2(*reinterpret_cast<const __half2*>(&h[i]), sc));
-        o[4 * j + i] = pack_bf16x2(f.x, f.y);
-      }
+constexpr float kNarrowUnit = kFmt == 2 ? 0x1p26f : 1.f;
+// 16 weights of a row (inputs 16 g16 .. + 15 of a chunk of N rows) as stored, and as bf16 (exact for e4m3 and for e2m1 code times
+// block scale), divided by kNarrowUnit.
+template <int kFmt>
+struct Narrow {
+  uint32_t v[kFmt == 1 ? 4 : 2], scale;
+  __device__ __forceinline__ void load(const uint8_t* src, int N, int row, int g16) {
+    if constexpr (kFmt == 1) {
+      const uint4 w = lds128(src + (g16 * N + row) * 16);
+      v[0] = w.x; v[1] = w.y; v[2] = w.z; v[3] = w.w;
+    } else {
+      const uint8_t* g = src + g16 * 9 * N;
+      const uint2 w = *reinterpret_cast<const uint2*>(g + row * 8);
+      v[0] = w.x; v[1] = w.y;
+      scale = g[8 * N + row];
     }
   }
-}
+  __device__ __forceinline__ void widen(uint32_t (&o)[8]) const {
+    if constexpr (kFmt == 1) {
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        const float2 lo = e4m3x2_to_float2(v[j] & 0xFFFFu), hi = e4m3x2_to_float2(v[j] >> 16);
+        o[2 * j] = pack_bf16x2(lo.x, lo.y);
+        o[2 * j + 1] = pack_bf16x2(hi.x, hi.y);
+      }
+    } else {
+      // A code's upper two bits (sign, exponent) select the upper byte of its bf16 number, the lower two (exponent, mantissa) the
+      // lower byte: 2^-126 of its value, which the block's scale times 2^100 makes 2^-26 (kNarrowUnit) of the weight, exactly.
+      // Nine integer instructions for eight codes; by way of f16 and fp32 they are four conversions of a quarter, eight of half
+      // and four of half a pipe's rate.
+      const __half_raw hr = __nv_cvt_fp8_to_halfraw((__nv_fp8_storage_t)scale, __NV_E4M3);
+      const __nv_bfloat162 sc = __float2bfloat162_rn(__half2float(*reinterpret_cast<const __half*>(&hr)) * 0x1p100f);
+#pragma unroll
+      for (int j = 0; j < 2; ++j)
+#pragma unroll
+        for (int i = 0; i < 2; ++i) {
+          const uint32_t sel = ((v[j] >> (2 * i)) & 0x33333333u) | 0x04040404u;
+#pragma unroll
+          for (int e = 0; e < 2; ++e) {
+            uint32_t w;      // of the selector's nibbles the lower four count, none of them above 7
+            asm("prmt.b32 %0, %1, %2, %3;" : "=r"(w) : "r"(0x81800100u), "r"(0xC0804000u), "r"(sel >> (16 * e)));
+            const __nv_bfloat162 p = __hmul2(*reinterpret_cast<const __nv_bfloat162*>(&w), sc);
+            o[4 * j + 2 * i + e] = *reinterpret_cast<const uint32_t*>(&p);
+          }
+        }
+    }
+  }
+};
 // The same as pieces of the tensor cores' operand layout in shared memory.
 template <int kFmt>
 __device__ __forceinline__ void widen16(uint8_t* dst, const uint8_t* src, int N, int row, int g16) {
   uint32_t o[8];
-  widen16<kFmt>(o, src, N, row, g16);
+  Narrow<kFmt> w;
+  w.load(src, N, row, g16);
+  w.widen(o);
   *reinterpret_cast<uint4*>(dst + ((2 * g16) * N + row) * 16) = make_uint4(o[0], o[1], o[2], o[3]);
   *reinterpret_cast<uint4*>(dst + ((2 * g16 + 1) * N + row) * 16) = make_uint4(o[4], o[5], o[6], o[7]);
 }

@@ -220,12 +220,19 @@ __global__ void __launch_bounds__(kGemmThreads, 2) stage_gemm(const __grid_const
         if (!__all_sync(0xffffffffu, seen)) break;      // as in warp_wait, one vote for both
         tc_fence_after();
         const uint8_t* src = ring + st * stage_bytes + xbytes;
-#pragma unroll 2
-        for (int g16 = tt >> 7; g16 < kKc / 16; g16 += team >> 7) {
-          uint32_t o[8];
-          widen16<kFmt == 0 ? 1 : kFmt>(o, src, N, min(row, N - 1), g16);
-          tmem_st8(to + buf * (kKc / 2) + g16 * 8, o);
-        }
+        // all loads before the first store to tensor memory, which no later load passes
+        constexpr int kGroups = kKc / 16;
+        Narrow<kFmt == 0 ? 1 : kFmt> w[kGroups];
+#pragma unroll
+        for (int g = 0; g < kGroups; ++g)
+          if (teams == 2 || (g & 1) == tt >> 7) w[g].load(src, N, min(row, N - 1), g);
+#pragma unroll
+        for (int g = 0; g < kGroups; ++g)
+          if (teams == 2 || (g & 1) == tt >> 7) {
+            uint32_t o[8];
+            w[g].widen(o);
+            tmem_st8(to + buf * (kKc / 2) + g * 8, o);
+          }
         tmem_st_wait();
         tc_fence_before();
         fence_proxy_async_smem();      // the place's next weights come through the other proxy
@@ -266,6 +273,7 @@ __global__ void __launch_bounds__(kGemmThreads, 2) stage_gemm(const __grid_const
 #pragma unroll
           for (int j = 0; j < 16; ++j) {
             const int row = g * 16 + j;
+            r[j] = __float_as_uint(__uint_as_float(r[j]) * kNarrowUnit<kFmt>);
             const uint32_t at = tile_at(tile, rank, nb, n >> 2, row & (nb - 1)) + (uint32_t)(n & 3) * 4u;
             if (splits > 1) st_cluster1(peer_smem(at, (uint32_t)(row >> lg)), r[j]);
             else st_shared1(at, r[j]);
