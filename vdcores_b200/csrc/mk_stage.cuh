@@ -39,6 +39,10 @@ __device__ __forceinline__ float ld_cluster1(uint32_t a) {
   return v;
 }
 
+// Dynamic shared memory from its first multiple of 128 bytes.  An offset and no cast, so that the compiler still knows whose memory
+// it is: through a pointer rounded up as a number every access would be a generic one.
+__device__ __forceinline__ uint8_t* aligned128(uint8_t* dyn) { return dyn + (-(int)smem_u32(dyn) & 127); }
+
 // The first error since the host last looked goes to the status block.
 static __device__ void report(vdc_status* status, int code, int kind, int role, int at, int aux) {
   if (atomicCAS(&status->abort, 0, 1) == 0) {

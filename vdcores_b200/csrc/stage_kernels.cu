@@ -115,7 +115,7 @@ __global__ void __launch_bounds__(kGemmThreads, 2) stage_gemm(const __grid_const
   // rounds on, and the barrier's parity cannot tell those apart).  Teams, because a team's wait for the tensor cores to
   // leave its staging buffer then falls into the other's conversion: e4m3 gate/up at 32 rows 74.7 -> 65.6 us.
   const int teams = n_ring & 1 ? 1 : 2;
-  uint8_t* ring = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(dyn) + 127) & ~(uintptr_t)127);
+  uint8_t* ring = aligned128(dyn);
   const Waiter wait{&sh.fail, status, timeout_ns, s.kind};
 
   if (warp == 1) tmem_alloc(&sh.tmem, kTmem);
@@ -516,7 +516,7 @@ __global__ void __launch_bounds__(kAttnThreads, 2) stage_attn(const __grid_const
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int splits = s.splits, rank = splits > 1 ? (int)cluster_rank() : 0;
   const int unit = first_unit + (int)blockIdx.x / splits, h = unit % s.n_kv, b = unit / s.n_kv, G = s.group;
-  uint8_t* ring = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(dyn) + 127) & ~(uintptr_t)127);
+  uint8_t* ring = aligned128(dyn);
   const Waiter wait{&sh.fail, status, timeout_ns, s.kind};
   attn_setup(sh, tid);
   const int* st = reinterpret_cast<const int*>(s.state) + (size_t)b * s.state_stride;
@@ -682,7 +682,7 @@ __global__ void __launch_bounds__(kAttnThreads, 2) stage_attn_prefill(const __gr
   const int rows = kWide ? ld_relaxed_gpu(st + VDC_WIDE_N) : s.B;
   const int b0 = (kWide ? s.Bpad / per_tile - 1 - unit / s.n_kv : unit / s.n_kv) * per_tile;
   if (kWide && b0 >= rows) return;
-  uint8_t* ring = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(dyn) + 127) & ~(uintptr_t)127);
+  uint8_t* ring = aligned128(dyn);
   const Waiter wait{&sh.fail, status, timeout_ns, s.kind};
   attn_setup(sh, tid);
   const int pos0 = ld_relaxed_gpu(st + (kWide ? VDC_WIDE_POS : VDC_ST_POS));

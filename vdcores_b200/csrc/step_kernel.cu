@@ -1087,7 +1087,7 @@ __global__ void __launch_bounds__(kStepThreads + 32, 1) decode_step(const __grid
   const StepLayout& lay = args.lay;
   const StepWork& wk = args.wk;
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, sm = blockIdx.x, sms = gridDim.x;
-  uint8_t* base = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(dyn) + 127) & ~(uintptr_t)127);
+  uint8_t* base = aligned128(dyn);
   const Waiter wait{&sh.fail, status, timeout_ns, VDC_STEP_KIND};
   constexpr int D = VDC_HEAD_DIM;
   if (tid < kStages) {
