@@ -78,6 +78,7 @@ int vdc_launch_async_full(int num_sms, int insts_per_sm, const void* compute_ins
  *       VDC_STAGE_RESID  hid += result; stats_out += squares of hid
  *       VDC_STAGE_SILU   gate/up row pairs to out = silu(gate) * up
  *       VDC_STAGE_ARGMAX the rows' largest logit into keys
+ *       VDC_STAGE_SUMS   fp32 sums to out [M / 4][Bpad][4]
  *   kind VDC_STAGE_ATTN: attention of every row over its own pages (one row per sequence), queries `q`, result `out`
  *   kind VDC_STAGE_ATTN_PREFILL: the same for rows that are consecutive positions of ONE sequence
  *     (both read the state blocks, and pages without a new row, while the stage directly in front still runs: that stage

@@ -470,3 +470,22 @@ def test_logits_without_a_number_end_a_generation_with_an_error(cuda_device):
     eng.norm_w.fill_(1.0)
     start()
     assert eng.generate(4) == good
+
+
+@pytest.mark.parametrize("fmt", ["bf16", "fp8", "nvfp4"])
+@pytest.mark.parametrize("M,K,splits,B", [(48, 1024, 1, 128), (1040, 2048, 2, 128), (4096, 4096, 8, 77), (256, 1024, 4, 16), (400, 1024, 1, 33)])
+def test_projection_leaves_fp32_sums(cuda_device, fmt, M, K, splits, B):
+    """A block of 48, 16 or 128 weight rows, K whole and shared, rows that do not fill the accumulator: fp32 sums of bf16 products,
+    so only the order of the additions differs from the matmul's (1e-5 of the result's norm)."""
+    from vdcores_b200 import isa
+    dev = cuda_device
+    w, sc, wd = weights(M, K, fmt, dev)
+    x = seeded((B, K), 9).to(BF16)
+    xd = packed_rows(x, dev)
+    Bp = next(p for p in (16, 32, 64, 128) if B <= p)
+    out = torch.full((M // 4, Bp, 4), -7.0, device=dev)
+    run(dev, gemm(dev, fmt, B, M, K, splits, w, sc, xd, mode=isa.STAGE_SUMS, out=out.data_ptr()))
+    got = out.permute(1, 0, 2).reshape(Bp, M)
+    want = x.double().to(dev) @ wd.double().to(dev).t()
+    assert rel(got[:B].double(), want) < 1e-5
+    assert bool((got[B:] == -7.0).all())

@@ -228,6 +228,7 @@ static const char* check_stage(const vdc_stage& s) {
     case VDC_STAGE_RESID:
       return s.hid && s.stats_out && al16(s.hid) && al4(s.stats_out) ? nullptr : "residual stage: null or misaligned pointer";
     case VDC_STAGE_SILU: return s.out && al16(s.out) ? nullptr : "gate/up stage: null or misaligned pointer";
+    case VDC_STAGE_SUMS: return s.out && al16(s.out) ? nullptr : "sums stage: null or misaligned pointer";
     case VDC_STAGE_ARGMAX: return s.keys && al8(s.keys) ? nullptr : "argmax stage: null or misaligned pointer";
     default: return "projection stage: unknown mode";
   }

@@ -352,6 +352,15 @@ __global__ void __launch_bounds__(kGemmThreads, 2) stage_gemm(const __grid_const
             }
             *reinterpret_cast<uint4*>(reinterpret_cast<uint8_t*>(s.out) + kc_piece(s.Bpad, b, (n0 >> 1) + f * 8)) = pack8(o);
           }
+        } else if (s.mode == VDC_STAGE_SUMS) {
+          for (int f = f0; f < N / 8; f += fstep) {
+            float v[8];
+            sum8(v, ring, splits, nb, bl, f * 8);
+            scale8(v, scales ? scales + n0 + f * 8 : nullptr);
+            float4* to = reinterpret_cast<float4*>(s.out) + (size_t)((n0 >> 2) + f * 2) * s.Bpad + b;
+            to[0] = make_float4(v[0], v[1], v[2], v[3]);
+            to[s.Bpad] = make_float4(v[4], v[5], v[6], v[7]);
+          }
         } else {   // VDC_STAGE_ARGMAX over bf16 logits, the lowest row wins ties
           float best = -INFINITY;
           int row = 0x7fffffff;
@@ -682,7 +691,8 @@ __global__ void __launch_bounds__(kAttnThreads, 2) stage_attn_prefill(const __gr
   const int rows = kWide ? ld_relaxed_gpu(st + VDC_WIDE_N) : s.B;
   const int b0 = (kWide ? s.Bpad / per_tile - 1 - unit / s.n_kv : unit / s.n_kv) * per_tile;
   if (kWide && b0 >= rows) return;
-  uint8_t* ring = aligned128(dyn);
+  // rounded up as a number: with the registers that known shared memory takes here, 24 bytes are spilled (2048 positions +0.5 %)
+  uint8_t* ring = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(dyn) + 127) & ~(uintptr_t)127);
   const Waiter wait{&sh.fail, status, timeout_ns, s.kind};
   attn_setup(sh, tid);
   const int pos0 = ld_relaxed_gpu(st + (kWide ? VDC_WIDE_POS : VDC_ST_POS));
