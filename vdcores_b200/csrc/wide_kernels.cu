@@ -72,7 +72,7 @@ __global__ void __launch_bounds__(kWideThreads, 1) wide_gemm(const __grid_consta
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int per = s.group, NT = s.n_kv;
   const int stage_bytes = wide_stage_bytes(kFmt, per, NT), n_ring = wide_ring(kFmt, per, NT);
-  uint8_t* ring = aligned128(dyn);
+  uint8_t* ring = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(dyn) + 127) & ~(uintptr_t)127);
   uint8_t* staging = ring + n_ring * stage_bytes;
   const Waiter wait{&sh.fail, status, timeout_ns, s.kind};
 
