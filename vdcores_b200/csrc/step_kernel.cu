@@ -9,9 +9,9 @@
 // The same step as a program of the megakernel (csrc/megakernel.cu) counts barriers down: fence, atomic, poll, then a copy,
 // about 7 us per boundary.
 //
-// Measured against that program (B200): three layers of width 512 109 -> 69 us, eight 8B-shaped bf16 layers and a 128256-row
-// vocabulary projection 1012 -> 981, four such layers e4m3 387 -> 331, NVFP4 388 -> 326, four layers of a 30B mixture of experts
-// 437 -> 260.
+// Measured against that program (B200): three layers of width 512 109 -> 50 us, eight 8B-shaped bf16 layers and a 128256-row
+// vocabulary projection 1012 -> 813, four such layers e4m3 387 -> 245, NVFP4 388 -> 232, four layers of a 30B mixture of experts
+// 437 -> 208.
 //
 // An entry buffer is written again one layer later, when everything that read it must have been read: whoever polls a buffer
 // has rows in the same or the following stage, and those rows go into what the next writer of the buffer waits for.
@@ -45,6 +45,26 @@ struct Plan {
   int r0, n, per, units, lt, lk, slice, most;
 };
 
+// An SM's share of the attention: one KV head's pages first .. first + count - 1; `live` splits of the head have pages.  Up to
+// kAlone pages stay with one SM: there is nothing to merge then.  Few KV heads leave a head more splits than a warp has lanes;
+// they are used once 32 splits would walk more than kAlone pages each.  Eight layers of width 1024 with one KV head at 32000 /
+// 128000 positions 373 -> 274 and 839 -> 396 us, two 382 -> 315 and 876 -> 533 (with 8 or 16 pages in place of kAlone one head
+// at 32000 positions takes 309 and 386).
+struct Pages {
+  int h, split, live, first, count;
+};
+__device__ __forceinline__ Pages pages_of(const vdc_step& s, int pos, int sm) {
+  Pages p{sm % s.n_kv, sm / s.n_kv, 0, 0, 0};
+  const int n = min(pos / VDC_KV_PAGE + 1, s.max_pages);
+  const int per = n <= kAlone ? n : max((n + s.n_splits - 1) / s.n_splits, min((n + kFewSplits - 1) / kFewSplits, kAlone));
+  p.live = (n + per - 1) / per;
+  if (p.split < p.live) {
+    p.first = p.split * per;
+    p.count = min(per, n - p.first);
+  }
+  return p;
+}
+
 struct StepShared {
   uint64_t full[kItems], empty[kItems], routed;
   int start[kItems];                                 // offset of an item in the ring
@@ -54,6 +74,8 @@ struct StepShared {
   int best_row[kStepWarps];
   alignas(16) Plan plan[kStages];
   int slot0, head;                                   // experts: the slot of this SM's first gate/up row, its rows there are
+  int pos, token, new_row;                           // of the step; the new row's place in the cache pools
+  Pages pages;
   int four0, four1;                                  // fours of a head's dims that this SM merges
 };
 // Behind the ring: what the consumers share.
@@ -126,6 +148,8 @@ struct StepArgs {
   StepLayout lay;
   StepWork wk;
   Deal deal[kStages];
+  float inv_hidden;
+  int q_width, qkv_width;
 };
 // Rows of a stage that one SM takes.
 struct Share {
@@ -142,6 +166,12 @@ __device__ __forceinline__ void put2(uint64_t* p, uint32_t a, uint32_t b, uint32
   asm volatile("st.relaxed.gpu.global.v2.u64 [%0], {%1,%2};" ::"l"(p), "l"(((uint64_t)tag << 32) | a),
                "l"(((uint64_t)tag << 32) | b)
                : "memory");
+}
+// 1 / x of a normal x to one ulp (0 for infinity): an instruction, where a division takes 350 cycles of a boundary.
+__device__ __forceinline__ float reciprocal(float x) {
+  float r;
+  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
+  return r;
 }
 struct Two {
   uint64_t a, b;
@@ -286,8 +316,9 @@ __device__ __forceinline__ void dot_steps(float (&d)[kFmt == 2 ? 2 : 1][kPairs][
   }
 }
 // Steps of a warp whose loads are on their way together.  With one (and the products in the order of the source) a warp took 290
-// cycles for a step of four bf16 rows, a chain of a load, two products and an addition.
-__host__ __device__ constexpr int steps_of(int fmt, int pairs) { return fmt == 0 ? 4 : 2; }
+// cycles for a step of four bf16 rows, a chain of a load, two products and an addition.  A step of NVFP4 rows is as many products
+// by itself as four of bf16 (four 8B-shaped layers 232 us, 246 with two steps and the registers they spill).
+__host__ __device__ constexpr int steps_of(int fmt) { return fmt == 0 ? 4 : fmt == 1 ? 2 : 1; }
 
 // Units of q rows; the first SMs' shares are never empty while there are any.
 __host__ __device__ inline Share share_of(int rows, int q, int sm, int sms) {
@@ -408,30 +439,24 @@ struct Producer {
   }
 };
 
-// An SM's share of the attention: one KV head's pages first .. first + count - 1; `live` splits of the head have pages.  Up to
-// kAlone pages stay with one SM: there is nothing to merge then.  Few KV heads leave a head more splits than a warp has lanes;
-// they are used once 32 splits would walk more than kAlone pages each.  Eight layers of width 1024 with one KV head at 32000 /
-// 128000 positions 373 -> 274 and 839 -> 396 us, two 382 -> 315 and 876 -> 533 (with 8 or 16 pages in place of kAlone one head
-// at 32000 positions takes 309 and 386).
-struct Pages {
-  int h, split, live, first, count;
-};
-__device__ __forceinline__ Pages pages_of(const vdc_step& s, int pos, int sm) {
-  Pages p{sm % s.n_kv, sm / s.n_kv, 0, 0, 0};
-  const int n = min(pos / VDC_KV_PAGE + 1, s.max_pages);
-  const int per = n <= kAlone ? n : max((n + s.n_splits - 1) / s.n_splits, min((n + kFewSplits - 1) / kFewSplits, kAlone));
-  p.live = (n + per - 1) / per;
-  if (p.split < p.live) {
-    p.first = p.split * per;
-    p.count = min(per, n - p.first);
-  }
-  return p;
-}
-
 // ------------------------------------------------------------------------- //
 // consumers
 // ------------------------------------------------------------------------- //
 __device__ __forceinline__ void consumers_sync() { asm volatile("bar.sync 1, %0;" ::"n"(kStepThreads) : "memory"); }
+
+// Whether to look again for entries that are not there yet (it: looks so far): the time of the first such question, 0 when the wait
+// was given up.  Everything by value: what a call could reach by its address would have to be in memory.
+static __device__ __noinline__ uint64_t look_again(volatile int* fail, vdc_status* status, uint64_t timeout_ns, uint64_t t0, int at, int it) {
+  if (*fail) return 0;
+  if (ld_relaxed_gpu(&status->abort) == 0) {
+    const uint64_t now = globaltimer_ns();
+    if (t0 == 0) return now;
+    if (now - t0 <= timeout_ns) return t0;
+    report(status, VDC_ERR_TIMEOUT, VDC_STEP_KIND, 1, at, it);
+  }
+  *fail = 1;
+  return 0;
+}
 
 template <int n>
 struct Steps {
@@ -455,17 +480,9 @@ struct Consumer {
   __device__ __forceinline__ uint32_t* hs() const { return reinterpret_cast<uint32_t*>(base + lay.h); }
   __device__ __forceinline__ uint8_t* x() const { return base + lay.x; }
 
-  // Whether to look again for entries that are not there yet (it: looks so far); false when the wait was given up.
-  __device__ __noinline__ bool again(const uint64_t* p, uint32_t it, uint64_t& t0) const {
-    if (*wait.fail) return false;
-    if (ld_relaxed_gpu(&wait.status->abort) == 0) {
-      const uint64_t now = globaltimer_ns();
-      if (t0 == 0) t0 = now;
-      if (now - t0 <= wait.timeout_ns) return true;
-      report(wait.status, VDC_ERR_TIMEOUT, VDC_STEP_KIND, 1, (int)(p - reinterpret_cast<const uint64_t*>(s.work)), (int)it);
-    }
-    *wait.fail = 1;
-    return false;
+  __device__ __forceinline__ bool again(const uint64_t* p, uint32_t it, uint64_t& t0) const {
+    t0 = look_again(wait.fail, wait.status, wait.timeout_ns, t0, (int)(p - reinterpret_cast<const uint64_t*>(s.work)), (int)it);
+    return t0 != 0;
   }
   __device__ __forceinline__ bool poll2(const uint64_t* p, uint32_t tag, Two& v) const {
     uint64_t t0 = 0;
@@ -575,7 +592,7 @@ struct Consumer {
       const float4 r = *reinterpret_cast<const float4*>(sh.red + k);
       tot += r.x; tot += r.y; tot += r.z; tot += r.w;
     }
-    const float rstd = rsqrtf(tot / (float)H + s.eps);
+    const float rstd = rsqrtf(fmaf(tot, args.inv_hidden, s.eps));
     copies_wait();
 #pragma unroll
     for (int j = 0; j < kMost; ++j) {
@@ -658,7 +675,7 @@ struct Consumer {
 #pragma unroll
           for (int i = 0; i < 4; ++i) off[i] = min(i, nr - 1) * nu * 512;
           const uint8_t* xs = xp + u0 * (unit_of(kFmt) * 2);
-          walk<steps_of(kFmt, 2)>(warp & 3, 4, nu, [&](auto steps, int u) { dot_steps<kFmt, 2, decltype(steps)::value>(d, w, off, false, xs, u, 4, lane, 0); });
+          walk<steps_of(kFmt)>(warp & 3, 4, nu, [&](auto steps, int u) { dot_steps<kFmt, 2, decltype(steps)::value>(d, w, off, false, xs, u, 4, lane, 0); });
           // the place's next bytes come through the other proxy, and nothing that depends on these reads is stored before
           fence_proxy_async_smem();
         }
@@ -705,12 +722,12 @@ struct Consumer {
           a = d[0].x + d[0].y; b = d[1].x + d[1].y;
         } else if (r + 2 * rw < nr) {
           float d[kFmt == 2 ? 2 : 1][2][4] = {};
-          walk<steps_of(kFmt, 2)>(kg, kw, units, [&](auto steps, int u) { dot_steps<kFmt, 2, decltype(steps)::value>(d, w, off, false, xp, u, kw, lane, K); });
+          walk<steps_of(kFmt)>(kg, kw, units, [&](auto steps, int u) { dot_steps<kFmt, 2, decltype(steps)::value>(d, w, off, false, xp, u, kw, lane, K); });
           diagonal<kFmt, 2>(d, 0, a, b);
           diagonal<kFmt, 2>(d, 1, c, e);
         } else {
           float d[kFmt == 2 ? 2 : 1][1][4] = {};
-          walk<steps_of(kFmt, 1)>(kg, kw, units, [&](auto steps, int u) { dot_steps<kFmt, 1, decltype(steps)::value>(d, w, off, r + rw >= nr, xp, u, kw, lane, K); });
+          walk<steps_of(kFmt)>(kg, kw, units, [&](auto steps, int u) { dot_steps<kFmt, 1, decltype(steps)::value>(d, w, off, r + rw >= nr, xp, u, kw, lane, K); });
           diagonal<kFmt, 1>(d, 0, a, b);
         }
         const float v = sum_lanes(a, b, c, e);
@@ -826,7 +843,7 @@ struct Consumer {
           const int r = pos % VDC_KV_PAGE, piece = lane & 15;
           const uint4 v = reinterpret_cast<const uint4*>(krow)[lane];
           *reinterpret_cast<uint4*>(page + (lane < 16 ? 0 : kPageBytes) + r * (D * 2) + ((piece ^ (r & 7)) << 4)) = v;
-          const size_t row = (size_t)ld_relaxed_gpu(reinterpret_cast<const int*>(s.state) + VDC_ST_NEWROW) * (D * 2);
+          const size_t row = (size_t)sh.new_row * (D * 2);
           const size_t pool = (size_t)layer * s.max_pages * s.n_kv * kPageBytes + (size_t)pg.h * kPageBytes;
           uint8_t* to = reinterpret_cast<uint8_t*>(lane < 16 ? s.kpool : s.vpool) + pool + row;
           if (!failed()) *reinterpret_cast<uint4*>(to + ((piece ^ (r & 7)) << 4)) = v;
@@ -863,9 +880,9 @@ struct Consumer {
 #pragma unroll
           for (int w = 0; w < 4; ++w) mn = fmaxf(mn, gm[w * 8 + 2 * t4 + j]);
           const bool none = mn == -INFINITY;
-          al[j] = none ? 1.f : exp2f(m[j] - mn);
-          e[j] = none ? 0.f : exp2f(e[j] - mn);
-          e[j + 2] = none ? 0.f : exp2f(e[j + 2] - mn);
+          al[j] = none ? 1.f : exp2_ftz(m[j] - mn);
+          e[j] = none ? 0.f : exp2_ftz(e[j] - mn);
+          e[j + 2] = none ? 0.f : exp2_ftz(e[j + 2] - mn);
           m[j] = mn;
           l[j] = l[j] * al[j] + e[j] + e[j + 2];      // this warp's positions only
         }
@@ -923,14 +940,14 @@ struct Consumer {
       float n0 = 0.f, n1 = 0.f, den = 0.f;
 #pragma unroll
       for (int k = 0; k < kGroups; ++k) {
-        const float mk = w0[k * 40 + 32 + g], wt = mk == -INFINITY ? 0.f : exp2f(mk - mm);
+        const float mk = w0[k * 40 + 32 + g], wt = mk == -INFINITY ? 0.f : exp2_ftz(mk - mm);
         const float2 v = *reinterpret_cast<const float2*>(part() + (k * 8 + g) * kOutLd + 2 * d2);
         n0 = fmaf(wt, v.x, n0);
         n1 = fmaf(wt, v.y, n1);
         den = fmaf(wt, w0[k * 40 + g] + w0[k * 40 + 8 + g] + w0[k * 40 + 16 + g] + w0[k * 40 + 24 + g], den);
       }
       if (pg.live == 1) {
-        const float inv = den > 0.f ? 1.f / den : 0.f;       // 0 where no score was a number
+        const float inv = den > 0.f ? reciprocal(den) : 0.f;       // 0 where no score was a number
         put(out + (size_t)pg.h * G * (D / 2) + t, pack_bf16x2(n0 * inv, n1 * inv), tag_out);
       } else {
         const size_t u = (size_t)pg.h * s.n_splits + pg.split;
@@ -977,7 +994,7 @@ struct Consumer {
         float m1, l1;
         take(sp, n1, m1, l1);
         if (!ok) continue;
-        const float m2 = fmaxf(mk, m1), w0 = mk == -INFINITY ? 0.f : exp2f(mk - m2), w1 = m1 == -INFINITY ? 0.f : exp2f(m1 - m2);
+        const float m2 = fmaxf(mk, m1), w0 = mk == -INFINITY ? 0.f : exp2_ftz(mk - m2), w1 = m1 == -INFINITY ? 0.f : exp2_ftz(m1 - m2);
         n = make_float4(fmaf(w0, n.x, w1 * n1.x), fmaf(w0, n.y, w1 * n1.y), fmaf(w0, n.z, w1 * n1.z), fmaf(w0, n.w, w1 * n1.w));
         lk = fmaf(w0, lk, w1 * l1);
         mk = m2;
@@ -986,7 +1003,7 @@ struct Consumer {
       float mm = mk;
 #pragma unroll 1
       for (int z = lanes >> 1; z > 0; z >>= 1) mm = fmaxf(mm, __shfl_xor_sync(0xffffffffu, mm, z));
-      const float wt = mk == -INFINITY ? 0.f : exp2f(mk - mm);
+      const float wt = mk == -INFINITY ? 0.f : exp2_ftz(mk - mm);
       n = make_float4(wt * n.x, wt * n.y, wt * n.z, wt * n.w);
       float den = wt * lk;
 #pragma unroll 1
@@ -997,7 +1014,7 @@ struct Consumer {
         n.w += __shfl_xor_sync(0xffffffffu, n.w, z);
         den += __shfl_xor_sync(0xffffffffu, den, z);
       }
-      const float inv = den > 0.f ? 1.f / den : 0.f;
+      const float inv = den > 0.f ? reciprocal(den) : 0.f;
       if (mine == 0 && i < hi) put2(out + ((size_t)pg.h * fours + i) * 2, pack_bf16x2(n.x * inv, n.y * inv), pack_bf16x2(n.z * inv, n.w * inv), tag_out);
     }
   }
@@ -1015,7 +1032,7 @@ struct Consumer {
     consumers_sync();
     if (warp == 0) {
       constexpr int kMost = kMaxExperts / 32;
-      float v[kMost], mx = -INFINITY, sum = 0.f;
+      float v[kMost], mx = -INFINITY;
 #pragma unroll
       for (int j = 0; j < kMost; ++j) {
         v[j] = lane + 32 * j < E ? lg[lane + 32 * j] : -INFINITY;
@@ -1024,39 +1041,30 @@ struct Consumer {
 #pragma unroll
       for (int o = 16; o > 0; o >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, o));
 #pragma unroll
-      for (int j = 0; j < kMost; ++j) {
-        v[j] = v[j] == -INFINITY ? 0.f : __expf(v[j] - mx);
-        sum += v[j];
-      }
-      sum = warp_sum(sum);
+      for (int j = 0; j < kMost; ++j) v[j] = lane + 32 * j < E ? __expf(v[j] - mx) : -1.f;
+      // The largest, k times over; of equal ones the lowest number.  Their weights are renormalised, so the softmax's own sum does
+      // not matter.
       float all = 0.f, mine = 0.f;
       int id = 0;
 #pragma unroll 1
       for (int k = 0; k < s.top_k; ++k) {
-        float bv = -1.f;
-        int bi = 0x7fffffff;
+        float bv = v[0];
+        int bi = lane;
 #pragma unroll
-        for (int j = 0; j < kMost; ++j)
-          if (lane + 32 * j < E && v[j] > bv) {
+        for (int j = 1; j < kMost; ++j)
+          if (v[j] > bv) {
             bv = v[j];
             bi = lane + 32 * j;
           }
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) {
-          const float ov = __shfl_xor_sync(0xffffffffu, bv, o);
-          const int oi = __shfl_xor_sync(0xffffffffu, bi, o);
-          if (ov > bv || (ov == bv && oi < bi)) {
-            bv = ov;
-            bi = oi;
-          }
-        }
-        bi = min(bi, E - 1);               // logits without a number select nothing: any expert will do
+        // a number that was not chosen yet is not negative, so that its bits order it as an integer
+        const int top = __reduce_max_sync(0xffffffffu, __float_as_int(bv));
+        bi = min((int)__reduce_min_sync(0xffffffffu, __float_as_int(bv) == top ? (unsigned)bi : 0x7fffffffu), E - 1);
 #pragma unroll
         for (int j = 0; j < kMost; ++j)
           if (bi == lane + 32 * j) v[j] = -1.f;
-        all += bv / sum;
+        all += __int_as_float(top);
         if (lane == k) {
-          mine = bv / sum;
+          mine = __int_as_float(top);
           id = bi;
         }
       }
@@ -1114,20 +1122,26 @@ __global__ void __launch_bounds__(kStepThreads + 32, 1) decode_step(const __grid
   // Read before the error is looked for: in a launch that fails, SM 0 counts the launch behind the error.  An SM that starts late
   // and took the number from there would leave entries that the next launch takes for its own.
   const uint32_t launches = (uint32_t)ld_acquire_gpu(reinterpret_cast<const int*>(s.work));
-  if (__syncthreads_or(ld_relaxed_gpu(&status->abort))) {      // behind an unread error nothing runs
+  const int* state = reinterpret_cast<const int*>(s.state);
+  const int aborted = ld_relaxed_gpu(&status->abort);
+  if (tid == 0) {
+    const int pos = ld_relaxed_gpu(state + VDC_ST_POS), token = ld_relaxed_gpu(state + VDC_ST_TOKEN);
+    sh.new_row = ld_relaxed_gpu(state + VDC_ST_NEWROW);
+    sh.pos = pos;
+    sh.token = token < 0 || token >= s.vocab ? 0 : token;
+    if (sh.token != token && sm == 0 && !aborted) report(status, VDC_ERR_TOKEN, VDC_STEP_KIND, 0, 0, token);
+    const Pages pg = pages_of(s, pos, sm);
+    sh.pages = pg;
+    sh.four0 = s.group * (D / 4) * pg.split / pg.live;
+    sh.four1 = s.group * (D / 4) * (pg.split + 1) / pg.live;
+  }
+  if (__syncthreads_or(aborted)) {      // behind an unread error nothing runs
     if (sm == 0 && tid == 0) red_release_gpu_add(reinterpret_cast<int*>(s.work), 1);
     return;
   }
 
-  const int H = s.hidden, F = s.ffn, G = s.group, Q = s.n_kv * G * D, QKV = Q + 2 * s.n_kv * D, L = s.n_layers, E = kExperts ? s.n_experts : 0;
-  const int* state = reinterpret_cast<const int*>(s.state);
-  const int pos = ld_relaxed_gpu(state + VDC_ST_POS);
-  const Pages pg = pages_of(s, pos, sm);
+  const int H = s.hidden, F = s.ffn, Q = args.q_width, QKV = args.qkv_width, L = s.n_layers, E = kExperts ? s.n_experts : 0;
   const int slots = E ? s.top_k : 1;
-  if (tid == 0 && pg.count > 0) {      // read behind the attention's barriers
-    sh.four0 = G * (D / 4) * pg.split / pg.live;
-    sh.four1 = G * (D / 4) * (pg.split + 1) / pg.live;
-  }
   const int rbH = row_bytes(kFmt, H), rbQ = row_bytes(kFmt, Q), rbF = row_bytes(kFmt, F);
   int* ids = reinterpret_cast<int*>(base + lay.route + kMaxExperts * 4);
   float* weights = reinterpret_cast<float*>(ids + kMaxTopK);
@@ -1137,6 +1151,7 @@ __global__ void __launch_bounds__(kStepThreads + 32, 1) decode_step(const __grid
       fence_proxy_async();      // the cache rows of the steps before were written with ordinary stores
       Producer p{sh, wait, base + lay.ring, lay.total - lay.ring, lane};
       const int* table = state + VDC_ST_PAGETABLE;
+      const Pages pg = sh.pages;
       // stage after stage; a stage is one run of rows or several (experts), the attention one run per page
       int l = 0, stage = kQkv, sub = 0;
 #pragma unroll 1
@@ -1217,28 +1232,19 @@ __global__ void __launch_bounds__(kStepThreads + 32, 1) decode_step(const __grid
     };
     auto silu = [&](float g, float u) {
       g = bf16_round(g);
-      return bf16_round(g / (1.f + __expf(-g))) * bf16_round(u);
+      return bf16_round(g * reciprocal(1.f + __expf(-g))) * bf16_round(u);
     };
     auto keep_hidden = [&](uint64_t to) {        // SM 0: the hidden state as it came in, for whoever asks
       if (sm == 0 && to && !c.failed())
 #pragma unroll 1
         for (int i = tid; i < H / 2; i += kStepThreads) reinterpret_cast<uint32_t*>(to)[i] = c.hs()[i];
     };
-    const uint8_t* row = nullptr;
-    {
-      int token = ld_relaxed_gpu(state + VDC_ST_TOKEN);
-      if (token < 0 || token >= s.vocab) {
-        if (sm == 0 && tid == 0) report(status, VDC_ERR_TOKEN, VDC_STEP_KIND, 0, 0, token);
-        token = 0;
-      }
-      row = reinterpret_cast<const uint8_t*>(s.embed) + (size_t)token * H * 2;
-    }
-    float best = -INFINITY;
-    int best_row = 0x7fffffff;
+    float best;
+    int best_row;
     // One loop over the layers' stages, with the vocabulary projection as the first stage behind the last layer: each piece of
     // code is there once, since what falls out of the instruction caches between two stages costs as much as the stage.
 #pragma unroll 1
-    for (int l = 0, stage = kQkv; l < L || stage == kQkv;) {
+    for (int l = 0, stage = kQkv;;) {
       asm volatile("" : "+r"(stage), "+r"(l));      // the compiler would otherwise make a copy of the loop for every stage
       const uint32_t tag = tag0 + (uint32_t)l * 8u;
       const bool lm = l == L;
@@ -1272,7 +1278,7 @@ __global__ void __launch_bounds__(kStepThreads + 32, 1) decode_step(const __grid
         skip = !r.n && (lm ? sm != 0 : !sh.plan[kOut].n && (stage == kQkv || !sh.plan[kGateUp].n));
         if (!skip) {
           const uint64_t w = lm ? s.norm_w : (stage == kQkv ? s.ln1 : s.ln2) + (size_t)l * H * 2;
-          c.template hidden<kFmt>(work + wk.h + (stage == kQkv ? H / 2 : 0), stage == kQkv ? tag - 8u + 5u : tag + 4u, l == 0 && stage == kQkv ? row : nullptr, w, lm);
+          c.template hidden<kFmt>(work + wk.h + (stage == kQkv ? H / 2 : 0), stage == kQkv ? tag - 8u + 5u : tag + 4u, l == 0 && stage == kQkv ? reinterpret_cast<const uint8_t*>(s.embed) + (size_t)sh.token * H * 2 : nullptr, w, lm);
           if (stage == kQkv && l > 0 && s.taps) keep_hidden(s.taps + (size_t)(l - 1) * H * 2);
           if (lm) keep_hidden(s.hidden_out);
         }
@@ -1285,6 +1291,10 @@ __global__ void __launch_bounds__(kStepThreads + 32, 1) decode_step(const __grid
         }
       } else if (r.n || sh.plan[kDown].n) {      // kGateUp behind a router: its inputs are there, the experts are not
         c.route(work + wk.router, tag + 7u);
+      }
+      if (lm) {
+        best = -INFINITY;
+        best_row = 0x7fffffff;
       }
       // ---- rows, as many at a time as their partial sums have room for
 #pragma unroll 1
@@ -1360,8 +1370,8 @@ __global__ void __launch_bounds__(kStepThreads + 32, 1) decode_step(const __grid
         if (lm) consumers_sync();
       }
       if (lm) break;
-      if (stage == kQkv && pg.count > 0)
-        c.attention(l, pos, pg, work + wk.qkv, work + wk.rec, work + wk.ml, work + wk.attn, tag + 1u, tag + 2u, tag + 3u);
+      if (stage == kQkv && sh.pages.count > 0)
+        c.attention(l, sh.pos, sh.pages, work + wk.qkv, work + wk.rec, work + wk.ml, work + wk.attn, tag + 1u, tag + 2u, tag + 3u);
       if (stage == kDown) ++l;
       stage = stage == kDown ? kQkv : stage == kOut ? (E ? kRouter : kGateUp) : stage + 1;
     }
@@ -1410,7 +1420,7 @@ __global__ void __launch_bounds__(kStepThreads + 32, 1) decode_step(const __grid
           if (ok && best_row == 0x7fffffff) {         // no logit is a number: no next token, the state stays
             report(status, VDC_ERR_TOKEN, VDC_STEP_KIND, 1, 0, -1);
           } else if (ok && !c.failed() && !ld_relaxed_gpu(&status->abort)) {
-            const int step = st[VDC_ST_STEP], next = pos + 1, page = next / VDC_KV_PAGE;
+            const int step = st[VDC_ST_STEP], next = sh.pos + 1, page = next / VDC_KV_PAGE;
             reinterpret_cast<int*>(s.log)[step] = best_row;
             st[VDC_ST_TOKEN] = best_row;
             st[VDC_ST_STEP] = step + 1;
@@ -1491,7 +1501,7 @@ extern "C" cudaError_t vdc_step_launch(const vdc_step* s, vdc_status* status, ui
   cfg.dynamicSmemBytes = vdc::kStepSmem;
   auto f = s->n_experts ? vdc::decode_step<0, true> : s->wfmt == 0 ? vdc::decode_step<0, false>
            : s->wfmt == 1 ? vdc::decode_step<1, false> : vdc::decode_step<2, false>;
-  vdc::StepArgs args{*s, vdc::step_layout(*s), vdc::step_work(*s), {}};
+  vdc::StepArgs args{*s, vdc::step_layout(*s), vdc::step_work(*s), {}, 1.f / (float)s->hidden, s->n_kv * s->group * VDC_HEAD_DIM, s->n_kv * (s->group + 2) * VDC_HEAD_DIM};
   for (int i = 0; i < vdc::kStages; ++i) args.deal[i] = vdc::deal_of(*s, i);
   return cudaLaunchKernelEx(&cfg, f, args, status, timeout_ns);
 }
