@@ -317,8 +317,9 @@ __device__ __forceinline__ void dot_steps(float (&d)[kFmt == 2 ? 2 : 1][kPairs][
 }
 // Steps of a warp whose loads are on their way together.  With one (and the products in the order of the source) a warp took 290
 // cycles for a step of four bf16 rows, a chain of a load, two products and an addition.  A step of NVFP4 rows is as many products
-// by itself as four of bf16 (four 8B-shaped layers 232 us, 246 with two steps and the registers they spill).
-__host__ __device__ constexpr int steps_of(int fmt) { return fmt == 0 ? 4 : fmt == 1 ? 2 : 1; }
+// by itself as four of bf16 (four 8B-shaped layers 232 us, 246 with two steps and the registers they spill), and so is one of two
+// pairs of e4m3 rows; of one pair four at once (four 8B-shaped layers 237 us with two steps of either, 232.7 so).
+__host__ __device__ constexpr int steps_of(int fmt, int pairs) { return fmt == 0 || (fmt == 1 && pairs == 1) ? 4 : 1; }
 
 // Units of q rows; the first SMs' shares are never empty while there are any.
 __host__ __device__ inline Share share_of(int rows, int q, int sm, int sms) {
@@ -519,7 +520,9 @@ struct Consumer {
     for (int j = 0; j < kBatch; ++j) out[j] = make_uint2((uint32_t)v[j].a, (uint32_t)v[j].b);
     return true;
   }
-  // n 2-byte values (a multiple of 4) of an entry buffer: f(i, values 4i .. 4i + 3 as two words) for this thread's i.
+  // n 2-byte values (a multiple of 4) of an entry buffer: f(i, values 4i .. 4i + 3 as two words) for this thread's i.  As many at a
+  // time as registers allow: with 14 of them for a down projection's inputs instead of two times 7 values were spilled and eight
+  // 8B-shaped layers took 865 instead of 813 us, with four 799.
   template <int kBatch, class F>
   __device__ __forceinline__ void collect(const uint64_t* buf, int n, uint32_t tag, F f) const {
 #pragma unroll 1
@@ -552,29 +555,29 @@ struct Consumer {
   }
   // The hidden state (entries, or a row of the embedding table) into shared memory and, RMS-normalised with the weights w,
   // into the input vector.  Rounded like a bf16 tensor expression.
-  template <int kFmt>
+  template <int kFmt, int kKept>
   __device__ __forceinline__ void hidden(const uint64_t* buf, uint32_t tag, const uint8_t* row, uint64_t w, bool plain) const {
     const int H = s.hidden;
-    constexpr int kMost = 8, kHalf = kMost / 2;                   // hidden <= 8192; its first half stays in registers
-    uint2 v[kHalf];
+    constexpr int kMost = 8;                                      // hidden <= 8192; the first kKept stay in registers
+    uint2 v[kKept];
     // The weights are on their way while the entries are waited for, to the places of the inputs that they make.  The last stage's
     // inputs there have been read: its partial sums are complete.
 #pragma unroll 2
     for (int i = tid; i < H / 4; i += kStepThreads) copy8_async(x() + input_at<kFmt>(i, plain), w + (size_t)i * 8);
     float ssq = 0.f;
 #pragma unroll 1
-    for (int j0 = kHalf * (H > kHalf * 4 * kStepThreads); j0 >= 0; j0 -= kHalf) {
+    for (int j0 = (H / 4 - 1) / kStepThreads / kKept * kKept; j0 >= 0; j0 -= kKept) {
       if (row != nullptr) {
 #pragma unroll
-        for (int j = 0; j < kHalf; ++j) {
+        for (int j = 0; j < kKept; ++j) {
           const int i = tid + (j0 + j) * kStepThreads;
           if (i < H / 4) v[j] = __ldg(reinterpret_cast<const uint2*>(row) + i);
         }
-      } else if (!take<kHalf>(buf, H / 4, j0, tag, v)) {
+      } else if (!take<kKept>(buf, H / 4, j0, tag, v)) {
         break;
       }
 #pragma unroll
-      for (int j = 0; j < kHalf; ++j) {
+      for (int j = 0; j < kKept; ++j) {
         const int i = tid + (j0 + j) * kStepThreads;
         if (i < H / 4) {
           const uint32_t a = v[j].x, b = v[j].y;
@@ -597,9 +600,9 @@ struct Consumer {
 #pragma unroll
     for (int j = 0; j < kMost; ++j) {
       const int i = tid + j * kStepThreads;
-      if (j == kHalf && H <= kHalf * 4 * kStepThreads) break;
+      if (j >= kKept && H <= j * 4 * kStepThreads) break;
       if (i < H / 4) {
-        const uint2 h = j < kHalf ? v[j < kHalf ? j : 0] : *reinterpret_cast<const uint2*>(hs() + 2 * i);
+        const uint2 h = j < kKept ? v[j < kKept ? j : 0] : *reinterpret_cast<const uint2*>(hs() + 2 * i);
         const uint2 wv = *reinterpret_cast<const uint2*>(x() + input_at<kFmt>(i, plain));
         set_input<kFmt>(i, scaled(h.x, rstd, wv.x), scaled(h.y, rstd, wv.y), plain);
       }
@@ -675,7 +678,7 @@ struct Consumer {
 #pragma unroll
           for (int i = 0; i < 4; ++i) off[i] = min(i, nr - 1) * nu * 512;
           const uint8_t* xs = xp + u0 * (unit_of(kFmt) * 2);
-          walk<steps_of(kFmt)>(warp & 3, 4, nu, [&](auto steps, int u) { dot_steps<kFmt, 2, decltype(steps)::value>(d, w, off, false, xs, u, 4, lane, 0); });
+          walk<steps_of(kFmt, 2)>(warp & 3, 4, nu, [&](auto steps, int u) { dot_steps<kFmt, 2, decltype(steps)::value>(d, w, off, false, xs, u, 4, lane, 0); });
           // the place's next bytes come through the other proxy, and nothing that depends on these reads is stored before
           fence_proxy_async_smem();
         }
@@ -722,12 +725,12 @@ struct Consumer {
           a = d[0].x + d[0].y; b = d[1].x + d[1].y;
         } else if (r + 2 * rw < nr) {
           float d[kFmt == 2 ? 2 : 1][2][4] = {};
-          walk<steps_of(kFmt)>(kg, kw, units, [&](auto steps, int u) { dot_steps<kFmt, 2, decltype(steps)::value>(d, w, off, false, xp, u, kw, lane, K); });
+          walk<steps_of(kFmt, 2)>(kg, kw, units, [&](auto steps, int u) { dot_steps<kFmt, 2, decltype(steps)::value>(d, w, off, false, xp, u, kw, lane, K); });
           diagonal<kFmt, 2>(d, 0, a, b);
           diagonal<kFmt, 2>(d, 1, c, e);
         } else {
           float d[kFmt == 2 ? 2 : 1][1][4] = {};
-          walk<steps_of(kFmt)>(kg, kw, units, [&](auto steps, int u) { dot_steps<kFmt, 1, decltype(steps)::value>(d, w, off, r + rw >= nr, xp, u, kw, lane, K); });
+          walk<steps_of(kFmt, 1)>(kg, kw, units, [&](auto steps, int u) { dot_steps<kFmt, 1, decltype(steps)::value>(d, w, off, r + rw >= nr, xp, u, kw, lane, K); });
           diagonal<kFmt, 1>(d, 0, a, b);
         }
         const float v = sum_lanes(a, b, c, e);
@@ -1278,14 +1281,14 @@ __global__ void __launch_bounds__(kStepThreads + 32, 1) decode_step(const __grid
         skip = !r.n && (lm ? sm != 0 : !sh.plan[kOut].n && (stage == kQkv || !sh.plan[kGateUp].n));
         if (!skip) {
           const uint64_t w = lm ? s.norm_w : (stage == kQkv ? s.ln1 : s.ln2) + (size_t)l * H * 2;
-          c.template hidden<kFmt>(work + wk.h + (stage == kQkv ? H / 2 : 0), stage == kQkv ? tag - 8u + 5u : tag + 4u, l == 0 && stage == kQkv ? reinterpret_cast<const uint8_t*>(s.embed) + (size_t)sh.token * H * 2 : nullptr, w, lm);
+          c.template hidden<kFmt, kExperts ? 4 : 2>(work + wk.h + (stage == kQkv ? H / 2 : 0), stage == kQkv ? tag - 8u + 5u : tag + 4u, l == 0 && stage == kQkv ? reinterpret_cast<const uint8_t*>(s.embed) + (size_t)sh.token * H * 2 : nullptr, w, lm);
           if (stage == kQkv && l > 0 && s.taps) keep_hidden(s.taps + (size_t)(l - 1) * H * 2);
           if (lm) keep_hidden(s.hidden_out);
         }
       } else if (stage == kOut || stage == kDown) {
         skip = !r.n;
         if (!skip) {
-          c.template collect<7>(work + (stage == kOut ? wk.attn : wk.act), stage == kOut ? Q : F * slots, tag + (stage == kOut ? 3u : 6u),
+          c.template collect<kExperts ? 7 : 4>(work + (stage == kOut ? wk.attn : wk.act), stage == kOut ? Q : F * slots, tag + (stage == kOut ? 3u : 6u),
                     [&](int i, uint32_t a, uint32_t b) { c.template set_input<kFmt>(i, a, b, false); });
           consumers_sync();
         }
