@@ -244,3 +244,36 @@ def test_sums_lose_no_more_bits_than_fp32_fmas(cuda_device, wkind):
                        for got, want in ((v, torch.stack(exact_v)), (eng.logits, exact_l))])
     for a, b in zip(*missed):
         assert a <= b + 5 * (a + b) ** 0.5, missed
+
+
+# rows of which four make more than a copy: K of 18, 32, 33 and 56 steps, groups that end with two rows; an SM's gate/up rows too many
+# for the sums of slices (542 of 4608 inputs); the vocabulary projection of quantised models
+SLICED = [
+    (dict(hidden=8192, n_heads=64, n_kv_heads=8, ffn=8448, vocab=1002, n_layers=1), (70,), None),
+    (dict(hidden=4608, n_heads=32, n_kv_heads=8, ffn=4608, vocab=700, n_layers=2), (64,), 17),
+    (dict(hidden=4096, n_heads=32, n_kv_heads=8, ffn=14336, vocab=512, n_layers=1), (130,), 132),
+    (dict(hidden=8192, n_heads=64, n_kv_heads=8, ffn=14336, vocab=1000, n_layers=1, wkind="fp8"), (70,), None),
+    (dict(hidden=8192, n_heads=64, n_kv_heads=8, ffn=1024, vocab=4098, n_layers=1, wkind="nvfp4"), (70,), None)]
+
+
+@pytest.mark.parametrize("kw,positions,num_sms", SLICED)
+def test_rows_that_come_in_slices(cuda_device, kw, positions, num_sms):
+    test_step_kernel_against_the_megakernels_program(cuda_device, kw, positions, num_sms)
+
+
+def test_of_equal_experts_the_lowest_are_chosen(cuda_device):
+    """Router rows that are copies of one another give equal logits; two rows are the others' negative, so either all that are not
+    chosen last or the first two."""
+    eng = _engine(cuda_device, 128, hidden=512, n_heads=8, n_kv_heads=2, ffn=256, vocab=512, n_layers=1, n_experts=96, top_k=6)
+    row = eng.router[0][0].clone()
+    for odd in ((), (3, 64), (40, 95)):
+        eng.router[0].copy_(row)
+        for i in odd:
+            eng.router[0][i].neg_()
+        eng.set_state(70, 5)
+        eng.generate(1)
+        ids, weights = eng.route[:6].tolist(), eng.route[16:22].view(torch.float32)
+        rest = [i for i in range(96) if i not in odd]
+        assert ids in (rest[:6], list(odd) + rest[:6 - len(odd)])
+        if ids == rest[:6]:
+            assert torch.equal(weights, torch.full_like(weights, 1 / 6).to(torch.bfloat16).float())

@@ -162,3 +162,28 @@ def test_a_wait_that_runs_out_ends_with_an_error(cuda_device, fmt):
             continue
         want = out.clone() if want is None else want
         assert torch.equal(out, want)
+
+
+@pytest.mark.parametrize("K,splits", [(512, 0), (4096, 1), (4096, 3), (5120, 2), (8192, 8)])
+def test_norm_of_a_prompts_rows(cuda_device, K, splits):
+    """Fewer pieces than threads, as many as stay in registers, more than those: the hidden state is the bf16 sum to the bit, its
+    norm two bf16 roundings (2^-9 each) from fp32's."""
+    from vdcores_b200 import isa, runtime
+    dev, R = cuda_device, 128
+    h, parts, w = seeded((R, K), 4).to(BF16).to(dev), seeded((max(splits, 1), R, K), 5).float().to(dev), (1 + 0.1 * seeded((K,), 6).float()).to(BF16).to(dev)
+    hd, out = _rows(h), torch.zeros(R * K, dtype=BF16, device=dev)
+    x = parts.permute(0, 2, 1).reshape(max(splits, 1), K // 4, 4, R).transpose(2, 3).contiguous()
+    s = runtime.Stage(kind=isa.STAGE_WIDE_NORM, Bpad=R, K=K, hid=hd.data_ptr(), out=out.data_ptr(), norm_w=w.data_ptr(), eps=1e-5,
+                      x=x.data_ptr() if splits else 0, splits=max(splits, 1))
+    stream = torch.cuda.current_stream(dev).cuda_stream
+    runtime.launch_stages((runtime.Stage * 1)(s), stream, 500_000_000)
+    runtime.read_status(stream)
+    want = h
+    if splits:
+        total = parts[0].clone()
+        for p in parts[1:]:
+            total += p
+        want = (h.float() + total.to(BF16).float()).to(BF16)
+    assert torch.equal(hd, _rows(want))
+    norm = want.double() * torch.rsqrt(want.double().pow(2).mean(1, keepdim=True) + 1e-5) * w.double()
+    assert rel(out.double(), _rows(norm.to(BF16)).double()) < 2 * 2.0 ** -9

@@ -2,7 +2,9 @@
 //
 // A step of 2..128 rows runs, per layer: QKV projection (with per-head norm, rotation and the cache append in its
 // epilogue), attention, output projection, gate/up projection, down projection.  The rows sit on the 128 lanes of a
-// tcgen05 accumulator, a block of 128 weight rows on its columns.  Why kernels and not tasks of the megakernel: with
+// tcgen05 accumulator, a block of 128 weight rows on its columns; with quantised weights, which are widened into tensor
+// memory as the A operand, it is the other way round: 32 rows took 68 KB of shared-memory traffic per 8 KB of e4m3 weights
+// when they were widened into shared memory, 24 KB so (two layers 321.5 -> 303.4 us).  Why kernels and not tasks of the megakernel: with
 // many rows a projection block needs a K-split whose partial sums meet (here through distributed shared memory inside
 // one cluster, in the megakernel through fp32 atomics in L2 and a last arrival that ran the block's epilogue alone), and
 // a stage boundary needs no spinning: programmatic dependent launch starts the next kernel's CTAs while this one drains,
@@ -10,8 +12,8 @@
 // 128256-row vocabulary projection at 3 rows).
 //
 // Measured against the megakernel's program, two Llama-3.1-8B-shaped layers and a small vocabulary (B200): 3 rows at
-// 1000 positions 416 -> 247 us, 32 rows with e4m3 weights 759 -> 336, 64 rows at 2100 positions 929 -> 427, 128 rows
-// 1024 -> 405 (up to 4 % less from one GPU to another).
+// 1000 positions 416 -> 235 us, 32 rows with e4m3 weights 759 -> 283, 64 rows at 2100 positions 929 -> 402, 128 rows
+// 1024 -> 397 (up to 4 % more or less from one GPU to another).
 #include "mk_stage.cuh"
 
 namespace vdc {
@@ -112,8 +114,8 @@ __global__ void __launch_bounds__(kGemmThreads, 2) stage_gemm(const __grid_const
   const int stage_bytes = stage_size(kFmt, s.Bpad);
   // Quantised weights are converted by two teams of warps that take the chunks in turn where the ring's length is even, so
   // that a team sees every round of its stages; by all warps together where it is not (a team would then meet a stage two
-  // rounds on, and the barrier's parity cannot tell those apart).  Teams, because a team's wait for the tensor cores to
-  // leave its staging buffer then falls into the other's conversion: e4m3 gate/up at 32 rows 74.7 -> 65.6 us.
+  // rounds on, and the barrier's parity cannot tell those apart).  Teams, because a team's waits then fall into the other's
+  // conversion.
   const int teams = n_ring & 1 ? 1 : 2;
   uint8_t* ring = aligned128(dyn);
   const Waiter wait{&sh.fail, status, timeout_ns, s.kind};

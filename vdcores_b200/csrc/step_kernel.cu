@@ -19,8 +19,8 @@
 
 namespace vdc {
 
-// Consumer warps; one more warp produces.  All of them execute what a stage's boundary needs, each an instruction every ten
-// cycles (it waits for entries in L2, and for the instruction before): eight warps, not sixteen, which took 515 us for four
+// Consumer warps; one more warp produces.  All of them execute what a stage's boundary needs, and wait for entries in L2 and for the
+// instruction before: eight warps, not sixteen, which took 515 us for four
 // 8B-shaped layers where eight took 451.
 constexpr int kStepWarps = 8;
 constexpr int kStepThreads = 32 * kStepWarps;
@@ -348,8 +348,8 @@ __host__ __device__ inline Split split_of(int fmt, bool experts, bool vocab, int
   if (fmt == 0 && !experts && steps > most && n >= 4 && (vocab || n <= kPartFloats / kStepWarps)) return {2, kStepWarps, most};
   const int units = K / unit_of(fmt), chunks = n / chunk_rows(row_bytes(fmt, K));
   // Two teams, since a chunk's place in the ring is held for as long as its team works on it; four where there is more work per
-  // byte.  Four 8B-shaped layers with 1 / 2 / 4 teams: bf16 459 / 447 / 456 us, e4m3 358 / 328 / 335, NVFP4 348 / 339 / 334,
-  // the 30B mixture of experts 273 / 261 / 260.
+  // byte.  With 2 / 4 teams: eight 8B-shaped bf16 layers 813 / 819 us, four e4m3 244 / 253, NVFP4 236 / 231, the 30B mixture of
+  // experts 211 / 209.5.
   const bool four = fmt == 2 || experts;
   Split s{four && chunks >= 4 ? 4 : chunks >= 2 ? 2 : 1, 1, 0};
   while (s.kw < kStepWarps / s.teams && 2 * s.kw <= units) s.kw *= 2;
@@ -1127,12 +1127,15 @@ __global__ void __launch_bounds__(kStepThreads + 32, 1) decode_step(const __grid
   const uint32_t launches = (uint32_t)ld_acquire_gpu(reinterpret_cast<const int*>(s.work));
   const int* state = reinterpret_cast<const int*>(s.state);
   const int aborted = ld_relaxed_gpu(&status->abort);
+  int id = 0;
+  bool wrong = false;
   if (tid == 0) {
     const int pos = ld_relaxed_gpu(state + VDC_ST_POS), token = ld_relaxed_gpu(state + VDC_ST_TOKEN);
     sh.new_row = ld_relaxed_gpu(state + VDC_ST_NEWROW);
     sh.pos = pos;
     sh.token = token < 0 || token >= s.vocab ? 0 : token;
-    if (sh.token != token && sm == 0 && !aborted) report(status, VDC_ERR_TOKEN, VDC_STEP_KIND, 0, 0, token);
+    wrong = sh.token != token;
+    id = token;
     const Pages pg = pages_of(s, pos, sm);
     sh.pages = pg;
     sh.four0 = s.group * (D / 4) * pg.split / pg.live;
@@ -1142,6 +1145,7 @@ __global__ void __launch_bounds__(kStepThreads + 32, 1) decode_step(const __grid
     if (sm == 0 && tid == 0) red_release_gpu_add(reinterpret_cast<int*>(s.work), 1);
     return;
   }
+  if (wrong && sm == 0) report(status, VDC_ERR_TOKEN, VDC_STEP_KIND, 0, 0, id);
 
   const int H = s.hidden, F = s.ffn, Q = args.q_width, QKV = args.qkv_width, L = s.n_layers, E = kExperts ? s.n_experts : 0;
   const int slots = E ? s.top_k : 1;

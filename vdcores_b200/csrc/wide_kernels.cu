@@ -172,8 +172,8 @@ __global__ void __launch_bounds__(kWideThreads, 1) wide_gemm(const __grid_consta
         const int slot0 = per == 2 ? 0 : j & 1;
         for (int c = 0; c < t.n_ch; ++c, ++it, at.next()) {
           const int st = at.st;
+          // widened weights stand for the chunk's arrival too: the warps that widened them have seen it
           ok = wait(kFmt != 0 ? &sh.ready[st] : &sh.full[st], at.parity, 1, it);
-          if (kFmt != 0 && ok) ok = wait(&sh.full[st], at.parity, 1, it);
           if (!ok) break;
           if (c == 0) {
 #pragma unroll
@@ -319,45 +319,52 @@ __global__ void __launch_bounds__(128) wide_embed(const __grid_constant__ vdc_st
 }
 
 // hid += the projection's sums (x; 0: none), then (out) its RMSNorm, both rounded like a bf16 tensor expression.  Two rows per
-// block: the two share the 32-byte sectors of the matrix; 256 threads each, so that few rows are many loads at a time.
+// block: the two share the 32-byte sectors of the matrix; 256 threads each, so that few rows are many loads at a time.  A row's
+// first kKept pieces of a thread stay in registers between the sum of squares and the products, and their norm weights are on
+// their way while the projection ends: 600 rows of two 8B-shaped layers NVFP4 1012 -> 996 us, e4m3 1034 -> 1022.
 constexpr int kNormThreads = 512;
-__global__ void __launch_bounds__(kNormThreads) wide_norm(const __grid_constant__ vdc_stage s, vdc_status* status) {
-  constexpr int kStep = kNormThreads / 2, kBatch = 2;
+__global__ void __launch_bounds__(kNormThreads, 2) wide_norm(const __grid_constant__ vdc_stage s, vdc_status* status) {
+  constexpr int kStep = kNormThreads / 2, kKept = 2;
   __shared__ float red[kNormThreads / 32][2];
-  const int tid = threadIdx.x, r = tid & 1, b = (int)blockIdx.x * 2 + r;
+  const int tid = threadIdx.x, r = tid & 1, b = (int)blockIdx.x * 2 + r, t = tid >> 1, pieces = s.K / 8;
   const size_t sub = (size_t)(b / 128) * 128 * s.K * 2;
   uint8_t* hid = reinterpret_cast<uint8_t*>(s.hid) + sub;
+  const uint4 none = make_uint4(0u, 0u, 0u, 0u);
+  uint4 kept[kKept], w[kKept];
+#pragma unroll
+  for (int q = 0; q < kKept; ++q)
+    w[q] = s.out && t + q * kStep < pieces ? __ldg(reinterpret_cast<const uint4*>(s.norm_w) + t + q * kStep) : none;
   grid_dep_wait();
   grid_dep_launch();
   const int aborted = ld_relaxed_gpu(&status->abort);
   float ssq = 0.f;
   const float4* sums = reinterpret_cast<const float4*>(s.x) + b;
   const size_t split = (size_t)(s.K >> 2) * s.Bpad;
-  for (int k0 = tid >> 1; k0 < s.K / 8; k0 += kBatch * kStep) {
-    uint4 h[kBatch];
-    float4 y[kBatch][2];
+  // kKept pieces from k0 on: the hidden state with the sums added, its squares
+  auto add = [&](int k0, uint4 (&h)[kKept]) {
+    float4 y[kKept][2];
 #pragma unroll
-    for (int q = 0; q < kBatch; ++q) {
+    for (int q = 0; q < kKept; ++q) {
       const int k8 = k0 + q * kStep;
-      h[q] = k8 < s.K / 8 ? __ldcg(reinterpret_cast<const uint4*>(hid + kc_piece(128, b % 128, k8 * 8))) : make_uint4(0u, 0u, 0u, 0u);
+      h[q] = k8 < pieces ? __ldcg(reinterpret_cast<const uint4*>(hid + kc_piece(128, b % 128, k8 * 8))) : none;
       y[q][0] = y[q][1] = make_float4(0.f, 0.f, 0.f, 0.f);
     }
     if (s.x) {
 #pragma unroll 4
       for (int i = 0; i < s.splits; ++i)
 #pragma unroll
-        for (int q = 0; q < kBatch; ++q)
+        for (int q = 0; q < kKept; ++q)
 #pragma unroll
           for (int e = 0; e < 2; ++e) {
             const int k8 = k0 + q * kStep;
-            const float4 v = k8 < s.K / 8 ? __ldcg(sums + i * split + (size_t)(2 * k8 + e) * s.Bpad) : make_float4(0.f, 0.f, 0.f, 0.f);
+            const float4 v = k8 < pieces ? __ldcg(sums + i * split + (size_t)(2 * k8 + e) * s.Bpad) : make_float4(0.f, 0.f, 0.f, 0.f);
             y[q][e].x += v.x; y[q][e].y += v.y; y[q][e].z += v.z; y[q][e].w += v.w;
           }
     }
 #pragma unroll
-    for (int q = 0; q < kBatch; ++q) {
+    for (int q = 0; q < kKept; ++q) {
       const int k8 = k0 + q * kStep;
-      if (k8 >= s.K / 8) break;
+      if (k8 >= pieces) break;
       const uint32_t hv[4] = {h[q].x, h[q].y, h[q].z, h[q].w};
       const float yv[8] = {y[q][0].x, y[q][0].y, y[q][0].z, y[q][0].w, y[q][1].x, y[q][1].y, y[q][1].z, y[q][1].w};
       float v[8];
@@ -369,11 +376,17 @@ __global__ void __launch_bounds__(kNormThreads) wide_norm(const __grid_constant_
       if (s.x) {
 #pragma unroll
         for (int j = 0; j < 8; ++j) v[j] = bf16_round(v[j] + bf16_round(yv[j]));
-        if (!aborted) *reinterpret_cast<uint4*>(hid + kc_piece(128, b % 128, k8 * 8)) = pack8(v);
+        h[q] = pack8(v);
+        if (!aborted) *reinterpret_cast<uint4*>(hid + kc_piece(128, b % 128, k8 * 8)) = h[q];
       }
 #pragma unroll
       for (int j = 0; j < 8; ++j) ssq = fmaf(v[j], v[j], ssq);
     }
+  };
+  add(t, kept);
+  for (int k0 = t + kKept * kStep; k0 < pieces; k0 += kKept * kStep) {
+    uint4 h[kKept];
+    add(k0, h);
   }
   if (!s.out || __syncthreads_or(aborted)) return;
 #pragma unroll
@@ -382,18 +395,21 @@ __global__ void __launch_bounds__(kNormThreads) wide_norm(const __grid_constant_
   __syncthreads();
   float sum = 0.f;
 #pragma unroll
-  for (int w = 0; w < kNormThreads / 32; ++w) sum += red[w][r];
+  for (int i = 0; i < kNormThreads / 32; ++i) sum += red[i][r];
   const float rstd = rsqrtf(sum / (float)s.K + s.eps);
-  for (int k8 = tid >> 1; k8 < s.K / 8; k8 += kStep) {
-    const size_t at = kc_piece(128, b % 128, k8 * 8);
-    const uint4 h = ldcg128(hid + at), w = __ldg(reinterpret_cast<const uint4*>(s.norm_w) + k8);
+  auto scale = [&](int k8, const uint4& h, const uint4& w) {
     const uint32_t hv[4] = {h.x, h.y, h.z, h.w}, wv[4] = {w.x, w.y, w.z, w.w};
     uint32_t o[4];
 #pragma unroll
     for (int j = 0; j < 4; ++j)
       o[j] = pack_bf16x2(bf16_round(bf_lo(hv[j]) * rstd) * bf_lo(wv[j]), bf16_round(bf_hi(hv[j]) * rstd) * bf_hi(wv[j]));
-    *reinterpret_cast<uint4*>(reinterpret_cast<uint8_t*>(s.out) + sub + at) = make_uint4(o[0], o[1], o[2], o[3]);
-  }
+    *reinterpret_cast<uint4*>(reinterpret_cast<uint8_t*>(s.out) + sub + kc_piece(128, b % 128, k8 * 8)) = make_uint4(o[0], o[1], o[2], o[3]);
+  };
+#pragma unroll
+  for (int q = 0; q < kKept; ++q)
+    if (t + q * kStep < pieces) scale(t + q * kStep, kept[q], w[q]);
+  for (int k8 = t + kKept * kStep; k8 < pieces; k8 += kStep)
+    scale(k8, ldcg128(hid + kc_piece(128, b % 128, k8 * 8)), __ldg(reinterpret_cast<const uint4*>(s.norm_w) + k8));
 }
 
 // Heads of the QKV projection's sums, eight rows to a block and a warp to a row: q/k norm, rotation, query rows and cache
