@@ -206,23 +206,3 @@ def test_slices_of_a_limited_launch(limit):
         launches, largest = runtime.count_stage_launches(st, limit)
         per = limit // splits
         assert launches == -(-units // per) and largest == min(units, per) * splits <= limit
-
-
-def test_split_codes_select_the_bytes_of_bf16_numbers():
-    """The halves of an e2m1 code, as the packed blocks hold them, pick two bytes that are 2^-126 of its value."""
-    from vdcores_b200.batch import split_codes
-    codes = torch.randint(0, 256, (3, 5, 8), dtype=torch.uint8, generator=torch.Generator().manual_seed(3))
-    words = split_codes(codes).reshape(-1, 4).to(torch.int64)
-    words = words[:, 0] | words[:, 1] << 8 | words[:, 2] << 16 | words[:, 3] << 24
-    table = torch.tensor([0x00, 0x01, 0x80, 0x81, 0x00, 0x40, 0x80, 0xC0])
-    got = []
-    for i in range(2):
-        sel = (words >> (2 * i)) & 0x33333333 | 0x04040404
-        nibbles = torch.stack([(sel >> (4 * n)) & 7 for n in range(8)], 1)
-        lo, hi = table[nibbles[:, 0::2]], table[nibbles[:, 1::2]]
-        got.append((lo | hi << 8).to(torch.int32).bitwise_left_shift(16).view(torch.float32))
-    got = torch.cat(got, 1).double() * 2.0 ** 126
-    grid = torch.tensor([0.0, 0.5, 1.0, 1.5, 2.0, 3.0, 4.0, 6.0])
-    grid = torch.cat((grid, -grid)).double()
-    w = codes.reshape(-1, 4).long()
-    assert torch.equal(got, grid[torch.stack((w & 15, w >> 4), -1).reshape(-1, 8)])

@@ -70,25 +70,12 @@ def pack_blocks_fp8(codes: torch.Tensor, rows: int = BLOCK_ROWS) -> torch.Tensor
                         M, K, torch.empty(M * K, dtype=codes.dtype, device=codes.device), rows)
 
 
-def split_codes(codes: torch.Tensor) -> torch.Tensor:
-    """Bytes of e2m1 pairs, words of eight codes: byte j of a word becomes [upper halves of codes j + 4, j | lower halves of
-    codes j + 4, j], two bits each.  A half selects one byte of a bf16 number, so that a byte permutation with the word (and with
-    the word two bits on) as its selector widens four codes."""
-    w = codes.reshape(-1, 4)
-    c = torch.stack((w & 15, w >> 4), -1).view(-1, 8)
-    a, b = c[:, :4], c[:, 4:]
-    return ((a & 3) | (b & 3) << 2 | (a >> 2) << 4 | (b >> 2) << 6).view(codes.shape)
-
-
 def pack_blocks_nvfp4(w: torch.Tensor, K: int, rows: int = BLOCK_ROWS) -> torch.Tensor:
     """[M, K/2 + K/16] NVFP4 rows (e2m1 pairs, then the e4m3 block scales) -> flat: per block of `rows` rows
     and per 16 inputs, the rows' 8 code bytes followed by the rows' scale bytes ([K/16][N x 8 | N]), so that
-    any K-range of a block is one contiguous piece of 9 N bytes per 16 inputs.  In the stage kernels' blocks a word's eight
-    codes lie as the widening selects them (split_codes)."""
+    any K-range of a block is one contiguous piece of 9 N bytes per 16 inputs."""
     M = w.shape[0]
     codes, bs = w[:, :K // 2].reshape(M, K // 16, 8), w[:, K // 2:]
-    if rows == isa.STAGE_BLOCK:
-        codes = split_codes(codes)
 
     def rows_of(r0, nb, n):
         c = codes[r0:r0 + nb * n].reshape(nb, n, K // 16, 8).transpose(1, 2).reshape(nb, K // 16, n * 8)

@@ -139,11 +139,8 @@ __device__ __forceinline__ void scale8(float (&v)[8], const float* sc) {
 // Bytes of a chunk of n weight rows x 64 inputs as stored: bf16, e4m3, or e2m1 pairs with one e4m3 scale per 16.
 __host__ __device__ constexpr int chunk_bytes(int wfmt, int n) { return wfmt == 0 ? n * 128 : wfmt == 1 ? n * 64 : n * 36; }
 
-// What a sum of products with widened weights is to be multiplied by.
-template <int kFmt>
-constexpr float kNarrowUnit = kFmt == 2 ? 0x1p26f : 1.f;
 // 16 weights of a row (inputs 16 g16 .. + 15 of a chunk of N rows) as stored, and as bf16 (exact for e4m3 and for e2m1 code times
-// block scale), divided by kNarrowUnit.
+// block scale).
 template <int kFmt>
 struct Narrow {
   uint32_t v[kFmt == 1 ? 4 : 2], scale;
@@ -167,25 +164,20 @@ struct Narrow {
         o[2 * j + 1] = pack_bf16x2(hi.x, hi.y);
       }
     } else {
-      // A code's upper two bits (sign, exponent) select the upper byte of its bf16 number, the lower two (exponent, mantissa) the
-      // lower byte: 2^-126 of its value, which the block's scale times 2^100 makes 2^-26 (kNarrowUnit) of the weight, exactly.
-      // Nine integer instructions for eight codes; by way of f16 and fp32 they are four conversions of a quarter, eight of half
-      // and four of half a pipe's rate.
+      // Conversions of a quarter (e2m1) and half of a pipe's rate.  Nine integer instructions for eight codes instead (byte
+      // permutations whose selectors the packed codes are) are slower: two layers of 16 rows 291 us, 304 with those.
       const __half_raw hr = __nv_cvt_fp8_to_halfraw((__nv_fp8_storage_t)scale, __NV_E4M3);
-      const __nv_bfloat162 sc = __float2bfloat162_rn(__half2float(*reinterpret_cast<const __half*>(&hr)) * 0x1p100f);
+      const __half2 sc = __half2half2(*reinterpret_cast<const __half*>(&hr));
 #pragma unroll
-      for (int j = 0; j < 2; ++j)
+      for (int j = 0; j < 2; ++j) {
+        uint32_t h[4];
+        e2m1x8_to_half2(v[j], h);
 #pragma unroll
-        for (int i = 0; i < 2; ++i) {
-          const uint32_t sel = ((v[j] >> (2 * i)) & 0x33333333u) | 0x04040404u;
-#pragma unroll
-          for (int e = 0; e < 2; ++e) {
-            uint32_t w;      // of the selector's nibbles the lower four count, none of them above 7
-            asm("prmt.b32 %0, %1, %2, %3;" : "=r"(w) : "r"(0x81800100u), "r"(0xC0804000u), "r"(sel >> (16 * e)));
-            const __nv_bfloat162 p = __hmul2(*reinterpret_cast<const __nv_bfloat162*>(&w), sc);
-            o[4 * j + 2 * i + e] = *reinterpret_cast<const uint32_t*>(&p);
-          }
+        for (int i = 0; i < 4; ++i) {
+          const float2 f = __half22float2(__hmul2(*reinterpret_cast<const __half2*>(&h[i]), sc));
+          o[4 * j + i] = pack_bf16x2(f.x, f.y);
         }
+      }
     }
   }
 };

@@ -275,7 +275,6 @@ __global__ void __launch_bounds__(kGemmThreads, 2) stage_gemm(const __grid_const
 #pragma unroll
           for (int j = 0; j < 16; ++j) {
             const int row = g * 16 + j;
-            r[j] = __float_as_uint(__uint_as_float(r[j]) * kNarrowUnit<kFmt>);
             const uint32_t at = tile_at(tile, rank, nb, n >> 2, row & (nb - 1)) + (uint32_t)(n & 3) * 4u;
             if (splits > 1) st_cluster1(peer_smem(at, (uint32_t)(row >> lg)), r[j]);
             else st_shared1(at, r[j]);

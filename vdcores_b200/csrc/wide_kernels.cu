@@ -260,8 +260,6 @@ __global__ void __launch_bounds__(kWideThreads, 1) wide_gemm(const __grid_consta
 #pragma unroll
           for (int e = 0; e < 4; ++e) {
             const float4 sc = __ldg(reinterpret_cast<const float4*>(scales + col) + e);
-#pragma unroll
-            for (int j = 0; j < 4; ++j) v[4 * e + j] *= kNarrowUnit<kFmt>;
             v[4 * e] *= sc.x; v[4 * e + 1] *= sc.y; v[4 * e + 2] *= sc.z; v[4 * e + 3] *= sc.w;
           }
         }
