@@ -342,15 +342,18 @@ __host__ __device__ constexpr int chunk_rows(int rb) {        // an even number 
 struct Split {
   int teams, kw, slice;
 };
+// Two teams, since a chunk's place in the ring is held for as long as its team works on it; four where there is more work per byte.
+// With 2 / 4 teams: eight 8B-shaped bf16 layers 813 / 819 us, four e4m3 244 / 253, NVFP4 236 / 231, the 30B mixture of experts 211 /
+// 209.5.
+__host__ __device__ inline int teams_of(int fmt, bool experts, int K, int n) {
+  const int chunks = n / chunk_rows(row_bytes(fmt, K));
+  return (fmt == 2 || experts) && chunks >= 4 ? 4 : chunks >= 2 ? 2 : 1;
+}
 __host__ __device__ inline Split split_of(int fmt, bool experts, bool vocab, int K, int n) {
   const int steps = K / unit_of(fmt), most = kItemBytes / (4 * 512);
   if (fmt == 0 && !experts && steps > most && n >= 4 && (vocab || n <= kPartFloats / kStepWarps)) return {2, kStepWarps, most};
-  const int units = K / unit_of(fmt), chunks = n / chunk_rows(row_bytes(fmt, K));
-  // Two teams, since a chunk's place in the ring is held for as long as its team works on it; four where there is more work per
-  // byte.  With 2 / 4 teams: eight 8B-shaped bf16 layers 813 / 819 us, four e4m3 244 / 253, NVFP4 236 / 231, the 30B mixture of
-  // experts 211 / 209.5.
-  const bool four = fmt == 2 || experts;
-  Split s{four && chunks >= 4 ? 4 : chunks >= 2 ? 2 : 1, 1, 0};
+  const int units = K / unit_of(fmt);
+  Split s{teams_of(fmt, experts, K, n), 1, 0};
   // Along the inputs only as far as a warp would otherwise have fewer than four rows of a chunk: the sums over its lanes come once
   // per four rows, whatever the inputs.  With the inputs divided as far as possible four 8B-shaped e4m3 layers took 232.6 us, 228.8 so,
   // NVFP4 229.9 and 225.4, the mixture of experts 208.8 and 201.
@@ -1469,9 +1472,14 @@ extern "C" const char* vdc_step_refuses(const vdc_step* s, bool pointers) {
   if (l.total - l.ring < 3 * kItemBytes) return "step: no room for the ring";
   // the partial sums of an SM's rows: of those SMs with the most, and of those with a unit less
   auto fits = [&](int rows, int q, int K, int slots) {
-    const int most = share_of(rows, q, 0, s->num_sms).n;
-    for (int n = most; n > 0 && n >= most - q; n -= q)
+    const int most = share_of(rows, q, 0, s->num_sms).n, units = K / unit_of(s->wfmt);
+    for (int n = most; n > 0 && n >= most - q; n -= q) {
       if (n * slots > kPartFloats / split_of(s->wfmt, s->n_experts != 0, false, K, n * slots).kw) return false;
+      // what was refused when a team's warps divided the inputs as far as they go still is
+      int kw = 1;
+      while (kw < kStepWarps / teams_of(s->wfmt, s->n_experts != 0, K, n * slots) && 2 * kw <= units) kw *= 2;
+      if (n * slots > kPartFloats / kw) return false;
+    }
     return true;
   };
   const int k = s->n_experts ? s->top_k : 1;
