@@ -277,3 +277,31 @@ def test_of_equal_experts_the_lowest_are_chosen(cuda_device):
         assert ids in (rest[:6], list(odd) + rest[:6 - len(odd)])
         if ids == rest[:6]:
             assert torch.equal(weights, torch.full_like(weights, 1 / 6).to(torch.bfloat16).float())
+
+
+@pytest.mark.parametrize("expert", [8, 40, 95])
+@pytest.mark.parametrize("value", ["nan", "-nan", "inf"])
+def test_a_router_logit_without_a_number_ends_a_step(cuda_device, expert, value):
+    """The softmax's sum carries it into every expert's weight, wherever among a lane's logits it stands: the step ends with an error
+    and no token.  An infinite logit leaves the softmax without a number too."""
+    from vdcores_b200 import runtime
+    eng = _engine(cuda_device, 128, hidden=512, n_heads=8, n_kv_heads=2, ffn=256, vocab=512, n_layers=1, n_experts=96, top_k=6)
+    eng.set_state(70, 5)
+    want, router = eng.generate(1), eng.router.clone()
+    eng.router[0][expert].fill_(0.0)
+    if value == "inf":      # of an input whose sign is not known: two rows, one of which gets +inf
+        eng.router[0][expert, 0] = float("inf")
+        eng.router[0][expert - 1].fill_(0.0)
+        eng.router[0][expert - 1, 0] = float("-inf")
+    else:
+        eng.router[0][expert] = float(value)
+    eng.set_state(70, 5)
+    before = eng.state.clone()
+    with pytest.raises(runtime.VdcError, match="no number among"):
+        eng.generate(1)
+    assert torch.equal(eng.state, before)
+    weights = eng.route[16:22].view(torch.float32)
+    assert bool(torch.isnan(weights).all())
+    eng.router.copy_(router)
+    eng.set_state(70, 5)
+    assert eng.generate(1) == want

@@ -1049,24 +1049,30 @@ struct Consumer {
       }
 #pragma unroll
       for (int o = 16; o > 0; o >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, o));
+      // One logit without a number and the softmax's sum has none, nor has any expert's weight, whichever experts are chosen.
+      bool none = false;
 #pragma unroll
-      for (int j = 0; j < kMost; ++j) v[j] = lane + 32 * j < E ? __expf(v[j] - mx) : -1.f;
+      for (int j = 0; j < kMost; ++j) {
+        v[j] = lane + 32 * j < E ? __expf(v[j] - mx) : -1.f;
+        none |= v[j] != v[j];
+      }
       // The largest, k times over; of equal ones the lowest number.  Their weights are renormalised, so the softmax's own sum does
-      // not matter.
-      float all = 0.f, mine = 0.f;
+      // not matter otherwise.
+      float all = __any_sync(0xffffffffu, none) ? NAN : 0.f, mine = 0.f;
       int id = 0;
 #pragma unroll 1
       for (int k = 0; k < s.top_k; ++k) {
-        float bv = v[0];
-        int bi = lane;
+        float bv = -1.f;
+        int bi = 0x7fffffff;
 #pragma unroll
-        for (int j = 1; j < kMost; ++j)
+        for (int j = 0; j < kMost; ++j)
           if (v[j] > bv) {
             bv = v[j];
             bi = lane + 32 * j;
           }
         // a number that was not chosen yet is not negative, so that its bits order it as an integer
         const int top = __reduce_max_sync(0xffffffffu, __float_as_int(bv));
+        // logits without a number select nothing: any expert will do
         bi = min((int)__reduce_min_sync(0xffffffffu, __float_as_int(bv) == top ? (unsigned)bi : 0x7fffffffu), E - 1);
 #pragma unroll
         for (int j = 0; j < kMost; ++j)
