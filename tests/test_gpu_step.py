@@ -305,3 +305,20 @@ def test_a_router_logit_without_a_number_ends_a_step(cuda_device, expert, value)
     eng.router.copy_(router)
     eng.set_state(70, 5)
     assert eng.generate(1) == want
+
+
+def test_silu_of_gates_whose_exponentials_are_close_to_infinity(cuda_device):
+    """exp(88) is 1.65e38, and 1 / (1 + exp(88)) below the smallest normal number: the quotient -88 / (1 + exp(88)) is not."""
+    eng = _engine(cuda_device, 64, hidden=512, n_heads=8, n_kv_heads=2, ffn=256, vocab=64, n_layers=1)
+    eng.embed.fill_(1.0)
+    eng.ln2.fill_(1.0)
+    for w in (eng.wo, eng.wgu, eng.wd):
+        w.zero_()
+    eng.wgu[0][0::2, 0], eng.wgu[0][1::2, 0] = -88.0, 2.0 ** 120
+    eng.wd[0][:, 7] = 1.0
+    caches = eng.kpool.clone(), eng.vpool.clone()
+    (a, _, _, _), = _steps(eng, 20, 1, True, caches)[0]
+    (b, _, _, _), = _steps(eng, 20, 1, False, caches)[0]
+    want = 1 - 88 / (1 + torch.tensor(88.0).double().exp()) * 2.0 ** 120
+    for got in (a, b):      # bf16: the SiLU, its product, the sum; __expf has 2 + 1.16 * 88 ulp at 88
+        assert bool(((got.double().cpu() - want).abs() < 3 * 2.0 ** -8).all()), (float(got.flatten()[0]), float(want))
