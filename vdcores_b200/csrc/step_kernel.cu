@@ -622,7 +622,7 @@ struct Consumer {
     static_assert(kStepWarps == 8, "log2");
     teams = 1 << p.lt;
     kw = 1 << p.lk;
-    rw = 1 << (lw - p.lk);
+    rw = (1 << lw) >> p.lk;                                    // 0 for slices, which all eight warps divide among themselves
     kg = warp & (kw - 1);
     rg = (warp & ((1 << lw) - 1)) >> p.lk;
     turn = warp >> lw;
