@@ -261,6 +261,24 @@ def test_rows_that_come_in_slices(cuda_device, kw, positions, num_sms):
     test_step_kernel_against_the_megakernels_program(cuda_device, kw, positions, num_sms)
 
 
+def test_widest_quantised_rows(cuda_device, monkeypatch):
+    """Inputs of 96 KB: the scales' place leaves the ring a little less than three copies of 32 KB, pages of the cache among them.
+    Longer than what the program's tasks take, so against PyTorch: the second layer's cache rows hang on all that stands in front."""
+    from vdcores_b200.decode import DecodeEngine
+    monkeypatch.setattr(DecodeEngine, "_build_program", lambda self: setattr(self, "program", True))
+    eng = _engine(cuda_device, 768, hidden=4096, n_heads=32, n_kv_heads=8, ffn=49152, vocab=512, n_layers=2, wkind="nvfp4")
+    assert eng.step_kernel is not None
+    tokens = torch.randint(0, 512, (701,), generator=torch.Generator().manual_seed(2))
+    eng.prefill(tokens)
+    want = [t[-1].clone() for t in eng.read_kv(1, 701)]
+    page, row = int(eng.page_table[700 // 64]), 700 % 64
+    eng.kpool[1, page, :, row] = eng.vpool[1, page, :, row] = 0.0
+    eng.set_state(700, int(tokens[-1]))
+    eng.generate(1)
+    for got, w in zip(eng.read_kv(1, 701), want):
+        assert rel(got[-1], w) < 1.5e-2
+
+
 def test_of_equal_experts_the_lowest_are_chosen(cuda_device):
     """Router rows that are copies of one another give equal logits; two rows are the others' negative, so either all that are not
     chosen last or the first two."""

@@ -39,3 +39,16 @@ def test_partial_sums_of_a_taken_step_fit(hidden, ffn, num_sms, experts, top_k, 
                for need, have in sums_and_room(rows, unit, K, num_sms, slots, experts > 0))
     assert room == taken
     assert (runtime.step_workspace(step(hidden, ffn, num_sms, experts=experts, top_k=top_k)) is not None) == taken
+
+
+@pytest.mark.parametrize("hidden,ffn,taken", [
+    (4096, 49152, True),         # inputs and hidden state leave 96 KB, of which the scales take 4
+    (8192, 45056, True),
+    (4096, 50176, False),
+    (8192, 46080, False)])
+def test_scales_take_nothing_from_what_a_wide_step_needs(hidden, ffn, taken):
+    """NVFP4 rows of the widest projections: 2-byte inputs and hidden state, 26496 bytes of sums, heads and probabilities, and a ring
+    of three copies of 32 KB share 231296 bytes."""
+    from vdcores_b200 import runtime
+    assert (2 * (hidden + ffn) + 26496 + 3 * 32768 <= 231296) == taken
+    assert (runtime.step_workspace(step(hidden, ffn, 148, n_kv=8, wfmt=2, splits=4)) is not None) == taken

@@ -35,6 +35,7 @@ constexpr int kPartFloats = 4 * 8 * kOutLd;          // partial sums of rows; al
 constexpr int kQLd = VDC_HEAD_DIM / 2 + 4;           // words of a query row in shared memory
 constexpr int kPLd = VDC_KV_PAGE / 2 + 4;            // words of a row of probabilities
 constexpr int kMaxTopK = 16, kMaxExperts = 256;
+constexpr int kScaleBytes = kStepThreads * 16;       // four scales of quantised rows per thread
 constexpr int kStepSmem = 227 * 1024 - 1024;         // dynamic; the rest is StepShared's barriers
 
 enum { kQkv, kOut, kRouter, kGateUp, kDown, kVocab, kStages };
@@ -104,7 +105,7 @@ __host__ __device__ inline StepLayout step_layout(const vdc_step& s) {
   l.gm = take(kGroups * 4 * 8 * 4);
   l.wl = take(kGroups * 5 * 8 * 4);
   l.route = take(kMaxExperts * 4 + 2 * kMaxTopK * 4);
-  l.scales = take(s.wfmt ? kStepThreads * 16 : 0);
+  l.scales = take(s.wfmt ? kScaleBytes : 0);
   l.ring = at;
   l.total = kStepSmem - 128;
   return l;
@@ -1471,7 +1472,8 @@ extern "C" const char* vdc_step_refuses(const vdc_step* s, bool pointers) {
   if (s->n_experts && (s->wfmt || s->n_experts > kMaxExperts || s->n_experts % 2 || s->top_k < 1 || s->top_k > kMaxTopK || s->top_k > s->n_experts))
     return "step: experts not supported";
   const StepLayout l = step_layout(*s);
-  if (l.total - l.ring < 3 * kItemBytes) return "step: no room for the ring";
+  // three copies, or, where weights have scales, what those leave of them: the ring needs room for one
+  if (l.total - l.ring + (s->wfmt ? kScaleBytes : 0) < 3 * kItemBytes) return "step: no room for the ring";
   // the partial sums of an SM's rows: of those SMs with the most, and of those with a unit less
   auto fits = [&](int rows, int q, int K, int slots) {
     const int most = share_of(rows, q, 0, s->num_sms).n, units = K / unit_of(s->wfmt);
