@@ -261,6 +261,18 @@ def test_rows_that_come_in_slices(cuda_device, kw, positions, num_sms):
     test_step_kernel_against_the_megakernels_program(cuda_device, kw, positions, num_sms)
 
 
+# sums of rows that nobody else adds to, as many as there is room for: 1088 and 4172 gate/up rows, 302 rows of 13 experts' sums
+CROWDED = [
+    (dict(hidden=1024, n_heads=4, n_kv_heads=1, ffn=4352, vocab=66, n_layers=1), (70,), 8),
+    (dict(hidden=1024, n_heads=4, n_kv_heads=1, ffn=14592, vocab=66, n_layers=1), (70,), 7),
+    (dict(hidden=6912, n_heads=4, n_kv_heads=1, ffn=512, vocab=66, n_layers=1, n_experts=16, top_k=13), (70,), 23)]
+
+
+@pytest.mark.parametrize("kw,positions,num_sms", CROWDED)
+def test_many_rows_per_sm(cuda_device, kw, positions, num_sms):
+    test_step_kernel_against_the_megakernels_program(cuda_device, kw, positions, num_sms)
+
+
 def test_widest_quantised_rows(cuda_device, monkeypatch):
     """Inputs of 96 KB: the scales' place leaves the ring a little less than three copies of 32 KB, pages of the cache among them.
     Longer than what the program's tasks take, so against PyTorch: the second layer's cache rows hang on all that stands in front."""

@@ -8,29 +8,40 @@ def step(hidden, ffn, num_sms, n_kv=1, group=4, vocab=64, experts=0, top_k=0, wf
                         max_pages=4, n_splits=splits, n_experts=experts, top_k=top_k, eps=1e-5, qk_eps=1e-5)
 
 
+def division(K, n, experts, wfmt=0):
+    """Warps that keep a sum of every one of an SM's n rows of K inputs.  Four dense bf16 rows that are longer than a copy of 32 KB
+    come in slices, which all eight warps divide, while 4224 floats hold eight sums of each; otherwise two teams of warps take the
+    chunks in turn (four for NVFP4 rows and experts), and a team's warps divide the inputs as far as they would have fewer than
+    four rows of a chunk each."""
+    steps, row = K // (256 << wfmt), (2 * K, K, K // 2 + K // 16)[wfmt]
+    if wfmt == 0 and not experts and steps > 16 and 4 <= n <= 528:
+        return 8
+    per = max(1, min(32, 32768 // row) // 2 * 2)
+    teams = 4 if (experts or wfmt == 2) and n // per >= 4 else 2 if n // per >= 2 else 1
+    warps, kw = 8 // teams, 1
+    while kw < warps and 2 * kw <= steps and min(n, per) < 4 * (warps // kw):
+        kw *= 2
+    return kw
+
+
 def sums_and_room(rows, unit, K, num_sms, slots, experts):
-    """Partial sums of the SMs with the most rows and of those with a unit less, and the room for them: 4224 floats shared by the
-    warps that divide K (bf16: steps of 256 inputs; eight warps in one, two or, with experts, four teams)."""
+    """Partial sums of the SMs with the most rows and of those with a unit less, and the room for them."""
     most = -(-(rows // unit) // num_sms) * unit
-    out = []
-    for n in (most, most - unit):
-        per = max(1, min(32, 32768 // (2 * K)) // 2 * 2)
-        chunks = n * slots // per
-        teams = 4 if experts and chunks >= 4 else 2 if chunks >= 2 else 1
-        kw = 1
-        while kw < 8 // teams and 2 * kw <= K // 256:
-            kw *= 2
-        out.append((n * slots, 4224 // kw))
-    return out
+    return [(n * slots, 4224 // division(K, n * slots, experts)) for n in (most, most - unit) if n]
 
 
 @pytest.mark.parametrize("hidden,ffn,num_sms,experts,top_k,taken", [
-    (6912, 512, 23, 8, 7, False),        # the down projection of 7 experts: 302 rows of 7 sums, room for 2112
-    (6912, 512, 24, 8, 7, True),
+    (6912, 512, 23, 8, 7, True),         # the down projection of 7 experts: 302 rows of 7 sums, of 13 and of 14; room for 4224
+    (6912, 512, 23, 16, 13, True),
+    (6912, 512, 23, 16, 14, False),
     (2560, 768, 79, 64, 16, True),       # 34 rows of 16 sums
-    (1024, 4096, 8, 0, 0, True),         # gate and up: 1024 rows, room for 1056
-    (1024, 4352, 8, 0, 0, False),
-    (1024, 4096, 7, 0, 0, False)])
+    (1024, 4352, 8, 0, 0, True),         # gate and up: 1088 rows that no two warps divide
+    (1024, 14592, 7, 0, 0, True),        # 4172 rows
+    (1024, 14848, 7, 0, 0, False),       # 4244
+    (4608, 4608, 17, 0, 0, True),        # rows of 9 KB: 544 whole, 540 of them
+    (5120, 2048, 16, 0, 0, True),        # 256 in slices
+    (8192, 1024, 2, 0, 0, True),         # two rows to a chunk, inputs divided by four: 1024 rows, room for 1056
+    (8192, 1280, 2, 0, 0, False)])
 def test_partial_sums_of_a_taken_step_fit(hidden, ffn, num_sms, experts, top_k, taken):
     from vdcores_b200 import runtime
     k = top_k or 1

@@ -345,9 +345,8 @@ __host__ __device__ inline int teams_of(int fmt, bool experts, int K, int n) {
   return (fmt == 2 || experts) && chunks >= 4 ? 4 : chunks >= 2 ? 2 : 1;
 }
 __host__ __device__ inline Split split_of(int fmt, bool experts, bool vocab, int K, int n) {
-  const int steps = K / unit_of(fmt), most = kItemBytes / (4 * 512);
-  if (fmt == 0 && !experts && steps > most && n >= 4 && (vocab || n <= kPartFloats / kStepWarps)) return {2, kStepWarps, most};
-  const int units = K / unit_of(fmt);
+  const int units = K / unit_of(fmt), most = kItemBytes / (4 * 512);
+  if (fmt == 0 && !experts && units > most && n >= 4 && (vocab || n <= kPartFloats / kStepWarps)) return {2, kStepWarps, most};
   Split s{teams_of(fmt, experts, K, n), 1, 0};
   // Along the inputs only as far as a warp would otherwise have fewer than four rows of a chunk: the sums over its lanes come once
   // per four rows, whatever the inputs.  With the inputs divided as far as possible four 8B-shaped e4m3 layers took 232.6 us, 228.8 so,
@@ -1476,14 +1475,9 @@ extern "C" const char* vdc_step_refuses(const vdc_step* s, bool pointers) {
   if (l.total - l.ring + (s->wfmt ? kScaleBytes : 0) < 3 * kItemBytes) return "step: no room for the ring";
   // the partial sums of an SM's rows: of those SMs with the most, and of those with a unit less
   auto fits = [&](int rows, int q, int K, int slots) {
-    const int most = share_of(rows, q, 0, s->num_sms).n, units = K / unit_of(s->wfmt);
-    for (int n = most; n > 0 && n >= most - q; n -= q) {
+    const int most = share_of(rows, q, 0, s->num_sms).n;
+    for (int n = most; n > 0 && n >= most - q; n -= q)
       if (n * slots > kPartFloats / split_of(s->wfmt, s->n_experts != 0, false, K, n * slots).kw) return false;
-      // what was refused when a team's warps divided the inputs as far as they go still is
-      int kw = 1;
-      while (kw < kStepWarps / teams_of(s->wfmt, s->n_experts != 0, K, n * slots) && 2 * kw <= units) kw *= 2;
-      if (n * slots > kPartFloats / kw) return false;
-    }
     return true;
   };
   const int k = s->n_experts ? s->top_k : 1;
