@@ -50,10 +50,15 @@ __host__ __device__ constexpr int stage_size(int wfmt, int bpad) {
 }
 __host__ __device__ inline int ring_stages(int wfmt, int bpad) {
   const int n = (kGemmSmem - 2048 - 128) / stage_size(wfmt, bpad), most = wfmt ? kMaxRing : 8;
-  return n >= most ? most : wfmt && n >= 4 ? n & ~1 : n;    // even where weights are converted, see `teams`
+  return n >= most ? most : wfmt ? n & ~1 : n;      // even where weights are converted, see kTeams
 }
-
-static_assert((kGemmSmem - 2048 - 128) / stage_size(1, 128) >= kBufs, "a place for every buffer of widened weights");
+// Quantised weights are converted by two teams of warps that take the chunks in turn, so that a team's waits fall into the other's
+// conversion.  The ring's length is even then: a team sees every round of its places (it would otherwise meet a place two rounds
+// on, and the barrier's parity cannot tell those apart).
+constexpr int kTeams = 2, kTeam = kEpiThreads / kTeams;
+static_assert(kTeam == 128, "a thread of a team for every lane of tensor memory");
+static_assert((kGemmSmem - 2048 - 128) / stage_size(1, 128) >= kBufs && kBufs % kTeams == 0,
+              "a place for every buffer of widened weights (128 rows of e4m3 weights are the largest places)");
 
 // The exchange tile of a CTA: [source CTA][four columns][its row, one spare][4] fp32.  Every CTA of the cluster writes the
 // sums of its K-range straight from tensor memory into the tile of the CTA that finishes the row (consecutive rows lie
@@ -112,11 +117,6 @@ __global__ void __launch_bounds__(kGemmThreads, 2) stage_gemm(const __grid_const
   const int chunks = s.K / kKc, c0 = chunks * rank / splits, n_ch = chunks * (rank + 1) / splits - c0;
   const int xbytes = s.Bpad * kKc * 2, wbytes = chunk_bytes(kFmt, N);
   const int stage_bytes = stage_size(kFmt, s.Bpad);
-  // Quantised weights are converted by two teams of warps that take the chunks in turn where the ring's length is even, so
-  // that a team sees every round of its stages; by all warps together where it is not (a team would then meet a stage two
-  // rounds on, and the barrier's parity cannot tell those apart).  Teams, because a team's waits then fall into the other's
-  // conversion.
-  const int teams = n_ring & 1 ? 1 : 2;
   uint8_t* ring = aligned128(dyn);
   const Waiter wait{&sh.fail, status, timeout_ns, s.kind};
 
@@ -125,7 +125,7 @@ __global__ void __launch_bounds__(kGemmThreads, 2) stage_gemm(const __grid_const
     for (int i = 0; i < n_ring; ++i) {
       mbar_init(&sh.full[i], 1);
       mbar_init(&sh.empty[i], 1);
-      mbar_init(&sh.ready[i], kEpiThreads / 32 / teams);
+      mbar_init(&sh.ready[i], kTeam / 32);
     }
     mbar_init(&sh.done, 1);
     sh.fail = 0;
@@ -207,16 +207,16 @@ __global__ void __launch_bounds__(kGemmThreads, 2) stage_gemm(const __grid_const
     if (kFmt != 0) {
       // A warp widens the rows whose lanes of tensor memory it reaches; rows past N are whatever lies there, for sums that nobody
       // reads.
-      const int team = kEpiThreads / teams, tt = t & (team - 1), quarter = warp & 3, row = quarter * 32 + lane;
+      const int quarter = warp & 3, row = quarter * 32 + lane;
       const uint32_t to = tmem + ((uint32_t)(quarter * 32) << 16) + kRowCols;
       // `old`: the place of the chunk whose buffer chunk i takes, kBufs chunks back.  It cannot be given back a second time before
       // chunk i is converted, since the ring has kBufs places at least.
       RingAt at{n_ring}, old{n_ring};
-      if (t >= team) {
+      if (t >= kTeam) {
         at.next();
         old.next();
       }
-      for (int i = t / team; i < n_ch; i += teams) {
+      for (int i = t / kTeam; i < n_ch; i += kTeams) {
         const int st = at.st, buf = i & (kBufs - 1);
         const bool seen = wait(&sh.full[st], at.parity, 2, i) && (i < kBufs || wait(&sh.empty[old.st], old.parity, 2, i));
         if (!__all_sync(0xffffffffu, seen)) break;      // as in warp_wait, one vote for both
@@ -227,24 +227,23 @@ __global__ void __launch_bounds__(kGemmThreads, 2) stage_gemm(const __grid_const
         Narrow<kFmt == 0 ? 1 : kFmt> w[kGroups];
 #pragma unroll
         for (int g = 0; g < kGroups; ++g)
-          if (teams == 2 || (g & 1) == tt >> 7) w[g].load(src, N, min(row, N - 1), g);
+          w[g].load(src, N, min(row, N - 1), g);
 #pragma unroll
-        for (int g = 0; g < kGroups; ++g)
-          if (teams == 2 || (g & 1) == tt >> 7) {
-            uint32_t o[8];
-            w[g].widen(o);
-            tmem_st8(to + buf * (kKc / 2) + g * 8, o);
-          }
+        for (int g = 0; g < kGroups; ++g) {
+          uint32_t o[8];
+          w[g].widen(o);
+          tmem_st8(to + buf * (kKc / 2) + g * 8, o);
+        }
         tmem_st_wait();
         tc_fence_before();
         fence_proxy_async_smem();      // the place's next weights come through the other proxy
         __syncwarp();
         if (lane == 0) mbar_arrive(&sh.ready[st]);   // one arrival per warp: one per thread would queue on the barrier's word
         at.next();
-        if (teams == 2) at.next();
+        at.next();
         if (i >= kBufs) {
           old.next();
-          if (teams == 2) old.next();
+          old.next();
         }
       }
     }
