@@ -55,10 +55,13 @@ def test_prompt_in_one_pass_agrees_with_its_chunks(cuda_device, kind, fmt, T, ch
     """Ragged prompts, shuffled pages, chunks that do not divide 128, prompts of two passes: cache rows of every layer, the last
     chunk's hidden rows (its repeated ones too) and the first id."""
     from tests.helpers import engine_config, small_cfg
+    _one_pass_against_chunks(cuda_device, engine_config(small_cfg(kind)), fmt, T, chunk, perm)
+
+
+def _one_pass_against_chunks(dev, cfg, fmt, T, chunk, perm):
+    """The prompt's stages of one pass, when it has agreed."""
     from vdcores_b200.decode import DecodeEngine
     from vdcores_b200.prefill import PrefillEngine
-    dev = cuda_device
-    cfg = engine_config(small_cfg(kind))
     eng = DecodeEngine(cfg, (T + 70) // 64 * 64, device=dev, wkind=fmt, page_perm_seed=perm)
     eng.init_random_weights(3)
     prompt = torch.randint(0, cfg.vocab, (T,), generator=torch.Generator().manual_seed(T))
@@ -92,6 +95,28 @@ def test_prompt_in_one_pass_agrees_with_its_chunks(cuda_device, kind, fmt, T, ch
         rows = (a.float() - b.float()).flatten(0, 2).norm(dim=1) / b.float().flatten(0, 2).norm(dim=1).clamp_min(1e-6)
         assert float(rows.max()) < 1e-2
     assert bool(((k1 == 0) == (k0 == 0)).float().mean() > 0.999)     # nothing written past the prompt
+    return lists[-(-min(T, 2048) // 128) * 128]
+
+
+@pytest.mark.parametrize("fmt,hidden,kv,ffn,T,chunk,batched", [
+    ("fp8", 2048, 4, 2048, 77, 64, ("wo", "wgu", "wd")),
+    ("nvfp4", 2048, 4, 2048, 128, 48, ("wo", "wgu", "wd")),
+    ("fp8", 2048, 4, 1536, 65, 64, ("wo", "wgu")),      # inputs shorter than 2048; rows shorter than that
+    ("fp8", 1024, 2, 3072, 70, 64, ()),
+    ("nvfp4", 1024, 2, 3072, 120, 100, ()),
+    ("bf16", 512, 1, 4096, 65, 64, ()),
+    ("bf16", 1024, 2, 9472, 101, 64, ("wgu",)),         # 148 blocks of gate/up, 152
+    ("bf16", 1024, 2, 9728, 128, 100, ()),
+    ("bf16", 2048, 4, 1024, 90, 32, ("wo", "wgu", "wd"))])
+def test_a_prompt_of_up_to_128_rows(cuda_device, fmt, hidden, kv, ffn, T, chunk, batched):
+    """Projections as stages of the batched step and as wide tiles, on either side of what decides between them."""
+    from vdcores_b200 import isa
+    from vdcores_b200.decode import DecodeConfig
+    cfg = DecodeConfig(hidden=hidden, n_heads=4 * kv, n_kv_heads=kv, head_dim=128, ffn=ffn, vocab=1024, n_layers=2, eps=1e-5, theta=5e5)
+    stages = _one_pass_against_chunks(cuda_device, cfg, fmt, T, chunk, 3)
+    for layer in range(2):
+        for name, at in (("wqkv", 1), ("wo", 4), ("wgu", 6), ("wd", 7)):
+            assert (stages[1 + 8 * layer + at].kind == isa.STAGE_GEMM) == (name in batched), name
 
 
 def test_prompts_go_chunk_by_chunk_without_the_wide_buffers(cuda_device, monkeypatch):

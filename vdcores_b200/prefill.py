@@ -139,6 +139,21 @@ class PrefillEngine(BatchDecodeEngine):
         return first
 
 
+def batched_projection(name: str, M: int, K: int, fmt: int, splits: int) -> bool:
+    """Whether 128 rows of a prompt go through a layer's M x K projection as a stage of the batched step (`splits` CTAs to a block
+    of its rows) and not as wide tiles.  What bounds 128 rows of a large projection is the weights, and the stage's two CTAs per SM
+    bring them faster than a wide tile's one; where there are few of them it is its cluster's exchange and its longer prologue.
+    What a layer of 100 rows gains from the one in place of the other (us, B200, weights from HBM; from L2 within 1 us of it):
+      bf16   wo 4096 x 4096  6.2, wd 4096 x 14336  8.1, 2048 x 1024  1.2, 1024 x 3072  0.1, 1024 x 1024  -0.3, 512 x 1024  -0.8
+             gate/up 8192 x 4096  12.7, 12288 x 2048  2.3, 6144 x 1024  0.2, 8192 x 512  -1.9
+      e4m3   wo 4096 x 4096  7.0, wd 4096 x 14336  16.6, wo 2048 x 2048  0.9, wd 2048 x 1024  -4.9, 1024 x 3072  -5.4
+             gate/up 28672 x 4096  10.6, 12288 x 2048  5.3, 6144 x 1024  -3.0      (NVFP4 within 2 us of these, 28672 x 4096  17)
+    A bf16 gate/up of more blocks than SMs leaves some SMs two CTAs of whole rows (24576 x 4096  -5.7, 28672 x 4096  -3.8).  QKV sums
+    come faster from wide tiles everywhere (6144 x 4096 bf16 -1.4, e4m3 -5.7; 1536 x 1024  -3.1, -7.2): the tiles' K ranges leave
+    several sums of a value, for each of which heads take 0.1 us more and a norm 0.5."""
+    return name != "wqkv" and M >= 2048 and (K >= 1024 and splits > 1 if fmt == 0 else K >= 2048)
+
+
 class WideStages:
     """Buffers and stages of a prompt whose rows go through a layer together.  Rows are taken in passes of `rows` (whole chunks
     of the engine, at most isa.WIDE_ROWS); a pass over R rows (a multiple of 128) has a list of stages of its own."""
@@ -208,11 +223,9 @@ class WideStages:
         n = 8 * cfg.n_layers
         v["splits"][1 + 3:1 + n:8] = e._splits(cfg.n_kv_heads * (R // (64 // cfg.group)), 2, e.max_pages)
         for name, (at, reader, M, K) in self.places.items():
-            if R == 128:
-                # a batched step's projection: what bounds 128 rows is the weights, and two CTAs per SM bring them faster than
-                # a wide tile's one.  Two 8B-shaped layers, bf16 77 rows 510 -> 494 us, e4m3 70 rows 565 -> 489
-                v["kind"][1 + at:1 + n:8], v["B"][1 + at:1 + n:8] = isa.STAGE_GEMM, R
-                v["splits"][1 + at:1 + n:8], ks = e._splits(-(-M // isa.STAGE_BLOCK), 2, K // 64), 1
+            splits, ks = e._splits(-(-M // isa.STAGE_BLOCK), 2, K // 64), 1
+            if R == 128 and batched_projection(name, M, K, self.fmt, splits):
+                v["kind"][1 + at:1 + n:8], v["B"][1 + at:1 + n:8], v["splits"][1 + at:1 + n:8] = isa.STAGE_GEMM, R, splits
             else:
                 subs, cols, ks = runtime.wide_tiles(R, M, K, self.fmt, self.sms, name == "wgu")
                 v["group"][1 + at:1 + n:8], v["n_kv"][1 + at:1 + n:8], v["splits"][1 + at:1 + n:8] = subs, cols, ks
