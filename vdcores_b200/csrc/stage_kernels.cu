@@ -102,18 +102,45 @@ __device__ __forceinline__ void qkv_head(const vdc_stage& s, const uint8_t* tile
   head_row(s, x, b, block, lane, ld_relaxed_gpu(st + VDC_ST_POS), new_row, first);
 }
 
-// Sixteen values of sixteen lanes (two such halves of a warp): lane i gets the i-th of all of them, in the lanes' order.
-__device__ __forceinline__ void transpose16(uint32_t (&r)[16], int lane) {
+// The exchange of a block whose weight rows lie on the accumulator's lanes: [source CTA][kPiece of its rows][128 columns][kPiece]
+// fp32, so that a lane has a piece of consecutive rows and a warp stores 32 of them side by side.  A store to another CTA costs what
+// the pieces cost into which it falls.  Eight CTAs to a block, 128 rows, e4m3: 4096 x 1024 17.1 us with a lane storing single words of
+// the layout of tile_at, 12.6 with sixteen lanes exchanging sixteen values each in front of the stores, 12.5 so; 2048 x 4096 16.3, 13.1
+// and 12.7; of 32 rows 9.1, 8.8 and 8.4.  kPiece is 2 where a CTA finishes two rows.
+template <int kPiece>
+__device__ __forceinline__ uint32_t piece_at(uint32_t tile, int src, int nb, int row, int col) {
+  return tile + (uint32_t)(((src * nb + row) / kPiece * kBlk + col) * kPiece) * 4u;
+}
+// This warp's accumulator columns (rows row0 .. row0 + 15 of a lane's weight row n) to the CTAs that finish them.
+template <int kPiece>
+__device__ __forceinline__ void send_pieces(const uint32_t (&r)[16], uint32_t tile, int rank, int nb, int row0, int n) {
+  const int lg = 31 - __clz(nb);
 #pragma unroll
-  for (int b = 1; b < 16; b <<= 1) {
-    const bool up = lane & b;
+  for (int j = 0; j < 16; j += kPiece) {
+    const uint32_t to = peer_smem(piece_at<kPiece>(tile, rank, nb, (row0 + j) & (nb - 1), n), (uint32_t)((row0 + j) >> lg));
+    if constexpr (kPiece == 4) st_cluster4(to, r[j], r[j + 1], r[j + 2], r[j + 3]);
+    else st_cluster2(to, r[j], r[j + 1]);
+  }
+}
+// The sums over the cluster's K-ranges, in rank order, from pieces to the layout of tile_at (one source; rows and columns of a warp's
+// stores lie in different banks).
+template <int kPiece>
+__device__ __forceinline__ void sum_pieces(uint8_t* to, const uint8_t* from, int splits, int nb, int N, int t) {
+  using Piece = typename std::conditional<kPiece == 4, float4, float2>::type;
+  for (int i = t; i < nb / kPiece * kBlk; i += kEpiThreads) {
+    const int n = i & (kBlk - 1), row = i / kBlk * kPiece;
+    if (n >= N) continue;
+    float v[kPiece];
 #pragma unroll
-    for (int i = 0; i < 16; ++i) {
-      if (i & b) continue;
-      const uint32_t got = __shfl_xor_sync(0xffffffffu, up ? r[i] : r[i | b], b);
-      if (up) r[i] = got;
-      else r[i | b] = got;
+    for (int j = 0; j < kPiece; ++j) v[j] = 0.f;
+    for (int src = 0; src < splits; ++src) {
+      const Piece p = *reinterpret_cast<const Piece*>(from + (size_t)piece_at<kPiece>(0u, src, nb, row, n));
+      v[0] += p.x; v[1] += p.y;
+      if constexpr (kPiece == 4) { v[2] += p.z; v[3] += p.w; }
     }
+    float* out = reinterpret_cast<float*>(to + tile_at(0u, 0, nb, n >> 2, row)) + (n & 3);
+#pragma unroll
+    for (int j = 0; j < kPiece; ++j) out[4 * j] = v[j];
   }
 }
 
@@ -280,23 +307,19 @@ __global__ void __launch_bounds__(kGemmThreads, 2) stage_gemm(const __grid_const
     const int quarter = warp & 3, half = (warp - 2) >> 2;
     const int b = quarter * 32 + lane, ng = N >> 4;
     if (kFmt != 0) {
-      // A lane has a weight row, its columns the rows.  Half a warp exchanges sixteen of each, so that its lanes store four columns
-      // of sixteen rows side by side: a store to another CTA costs what the pieces cost into which it falls.  Eight CTAs to a block,
-      // 128 rows, e4m3: 4096 x 1024 17.1 us with a lane storing its own column's words, 15.9 with pieces of 64 bytes (four lanes
-      // exchanging four), 13.3 with 128, 12.6 so; 4096 x 14336 31.1, 29.7, 27.7 and 26.7.  16 rows within 0.15 us of one another.
-      const int col4 = quarter * 8 + (lane >> 4) * 4, lg = 31 - __clz(nb);
+      // A lane has a weight row, its columns the rows.
+      const int n = quarter * 32 + lane;
       for (int g = half; g < s.Bpad / 16; g += 2) {
         uint32_t r[16];
         tmem_ld16(tmem + ((uint32_t)(quarter * 32) << 16) + (uint32_t)(g * 16), r);
-        transpose16(r, lane);
-        const int row = g * 16 + (lane & 15);
-        const uint32_t at = tile_at(tile, rank, nb, col4, row & (nb - 1)), step = (uint32_t)(nb + 1) * 16u;
-        const uint32_t to = splits > 1 ? peer_smem(at, (uint32_t)(row >> lg)) : at;
-        if (col4 * 4 < N) {        // a multiple of 16, as N is
+        if (n < N) {
+          if (splits == 1) {
 #pragma unroll
-          for (int j = 0; j < 4; ++j) {
-            if (splits > 1) st_cluster4(to + j * step, r[4 * j], r[4 * j + 1], r[4 * j + 2], r[4 * j + 3]);
-            else st_shared4(to + j * step, r[4 * j], r[4 * j + 1], r[4 * j + 2], r[4 * j + 3]);
+            for (int j = 0; j < 16; ++j) st_shared1(tile_at(tile, 0, nb, n >> 2, g * 16 + j) + (uint32_t)(n & 3) * 4u, r[j]);
+          } else if (nb >= 4) {
+            send_pieces<4>(r, tile, rank, nb, g * 16, n);
+          } else {
+            send_pieces<2>(r, tile, rank, nb, g * 16, n);
           }
         }
         __syncwarp();
@@ -330,10 +353,20 @@ __global__ void __launch_bounds__(kGemmThreads, 2) stage_gemm(const __grid_const
   if (warp >= 2 && !failed) {
     const int t = tid - 64;
     const int b_lo = rank * nb;
+    const uint8_t* sums = ring;       // laid out as tile_at has it, from `parts` sources
+    int parts = splits;
+    if (kFmt != 0 && splits > 1) {
+      uint8_t* to = ring + s.Bpad * kBlk * 4;
+      if (nb >= 4) sum_pieces<4>(to, ring, splits, nb, N, t);
+      else sum_pieces<2>(to, ring, splits, nb, N, t);
+      asm volatile("bar.sync 1, %0;" ::"n"(kEpiThreads) : "memory");
+      sums = to;
+      parts = 1;
+    }
     const float* scales = reinterpret_cast<const float*>(s.scales);
     if (s.mode == VDC_STAGE_QKV) {
       for (int bl = warp - 2; bl < nb; bl += kEpiThreads / 32)
-        if (b_lo + bl < s.B) qkv_head(s, ring, splits, nb, bl, b_lo + bl, block, lane);
+        if (b_lo + bl < s.B) qkv_head(s, sums, parts, nb, bl, b_lo + bl, block, lane);
     } else {
       const int bl = t & (nb - 1), b = b_lo + bl;      // nb is a power of two, at most 128
       const int f0 = t / nb, fstep = kEpiThreads / nb;
@@ -342,7 +375,7 @@ __global__ void __launch_bounds__(kGemmThreads, 2) stage_gemm(const __grid_const
           float ssq = 0.f;
           for (int f = f0; f < N / 8; f += fstep) {
             float v[8];
-            sum8(v, ring, splits, nb, bl, f * 8);
+            sum8(v, sums, parts, nb, bl, f * 8);
             scale8(v, scales ? scales + n0 + f * 8 : nullptr);
             uint4* hp = reinterpret_cast<uint4*>(reinterpret_cast<uint8_t*>(s.hid) + kc_piece(s.Bpad, b, n0 + f * 8));
             const uint4 h = *hp;
@@ -362,7 +395,7 @@ __global__ void __launch_bounds__(kGemmThreads, 2) stage_gemm(const __grid_const
 #pragma unroll
             for (int h = 0; h < 2; ++h) {
               float v[8];
-              sum8(v, ring, splits, nb, bl, f * 16 + h * 8);
+              sum8(v, sums, parts, nb, bl, f * 16 + h * 8);
               scale8(v, scales ? scales + n0 + f * 16 + h * 8 : nullptr);
 #pragma unroll
               for (int j = 0; j < 4; ++j) {
@@ -375,7 +408,7 @@ __global__ void __launch_bounds__(kGemmThreads, 2) stage_gemm(const __grid_const
         } else if (s.mode == VDC_STAGE_SUMS) {
           for (int f = f0; f < N / 8; f += fstep) {
             float v[8];
-            sum8(v, ring, splits, nb, bl, f * 8);
+            sum8(v, sums, parts, nb, bl, f * 8);
             scale8(v, scales ? scales + n0 + f * 8 : nullptr);
             float4* to = reinterpret_cast<float4*>(s.out) + (size_t)((n0 >> 2) + f * 2) * s.Bpad + b;
             to[0] = make_float4(v[0], v[1], v[2], v[3]);
@@ -386,7 +419,7 @@ __global__ void __launch_bounds__(kGemmThreads, 2) stage_gemm(const __grid_const
           int row = 0x7fffffff;
           for (int f = f0; f < N / 8; f += fstep) {
             float v[8];
-            sum8(v, ring, splits, nb, bl, f * 8);
+            sum8(v, sums, parts, nb, bl, f * 8);
             scale8(v, scales ? scales + n0 + f * 8 : nullptr);
 #pragma unroll
             for (int j = 0; j < 8; ++j) {
