@@ -12,7 +12,7 @@
 // 128256-row vocabulary projection at 3 rows).
 //
 // Measured against the megakernel's program, two Llama-3.1-8B-shaped layers and a small vocabulary (B200): 3 rows at
-// 1000 positions 416 -> 235 us, 32 rows with e4m3 weights 759 -> 283, 64 rows at 2100 positions 929 -> 402, 128 rows
+// 1000 positions 416 -> 235 us, 32 rows with e4m3 weights 759 -> 276, 64 rows at 2100 positions 929 -> 402, 128 rows
 // 1024 -> 397 (up to 4 % more or less from one GPU to another).
 #include "mk_stage.cuh"
 
@@ -122,6 +122,7 @@ __device__ __forceinline__ void send_pieces(const uint32_t (&r)[16], uint32_t ti
     else st_cluster2(to, r[j], r[j + 1]);
   }
 }
+static_assert(128 * kBlk * 4 + kCol4 * (64 + 1) * 16 <= kGemmSmem - 128, "pieces of 128 rows, and behind them the sums of a CTA's 64");
 // The sums over the cluster's K-ranges, in rank order, from pieces to the layout of tile_at (one source; rows and columns of a warp's
 // stores lie in different banks).
 template <int kPiece>

@@ -9,9 +9,9 @@
 // The same step as a program of the megakernel (csrc/megakernel.cu) counts barriers down: fence, atomic, poll, then a copy,
 // about 7 us per boundary.
 //
-// Measured against that program (B200): three layers of width 512 109 -> 50 us, eight 8B-shaped bf16 layers and a 128256-row
-// vocabulary projection 1012 -> 813, four such layers e4m3 387 -> 245, NVFP4 388 -> 232, four layers of a 30B mixture of experts
-// 437 -> 208.
+// Measured against that program (B200): three layers of width 512 109 -> 46 us, eight 8B-shaped bf16 layers and a 128256-row
+// vocabulary projection 1012 -> 800, four such layers e4m3 387 -> 230, NVFP4 388 -> 225, four layers of a 30B mixture of experts
+// 437 -> 201 (up to 2 % more or less from one GPU to another).
 //
 // An entry buffer is written again one layer later, when everything that read it must have been read: whoever polls a buffer
 // has rows in the same or the following stage, and those rows go into what the next writer of the buffer waits for.
@@ -19,9 +19,9 @@
 
 namespace vdc {
 
-// Consumer warps; one more warp produces.  All of them execute what a stage's boundary needs, and wait for entries in L2 and for the
-// instruction before: eight warps, not sixteen, which took 515 us for four
-// 8B-shaped layers where eight took 451.
+// Consumer warps; one more warp produces.  All of them execute what a stage's boundary needs and wait there for entries in L2 and,
+// instruction by instruction, for the one before: twice as many would execute it all twice as often (four 8B-shaped layers 515 us with
+// sixteen, 451 with eight).
 constexpr int kStepWarps = 8;
 constexpr int kStepThreads = 32 * kStepWarps;
 constexpr int kItems = 16;                           // copies in the ring, at most
@@ -136,14 +136,14 @@ __host__ __device__ inline StepWork step_work(const vdc_step& s) {
   return w;
 }
 
-// What a launch passes: the step, and where its shared memory and its entries lie.  From the constant bank these cost no
-// registers.
 // A stage as the host divides it: the first `more` SMs take each + 1 units of q rows, the others `each`; lt, lk and most for
 // either.  A stage's boundary on the device had 1000 to 2300 cycles of integer divisions for this (of 8000 to 11000).
 struct Deal {
   int q, each, more, per, units;
   int lt[2], lk[2], slice[2], most[2];
 };
+// What a launch passes: the step, where its shared memory and its entries lie, how its stages are divided.  From the constant bank
+// these cost no registers.
 struct StepArgs {
   vdc_step s;
   StepLayout lay;
@@ -252,7 +252,7 @@ __device__ __forceinline__ void add2(float& a, float& b, float x, float y) {
 // by 16 x 8 tiles.  Row g of a tile is what the four lanes 4g .. 4g + 3 hold of the pair's first row (8 + g: of its second), column
 // g what they hold of the inputs: the tile's element (g, g) is the sum of the four lanes' products, the other elements mean nothing.
 // A product of tiles is one instruction where FMAs of four rows are 12 (32 KB of bf16 took 0.8 us with those, HBM 0.73).
-// All loads of the steps are issued before the first product waits for one: see kStepsOf.
+// All loads of the steps are issued before the first product waits for one: see steps_of.
 // The tensor cores cut off what an fp32 sum cannot hold.  So bf16 and e4m3 rows have only two products of tiles (8 of a lane's
 // inputs) added up by them, from zero; those sums meet in rounded additions.  Of 32768 sums of 8192 products around two large
 // ones that cancel, 2.0 % miss their bf16 rounding (FMAs 2.1 %, all products in one sum of the tensor cores 7.2 %).  Four
@@ -337,9 +337,10 @@ __host__ __device__ constexpr int chunk_rows(int rb) {        // an even number 
 struct Split {
   int teams, kw, slice;
 };
-// Two teams, since a chunk's place in the ring is held for as long as its team works on it; four where there is more work per byte.
-// With 2 / 4 teams: eight 8B-shaped bf16 layers 813 / 819 us, four e4m3 244 / 253, NVFP4 236 / 231, the 30B mixture of experts 211 /
-// 209.5.
+// Two teams, since a chunk's place in the ring is held for as long as its team works on it.  With 2 / 4 teams: eight 8B-shaped bf16
+// layers 799 / 808 us, four e4m3 230 / 238, NVFP4 224 / 224.5, the 30B mixture of experts 198 / 201.  NVFP4 rows and experts keep four
+// for their sums' sake: where a chunk has fewer than eight rows two warps keep two sums of each, a team of four four, and there would be
+// room for half as many rows (hidden 6912: 1056 gate/up rows of the chosen experts to an SM instead of 2112).
 __host__ __device__ inline int teams_of(int fmt, bool experts, int K, int n) {
   const int chunks = n / chunk_rows(row_bytes(fmt, K));
   return (fmt == 2 || experts) && chunks >= 4 ? 4 : chunks >= 2 ? 2 : 1;
@@ -595,6 +596,7 @@ struct Consumer {
       const float4 r = *reinterpret_cast<const float4*>(sh.red + k);
       tot += r.x; tot += r.y; tot += r.z; tot += r.w;
     }
+    // 1 / hidden is exact for powers of two; otherwise its rounding stands for the one that the product in the sum has not
     const float rstd = rsqrtf(fmaf(tot, args.inv_hidden, s.eps));
     copies_wait();
 #pragma unroll
@@ -883,6 +885,7 @@ struct Consumer {
 #pragma unroll
           for (int w = 0; w < 4; ++w) mn = fmaxf(mn, gm[w * 8 + 2 * t4 + j]);
           const bool none = mn == -INFINITY;
+          // of exp2f's numbers exp2_ftz lacks those below 2^-126, which a row's sum (1 at least) cannot hold
           al[j] = none ? 1.f : exp2_ftz(m[j] - mn);
           e[j] = none ? 0.f : exp2_ftz(e[j] - mn);
           e[j + 2] = none ? 0.f : exp2_ftz(e[j + 2] - mn);

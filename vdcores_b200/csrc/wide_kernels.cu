@@ -10,7 +10,8 @@
 // adds the splits up in order: no atomics, the same bits every time.
 //
 // Measured (B200): two such layers and a small vocabulary, 2048 tokens 5.1 -> 2.2 ms, 77 tokens (two chunks of 64 before)
-// 667 -> 495 us.  Gate/up of 2048 rows 352 us (1.37 PFLOP/s; cuBLAS 331), down 166 us (1.45; 155).
+// 667 -> 465 us.  Gate/up of 2048 rows 352 us (1.37 PFLOP/s; cuBLAS 331), down 166 us (1.45; 155).  A prompt's large projections of
+// up to 128 rows are stages of the batched step (csrc/stage_kernels.cu); which, prefill.py decides.
 #include "mk_stage.cuh"
 
 namespace vdc {

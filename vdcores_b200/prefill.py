@@ -146,11 +146,12 @@ def batched_projection(name: str, M: int, K: int, fmt: int, splits: int) -> bool
     What a layer of 100 rows gains from the one in place of the other (us, B200, weights from HBM; from L2 within 1 us of it):
       bf16   wo 4096 x 4096  6.2, wd 4096 x 14336  8.1, 2048 x 1024  1.2, 1024 x 3072  0.1, 1024 x 1024  -0.3, 512 x 1024  -0.8
              gate/up 8192 x 4096  12.7, 12288 x 2048  2.3, 6144 x 1024  0.2, 8192 x 512  -1.9
-      e4m3   wo 4096 x 4096  7.0, wd 4096 x 14336  16.6, wo 2048 x 2048  0.9, wd 2048 x 1024  -4.9, 1024 x 3072  -5.4
-             gate/up 28672 x 4096  10.6, 12288 x 2048  5.3, 6144 x 1024  -3.0      (NVFP4 within 2 us of these, 28672 x 4096  17)
-    A bf16 gate/up of more blocks than SMs leaves some SMs two CTAs of whole rows (24576 x 4096  -5.7, 28672 x 4096  -3.8).  QKV sums
-    come faster from wide tiles everywhere (6144 x 4096 bf16 -1.4, e4m3 -5.7; 1536 x 1024  -3.1, -7.2): the tiles' K ranges leave
-    several sums of a value, for each of which heads take 0.1 us more and a norm 0.5."""
+      e4m3   wo 4096 x 4096  13.4, wd 4096 x 14336  20.9, wo 2048 x 2048  5.1, wd 2048 x 1024  -0.7, 1024 x 3072  -1.0, 512 x 1024  -1.1
+             gate/up 28672 x 4096  12.1, 12288 x 2048  5.1, 6144 x 1024  0.6, 2048 x 512  -3.9     (NVFP4 up to 4 us more, 28672 x 4096
+             18.8)
+    A bf16 gate/up of more blocks than SMs leaves some SMs two CTAs of whole rows (24576 x 4096  -5.3, 28672 x 4096  -3.8).  QKV sums
+    come from wide tiles as fast or faster everywhere (6144 x 4096 bf16 -1.7, e4m3 -2.0, NVFP4 -0.4; 1536 x 1024  -3.1, -3.7, -3.7): the
+    tiles' K ranges leave several sums of a value, for each of which heads take 0.1 us more and a norm 0.5."""
     return name != "wqkv" and M >= 2048 and (K >= 1024 and splits > 1 if fmt == 0 else K >= 2048)
 
 
