@@ -72,3 +72,31 @@ def test_prefill_chunk_by_chunk_matches_oracle(cuda_device, monkeypatch, kind, p
     from vdcores_b200.prefill import PrefillEngine
     monkeypatch.setattr(PrefillEngine, "_goes_wide", lambda self, T: False)
     test_gpu_prefill.test_chunked_prefill_matches_oracle(cuda_device, kind, prompt_len, chunk, perm)
+
+
+@pytest.mark.parametrize("kw,eng_kw", [(dict(vocab=2051), dict()), (dict(vocab=2058), dict(shared_counters=True)), (dict(vocab=5), dict()),
+                                       (dict(vocab=64, hidden=2048, n_experts=76, top_k=4, ffn=256), dict())])
+def test_rows_behind_the_last_whole_chunk(cuda_device, program, kw, eng_kw):
+    """Vocabularies and experts that whole copies of a router's or a head's rows do not make up: every logit, and the largest."""
+    from vdcores_b200.decode import DecodeConfig, DecodeEngine
+    cfg = DecodeConfig(**{**dict(hidden=512, n_heads=8, n_kv_heads=2, ffn=512, n_layers=1, eps=1e-5, theta=5e5), **kw})
+    eng = DecodeEngine(cfg, 128, device=cuda_device, timeout_ns=500_000_000, **eng_kw)
+    eng.init_random_weights(3)
+    for last in (False, True):
+        if last:                # the last row is the largest for whatever the hidden state is then
+            eng.lm_head[-1] = eng.norm_w * (20 * x)
+        eng.set_state(20, 4)
+        tok = eng.generate(1)[0]
+        h = eng.hidden.float()
+        x = (h * torch.rsqrt(h.pow(2).mean() + cfg.eps)).to(torch.bfloat16)
+        want = (x * eng.norm_w).float() @ eng.lm_head.float().t()
+        assert O.rel_l2(eng.logits.cpu(), want.cpu()) < 4e-3          # one rounding to bf16, 2^-9
+        assert tok == int(eng.logits.float().argmax()) and (tok == cfg.vocab - 1 or not last)
+    if cfg.n_experts:
+        eng.router[0][:-4] = 0.0                                          # logits of zero and four that are not
+        eng.router[0][-4:] = 0.1
+        eng.set_state(20, 4)
+        eng.generate(1)
+        logits = eng.router_logits
+        assert torch.equal(torch.topk(logits, 4).indices.sort().values, eng.route[:4].sort().values.to(torch.int64))
+        assert not bool((logits[-4:] == 0).any())

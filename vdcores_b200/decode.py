@@ -98,11 +98,11 @@ def kv_page_swizzle(pages: torch.Tensor) -> torch.Tensor:
     return v[..., rows[:, None], idx, :].reshape(pages.shape)
 
 
-def rows_per_chunk(K: int, even: bool = False, row_bytes: Optional[int] = None) -> int:
-    """Largest power-of-two row count whose rows (bf16 unless row_bytes is given) fit one 32 KB bulk copy."""
+def rows_per_chunk(K: int, even: bool = False, row_bytes: Optional[int] = None, rows: int = 0) -> int:
+    """Largest power-of-two row count whose rows (bf16 unless row_bytes is given) fit one 32 KB bulk copy and that divides `rows`."""
     row_bytes = 2 * K if row_bytes is None else row_bytes
     r = 16
-    while r > 1 and r * row_bytes > 32768:
+    while r > 1 and (r * row_bytes > 32768 or rows % r):
         r //= 2
     if r * row_bytes > 32768 or (even and r < 2):
         raise ValueError(f"K={K} rows do not fit the 32 KB chunk limit")
@@ -227,7 +227,7 @@ class DecodeEngine:
         self.qkv_perm = torch.tensor(perm, dtype=torch.long)            # packed row -> standard row
         self.qkv_inv = torch.empty_like(self.qkv_perm)
         self.qkv_inv[self.qkv_perm] = torch.arange(len(perm))           # standard row -> packed row
-        self.argmax_rec = z(self.num_sms, 4, dt=torch.float32)
+        self.argmax_rec = z(self.num_sms + 1, 4, dt=torch.float32)      # one more for the rows behind the last whole chunk
         self.state = z(isa.ST_PAGETABLE + self.max_pages, dt=torch.int32)
         self.state_host = torch.zeros(isa.ST_PAGETABLE + self.max_pages, dtype=torch.int32).pin_memory()
         self.token_log = z(max_steps, dt=torch.int32)
@@ -593,11 +593,12 @@ class DecodeEngine:
             b_tap = P.new_barrier()
             plan[sm].append((lambda sm=sm: P.copy(sm, Src(hid, H * 2, wait=b_hid),
                                                   Dst(self.taps[L - 1].data_ptr(), H * 2, release=b_tap), H * 2), None))
-        lm_ranges = stage_ranges(V // R, R * H * 2)
-        for i, (sm, u0, cnt, ctr) in enumerate(lm_ranges):
-            r0, n = u0 * R, cnt * R
+        lm_ranges = [(sm, u0 * R, cnt * R, R, ctr) for sm, u0, cnt, ctr in stage_ranges(V // R, R * H * 2)]
+        if V % R:                       # the rows behind the last whole chunk, one by one
+            lm_ranges.append((self._pick(load, 1)[0], V - V % R, V % R, 1, None))
+        for i, (sm, r0, n, rows, ctr) in enumerate(lm_ranges):
             wa = self.lm_head.data_ptr() + r0 * H * 2
-            add_gemv(sm, (wa, n * H * 2), w_addr=wa, n_rows=n, K=H, R=R, x=Src(hid, H * 2, wait=b_hid),
+            add_gemv(sm, (wa, n * H * 2), w_addr=wa, n_rows=n, K=H, R=rows, x=Src(hid, H * 2, wait=b_hid),
                      out=Dst(self.logits.data_ptr() + r0 * 2, n * 2, "store", release=b_logits),
                      mode=isa.GEMV_MODE_ARGMAX, norm_w=Src(self.norm_w.data_ptr(), H * 2), eps=cfg.eps,
                      pair_out=Dst(self.argmax_rec[i].data_ptr(), 16, release=b_logits), row_base=r0,
@@ -697,7 +698,7 @@ class DecodeEngine:
         wts_addr = ids_addr + 64
         # ---- router logits (fp32) over all SMs that get a chunk
         b_rl = P.new_barrier()
-        R = rows_per_chunk(H)
+        R = rows_per_chunk(H, rows=E)
         for sm, u0, cnt in self._ranges(load, E // R, R * H * 2):
             r0, n = u0 * R, cnt * R
             wa = self.router[l].data_ptr() + r0 * H * 2
