@@ -88,6 +88,17 @@ def test_fused_exchange_one_rank(cuda_device):
     check(results, 1)
 
 
+@pytest.mark.parametrize("kind,fused,change", [("llama", False, dict(vocab=2051)), ("llama", True, dict(vocab=2051)),
+                                               ("moe", False, dict(n_experts=20))])
+def test_rows_behind_the_last_whole_chunk_one_rank(cuda_device, monkeypatch, kind, fused, change):
+    """A vocabulary and experts that whole copies of sixteen rows do not make up: the logits left out are 4 % of their norm."""
+    import dataclasses
+    monkeypatch.setattr("tests.test_gpu_tp.small_cfg", lambda kind, small=small_cfg: dataclasses.replace(small(kind), **change))
+    results = {}
+    run_rank(0, 1, free_port(), 4, results, kind=kind, fused=fused)
+    check(results, 1, bar=2e-2 if kind == "moe" else 1e-2)
+
+
 def test_expert_parallel_one_rank_group(cuda_device):
     """The mixture-of-experts model through the expert-parallel path with one rank: router,
     selection, dynamically counted expert tasks, fp32 partial sum, collectives."""

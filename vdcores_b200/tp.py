@@ -297,7 +297,7 @@ class TPDecodeEngine:
         # ---- vocabulary shard: candidates per SM, then this rank's best as one record
         P = Program(S)
         b_logits = P.new_barrier()
-        R = rows_per_chunk(H)
+        R = rows_per_chunk(H, rows=self.V)
         lm = self._ranges(load, self.V // R, R * H * 2)
         for i, (sm, u0, cnt) in enumerate(lm):
             r0, n = u0 * R, cnt * R
@@ -325,7 +325,7 @@ class TPDecodeEngine:
         wts, lid, cnt = ids + 64, ids + 128, ids + 192
         P = Program(S)
         b_rl, b_route, b_gu = P.new_barrier(), P.new_barrier(), P.new_barrier()
-        R = rows_per_chunk(H)
+        R = rows_per_chunk(H, rows=E)
         for sm, u0, n_u in self._ranges(load, E // R, R * H * 2):
             r0, n = u0 * R, n_u * R
             P.gemv(sm, w_addr=self.router[l].data_ptr() + r0 * H * 2, n_rows=n, K=H, R=R, x=Src(hid, H * 2),
@@ -649,7 +649,7 @@ class TPFusedEngine(TPDecodeEngine):
             exchange(2 * l + 1, b_hid)
         # ---- vocabulary shard, this rank's best candidate to every rank, global winner
         b_logits = P.new_barrier()
-        R = rows_per_chunk(H)
+        R = rows_per_chunk(H, rows=self.V)
         lm = self._ranges(load, self.V // R, R * H * 2)
         for i, (sm, u0, cnt) in enumerate(lm):
             r0, n = u0 * R, cnt * R
